@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <mutex>
 
 namespace ftk {
@@ -64,10 +65,67 @@ inline int encode_tmap_bnhd(CUtensorMap* out, const void* base, int dtype, int64
   cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
   CUtensorMapDataType dt =
       dtype == FTK_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  CUresult r = fn(out, dt, 4, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&]() {
+    return fn(out, dt, 4, const_cast<void*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // a thread that has made no runtime call yet (autograd's): bind its device's context
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess)
+      return FTK_ERR_CUDA;
+    r = encode();
+  }
   return r == CUDA_SUCCESS ? FTK_OK : FTK_ERR_DRIVER;
+}
+
+// Dynamic shared memory of a kernel, raised once per device and size instead of
+// at every launch (the attribute call costs about a microsecond of host time).
+template <auto KERNEL>
+inline int allow_smem(size_t bytes) {
+  constexpr int MAX_DEVICES = 64;
+  static std::atomic<size_t> allowed[MAX_DEVICES];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return FTK_ERR_CUDA;
+  const bool known = dev >= 0 && dev < MAX_DEVICES;
+  if (known && allowed[dev].load(std::memory_order_relaxed) >= bytes) return FTK_OK;
+  if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(bytes)) != cudaSuccess)
+    return FTK_ERR_CUDA;
+  if (known) {
+    size_t seen = allowed[dev].load(std::memory_order_relaxed);
+    while (seen < bytes && !allowed[dev].compare_exchange_weak(seen, bytes)) {
+    }
+  }
+  return FTK_OK;
+}
+
+// A kernel as a type, for code that is generic over kernels of one signature
+template <auto KERNEL>
+struct Kernel {
+  static constexpr auto kernel = KERNEL;
+};
+
+// Launch that may overlap the tail of the stream's previous kernel.  Only for
+// kernels that call pdl_wait() in every block before they touch global memory.
+template <typename... Params, typename... Args>
+inline int launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                      cudaStream_t st, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) == cudaSuccess
+             ? FTK_OK
+             : FTK_ERR_CUDA;
 }
 
 inline int sm_count() {

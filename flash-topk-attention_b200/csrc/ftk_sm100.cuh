@@ -33,9 +33,26 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// ------------------------------------------- overlapped launches of a stream
+// The launches of one chain of kernels overlap (programmatic stream
+// serialisation, see launch_pdl): a kernel may start while its predecessor
+// drains.  Each kernel therefore waits before its first access to global
+// memory, in every thread block (a block that left without waiting would let
+// the kernel complete before its predecessor, and break the chain), and only
+// then allows its own successor to start.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ------------------------------------------------------------------ mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_inval(uint32_t bar) {
+  asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void mbar_init_fence() {
   // make the inits visible to the async proxy (TMA, tcgen05.commit)

@@ -15,11 +15,13 @@
 // Softmax is single pass against a fixed per-row reference exponent `mref`
 // (an integer in log2 units): sum_j[t] = sum_{i in block j} 2^(c*s_ti - mref),
 // L[t] = sum_j sum_j[t]; the block score is sum_j / L.  mref comes from the
-// row maximum over the first key tile (mode 0).  Should any later logit
-// exceed it by more than the fp32 exponent range the row total overflows;
-// the kernel then raises `*fallback` and the launcher's two follow-up
-// launches (mode 1: exact row maximum, mode 2: sums against it) redo the work.
-// They return at once when the flag is clear.
+// row maximum over the first key tile (pass 0).  Should any later logit
+// exceed it by more than the fp32 exponent range the row total overflows; a
+// CTA that sees this walks its keys twice more (pass 1: exact row maximum,
+// pass 2: sums against it).  The CTA owns its rows, so nobody else has to know:
+// two follow-up launches and the clearing of their flag, which every call paid
+// for (about 2 us of device time each at the smallest sizes, 6-7 us at the
+// largest, and 3 of 5 launches), are not there.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -45,13 +47,10 @@ struct ScoreParams {
   int tiles_per_block;        // bsz > 128: tiles per block, else 0
   int num_tiles;
   int fmt;                    // 0 fp16, 1 bf16
-  int mode;                   // 0 first-tile reference, 1 row max only, 2 given reference
   int H, bh_begin;
   float scale_log2;           // log2(e) * softmax scale
   float* sums;                // [bh_count][N][M]   unnormalised block sums
   float* row_total;           // [bh_count][N]      L
-  float* row_max;             // [bh_count][N]      raw-logit row maximum (modes 1, 2)
-  int* fallback;              // device flag
   int* status;
 };
 
@@ -103,8 +102,6 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
   constexpr int NSTG = score_stages(D);
   constexpr int K_STAGE_BYTES = NCHS * SC_CHUNK_BYTES;
 
-  if (p.mode != 0 && *p.fallback == 0) return;  // uniform: follow-up launches idle
-
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -113,7 +110,8 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
   __shared__ __align__(8) uint64_t bars[1 + 2 * SC_STAGES + 8 + 2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
-  __shared__ float s_mref[SC_QROWS];   // group 0 -> group 1: reference exponent
+  __shared__ int s_redo;
+  __shared__ float s_mref[SC_QROWS];   // group 0 -> group 1: reference exponent / row maximum
   __shared__ float s_part[SC_QROWS];   // group 1 -> group 0: partial total / maximum
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -137,6 +135,7 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
 
   if (tid == 0) {
     abort_flag = 0;
+    s_redo = 0;
     mbar_init(bar_q, 1);
     for (int s = 0; s < SC_STAGES; s++) {
       mbar_init(bar_kfull(s), 1);
@@ -163,19 +162,29 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
   const uint32_t tmem = tmem_base_s;
   WaitCtx w{&abort_flag, p.status};
   const int T = p.num_tiles;
+  float mref = 0.f;    // softmax threads: the row's reference exponent
+  pdl_wait();
+  pdl_launch();
 
+  // Pass 0 is all there is unless a row total overflows.  Every barrier's
+  // phases run on from pass to pass: accumulator a has been used
+  // pass * ((T + 1 - a) / 2) times before, the K ring pass * T * KSPLIT times.
+  for (int pass = 0; pass < 3; pass++) {
   if (warp == 0) {
     // ------------------------------------------------------- TMA producer
     if (lane == 0) {
-      mbar_expect_tx(bar_q, Q_BYTES);
-      for (int half = 0; half < 2; half++)
-        for (int c = 0; c < NCH; c++)
-          tma_load_4d(smem_u32(sQ) + (half * NCH + c) * SC_CHUNK_BYTES, &tm_q, bar_q, c * 64,
-                      h_idx, q0 + half * 128, b_idx);
+      if (pass == 0) {
+        mbar_expect_tx(bar_q, Q_BYTES);
+        for (int half = 0; half < 2; half++)
+          for (int c = 0; c < NCH; c++)
+            tma_load_4d(smem_u32(sQ) + (half * NCH + c) * SC_CHUNK_BYTES, &tm_q, bar_q, c * 64,
+                        h_idx, q0 + half * 128, b_idx);
+      }
       const uint32_t tile_bytes = static_cast<uint32_t>(p.tile_rows) * 128u * NCHS;
+      const int u0 = pass * T * KSPLIT;
       for (int u = 0; u < T * KSPLIT; u++) {
-        const int s = u % NSTG;
-        const uint32_t ph = (u / NSTG) & 1;
+        const int s = (u0 + u) % NSTG;
+        const uint32_t ph = ((u0 + u) / NSTG) & 1;
         if (!mbar_wait(bar_kempty(s), ph ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
         const int t = u / KSPLIT, part = u % KSPLIT;
         const TileInfo ti = tile_info(p, t);
@@ -194,9 +203,9 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
       const uint64_t kdesc0 = smem_desc_sw128(smem_u32(sK), 16, 1024);
       bool ok = mbar_wait(bar_q, 0, w, FTK_DEV_TIMEOUT_MMA);
       for (int t = 0; ok && t < T; t++) {
-        const int u0 = t * KSPLIT;
+        const int u0 = (pass * T + t) * KSPLIT;
         const int a = t & 1;
-        const uint32_t pa = (t >> 1) & 1;
+        const uint32_t pa = (pass * ((T + 1 - a) >> 1) + (t >> 1)) & 1;
         // the three barriers of a tile are waited for together (a test of a
         // completed barrier still takes ~110 cycles) and the tile's UMMAs go
         // out as one batch, so the tensor core is not left idle in between
@@ -253,14 +262,13 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
     float* out_row = p.sums + row_off * p.M;
     const float c = p.scale_log2;
 
-    float mref = 0.f;
     float run_max = -INFINITY;
     float total = 0.f;
     bool ok = true;
 
-    if (p.mode == 2) mref = ceilf(p.row_max[row_off] * c);
+    if (pass == 2) mref = ceilf(s_mref[row_in_cta] * c);
 
-    if (p.mode == 0) {
+    if (pass == 0) {
       if (group == 0) {
         // reference exponent from the row maximum over the first key tile
         ok = mbar_wait(bar_afull(0, half), 0, w, FTK_DEV_TIMEOUT_CONSUMER);
@@ -296,7 +304,7 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
     for (int t = 0; ok && t < T; t++) {
       if (tile_owner(p, t) != group) continue;
       const int a = t & 1;
-      const uint32_t pa = (t >> 1) & 1;
+      const uint32_t pa = (pass * ((T + 1 - a) >> 1) + (t >> 1)) & 1;
       if (!mbar_wait(bar_afull(a, half), pa, w, FTK_DEV_TIMEOUT_CONSUMER)) { ok = false; break; }
       tc_fence_after();
       const TileInfo ti = tile_info(p, t);
@@ -311,7 +319,7 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
         for (int hc = 0; hc < 2; hc++) {
           const int cb = c0 + hc * 16;
           if (cb < ti.used) {
-            if (p.mode == 1) {
+            if (pass == 1) {
 #pragma unroll
               for (int i = 0; i < 16; i++) {
                 const int col = cb + i;
@@ -396,24 +404,27 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
     }
     // combine the two groups' partial results per row: group 1 publishes,
     // group 0 adds (total) or takes the larger (maximum) and writes
-    const float mine = (p.mode == 1) ? run_max : total;
+    const float mine = (pass == 1) ? run_max : total;
     if (group == 1) {
       s_part[row_in_cta] = mine;
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_part);
     } else {
-      if (ok) ok = mbar_wait(bar_part, 0, w, FTK_DEV_TIMEOUT_CONSUMER);
+      if (ok) ok = mbar_wait(bar_part, pass & 1, w, FTK_DEV_TIMEOUT_CONSUMER);
       if (ok && row_ok) {
         const float other = s_part[row_in_cta];
-        if (p.mode == 1) {
-          p.row_max[row_off] = fmaxf(mine, other);
+        if (pass == 1) {
+          s_mref[row_in_cta] = fmaxf(mine, other);
         } else {
           const float tot = mine + other;
           p.row_total[row_off] = tot;
-          if (!(tot > 0.f && tot < 3.0e38f)) atomicExch(p.fallback, 1);
+          if (pass == 0 && !(tot > 0.f && tot < 3.0e38f)) s_redo = 1;
         }
       }
     }
+  }
+  __syncthreads();
+  if (!s_redo || abort_flag) break;
   }
 
   // ------------------------------------------------------------- teardown
@@ -444,22 +455,13 @@ static int launch_score_d(const CUtensorMap& tq, const CUtensorMap& tk, ScorePar
   constexpr int NCH = D / 64;
   const size_t smem =
       1024 + (2 * NCH + score_stages(D) * (NCH / score_ksplit(D))) * SC_CHUNK_BYTES;
-  if (cudaFuncSetAttribute(score_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(smem)) != cudaSuccess)
-    return FTK_ERR_CUDA;
+  if (int e = allow_smem<score_kernel<D>>(smem)) return e;
   dim3 grid((p.N + SC_QROWS - 1) / SC_QROWS, static_cast<unsigned>(bh_count));
-  for (int mode = 0; mode < 3; mode++) {
-    p.mode = mode;
-    score_kernel<D><<<grid, SC_THREADS, smem, st>>>(tq, tk, p);
-    if (cudaGetLastError() != cudaSuccess) return FTK_ERR_CUDA;
-  }
-  return FTK_OK;
+  return launch_pdl(score_kernel<D>, grid, SC_THREADS, smem, st, tq, tk, p);
 }
 
 struct ScoreWs {
   float* row_total;
-  float* row_max;
-  int* fallback;
   float* sums;
 };
 
@@ -469,19 +471,16 @@ static size_t score_ws_layout(int64_t bh_count, int64_t N, int64_t M, bool with_
                               ScoreWs* ws) {
   size_t off = 0;
   const size_t rows = static_cast<size_t>(bh_count) * N;
-  if (ws) ws->fallback = reinterpret_cast<int*>(base + off);
   off += 256;
   if (ws) ws->row_total = reinterpret_cast<float*>(base + off);
-  off += align256(rows * 4);
-  if (ws) ws->row_max = reinterpret_cast<float*>(base + off);
-  off += align256(rows * 4);
+  off += 2 * align256(rows * 4);   // the second row array is no longer used; the size is part of the ABI
   if (ws) ws->sums = reinterpret_cast<float*>(base + off);
   if (with_sums) off += align256(rows * static_cast<size_t>(M) * 4);
   return off;
 }
 
-// Validates arguments, encodes the tensor maps and launches the three score
-// passes; sums go to `sums` ([bh_count][N][M]).
+// Validates arguments, encodes the tensor maps and launches the scoring kernel;
+// sums go to `sums` ([bh_count][N][M]).
 static int run_score(const void* q, const void* k, int dtype, int64_t B, int64_t H, int64_t N,
                      int64_t D, int64_t sq_b, int64_t sq_n, int64_t sq_h, int64_t sk_b,
                      int64_t sk_n, int64_t sk_h, int64_t bh_begin, int64_t bh_count, int bsz,
@@ -493,7 +492,8 @@ static int run_score(const void* q, const void* k, int dtype, int64_t B, int64_t
   if (pad_head < 0 || pad_tail < 0 || pad_head >= bsz || pad_tail >= bsz) return FTK_ERR_BAD_ARG;
   if ((pad_head + N + pad_tail) % bsz != 0) return FTK_ERR_BAD_ARG;
   if (bh_begin < 0 || bh_count <= 0 || bh_begin + bh_count > B * H) return FTK_ERR_BAD_ARG;
-  if (D != 64 && D != 128 && D != 256) return FTK_ERR_UNSUPPORTED;
+  // the tensor maps read columns beyond D as zeros: the kernels' head dims are 64, 128, 256
+  if (D <= 0 || D % 8 != 0 || D > 256) return FTK_ERR_UNSUPPORTED;
   if (bsz % 16 != 0) return FTK_ERR_UNSUPPORTED;
   if (bh_count > 65535) return FTK_ERR_BAD_ARG;
 
@@ -520,8 +520,6 @@ static int run_score(const void* q, const void* k, int dtype, int64_t B, int64_t
   p.scale_log2 = static_cast<float>(1.4426950408889634 * static_cast<double>(scale));
   p.sums = sums;
   p.row_total = ws.row_total;
-  p.row_max = ws.row_max;
-  p.fallback = ws.fallback;
   p.status = status;
 
   CUtensorMap tq, tk;
@@ -529,9 +527,8 @@ static int run_score(const void* q, const void* k, int dtype, int64_t B, int64_t
   if (e) return e;
   e = encode_tmap_bnhd(&tk, k, dtype, B, N, H, D, sk_b, sk_n, sk_h, 64, p.tile_rows);
   if (e) return e;
-  if (cudaMemsetAsync(ws.fallback, 0, 4, st) != cudaSuccess) return FTK_ERR_CUDA;
-  if (D == 64) return launch_score_d<64>(tq, tk, p, bh_count, st);
-  if (D == 256) return launch_score_d<256>(tq, tk, p, bh_count, st);
+  if (D <= 64) return launch_score_d<64>(tq, tk, p, bh_count, st);
+  if (D > 128) return launch_score_d<256>(tq, tk, p, bh_count, st);
   return launch_score_d<128>(tq, tk, p, bh_count, st);
 }
 
@@ -556,6 +553,7 @@ extern "C" int ftk_block_score(const void* q, const void* k, int dtype, int64_t 
                                int32_t* status, void* stream) {
   if (!block_scores) return FTK_ERR_BAD_ARG;
   if (bh_count <= 0 || N <= 0) return FTK_ERR_BAD_ARG;
+  if (D != 64 && D != 128 && D != 256) return FTK_ERR_UNSUPPORTED;
   if (!workspace || workspace_bytes < ftk_block_score_workspace(bh_count, N))
     return FTK_ERR_WORKSPACE;
   if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return FTK_ERR_BAD_ARG;

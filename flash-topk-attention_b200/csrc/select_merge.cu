@@ -29,6 +29,8 @@ topk_select_kernel(const float* __restrict__ scores, const float* __restrict__ r
                    float threshold, int32_t* __restrict__ out_idx, float* __restrict__ out_raw,
                    float* __restrict__ out_avg) {
   extern __shared__ float sel_smem[];
+  pdl_wait();
+  pdl_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * SEL_WARPS + warp;
   if (row >= rows) return;
@@ -118,6 +120,8 @@ topk_select_reg_kernel(const float* __restrict__ scores, const float* __restrict
   constexpr int CAP = IPT >= 4 ? 256 : 128;
   __shared__ float sraw_all[WPC][32 * IPT];
   __shared__ unsigned long long scand_all[IPT >= 2 ? WPC : 1][CAP];
+  pdl_wait();
+  pdl_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // a warp walks rows warp_id, warp_id + warps, ...; the loads of its next row are in
   // flight while it works on the current one (the kernel is otherwise bound by their latency)
@@ -146,7 +150,7 @@ topk_select_reg_kernel(const float* __restrict__ scores, const float* __restrict
 }
 
 template <int IPT>
-static void launch_select_reg(const float* block_scores, const float* row_scale, int64_t rows,
+static int launch_select_reg(const float* block_scores, const float* row_scale, int64_t rows,
                               int M, int M_out, int bsz, int pad_head, int pad_tail,
                               float threshold, int32_t* topk_idx, float* topk_raw,
                               float* topk_avg, cudaStream_t st) {
@@ -154,9 +158,9 @@ static void launch_select_reg(const float* block_scores, const float* row_scale,
   // a few CTAs per SM, each warp looping over rows
   const int64_t want = (rows + WPC - 1) / WPC;
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(want, sm_count() * 16LL));
-  topk_select_reg_kernel<IPT><<<grid, WPC * 32, 0, st>>>(
-      block_scores, row_scale, rows, M, M_out, bsz, pad_head, pad_tail, threshold, topk_idx,
-      topk_raw, topk_avg);
+  return launch_pdl(topk_select_reg_kernel<IPT>, grid, WPC * 32, 0, st, block_scores, row_scale,
+                    rows, M, M_out, bsz, pad_head, pad_tail, threshold, topk_idx, topk_raw,
+                    topk_avg);
 }
 
 int select_launch(const float* block_scores, const float* row_scale, int64_t rows, int M,
@@ -171,7 +175,7 @@ int select_launch(const float* block_scores, const float* row_scale, int64_t row
   if (2 * grid > 0x7fffffffLL) return FTK_ERR_BAD_ARG;
   const unsigned g = static_cast<unsigned>(grid);
 #define FTK_SEL_REG(IPT)                                                                        \
-  launch_select_reg<IPT>(block_scores, row_scale, rows, M, M_out, bsz, pad_head, pad_tail,     \
+  return launch_select_reg<IPT>(block_scores, row_scale, rows, M, M_out, bsz, pad_head, pad_tail,     \
                          threshold, topk_idx, topk_raw, topk_avg, st)
   if (M <= 32) FTK_SEL_REG(1);
   else if (M <= 64) FTK_SEL_REG(2);
@@ -179,20 +183,12 @@ int select_launch(const float* block_scores, const float* row_scale, int64_t row
   else if (M <= 256) FTK_SEL_REG(8);
   else if (M <= 512) FTK_SEL_REG(16);
   else if (M <= 1024) FTK_SEL_REG(32);
-  else {
-    const int Mp = (M + 31) & ~31;
-    const size_t smem = static_cast<size_t>(SEL_WARPS) * 2 * Mp * sizeof(float);
-    if (smem > 48 * 1024) {
-      if (cudaFuncSetAttribute(topk_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(smem)) != cudaSuccess)
-        return FTK_ERR_CUDA;
-    }
-    topk_select_kernel<<<g, SEL_WARPS * 32, smem, st>>>(
-        block_scores, row_scale, rows, M, M_out, bsz, pad_head, pad_tail, threshold, topk_idx,
-        topk_raw, topk_avg);
-  }
 #undef FTK_SEL_REG
-  return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
+  const int Mp = (M + 31) & ~31;
+  const size_t smem = static_cast<size_t>(SEL_WARPS) * 2 * Mp * sizeof(float);
+  if (int e = allow_smem<topk_select_kernel>(smem)) return e;
+  return launch_pdl(topk_select_kernel, g, SEL_WARPS * 32, smem, st, block_scores, row_scale, rows,
+                    M, M_out, bsz, pad_head, pad_tail, threshold, topk_idx, topk_raw, topk_avg);
 }
 
 // ------------------------------------------------------------------- merge
@@ -212,6 +208,8 @@ qblock_merge_kernel(const int32_t* __restrict__ idx, const float* __restrict__ s
                     int32_t* __restrict__ out_idx, float* __restrict__ out_scr,
                     int32_t* __restrict__ counts, int* status) {
   extern __shared__ unsigned long long mg_keys[];
+  pdl_wait();
+  pdl_launch();
   float* agg = reinterpret_cast<float*>(mg_keys + Mp);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t qb = blockIdx.x;  // bh * QM + m
@@ -360,6 +358,8 @@ qblock_merge_warp_kernel(const int32_t* __restrict__ idx, const float* __restric
   constexpr int U = 4;   // steps fetched and checked together
   __shared__ float agg_all[MGW_WARPS][MP];
   __shared__ uint8_t tag_all[MGW_WARPS][U * MP];
+  pdl_wait();
+  pdl_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t qb = static_cast<int64_t>(blockIdx.x) * MGW_WARPS + warp;  // bh * QM + m
   if (qb >= total_qb) return;
@@ -852,29 +852,24 @@ extern "C" int ftk_qblock_merge(const int32_t* topk_idx, const float* topk_score
     // one warp per q-block
     const int64_t total_qb = BH * QM;
     const unsigned grid = static_cast<unsigned>((total_qb + MGW_WARPS - 1) / MGW_WARPS);
-#define FTK_MGW(E)                                                                          \
-  qblock_merge_warp_kernel<E><<<grid, MGW_WARPS * 32, 0, st>>>(                             \
-      topk_idx, topk_scores, N, K, q_block_size, q_pad_head, static_cast<int>(QM), total_qb, \
-      num_score_blocks, qblock_topk, merged_idx, merged_scores, counts, status)
+#define FTK_MGW(E)                                                                             \
+  return launch_pdl(qblock_merge_warp_kernel<E>, grid, MGW_WARPS * 32, 0, st, topk_idx,         \
+                    topk_scores, N, K, q_block_size, q_pad_head, static_cast<int>(QM), total_qb, \
+                    num_score_blocks, qblock_topk, merged_idx, merged_scores, counts, status)
     switch (Mp) {
-      case 32: FTK_MGW(1); break;
-      case 64: FTK_MGW(2); break;
-      case 128: FTK_MGW(4); break;
-      case 256: FTK_MGW(8); break;
-      case 512: FTK_MGW(16); break;
-      default: FTK_MGW(32); break;
+      case 32: FTK_MGW(1);
+      case 64: FTK_MGW(2);
+      case 128: FTK_MGW(4);
+      case 256: FTK_MGW(8);
+      case 512: FTK_MGW(16);
+      default: FTK_MGW(32);
     }
 #undef FTK_MGW
-    return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
   }
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(qblock_merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(smem)) != cudaSuccess)
-    return FTK_ERR_CUDA;
-  qblock_merge_kernel<<<static_cast<unsigned>(BH * QM), MG_THREADS, smem, st>>>(
-      topk_idx, topk_scores, N, K, q_block_size, q_pad_head, static_cast<int>(QM),
-      num_score_blocks, Mp, qblock_topk, merged_idx, merged_scores, counts, status);
-  return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
+  if (int e = allow_smem<qblock_merge_kernel>(smem)) return e;
+  return launch_pdl(qblock_merge_kernel, static_cast<unsigned>(BH * QM), MG_THREADS, smem, st,
+                    topk_idx, topk_scores, N, K, q_block_size, q_pad_head, static_cast<int>(QM),
+                    num_score_blocks, Mp, qblock_topk, merged_idx, merged_scores, counts, status);
 }
 
 extern "C" int ftk_qblock_union(const int32_t* topk_idx, int64_t BH, int64_t N, int K,

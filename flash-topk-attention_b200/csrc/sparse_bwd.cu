@@ -21,44 +21,100 @@
 #include <cstdlib>
 
 #include "attn_common.cuh"
+#include "attn_host.cuh"
 #include "ftk_host.cuh"
 #include "ftk_sm100.cuh"
 
 namespace ftk {
 
+constexpr int BW_THREADS = 576;  // 2 + 2 x 8 warps
+constexpr int BW_MAX_STAGES = 4;
+constexpr int DQ_KST = 7;        // dQ kernel: K tiles in the ring (held until dQ += dS K ran)
+constexpr int DQ_VST = 5;        // dQ kernel: V tiles in the ring (free once dP is computed)
+
+struct BwdParams {
+  int N, H, D, QM, W, Mkv;
+  int g, kvb, q_pad_head, kv_pad_head;
+  int G, fmt, nstages;
+  float scale, scale_log2;
+  const int32_t* lists;      // dQ: [BH][list_rows][W]; dKV: reverse_idx [BH][Mkv][QM] or null
+  int list_rows;
+  ListMap lm;
+  const int32_t* counts;     // dKV with `lists`: reverse_counts [BH][Mkv]
+  uint8_t* masks;            // [BH][mask_tiles][mask_stride]: dQ writes (when given), dKV reads
+  int mask_stride, mask_tiles, mask_g;
+  const float* lse;
+  float* delta;              // [BH][N]: dQ writes, dKV reads
+  const uint8_t* o;          // dQ: forward result and its gradient, for delta
+  const uint8_t* dout;
+  int64_t so_b, so_n, so_h, sd_b, sd_n, sd_h;
+  void* out0;                // dQ kernel: dq ; dKV kernel: dk
+  void* out1;                //                  dKV kernel: dv
+  int64_t s0_b, s0_n, s0_h, s1_b, s1_n, s1_h;
+  int out_f32;               // o, dq, dk, dv are float32
+  int* status;
+  int kv_hdiv;               // query heads per kv head (grouped-query attention), 1 otherwise
+  int heads;                 // dKV: query heads one CTA walks (kv_hdiv, or 1: one result per query head)
+  int span;                  // dKV with heads > 1: ids per head in the union (multiple of 32)
+  const int32_t* order;      // dKV: kv blocks by fan-in, heaviest first ([BH][Mkv]) or null
+  const int32_t* tile_order; // dKV: 128-row kv tiles by number of q-blocks, heaviest first, or null
+};
+
 // ------------------------------------------------------------------- delta
-// delta[bh][n] = sum_d o * do.  D / 8 lanes per (b, n, h) row, each with one
-// 16-byte load per tensor (rows start on 16-byte boundaries: base pointers are
-// 16-byte aligned and strides multiples of 8 elements), so a warp covers
-// 256 / D rows at once.
-__global__ void delta_kernel(const uint8_t* __restrict__ o, const uint8_t* __restrict__ dout,
-                             int fmt, int64_t B, int64_t N, int64_t H, int D, int64_t so_b,
-                             int64_t so_n, int64_t so_h, int64_t sd_b, int64_t sd_n, int64_t sd_h,
-                             float* __restrict__ delta) {
-  const int lpr = D >> 3;                         // lanes per row: 8, 16 or 32
-  const int rpw = 32 / lpr;                       // rows per warp
-  const int lane = threadIdx.x & 31;
-  const int64_t wid = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
-  const int64_t row = wid * rpw + lane / lpr;
-  const int c = lane % lpr;
-  float acc = 0.f;
-  if (row < B * N * H) {
-    const int64_t h = row % H, n = (row / H) % N, b = row / (H * N);
-    const uint4 vo = __ldg(reinterpret_cast<const uint4*>(o + 2 * (b * so_b + n * so_n + h * so_h)) + c);
-    const uint4 vd =
-        __ldg(reinterpret_cast<const uint4*>(dout + 2 * (b * sd_b + n * sd_n + h * sd_h)) + c);
-    const uint32_t wo[4] = {vo.x, vo.y, vo.z, vo.w}, wd[4] = {vd.x, vd.y, vd.z, vd.w};
+// delta[row] = sum_d o * do for the 128 rows of a dQ tile, by all warps of the
+// CTA, into shared memory (for the tile itself) and global memory (for dK/dV).
+// kd / 8 lanes per row, each with one 16-byte load per tensor, so a warp covers
+// 256 / kd rows at once and a thread has all of its loads in flight together.
+// As a kernel of its own this cost a launch and 258 us at N = 32768, H = 32,
+// D = 128 (122 us at B = 4, N = 8192, H = 16), reading O and dO at 4.2 TB/s;
+// here the reads hide behind the other CTAs' UMMAs.
+template <int KD>
+__device__ __forceinline__ void tile_delta(const BwdParams& p, float* s_delta, int bh, int b, int h,
+                                           int tile_row0, int rows) {
+  constexpr int LPR = KD / 8, RPW = 32 / LPR, WARPS = BW_THREADS / 32;
+  constexpr int STEPS = (128 + RPW * WARPS - 1) / (RPW * WARPS);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = lane % LPR;
+  const int64_t ob = static_cast<int64_t>(b) * p.so_b + static_cast<int64_t>(h) * p.so_h,
+                db = static_cast<int64_t>(b) * p.sd_b + static_cast<int64_t>(h) * p.sd_h;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const float2 a = unpack2(wo[i], fmt), g = unpack2(wd[i], fmt);
-      acc = fmaf(a.x, g.x, acc);
-      acc = fmaf(a.y, g.y, acc);
+  for (int i = 0; i < STEPS; i++) {
+    const int r = (i * WARPS + warp) * RPW + lane / LPR;
+    const int n = tile_row0 + r;
+    const bool in = r < rows && n >= 0 && n < p.N && c * 8 < p.D;
+    float acc = 0.f;
+    if (in) {
+      const uint4 vd = __ldg(reinterpret_cast<const uint4*>(
+          p.dout + 2 * (db + static_cast<int64_t>(n) * p.sd_n)) + c);
+      const uint32_t wd[4] = {vd.x, vd.y, vd.z, vd.w};
+      float2 fo[4];
+      const int64_t oe = ob + static_cast<int64_t>(n) * p.so_n;
+      if (p.out_f32) {
+        const float4* src = reinterpret_cast<const float4*>(p.o + 4 * oe) + 2 * c;
+        const float4 x = __ldg(src), y = __ldg(src + 1);
+        fo[0] = make_float2(x.x, x.y);
+        fo[1] = make_float2(x.z, x.w);
+        fo[2] = make_float2(y.x, y.y);
+        fo[3] = make_float2(y.z, y.w);
+      } else {
+        const uint4 vo = __ldg(reinterpret_cast<const uint4*>(p.o + 2 * oe) + c);
+        fo[0] = unpack2(vo.x, p.fmt);
+        fo[1] = unpack2(vo.y, p.fmt);
+        fo[2] = unpack2(vo.z, p.fmt);
+        fo[3] = unpack2(vo.w, p.fmt);
+      }
+#pragma unroll
+      for (int x = 0; x < 4; x++) {
+        const float2 gd = unpack2(wd[x], p.fmt);
+        acc = fmaf(fo[x].x, gd.x, acc);
+        acc = fmaf(fo[x].y, gd.y, acc);
+      }
     }
-  }
-  for (int d = lpr >> 1; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
-  if (c == 0 && row < B * N * H) {
-    const int64_t h = row % H, n = (row / H) % N, b = row / (H * N);
-    delta[(b * H + h) * N + n] = acc;
+#pragma unroll
+    for (int d = LPR >> 1; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+    if (c == 0 && r < 128) {
+      s_delta[r] = acc;
+      if (in) p.delta[static_cast<int64_t>(bh) * p.N + n] = acc;
+    }
   }
 }
 
@@ -123,28 +179,6 @@ __device__ __forceinline__ void pt_pairs(const uint32_t (&sv)[16], const uint32_
   }
 }
 
-constexpr int BW_THREADS = 576;  // 2 + 2 x 8 warps
-constexpr int BW_MAX_STAGES = 4;
-constexpr int DQ_KST = 7;        // dQ kernel: K tiles in the ring (held until dQ += dS K ran)
-constexpr int DQ_VST = 5;        // dQ kernel: V tiles in the ring (free once dP is computed)
-
-struct BwdParams {
-  int N, H, QM, W, Mkv;
-  int g, kvb, q_pad_head, kv_pad_head;
-  int G, fmt, nstages;
-  float scale, scale_log2;
-  const int32_t* lists;      // dQ: merged [BH][QM][W]; dKV: reverse_idx [BH][Mkv][QM]
-  const int32_t* counts;     // dKV: reverse_counts [BH][Mkv]
-  const float* lse;
-  const float* delta;
-  void* out0;                // dQ kernel: dq ; dKV kernel: dk
-  void* out1;                //                  dKV kernel: dv
-  int64_t s0_b, s0_n, s0_h, s1_b, s1_n, s1_h;
-  int* status;
-  int kv_hdiv;               // query heads per kv head (grouped-query attention), 1 otherwise
-  const int32_t* order;      // dKV: kv blocks by fan-in, heaviest first ([BH][Mkv]) or null
-};
-
 // ---------------------------------------------------------------------- dQ
 // TMEM columns: Q 0..63 and dO 64..127 (16-bit pairs: the A operands of the
 // S and dP UMMAs are read from TMEM, which leaves shared-memory bandwidth to
@@ -179,6 +213,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   uint8_t* sV = smem;                          // over Q / dO once they are in TMEM
   uint8_t* sK = smem + 2 * ROW_TILE_BYTES;
   __shared__ UnionScratch un;
+  __shared__ float s_delta[128];
   __shared__ __align__(8) uint64_t bars[1 + 2 * DQ_KST + 2 * DQ_VST + 6];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
@@ -237,8 +272,15 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_alloc(smem_u32(&tmem_base_s), 512);
     tmem_relinquish();
   }
-  const int n = build_union(un, p.lists + (static_cast<int64_t>(bh) * p.QM + m0) * p.W, p.W,
-                            groups, p.W, nullptr, p.Mkv, p.status);
+  clear_bitmaps(un);
+  pdl_wait();
+  pdl_launch();
+  tile_delta<D>(p, s_delta, bh, b_idx, h_idx, tile_row0, groups * p.g);
+  const int n = build_union(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
+                            p.W, nullptr, p.Mkv, p.lm, p.status);
+  if (p.masks)
+    write_tile_masks(un, p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + blockIdx.x) * p.mask_stride,
+                     p.mask_stride, 0, groups);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -393,7 +435,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
     float lse2 = 0.f, dl = 0.f;
     if (row_valid) {
       lse2 = p.lse[static_cast<int64_t>(bh) * p.N + qrow] * 1.4426950408889634f;
-      dl = p.delta[static_cast<int64_t>(bh) * p.N + qrow];
+      dl = s_delta[r];
     }
     bool ok = true;
     if (!BIG && n > 0 && colhalf == 0) {
@@ -434,12 +476,19 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       const int lo = max(0, -tok0), hi = min(p.kvb, p.N - tok0);
       const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == p.kvb;
+      const bool none = !fast && !__any_sync(0xffffffffu, act);
       // dS of columns [c0, c0+w) is written over dP columns [cbeg + (c0-cbeg)/2, ..):
       // columns this thread has already read, never another warp's
       for (int c0 = cbeg; c0 < cend; c0 += 32) {
         const uint32_t ds_addr = dp_addr + cbeg + ((c0 - cbeg) >> 1);
         if (cend - c0 >= 32) {
           uint32_t sv[32], dv[32], pk[16];
+          if (none) {   // the other group's block: dS = 0, nothing to read
+#pragma unroll
+            for (int x = 0; x < 16; x++) pk[x] = 0u;
+            tmem_st16(ds_addr, pk);
+            continue;
+          }
           tmem_ld32(s_addr + c0, sv);
           tmem_ld32(dp_addr + c0, dv);
           tmem_wait_ld();
@@ -492,7 +541,8 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       uint8_t* orow = nullptr;
       if (row_valid)
         orow = static_cast<uint8_t*>(p.out0) +
-               2 * (static_cast<int64_t>(b_idx) * p.s0_b + static_cast<int64_t>(qrow) * p.s0_n +
+               (p.out_f32 ? 4 : 2) *
+                   (static_cast<int64_t>(b_idx) * p.s0_b + static_cast<int64_t>(qrow) * p.s0_n +
                     static_cast<int64_t>(h_idx) * p.s0_h);
       // 32-column chunks of the head dim are dealt round-robin to the four
       // warps of a lane quarter
@@ -510,10 +560,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
             const float b = n > 0 ? __uint_as_float(v[x + 1]) * p.scale : 0.f;
             pk[x >> 1] = pack2(a, b, p.fmt);
           }
-          uint4* dst = reinterpret_cast<uint4*>(orow + c0 * 2);
-#pragma unroll
-          for (int x = 0; x < 4; x++)
-            dst[x] = make_uint4(pk[4 * x], pk[4 * x + 1], pk[4 * x + 2], pk[4 * x + 3]);
+          store_row_part(orow, c0, p.D, pk, p.fmt, p.out_f32 != 0);
         }
       }
     }
@@ -526,6 +573,37 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
 }
 
 // -------------------------------------------------------------------- dK/dV
+// Union of the lists of kv blocks j0 .. j0 + groups - 1, from the dQ kernel's
+// tile masks or from a reverse index.
+__device__ __forceinline__ int dkv_union(UnionScratch& un, const BwdParams& p, int bhq, int j0,
+                                         int groups) {
+  clear_bitmaps(un);
+  pdl_wait();
+  pdl_launch();
+  if (p.masks) {
+    const int64_t per_head = static_cast<int64_t>(p.mask_tiles) * p.mask_stride;
+    return build_union_masks(un, p.masks + bhq * per_head, p.mask_stride, p.mask_tiles, p.mask_g, j0,
+                             groups, p.heads, per_head, p.span);
+  }
+  const int64_t kv_row = static_cast<int64_t>(bhq) * p.Mkv + j0;
+  return build_union(un, p.lists + kv_row * p.QM, 0, groups, p.QM, p.counts + kv_row, p.QM,
+                     ListMap{0, 0, 0, 0}, p.status);
+}
+
+// Entry id of the union -> q-block, with the query head it belongs to (ids come
+// in ascending order, head by head).  Without WALK ids are q-blocks.
+template <bool WALK>
+struct HeadWalk {
+  int head = 0, first = 0;
+  __device__ __forceinline__ int at(int id, const BwdParams& p) {
+    while (WALK && id - first >= p.span) {
+      first += p.span;
+      head++;
+    }
+    return id - first;
+  }
+};
+
 // TMEM columns: S^T[2] 0/64 (P^T written over their first half), dP^T[2]
 // 128/192 (dS^T likewise), dV 256.., dK 384..
 // MODE 0 (head dims up to 128) produces dV and dK in one launch.  At head dim
@@ -533,7 +611,8 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
 // work goes in two launches with one accumulator at columns 256..511 each:
 // MODE 1 = dV only (needs neither V nor dP^T: K alone stays resident, which
 // leaves room for four ring stages), MODE 2 = dK only.
-template <int D, int MODE>
+// WALK: see sparse_bwd_dkv2_kernel.
+template <int D, int MODE, bool WALK>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
                       const __grid_constant__ CUtensorMap tm_do,
@@ -557,10 +636,16 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int bh = blockIdx.y;
   int j0 = blockIdx.x * p.G;                // first kv block of the tile
-  if (p.order) {
-    // Heaviest tiles first: the grid has one CTA per kv block, in the order of
-    // `order` (fan-in descending, ties by lower id); the CTA whose block is the
-    // first of its tile in that order does the tile, the others leave at once.
+  if (p.tile_order) {
+    // heaviest tiles first, see fan_in_kernel
+    pdl_wait();
+    j0 = p.tile_order[static_cast<int64_t>(bh) * gridDim.x + blockIdx.x] * p.G;
+  } else if (p.order) {
+    // The same from a reverse index, which orders kv blocks: the grid has one CTA
+    // per kv block, in the order of `order` (fan-in descending, ties by lower id);
+    // the CTA whose block is the first of its tile in that order does the tile,
+    // the others leave at once.
+    pdl_wait();
     const int32_t* cnt = p.counts + static_cast<int64_t>(bh) * p.Mkv;
     const int j = p.order[static_cast<int64_t>(bh) * p.Mkv + blockIdx.x];
     if (j < 0 || j >= p.Mkv) return;
@@ -571,7 +656,10 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
       if (jj != j && (cc > cj || (cc == cj && jj < j))) return;
     }
   }
-  const int b_idx = bh / p.H, h_idx = bh - b_idx * p.H;
+  // slice = (batch, first of the query heads this CTA walks)
+  const int slices = WALK ? p.H / p.heads : p.H;
+  const int b_idx = bh / slices, h_idx = (bh - b_idx * slices) * (WALK ? p.heads : 1);
+  const int bhq = WALK ? b_idx * p.H + h_idx : bh;
   const int groups = min(p.G, p.Mkv - j0);
   const int tile_tok0 = j0 * p.kvb - p.kv_pad_head;
   const int q_chunk_bytes = p.g * 128;
@@ -608,9 +696,7 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_alloc(smem_u32(&tmem_base_s), 512);
     tmem_relinquish();
   }
-  const int64_t kv_row = static_cast<int64_t>(bh) * p.Mkv + j0;
-  const int n = build_union(un, p.lists + kv_row * p.QM, p.QM, groups, p.QM, p.counts + kv_row,
-                            p.QM, p.status);
+  const int n = dkv_union(un, p, bhq, j0, groups);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -628,16 +714,18 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
           tma_load_4d(smem_u32(sV) + c * 128 * 128, &tm_v, bar_kv, c * 64, h_idx / p.kv_hdiv,
                       tile_tok0, b_idx);
       }
+      HeadWalk<WALK> hw;
       for (int i = 0; i < n; i++) {
         const int s = i % NST;
         if (!mbar_wait(bar_qempty(s), ((i / NST) & 1) ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
-        const int row0 = static_cast<int>(un.ids[i]) * p.g - p.q_pad_head;
+        const int row0 = hw.at(un.ids[i], p) * p.g - p.q_pad_head;
         const uint32_t base = smem_u32(sQD) + s * stage_bytes;
         mbar_expect_tx(bar_qfull(s), stage_bytes);
         for (int c = 0; c < NCH; c++) {
-          tma_load_4d(base + c * q_chunk_bytes, &tm_q, bar_qfull(s), c * 64, h_idx, row0, b_idx);
-          tma_load_4d(base + (NCH + c) * q_chunk_bytes, &tm_do, bar_qfull(s), c * 64, h_idx, row0,
+          tma_load_4d(base + c * q_chunk_bytes, &tm_q, bar_qfull(s), c * 64, h_idx + hw.head, row0,
                       b_idx);
+          tma_load_4d(base + (NCH + c) * q_chunk_bytes, &tm_do, bar_qfull(s), c * 64,
+                      h_idx + hw.head, row0, b_idx);
         }
       }
     }
@@ -759,15 +847,17 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
     // every thread of a group runs all of the group's rounds (its named
     // barrier needs all 256); after a failed wait a thread only keeps the
     // barrier company and does no more work.
+    HeadWalk<WALK> hw;
     for (int i = wg; i < n; i += 2) {
       const int pb = (i >> 1) & 1;           // per-group double buffer of lse / delta
-      const int row0 = static_cast<int>(un.ids[i]) * p.g - p.q_pad_head;
+      const int row0 = hw.at(un.ids[i], p) * p.g - p.q_pad_head;
       if (ct < p.g) {
         const int t = row0 + ct;
         float l2 = 0.f, dl = 0.f;
         if (t >= 0 && t < p.N) {   // staged negated: the packed fma / add take them as they are
-          l2 = -p.lse[static_cast<int64_t>(bh) * p.N + t] * 1.4426950408889634f;
-          dl = -p.delta[static_cast<int64_t>(bh) * p.N + t];
+          const int64_t e = static_cast<int64_t>(bhq + hw.head) * p.N + t;
+          l2 = -p.lse[e] * 1.4426950408889634f;
+          dl = -p.delta[e];
         }
         s_lse2[wg][pb][ct] = l2;
         s_delta[wg][pb][ct] = dl;
@@ -785,12 +875,21 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
       const int lo = max(0, -row0), hi = min(p.g, p.N - row0);
       const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == p.g;
+      const bool none = !fast && !__any_sync(0xffffffffu, act);
       const float4* l4 = reinterpret_cast<const float4*>(s_lse2[wg][pb]);
       const float4* d4 = reinterpret_cast<const float4*>(s_delta[wg][pb]);
       // P^T / dS^T of columns [c0, c0+16) go over columns cbeg + (c0-cbeg)/2 ..
       // of the S^T / dP^T regions: columns this thread has already read
       for (int c0 = cbeg; c0 < cend; c0 += 16) {
         uint32_t sv[16], dv[16], pp[8], pd[8];
+        const int oc = cbeg + ((c0 - cbeg) >> 1);
+        if (none) {   // the other group's q-block: P^T = dS^T = 0, nothing to read
+#pragma unroll
+          for (int x = 0; x < 8; x++) pp[x] = 0u;
+          if (MODE != 2) tmem_st8(st_addr + oc, pp);
+          if (MODE != 1) tmem_st8(dp_addr + oc, pp);
+          continue;
+        }
         tmem_ld16(st_addr + c0, sv);
         if (MODE != 1) tmem_ld16(dp_addr + c0, dv);
         tmem_wait_ld();
@@ -822,7 +921,6 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
             pd[(x >> 1) + 1] = pack2(dsv[2], dsv[3], p.fmt);
           }
         }
-        const int oc = cbeg + ((c0 - cbeg) >> 1);
         if (MODE != 2) tmem_st8(st_addr + oc, pp);
         if (MODE != 1) tmem_st8(dp_addr + oc, pd);
       }
@@ -844,8 +942,9 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
       const float mul = which == 0 ? 1.f : p.scale;
       uint8_t* orow = nullptr;
       if (row_valid)
-        orow = base + 2 * (static_cast<int64_t>(b_idx) * sb_ + static_cast<int64_t>(tok) * sn_ +
-                           static_cast<int64_t>(h_idx) * sh_);
+        orow = base + (p.out_f32 ? 4 : 2) *
+                          (static_cast<int64_t>(b_idx) * sb_ + static_cast<int64_t>(tok) * sn_ +
+                           static_cast<int64_t>(WALK ? h_idx / p.heads : h_idx) * sh_);
       const int cfirst = MODE == 0 ? colhalf * 32 : (wg * 2 + colhalf) * 32;
       for (int c0 = cfirst; c0 < D; c0 += (MODE == 0 ? 64 : 128)) {
         uint32_t v[32];
@@ -861,10 +960,7 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
             const float b = n > 0 ? __uint_as_float(v[x + 1]) * mul : 0.f;
             pk[x >> 1] = pack2(a, b, p.fmt);
           }
-          uint4* dst = reinterpret_cast<uint4*>(orow + c0 * 2);
-#pragma unroll
-          for (int x = 0; x < 4; x++)
-            dst[x] = make_uint4(pk[4 * x], pk[4 * x + 1], pk[4 * x + 2], pk[4 * x + 3]);
+          store_row_part(orow, c0, p.D, pk, p.fmt, p.out_f32 != 0);
         }
       }
     }
@@ -883,27 +979,438 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
 
 namespace ftk {
 
-static int bwd_common_checks(int dtype, int64_t B, int64_t H, int64_t N, int64_t D, int QM, int g,
-                             int kvb, int q_pad_head, int kv_pad_head) {
-  if (B <= 0 || H <= 0 || N <= 0 || QM <= 0) return FTK_ERR_BAD_ARG;
-  if (dtype != FTK_DTYPE_F16 && dtype != FTK_DTYPE_BF16) return FTK_ERR_BAD_ARG;
-  if (g <= 0 || kvb <= 0) return FTK_ERR_BAD_ARG;
-  if (q_pad_head < 0 || q_pad_head >= g || kv_pad_head < 0 || kv_pad_head >= kvb)
-    return FTK_ERR_BAD_ARG;
-  if (static_cast<int64_t>(QM) * g < q_pad_head + N) return FTK_ERR_BAD_ARG;
-  if (D != 64 && D != 128 && D != 256) return FTK_ERR_UNSUPPORTED;
-  if (kvb % 16 != 0 || kvb > 64) return FTK_ERR_UNSUPPORTED;
-  if (B * H > 65535) return FTK_ERR_BAD_ARG;
+// ---------------------------------------------------- order of the dK/dV tiles
+// Per slice: q-blocks that each 128-row kv tile has to walk, from the dQ
+// kernel's tile masks, and the tiles sorted by that number, largest first (ties:
+// lower tile).  With skewed lists a few tiles take many times the others' time;
+// issued last they would run alone.  One CTA per slice, key = (count + 1, ~tile).
+constexpr int FAN_THREADS = 1024;
+
+__global__ void __launch_bounds__(FAN_THREADS)
+fan_in_kernel(const uint8_t* __restrict__ masks, int stride, int tiles, int64_t head_stride,
+              int heads, int slices_per_b, int H, int Mkv, int G, int cols, int colsp,
+              int32_t* __restrict__ order) {
+  extern __shared__ unsigned long long fan_keys[];
+  unsigned* cnt = reinterpret_cast<unsigned*>(fan_keys + colsp);
+  pdl_wait();
+  pdl_launch();
+  const int tid = threadIdx.x;
+  const int slice = blockIdx.x;
+  const int bhq = slice / slices_per_b * H + slice % slices_per_b * heads;
+  for (int x = tid; x < colsp; x += FAN_THREADS) cnt[x] = 0u;
+  __syncthreads();
+  const int parts = max(1, FAN_THREADS / cols);
+  for (int u = tid; u < cols * parts; u += FAN_THREADS) {
+    const int col = u % cols, part = u / cols;
+    const int j0 = col * G, jn = min(G, Mkv - j0);
+    unsigned c = 0;
+    for (int r = part; r < heads * tiles; r += parts) {
+      const int h = r / tiles;
+      const uint8_t* src = masks + (bhq + h) * head_stride +
+                           static_cast<int64_t>(r - h * tiles) * stride + j0;
+      unsigned m = 0;
+      for (int j = 0; j < jn; j++) m |= src[j];
+      c += __popc(m);
+    }
+    atomicAdd(&cnt[col], c);
+  }
+  __syncthreads();
+  for (int x = tid; x < colsp; x += FAN_THREADS)
+    fan_keys[x] = x < cols ? (static_cast<unsigned long long>(cnt[x] + 1u) << 32) |
+                                 (0xffffffffu - static_cast<unsigned>(x))
+                           : 0ull;
+  __syncthreads();
+  for (int k = 2; k <= colsp; k <<= 1)
+    for (int d = k >> 1; d > 0; d >>= 1) {
+      for (int i = tid; i < colsp; i += FAN_THREADS) {
+        const int o = i ^ d;
+        if (o > i) {
+          const unsigned long long a = fan_keys[i], b = fan_keys[o];
+          if (((i & k) == 0) ? (a < b) : (a > b)) {
+            fan_keys[i] = b;
+            fan_keys[o] = a;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  for (int x = tid; x < cols; x += FAN_THREADS)
+    order[static_cast<int64_t>(slice) * cols + x] =
+        static_cast<int32_t>(0xffffffffu - static_cast<unsigned>(fan_keys[x]));
+}
+
+// ------------------------------------------- sum over the heads of a kv head
+// dk, dv of every query head ([B][N][H][D], 16-bit) -> one per kv head: the
+// heads of a group added up in fp32, in order, and rounded once.  Bound by
+// memory (2 * H * D * 2 B read per token, 16 bytes per thread and load); used
+// where the grid is too small for one CTA to walk all heads of a group.
+__global__ void __launch_bounds__(256)
+head_sum_kernel(const uint8_t* __restrict__ dk_part, const uint8_t* __restrict__ dv_part, int fmt,
+                int64_t N, int Hkv, int grp, int D, int64_t vecs, void* dk, int64_t k_b, int64_t k_n,
+                int64_t k_h, void* dv, int64_t v_b, int64_t v_n, int64_t v_h, int f32) {
+  pdl_wait();
+  pdl_launch();
+  const int dvec = D >> 3;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= vecs) return;
+  const uint4* src = reinterpret_cast<const uint4*>(blockIdx.y ? dv_part : dk_part);
+  const int64_t head = i / dvec;                 // (b * N + n) * Hkv + hk
+  const int c = static_cast<int>(i - head * dvec);
+  const int64_t row = head / Hkv;
+  const int hk = static_cast<int>(head - row * Hkv);
+  const int64_t b = row / N, n = row - b * N;
+  float acc[8];
+#pragma unroll
+  for (int x = 0; x < 8; x++) acc[x] = 0.f;
+  const uint4* s = src + head * grp * dvec + c;
+  for (int g = 0; g < grp; g++) {
+    const uint4 t = __ldg(s + static_cast<int64_t>(g) * dvec);
+    const uint32_t w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+      const float2 f = unpack2(w[x], fmt);
+      acc[2 * x] += f.x;
+      acc[2 * x + 1] += f.y;
+    }
+  }
+  uint32_t pk[4];
+#pragma unroll
+  for (int x = 0; x < 4; x++) pk[x] = pack2(acc[2 * x], acc[2 * x + 1], fmt);
+  uint8_t* out = static_cast<uint8_t*>(blockIdx.y ? dv : dk);
+  const int64_t e = blockIdx.y ? b * v_b + n * v_n + hk * v_h : b * k_b + n * k_n + hk * k_h;
+  store_row_part(out + (f32 ? 4 : 2) * e, c * 8, D, pk, fmt, f32 != 0);
+}
+
+// ------------------------------------------------------------------- host side
+// What a backward pass shares between its two calls: the grid of blocks and
+// where things lie in the workspace.
+struct BwdPlan {
+  AttnGrid gr;
+  bool pair;                 // kernels on pairs of SMs
+  bool walk;                 // dK/dV: one CTA walks all query heads of its kv head
+  int tiles, stride, span;   // tile masks (see write_tile_masks)
+  int kv_tiles;              // 128-row kv tiles per slice
+  bool order;                // dK/dV tiles sorted by the work they have
+  size_t off_masks, off_order, off_dk, off_dv, bytes;
+};
+
+static size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
+
+static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
+  BwdPlan b{};
+  // head dim 256: the kernels hold Q / dO (dQ) or K / V (dK, dV) of 256 columns in
+  // shared memory and have room for 32-row partner tiles only
+  if (int e = attn_grid(a, a.D > 128 ? 32 : 64, &b.gr)) return e;
+  const AttnGrid& gr = b.gr;
+  if (gr.g % 16 != 0) return FTK_ERR_UNSUPPORTED;
+  if (gr.QM > AT_MAX_BLOCKS) return FTK_ERR_UNSUPPORTED;
+  const int64_t BH = a.B * a.H;
+  const int per = attn_groups(gr.g), G = attn_groups(gr.kvb);
+  b.tiles = (gr.QM + per - 1) / per;
+  b.stride = (gr.Mkv + 15) & ~15;
+  b.span = (b.tiles * per + 31) & ~31;
+  b.kv_tiles = (gr.Mkv + G - 1) / G;
+  // Pairs walk the union of four lists: only when the lists can cover a good part
+  // of the blocks (see ftk_attn_fwd)
+  b.pair = gr.kd == 128 && gr.g == 64 && gr.kvb == 64 && 4 * gr.width >= gr.Mkv;
+  // Query heads that share a kv head: walked one after the other by the CTA that
+  // owns the kv rows, so that their sum stays in its fp32 accumulators, unless
+  // that leaves SMs idle: waves of CTAs times heads per CTA against waves of one
+  // CTA per head, with a quarter's lead for the per-head results that are then
+  // neither written nor read again.
+  const int64_t grp = a.H / a.Hkv, ctas = a.B * a.Hkv * b.kv_tiles, sms = sm_count();
+  auto waves = [&](int64_t n) { return (n + sms - 1) / sms; };
+  b.walk = grp > 1 && grp * b.span <= AT_MAX_BLOCKS &&
+           4 * grp * waves(ctas) <= 5 * waves(ctas * grp);
+  const int64_t slices = b.walk ? a.B * a.Hkv : BH;
+  // sorting pays once the tiles come in several waves
+  b.order = !b.pair && slices * b.kv_tiles >= 2 * sms;
+  size_t off = up256(static_cast<size_t>(BH) * a.N * 4);   // delta
+  b.off_masks = off;
+  off += up256(static_cast<size_t>(BH) * b.tiles * b.stride);
+  b.off_order = off;
+  if (b.order) off += up256(static_cast<size_t>(slices) * b.kv_tiles * 4);
+  b.off_dk = b.off_dv = off;
+  if (grp > 1 && !b.walk) {
+    const size_t part = up256(static_cast<size_t>(BH) * a.N * a.D * 2);
+    b.off_dv = off + part;
+    off += 2 * part;
+  }
+  b.bytes = off;
+  *out = b;
   return FTK_OK;
 }
 
-static bool aligned_out(const void* p, int64_t a, int64_t b, int64_t c) {
-  return p && !(reinterpret_cast<uintptr_t>(p) & 15u) && !(a & 7) && !(b & 7) && !(c & 7);
+static bool env_off(const char* name) {
+  const char* e = getenv(name);
+  return e && e[0] == '0';
+}
+
+static BwdParams bwd_params(const ftk_attn& a, const AttnGrid& gr, const float* lse, float* delta,
+                            int32_t* status) {
+  BwdParams p{};
+  p.N = static_cast<int>(a.N);
+  p.H = static_cast<int>(a.H);
+  p.D = static_cast<int>(a.D);
+  p.QM = gr.QM;
+  p.W = a.W;
+  p.Mkv = gr.Mkv;
+  p.g = gr.g;
+  p.kvb = gr.kvb;
+  p.q_pad_head = gr.q_pad_head;
+  p.kv_pad_head = gr.kv_pad_head;
+  p.fmt = a.dtype;
+  p.scale = a.scale;
+  p.scale_log2 = a.scale * 1.4426950408889634f;
+  p.lse = lse;
+  p.delta = delta;
+  p.out_f32 = a.out_f32;
+  p.status = status;
+  p.kv_hdiv = static_cast<int>(a.H / a.Hkv);
+  p.heads = 1;
+  p.span = 1 << 30;
+  return p;
+}
+
+struct Rows {   // a 16-bit tensor [b][n][h][d]
+  const void* base;
+  int64_t heads, sb, sn, sh;
+};
+
+static int tmap_of(CUtensorMap* t, const ftk_attn& a, const Rows& r, int rows) {
+  return encode_tmap_bnhd(t, r.base, a.dtype, a.B, a.N, r.heads, a.D, r.sb, r.sn, r.sh, 64, rows);
+}
+
+static int launch_dq(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, bool pair,
+                     cudaStream_t st) {
+  const Rows q = {a.q, a.H, a.sq_b, a.sq_n, a.sq_h}, k = {a.k, a.Hkv, a.sk_b, a.sk_n, a.sk_h},
+             v = {a.v, a.Hkv, a.sv_b, a.sv_n, a.sv_h};
+  const unsigned bh = static_cast<unsigned>(a.B * a.H);
+  p.G = attn_groups(p.g);
+  CUtensorMap tq, tdo, tk, tv;
+  int e;
+  if ((e = tmap_of(&tq, a, q, 128)) || (e = tmap_of(&tdo, a, dout, 128)) ||
+      (e = tmap_of(&tk, a, k, p.kvb)))
+    return e;
+  if (pair && !env_off("FTK_DQ_2CTA")) {
+    CUtensorMap tk32, tv32;
+    if ((e = tmap_of(&tk32, a, k, 32)) || (e = tmap_of(&tv32, a, v, 32))) return e;
+    const size_t smem = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DQ2_STAGES) * 24576;
+    const dim3 grid(2 * ((p.QM + 3) / 4), bh);
+    if (a.dtype == FTK_DTYPE_BF16) {
+      if ((e = allow_smem<sparse_bwd_dq2_kernel<1>>(smem))) return e;
+      return launch_pdl(sparse_bwd_dq2_kernel<1>, grid, BW_THREADS, smem, st, tq, tdo, tk, tk32,
+                        tv32, p);
+    }
+    if ((e = allow_smem<sparse_bwd_dq2_kernel<0>>(smem))) return e;
+    return launch_pdl(sparse_bwd_dq2_kernel<0>, grid, BW_THREADS, smem, st, tq, tdo, tk, tk32, tv32,
+                      p);
+  }
+  if ((e = tmap_of(&tv, a, v, p.kvb))) return e;
+  const int nch = kd / 64;
+  const dim3 grid((p.QM + p.G - 1) / p.G, bh);
+  if (kd == 256) {
+    // Q and dO resident, three K and two V tiles behind them: kv blocks of at most 32 rows
+    if (p.kvb > 32) return FTK_ERR_UNSUPPORTED;
+    const size_t smem = 1024 + 2 * nch * 128 * 128 + static_cast<size_t>(3 + 2) * nch * p.kvb * 128;
+    if ((e = allow_smem<sparse_bwd_dq_kernel<256>>(smem))) return e;
+    return launch_pdl(sparse_bwd_dq_kernel<256>, grid, BW_THREADS, smem, st, tq, tdo, tk, tv, p);
+  }
+  // four V slots lie over the Q / dO tiles, the rest of the V ring behind the K ring
+  const size_t smem = 1024 + 2 * nch * 128 * 128 +
+                      static_cast<size_t>(DQ_KST + DQ_VST - 4) * nch * p.kvb * 128;
+  if (kd == 64) {
+    if ((e = allow_smem<sparse_bwd_dq_kernel<64>>(smem))) return e;
+    return launch_pdl(sparse_bwd_dq_kernel<64>, grid, BW_THREADS, smem, st, tq, tdo, tk, tv, p);
+  }
+  if ((e = allow_smem<sparse_bwd_dq_kernel<128>>(smem))) return e;
+  return launch_pdl(sparse_bwd_dq_kernel<128>, grid, BW_THREADS, smem, st, tq, tdo, tk, tv, p);
+}
+
+static int launch_dkv(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, bool pair,
+                      cudaStream_t st) {
+  const Rows q = {a.q, a.H, a.sq_b, a.sq_n, a.sq_h}, k = {a.k, a.Hkv, a.sk_b, a.sk_n, a.sk_h},
+             v = {a.v, a.Hkv, a.sv_b, a.sv_n, a.sv_h};
+  const unsigned slices = static_cast<unsigned>(a.B * a.H / p.heads);
+  p.G = attn_groups(p.kvb);
+  CUtensorMap tq, tdo, tk, tv;
+  int e;
+  if ((e = tmap_of(&tq, a, q, p.g)) || (e = tmap_of(&tdo, a, dout, p.g)) ||
+      (e = tmap_of(&tk, a, k, 128)) || (e = tmap_of(&tv, a, v, 128)))
+    return e;
+  if (pair && !env_off("FTK_DKV_2CTA")) {
+    CUtensorMap tq32, tdo32;
+    if ((e = tmap_of(&tq32, a, q, 32)) || (e = tmap_of(&tdo32, a, dout, 32))) return e;
+    const size_t smem = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DK2_STAGES) * 32768;
+    const dim3 grid(2 * ((p.Mkv + 3) / 4), slices);
+    auto go = [&](auto kernel_tag) -> int {
+      constexpr auto kernel = decltype(kernel_tag)::kernel;
+      if (int r = allow_smem<kernel>(smem)) return r;
+      return launch_pdl(kernel, grid, BW_THREADS, smem, st, tq, tdo, tq32, tdo32, tk, tv, p);
+    };
+    if (a.dtype == FTK_DTYPE_BF16)
+      return p.heads > 1 ? go(Kernel<sparse_bwd_dkv2_kernel<1, true>>{})
+                         : go(Kernel<sparse_bwd_dkv2_kernel<1, false>>{});
+    return p.heads > 1 ? go(Kernel<sparse_bwd_dkv2_kernel<0, true>>{})
+                       : go(Kernel<sparse_bwd_dkv2_kernel<0, false>>{});
+  }
+  const int nch = kd / 64;
+  const int stage_bytes = 2 * nch * p.g * 128;
+  const int tile_bytes = nch * 128 * 128;          // K or V of the CTA's 128 kv rows
+  // 227 KB per CTA less the static part (union scratch, lse / delta staging: ~22 KB) and the
+  // resident tiles; at head dim 256 that leaves two stages of q blocks of up to 32 rows next to
+  // K and V, four next to K alone
+  auto stages = [&](int resident) {
+    const int ring_bytes = (227 - 23) * 1024 - resident * tile_bytes;
+    return std::min(BW_MAX_STAGES, std::min(128 * 1024, ring_bytes) / stage_bytes);
+  };
+  auto smem_for = [&](int resident, int nst) {
+    return static_cast<size_t>(1024) + static_cast<size_t>(resident) * tile_bytes +
+           static_cast<size_t>(nst) * stage_bytes;
+  };
+  const dim3 grid(p.order ? p.Mkv : (p.Mkv + p.G - 1) / p.G, slices);
+  auto go = [&](auto kernel_tag, int resident) -> int {
+    constexpr auto kernel = decltype(kernel_tag)::kernel;
+    p.nstages = stages(resident);
+    if (p.nstages < 2) return FTK_ERR_UNSUPPORTED;
+    const size_t smem = smem_for(resident, p.nstages);
+    if (int r = allow_smem<kernel>(smem)) return r;
+    return launch_pdl(kernel, grid, BW_THREADS, smem, st, tq, tdo, tk, tv, p);
+  };
+  const bool walk = p.heads > 1;
+  if (kd == 256) {
+    if (stages(2) < 2) return FTK_ERR_UNSUPPORTED;
+    if ((e = walk ? go(Kernel<sparse_bwd_dkv_kernel<256, 1, true>>{}, 1)
+                  : go(Kernel<sparse_bwd_dkv_kernel<256, 1, false>>{}, 1)))
+      return e;
+    return walk ? go(Kernel<sparse_bwd_dkv_kernel<256, 2, true>>{}, 2)
+                : go(Kernel<sparse_bwd_dkv_kernel<256, 2, false>>{}, 2);
+  }
+  if (kd == 64)
+    return walk ? go(Kernel<sparse_bwd_dkv_kernel<64, 0, true>>{}, 2)
+                : go(Kernel<sparse_bwd_dkv_kernel<64, 0, false>>{}, 2);
+  return walk ? go(Kernel<sparse_bwd_dkv_kernel<128, 0, true>>{}, 2)
+              : go(Kernel<sparse_bwd_dkv_kernel<128, 0, false>>{}, 2);
 }
 
 }  // namespace ftk
 
 using namespace ftk;
+
+extern "C" size_t ftk_attn_bwd_workspace(const ftk_attn* a) {
+  BwdPlan b;
+  return a && bwd_plan(*a, &b) == FTK_OK ? b.bytes : 0;
+}
+
+extern "C" int ftk_attn_bwd_dq(const ftk_attn* a, const void* o, int64_t so_b, int64_t so_n,
+                               int64_t so_h, const void* dout, int64_t sdo_b, int64_t sdo_n,
+                               int64_t sdo_h, const float* lse, void* workspace,
+                               size_t workspace_bytes, void* dq, int64_t sdq_b, int64_t sdq_n,
+                               int64_t sdq_h, int32_t* status, void* stream) {
+  if (!a || !lse) return FTK_ERR_BAD_ARG;
+  BwdPlan b;
+  if (int e = bwd_plan(*a, &b)) return e;
+  if (!aligned16(o, so_b, so_n, so_h) || !aligned16(dout, sdo_b, sdo_n, sdo_h) ||
+      !aligned16(dq, sdq_b, sdq_n, sdq_h))
+    return FTK_ERR_BAD_ARG;
+  if (!workspace || workspace_bytes < b.bytes) return FTK_ERR_WORKSPACE;
+  if (reinterpret_cast<uintptr_t>(workspace) & 255u) return FTK_ERR_BAD_ARG;
+  uint8_t* ws = static_cast<uint8_t*>(workspace);
+  BwdParams p = bwd_params(*a, b.gr, lse, reinterpret_cast<float*>(ws), status);
+  p.lists = a->lists;
+  p.list_rows = a->list_rows;
+  p.lm = b.gr.lm;
+  p.masks = ws + b.off_masks;
+  p.mask_stride = b.stride;
+  p.mask_tiles = b.tiles;
+  p.o = static_cast<const uint8_t*>(o);
+  p.so_b = so_b;
+  p.so_n = so_n;
+  p.so_h = so_h;
+  p.dout = static_cast<const uint8_t*>(dout);
+  p.sd_b = sdo_b;
+  p.sd_n = sdo_n;
+  p.sd_h = sdo_h;
+  p.out0 = dq;
+  p.s0_b = sdq_b;
+  p.s0_n = sdq_n;
+  p.s0_h = sdq_h;
+  return launch_dq(*a, Rows{dout, a->H, sdo_b, sdo_n, sdo_h}, p, b.gr.kd, b.pair,
+                   static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int ftk_attn_bwd_dkv(const ftk_attn* a, const void* dout, int64_t sdo_b, int64_t sdo_n,
+                                int64_t sdo_h, const float* lse, void* workspace,
+                                size_t workspace_bytes, void* dk, int64_t sdk_b, int64_t sdk_n,
+                                int64_t sdk_h, void* dv, int64_t sdv_b, int64_t sdv_n,
+                                int64_t sdv_h, int32_t* status, void* stream) {
+  if (!a || !lse) return FTK_ERR_BAD_ARG;
+  BwdPlan b;
+  if (int e = bwd_plan(*a, &b)) return e;
+  if (!aligned16(dout, sdo_b, sdo_n, sdo_h) || !aligned16(dk, sdk_b, sdk_n, sdk_h) ||
+      !aligned16(dv, sdv_b, sdv_n, sdv_h))
+    return FTK_ERR_BAD_ARG;
+  if (!workspace || workspace_bytes < b.bytes) return FTK_ERR_WORKSPACE;
+  if (reinterpret_cast<uintptr_t>(workspace) & 255u) return FTK_ERR_BAD_ARG;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  uint8_t* ws = static_cast<uint8_t*>(workspace);
+  BwdParams p = bwd_params(*a, b.gr, lse, reinterpret_cast<float*>(ws), status);
+  p.masks = ws + b.off_masks;
+  p.mask_stride = b.stride;
+  p.mask_tiles = b.tiles;
+  p.mask_g = attn_groups(b.gr.g);
+  p.span = b.span;
+  p.heads = b.walk ? p.kv_hdiv : 1;
+  const bool parts = p.kv_hdiv > 1 && !b.walk;
+  if (parts) {   // one 16-bit result per query head first
+    const int64_t row = a->H * a->D;
+    p.out0 = ws + b.off_dk;
+    p.out1 = ws + b.off_dv;
+    p.s0_b = p.s1_b = a->N * row;
+    p.s0_n = p.s1_n = row;
+    p.s0_h = p.s1_h = a->D;
+    p.out_f32 = 0;
+  } else {
+    p.out0 = dk;
+    p.s0_b = sdk_b;
+    p.s0_n = sdk_n;
+    p.s0_h = sdk_h;
+    p.out1 = dv;
+    p.s1_b = sdv_b;
+    p.s1_n = sdv_n;
+    p.s1_h = sdv_h;
+  }
+  if (b.order && !env_off("FTK_DKV_ORDER")) {
+    int colsp = 32;
+    while (colsp < b.kv_tiles) colsp <<= 1;
+    const size_t smem = static_cast<size_t>(colsp) * 12;
+    int32_t* order = reinterpret_cast<int32_t*>(ws + b.off_order);
+    int e = allow_smem<fan_in_kernel>(smem);
+    if (!e)
+      e = launch_pdl(fan_in_kernel, static_cast<unsigned>(a->B * a->H / p.heads), FAN_THREADS, smem,
+                     st, p.masks, b.stride, b.tiles,
+                     static_cast<int64_t>(b.tiles) * b.stride, p.heads,
+                     static_cast<int>(a->H / p.heads), static_cast<int>(a->H), b.gr.Mkv,
+                     attn_groups(b.gr.kvb), b.kv_tiles, colsp, order);
+    if (e) return e;
+    p.tile_order = order;
+  }
+  if (int e = launch_dkv(*a, Rows{dout, a->H, sdo_b, sdo_n, sdo_h}, p, b.gr.kd, b.pair, st))
+    return e;
+  if (!parts) return FTK_OK;
+  const int64_t vecs = a->B * a->N * a->Hkv * (a->D / 8);
+  if ((vecs + 255) / 256 > 0x7fffffffLL) return FTK_ERR_BAD_ARG;
+  return launch_pdl(head_sum_kernel, dim3(static_cast<unsigned>((vecs + 255) / 256), 2), 256, 0, st,
+                    ws + b.off_dk, ws + b.off_dv, a->dtype, a->N, static_cast<int>(a->Hkv),
+                    p.kv_hdiv, static_cast<int>(a->D), vecs, dk, sdk_b, sdk_n, sdk_h, dv, sdv_b,
+                    sdv_n, sdv_h, a->out_f32);
+}
+
+static int old_bwd_grid(const ftk_attn& a, AttnGrid* gr) {
+  if (a.D != 64 && a.D != 128 && a.D != 256) return FTK_ERR_UNSUPPORTED;
+  if (a.kv_block > 64) return FTK_ERR_UNSUPPORTED;
+  return attn_grid(a, 128, gr);   // blocks as they are
+}
 
 extern "C" int ftk_sparse_bwd_dq(
     const void* q, const void* k, const void* v, const void* o, const void* dout, int dtype,
@@ -913,117 +1420,34 @@ extern "C" int ftk_sparse_bwd_dq(
     const int32_t* merged_idx, int QM, int W, int q_block_size, int kv_block_size, int q_pad_head,
     int kv_pad_head, float scale, const float* lse, float* delta, void* dq, int64_t sdq_b,
     int64_t sdq_n, int64_t sdq_h, int32_t* status, void* stream) {
-  if (!q || !k || !v || !o || !dout || !merged_idx || !lse || !delta || W <= 0)
+  const ftk_attn a = {q,    k,    v,    dtype, 0,    B,    H,    Hkv <= 0 ? H : Hkv,
+                      N,    D,    sq_b, sq_n,  sq_h, sk_b, sk_n, sk_h,
+                      sv_b, sv_n, sv_h, merged_idx, QM, W, q_block_size, kv_block_size,
+                      q_pad_head, kv_pad_head, scale};
+  AttnGrid gr;
+  if (int e = old_bwd_grid(a, &gr)) return e;
+  if (!lse || !delta || !aligned16(o, so_b, so_n, so_h) || !aligned16(dout, sdo_b, sdo_n, sdo_h) ||
+      !aligned16(dq, sdq_b, sdq_n, sdq_h))
     return FTK_ERR_BAD_ARG;
-  int e = bwd_common_checks(dtype, B, H, N, D, QM, q_block_size, kv_block_size, q_pad_head,
-                            kv_pad_head);
-  if (e) return e;
-  if (Hkv <= 0) Hkv = H;
-  if (H % Hkv != 0) return FTK_ERR_BAD_ARG;
-  if (q_block_size > 128) return FTK_ERR_UNSUPPORTED;
-  if (!aligned_out(dq, sdq_b, sdq_n, sdq_h)) return FTK_ERR_BAD_ARG;
-  // delta reads O and dO with 16-byte loads
-  if ((so_b | so_n | so_h | sdo_b | sdo_n | sdo_h) & 7) return FTK_ERR_BAD_ARG;
-  if ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout)) & 15u)
-    return FTK_ERR_BAD_ARG;
-  const int64_t Mkv = (kv_pad_head + N + kv_block_size - 1) / kv_block_size;
-  if (Mkv > AT_MAX_BLOCKS) return FTK_ERR_UNSUPPORTED;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-
-  const int64_t rows = B * N * H;
-  const int64_t delta_warps = (rows + 256 / D - 1) / (256 / D);   // 256 / D rows per warp
-  delta_kernel<<<static_cast<unsigned>((delta_warps * 32 + 255) / 256), 256, 0, st>>>(
-      static_cast<const uint8_t*>(o), static_cast<const uint8_t*>(dout), dtype, B, N, H,
-      static_cast<int>(D), so_b, so_n, so_h, sdo_b, sdo_n, sdo_h, delta);
-  if (cudaGetLastError() != cudaSuccess) return FTK_ERR_CUDA;
-
-  BwdParams p{};
-  p.N = static_cast<int>(N);
-  p.H = static_cast<int>(H);
-  p.QM = QM;
-  p.W = W;
-  p.Mkv = static_cast<int>(Mkv);
-  p.g = q_block_size;
-  p.kvb = kv_block_size;
-  p.q_pad_head = q_pad_head;
-  p.kv_pad_head = kv_pad_head;
-  p.G = std::max(1, std::min(AT_MAX_GROUPS, 128 / q_block_size));
-  p.fmt = dtype;
-  p.scale = scale;
-  p.scale_log2 = scale * 1.4426950408889634f;
+  BwdParams p = bwd_params(a, gr, lse, delta, status);
   p.lists = merged_idx;
-  p.lse = lse;
-  p.delta = delta;
+  p.list_rows = QM;
+  p.o = static_cast<const uint8_t*>(o);
+  p.so_b = so_b;
+  p.so_n = so_n;
+  p.so_h = so_h;
+  p.dout = static_cast<const uint8_t*>(dout);
+  p.sd_b = sdo_b;
+  p.sd_n = sdo_n;
+  p.sd_h = sdo_h;
   p.out0 = dq;
   p.s0_b = sdq_b;
   p.s0_n = sdq_n;
   p.s0_h = sdq_h;
-  p.status = status;
-  p.kv_hdiv = static_cast<int>(H / Hkv);
-
-  CUtensorMap tq, tdo, tk, tv;
-  if ((e = encode_tmap_bnhd(&tq, q, dtype, B, N, H, D, sq_b, sq_n, sq_h, 64, 128))) return e;
-  if ((e = encode_tmap_bnhd(&tdo, dout, dtype, B, N, H, D, sdo_b, sdo_n, sdo_h, 64, 128))) return e;
-  if ((e = encode_tmap_bnhd(&tk, k, dtype, B, N, Hkv, D, sk_b, sk_n, sk_h, 64, kv_block_size)))
-    return e;
-  if ((e = encode_tmap_bnhd(&tv, v, dtype, B, N, Hkv, D, sv_b, sv_n, sv_h, 64, kv_block_size)))
-    return e;
-  // head dim 128 with 64-row q and kv blocks: the kernel on pairs of SMs
-  // (pairs walk the union of four lists: only when the lists can cover a good
-  // part of the blocks, see ftk_sparse_fwd)
-  const char* env2 = getenv("FTK_DQ_2CTA");
-  if (D == 128 && q_block_size == 64 && kv_block_size == 64 &&
-      4 * static_cast<int64_t>(W) >= Mkv && !(env2 && env2[0] == '0')) {
-    CUtensorMap tk32, tv32;
-    if ((e = encode_tmap_bnhd(&tk32, k, dtype, B, N, Hkv, D, sk_b, sk_n, sk_h, 64, 32))) return e;
-    if ((e = encode_tmap_bnhd(&tv32, v, dtype, B, N, Hkv, D, sv_b, sv_n, sv_h, 64, 32))) return e;
-    const size_t smem2 = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DQ2_STAGES) * 24576;
-    dim3 grid2(2 * ((QM + 3) / 4), static_cast<unsigned>(B * H));
-    if (dtype == FTK_DTYPE_BF16) {
-      if (cudaFuncSetAttribute(sparse_bwd_dq2_kernel<1>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(smem2)) != cudaSuccess)
-        return FTK_ERR_CUDA;
-      sparse_bwd_dq2_kernel<1><<<grid2, BW_THREADS, smem2, st>>>(tq, tdo, tk, tk32, tv32, p);
-    } else {
-      if (cudaFuncSetAttribute(sparse_bwd_dq2_kernel<0>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(smem2)) != cudaSuccess)
-        return FTK_ERR_CUDA;
-      sparse_bwd_dq2_kernel<0><<<grid2, BW_THREADS, smem2, st>>>(tq, tdo, tk, tk32, tv32, p);
-    }
-    return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
-  }
-  const int nch = static_cast<int>(D / 64);
-  dim3 grid((QM + p.G - 1) / p.G, static_cast<unsigned>(B * H));
-  if (D == 256) {
-    // Q and dO resident, three K and two V tiles behind them: kv blocks of at most 32 rows
-    if (kv_block_size > 32) return FTK_ERR_UNSUPPORTED;
-    const size_t smem_big =
-        1024 + 2 * nch * 128 * 128 + static_cast<size_t>(3 + 2) * nch * kv_block_size * 128;
-    if (cudaFuncSetAttribute(sparse_bwd_dq_kernel<256>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem_big)) != cudaSuccess)
-      return FTK_ERR_CUDA;
-    sparse_bwd_dq_kernel<256><<<grid, BW_THREADS, smem_big, st>>>(tq, tdo, tk, tv, p);
-    return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
-  }
-  // four V slots lie over the Q / dO tiles, the rest of the V ring behind the K ring
-  const size_t smem = 1024 + 2 * nch * 128 * 128 +
-                      static_cast<size_t>(DQ_KST + DQ_VST - 4) * nch * kv_block_size * 128;
-  if (D == 64) {
-    if (cudaFuncSetAttribute(sparse_bwd_dq_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
-      return FTK_ERR_CUDA;
-    sparse_bwd_dq_kernel<64><<<grid, BW_THREADS, smem, st>>>(tq, tdo, tk, tv, p);
-  } else {
-    if (cudaFuncSetAttribute(sparse_bwd_dq_kernel<128>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
-      return FTK_ERR_CUDA;
-    sparse_bwd_dq_kernel<128><<<grid, BW_THREADS, smem, st>>>(tq, tdo, tk, tv, p);
-  }
-  return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
+  const bool pair = D == 128 && q_block_size == 64 && kv_block_size == 64 &&
+                    4 * static_cast<int64_t>(W) >= gr.Mkv;
+  return launch_dq(a, Rows{dout, H, sdo_b, sdo_n, sdo_h}, p, gr.kd, pair,
+                   static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int ftk_sparse_bwd_dkv(
@@ -1035,38 +1459,22 @@ extern "C" int ftk_sparse_bwd_dkv(
     int kv_pad_head, float scale, const float* lse, const float* delta, void* dk, int64_t sdk_b,
     int64_t sdk_n, int64_t sdk_h, void* dv, int64_t sdv_b, int64_t sdv_n, int64_t sdv_h,
     int fwd_list_width, int32_t* status, void* stream) {
-  if (!q || !k || !v || !dout || !reverse_idx || !reverse_counts || !lse || !delta)
-    return FTK_ERR_BAD_ARG;
-  int e = bwd_common_checks(dtype, B, H, N, D, QM, q_block_size, kv_block_size, q_pad_head,
-                            kv_pad_head);
-  if (e) return e;
-  if (Hkv <= 0) Hkv = H;
-  if (H % Hkv != 0) return FTK_ERR_BAD_ARG;
+  const ftk_attn a = {q,    k,    v,    dtype, 0,    B,    H,    Hkv <= 0 ? H : Hkv,
+                      N,    D,    sq_b, sq_n,  sq_h, sk_b, sk_n, sk_h,
+                      sv_b, sv_n, sv_h, reverse_idx, QM, QM, q_block_size, kv_block_size,
+                      q_pad_head, kv_pad_head, scale};
+  AttnGrid gr;
+  if (int e = old_bwd_grid(a, &gr)) return e;
   if (q_block_size % 16 != 0 || q_block_size > 64) return FTK_ERR_UNSUPPORTED;
   if (QM > AT_MAX_BLOCKS) return FTK_ERR_UNSUPPORTED;
   if (M <= 0 || static_cast<int64_t>(M) * kv_block_size < kv_pad_head + N) return FTK_ERR_BAD_ARG;
-  if (!aligned_out(dk, sdk_b, sdk_n, sdk_h) || !aligned_out(dv, sdv_b, sdv_n, sdv_h))
+  if (!reverse_counts || !lse || !delta || !aligned16(dout, sdo_b, sdo_n, sdo_h) ||
+      !aligned16(dk, sdk_b, sdk_n, sdk_h) || !aligned16(dv, sdv_b, sdv_n, sdv_h))
     return FTK_ERR_BAD_ARG;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-
-  BwdParams p{};
-  p.N = static_cast<int>(N);
-  p.H = static_cast<int>(H);
-  p.QM = QM;
-  p.W = QM;
+  BwdParams p = bwd_params(a, gr, lse, const_cast<float*>(delta), status);
   p.Mkv = M;
-  p.g = q_block_size;
-  p.kvb = kv_block_size;
-  p.q_pad_head = q_pad_head;
-  p.kv_pad_head = kv_pad_head;
-  p.G = std::max(1, std::min(AT_MAX_GROUPS, 128 / kv_block_size));
-  p.fmt = dtype;
-  p.scale = scale;
-  p.scale_log2 = scale * 1.4426950408889634f;
   p.lists = reverse_idx;
   p.counts = reverse_counts;
-  p.lse = lse;
-  p.delta = delta;
   p.out0 = dk;
   p.s0_b = sdk_b;
   p.s0_n = sdk_n;
@@ -1075,91 +1483,11 @@ extern "C" int ftk_sparse_bwd_dkv(
   p.s1_b = sdv_b;
   p.s1_n = sdv_n;
   p.s1_h = sdv_h;
-  p.status = status;
-  p.kv_hdiv = static_cast<int>(H / Hkv);
-
-  CUtensorMap tq, tdo, tk, tv;
-  if ((e = encode_tmap_bnhd(&tq, q, dtype, B, N, H, D, sq_b, sq_n, sq_h, 64, q_block_size)))
-    return e;
-  if ((e = encode_tmap_bnhd(&tdo, dout, dtype, B, N, H, D, sdo_b, sdo_n, sdo_h, 64, q_block_size)))
-    return e;
-  if ((e = encode_tmap_bnhd(&tk, k, dtype, B, N, Hkv, D, sk_b, sk_n, sk_h, 64, 128))) return e;
-  if ((e = encode_tmap_bnhd(&tv, v, dtype, B, N, Hkv, D, sv_b, sv_n, sv_h, 64, 128))) return e;
-  // head dim 128 with 64-row q and kv blocks: the kernel on pairs of SMs
-  const char* env2 = getenv("FTK_DKV_2CTA");
-  const bool long_lists = fwd_list_width <= 0 || 4 * static_cast<int64_t>(fwd_list_width) >= M;
-  if (D == 128 && q_block_size == 64 && kv_block_size == 64 && long_lists &&
-      !(env2 && env2[0] == '0')) {
-    CUtensorMap tq32, tdo32;
-    if ((e = encode_tmap_bnhd(&tq32, q, dtype, B, N, H, D, sq_b, sq_n, sq_h, 64, 32))) return e;
-    if ((e = encode_tmap_bnhd(&tdo32, dout, dtype, B, N, H, D, sdo_b, sdo_n, sdo_h, 64, 32)))
-      return e;
-    const size_t smem2 = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DK2_STAGES) * 32768;
-    dim3 grid2(2 * ((M + 3) / 4), static_cast<unsigned>(B * H));
-    if (dtype == FTK_DTYPE_BF16) {
-      if (cudaFuncSetAttribute(sparse_bwd_dkv2_kernel<1>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(smem2)) != cudaSuccess)
-        return FTK_ERR_CUDA;
-      sparse_bwd_dkv2_kernel<1><<<grid2, BW_THREADS, smem2, st>>>(tq, tdo, tq32, tdo32, tk, tv, p);
-    } else {
-      if (cudaFuncSetAttribute(sparse_bwd_dkv2_kernel<0>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(smem2)) != cudaSuccess)
-        return FTK_ERR_CUDA;
-      sparse_bwd_dkv2_kernel<0><<<grid2, BW_THREADS, smem2, st>>>(tq, tdo, tq32, tdo32, tk, tv, p);
-    }
-    return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
-  }
-  const int nch = static_cast<int>(D / 64);
-  const int stage_bytes = 2 * nch * q_block_size * 128;
-  const int tile_bytes = nch * 128 * 128;          // K or V of the CTA's 128 kv rows
-  // 227 KB per CTA less the static part (union scratch, lse / delta staging: ~21 KB) and the
-  // resident tiles; at head dim 256 that leaves two stages of q blocks of up to 32 rows next to
-  // K and V, four next to K alone
-  auto stages = [&](int resident) {
-    const int ring_bytes = (227 - 23) * 1024 - resident * tile_bytes;
-    return std::min(BW_MAX_STAGES, std::min(128 * 1024, ring_bytes) / stage_bytes);
-  };
-  auto smem_for = [&](int resident, int nst) {
-    return static_cast<size_t>(1024) + static_cast<size_t>(resident) * tile_bytes +
-           static_cast<size_t>(nst) * stage_bytes;
-  };
+  const bool pair = D == 128 && q_block_size == 64 && kv_block_size == 64 &&
+                    (fwd_list_width <= 0 || 4 * static_cast<int64_t>(fwd_list_width) >= M);
   // one-CTA kernels: tiles in order of fan-in when the caller brings the order
-  const char* oe = getenv("FTK_DKV_ORDER");
-  p.order = (sorted_kv && !(oe && oe[0] == '0')) ? sorted_kv : nullptr;
-  dim3 grid(p.order ? M : (M + p.G - 1) / p.G, static_cast<unsigned>(B * H));
-  if (D == 256) {
-    const int nst_dv = stages(1), nst_dk = stages(2);
-    if (nst_dk < 2) return FTK_ERR_UNSUPPORTED;
-    if (cudaFuncSetAttribute(sparse_bwd_dkv_kernel<256, 1>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem_for(1, nst_dv))) != cudaSuccess ||
-        cudaFuncSetAttribute(sparse_bwd_dkv_kernel<256, 2>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem_for(2, nst_dk))) != cudaSuccess)
-      return FTK_ERR_CUDA;
-    p.nstages = nst_dv;
-    sparse_bwd_dkv_kernel<256, 1><<<grid, BW_THREADS, smem_for(1, nst_dv), st>>>(tq, tdo, tk, tv, p);
-    p.nstages = nst_dk;
-    sparse_bwd_dkv_kernel<256, 2><<<grid, BW_THREADS, smem_for(2, nst_dk), st>>>(tq, tdo, tk, tv, p);
-    return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
-  }
-  p.nstages = stages(2);
-  if (p.nstages < 2) return FTK_ERR_UNSUPPORTED;
-  const size_t smem = smem_for(2, p.nstages);
-  if (D == 64) {
-    if (cudaFuncSetAttribute(sparse_bwd_dkv_kernel<64, 0>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
-      return FTK_ERR_CUDA;
-    sparse_bwd_dkv_kernel<64, 0><<<grid, BW_THREADS, smem, st>>>(tq, tdo, tk, tv, p);
-  } else {
-    if (cudaFuncSetAttribute(sparse_bwd_dkv_kernel<128, 0>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
-      return FTK_ERR_CUDA;
-    sparse_bwd_dkv_kernel<128, 0><<<grid, BW_THREADS, smem, st>>>(tq, tdo, tk, tv, p);
-  }
-  return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
+  if (!pair || env_off("FTK_DKV_2CTA"))
+    p.order = sorted_kv && !env_off("FTK_DKV_ORDER") ? sorted_kv : nullptr;
+  return launch_dkv(a, Rows{dout, H, sdo_b, sdo_n, sdo_h}, p, gr.kd, pair,
+                    static_cast<cudaStream_t>(stream));
 }

@@ -41,7 +41,11 @@ __device__ __forceinline__ uint32_t pack2f(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <int FMT>
+// WALK: p.heads query heads share the pair's kv head and are walked one after the
+// other.  A template parameter because the compute warps set this kernel's pace:
+// the head bookkeeping of WALK in every build took 28.3 -> 34.6 ms at N = 32768,
+// H = 32.
+template <int FMT, bool WALK>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(BW_THREADS, 1)
 sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
                        const __grid_constant__ CUtensorMap tm_do,
@@ -71,7 +75,10 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
   const uint32_t rank = cluster_ctarank();
   const int j0 = (blockIdx.x >> 1) * 4;      // first of the pair's four kv blocks
   const int bh = blockIdx.y;
-  const int b_idx = bh / p.H, h_idx = bh - b_idx * p.H;
+  // slice = (batch, first of the query heads this pair walks)
+  const int slices = WALK ? p.H / p.heads : p.H;
+  const int b_idx = bh / slices, h_idx = (bh - b_idx * slices) * (WALK ? p.heads : 1);
+  const int bhq = WALK ? b_idx * p.H + h_idx : bh;
   const int groups = min(4, p.Mkv - j0);     // kv blocks of the pair that exist
   const int tile_tok0 = (j0 + 2 * static_cast<int>(rank)) * G - p.kv_pad_head;   // my 128 rows
 
@@ -112,9 +119,7 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_relinquish2();
   }
   // both CTAs build the same union over the pair's four reverse lists
-  const int64_t kv_row = static_cast<int64_t>(bh) * p.Mkv + j0;
-  const int n = build_union(un, p.lists + kv_row * p.QM, p.QM, groups, p.QM, p.counts + kv_row,
-                            p.QM, p.status);
+  const int n = dkv_union(un, p, bhq, j0, groups);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();        // barriers of both CTAs are initialised before anyone signals them
@@ -133,19 +138,21 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
                     tile_tok0, b_idx);
       }
       const int dcol = 64 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
+      HeadWalk<WALK> hw;
       for (int i = 0; i < n; i++) {
         const int s = i % DK2_STAGES;
         if (!mbar_wait(bar_qempty(s), ((i / DK2_STAGES) & 1) ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
-        const int row0 = static_cast<int>(un.ids[i]) * G - p.q_pad_head;
+        const int row0 = hw.at(un.ids[i], p) * G - p.q_pad_head;
+        const int h = h_idx + hw.head;
         const uint32_t base = smem_u32(sQD) + s * STAGE;
         mbar_expect_tx(bar_qfull(s), STAGE);
         for (int c = 0; c < NCH; c++) {
-          tma_load_4d(base + c * 4096, &tm_q32, bar_qfull(s), c * 64, h_idx, row0 + rsub, b_idx);
-          tma_load_4d(base + OFF_DOROW + c * 4096, &tm_do32, bar_qfull(s), c * 64, h_idx,
-                      row0 + rsub, b_idx);
+          tma_load_4d(base + c * 4096, &tm_q32, bar_qfull(s), c * 64, h, row0 + rsub, b_idx);
+          tma_load_4d(base + OFF_DOROW + c * 4096, &tm_do32, bar_qfull(s), c * 64, h, row0 + rsub,
+                      b_idx);
         }
-        tma_load_4d(base + OFF_QCOL, &tm_q, bar_qfull(s), dcol, h_idx, row0, b_idx);
-        tma_load_4d(base + OFF_DOCOL, &tm_do, bar_qfull(s), dcol, h_idx, row0, b_idx);
+        tma_load_4d(base + OFF_QCOL, &tm_q, bar_qfull(s), dcol, h, row0, b_idx);
+        tma_load_4d(base + OFF_DOCOL, &tm_do, bar_qfull(s), dcol, h, row0, b_idx);
       }
     }
   } else if (warp == 1 && rank == 1) {
@@ -259,14 +266,16 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     // lse / delta of a q-block are fetched from global memory one round ahead
     // (into registers, while the previous tile is being worked on) and only
     // then staged in shared memory: their latency stays out of the chain.
+    HeadWalk<WALK> hw, hw_mine;
     auto fetch = [&](int i, float& l2, float& dl) {
       l2 = 0.f;
       dl = 0.f;
       if (ct < G && i < n) {
-        const int t = static_cast<int>(un.ids[i]) * G - p.q_pad_head + ct;
+        const int t = hw.at(un.ids[i], p) * G - p.q_pad_head + ct;
         if (t >= 0 && t < p.N) {   // stored negated: the packed fma / add take them as they are
-          l2 = -p.lse[static_cast<int64_t>(bh) * p.N + t] * 1.4426950408889634f;
-          dl = -p.delta[static_cast<int64_t>(bh) * p.N + t];
+          const int64_t e = static_cast<int64_t>(bhq + hw.head) * p.N + t;
+          l2 = -p.lse[e] * 1.4426950408889634f;
+          dl = -p.delta[e];
         }
       }
     };
@@ -274,7 +283,7 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     fetch(0, l2_next, dl_next);
     for (int i = 0; i < n; i++) {
       const int sb = i & 1;                  // S^T / dP^T buffer, and lse / delta buffer
-      const int row0 = static_cast<int>(un.ids[i]) * G - p.q_pad_head;
+      const int row0 = hw_mine.at(un.ids[i], p) * G - p.q_pad_head;
       if (ct < G) {
         s_lse2[0][sb][ct] = l2_next;
         s_delta[0][sb][ct] = dl_next;
@@ -292,6 +301,7 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
       const int lo = max(0, -row0), hi = min(G, p.N - row0);
       const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
+      const bool none = !fast && !__any_sync(0xffffffffu, act);
       const float4* l4 = reinterpret_cast<const float4*>(s_lse2[0][sb]);
       const float4* d4 = reinterpret_cast<const float4*>(s_delta[0][sb]);
       // P^T / dS^T of the thread's 16 columns go over the first 8 of them in
@@ -345,7 +355,11 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
         tmem_st8(st_addr + c0, pp);
         tmem_st8(dp_addr + c0, pd);
       };
-      {
+      if (none) {   // a q-block of the other groups: P^T = dS^T = 0, nothing to read
+        const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+        tmem_st8(st_addr + cbeg, z);
+        tmem_st8(dp_addr + cbeg, z);
+      } else {
         uint32_t sa[16], da[16];
         tmem_ld16(st_addr + cbeg, sa);
         tmem_ld16(dp_addr + cbeg, da);
@@ -368,8 +382,9 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
       const float mul = which == 0 ? 1.f : p.scale;
       uint8_t* orow = nullptr;
       if (row_valid)
-        orow = base + 2 * (static_cast<int64_t>(b_idx) * sb_ + static_cast<int64_t>(tok) * sn_ +
-                           static_cast<int64_t>(h_idx) * sh_);
+        orow = base + (p.out_f32 ? 4 : 2) *
+                          (static_cast<int64_t>(b_idx) * sb_ + static_cast<int64_t>(tok) * sn_ +
+                           static_cast<int64_t>(WALK ? h_idx / p.heads : h_idx) * sh_);
       for (int c0 = colhalf * 32; c0 < D; c0 += 64) {
         uint32_t v[32];
         if (n > 0) {
@@ -384,10 +399,7 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
             const float b = n > 0 ? __uint_as_float(v[x + 1]) * mul : 0.f;
             pk[x >> 1] = pack2f<FMT>(a, b);
           }
-          uint4* dst = reinterpret_cast<uint4*>(orow + c0 * 2);
-#pragma unroll
-          for (int x = 0; x < 4; x++)
-            dst[x] = make_uint4(pk[4 * x], pk[4 * x + 1], pk[4 * x + 2], pk[4 * x + 3]);
+          store_row_part(orow, c0, p.D, pk, FMT, p.out_f32 != 0);
         }
       }
     }

@@ -45,6 +45,7 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
   uint8_t* sDO = smem + ROW_TILE_BYTES;
   uint8_t* sKV = smem + 2 * ROW_TILE_BYTES;
   __shared__ UnionScratch un;
+  __shared__ float s_delta[128];
   __shared__ __align__(8) uint64_t bars[2 + 3 * DQ2_STAGES + 5];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
@@ -93,8 +94,18 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_relinquish2();
   }
   // both CTAs build the same union over the pair's four candidate lists
-  const int n = build_union(un, p.lists + (static_cast<int64_t>(bh) * p.QM + m0) * p.W, p.W,
-                            groups, p.W, nullptr, p.Mkv, p.status);
+  clear_bitmaps(un);
+  pdl_wait();
+  pdl_launch();
+  const int mine = min(2, groups - 2 * static_cast<int>(rank));   // q-blocks of my tile, if any
+  tile_delta<D>(p, s_delta, bh, b_idx, h_idx, tile_row0, mine * G);
+  const int n = build_union(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
+                            p.W, nullptr, p.Mkv, p.lm, p.status);
+  if (p.masks && mine > 0)
+    write_tile_masks(un,
+                     p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + m0 / 2 + rank) *
+                                   p.mask_stride,
+                     p.mask_stride, 2 * static_cast<int>(rank), mine);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();        // barriers of both CTAs are initialised before anyone signals them
@@ -230,7 +241,7 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
     float lse2 = 0.f, dl = 0.f;
     if (row_valid) {
       lse2 = p.lse[static_cast<int64_t>(bh) * p.N + qrow] * 1.4426950408889634f;
-      dl = p.delta[static_cast<int64_t>(bh) * p.N + qrow];
+      dl = s_delta[r];
     }
     bool ok = true;
     if (n > 0 && colhalf == 0) {
@@ -272,10 +283,16 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
       const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
       uint32_t sv[32], dv[32], pk[16];
-      tmem_ld32(s_addr + cbeg, sv);
-      tmem_ld32(dp_addr + cbeg, dv);
-      tmem_wait_ld();
-      if (fast) {
+      const bool none = !fast && !__any_sync(0xffffffffu, act);   // a block of the other groups: dS = 0
+      if (!none) {
+        tmem_ld32(s_addr + cbeg, sv);
+        tmem_ld32(dp_addr + cbeg, dv);
+        tmem_wait_ld();
+      }
+      if (none) {
+#pragma unroll
+        for (int x = 0; x < 16; x++) pk[x] = 0u;
+      } else if (fast) {
         ds_pairs<FMT>(sv, dv, pk, c, -lse2, -dl);
       } else {
 #pragma unroll
@@ -304,7 +321,8 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
       uint8_t* orow = nullptr;
       if (row_valid)
         orow = static_cast<uint8_t*>(p.out0) +
-               2 * (static_cast<int64_t>(b_idx) * p.s0_b + static_cast<int64_t>(qrow) * p.s0_n +
+               (p.out_f32 ? 4 : 2) *
+                   (static_cast<int64_t>(b_idx) * p.s0_b + static_cast<int64_t>(qrow) * p.s0_n +
                     static_cast<int64_t>(h_idx) * p.s0_h);
       const int c0 = (wg * 2 + colhalf) * 32;
       uint32_t v[32];
@@ -320,10 +338,7 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
           const float b = n > 0 ? __uint_as_float(v[x + 1]) * p.scale : 0.f;
           pk[x >> 1] = pack2f<FMT>(a, b);
         }
-        uint4* dst = reinterpret_cast<uint4*>(orow + c0 * 2);
-#pragma unroll
-        for (int x = 0; x < 4; x++)
-          dst[x] = make_uint4(pk[4 * x], pk[4 * x + 1], pk[4 * x + 2], pk[4 * x + 3]);
+        store_row_part(orow, c0, p.D, pk, FMT, p.out_f32 != 0);
       }
     }
   }

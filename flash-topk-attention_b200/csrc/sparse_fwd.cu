@@ -29,6 +29,7 @@
 #include <cstdlib>
 
 #include "attn_common.cuh"
+#include "attn_host.cuh"
 #include "ftk_host.cuh"
 #include "ftk_sm100.cuh"
 
@@ -54,18 +55,26 @@ struct FwdParams {
   float* lse;
   int* status;
   int kv_hdiv;          // query heads per kv head (grouped-query attention), 1 otherwise
-  int* redo_out;        // pipelined kernel: one word per CTA, 1 = redo with the exact kernel
-  const int* redo_in;   // exact kernel: when set, CTAs whose word is 0 return at once
-  int v_off;            // first head-dim column of V / O this launch produces (head dim 256)
+  int* redo_out;        // pipelined kernel: one word per 128-row tile, 1 = redo with the exact kernel
+  const int* redo_in;   // exact kernel: when set, only tiles whose word is 1 are done
+  int list_rows;        // rows of the caller's lists per slice
+  int tiles_x, tiles;   // 128-row tiles per slice, and of all slices
+  int D;                // columns of a row of O (the kernel's head dim less its padding)
+  int out_f32;          // O is float32 (the 16-bit result, widened)
+  ListMap lm;
 };
 
-// D = head dim of the Q.K^T contraction, DV = columns of V / O per launch
-// (p.v_off = first column).  Head dim 256: two 256-column accumulators do not
+// D = head dim of the Q.K^T contraction, DV = columns of V / O.  Head dim 256: two 256-column accumulators do not
 // fit TMEM next to S, so there is ONE accumulator (columns 256..511) and one
 // softmax group with one running maximum drains both S buffers in turn; Q
 // stays in shared memory.  The tile's UMMAs (16 + 4 k-steps) outlast its
 // softmax, so one group keeps up.  The second group only helps in the epilogue.
-template <int D, int DV>
+//
+// One CTA per 128-row tile; behind the pipelined kernel instead a few CTAs per
+// SM that look through that kernel's redo words together and loop over the
+// tiles they find (as a rule none): a grid of one CTA per tile, each leaving on
+// its first instruction, took 69 us at 8192 tiles.
+template <int D, int DV, bool REDO>
 __global__ void __launch_bounds__(FW_THREADS, 1)
 sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const FwdParams p) {
@@ -83,11 +92,41 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
   __shared__ float s_m[2][128], s_l[2][128];
+  __shared__ unsigned s_todo[(FW_THREADS + 31) / 32];
 
-  if (p.redo_in && p.redo_in[blockIdx.y * gridDim.x + blockIdx.x] == 0) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.x * p.G;
-  const int bh = blockIdx.y;
+  pdl_wait();
+  pdl_launch();
+  bool first_tile = true;
+  uint32_t tmem = 0;
+  // REDO: FW_THREADS redo words are looked at together, tiles blockIdx.x,
+  // blockIdx.x + gridDim.x, ...; returns the next one to do, -1 behind the last
+  int64_t base = blockIdx.x - static_cast<int64_t>(gridDim.x) * FW_THREADS;
+  int word = FW_THREADS / 32;
+  unsigned left = 0;
+  auto next_tile = [&]() -> int {
+    if (!REDO) return first_tile ? static_cast<int>(blockIdx.x) : -1;
+    while (left == 0) {
+      if (word < FW_THREADS / 32) {
+        left = s_todo[word++];
+        continue;
+      }
+      base += static_cast<int64_t>(gridDim.x) * FW_THREADS;
+      if (base >= p.tiles) return -1;
+      __syncthreads();
+      const int64_t t = base + static_cast<int64_t>(tid) * gridDim.x;
+      const unsigned bal = __ballot_sync(0xffffffffu, t < p.tiles && p.redo_in[t] != 0);
+      if (lane == 0) s_todo[warp] = bal;
+      __syncthreads();
+      word = 0;
+    }
+    const int bit = __ffs(left) - 1;
+    left &= left - 1;
+    return static_cast<int>(base + static_cast<int64_t>((word - 1) * 32 + bit) * gridDim.x);
+  };
+  for (int tile = next_tile(); tile >= 0; tile = next_tile()) {
+  const int bh = tile / p.tiles_x;
+  const int m0 = (tile - bh * p.tiles_x) * p.G;
   const int b_idx = bh / p.H, h_idx = bh - b_idx * p.H;
   const int groups = min(p.G, p.QM - m0);
   const int tile_row0 = m0 * p.g - p.q_pad_head;
@@ -106,7 +145,11 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const uint32_t s_col0 = q_tmem ? 64u : 0u, s_stride = q_tmem ? 64u : 128u;
 
   if (tid == 0) {
-    abort_flag = 0;
+    if (!REDO || first_tile) {
+      abort_flag = 0;
+    } else {
+      for (auto& b : bars) mbar_inval(smem_u32(&b));
+    }
     mbar_init(bar_q, 1);
     mbar_init(bar_final, 1);
     mbar_init(bar_qt, 4);
@@ -123,16 +166,18 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
   }
-  if (warp == 0) {
+  if (warp == 0 && (!REDO || first_tile)) {
     tmem_alloc(smem_u32(&tmem_base_s), 512);
     tmem_relinquish();
   }
-  const int n = build_union(un, p.merged + (static_cast<int64_t>(bh) * p.QM + m0) * p.W, p.W,
-                            groups, p.W, nullptr, p.Mkv, p.status);
+  clear_bitmaps(un);
+  const int n = build_union(un, p.merged + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
+                            p.W, nullptr, p.Mkv, p.lm, p.status);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base_s;
+  first_tile = false;
+  tmem = tmem_base_s;
   WaitCtx w{&abort_flag, p.status};
 
   if (warp == 0) {
@@ -152,9 +197,12 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           tma_load_4d(base + c * kv_chunk_bytes, &tm_k, bar_kvfull(s), c * 64, h_idx / p.kv_hdiv,
                       tok0, b_idx);
         for (int c = 0; c < NCV; c++)
-          tma_load_4d(base + (NCH + c) * kv_chunk_bytes, &tm_v, bar_kvfull(s), p.v_off + c * 64,
+          tma_load_4d(base + (NCH + c) * kv_chunk_bytes, &tm_v, bar_kvfull(s), c * 64,
                       h_idx / p.kv_hdiv, tok0, b_idx);
       }
+      // before the barriers are set up anew for another tile, every commit has arrived
+      for (int i = max(0, n - NST); REDO && i < n; i++)
+        if (!mbar_wait(bar_kvempty(i % NST), (i / NST) & 1, w, FTK_DEV_TIMEOUT_TMA)) break;
     }
   } else if (warp == 1) {
     // -------------------------------------------------------- UMMA issuer
@@ -440,8 +488,9 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       uint8_t* orow = nullptr;
       if (row_valid)
         orow = static_cast<uint8_t*>(p.o) +
-               2 * (static_cast<int64_t>(b_idx) * p.so_b + static_cast<int64_t>(qrow) * p.so_n +
-                    static_cast<int64_t>(h_idx) * p.so_h + p.v_off);
+               (p.out_f32 ? 4 : 2) *
+                   (static_cast<int64_t>(b_idx) * p.so_b + static_cast<int64_t>(qrow) * p.so_n +
+                    static_cast<int64_t>(h_idx) * p.so_h);
       constexpr int HALF = DV / 2;
       for (int c0 = grp_w * HALF; c0 < (grp_w + 1) * HALF; c0 += 32) {
         uint32_t va[32], vb[32];
@@ -463,10 +512,7 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             }
             pk[x >> 1] = pack2(a, b, p.fmt);
           }
-          uint4* dst = reinterpret_cast<uint4*>(orow + c0 * 2);
-#pragma unroll
-          for (int x = 0; x < 4; x++)
-            dst[x] = make_uint4(pk[4 * x], pk[4 * x + 1], pk[4 * x + 2], pk[4 * x + 3]);
+          store_row_part(orow, c0, p.D, pk, p.fmt, p.out_f32 != 0);
         }
       }
       if (row_valid && grp_w == 0)
@@ -477,9 +523,13 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
   tc_fence_before();
   __syncthreads();
-  if (abort_flag)
+  tc_fence_after();
+  if (abort_flag) {
     for (int i = 0; i < 200; i++) __nanosleep(1000);
-  if (warp == 0) tmem_dealloc(tmem, 512);
+    break;   // uniform: barriers and TMEM are not in a state to go on with
+  }
+  }
+  if (warp == 0 && !first_tile) tmem_dealloc(tmem, 512);
 }
 
 }  // namespace ftk
@@ -489,51 +539,159 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
 namespace ftk {
 
+static int tmap_rows(CUtensorMap* out, const ftk_attn& a, char which, int rows) {
+  const void* base = which == 'q' ? a.q : which == 'k' ? a.k : a.v;
+  const int64_t sb = which == 'q' ? a.sq_b : which == 'k' ? a.sk_b : a.sv_b,
+                sn = which == 'q' ? a.sq_n : which == 'k' ? a.sk_n : a.sv_n,
+                sh = which == 'q' ? a.sq_h : which == 'k' ? a.sk_h : a.sv_h;
+  return encode_tmap_bnhd(out, base, a.dtype, a.B, a.N, which == 'q' ? a.H : a.Hkv, a.D, sb, sn, sh,
+                          64, rows);
+}
+
 template <int D, int FMT>
 static int launch_fwd_pipe(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                            const FwdParams& p, int64_t BH, cudaStream_t st) {
   constexpr int NCH = D / 64;
   const size_t smem = 1024 + NCH * 128 * 128 +
                       static_cast<size_t>(FP_KST + FP_VST) * NCH * 64 * 128;
-  if (cudaFuncSetAttribute(sparse_fwd_pipe_kernel<D, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(smem)) != cudaSuccess)
-    return FTK_ERR_CUDA;
-  dim3 grid((p.QM + p.G - 1) / p.G, static_cast<unsigned>(BH));
-  sparse_fwd_pipe_kernel<D, FMT><<<grid, FP_THREADS, smem, st>>>(tq, tk, tv, p);
-  return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
+  if (int e = allow_smem<sparse_fwd_pipe_kernel<D, FMT>>(smem)) return e;
+  return launch_pdl(sparse_fwd_pipe_kernel<D, FMT>,
+                    dim3(p.tiles_x, static_cast<unsigned>(BH)), FP_THREADS, smem, st, tq, tk, tv, p);
 }
 
-template <int D, int DV = D>
+template <int FMT>
+static int launch_fwd_pipe2(const CUtensorMap& tq, const CUtensorMap& tk32, const CUtensorMap& tv,
+                            const FwdParams& p, int64_t BH, cudaStream_t st) {
+  const size_t smem = 1024 + 2 * 128 * 128 + static_cast<size_t>(FP2_KST + FP2_VST) * 8192;
+  if (int e = allow_smem<sparse_fwd_pipe2_kernel<FMT>>(smem)) return e;
+  return launch_pdl(sparse_fwd_pipe2_kernel<FMT>,
+                    dim3(2 * ((p.QM + 3) / 4), static_cast<unsigned>(BH)), FP_THREADS, smem, st, tq,
+                    tk32, tv, p);
+}
+
+template <int D>
 static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                      FwdParams p, int64_t BH, cudaStream_t st) {
-  constexpr int NCH = D / 64, NCV = DV / 64;
-  const int stage_bytes = (NCH + NCV) * p.kvb * 128;
-  // 227 KB per CTA less the static part (union scratch, softmax state: ~19 KB) and the Q tile
+                      FwdParams p, cudaStream_t st) {
+  constexpr int NCH = D / 64;
+  const int stage_bytes = 2 * NCH * p.kvb * 128;
+  // 227 KB per CTA less the static part (union scratch, softmax state: ~20 KB) and the Q tile
   const int ring_bytes = (227 - 21) * 1024 - NCH * 128 * 128;
   int nst = std::min(FW_MAX_STAGES, std::min(168 * 1024, ring_bytes) / stage_bytes);
   if (nst < 2) return FTK_ERR_UNSUPPORTED;
   p.nstages = nst;
   const size_t smem = 1024 + NCH * 128 * 128 + static_cast<size_t>(nst) * stage_bytes;
-  if (cudaFuncSetAttribute(sparse_fwd_kernel<D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(smem)) != cudaSuccess)
-    return FTK_ERR_CUDA;
-  dim3 grid((p.QM + p.G - 1) / p.G, static_cast<unsigned>(BH));
-  for (int v_off = 0; v_off < D; v_off += DV) {
-    p.v_off = v_off;
-    sparse_fwd_kernel<D, DV><<<grid, FW_THREADS, smem, st>>>(tq, tk, tv, p);
+  if constexpr (D <= 128) {
+    if (p.redo_in) {   // finds its tiles itself: as many CTAs as run at once
+      if (int e = allow_smem<sparse_fwd_kernel<D, D, true>>(smem)) return e;
+      return launch_pdl(sparse_fwd_kernel<D, D, true>, std::min(p.tiles, sm_count()), FW_THREADS,
+                        smem, st, tq, tk, tv, p);
+    }
   }
-  return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
+  if (int e = allow_smem<sparse_fwd_kernel<D, D, false>>(smem)) return e;
+  return launch_pdl(sparse_fwd_kernel<D, D, false>, p.tiles, FW_THREADS, smem, st, tq, tk, tv, p);
+}
+
+static size_t fwd_workspace(int64_t BH, int QM, int g) {
+  const int G = attn_groups(g);
+  return static_cast<size_t>(BH) * ((QM + G - 1) / G) * sizeof(int32_t);
+}
+
+static int attn_fwd(const ftk_attn& a, const AttnGrid& gr, void* o, int64_t so_b, int64_t so_n,
+                    int64_t so_h, float* lse, void* workspace, size_t workspace_bytes,
+                    int32_t* status, cudaStream_t st) {
+  if (!aligned16(o, so_b, so_n, so_h) || !lse) return FTK_ERR_BAD_ARG;
+  const int64_t BH = a.B * a.H;
+  FwdParams p{};
+  p.N = static_cast<int>(a.N);
+  p.H = static_cast<int>(a.H);
+  p.D = static_cast<int>(a.D);
+  p.QM = gr.QM;
+  p.W = a.W;
+  p.list_rows = a.list_rows;
+  p.Mkv = gr.Mkv;
+  p.g = gr.g;
+  p.kvb = gr.kvb;
+  p.q_pad_head = gr.q_pad_head;
+  p.kv_pad_head = gr.kv_pad_head;
+  p.G = attn_groups(gr.g);
+  p.fmt = a.dtype;
+  p.out_f32 = a.out_f32;
+  p.scale_log2 = a.scale * 1.4426950408889634f;
+  p.merged = a.lists;
+  p.lm = gr.lm;
+  p.o = o;
+  p.so_b = so_b;
+  p.so_n = so_n;
+  p.so_h = so_h;
+  p.lse = lse;
+  p.status = status;
+  p.kv_hdiv = static_cast<int>(a.H / a.Hkv);
+  p.tiles_x = (gr.QM + p.G - 1) / p.G;
+  if (BH * p.tiles_x > 0x7fffffffLL) return FTK_ERR_BAD_ARG;
+  p.tiles = static_cast<int>(BH * p.tiles_x);
+
+  CUtensorMap tq, tk, tv;
+  int e;
+  if ((e = tmap_rows(&tq, a, 'q', 128))) return e;
+  if ((e = tmap_rows(&tk, a, 'k', gr.kvb))) return e;
+  if ((e = tmap_rows(&tv, a, 'v', gr.kvb))) return e;
+  // 64-row kv blocks, q blocks of 64 or 32 rows and a workspace: the
+  // pipelined kernel runs first and the exact kernel redoes the tiles it flags.
+  const char* env = getenv("FTK_FWD_PIPE");
+  const bool pipe = gr.kd <= 128 && gr.kvb == 64 && (gr.g == 64 || gr.g == 32) && workspace &&
+                    workspace_bytes >= fwd_workspace(BH, gr.QM, gr.g) && !(env && env[0] == '0');
+  if (pipe) {
+    p.redo_out = static_cast<int*>(workspace);
+    const char* env2 = getenv("FTK_FWD_2CTA");
+    // Pairs walk the union of four lists: worth it when the lists can cover a
+    // good part of the blocks (then the unions of two and of four are about
+    // the same length); short lists keep the one-CTA kernel's unions of two.
+    if (gr.kd == 128 && gr.g == 64 && 4 * gr.width >= gr.Mkv && !(env2 && env2[0] == '0')) {
+      // head dim 128: the same kernel on pairs of SMs
+      CUtensorMap tk32;
+      if ((e = tmap_rows(&tk32, a, 'k', 32))) return e;
+      e = a.dtype == FTK_DTYPE_BF16 ? launch_fwd_pipe2<1>(tq, tk32, tv, p, BH, st)
+                                    : launch_fwd_pipe2<0>(tq, tk32, tv, p, BH, st);
+    } else if (a.dtype == FTK_DTYPE_BF16) {
+      e = (gr.kd == 64) ? launch_fwd_pipe<64, 1>(tq, tk, tv, p, BH, st)
+                        : launch_fwd_pipe<128, 1>(tq, tk, tv, p, BH, st);
+    } else {
+      e = (gr.kd == 64) ? launch_fwd_pipe<64, 0>(tq, tk, tv, p, BH, st)
+                        : launch_fwd_pipe<128, 0>(tq, tk, tv, p, BH, st);
+    }
+    if (e) return e;
+    p.redo_out = nullptr;
+    p.redo_in = static_cast<const int*>(workspace);
+  }
+  if (gr.kd == 64) return launch_fwd<64>(tq, tk, tv, p, st);
+  if (gr.kd == 256) return launch_fwd<256>(tq, tk, tv, p, st);
+  return launch_fwd<128>(tq, tk, tv, p, st);
 }
 
 }  // namespace ftk
 
 using namespace ftk;
 
-// One redo word per CTA of the pipelined kernel.
+// One redo word per tile of the pipelined kernel.
+extern "C" size_t ftk_attn_fwd_workspace(const ftk_attn* a) {
+  AttnGrid gr;
+  if (!a || attn_grid(*a, 64, &gr)) return 0;
+  return fwd_workspace(a->B * a->H, gr.QM, gr.g);
+}
+
+extern "C" int ftk_attn_fwd(const ftk_attn* a, void* o, int64_t so_b, int64_t so_n, int64_t so_h,
+                            float* lse, void* workspace, size_t workspace_bytes, int32_t* status,
+                            void* stream) {
+  if (!a) return FTK_ERR_BAD_ARG;
+  AttnGrid gr;
+  if (int e = attn_grid(*a, 64, &gr)) return e;
+  return attn_fwd(*a, gr, o, so_b, so_n, so_h, lse, workspace, workspace_bytes, status,
+                  static_cast<cudaStream_t>(stream));
+}
+
 extern "C" size_t ftk_sparse_fwd_workspace(int64_t B, int64_t H, int QM, int q_block_size) {
   if (B <= 0 || H <= 0 || QM <= 0 || q_block_size <= 0) return 0;
-  const int G = std::max(1, std::min(AT_MAX_GROUPS, 128 / q_block_size));
-  return static_cast<size_t>(B * H) * ((QM + G - 1) / G) * sizeof(int32_t);
+  return fwd_workspace(B * H, QM, q_block_size);
 }
 
 extern "C" int ftk_sparse_fwd(const void* q, const void* k, const void* v, int dtype, int64_t B,
@@ -544,101 +702,13 @@ extern "C" int ftk_sparse_fwd(const void* q, const void* k, const void* v, int d
                               float scale, void* o, int64_t so_b, int64_t so_n, int64_t so_h,
                               float* lse, void* workspace, size_t workspace_bytes,
                               int32_t* status, void* stream) {
-  if (!q || !k || !v || !merged_idx || !o || !lse) return FTK_ERR_BAD_ARG;
-  if (B <= 0 || H <= 0 || N <= 0 || QM <= 0 || W <= 0) return FTK_ERR_BAD_ARG;
-  if (dtype != FTK_DTYPE_F16 && dtype != FTK_DTYPE_BF16) return FTK_ERR_BAD_ARG;
-  if (Hkv <= 0) Hkv = H;
-  if (H % Hkv != 0) return FTK_ERR_BAD_ARG;
-  if (q_block_size <= 0 || kv_block_size <= 0) return FTK_ERR_BAD_ARG;
-  if (q_pad_head < 0 || q_pad_head >= q_block_size || kv_pad_head < 0 ||
-      kv_pad_head >= kv_block_size)
-    return FTK_ERR_BAD_ARG;
-  if (static_cast<int64_t>(QM) * q_block_size < q_pad_head + N) return FTK_ERR_BAD_ARG;
   if (D != 64 && D != 128 && D != 256) return FTK_ERR_UNSUPPORTED;
-  if (q_block_size > 128) return FTK_ERR_UNSUPPORTED;
-  if (kv_block_size % 16 != 0 || kv_block_size > 128) return FTK_ERR_UNSUPPORTED;
-  const int64_t Mkv = (kv_pad_head + N + kv_block_size - 1) / kv_block_size;
-  if (Mkv > AT_MAX_BLOCKS) return FTK_ERR_UNSUPPORTED;
-  if (B * H > 65535) return FTK_ERR_BAD_ARG;
-  if ((reinterpret_cast<uintptr_t>(o) & 15u) || (so_b & 7) || (so_n & 7) || (so_h & 7))
-    return FTK_ERR_BAD_ARG;
-
-  FwdParams p{};
-  p.N = static_cast<int>(N);
-  p.H = static_cast<int>(H);
-  p.QM = QM;
-  p.W = W;
-  p.Mkv = static_cast<int>(Mkv);
-  p.g = q_block_size;
-  p.kvb = kv_block_size;
-  p.q_pad_head = q_pad_head;
-  p.kv_pad_head = kv_pad_head;
-  p.G = std::max(1, std::min(AT_MAX_GROUPS, 128 / q_block_size));
-  p.fmt = dtype;
-  p.scale_log2 = scale * 1.4426950408889634f;
-  p.merged = merged_idx;
-  p.o = o;
-  p.so_b = so_b;
-  p.so_n = so_n;
-  p.so_h = so_h;
-  p.lse = lse;
-  p.status = status;
-  p.kv_hdiv = static_cast<int>(H / Hkv);
-
-  CUtensorMap tq, tk, tv;
-  int e = encode_tmap_bnhd(&tq, q, dtype, B, N, H, D, sq_b, sq_n, sq_h, 64, 128);
-  if (e) return e;
-  e = encode_tmap_bnhd(&tk, k, dtype, B, N, Hkv, D, sk_b, sk_n, sk_h, 64, kv_block_size);
-  if (e) return e;
-  e = encode_tmap_bnhd(&tv, v, dtype, B, N, Hkv, D, sv_b, sv_n, sv_h, 64, kv_block_size);
-  if (e) return e;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // 64-row kv blocks, q blocks of 64 or 32 rows and a workspace: the
-  // pipelined kernel runs first and the exact kernel redoes the CTAs it flags.
-  const char* env = getenv("FTK_FWD_PIPE");
-  const bool pipe = D <= 128 && kv_block_size == 64 && (q_block_size == 64 || q_block_size == 32) && workspace &&
-                    workspace_bytes >= ftk_sparse_fwd_workspace(B, H, QM, q_block_size) &&
-                    !(env && env[0] == '0');
-  if (pipe) {
-    p.redo_out = static_cast<int*>(workspace);
-    const char* env2 = getenv("FTK_FWD_2CTA");
-    // Pairs walk the union of four lists: worth it when the lists can cover a
-    // good part of the blocks (then the unions of two and of four are about
-    // the same length); short lists keep the one-CTA kernel's unions of two.
-    if (D == 128 && q_block_size == 64 && 4 * static_cast<int64_t>(W) >= Mkv &&
-        !(env2 && env2[0] == '0')) {
-      // head dim 128: the same kernel on pairs of SMs
-      CUtensorMap tk32;
-      e = encode_tmap_bnhd(&tk32, k, dtype, B, N, Hkv, D, sk_b, sk_n, sk_h, 64, 32);
-      if (e) return e;
-      const size_t smem2 = 1024 + 2 * 128 * 128 + static_cast<size_t>(FP2_KST + FP2_VST) * 8192;
-      dim3 grid2(2 * ((QM + 3) / 4), static_cast<unsigned>(B * H));
-      if (dtype == FTK_DTYPE_BF16) {
-        if (cudaFuncSetAttribute(sparse_fwd_pipe2_kernel<1>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem2)) != cudaSuccess)
-          return FTK_ERR_CUDA;
-        sparse_fwd_pipe2_kernel<1><<<grid2, FP_THREADS, smem2, st>>>(tq, tk32, tv, p);
-      } else {
-        if (cudaFuncSetAttribute(sparse_fwd_pipe2_kernel<0>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem2)) != cudaSuccess)
-          return FTK_ERR_CUDA;
-        sparse_fwd_pipe2_kernel<0><<<grid2, FP_THREADS, smem2, st>>>(tq, tk32, tv, p);
-      }
-      e = cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
-    } else if (dtype == FTK_DTYPE_BF16) {
-      e = (D == 64) ? launch_fwd_pipe<64, 1>(tq, tk, tv, p, B * H, st)
-                    : launch_fwd_pipe<128, 1>(tq, tk, tv, p, B * H, st);
-    } else {
-      e = (D == 64) ? launch_fwd_pipe<64, 0>(tq, tk, tv, p, B * H, st)
-                    : launch_fwd_pipe<128, 0>(tq, tk, tv, p, B * H, st);
-    }
-    if (e) return e;
-    p.redo_out = nullptr;
-    p.redo_in = static_cast<const int*>(workspace);
-  }
-  if (D == 64) return launch_fwd<64>(tq, tk, tv, p, B * H, st);
-  if (D == 256) return launch_fwd<256, 256>(tq, tk, tv, p, B * H, st);
-  return launch_fwd<128>(tq, tk, tv, p, B * H, st);
+  const ftk_attn a = {q,    k,    v,    dtype, 0,    B,    H,    Hkv <= 0 ? H : Hkv,
+                      N,    D,    sq_b, sq_n,  sq_h, sk_b, sk_n, sk_h,
+                      sv_b, sv_n, sv_h, merged_idx, QM, W, q_block_size, kv_block_size,
+                      q_pad_head, kv_pad_head, scale};
+  AttnGrid gr;
+  if (int e = attn_grid(a, 128, &gr)) return e;   // blocks of up to 128 rows as they are
+  return attn_fwd(a, gr, o, so_b, so_n, so_h, lse, workspace, workspace_bytes, status,
+                  static_cast<cudaStream_t>(stream));
 }

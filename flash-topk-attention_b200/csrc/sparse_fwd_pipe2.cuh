@@ -101,8 +101,11 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_alloc2(smem_u32(&tmem_base_s), 512);
     tmem_relinquish2();
   }
-  const int n = build_union(un, p.merged + (static_cast<int64_t>(bh) * p.QM + m0) * p.W, p.W,
-                            groups, p.W, nullptr, p.Mkv, p.status);
+  clear_bitmaps(un);
+  pdl_wait();
+  pdl_launch();
+  const int n = build_union(un, p.merged + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
+                            p.W, nullptr, p.Mkv, p.lm, p.status);
   // lowest listed block of each q-block: its scores give the rows' reference
   if (warp < 4) {
     int best = 0x7fffffff;
@@ -428,7 +431,8 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
       uint8_t* orow = nullptr;
       if (row_valid)
         orow = static_cast<uint8_t*>(p.o) +
-               2 * (static_cast<int64_t>(b_idx) * p.so_b + static_cast<int64_t>(qrow) * p.so_n +
+               (p.out_f32 ? 4 : 2) *
+                   (static_cast<int64_t>(b_idx) * p.so_b + static_cast<int64_t>(qrow) * p.so_n +
                     static_cast<int64_t>(h_idx) * p.so_h);
       constexpr int QUART = D / 4;   // 32 columns per group
       const int c0 = gw * QUART;
@@ -445,10 +449,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
           const float b = have ? __uint_as_float(ov[x + 1]) * inv : 0.f;
           pk[x >> 1] = pack16<FMT>(a, b);
         }
-        uint4* dst = reinterpret_cast<uint4*>(orow + c0 * 2);
-#pragma unroll
-        for (int x = 0; x < QUART / 8; x++)
-          dst[x] = make_uint4(pk[4 * x], pk[4 * x + 1], pk[4 * x + 2], pk[4 * x + 3]);
+        store_row_part(orow, c0, p.D, pk, FMT, p.out_f32 != 0);
       }
       if (row_valid && gw == 0)
         p.lse[static_cast<int64_t>(bh) * p.N + qrow] =

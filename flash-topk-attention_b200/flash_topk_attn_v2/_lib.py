@@ -40,6 +40,14 @@ SIGNATURES = {
     "ftk_build_reverse_noalloc": (i32, [vp, vp, i64, i32, i32, i32, vp, vp, vp, vp, vp]),
     "ftk_sort_by_count_workspace": (sz, [i64, i32]),
     "ftk_sort_by_count": (i32, [vp, i64, i32, vp, vp, vp, sz, vp]),
+    "ftk_cast_bf16": (i32, [vp, i64, vp, vp, i64, vp, vp, i64, vp, vp]),
+    "ftk_attn_fwd_workspace": (sz, [vp]),
+    "ftk_attn_fwd": (i32, [vp, vp, *_STRIDES3, vp, vp, sz, vp, vp]),
+    "ftk_attn_bwd_workspace": (sz, [vp]),
+    "ftk_attn_bwd_dq": (i32, [vp, vp, *_STRIDES3, vp, *_STRIDES3, vp, vp, sz, vp, *_STRIDES3, vp,
+                              vp]),
+    "ftk_attn_bwd_dkv": (i32, [vp, vp, *_STRIDES3, vp, vp, sz, vp, *_STRIDES3, vp, *_STRIDES3, vp,
+                               vp]),
     "ftk_sparse_fwd_workspace": (sz, [i64, i64, i32, i32]),
     "ftk_sparse_fwd": (i32, [vp, vp, vp, i32, i64, i64, i64, i64, i64, *_STRIDES3, *_STRIDES3,
                              *_STRIDES3, vp, i32, i32, i32, i32, i32, i32, f32, vp, *_STRIDES3,

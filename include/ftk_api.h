@@ -16,7 +16,8 @@
  *   - Return value: FTK_OK or a negative FTK_ERR_* code; nothing is launched
  *     when an argument check fails.  Device-side problems (a bounded wait
  *     that ran out, an out-of-range block id) are reported asynchronously in
- *     `*status` (device int32, see FTK_DEV_*).  The word is sticky: the
+ *     `*status` (int32 the device can write: device memory or mapped pinned host
+ *     memory, see FTK_DEV_*).  The word is sticky: the
  *     library only ever writes it on a failure and the first failure wins, so
  *     the caller zeroes it once and may read it after any number of calls.
  *     `status` may be NULL.
@@ -33,6 +34,8 @@
 
 #include <stddef.h>
 #include <stdint.h>
+
+#include "ftk_attn.h"
 
 #ifdef __cplusplus
 extern "C" {
@@ -192,6 +195,42 @@ size_t ftk_sort_by_count_workspace(int64_t total, int max_count);
 int ftk_sort_by_count(const int32_t* counts, int64_t total, int max_count,
                       int32_t* sorted_counts, int32_t* sorted_ids, void* workspace,
                       size_t workspace_bytes, void* stream);
+
+/* float -> bf16 (round to nearest even) of up to three contiguous arrays in one
+ * launch; NULL source = none.  Counts are multiples of 8, pointers 16-byte
+ * aligned.  The reference converts float32 activations with PyTorch
+ * (block_score_cuda.py:115-118, sparse_attn.py:270-273). */
+int ftk_cast_bf16(const float* a, int64_t na, void* to_a, const float* b, int64_t nb, void* to_b,
+                  const float* c, int64_t nc, void* to_c, void* stream);
+
+/* ------------------------------------------- block-sparse attention, by problem
+ * The same attention as the calls further down, one problem description
+ * (ftk_attn.h) for all three, and
+ *   - any head dim that is a multiple of 8 up to 256 (columns beyond D are
+ *     never read or written: nothing has to be padded by the caller);
+ *   - q and kv blocks of up to 128 rows (multiples of 32 above 64; in the
+ *     backward at D > 128 sizes that halve down to 16 or 32): the lists are read
+ *     in place as lists over parts of the block;
+ *   - float results for callers whose activations are float32;
+ *   - the backward in two launches: ftk_attn_bwd_dq computes delta and dQ and
+ *     leaves in the workspace, one byte per (q tile, kv block), which q-blocks
+ *     list which kv block; ftk_attn_bwd_dkv reads those instead of a reverse
+ *     index.  Both get the same workspace (256-byte aligned) and `a`, in this
+ *     order; dk and dv have Hkv heads (the heads of a group are summed here).
+ * Outputs have strides (s*_b, s*_n, s*_h) in elements, multiples of 8; `o` of the
+ * backward has the type that the forward wrote. */
+size_t ftk_attn_fwd_workspace(const ftk_attn* a);
+int ftk_attn_fwd(const ftk_attn* a, void* o, int64_t so_b, int64_t so_n, int64_t so_h, float* lse,
+                 void* workspace, size_t workspace_bytes, int32_t* status, void* stream);
+size_t ftk_attn_bwd_workspace(const ftk_attn* a);
+int ftk_attn_bwd_dq(const ftk_attn* a, const void* o, int64_t so_b, int64_t so_n, int64_t so_h,
+                    const void* dout, int64_t sdo_b, int64_t sdo_n, int64_t sdo_h,
+                    const float* lse, void* workspace, size_t workspace_bytes, void* dq,
+                    int64_t sdq_b, int64_t sdq_n, int64_t sdq_h, int32_t* status, void* stream);
+int ftk_attn_bwd_dkv(const ftk_attn* a, const void* dout, int64_t sdo_b, int64_t sdo_n,
+                     int64_t sdo_h, const float* lse, void* workspace, size_t workspace_bytes,
+                     void* dk, int64_t sdk_b, int64_t sdk_n, int64_t sdk_h, void* dv,
+                     int64_t sdv_b, int64_t sdv_n, int64_t sdv_h, int32_t* status, void* stream);
 
 /* -------------------------------------------------------- sparse attention
  * Replaces sparse_attn_fwd_launch (csrc/sparse_attn.cpp:3-12,
