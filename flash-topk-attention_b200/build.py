@@ -5,7 +5,9 @@
 Each csrc/*.cu is compiled to an object under build/ and the objects are
 linked into lib/libftk_sm100.so (CUDA runtime linked statically; the driver
 API is reached through cudaGetDriverEntryPoint, so the library also loads on
-a machine without a GPU driver).
+a machine without a GPU driver).  csrc/host/torch_ops.cpp, the native layer
+between the Python operators and that library, becomes
+flash_topk_attn_v2/_native.so (host code only: g++ against PyTorch's headers).
 """
 
 from __future__ import annotations
@@ -33,7 +35,9 @@ def _sources():
 
 
 def _headers_mtime():
-    hs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
+    include = os.path.join(os.path.dirname(HERE), "include")
+    hs = [os.path.join(d, f) for d in (CSRC, include) for f in os.listdir(d)
+          if f.endswith((".cuh", ".h"))]
     return max(os.path.getmtime(h) for h in hs) if hs else 0.0
 
 
@@ -67,6 +71,38 @@ def build(force: bool = False) -> str:
     return LIB
 
 
+HOST_SRC = os.path.join(CSRC, "host", "torch_ops.cpp")
+NATIVE = os.path.join(HERE, "flash_topk_attn_v2", "_native.so")
+CXX = os.environ.get("CXX", "g++")
+
+
+def build_native(force: bool = False) -> str:
+    """flash_topk_attn_v2/_native.so; links lib/libftk_sm100.so (built first)."""
+    include = os.path.join(os.path.dirname(HERE), "include")
+    newest = max(os.path.getmtime(p) for p in
+                 [HOST_SRC] + [os.path.join(include, f) for f in os.listdir(include)])
+    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= newest:
+        return NATIVE
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension as ext
+
+    cuda = os.path.dirname(os.path.dirname(NVCC))
+    dirs = [*ext.include_paths(), os.path.join(cuda, "include"), sysconfig.get_path("include")]
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = [CXX, "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           *[x for d in dirs for x in ("-isystem", d)], HOST_SRC, "-o", NATIVE,
+           "-L", LIBDIR, "-l:libftk_sm100.so", "-Wl,-rpath,$ORIGIN/../lib",
+           "-L", torch_lib, "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+           "-ltorch_python", f"-Wl,-rpath,{torch_lib}"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{CXX} failed for torch_ops.cpp:\n{r.stdout}\n{r.stderr}")
+    return NATIVE
+
+
 PROBE_SRC = os.path.join(os.path.dirname(HERE), "tests", "native", "wait_probe.cu")
 PROBE_LIB = os.path.join(os.path.dirname(HERE), "tests", "native", "libftk_wait_probe.so")
 
@@ -89,4 +125,5 @@ def build_wait_probe(force: bool = False) -> str:
 
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv))
+    print(build_native(force="--force" in sys.argv))
     print(build_wait_probe(force="--force" in sys.argv))

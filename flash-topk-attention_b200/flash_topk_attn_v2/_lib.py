@@ -78,6 +78,14 @@ def _load() -> C.CDLL:
 
 lib = _load()
 
+try:
+    from . import _native as native  # links the library loaded above
+except ImportError as e:
+    raise ImportError(
+        f"the native host layer of this package is missing or does not load ({e}): build it with "
+        "`python flash-topk-attention_b200/build.py`. This package has no fallback path."
+    ) from e
+
 
 def error_text(code: int) -> str:
     return lib.ftk_error_string(int(code)).decode()

@@ -3,8 +3,10 @@
 Same names, arguments, checks and exceptions as the reference's operator layer
 (flash_topk_attn_v2/block_score.py, topk_select.py, qblock_merge.py,
 sparse_attn.py, build_reverse_indices_cuda.py, sort_by_count_cuda.py); the
-work itself is done by libftk_sm100.so.  PyTorch is used for device memory and
-streams only.
+work itself is done by libftk_sm100.so.  The operators of the hot path
+(scoring, merge, attention and its backward) reach it through the native host
+layer _native.so, which allocates, launches and holds the autograd node; the
+others through ctypes.  PyTorch is used for device memory and streams only.
 """
 
 from __future__ import annotations
@@ -15,17 +17,17 @@ import os
 import torch
 
 from . import _lib
-from ._lib import check, lib, ptr, stream_ptr
+from ._lib import check, lib, native, ptr, stream_ptr
 
 _SCORE_SCRATCH_BYTES = int(os.environ.get("FTK_SCORE_SCRATCH_BYTES", 4 << 30))
 _DEBUG = os.environ.get("FTK_DEBUG", "0") not in ("", "0")
-_status_words = {}
+native.set_debug(_DEBUG)
 _launches = 0
 
 
 def launch_count() -> int:
     """Kernels of libftk_sm100.so enqueued by this process so far."""
-    return _launches
+    return _launches + native.launch_count()
 
 
 def _count(n: int) -> None:
@@ -34,7 +36,7 @@ def _count(n: int) -> None:
 
 
 # Optional per-call CUDA-event timing (off by default; bench.py switches it on
-# around its timed loop).  Every C-ABI call is bracketed by two events on the
+# around its timed loop).  Every entry point is bracketed by two events on the
 # stream it launches on; `event_times()` returns milliseconds per entry point.
 _events = None
 
@@ -42,109 +44,83 @@ _events = None
 def enable_event_timing(on: bool) -> None:
     global _events
     _events = [] if on else None
+    native.set_timing(on)
 
 
-def _call(name, fn, *args) -> None:
-    """Run one C-ABI entry point, map its return code, time it when asked."""
+def _call(name, fn, *args):
+    """Run one entry point (C ABI: map its return code; native: hand back what it
+    returns), timed when asked."""
     if _events is None:
-        check(fn(*args), name)
-        return
-    e0 = torch.cuda.Event(enable_timing=True)
-    e1 = torch.cuda.Event(enable_timing=True)
-    e0.record()
-    rc = fn(*args)
-    e1.record()
-    _events.append((name, e0, e1))
-    check(rc, name)
+        out = fn(*args)
+    else:
+        e0 = torch.cuda.Event(enable_timing=True)
+        e1 = torch.cuda.Event(enable_timing=True)
+        e0.record()
+        out = fn(*args)
+        e1.record()
+        _events.append((name, e0, e1))
+    if out.__class__ is int:
+        check(out, name)
+    return out
 
 
 def event_times() -> dict:
     """Sum of device milliseconds and call count per entry point since
     enable_event_timing(True); synchronises."""
     out = {}
-    if _events:
+    if _events is not None:
         torch.cuda.synchronize()
-        for name, e0, e1 in _events:
+        times = [(name, e0.elapsed_time(e1)) for name, e0, e1 in _events] + native.take_times()
+        for name, t in times:
             ms, n = out.get(name, (0.0, 0))
-            out[name] = (ms + e0.elapsed_time(e1), n + 1)
+            out[name] = (ms + t, n + 1)
     return out
 
 
+def _device_index(device) -> int:
+    index = torch.device(device).index
+    return torch.cuda.current_device() if index is None else index
+
+
+# A device-side failure (a bounded wait that ran out, a block id out of range)
+# only sets a sticky status word, one per device, in pinned host memory.  So that
+# a caller who never calls check_errors() still hears of it, every operator
+# begins by looking at the word: the failure raises at the first call that finds
+# it.  FTK_DEBUG=1 checks synchronously after every operator instead.
 def status_word(device) -> torch.Tensor:
-    """Sticky per-device status word handed to every launch."""
-    dev = torch.device(device)
-    key = dev.index if dev.index is not None else torch.cuda.current_device()
-    t = _status_words.get(key)
-    if t is None:
-        t = torch.zeros(1, dtype=torch.int32, device=dev)
-        _status_words[key] = t
-    return t
+    """Sticky per-device status word handed to every launch (pinned host memory)."""
+    return native.status_word(_device_index(device))
 
 
 def check_errors(device=None) -> None:
-    """Synchronise and raise if any launch since the last check reported a
-    device-side failure (bounded wait ran out, block id out of range)."""
-    for key, t in list(_status_words.items()):
-        if device is not None and torch.device(device).index not in (None, key):
-            continue
-        code = int(t.item())
-        snap = _snapshots.get(key)
-        if snap is not None:
-            snap[0][0] = 0
-            snap[1] = None
+    """Synchronise the current stream and raise if any launch since the last
+    check reported a device-side failure."""
+    if device is None or torch.device(device).index is None:
+        indices = range(torch.cuda.device_count()) if device is None else [_device_index(device)]
+    else:
+        indices = [torch.device(device).index]
+    for index in indices:
+        torch.cuda.current_stream(index).synchronize()
+        code = native.take_status(index)
         if code != 0:
-            t.zero_()
             raise RuntimeError(
                 f"flash_topk_attn_v2 device error: {_lib.error_text(code)} (status {code})"
             )
 
 
-# A device-side failure (a bounded wait that ran out, a block id out of range)
-# only sets the sticky status word.  So that a caller who never calls
-# check_errors() still hears of it, every operator ends by copying the word to
-# pinned host memory on its stream (4 bytes, no synchronisation) and begins by
-# looking at the copy the previous operator left, if that copy has landed: the
-# failure raises at the next call that finds it, usually one call late.
-# FTK_DEBUG=1 checks synchronously after every operator instead.
-_snapshots = {}
-_deferred = True
-
-
 def deferred_checks(on: bool) -> None:
-    """Switch the look at the previous operator's status copy on or off (on by
-    default).  Off, a device-side failure is only reported by check_errors()."""
-    global _deferred
-    _deferred = bool(on)
+    """Switch the operators' look at the status word on or off (on by default).
+    Off, a device-side failure is only reported by check_errors()."""
+    native.set_deferred(bool(on))
+
+
+def _before(device) -> None:
+    native.look(_device_index(device))
 
 
 def _after(device) -> None:
-    if _DEBUG:
-        if not torch.cuda.is_current_stream_capturing():   # a capture cannot synchronise
-            check_errors(device)
-        return
-    dev = torch.device(device)
-    key = dev.index if dev.index is not None else torch.cuda.current_device()
-    if not _deferred or torch.cuda.is_current_stream_capturing():
-        return
-    snap = _snapshots.get(key)
-    if snap is None:
-        snap = _snapshots[key] = [torch.zeros(1, dtype=torch.int32).pin_memory(), None]
-    host, ev = snap
-    if ev is not None:
-        if not ev.query():
-            return                       # previous copy still in flight: look next time
-        code = int(host[0])
-        if code != 0:
-            host[0] = 0
-            snap[1] = None
-            status_word(dev).zero_()
-            raise RuntimeError(
-                f"flash_topk_attn_v2 device error in an earlier call: {_lib.error_text(code)} "
-                f"(status {code})")
-    host.copy_(status_word(dev), non_blocking=True)
-    ev = torch.cuda.Event()
-    ev.record(torch.cuda.current_stream(dev))
-    snap[1] = ev
+    if _DEBUG and not torch.cuda.is_current_stream_capturing():   # a capture cannot synchronise
+        check_errors(device)
 
 
 def _next_pow2(x: int) -> int:
@@ -264,6 +240,7 @@ def flash_block_score(q, k, num_heads, score_block_size, padding=(0, 0)):
     Mirrors flash_block_score (flash_topk_attn_v2/block_score.py:417-452)."""
     input_4d, B, H, N, D, M, ph, pt = _parse_block_score_args(
         q, k, num_heads, score_block_size, padding)
+    _before(q.device)
     qq, sq, kk, sk, Dk = _prep_qk(q, k, input_4d, H, D)
     out = torch.empty(B, H, N, M, dtype=torch.float32, device=q.device)
     status = status_word(q.device)
@@ -277,7 +254,7 @@ def flash_block_score(q, k, num_heads, score_block_size, padding=(0, 0)):
             ptr(qq), ptr(kk), _lib.dtype_code(qq), B, H, N, Dk, *sq, *sk, b0, cnt,
             score_block_size, ph, pt, float(D) ** -0.5, ptr(flat[b0]), ptr(ws), ws.numel(),
             ptr(status), stream_ptr(q.device))
-        _count(4)
+        _count(2)
     _after(q.device)
     return out
 
@@ -317,6 +294,7 @@ def flash_topk_select(block_scores, threshold, max_topk, score_block_size, paddi
     m_out = min(max_topk, M) if max_topk > 0 else M
     scores = block_scores.float().contiguous()
     dev = scores.device
+    _before(dev)
     idx = torch.empty(B, H, N, m_out, dtype=torch.int32, device=dev)
     raw = torch.empty(B, H, N, m_out, dtype=torch.float32, device=dev)
     avg = torch.empty(B, H, N, m_out, dtype=torch.float32, device=dev)
@@ -336,26 +314,22 @@ def flash_topk_score_fused(q, k, num_heads, score_block_size, topk, padding, thr
         raise ValueError("max_topk must be >= 0")
     if M > 4096:
         raise NotImplementedError(f"select requires M <= 4096, got M={M}")
-    qq, sq, kk, sk, Dk = _prep_qk(q, k, input_4d, H, D)
-    dev = q.device
-    m_out = min(topk, M) if topk > 0 else M
-    idx = torch.empty(B, H, N, m_out, dtype=torch.int32, device=dev)
-    raw = torch.empty(B, H, N, m_out, dtype=torch.float32, device=dev)
-    avg = torch.empty(B, H, N, m_out, dtype=torch.float32, device=dev)
-    per_slice = lib.ftk_score_topk_workspace(1, N, M)
-    step = int(max(1, min(B * H, 32768, _SCORE_SCRATCH_BYTES // max(per_slice, 1))))
-    ws = torch.empty(lib.ftk_score_topk_workspace(step, N, M), dtype=torch.uint8, device=dev)
-    status = status_word(dev)
-    fi, fr, fa = (t.view(B * H, N, m_out) for t in (idx, raw, avg))
-    for b0 in range(0, B * H, step):
-        cnt = min(step, B * H - b0)
-        _call("ftk_score_topk", lib.ftk_score_topk, 
-            ptr(qq), ptr(kk), _lib.dtype_code(qq), B, H, N, Dk, *sq, *sk, b0, cnt,
-            score_block_size, ph, pt, float(D) ** -0.5, topk, float(threshold),
-            ptr(fi[b0]), ptr(fr[b0]), ptr(fa[b0]), ptr(ws), ws.numel(), ptr(status),
-            stream_ptr(dev))
-        _count(4)
-    _after(dev)
+    if D % 8 or D > 256:   # head dims that a tensor map cannot read in place
+        Dk = _kernel_head_dim(D)
+        q = _pad_head_dim(q, input_4d, H, D, Dk)
+        k = _pad_head_dim(k, input_4d, H, D, Dk)
+    slices = B * H
+    step = min(slices, 32768,
+               max(1, _SCORE_SCRATCH_BYTES // native.score_topk_workspace(1, N, M)))
+    if step < slices and q.dtype == torch.float32:
+        q, k = q.bfloat16(), k.bfloat16()
+    outs = []
+    for b0 in range(0, slices, step):
+        outs = _call("ftk_score_topk", native.score_topk, q, k, input_4d, H, score_block_size, topk,
+                     ph, pt, threshold, float(D) ** -0.5, b0, min(step, slices - b0), outs)
+    if _DEBUG:
+        _after(q.device)
+    idx, raw, avg = outs
     # lets build_qblock_topk_indices size its table without a device round trip
     idx._ftk_num_score_blocks = M
     return idx, raw, avg
@@ -378,19 +352,20 @@ def num_score_blocks_of(topk_indices) -> int:
 
 
 def flash_qblock_merge(topk_indices, topk_scores, q_block_size, qblock_topk, num_score_blocks,
-                       q_padding=(0, 0), return_counts=False):
+                       q_padding=(0, 0), return_counts=False, want_scores=True):
     """Per-q-block aggregation + ranking of (block, score) pairs.
 
     Mirrors flash_qblock_merge (flash_topk_attn_v2/qblock_merge.py:85-156).
     `q_padding` is an extension: the reference pads the index tensor on the
-    host first (__init__.py:90-96); here the kernel skips the virtual rows."""
+    host first (__init__.py:90-96); here the kernel skips the virtual rows.
+    `want_scores=False` leaves the aggregated scores out (None in their place)."""
     if topk_indices.ndim != 4:
         raise ValueError("topk_indices must be [B, H, N, M_out]")
     if topk_scores is not None and topk_scores.ndim != 4:
         raise ValueError("topk_scores must be [B, H, N, M_out]")
     if topk_indices.device.type != "cuda":
         raise ValueError("flash_qblock_merge requires CUDA tensors")
-    B, H, N, K = topk_indices.shape
+    N = topk_indices.shape[2]
     qh, qt = q_padding
     if (qh + N + qt) % q_block_size != 0:
         raise ValueError(f"N ({qh + N + qt}) must be divisible by q_block_size ({q_block_size})")
@@ -401,18 +376,11 @@ def flash_qblock_merge(topk_indices, topk_scores, q_block_size, qblock_topk, num
             f"num_score_blocks={num_score_blocks} exceeds CUDA block sort limit 4096")
     if qblock_topk <= 0:
         raise ValueError("qblock_topk must be positive")
-    QM = (qh + N + qt) // q_block_size
-    dev = topk_indices.device
-    idx = topk_indices.to(torch.int32).contiguous()
-    scr = None if topk_scores is None else topk_scores.float().contiguous()
-    merged = torch.empty(B, H, QM, qblock_topk, dtype=torch.int32, device=dev)
-    mscores = torch.empty(B, H, QM, qblock_topk, dtype=torch.float32, device=dev)
-    counts = torch.empty(B, H, QM, dtype=torch.int32, device=dev)
-    _call("ftk_qblock_merge", lib.ftk_qblock_merge, 
-        ptr(idx), ptr(scr), B * H, N, K, q_block_size, qh, qt, num_score_blocks, qblock_topk,
-        ptr(merged), ptr(mscores), ptr(counts), ptr(status_word(dev)), stream_ptr(dev))
-    _count(1)
-    _after(dev)
+    merged, mscores, counts = _call(
+        "ftk_qblock_merge", native.qblock_merge, topk_indices, topk_scores, q_block_size, qh, qt,
+        num_score_blocks, qblock_topk, want_scores)
+    if _DEBUG:
+        _after(merged.device)
     if return_counts:
         return merged, mscores, counts
     return merged, mscores
@@ -435,6 +403,7 @@ def flash_qblock_union(topk_indices, q_block_size, q_padding=(0, 0), num_score_b
     qh, qt = q_padding
     QM = (qh + N + qt) // q_block_size
     dev = topk_indices.device
+    _before(dev)
     idx = topk_indices.to(torch.int32).contiguous()
     if num_score_blocks is None:
         num_score_blocks = max(int(idx.max().item()) + 1, 1)
@@ -463,6 +432,7 @@ def flash_build_reverse_indices_cuda(merged_indices, counts, num_kv_blocks):
     B, H, QM, W = merged_indices.shape
     M = num_kv_blocks
     dev = merged_indices.device
+    _before(dev)
     merged = merged_indices.contiguous()
     cnt = None if counts is None else counts.to(torch.int32).contiguous()
     rev = torch.empty(B, H, M, QM, dtype=torch.int32, device=dev)
@@ -500,94 +470,11 @@ def flash_sort_by_count_cuda(reverse_counts, num_heads, num_kv_blocks):
 # --------------------------------------------------------------------------
 def preprocess_delta(o, do, num_heads):
     """delta = rowsum(O * dO), [B, H, N] fp32 (sparse_attn_bwd.py:12-33).
-    Host-side convenience; the backward computes it inside ftk_sparse_bwd_dq."""
+    Host-side convenience; the backward computes it inside the dQ kernel."""
     B, N, C = o.shape
     D = C // num_heads
     return (o.float().view(B, N, num_heads, D) * do.float().view(B, N, num_heads, D)).sum(-1) \
         .permute(0, 2, 1).contiguous()
-
-
-class FlashSparseAttnFunc(torch.autograd.Function):
-    """Forward and backward of the gathered-KV attention
-    (reference: FlashSparseAttnFunc, flash_topk_attn_v2/sparse_attn.py:130-224)."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, merged_indices, num_heads, q_block_size, kv_block_size, scale,
-                q_pad_head, kv_pad_head, num_kv_blocks, num_kv_heads=None):
-        B, N, C = q.shape
-        H = num_heads
-        Hkv = num_kv_heads or H
-        D = C // H
-        dev = q.device
-        qq, sq_b, sq_n, sq_h = _as_bnhd(q, False, H, D)
-        kk, sk_b, sk_n, sk_h = _as_bnhd(k, False, Hkv, D)
-        vv, sv_b, sv_n, sv_h = _as_bnhd(v, False, Hkv, D)
-        merged = merged_indices.contiguous()
-        QM, W = merged.shape[2], merged.shape[3]
-        o = torch.empty(B, N, C, dtype=q.dtype, device=dev)
-        lse = torch.empty(B, H, N, dtype=torch.float32, device=dev)
-        ws_bytes = int(lib.ftk_sparse_fwd_workspace(B, H, QM, q_block_size))
-        ws = torch.empty(max(ws_bytes, 4), dtype=torch.uint8, device=dev)
-        _call("ftk_sparse_fwd", lib.ftk_sparse_fwd, 
-            ptr(qq), ptr(kk), ptr(vv), _lib.dtype_code(qq), B, H, Hkv, N, D,
-            sq_b, sq_n, sq_h, sk_b, sk_n, sk_h, sv_b, sv_n, sv_h,
-            ptr(merged), QM, W, q_block_size, kv_block_size, q_pad_head, kv_pad_head,
-            float(scale), ptr(o), N * C, C, D, ptr(lse), ptr(ws), ws_bytes,
-            ptr(status_word(dev)), stream_ptr(dev))
-        piped = (kv_block_size == 64 and q_block_size in (32, 64)
-                 and os.environ.get("FTK_FWD_PIPE", "1")[:1] != "0")
-        _count(2 if piped else 1)
-        _after(dev)
-        ctx.save_for_backward(qq, kk, vv, o, lse, merged)
-        ctx.meta = (H, D, q_block_size, kv_block_size, float(scale), q_pad_head, kv_pad_head,
-                    num_kv_blocks, Hkv)
-        ctx.mark_non_differentiable(lse)
-        return o, lse
-
-    @staticmethod
-    def backward(ctx, grad_o, _grad_lse):
-        qq, kk, vv, o, lse, merged = ctx.saved_tensors
-        H, D, g, kvb, scale, qph, kph, M, Hkv = ctx.meta
-        B, N, C = qq.shape
-        dev = qq.device
-        _check_backward_blocks(D, g, kvb)
-        if D > 128 and (g > 32 or kvb > 32):
-            # head dim 256: the gradient kernels hold Q / dO (dQ) or K / V (dK, dV) of 256
-            # columns in shared memory and have room for 32-row partner tiles only
-            merged, g, kvb, qph, kph, M = _split_large_blocks(merged, N, g, kvb, qph, kph, 32)
-        do, sdo_b, sdo_n, sdo_h = _as_bnhd(grad_o.to(qq.dtype), False, H, D)
-        _, sq_b, sq_n, sq_h = _as_bnhd(qq, False, H, D)
-        _, sk_b, sk_n, sk_h = _as_bnhd(kk, False, Hkv, D)
-        _, sv_b, sv_n, sv_h = _as_bnhd(vv, False, Hkv, D)
-        QM, W = merged.shape[2], merged.shape[3]
-        status = status_word(dev)
-        st = stream_ptr(dev)
-        delta = torch.empty(B, H, N, dtype=torch.float32, device=dev)
-        dq = torch.empty(B, N, C, dtype=qq.dtype, device=dev)
-        dk = torch.empty(B, N, C, dtype=qq.dtype, device=dev)
-        dv = torch.empty(B, N, C, dtype=qq.dtype, device=dev)
-        dt = _lib.dtype_code(qq)
-        _call("ftk_sparse_bwd_dq", lib.ftk_sparse_bwd_dq, 
-            ptr(qq), ptr(kk), ptr(vv), ptr(o), ptr(do), dt, B, H, Hkv, N, D,
-            sq_b, sq_n, sq_h, sk_b, sk_n, sk_h, sv_b, sv_n, sv_h, N * C, C, D,
-            sdo_b, sdo_n, sdo_h, ptr(merged), QM, W, g, kvb, qph, kph, scale,
-            ptr(lse), ptr(delta), ptr(dq), N * C, C, D, ptr(status), st)
-        _count(2)
-        rev, rc, skv = flash_build_reverse_indices_cuda(merged, None, M)
-        _call("ftk_sparse_bwd_dkv", lib.ftk_sparse_bwd_dkv, 
-            ptr(qq), ptr(kk), ptr(vv), ptr(do), dt, B, H, Hkv, N, D,
-            sq_b, sq_n, sq_h, sk_b, sk_n, sk_h, sv_b, sv_n, sv_h, sdo_b, sdo_n, sdo_h,
-            ptr(rev), ptr(rc), ptr(skv), QM, M, g, kvb, qph, kph, scale,
-            ptr(lse), ptr(delta), ptr(dk), N * C, C, D, ptr(dv), N * C, C, D, W, ptr(status), st)
-        _count(1)
-        _after(dev)
-        if Hkv != H:
-            # the kernel wrote one dK / dV per query head: add up each group of
-            # H / Hkv heads (fp32) to get the gradient of their shared kv head
-            grp = H // Hkv
-            dk = dk.view(B, N, Hkv, grp, D).float().sum(3).to(qq.dtype).view(B, N, Hkv * D)
-            dv = dv.view(B, N, Hkv, grp, D).float().sum(3).to(qq.dtype).view(B, N, Hkv * D)
-        return dq, dk, dv, None, None, None, None, None, None, None, None, None
 
 
 def _check_backward_blocks(D, g, kvb):
@@ -612,7 +499,9 @@ def _split_large_blocks(merged, N, g, kvb, q_pad_head, kv_pad_head, limit=64):
     """Lists over blocks of more than `limit` rows (65..128 for the default),
     restated over half-size blocks, repeatedly if need be.
 
-    The kernels work on q / kv blocks of at most 64 rows.  A block of `kvb` rows
+    The kernels work on q / kv blocks of at most 64 rows and read longer blocks'
+    lists in place by this rule (csrc/attn_host.cuh); this function writes the
+    restated lists out.  A block of `kvb` rows
     that starts at token j*kvb - pad is exactly the two half blocks
     2j - s, 2j - s + 1 of a grid with block kvb/2 and pad head pad - s*kvb/2,
     where s = 1 when the pad head covers the first half block; each listed id
@@ -659,8 +548,8 @@ def flash_sparse_attn(q, k, v, merged_indices, num_heads, q_block_size, kv_block
         raise ValueError("flash_sparse_attn requires CUDA tensors")
     if q.dtype not in (torch.float16, torch.bfloat16, torch.float32):
         raise ValueError("q must be float16, bfloat16, or float32")
-    orig_dtype = q.dtype
-    if orig_dtype == torch.float32:
+    mixed = q.dtype == torch.float32 and not (k.dtype == v.dtype == torch.float32)
+    if mixed:
         q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
     B, N, C = q.shape
     H = num_heads
@@ -719,24 +608,11 @@ def flash_sparse_attn(q, k, v, merged_indices, num_heads, q_block_size, kv_block
         raise ValueError(f"D ({D}) must be <= 256")
     if scale is None:
         scale = 1.0 / math.sqrt(D)
-    Dk = _kernel_head_dim(D)
-    if Dk != D:
-        q = _pad_head_dim(q, False, H, D, Dk)
-        k = _pad_head_dim(k, False, Hkv, D, Dk)
-        v = _pad_head_dim(v, False, Hkv, D, Dk)
-    num_kv_blocks = n_kv // kv_block_size
-    if q_block_size > 64 or kv_block_size > 64:
-        (merged_indices, q_block_size, kv_block_size, q_pad_head, kv_pad_head,
-         num_kv_blocks) = _split_large_blocks(
-            merged_indices, N, q_block_size, kv_block_size, q_pad_head, kv_pad_head)
     if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
         # say so now rather than inside backward()
-        _check_backward_blocks(Dk, q_block_size, kv_block_size)
-    o, lse = FlashSparseAttnFunc.apply(
-        q, k, v, merged_indices, H, q_block_size, kv_block_size, scale, q_pad_head, kv_pad_head,
-        num_kv_blocks, Hkv)
-    if Dk != D:
-        o = o.view(B, N, H, Dk)[..., :D].reshape(B, N, C)
-    if orig_dtype == torch.float32:
-        o = o.float()
-    return o, lse
+        _check_backward_blocks(D, q_block_size, kv_block_size)
+    o, lse = native.sparse_attn(q, k, v, merged_indices, H, Hkv, q_block_size, kv_block_size,
+                                q_pad_head, kv_pad_head, scale)
+    if _DEBUG:
+        _after(o.device)
+    return (o.float() if mixed else o), lse

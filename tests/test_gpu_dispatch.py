@@ -1,0 +1,143 @@
+"""Branches that a size rule chooses: each at the sizes where it can go wrong,
+against the oracle or against the other branch on the same inputs."""
+
+import numpy as np
+import pytest
+import torch
+
+import cases
+from oracle import ftk_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ftk():
+    import flash_topk_attn_v2 as m
+    return m
+
+
+def _lists(rng, heads, QM, M, W):
+    """Random lists with empty rows and -1 tails."""
+    out = np.full((heads, QM, W), -1, dtype=np.int32)
+    for h in range(heads):
+        for m in range(QM):
+            n = int(rng.integers(0, min(W, M) + 1))
+            out[h, m, :n] = rng.permutation(M)[:n]
+    return out
+
+
+def _grads(ftk, t, merged, H, g, kvb, **kw):
+    q, k, v = (t[n].cuda().requires_grad_(True) for n in "qkv")
+    o, lse = ftk.flash_topk_attn(q, k, v, torch.from_numpy(merged).cuda(), None, H, g, kvb, **kw)
+    dq, dk, dv = torch.autograd.grad(o, (q, k, v), t["do"].cuda())
+    ftk.check_errors()
+    return o.detach(), lse, dq, dk, dv
+
+
+@pytest.mark.parametrize("N,D,bsz,pad", [
+    (512, 64, 64, (0, 0)),       # four key tiles
+    (600, 128, 64, (20, 20)),    # five: the two accumulators take turns unevenly
+    (768, 128, 256, (0, 0)),     # score blocks of two tiles: one group drains them all
+    (640, 256, 128, (0, 0)),     # head dim in two slices
+])
+def test_score_overflow_is_redone_by_the_cta_that_saw_it(ftk, N, D, bsz, pad):
+    """Logits far above the first key tile's in the query rows of one CTA only:
+    that CTA walks the keys again (exact maximum, then sums), the others do not.
+    Bound as for the exact oracle comparison of overflowing rows: fp32 logits of a
+    few thousand carry 2^-24 relative error, 2e-4 in the exponential."""
+    gen = torch.Generator().manual_seed(7)
+    q = torch.randn(1, N, D, generator=gen)
+    k = torch.randn(1, N, D, generator=gen)
+    k[:, 300:] *= 40.0
+    q[:, :256] *= 3.0
+    q[:, 256:] *= 0.02
+    qh, kh = q.half(), k.half()
+    want = orc.block_score(qh.float().numpy(), kh.float().numpy(), 1, bsz, pad)
+    got = ftk.flash_block_score(qh.cuda(), kh.cuda(), 1, bsz, pad).cpu().numpy()
+    ftk.check_errors()
+    assert np.isfinite(got).all()
+    np.testing.assert_allclose(got, want, rtol=2e-4, atol=1e-7)
+
+
+@pytest.mark.parametrize("D,g", [(128, 64), (64, 32)])
+def test_redo_of_more_tiles_than_ctas(ftk, monkeypatch, D, g):
+    """Every tile of the pipelined forward leaves the safe exponent range: the redo
+    kernel's CTAs (one per SM) do more than one tile each, bit for bit as the
+    exact kernel alone."""
+    H, N, kvb = 80, 512, 64
+    t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype="fp16", seed=21, do_seed=22))
+    t["k"][:, 256:] *= 4.0
+    t["q"] *= 2.0
+    merged = np.tile(np.arange(8, dtype=np.int32), (1, H, N // g, 1))
+    merged[0, 1] = -1
+    args = (t["q"].cuda(), t["k"].cuda(), t["v"].cuda(), torch.from_numpy(merged).cuda(), None, H, g,
+            kvb)
+    o, lse = ftk.flash_topk_attn(*args)
+    monkeypatch.setenv("FTK_FWD_PIPE", "0")
+    o2, lse2 = ftk.flash_topk_attn(*args)
+    ftk.check_errors()
+    flagged = torch.ones(H, dtype=torch.bool, device="cuda")
+    flagged[1] = False
+    a, b = (x.view(N, H, D)[:, flagged] for x in (o, o2))
+    assert torch.equal(a, b) and torch.equal(lse[0][flagged], lse2[0][flagged])
+    assert not o.view(N, H, D)[:, 1].any() and torch.isinf(lse[0, 1]).all()
+
+
+@pytest.mark.parametrize("B,N,H,Hkv,D,g,kvb,dtype,f32", [
+    (2, 4736, 4, 2, 128, 64, 64, "bf16", False),   # 148 kv tiles: heads walked, pairs of SMs
+    (2, 4700, 4, 2, 64, 64, 64, "fp16", False),    # the same in one-CTA kernels, ragged
+    (1, 4736, 16, 4, 128, 64, 32, "bf16", True),   # four heads, float32 results
+    (1, 300, 6, 2, 128, 64, 64, "bf16", False),    # few tiles: one result per head, summed after
+    (1, 300, 6, 2, 96, 32, 64, "bf16", True),
+])
+def test_grouped_heads_sum(ftk, B, N, H, Hkv, D, g, kvb, dtype, f32):
+    """dK / dV of grouped kv heads against the same call with K / V repeated per
+    query head, its dK / dV added up per group.  Either side rounds: the walk
+    rounds the sum once, the other path each head's share and the sum, so the two
+    differ by at most half an ulp of every share plus one ulp of the sum (eps / 2
+    and eps relative, eps = 2^-7 or 2^-10), and by fp32 noise."""
+    grp = H // Hkv
+    tail_q, tail_k = -N % g, -N % kvb
+    t = cases.make_inputs(dict(B=B, N=N, H=H, D=D, dtype=dtype, seed=5, do_seed=6))
+    for n in "kv":
+        t[n] = t[n].view(B, N, Hkv, grp, D)[:, :, :, 0].reshape(B, N, Hkv * D).clone()
+    if f32:
+        t = {n: x.float() for n, x in t.items()}
+    QM, M = (N + tail_q) // g, (N + tail_k) // kvb
+    W = M if N < 1000 else 6
+    merged = _lists(np.random.default_rng(3), B * H, QM, M, W).reshape(B, H, QM, W)
+    kw = dict(q_padding=(0, tail_q), kv_padding=(0, tail_k))
+    got = _grads(ftk, t, merged, H, g, kvb, num_kv_heads=Hkv, **kw)
+    rep = dict(t)
+    for n in "kv":
+        rep[n] = t[n].view(B, N, Hkv, 1, D).expand(B, N, Hkv, grp, D).reshape(B, N, H * D)
+    want = _grads(ftk, rep, merged, H, g, kvb, **kw)
+    for i in range(3):
+        assert torch.equal(got[i], want[i])
+    eps = 2.0 ** -10 if dtype == "fp16" else 2.0 ** -7
+    for i in (3, 4):
+        assert got[i].dtype == (torch.float32 if f32 else want[i].dtype)
+        share = want[i].double().view(B, N, Hkv, grp, D)
+        total = share.sum(3).reshape(B, N, Hkv * D)
+        slack = (0.5 * eps * share.abs().sum(3).reshape(B, N, Hkv * D) + eps * total.abs() + 1e-6)
+        assert ((got[i].double() - total).abs() <= slack).all()
+
+
+@pytest.mark.parametrize("H,D,g,kvb", [(16, 64, 64, 64), (16, 64, 32, 16), (8, 128, 32, 32)])
+def test_dkv_tile_order(ftk, monkeypatch, H, D, g, kvb):
+    """Several waves of dK / dV tiles are sorted by the work they have; the order
+    decides when a tile runs, never what it computes."""
+    B, N = 2, 2500
+    tail_q, tail_k = -N % g, -N % kvb
+    t = cases.make_inputs(dict(B=B, N=N, H=H, D=D, dtype="bf16", seed=8, do_seed=9))
+    QM, M = (N + tail_q) // g, (N + tail_k) // kvb
+    merged = _lists(np.random.default_rng(4), B * H, QM, M, 6).reshape(B, H, QM, 6)
+    merged[:, :, :, 0] = M - 1          # one kv block that everybody reads
+    merged[:, :, :, 1:] = np.where(merged[:, :, :, 1:] == M - 1, -1, merged[:, :, :, 1:])
+    kw = dict(q_padding=(0, tail_q), kv_padding=(0, tail_k))
+    sorted_ = _grads(ftk, t, merged, H, g, kvb, **kw)
+    monkeypatch.setenv("FTK_DKV_ORDER", "0")
+    plain = _grads(ftk, t, merged, H, g, kvb, **kw)
+    for a, b in zip(sorted_, plain):
+        assert torch.equal(a, b)
