@@ -976,6 +976,7 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
 
 #include "sparse_bwd_dkv2.cuh"
 #include "sparse_bwd_dq2.cuh"
+#include "sparse_bwd_d256.cuh"
 
 namespace ftk {
 
@@ -1098,9 +1099,12 @@ static size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
 static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
   BwdPlan b{};
-  // head dim 256: the kernels hold Q / dO (dQ) or K / V (dK, dV) of 256 columns in
-  // shared memory and have room for 32-row partner tiles only
-  if (int e = attn_grid(a, a.D > 128 ? 32 : 64, &b.gr)) return e;
+  int e = attn_grid(a, 64, &b.gr);
+  // head dim 256 with blocks other than 64 rows: the one-CTA kernels hold Q / dO (dQ)
+  // or K / V (dK, dV) of 256 columns in shared memory and have room for 32-row partner
+  // tiles only
+  if (a.D > 128 && (e || b.gr.g != 64 || b.gr.kvb != 64)) e = attn_grid(a, 32, &b.gr);
+  if (e) return e;
   const AttnGrid& gr = b.gr;
   if (gr.g % 16 != 0) return FTK_ERR_UNSUPPORTED;
   if (gr.QM > AT_MAX_BLOCKS) return FTK_ERR_UNSUPPORTED;
@@ -1112,7 +1116,9 @@ static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
   b.kv_tiles = (gr.Mkv + G - 1) / G;
   // Pairs walk the union of four lists: only when the lists can cover a good part
   // of the blocks (see ftk_attn_fwd)
-  b.pair = gr.kd == 128 && gr.g == 64 && gr.kvb == 64 && 4 * gr.width >= gr.Mkv;
+  // at head dim 128; at 256 the pair kernels are several times the faster per tile.
+  b.pair = gr.g == 64 && gr.kvb == 64 &&
+           (gr.kd == 256 || (gr.kd == 128 && 4 * gr.width >= gr.Mkv));
   // Query heads that share a kv head: walked one after the other by the CTA that
   // owns the kv rows, so that their sum stays in its fp32 accumulators, unless
   // that leaves SMs idle: waves of CTAs times heads per CTA against waves of one
@@ -1192,19 +1198,24 @@ static int launch_dq(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, b
   if ((e = tmap_of(&tq, a, q, 128)) || (e = tmap_of(&tdo, a, dout, 128)) ||
       (e = tmap_of(&tk, a, k, p.kvb)))
     return e;
-  if (pair && !env_off("FTK_DQ_2CTA")) {
+  if (pair && (kd == 256 || !env_off("FTK_DQ_2CTA"))) {
     CUtensorMap tk32, tv32;
     if ((e = tmap_of(&tk32, a, k, 32)) || (e = tmap_of(&tv32, a, v, 32))) return e;
-    const size_t smem = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DQ2_STAGES) * 24576;
     const dim3 grid(2 * ((p.QM + 3) / 4), bh);
-    if (a.dtype == FTK_DTYPE_BF16) {
-      if ((e = allow_smem<sparse_bwd_dq2_kernel<1>>(smem))) return e;
-      return launch_pdl(sparse_bwd_dq2_kernel<1>, grid, BW_THREADS, smem, st, tq, tdo, tk, tk32,
-                        tv32, p);
+    auto go = [&](auto kernel_tag, size_t smem) -> int {
+      constexpr auto kernel = decltype(kernel_tag)::kernel;
+      if (int r = allow_smem<kernel>(smem)) return r;
+      return launch_pdl(kernel, grid, BW_THREADS, smem, st, tq, tdo, tk, tk32, tv32, p);
+    };
+    const bool bf = a.dtype == FTK_DTYPE_BF16;
+    if (kd == 256) {
+      const size_t smem = 1024 + 2 * B6_ROWS + static_cast<size_t>(DQ6_SLOTS) * B6_PIECE;
+      return bf ? go(Kernel<sparse_bwd_dq256_kernel<1>>{}, smem)
+                : go(Kernel<sparse_bwd_dq256_kernel<0>>{}, smem);
     }
-    if ((e = allow_smem<sparse_bwd_dq2_kernel<0>>(smem))) return e;
-    return launch_pdl(sparse_bwd_dq2_kernel<0>, grid, BW_THREADS, smem, st, tq, tdo, tk, tk32, tv32,
-                      p);
+    const size_t smem = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DQ2_STAGES) * 24576;
+    return bf ? go(Kernel<sparse_bwd_dq2_kernel<1>>{}, smem)
+              : go(Kernel<sparse_bwd_dq2_kernel<0>>{}, smem);
   }
   if ((e = tmap_of(&tv, a, v, p.kvb))) return e;
   const int nch = kd / 64;
@@ -1238,21 +1249,38 @@ static int launch_dkv(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, 
   if ((e = tmap_of(&tq, a, q, p.g)) || (e = tmap_of(&tdo, a, dout, p.g)) ||
       (e = tmap_of(&tk, a, k, 128)) || (e = tmap_of(&tv, a, v, 128)))
     return e;
-  if (pair && !env_off("FTK_DKV_2CTA")) {
+  if (pair && (kd == 256 || !env_off("FTK_DKV_2CTA"))) {
     CUtensorMap tq32, tdo32;
     if ((e = tmap_of(&tq32, a, q, 32)) || (e = tmap_of(&tdo32, a, dout, 32))) return e;
-    const size_t smem = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DK2_STAGES) * 32768;
     const dim3 grid(2 * ((p.Mkv + 3) / 4), slices);
-    auto go = [&](auto kernel_tag) -> int {
+    auto go = [&](auto kernel_tag, size_t smem) -> int {
       constexpr auto kernel = decltype(kernel_tag)::kernel;
       if (int r = allow_smem<kernel>(smem)) return r;
       return launch_pdl(kernel, grid, BW_THREADS, smem, st, tq, tdo, tq32, tdo32, tk, tv, p);
     };
-    if (a.dtype == FTK_DTYPE_BF16)
-      return p.heads > 1 ? go(Kernel<sparse_bwd_dkv2_kernel<1, true>>{})
-                         : go(Kernel<sparse_bwd_dkv2_kernel<1, false>>{});
-    return p.heads > 1 ? go(Kernel<sparse_bwd_dkv2_kernel<0, true>>{})
-                       : go(Kernel<sparse_bwd_dkv2_kernel<0, false>>{});
+    const bool bf = a.dtype == FTK_DTYPE_BF16, walk = p.heads > 1;
+    if (kd == 256) {
+      const size_t smem_dv = 1024 + B6_ROWS + static_cast<size_t>(DV6_SLOTS) * B6_PIECE,
+                   smem_dk = 1024 + 2 * B6_ROWS + static_cast<size_t>(DQ6_SLOTS) * B6_PIECE;
+      if (bf) {
+        e = walk ? go(Kernel<sparse_bwd_dkv256_kernel<1, 1, true>>{}, smem_dv)
+                 : go(Kernel<sparse_bwd_dkv256_kernel<1, 1, false>>{}, smem_dv);
+        if (e) return e;
+        return walk ? go(Kernel<sparse_bwd_dkv256_kernel<1, 2, true>>{}, smem_dk)
+                    : go(Kernel<sparse_bwd_dkv256_kernel<1, 2, false>>{}, smem_dk);
+      }
+      e = walk ? go(Kernel<sparse_bwd_dkv256_kernel<0, 1, true>>{}, smem_dv)
+               : go(Kernel<sparse_bwd_dkv256_kernel<0, 1, false>>{}, smem_dv);
+      if (e) return e;
+      return walk ? go(Kernel<sparse_bwd_dkv256_kernel<0, 2, true>>{}, smem_dk)
+                  : go(Kernel<sparse_bwd_dkv256_kernel<0, 2, false>>{}, smem_dk);
+    }
+    const size_t smem = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DK2_STAGES) * 32768;
+    if (bf)
+      return walk ? go(Kernel<sparse_bwd_dkv2_kernel<1, true>>{}, smem)
+                  : go(Kernel<sparse_bwd_dkv2_kernel<1, false>>{}, smem);
+    return walk ? go(Kernel<sparse_bwd_dkv2_kernel<0, true>>{}, smem)
+                : go(Kernel<sparse_bwd_dkv2_kernel<0, false>>{}, smem);
   }
   const int nch = kd / 64;
   const int stage_bytes = 2 * nch * p.g * 128;

@@ -1,0 +1,779 @@
+// Backward at head dim 256 on pairs of SMs (tcgen05 cta_group::2), for 64-row q
+// and kv blocks.  Included by sparse_bwd.cu after sparse_bwd_dq2.cuh.
+//
+// The scheme is that of the head-dim-128 pair kernels: a cluster of two CTAs owns
+// 256 rows, both walk the union of the pair's four lists, each CTA loads its half
+// of every B operand, CTA 0 issues every UMMA.  What 256 columns change:
+//   - the row operands (Q and dO, or K and V: 64 KB each) stay in shared memory;
+//     an M = 256 UMMA with both operands there costs the same 43 cycles at N = 64;
+//   - a 256-column accumulator leaves 256 TMEM columns for the tiles in flight:
+//     dK and dV cannot both be there, so they are two launches, dV with four
+//     S^T buffers (like the forward), dK with two S^T and two dP^T buffers (like dQ);
+//   - what is left of shared memory is one ring of 16 KB pieces (32 rows x 256 d
+//     or 64 rows x 128 d) that every operand goes through in the order in which
+//     the UMMAs read it; a piece is handed back as soon as its UMMAs retire.
+// Tensor time per 256 x 64 tile: dQ 16 x 43 x 2 + 4 x 128 = 1890 cycles, dV 1200,
+// dK 1890.  The one-CTA kernels that this replaces for 64-row blocks had to work on
+// 32-row tiles: 2.40 ms (dQ) and 1.76 + 3.73 ms (dV, dK) at N = 8192, H = 16.
+#pragma once
+
+namespace ftk {
+
+constexpr int B6_PIECE = 16384;
+constexpr int B6_ROWS = 4 * 128 * 128;   // a 128-row operand of 256 columns
+constexpr int DQ6_SLOTS = 5;             // behind two row operands
+constexpr int DV6_SLOTS = 8;             // behind one
+
+// Position in the ring of pieces
+template <int SLOTS>
+struct PieceWalk {
+  int slot = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void next() {
+    if (++slot == SLOTS) {
+      slot = 0;
+      phase ^= 1;
+    }
+  }
+};
+
+// The order of the pieces of a kernel with `ahead` tiles in flight: the operands
+// of tiles 0 .. ahead - 1's first step, then per tile i the operand of its second
+// step and the first step's of tile i + ahead.
+template <typename First, typename Second>
+__device__ __forceinline__ void in_piece_order(int n, int ahead, First&& first, Second&& second) {
+  for (int i = 0; i < ahead && i < n; i++)
+    if (!first(i)) return;
+  for (int i = 0; i < n; i++) {
+    if (!second(i)) return;
+    if (i + ahead < n && !first(i + ahead)) return;
+  }
+}
+
+template <int FMT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(BW_THREADS, 1)
+sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
+                        const __grid_constant__ CUtensorMap tm_do,
+                        const __grid_constant__ CUtensorMap tm_k,
+                        const __grid_constant__ CUtensorMap tm_k32,
+                        const __grid_constant__ CUtensorMap tm_v32, const BwdParams p) {
+  constexpr int D = 256, NCH = 4, G = 64, SLOTS = DQ6_SLOTS;
+  constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DQ = 256;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  uint8_t* sQ = smem;
+  uint8_t* sDO = smem + B6_ROWS;
+  uint8_t* sRing = smem + 2 * B6_ROWS;
+  __shared__ UnionScratch un;
+  __shared__ float s_delta[128];
+  __shared__ __align__(8) uint64_t bars[2 + 3 * SLOTS + 5];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int abort_flag;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int m0 = (blockIdx.x >> 1) * 4;       // first of the pair's four q-blocks
+  const int bh = blockIdx.y;
+  const int b_idx = bh / p.H, h_idx = bh - b_idx * p.H;
+  const int groups = min(4, p.QM - m0);
+  const int tile_row0 = (m0 + 2 * static_cast<int>(rank)) * G - p.q_pad_head;   // my 128 rows
+
+  const uint32_t bar_q = smem_u32(&bars[0]);         // my Q / dO tiles
+  const uint32_t bar_peer_q = smem_u32(&bars[1]);    // CTA 0: CTA 1's
+  auto bar_full = [&](int s) { return smem_u32(&bars[2 + s]); };
+  auto bar_empty = [&](int s) { return smem_u32(&bars[2 + SLOTS + s]); };
+  auto bar_peer = [&](int s) { return smem_u32(&bars[2 + 2 * SLOTS + s]); };   // CTA 0 only
+  constexpr int BAR_A0 = 2 + 3 * SLOTS;
+  auto bar_afull = [&](int s) { return smem_u32(&bars[BAR_A0 + s]); };
+  auto bar_dsfull = [&](int s) { return smem_u32(&bars[BAR_A0 + 2 + s]); };    // CTA 0 only
+  const uint32_t bar_final = smem_u32(&bars[BAR_A0 + 4]);
+
+  if (tid == 0) {
+    abort_flag = 0;
+    mbar_init(bar_q, 1);
+    mbar_init(bar_peer_q, 1);
+    for (int s = 0; s < SLOTS; s++) {
+      mbar_init(bar_full(s), 1);
+      mbar_init(bar_empty(s), 1);
+      mbar_init(bar_peer(s), 1);
+    }
+    for (int s = 0; s < 2; s++) {
+      mbar_init(bar_afull(s), 1);
+      mbar_init(bar_dsfull(s), 16);   // 8 warps of the owning group in each CTA
+    }
+    mbar_init(bar_final, 1);
+    mbar_init_fence();
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_do);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_k32);
+    tma_prefetch_desc(&tm_v32);
+  }
+  if (warp == 0) {
+    tmem_alloc2(smem_u32(&tmem_base_s), 512);
+    tmem_relinquish2();
+  }
+  clear_bitmaps(un);
+  pdl_wait();
+  pdl_launch();
+  const int mine = min(2, groups - 2 * static_cast<int>(rank));   // q-blocks of my tile, if any
+  tile_delta<D>(p, s_delta, bh, b_idx, h_idx, tile_row0, mine * G);
+  const int n = build_union(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
+                            p.W, nullptr, p.Mkv, p.lm, p.status);
+  if (p.masks && mine > 0)
+    write_tile_masks(un,
+                     p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + m0 / 2 + rank) *
+                                   p.mask_stride,
+                     p.mask_stride, 2 * static_cast<int>(rank), mine);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();        // barriers of both CTAs are initialised before anyone signals them
+  tc_fence_after();
+  const uint32_t tmem = tmem_base_s;
+  WaitCtx w{&abort_flag, p.status};
+
+  if (warp == 0) {
+    // ------------------------------------------------------- TMA producer
+    if (lane == 0 && n > 0) {
+      mbar_expect_tx(bar_q, 2 * B6_ROWS);
+      for (int c = 0; c < NCH; c++) {
+        tma_load_4d(smem_u32(sQ) + c * 128 * 128, &tm_q, bar_q, c * 64, h_idx, tile_row0, b_idx);
+        tma_load_4d(smem_u32(sDO) + c * 128 * 128, &tm_do, bar_q, c * 64, h_idx, tile_row0, b_idx);
+      }
+      const int dcol = 128 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
+      const int hk = h_idx / p.kv_hdiv;
+      PieceWalk<SLOTS> at;
+      auto piece = [&]() -> uint32_t {   // next free slot, 0 after a failed wait
+        if (!mbar_wait(bar_empty(at.slot), at.phase ^ 1, w, FTK_DEV_TIMEOUT_TMA)) return 0;
+        mbar_expect_tx(bar_full(at.slot), B6_PIECE);
+        return smem_u32(sRing) + at.slot * B6_PIECE;
+      };
+      auto tok0 = [&](int i) { return static_cast<int>(un.ids[i]) * G - p.kv_pad_head; };
+      in_piece_order(
+          n, 2,
+          [&](int i) {
+            for (int kv = 0; kv < 2; kv++) {
+              const uint32_t dst = piece();
+              if (!dst) return false;
+              for (int c = 0; c < NCH; c++)
+                tma_load_4d(dst + c * 4096, kv ? &tm_v32 : &tm_k32, bar_full(at.slot), c * 64, hk,
+                            tok0(i) + rsub, b_idx);
+              at.next();
+            }
+            return true;
+          },
+          [&](int i) {
+            const uint32_t dst = piece();
+            if (!dst) return false;
+            for (int c = 0; c < 2; c++)
+              tma_load_4d(dst + c * 8192, &tm_k, bar_full(at.slot), dcol + c * 64, hk, tok0(i), b_idx);
+            at.next();
+            return true;
+          });
+    }
+  } else if (warp == 1 && rank == 1) {
+    // ----------------------- CTA 1: tell CTA 0 when my tiles have landed
+    if (n > 0) {
+      bool ok = mbar_wait(bar_q, 0, w, FTK_DEV_TIMEOUT_MMA);
+      __syncwarp();
+      if (ok && lane == 0) mbar_arrive_cta(bar_peer_q, 0);
+      PieceWalk<SLOTS> at;
+      for (int u = 0; ok && u < 3 * n; u++) {
+        ok = mbar_wait(bar_full(at.slot), at.phase, w, FTK_DEV_TIMEOUT_MMA);
+        __syncwarp();
+        if (ok && lane == 0) mbar_arrive_cta(bar_peer(at.slot), 0);
+        at.next();
+      }
+    }
+  } else if (warp == 1) {
+    // ----------------------------- CTA 0: UMMA issuer for the CTA pair
+    if (n > 0) {
+      const uint32_t idesc_a = umma_idesc(256, G, FMT, 0, 0);
+      const uint32_t idesc_b = umma_idesc(256, D, FMT, 0, 1);
+      const uint64_t qdesc0 = smem_desc_sw128(smem_u32(sQ), 16, 1024);
+      const uint64_t dodesc0 = smem_desc_sw128(smem_u32(sDO), 16, 1024);
+      const uint64_t rowdesc0 = smem_desc_sw128(smem_u32(sRing), 16, 1024);
+      const uint64_t coldesc0 = smem_desc_sw128(smem_u32(sRing), 8192, 1024);
+      const uint32_t qb[2] = {bar_q, bar_peer_q};
+      const uint32_t qp[2] = {0u, 0u};
+      bool ok = mbar_wait_all<2>(qb, qp, w, FTK_DEV_TIMEOUT_MMA);
+      PieceWalk<SLOTS> at;
+      // S and dP of a tile: pieces `k` and `v` (elected lane only)
+      auto mma_a = [&](int i, int k, int v) {
+        const uint64_t kdesc = desc_advance(rowdesc0, k * B6_PIECE);
+        const uint64_t vdesc = desc_advance(rowdesc0, v * B6_PIECE);
+        const uint32_t sb = i & 1;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ks++)
+          umma2_ss(tmem + COL_S + sb * 64,
+                   desc_advance(qdesc0, (ks / 4) * 128 * 128 + (ks % 4) * 32),
+                   desc_advance(kdesc, (ks / 4) * 4096 + (ks % 4) * 32), idesc_a, ks > 0);
+        umma2_commit(bar_empty(k), 3);
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ks++)
+          umma2_ss(tmem + COL_DP + sb * 64,
+                   desc_advance(dodesc0, (ks / 4) * 128 * 128 + (ks % 4) * 32),
+                   desc_advance(vdesc, (ks / 4) * 4096 + (ks % 4) * 32), idesc_a, ks > 0);
+        umma2_commit(bar_afull(sb), 3);
+        umma2_commit(bar_empty(v), 3);
+      };
+      for (int i = 0; ok && i < 2 && i < n; i++) {
+        const PieceWalk<SLOTS> k = at;
+        at.next();
+        const PieceWalk<SLOTS> v = at;
+        at.next();
+        const uint32_t wb[4] = {bar_full(k.slot), bar_peer(k.slot), bar_full(v.slot),
+                                bar_peer(v.slot)};
+        const uint32_t wp[4] = {k.phase, k.phase, v.phase, v.phase};
+        ok = mbar_wait_all<4>(wb, wp, w, FTK_DEV_TIMEOUT_MMA);
+        tc_fence_after();
+        if (ok && elect_one()) mma_a(i, k.slot, v.slot);
+        __syncwarp();
+      }
+      for (int i = 0; ok && i < n; i++) {
+        const bool more = i + 2 < n;
+        const PieceWalk<SLOTS> kc = at;
+        at.next();
+        PieceWalk<SLOTS> k = kc, v = kc;
+        if (more) {
+          k = at;
+          at.next();
+          v = at;
+          at.next();
+        }
+        const uint32_t wb[7] = {bar_dsfull(i & 1),  bar_full(kc.slot), bar_peer(kc.slot),
+                                bar_full(k.slot),   bar_peer(k.slot),  bar_full(v.slot),
+                                bar_peer(v.slot)};
+        const uint32_t wp[7] = {static_cast<uint32_t>((i >> 1) & 1), kc.phase, kc.phase, k.phase,
+                                k.phase, v.phase, v.phase};
+        if (!mbar_wait_all<7>(wb, wp, w, FTK_DEV_TIMEOUT_MMA)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        if (elect_one()) {
+          const uint64_t kcol = desc_advance(coldesc0, kc.slot * B6_PIECE);
+#pragma unroll
+          for (int ks = 0; ks < 4; ks++)
+            umma2_ts(tmem + COL_DQ, tmem + COL_DP + (i & 1) * 64 + (ks >> 1) * 32 + (ks & 1) * 8,
+                     desc_advance(kcol, ks * 2048), idesc_b, (i > 0) || (ks > 0));
+          umma2_commit(bar_empty(kc.slot), 3);
+          if (more) mma_a(i + 2, k.slot, v.slot);
+        }
+        __syncwarp();
+      }
+      if (elect_one()) umma2_commit(bar_final, 3);
+      __syncwarp();
+    }
+  } else if (warp >= 2) {
+    // as in sparse_bwd_dq2_kernel: group w drains the buffers of tiles i = w (mod 2),
+    // two warps share each 32-row lane quarter and take one half of the kv columns each
+    const int cw = warp - 2;
+    const int wg = cw >> 3;
+    const int colhalf = (cw >> 2) & 1;
+    const int quarter = warp & 3;
+    const int r = quarter * 32 + lane;
+    const int grp = 2 * static_cast<int>(rank) + r / G;   // q-block of the pair
+    const int qrow = tile_row0 + r;
+    const bool row_valid = (grp < groups) && qrow >= 0 && qrow < p.N;
+    const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t s_addr = lane_addr + COL_S + wg * 64;
+    const uint32_t dp_addr = lane_addr + COL_DP + wg * 64;
+    const int cbeg = colhalf * 32;
+    const float c = p.scale_log2;
+    float lse2 = 0.f, dl = 0.f;
+    if (row_valid) {
+      lse2 = p.lse[static_cast<int64_t>(bh) * p.N + qrow] * 1.4426950408889634f;
+      dl = s_delta[r];
+    }
+    bool ok = true;
+    for (int i = wg; ok && i < n; i += 2) {
+      if (!mbar_wait(bar_afull(wg), (i >> 1) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      const int tok0 = static_cast<int>(un.ids[i]) * G - p.kv_pad_head;
+      const int lo = max(0, -tok0), hi = min(G, p.N - tok0);
+      const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
+      const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
+      const bool none = !fast && !__any_sync(0xffffffffu, act);
+      uint32_t sv[32], dv[32], pk[16];
+      if (!none) {
+        tmem_ld32(s_addr + cbeg, sv);
+        tmem_ld32(dp_addr + cbeg, dv);
+        tmem_wait_ld();
+      }
+      if (none) {
+#pragma unroll
+        for (int x = 0; x < 16; x++) pk[x] = 0u;
+      } else if (fast) {
+        ds_pairs<FMT>(sv, dv, pk, c, -lse2, -dl);
+      } else {
+#pragma unroll
+        for (int x = 0; x < 32; x += 2) {
+          float d0 = 0.f, d1 = 0.f;
+          if (act && cbeg + x >= lo && cbeg + x < hi)
+            d0 = fast_exp2(fmaf(__uint_as_float(sv[x]), c, -lse2)) * (__uint_as_float(dv[x]) - dl);
+          if (act && cbeg + x + 1 >= lo && cbeg + x + 1 < hi)
+            d1 = fast_exp2(fmaf(__uint_as_float(sv[x + 1]), c, -lse2)) *
+                 (__uint_as_float(dv[x + 1]) - dl);
+          pk[x >> 1] = pack2f<FMT>(d0, d1);
+        }
+      }
+      tmem_st16(dp_addr + cbeg, pk);   // over the dP columns this thread has read
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cta(bar_dsfull(wg), 0);
+    }
+    if (ok && n > 0) ok = mbar_wait(bar_final, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
+    if (ok) {
+      tc_fence_after();
+      uint8_t* orow = nullptr;
+      if (row_valid)
+        orow = static_cast<uint8_t*>(p.out0) +
+               (p.out_f32 ? 4 : 2) *
+                   (static_cast<int64_t>(b_idx) * p.s0_b + static_cast<int64_t>(qrow) * p.s0_n +
+                    static_cast<int64_t>(h_idx) * p.s0_h);
+      for (int c0 = (wg * 2 + colhalf) * 32; c0 < D; c0 += 128) {
+        uint32_t v[32];
+        if (n > 0) {
+          tmem_ld32(lane_addr + COL_DQ + c0, v);
+          tmem_wait_ld();
+        }
+        if (row_valid) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int x = 0; x < 32; x += 2) {
+            const float a = n > 0 ? __uint_as_float(v[x]) * p.scale : 0.f;
+            const float b = n > 0 ? __uint_as_float(v[x + 1]) * p.scale : 0.f;
+            pk[x >> 1] = pack2f<FMT>(a, b);
+          }
+          store_row_part(orow, c0, p.D, pk, FMT, p.out_f32 != 0);
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (abort_flag)
+    for (int i = 0; i < 200; i++) __nanosleep(1000);
+  // neither CTA may leave (or free TMEM) while the other can still touch it
+  cluster_sync_all();
+  if (warp == 0) tmem_dealloc2(tmem, 512);
+}
+
+// MODE 1 = dV (K resident), MODE 2 = dK (K and V resident); WALK as in
+// sparse_bwd_dkv2_kernel.  TMEM: MODE 1 S^T[4] 0/64/128/192, MODE 2 S^T[2] 0/64,
+// dP^T[2] 128/192; accumulator 256..511.
+template <int FMT, int MODE, bool WALK>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(BW_THREADS, 1)
+sparse_bwd_dkv256_kernel(const __grid_constant__ CUtensorMap tm_q,
+                         const __grid_constant__ CUtensorMap tm_do,
+                         const __grid_constant__ CUtensorMap tm_q32,
+                         const __grid_constant__ CUtensorMap tm_do32,
+                         const __grid_constant__ CUtensorMap tm_k,
+                         const __grid_constant__ CUtensorMap tm_v, const BwdParams p) {
+  constexpr int D = 256, NCH = 4, G = 64;
+  constexpr int SLOTS = MODE == 1 ? DV6_SLOTS : DQ6_SLOTS;
+  constexpr int AHEAD = MODE == 1 ? 4 : 2;       // tiles in flight = S^T buffers
+  constexpr int FIRST = MODE == 1 ? 1 : 2;       // pieces of a tile's first step
+  constexpr uint32_t COL_DP = 128, COL_OUT = 256;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  uint8_t* sK = smem;
+  uint8_t* sV = smem + B6_ROWS;
+  uint8_t* sRing = smem + FIRST * B6_ROWS;
+  __shared__ UnionScratch un;
+  __shared__ __align__(8) uint64_t bars[2 + 3 * SLOTS + 2 * AHEAD + 1];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int abort_flag;
+  // lse and delta of the q columns lie over the bitmaps, which are dead once the
+  // union is listed: [buffer][parity][column] (MODE 1), [what][buffer][column] (MODE 2)
+  static_assert(sizeof(un.bm) >= 8 * 64 * sizeof(float), "");
+  float* s_cols = reinterpret_cast<float*>(&un.bm[0][0]);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int j0 = (blockIdx.x >> 1) * 4;      // first of the pair's four kv blocks
+  const int bh = blockIdx.y;
+  const int slices = WALK ? p.H / p.heads : p.H;
+  const int b_idx = bh / slices, h_idx = (bh - b_idx * slices) * (WALK ? p.heads : 1);
+  const int bhq = WALK ? b_idx * p.H + h_idx : bh;
+  const int groups = min(4, p.Mkv - j0);     // kv blocks of the pair that exist
+  const int tile_tok0 = (j0 + 2 * static_cast<int>(rank)) * G - p.kv_pad_head;   // my 128 rows
+
+  const uint32_t bar_kv = smem_u32(&bars[0]);        // my K / V tiles
+  const uint32_t bar_peer_kv = smem_u32(&bars[1]);   // CTA 0: CTA 1's
+  auto bar_full = [&](int s) { return smem_u32(&bars[2 + s]); };
+  auto bar_empty = [&](int s) { return smem_u32(&bars[2 + SLOTS + s]); };
+  auto bar_peer = [&](int s) { return smem_u32(&bars[2 + 2 * SLOTS + s]); };   // CTA 0 only
+  constexpr int BAR_A0 = 2 + 3 * SLOTS;
+  auto bar_afull = [&](int s) { return smem_u32(&bars[BAR_A0 + s]); };
+  auto bar_pfull = [&](int s) { return smem_u32(&bars[BAR_A0 + AHEAD + s]); };  // CTA 0 only
+  const uint32_t bar_final = smem_u32(&bars[BAR_A0 + 2 * AHEAD]);
+
+  if (tid == 0) {
+    abort_flag = 0;
+    mbar_init(bar_kv, 1);
+    mbar_init(bar_peer_kv, 1);
+    for (int s = 0; s < SLOTS; s++) {
+      mbar_init(bar_full(s), 1);
+      mbar_init(bar_empty(s), 1);
+      mbar_init(bar_peer(s), 1);
+    }
+    for (int s = 0; s < AHEAD; s++) {
+      mbar_init(bar_afull(s), 1);
+      mbar_init(bar_pfull(s), MODE == 1 ? 8 : 32);   // the warps that work on a tile, of both CTAs
+    }
+    mbar_init(bar_final, 1);
+    mbar_init_fence();
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_do);
+    tma_prefetch_desc(&tm_q32);
+    tma_prefetch_desc(&tm_do32);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+  }
+  if (warp == 0) {
+    tmem_alloc2(smem_u32(&tmem_base_s), 512);
+    tmem_relinquish2();
+  }
+  const int n = dkv_union(un, p, bhq, j0, groups);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();        // barriers of both CTAs are initialised before anyone signals them
+  tc_fence_after();
+  const uint32_t tmem = tmem_base_s;
+  WaitCtx w{&abort_flag, p.status};
+
+  if (warp == 0) {
+    // ------------------------------------------------------- TMA producer
+    if (lane == 0 && n > 0) {
+      mbar_expect_tx(bar_kv, FIRST * B6_ROWS);
+      for (int c = 0; c < NCH; c++) {
+        tma_load_4d(smem_u32(sK) + c * 128 * 128, &tm_k, bar_kv, c * 64, h_idx / p.kv_hdiv,
+                    tile_tok0, b_idx);
+        if (MODE == 2)
+          tma_load_4d(smem_u32(sV) + c * 128 * 128, &tm_v, bar_kv, c * 64, h_idx / p.kv_hdiv,
+                      tile_tok0, b_idx);
+      }
+      const int dcol = 128 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
+      PieceWalk<SLOTS> at;
+      auto piece = [&]() -> uint32_t {   // next free slot, 0 after a failed wait
+        if (!mbar_wait(bar_empty(at.slot), at.phase ^ 1, w, FTK_DEV_TIMEOUT_TMA)) return 0;
+        mbar_expect_tx(bar_full(at.slot), B6_PIECE);
+        return smem_u32(sRing) + at.slot * B6_PIECE;
+      };
+      HeadWalk<WALK> hw1, hw2;   // first and second steps run through the tiles on their own
+      in_piece_order(
+          n, AHEAD,
+          [&](int i) {
+            const int row0 = hw1.at(un.ids[i], p) * G - p.q_pad_head + rsub;
+            for (int x = 0; x < FIRST; x++) {
+              const uint32_t dst = piece();
+              if (!dst) return false;
+              for (int c = 0; c < NCH; c++)
+                tma_load_4d(dst + c * 4096, x ? &tm_do32 : &tm_q32, bar_full(at.slot), c * 64,
+                            h_idx + hw1.head, row0, b_idx);
+              at.next();
+            }
+            return true;
+          },
+          [&](int i) {
+            const int row0 = hw2.at(un.ids[i], p) * G - p.q_pad_head;
+            const uint32_t dst = piece();
+            if (!dst) return false;
+            for (int c = 0; c < 2; c++)
+              tma_load_4d(dst + c * 8192, MODE == 1 ? &tm_do : &tm_q, bar_full(at.slot),
+                          dcol + c * 64, h_idx + hw2.head, row0, b_idx);
+            at.next();
+            return true;
+          });
+    }
+  } else if (warp == 1 && rank == 1) {
+    // ----------------------- CTA 1: tell CTA 0 when my tiles have landed
+    if (n > 0) {
+      bool ok = mbar_wait(bar_kv, 0, w, FTK_DEV_TIMEOUT_MMA);
+      __syncwarp();
+      if (ok && lane == 0) mbar_arrive_cta(bar_peer_kv, 0);
+      PieceWalk<SLOTS> at;
+      for (int u = 0; ok && u < (FIRST + 1) * n; u++) {
+        ok = mbar_wait(bar_full(at.slot), at.phase, w, FTK_DEV_TIMEOUT_MMA);
+        __syncwarp();
+        if (ok && lane == 0) mbar_arrive_cta(bar_peer(at.slot), 0);
+        at.next();
+      }
+    }
+  } else if (warp == 1) {
+    // ----------------------------- CTA 0: UMMA issuer for the CTA pair
+    if (n > 0) {
+      const uint32_t idesc_a = umma_idesc(256, G, FMT, 0, 0);
+      const uint32_t idesc_b = umma_idesc(256, D, FMT, 0, 1);
+      const uint64_t kdesc0 = smem_desc_sw128(smem_u32(sK), 16, 1024);
+      const uint64_t vdesc0 = smem_desc_sw128(smem_u32(sV), 16, 1024);
+      const uint64_t rowdesc0 = smem_desc_sw128(smem_u32(sRing), 16, 1024);
+      const uint64_t coldesc0 = smem_desc_sw128(smem_u32(sRing), 8192, 1024);
+      const uint32_t kvb[2] = {bar_kv, bar_peer_kv};
+      const uint32_t kvp[2] = {0u, 0u};
+      bool ok = mbar_wait_all<2>(kvb, kvp, w, FTK_DEV_TIMEOUT_MMA);
+      PieceWalk<SLOTS> at;
+      // S^T (and dP^T) of a tile: pieces `q` and `d` (elected lane only)
+      auto mma_a = [&](int i, int q, int d) {
+        const uint64_t qdesc = desc_advance(rowdesc0, q * B6_PIECE);
+        const uint32_t sb = i & (AHEAD - 1);
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ks++)
+          umma2_ss(tmem + sb * 64, desc_advance(kdesc0, (ks / 4) * 128 * 128 + (ks % 4) * 32),
+                   desc_advance(qdesc, (ks / 4) * 4096 + (ks % 4) * 32), idesc_a, ks > 0);
+        if (MODE == 2) {
+          umma2_commit(bar_empty(q), 3);
+          const uint64_t dodesc = desc_advance(rowdesc0, d * B6_PIECE);
+#pragma unroll
+          for (int ks = 0; ks < D / 16; ks++)
+            umma2_ss(tmem + COL_DP + sb * 64,
+                     desc_advance(vdesc0, (ks / 4) * 128 * 128 + (ks % 4) * 32),
+                     desc_advance(dodesc, (ks / 4) * 4096 + (ks % 4) * 32), idesc_a, ks > 0);
+        }
+        umma2_commit(bar_afull(sb), 3);
+        umma2_commit(bar_empty(MODE == 2 ? d : q), 3);
+      };
+      auto take = [&]() {
+        const PieceWalk<SLOTS> t = at;
+        at.next();
+        return t;
+      };
+      for (int i = 0; ok && i < AHEAD && i < n; i++) {
+        const PieceWalk<SLOTS> q = take();
+        const PieceWalk<SLOTS> d = MODE == 2 ? take() : q;
+        const uint32_t wb[4] = {bar_full(q.slot), bar_peer(q.slot), bar_full(d.slot),
+                                bar_peer(d.slot)};
+        const uint32_t wp[4] = {q.phase, q.phase, d.phase, d.phase};
+        ok = mbar_wait_all<4>(wb, wp, w, FTK_DEV_TIMEOUT_MMA);
+        tc_fence_after();
+        if (ok && elect_one()) mma_a(i, q.slot, d.slot);
+        __syncwarp();
+      }
+      for (int i = 0; ok && i < n; i++) {
+        const bool more = i + AHEAD < n;
+        const int sb = i & (AHEAD - 1);
+        const PieceWalk<SLOTS> c = take();
+        const PieceWalk<SLOTS> q = more ? take() : c;
+        const PieceWalk<SLOTS> d = MODE == 2 && more ? take() : q;
+        constexpr int NW = MODE == 2 ? 7 : 5;
+        const uint32_t all_b[7] = {bar_pfull(sb),    bar_full(c.slot), bar_peer(c.slot),
+                                   bar_full(q.slot), bar_peer(q.slot), bar_full(d.slot),
+                                   bar_peer(d.slot)};
+        const uint32_t all_p[7] = {static_cast<uint32_t>((i / AHEAD) & 1), c.phase, c.phase,
+                                   q.phase, q.phase, d.phase, d.phase};
+        uint32_t wb[NW], wp[NW];
+#pragma unroll
+        for (int x = 0; x < NW; x++) {
+          wb[x] = all_b[x];
+          wp[x] = all_p[x];
+        }
+        if (!mbar_wait_all<NW>(wb, wp, w, FTK_DEV_TIMEOUT_MMA)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        if (elect_one()) {
+          const uint64_t col = desc_advance(coldesc0, c.slot * B6_PIECE);
+#pragma unroll
+          for (int ks = 0; ks < 4; ks++) {
+            // MODE 1: P^T over the first half of S^T; MODE 2: dS^T of each column
+            // quarter over the dP^T columns of the warps that wrote it
+            const uint32_t a = MODE == 1 ? sb * 64 + ks * 8 : COL_DP + sb * 64 + ks * 16;
+            umma2_ts(tmem + COL_OUT, tmem + a, desc_advance(col, ks * 2048), idesc_b,
+                     (i > 0) || (ks > 0));
+          }
+          umma2_commit(bar_empty(c.slot), 3);
+          if (more) mma_a(i + AHEAD, q.slot, d.slot);
+        }
+        __syncwarp();
+      }
+      if (elect_one()) umma2_commit(bar_final, 3);
+      __syncwarp();
+    }
+  } else if (warp >= 2) {
+    const int cw = warp - 2;
+    const int gw = cw >> 2;                  // MODE 1: S^T buffer; MODE 2: quarter of the columns
+    const int quarter = warp & 3;
+    const int r = quarter * 32 + lane;
+    const int grp = 2 * static_cast<int>(rank) + r / G;   // kv block of the pair
+    const int tok = tile_tok0 + r;
+    const bool row_valid = (grp < groups) && tok >= 0 && tok < p.N;
+    const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+    const float c = p.scale_log2;
+    const float2 c2 = make_float2(c, c);
+    bool ok = true;
+    // lse (and delta) of a q-block, fetched a round ahead and staged negated
+    const int ct = MODE == 1 ? cw % 4 * 32 + lane : tid - 64;   // index among a tile's threads
+    HeadWalk<WALK> hw, hw_mine;
+    auto fetch = [&](int i, float& l2, float& dl) {
+      l2 = 0.f;
+      dl = 0.f;
+      if (ct < G && i < n) {
+        const int t = hw.at(un.ids[i], p) * G - p.q_pad_head + ct;
+        if (t >= 0 && t < p.N) {
+          const int64_t e = static_cast<int64_t>(bhq + hw.head) * p.N + t;
+          l2 = -p.lse[e] * 1.4426950408889634f;
+          if (MODE == 2) dl = -p.delta[e];
+        }
+      }
+    };
+    float l2_next, dl_next;
+    const int first = MODE == 1 ? gw : 0;
+    constexpr int STEP = MODE == 1 ? 4 : 1;
+    fetch(first, l2_next, dl_next);
+    for (int i = first; i < n; i += STEP) {
+      const int sb = i & (AHEAD - 1);
+      const int row0 = hw_mine.at(un.ids[i], p) * G - p.q_pad_head;
+      float* nl = MODE == 1 ? s_cols + (gw * 2 + ((i >> 2) & 1)) * 64 : s_cols + sb * 64;
+      float* nd = s_cols + (2 + sb) * 64;    // MODE 2 only
+      if (ct < G) {
+        nl[ct] = l2_next;
+        if (MODE == 2) nd[ct] = dl_next;
+      }
+      if (MODE == 1)
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + gw) : "memory");
+      else
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+      fetch(i + STEP, l2_next, dl_next);
+      if (!ok) continue;
+      if (!mbar_wait(bar_afull(sb), (i / AHEAD) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
+        ok = false;
+        continue;
+      }
+      tc_fence_after();
+      const int lo = max(0, -row0), hi = min(G, p.N - row0);
+      const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
+      const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
+      const bool none = !fast && !__any_sync(0xffffffffu, act);
+      const float4* l4 = reinterpret_cast<const float4*>(nl);
+      if (MODE == 1) {
+        const uint32_t st_addr = lane_addr + sb * 64;   // S^T, then P^T
+        if (none) {
+          uint32_t z[16];
+#pragma unroll
+          for (int x = 0; x < 16; x++) z[x] = 0u;
+          tmem_st16(st_addr, z);
+          tmem_st16(st_addr + 16, z);
+        } else {
+          uint32_t v[2][32];
+          tmem_ld32(st_addr, v[0]);
+          tmem_ld32(st_addr + 32, v[1]);
+          tmem_wait_ld();
+#pragma unroll
+          for (int half = 0; half < 2; half++) {
+            uint32_t pk[16];
+#pragma unroll
+            for (int x = 0; x < 32; x += 4) {
+              const float4 lq = l4[half * 8 + (x >> 2)];
+              const float2 t0 =
+                  __ffma2_rn(make_float2(__uint_as_float(v[half][x]), __uint_as_float(v[half][x + 1])),
+                             c2, make_float2(lq.x, lq.y));
+              const float2 t1 = __ffma2_rn(
+                  make_float2(__uint_as_float(v[half][x + 2]), __uint_as_float(v[half][x + 3])), c2,
+                  make_float2(lq.z, lq.w));
+              float e[4] = {fast_exp2(t0.x), fast_exp2(t0.y), fast_exp2(t1.x), fast_exp2(t1.y)};
+              if (!fast) {
+#pragma unroll
+                for (int y = 0; y < 4; y++) {
+                  const int col = half * 32 + x + y;
+                  if (!(act && col >= lo && col < hi)) e[y] = 0.f;
+                }
+              }
+              pk[x >> 1] = pack2f<FMT>(e[0], e[1]);
+              pk[(x >> 1) + 1] = pack2f<FMT>(e[2], e[3]);
+            }
+            tmem_st16(st_addr + half * 16, pk);
+          }
+        }
+      } else {
+        const int cbeg = gw * 16;
+        const uint32_t st_addr = lane_addr + sb * 64 + cbeg;
+        const uint32_t dp_addr = lane_addr + COL_DP + sb * 64 + cbeg;   // dP^T, then dS^T
+        if (none) {
+          const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+          tmem_st8(dp_addr, z);
+        } else {
+          const float4* d4 = reinterpret_cast<const float4*>(nd);
+          uint32_t sa[16], da[16], pd[8];
+          tmem_ld16(st_addr, sa);
+          tmem_ld16(dp_addr, da);
+          tmem_wait_ld();
+#pragma unroll
+          for (int x = 0; x < 16; x += 4) {
+            const float4 lq = l4[(cbeg + x) >> 2];
+            const float4 dq = d4[(cbeg + x) >> 2];
+#pragma unroll
+            for (int y = 0; y < 4; y += 2) {
+              const float2 nl2 = y == 0 ? make_float2(lq.x, lq.y) : make_float2(lq.z, lq.w);
+              const float2 nd2 = y == 0 ? make_float2(dq.x, dq.y) : make_float2(dq.z, dq.w);
+              const float2 t = __ffma2_rn(
+                  make_float2(__uint_as_float(sa[x + y]), __uint_as_float(sa[x + y + 1])), c2, nl2);
+              float2 pr = make_float2(fast_exp2(t.x), fast_exp2(t.y));
+              if (!fast) {
+                const int col = cbeg + x + y;
+                if (!(act && col >= lo && col < hi)) pr.x = 0.f;
+                if (!(act && col + 1 >= lo && col + 1 < hi)) pr.y = 0.f;
+              }
+              const float2 dd = __fadd2_rn(
+                  make_float2(__uint_as_float(da[x + y]), __uint_as_float(da[x + y + 1])), nd2);
+              const float2 ds = __fmul2_rn(pr, dd);
+              pd[(x + y) >> 1] = pack2f<FMT>(ds.x, ds.y);
+            }
+          }
+          tmem_st8(dp_addr, pd);
+        }
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cta(bar_pfull(sb), 0);
+    }
+    if (ok && n > 0) ok = mbar_wait(bar_final, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
+    if (ok) {
+      tc_fence_after();
+      uint8_t* base = static_cast<uint8_t*>(MODE == 1 ? p.out1 : p.out0);
+      const int64_t sb_ = MODE == 1 ? p.s1_b : p.s0_b, sn_ = MODE == 1 ? p.s1_n : p.s0_n,
+                    sh_ = MODE == 1 ? p.s1_h : p.s0_h;
+      const float mul = MODE == 1 ? 1.f : p.scale;
+      uint8_t* orow = nullptr;
+      if (row_valid)
+        orow = base + (p.out_f32 ? 4 : 2) *
+                          (static_cast<int64_t>(b_idx) * sb_ + static_cast<int64_t>(tok) * sn_ +
+                           static_cast<int64_t>(WALK ? h_idx / p.heads : h_idx) * sh_);
+      for (int c0 = gw * 32; c0 < D; c0 += 128) {
+        uint32_t v[32];
+        if (n > 0) {
+          tmem_ld32(lane_addr + COL_OUT + c0, v);
+          tmem_wait_ld();
+        }
+        if (row_valid) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int x = 0; x < 32; x += 2) {
+            const float a = n > 0 ? __uint_as_float(v[x]) * mul : 0.f;
+            const float b = n > 0 ? __uint_as_float(v[x + 1]) * mul : 0.f;
+            pk[x >> 1] = pack2f<FMT>(a, b);
+          }
+          store_row_part(orow, c0, p.D, pk, FMT, p.out_f32 != 0);
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (abort_flag)
+    for (int i = 0; i < 200; i++) __nanosleep(1000);
+  // neither CTA may leave (or free TMEM) while the other can still touch it
+  cluster_sync_all();
+  if (warp == 0) tmem_dealloc2(tmem, 512);
+}
+
+}  // namespace ftk

@@ -559,14 +559,13 @@ static int launch_fwd_pipe(const CUtensorMap& tq, const CUtensorMap& tk, const C
                     dim3(p.tiles_x, static_cast<unsigned>(BH)), FP_THREADS, smem, st, tq, tk, tv, p);
 }
 
-template <int FMT>
+template <int D, int FMT>
 static int launch_fwd_pipe2(const CUtensorMap& tq, const CUtensorMap& tk32, const CUtensorMap& tv,
                             const FwdParams& p, int64_t BH, cudaStream_t st) {
-  const size_t smem = 1024 + 2 * 128 * 128 + static_cast<size_t>(FP2_KST + FP2_VST) * 8192;
-  if (int e = allow_smem<sparse_fwd_pipe2_kernel<FMT>>(smem)) return e;
-  return launch_pdl(sparse_fwd_pipe2_kernel<FMT>,
-                    dim3(2 * ((p.QM + 3) / 4), static_cast<unsigned>(BH)), FP_THREADS, smem, st, tq,
-                    tk32, tv, p);
+  if (int e = allow_smem<sparse_fwd_pipe2_kernel<D, FMT>>(fp2_smem(D))) return e;
+  return launch_pdl(sparse_fwd_pipe2_kernel<D, FMT>,
+                    dim3(2 * ((p.QM + 3) / 4), static_cast<unsigned>(BH)), FP_THREADS, fp2_smem(D),
+                    st, tq, tk32, tv, p);
 }
 
 template <int D>
@@ -580,12 +579,10 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   if (nst < 2) return FTK_ERR_UNSUPPORTED;
   p.nstages = nst;
   const size_t smem = 1024 + NCH * 128 * 128 + static_cast<size_t>(nst) * stage_bytes;
-  if constexpr (D <= 128) {
-    if (p.redo_in) {   // finds its tiles itself: as many CTAs as run at once
-      if (int e = allow_smem<sparse_fwd_kernel<D, D, true>>(smem)) return e;
-      return launch_pdl(sparse_fwd_kernel<D, D, true>, std::min(p.tiles, sm_count()), FW_THREADS,
-                        smem, st, tq, tk, tv, p);
-    }
+  if (p.redo_in) {   // finds its tiles itself: as many CTAs as run at once
+    if (int e = allow_smem<sparse_fwd_kernel<D, D, true>>(smem)) return e;
+    return launch_pdl(sparse_fwd_kernel<D, D, true>, std::min(p.tiles, sm_count()), FW_THREADS, smem,
+                      st, tq, tk, tv, p);
   }
   if (int e = allow_smem<sparse_fwd_kernel<D, D, false>>(smem)) return e;
   return launch_pdl(sparse_fwd_kernel<D, D, false>, p.tiles, FW_THREADS, smem, st, tq, tk, tv, p);
@@ -638,7 +635,8 @@ static int attn_fwd(const ftk_attn& a, const AttnGrid& gr, void* o, int64_t so_b
   // 64-row kv blocks, q blocks of 64 or 32 rows and a workspace: the
   // pipelined kernel runs first and the exact kernel redoes the tiles it flags.
   const char* env = getenv("FTK_FWD_PIPE");
-  const bool pipe = gr.kd <= 128 && gr.kvb == 64 && (gr.g == 64 || gr.g == 32) && workspace &&
+  // (Head dim 256: q blocks of 64 rows only, the pair kernel.)
+  const bool pipe = gr.kvb == 64 && (gr.g == 64 || (gr.g == 32 && gr.kd <= 128)) && workspace &&
                     workspace_bytes >= fwd_workspace(BH, gr.QM, gr.g) && !(env && env[0] == '0');
   if (pipe) {
     p.redo_out = static_cast<int*>(workspace);
@@ -646,12 +644,18 @@ static int attn_fwd(const ftk_attn& a, const AttnGrid& gr, void* o, int64_t so_b
     // Pairs walk the union of four lists: worth it when the lists can cover a
     // good part of the blocks (then the unions of two and of four are about
     // the same length); short lists keep the one-CTA kernel's unions of two.
-    if (gr.kd == 128 && gr.g == 64 && 4 * gr.width >= gr.Mkv && !(env2 && env2[0] == '0')) {
-      // head dim 128: the same kernel on pairs of SMs
+    // Head dim 256 takes pairs whatever the lists: four disjoint lists cost twice
+    // the tiles of two, the one-CTA kernel three times the cycles per tile.
+    if (gr.kd == 256) {
       CUtensorMap tk32;
       if ((e = tmap_rows(&tk32, a, 'k', 32))) return e;
-      e = a.dtype == FTK_DTYPE_BF16 ? launch_fwd_pipe2<1>(tq, tk32, tv, p, BH, st)
-                                    : launch_fwd_pipe2<0>(tq, tk32, tv, p, BH, st);
+      e = a.dtype == FTK_DTYPE_BF16 ? launch_fwd_pipe2<256, 1>(tq, tk32, tv, p, BH, st)
+                                    : launch_fwd_pipe2<256, 0>(tq, tk32, tv, p, BH, st);
+    } else if (gr.kd == 128 && gr.g == 64 && 4 * gr.width >= gr.Mkv && !(env2 && env2[0] == '0')) {
+      CUtensorMap tk32;
+      if ((e = tmap_rows(&tk32, a, 'k', 32))) return e;
+      e = a.dtype == FTK_DTYPE_BF16 ? launch_fwd_pipe2<128, 1>(tq, tk32, tv, p, BH, st)
+                                    : launch_fwd_pipe2<128, 0>(tq, tk32, tv, p, BH, st);
     } else if (a.dtype == FTK_DTYPE_BF16) {
       e = (gr.kd == 64) ? launch_fwd_pipe<64, 1>(tq, tk, tv, p, BH, st)
                         : launch_fwd_pipe<128, 1>(tq, tk, tv, p, BH, st);

@@ -1,5 +1,5 @@
 // The pipelined forward kernel (sparse_fwd_pipe.cuh) on pairs of SMs (tcgen05
-// cta_group::2), head dim 128.  Included by sparse_fwd.cu after it.
+// cta_group::2), head dims 128 and 256.  Included by sparse_fwd.cu after it.
 //
 // A cluster of two CTAs owns 256 query rows (four q-blocks).  Each CTA keeps its
 // own 128 rows of Q in TMEM, its own four S / P buffers, O accumulator and
@@ -16,24 +16,38 @@
 // tcgen05.commit multicasts its arrivals; CTA 1's warp 1 forwards "my tiles
 // have landed"; softmax warps of CTA 1 arrive on CTA 0's barriers through the
 // cluster shared-memory window.  No TMA load is multicast.
+//
+// Head dim 256: the 256-column O accumulator and the four S / P buffers fill
+// TMEM, so Q stays in shared memory (an M = 256 UMMA with both operands there
+// costs the same 43 cycles at N = 64) and the rings hold four K and four V half
+// tiles of 16 KB.  Per tile 16 x 43 + 4 x 128 = 1200 cycles for 256 query rows,
+// where the one-CTA exact kernel (16 x 75 + 4 x 138 for 128 rows, one softmax
+// group, two stages) took 3700.
 #pragma once
 
 namespace ftk {
 
-constexpr int FP2_KST = 6;   // K half tiles (8 KB) in the ring
-constexpr int FP2_VST = 8;   // V half tiles (8 KB) in the ring
+__host__ __device__ constexpr int fp2_kst(int d) { return d > 128 ? 4 : 6; }   // K half tiles
+__host__ __device__ constexpr int fp2_vst(int d) { return d > 128 ? 4 : 8; }   // V half tiles
+__host__ __device__ constexpr int fp2_tile(int d) { return d * 64; }           // bytes of either
+__host__ __device__ constexpr size_t fp2_smem(int d) {
+  return 1024 + static_cast<size_t>(d) * 256 +
+         static_cast<size_t>(fp2_kst(d) + fp2_vst(d)) * fp2_tile(d);
+}
 
-template <int FMT>
+template <int D, int FMT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FP_THREADS, 1)
 sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
                         const __grid_constant__ CUtensorMap tm_k32,
                         const __grid_constant__ CUtensorMap tm_v, const FwdParams p) {
-  constexpr int D = 128;
+  constexpr bool BIG = D > 128;                // Q read from shared memory
   constexpr int NCH = D / 64;
   constexpr int Q_BYTES = NCH * 128 * 128;
   constexpr int KVB = 64;
-  constexpr int TILE = 8192;                   // half a K tile (32 rows x 128 d) or half a V tile
-                                               // (64 rows x 64 d)
+  constexpr int TILE = fp2_tile(D);            // half a K tile (32 rows x D) or half a V tile
+                                               // (64 rows x D / 2)
+  constexpr int FP2_KST = fp2_kst(D), FP2_VST = fp2_vst(D);
+  constexpr uint32_t COL_S = BIG ? 0 : FP_COL_S, COL_O = BIG ? 256 : FP_COL_O;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -59,6 +73,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
   const uint32_t bar_q = smem_u32(&bars[0]);
   const uint32_t bar_final = smem_u32(&bars[1]);
   const uint32_t bar_qt = smem_u32(&bars[2]);    // CTA 0: Q of both CTAs copied into TMEM
+                                                 // (BIG: CTA 1's Q has landed)
   const uint32_t bar_pro = smem_u32(&bars[3]);   // CTA 0: every softmax warp has its reference
   auto bar_kfull = [&](int s) { return smem_u32(&bars[4 + s]); };
   auto bar_kempty = [&](int s) { return smem_u32(&bars[4 + FP2_KST + s]); };
@@ -76,7 +91,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
     s_ovf = 0;
     mbar_init(bar_q, 1);
     mbar_init(bar_final, 1);
-    mbar_init(bar_qt, 8);                  // the 4 copying warps of each CTA
+    mbar_init(bar_qt, BIG ? 1 : 8);        // the 4 copying warps of each CTA
     mbar_init(bar_pro, 8 * FP_GROUPS);     // the 16 softmax warps of each CTA
     for (int s = 0; s < FP2_KST; s++) {
       mbar_init(bar_kfull(s), 1);
@@ -154,37 +169,54 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
       // K entry j: the prologue blocks first, then the union; V entry i: the
       // union only.  Every wait depends on tiles loaded earlier only.
       const int total = npro + n;
-      const int dcol = 64 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
-      for (int j = 0; j < total; j++) {
-        const int sk = j % FP2_KST;
-        if (!mbar_wait(bar_kempty(sk), ((j / FP2_KST) & 1) ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
-        const bool pro = j < npro;
-        const int id = pro ? pro_block(j) : static_cast<int>(un.ids[j - npro]);
-        const int tok0 = id * KVB - p.kv_pad_head;
-        const uint32_t kb = smem_u32(sK) + sk * TILE;
-        mbar_expect_tx(bar_kfull(sk), TILE);
-        for (int c = 0; c < NCH; c++)
-          tma_load_4d(kb + c * 4096, &tm_k32, bar_kfull(sk), c * 64, h_idx / p.kv_hdiv,
-                      tok0 + rsub, b_idx);
-        if (!pro) {
-          const int i = j - npro, sv = i % FP2_VST;
+      const int dcol = D / 2 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
+      // BIG: V follows two entries behind K, so that the wait for one of the four
+      // V slots (held until P V) does not keep back the K tiles, needed earlier
+      constexpr int LAG = BIG ? 2 : 0;
+      for (int j = 0; j < total + LAG; j++) {
+        if (j < total) {
+          const int sk = j % FP2_KST;
+          if (!mbar_wait(bar_kempty(sk), ((j / FP2_KST) & 1) ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
+          const int id = j < npro ? pro_block(j) : static_cast<int>(un.ids[j - npro]);
+          const int tok0 = id * KVB - p.kv_pad_head;
+          const uint32_t kb = smem_u32(sK) + sk * TILE;
+          mbar_expect_tx(bar_kfull(sk), TILE);
+          for (int c = 0; c < NCH; c++)
+            tma_load_4d(kb + c * 4096, &tm_k32, bar_kfull(sk), c * 64, h_idx / p.kv_hdiv,
+                        tok0 + rsub, b_idx);
+        }
+        const int i = j - npro - LAG;
+        if (i >= 0) {
+          const int sv = i % FP2_VST;
+          const int tok0 = static_cast<int>(un.ids[i]) * KVB - p.kv_pad_head;
           if (!mbar_wait(bar_vempty(sv), ((i / FP2_VST) & 1) ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
           mbar_expect_tx(bar_vfull(sv), TILE);
-          tma_load_4d(smem_u32(sV) + sv * TILE, &tm_v, bar_vfull(sv), dcol, h_idx / p.kv_hdiv,
-                      tok0, b_idx);
+#pragma unroll
+          for (int c = 0; c < NCH / 2; c++)
+            tma_load_4d(smem_u32(sV) + sv * TILE + c * 8192, &tm_v, bar_vfull(sv), dcol + c * 64,
+                        h_idx / p.kv_hdiv, tok0, b_idx);
         }
       }
     }
   } else if (warp == 1 && rank == 1) {
     // ----------------------- CTA 1: tell CTA 0 when my tiles have landed
     const int total = npro + n;
-    for (int j = 0; n > 0 && j < total; j++) {
-      const int sk = j % FP2_KST;
-      if (!mbar_wait(bar_kfull(sk), (j / FP2_KST) & 1, w, FTK_DEV_TIMEOUT_MMA)) break;
+    if (BIG && n > 0) {
+      const bool landed = mbar_wait(bar_q, 0, w, FTK_DEV_TIMEOUT_MMA);
       __syncwarp();
-      if (lane == 0) mbar_arrive_cta(bar_peer_k(sk), 0);
-      if (j >= npro) {
-        const int i = j - npro, sv = i % FP2_VST;
+      if (landed && lane == 0) mbar_arrive_cta(bar_qt, 0);
+    }
+    constexpr int LAG = BIG ? 2 : 0;   // in the order in which the tiles were asked for
+    for (int j = 0; n > 0 && j < total + LAG; j++) {
+      if (j < total) {
+        const int sk = j % FP2_KST;
+        if (!mbar_wait(bar_kfull(sk), (j / FP2_KST) & 1, w, FTK_DEV_TIMEOUT_MMA)) break;
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cta(bar_peer_k(sk), 0);
+      }
+      const int i = j - npro - LAG;
+      if (i >= 0) {
+        const int sv = i % FP2_VST;
         if (!mbar_wait(bar_vfull(sv), (i / FP2_VST) & 1, w, FTK_DEV_TIMEOUT_MMA)) break;
         __syncwarp();
         if (lane == 0) mbar_arrive_cta(bar_peer_v(sv), 0);
@@ -197,7 +229,9 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
       const uint32_t idesc_pv = umma_idesc(256, D, FMT, 0, 1);
       const uint64_t kdesc0 = smem_desc_sw128(smem_u32(sK), 16, 1024);
       const uint64_t vdesc0 = smem_desc_sw128(smem_u32(sV), 8192, 1024);
+      const uint64_t qdesc0 = smem_desc_sw128(smem_u32(sQ), 16, 1024);
       bool ok = mbar_wait(bar_qt, 0, w, FTK_DEV_TIMEOUT_MMA);
+      if (BIG && ok) ok = mbar_wait(bar_q, 0, w, FTK_DEV_TIMEOUT_MMA);
       tc_fence_after();
       auto wait_k = [&](int j) -> bool {
         const int s = j % FP2_KST;
@@ -210,11 +244,16 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
       auto mma_s = [&](int j, int buf) {
         const int s = j % FP2_KST;
         const uint64_t kdesc = desc_advance(kdesc0, s * TILE);
-        const uint32_t d_tmem = tmem + FP_COL_S + buf * 64;
+        const uint32_t d_tmem = tmem + COL_S + buf * 64;
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ks++)
-          umma2_ts(d_tmem, tmem + ks * 8, desc_advance(kdesc, (ks / 4) * 4096 + (ks % 4) * 32),
-                   idesc_s, ks > 0);
+        for (int ks = 0; ks < D / 16; ks++) {
+          const uint64_t b = desc_advance(kdesc, (ks / 4) * 4096 + (ks % 4) * 32);
+          if (BIG)
+            umma2_ss(d_tmem, desc_advance(qdesc0, (ks / 4) * 128 * 128 + (ks % 4) * 32), b, idesc_s,
+                     ks > 0);
+          else
+            umma2_ts(d_tmem, tmem + ks * 8, b, idesc_s, ks > 0);
+        }
         umma2_commit(bar_sfull(buf), 3);
         umma2_commit(bar_kempty(s), 3);
       };
@@ -251,7 +290,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
         if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < KVB / 16; ks++)
-            umma2_ts(tmem + FP_COL_O, tmem + FP_COL_S + sb * 64 + ks * 8,
+            umma2_ts(tmem + COL_O, tmem + COL_S + sb * 64 + ks * 8,
                      desc_advance(vdesc, ks * 2048), idesc_pv, (i > 0) || (ks > 0));
           umma2_commit(bar_vempty(s), 3);
           // S(i+4) lands on the columns PV(i) reads P from; UMMAs run in issue order
@@ -271,12 +310,12 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int qrow = tile_row0 + r;
     const bool row_valid = (grp < groups) && qrow >= 0 && qrow < p.N;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
-    const uint32_t s_addr = lane_addr + FP_COL_S + gw * 64;
+    const uint32_t s_addr = lane_addr + COL_S + gw * 64;
     const float c = p.scale_log2;
     float mref = 0.f, l = 0.f;
     bool ok = true, ovf = false;
 
-    if (n > 0 && gw == 0) {
+    if (!BIG && n > 0 && gw == 0) {
       // group 0 moves the Q tile from (swizzled) shared memory into TMEM
       ok = mbar_wait(bar_q, 0, w, FTK_DEV_TIMEOUT_CONSUMER);
       if (ok) {
@@ -316,8 +355,8 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
           const int tok0 = pro_block(pb) * KVB - p.kv_pad_head;
           const int lo = max(0, -tok0), hi = min(KVB, p.N - tok0);
           uint32_t v0[32], v1[32];
-          tmem_ld32(lane_addr + FP_COL_S + pb * 64, v0);
-          tmem_ld32(lane_addr + FP_COL_S + pb * 64 + 32, v1);
+          tmem_ld32(lane_addr + COL_S + pb * 64, v0);
+          tmem_ld32(lane_addr + COL_S + pb * 64 + 32, v1);
           tmem_wait_ld();
           float mx = -INFINITY;
 #pragma unroll
@@ -434,22 +473,24 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
                (p.out_f32 ? 4 : 2) *
                    (static_cast<int64_t>(b_idx) * p.so_b + static_cast<int64_t>(qrow) * p.so_n +
                     static_cast<int64_t>(h_idx) * p.so_h);
-      constexpr int QUART = D / 4;   // 32 columns per group
-      const int c0 = gw * QUART;
-      uint32_t ov[QUART];
-      if (n > 0) {
-        tmem_ld32(lane_addr + FP_COL_O + c0, ov);
-        tmem_wait_ld();
-      }
-      if (row_valid) {
-        uint32_t pk[QUART / 2];
+      constexpr int QUART = D / 4;   // 32 or 64 columns per group
 #pragma unroll
-        for (int x = 0; x < QUART; x += 2) {
-          const float a = have ? __uint_as_float(ov[x]) * inv : 0.f;
-          const float b = have ? __uint_as_float(ov[x + 1]) * inv : 0.f;
-          pk[x >> 1] = pack16<FMT>(a, b);
+      for (int c0 = gw * QUART; c0 < (gw + 1) * QUART; c0 += 32) {
+        uint32_t ov[32];
+        if (n > 0) {
+          tmem_ld32(lane_addr + COL_O + c0, ov);
+          tmem_wait_ld();
         }
-        store_row_part(orow, c0, p.D, pk, FMT, p.out_f32 != 0);
+        if (row_valid) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int x = 0; x < 32; x += 2) {
+            const float a = have ? __uint_as_float(ov[x]) * inv : 0.f;
+            const float b = have ? __uint_as_float(ov[x + 1]) * inv : 0.f;
+            pk[x >> 1] = pack16<FMT>(a, b);
+          }
+          store_row_part(orow, c0, p.D, pk, FMT, p.out_f32 != 0);
+        }
       }
       if (row_valid && gw == 0)
         p.lse[static_cast<int64_t>(bh) * p.N + qrow] =
