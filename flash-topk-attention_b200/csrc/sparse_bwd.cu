@@ -57,6 +57,7 @@ struct BwdParams {
   int heads;                 // dKV: query heads one CTA walks (kv_hdiv, or 1: one result per query head)
   int span;                  // dKV with heads > 1: ids per head in the union (multiple of 32)
   const int32_t* order;      // dKV: kv blocks by fan-in, heaviest first ([BH][Mkv]) or null
+  int step;                  // dKV pair kernel at head dim 128: its STEP variant
   const int32_t* tile_order; // dKV: 128-row kv tiles by number of q-blocks, heaviest first, or null
 };
 
@@ -1276,11 +1277,15 @@ static int launch_dkv(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, 
                   : go(Kernel<sparse_bwd_dkv256_kernel<0, 2, false>>{}, smem_dk);
     }
     const size_t smem = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DK2_STAGES) * 32768;
-    if (bf)
-      return walk ? go(Kernel<sparse_bwd_dkv2_kernel<1, true>>{}, smem)
-                  : go(Kernel<sparse_bwd_dkv2_kernel<1, false>>{}, smem);
-    return walk ? go(Kernel<sparse_bwd_dkv2_kernel<0, true>>{}, smem)
-                : go(Kernel<sparse_bwd_dkv2_kernel<0, false>>{}, smem);
+    if (walk)
+      return bf ? (p.step ? go(Kernel<sparse_bwd_dkv2_kernel<1, true, true>>{}, smem)
+                          : go(Kernel<sparse_bwd_dkv2_kernel<1, true, false>>{}, smem))
+                : (p.step ? go(Kernel<sparse_bwd_dkv2_kernel<0, true, true>>{}, smem)
+                          : go(Kernel<sparse_bwd_dkv2_kernel<0, true, false>>{}, smem));
+    return bf ? (p.step ? go(Kernel<sparse_bwd_dkv2_kernel<1, false, true>>{}, smem)
+                        : go(Kernel<sparse_bwd_dkv2_kernel<1, false, false>>{}, smem))
+              : (p.step ? go(Kernel<sparse_bwd_dkv2_kernel<0, false, true>>{}, smem)
+                        : go(Kernel<sparse_bwd_dkv2_kernel<0, false, false>>{}, smem));
   }
   const int nch = kd / 64;
   const int stage_bytes = 2 * nch * p.g * 128;
@@ -1389,6 +1394,7 @@ extern "C" int ftk_attn_bwd_dkv(const ftk_attn* a, const void* dout, int64_t sdo
   p.mask_g = attn_groups(b.gr.g);
   p.span = b.span;
   p.heads = b.walk ? p.kv_hdiv : 1;
+  p.step = 2 * b.gr.width >= b.gr.Mkv;   // lists that can cover most blocks
   const bool parts = p.kv_hdiv > 1 && !b.walk;
   if (parts) {   // one 16-bit result per query head first
     const int64_t row = a->H * a->D;
@@ -1513,6 +1519,7 @@ extern "C" int ftk_sparse_bwd_dkv(
   p.s1_h = sdv_h;
   const bool pair = D == 128 && q_block_size == 64 && kv_block_size == 64 &&
                     (fwd_list_width <= 0 || 4 * static_cast<int64_t>(fwd_list_width) >= M);
+  p.step = fwd_list_width <= 0 || 2 * static_cast<int64_t>(fwd_list_width) >= M;
   // one-CTA kernels: tiles in order of fan-in when the caller brings the order
   if (!pair || env_off("FTK_DKV_2CTA"))
     p.order = sorted_kv && !env_off("FTK_DKV_ORDER") ? sorted_kv : nullptr;

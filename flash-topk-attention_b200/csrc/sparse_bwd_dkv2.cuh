@@ -45,7 +45,12 @@ __device__ __forceinline__ uint32_t pack2f(float a, float b) {
 // other.  A template parameter because the compute warps set this kernel's pace:
 // the head bookkeeping of WALK in every build took 28.3 -> 34.6 ms at N = 32768,
 // H = 32.
-template <int FMT, bool WALK>
+// STEP: the compute warps of a CTA go from tile to tile together (a barrier per
+// tile).  With full lists tile i then comes out of all warps ahead of tile i + 1 and
+// its buffer is free earlier (28.8 against 29.1 ms there, 3.76 against 3.98 ms at B = 4,
+// N = 8192, H = 16); with short lists most warps of a tile have nothing to do and
+// should run ahead (610 -> 569 us at W = 16 of 64 blocks, four heads per kv head).
+template <int FMT, bool WALK, bool STEP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(BW_THREADS, 1)
 sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
                        const __grid_constant__ CUtensorMap tm_do,
@@ -69,7 +74,9 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
   __shared__ __align__(8) uint64_t bars[2 + 3 * DK2_STAGES + 5];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
-  __shared__ __align__(16) float s_lse2[2][2][128], s_delta[2][2][128];  // [group][parity][q row]
+  // per compute warp and parity: lse, then delta, of the warp's 16 q columns (STEP:
+  // per parity, of all 64)
+  __shared__ __align__(16) float s_cols[16][2][32];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
@@ -255,7 +262,6 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int colq = cw >> 2;
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
-    const int ct = tid - 64;                 // index among the compute threads
     const int grp = 2 * static_cast<int>(rank) + r / G;   // kv block of the pair
     const int tok = tile_tok0 + r;
     const bool row_valid = (grp < groups) && tok >= 0 && tok < p.N;
@@ -265,17 +271,21 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     bool ok = true;
     // lse / delta of a q-block are fetched from global memory one round ahead
     // (into registers, while the previous tile is being worked on) and only
-    // then staged in shared memory: their latency stays out of the chain.
+    // then staged in shared memory, negated: the packed fma / add take them as
+    // they are.  STEP: staged once per CTA, behind a barrier of all compute warps.
+    // Otherwise every warp stages the 32 values that it needs itself.
     HeadWalk<WALK> hw, hw_mine;
+    const int ct = STEP ? tid - 64 : lane;            // column (and, without STEP, kind) fetched
+    const int col = STEP ? ct : cbeg + (lane & 15);
     auto fetch = [&](int i, float& l2, float& dl) {
       l2 = 0.f;
       dl = 0.f;
-      if (ct < G && i < n) {
-        const int t = hw.at(un.ids[i], p) * G - p.q_pad_head + ct;
-        if (t >= 0 && t < p.N) {   // stored negated: the packed fma / add take them as they are
+      if ((!STEP || ct < G) && i < n) {
+        const int t = hw.at(un.ids[i], p) * G - p.q_pad_head + col;
+        if (t >= 0 && t < p.N) {
           const int64_t e = static_cast<int64_t>(bhq + hw.head) * p.N + t;
-          l2 = -p.lse[e] * 1.4426950408889634f;
-          dl = -p.delta[e];
+          if (STEP || lane < 16) l2 = -p.lse[e] * 1.4426950408889634f;
+          if (STEP || lane >= 16) dl = -p.delta[e];
         }
       }
     };
@@ -284,11 +294,17 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     for (int i = 0; i < n; i++) {
       const int sb = i & 1;                  // S^T / dP^T buffer, and lse / delta buffer
       const int row0 = hw_mine.at(un.ids[i], p) * G - p.q_pad_head;
-      if (ct < G) {
-        s_lse2[0][sb][ct] = l2_next;
-        s_delta[0][sb][ct] = dl_next;
+      float* cols = STEP ? &s_cols[0][0][0] + sb * 128 : s_cols[cw][sb];
+      if (STEP) {
+        if (ct < G) {
+          cols[ct] = l2_next;
+          cols[64 + ct] = dl_next;
+        }
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+      } else {
+        cols[lane] = lane < 16 ? l2_next : dl_next;
+        __syncwarp();
       }
-      asm volatile("bar.sync 1, 512;" ::: "memory");
       fetch(i + 1, l2_next, dl_next);
       if (!ok) continue;
       if (!mbar_wait(bar_afull(sb), (i >> 1) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
@@ -302,8 +318,8 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
       const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
       const bool none = !fast && !__any_sync(0xffffffffu, act);
-      const float4* l4 = reinterpret_cast<const float4*>(s_lse2[0][sb]);
-      const float4* d4 = reinterpret_cast<const float4*>(s_delta[0][sb]);
+      const float4* l4 = reinterpret_cast<const float4*>(cols + (STEP ? cbeg : 0));
+      const float4* d4 = reinterpret_cast<const float4*>(cols + (STEP ? 64 + cbeg : 16));
       // P^T / dS^T of the thread's 16 columns go over the first 8 of them in
       // the S^T / dP^T regions: columns this thread has already read.
       // full tiles: two columns per instruction (fma.f32x2, add.f32x2,
@@ -315,8 +331,8 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
         if (fast) {
 #pragma unroll
           for (int x = 0; x < 16; x += 4) {
-            const float4 lq = l4[(c0 + x) >> 2];
-            const float4 dq = d4[(c0 + x) >> 2];
+            const float4 lq = l4[x >> 2];
+            const float4 dq = d4[x >> 2];
 #pragma unroll
             for (int y = 0; y < 4; y += 2) {
               const float2 nl = y == 0 ? make_float2(lq.x, lq.y) : make_float2(lq.z, lq.w);
@@ -334,8 +350,8 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
         } else {
 #pragma unroll
           for (int x = 0; x < 16; x += 4) {
-            const float4 lq = l4[(c0 + x) >> 2];
-            const float4 dq = d4[(c0 + x) >> 2];
+            const float4 lq = l4[x >> 2];
+            const float4 dq = d4[x >> 2];
             const float ls[4] = {lq.x, lq.y, lq.z, lq.w};
             const float ds[4] = {dq.x, dq.y, dq.z, dq.w};
             float pv[4], dsv[4];
