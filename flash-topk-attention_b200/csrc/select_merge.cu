@@ -105,21 +105,23 @@ topk_select_kernel(const float* __restrict__ scores, const float* __restrict__ r
   }
 }
 
-// (bitonic_desc, sorted_emit and the per-row register select live in select_row.cuh)
-// warps (= rows) per CTA: 8, or 4 where a row's scratch takes 6 KB
+// (the select of one row lives in select_row.cuh)
+// warps (= rows) per CTA: 8, or 4 for the widest rows
 template <int IPT>
 __host__ __device__ constexpr int sel_wpc() { return IPT >= 32 ? 4 : SEL_WARPS; }
 
+// CTAs per SM that the register budget is for (latency is hidden by warps)
 template <int IPT>
-__global__ void __launch_bounds__(sel_wpc<IPT>() * 32, IPT == 16 ? 3 : (IPT == 32 ? 4 : 1))
+__host__ __device__ constexpr int sel_ctas() { return IPT <= 4 || IPT == 32 ? 4 : 3; }
+
+template <int IPT>
+__global__ void __launch_bounds__(sel_wpc<IPT>() * 32, sel_ctas<IPT>())
 topk_select_reg_kernel(const float* __restrict__ scores, const float* __restrict__ row_scale,
                        int64_t rows, int M, int M_out, int bsz, int pad_head, int pad_tail,
                        float threshold, int32_t* __restrict__ out_idx,
                        float* __restrict__ out_raw, float* __restrict__ out_avg) {
   constexpr int WPC = sel_wpc<IPT>();
-  constexpr int CAP = IPT >= 4 ? 256 : 128;
-  __shared__ float sraw_all[WPC][32 * IPT];
-  __shared__ unsigned long long scand_all[IPT >= 2 ? WPC : 1][CAP];
+  __shared__ unsigned long long cand_all[WPC][SEL_CAND];
   pdl_wait();
   pdl_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -140,9 +142,9 @@ topk_select_reg_kernel(const float* __restrict__ scores, const float* __restrict
   for (; row < rows; row += nwarps) {
     fetch(row + nwarps, nxt);
     const float inv_total = row_scale ? __frcp_rn(row_scale[row]) : 1.f;
-    select_row_reg<IPT>(cur, row_scale != nullptr, inv_total, M, M_out, bsz, pad_head, pad_tail,
-                        threshold, sraw_all[warp], scand_all[IPT >= 2 ? warp : 0], lane,
-                        out_idx + row * M_out, out_raw + row * M_out, out_avg + row * M_out);
+    select_row_reg<IPT>(cur, scores + row * M, inv_total, M, M_out, bsz, pad_head, pad_tail,
+                        threshold, cand_all[warp], lane, out_idx + row * M_out,
+                        out_raw + row * M_out, out_avg + row * M_out);
     __syncwarp();   // the warp's scratch is free again
 #pragma unroll
     for (int i = 0; i < IPT; i++) cur[i] = nxt[i];
