@@ -1126,7 +1126,7 @@ head_sum_kernel(const uint8_t* __restrict__ dk_part, const uint8_t* __restrict__
 // where things lie in the workspace.
 struct BwdPlan {
   AttnGrid gr;
-  bool pair;                 // kernels on pairs of SMs
+  bool pair_dq, pair_dkv;    // kernels on pairs of SMs
   bool walk;                 // dK/dV: one CTA walks all query heads of its kv head
   int tiles, stride, span;   // tile masks (see write_tile_masks)
   int kv_tiles;              // 128-row kv tiles per slice
@@ -1153,11 +1153,14 @@ static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
   b.stride = (gr.Mkv + 15) & ~15;
   b.span = (b.tiles * per + 31) & ~31;
   b.kv_tiles = (gr.Mkv + G - 1) / G;
-  // Pairs walk the union of four lists: only when the lists can cover a good part
-  // of the blocks (see ftk_attn_fwd)
-  // at head dim 128; at 256 the pair kernels are several times the faster per tile.
-  b.pair = gr.g == 64 && gr.kvb == 64 &&
-           (gr.kd == 256 || (gr.kd == 128 && 4 * gr.width >= gr.Mkv));
+  // Pairs walk the union of four lists.  For dQ the line is that of ftk_attn_fwd
+  // (f = 1/4 there: 451 us in pairs, 388 without); dK / dV gains more from them (its
+  // S^T and dP^T UMMAs read both operands from shared memory) and breaks even at
+  // f = 1/4 (585 against 597 us).  At head dim 256 the pair kernels are several times
+  // the faster per tile.
+  const bool rows64 = gr.g == 64 && gr.kvb == 64;
+  b.pair_dq = rows64 && (gr.kd == 256 || (gr.kd == 128 && 2 * gr.width >= gr.Mkv));
+  b.pair_dkv = rows64 && (gr.kd == 256 || (gr.kd == 128 && 4 * gr.width >= gr.Mkv));
   // Query heads that share a kv head: walked one after the other by the CTA that
   // owns the kv rows, so that their sum stays in its fp32 accumulators, unless
   // that leaves SMs idle: waves of CTAs times heads per CTA against waves of one
@@ -1169,7 +1172,7 @@ static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
            4 * grp * waves(ctas) <= 5 * waves(ctas * grp);
   const int64_t slices = b.walk ? a.B * a.Hkv : BH;
   // sorting pays once the tiles come in several waves
-  b.order = !b.pair && slices * b.kv_tiles >= 2 * sms;
+  b.order = !b.pair_dkv && slices * b.kv_tiles >= 2 * sms;
   size_t off = up256(static_cast<size_t>(BH) * a.N * 4);   // delta
   b.off_masks = off;
   off += up256(static_cast<size_t>(BH) * b.tiles * b.stride);
@@ -1406,7 +1409,7 @@ extern "C" int ftk_attn_bwd_dq(const ftk_attn* a, const void* o, int64_t so_b, i
   p.s0_b = sdq_b;
   p.s0_n = sdq_n;
   p.s0_h = sdq_h;
-  return launch_dq(*a, Rows{dout, a->H, sdo_b, sdo_n, sdo_h}, p, b.gr.kd, b.pair,
+  return launch_dq(*a, Rows{dout, a->H, sdo_b, sdo_n, sdo_h}, p, b.gr.kd, b.pair_dq,
                    static_cast<cudaStream_t>(stream));
 }
 
@@ -1467,7 +1470,7 @@ extern "C" int ftk_attn_bwd_dkv(const ftk_attn* a, const void* dout, int64_t sdo
     if (e) return e;
     p.tile_order = order;
   }
-  if (int e = launch_dkv(*a, Rows{dout, a->H, sdo_b, sdo_n, sdo_h}, p, b.gr.kd, b.pair, st))
+  if (int e = launch_dkv(*a, Rows{dout, a->H, sdo_b, sdo_n, sdo_h}, p, b.gr.kd, b.pair_dkv, st))
     return e;
   if (!parts) return FTK_OK;
   const int64_t vecs = a->B * a->N * a->Hkv * (a->D / 8);
@@ -1517,7 +1520,7 @@ extern "C" int ftk_sparse_bwd_dq(
   p.s0_n = sdq_n;
   p.s0_h = sdq_h;
   const bool pair = D == 128 && q_block_size == 64 && kv_block_size == 64 &&
-                    4 * static_cast<int64_t>(W) >= gr.Mkv;
+                    2 * static_cast<int64_t>(W) >= gr.Mkv;
   return launch_dq(a, Rows{dout, H, sdo_b, sdo_n, sdo_h}, p, gr.kd, pair,
                    static_cast<cudaStream_t>(stream));
 }

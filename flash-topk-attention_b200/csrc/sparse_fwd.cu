@@ -641,9 +641,11 @@ static int attn_fwd(const ftk_attn& a, const AttnGrid& gr, void* o, int64_t so_b
   if (pipe) {
     p.redo_out = static_cast<int*>(workspace);
     const char* env2 = getenv("FTK_FWD_2CTA");
-    // Pairs walk the union of four lists: worth it when the lists can cover a
-    // good part of the blocks (then the unions of two and of four are about
-    // the same length); short lists keep the one-CTA kernel's unions of two.
+    // Pairs walk the union of four lists where one CTA walks that of two, at 0.9 of
+    // the time per tile.  Unions of f = W / blocks grow by 1 + (1 - f)^2 with
+    // independent lists and not at all with equal ones, so the line is drawn at
+    // f = 1/2 (f = 1/4, lists half alike, B = 2, N = 4096, H = 32: 377 us in pairs, 307
+    // without).
     // Head dim 256 takes pairs whatever the lists: four disjoint lists cost twice
     // the tiles of two, the one-CTA kernel three times the cycles per tile.
     if (gr.kd == 256) {
@@ -651,7 +653,7 @@ static int attn_fwd(const ftk_attn& a, const AttnGrid& gr, void* o, int64_t so_b
       if ((e = tmap_rows(&tk32, a, 'k', 32))) return e;
       e = a.dtype == FTK_DTYPE_BF16 ? launch_fwd_pipe2<256, 1>(tq, tk32, tv, p, BH, st)
                                     : launch_fwd_pipe2<256, 0>(tq, tk32, tv, p, BH, st);
-    } else if (gr.kd == 128 && gr.g == 64 && 4 * gr.width >= gr.Mkv && !(env2 && env2[0] == '0')) {
+    } else if (gr.kd == 128 && gr.g == 64 && 2 * gr.width >= gr.Mkv && !(env2 && env2[0] == '0')) {
       CUtensorMap tk32;
       if ((e = tmap_rows(&tk32, a, 'k', 32))) return e;
       e = a.dtype == FTK_DTYPE_BF16 ? launch_fwd_pipe2<128, 1>(tq, tk32, tv, p, BH, st)
