@@ -69,55 +69,75 @@ struct BwdParams {
 // As a kernel of its own this cost a launch and 258 us at N = 32768, H = 32,
 // D = 128 (122 us at B = 4, N = 8192, H = 16), reading O and dO at 4.2 TB/s;
 // here the reads hide behind the other CTAs' UMMAs.
+// The loads are issued before the union is built and used after it.
 template <int KD>
-__device__ __forceinline__ void tile_delta(const BwdParams& p, float* s_delta, int bh, int b, int h,
-                                           int tile_row0, int rows) {
-  constexpr int LPR = KD / 8, RPW = 32 / LPR, WARPS = BW_THREADS / 32;
-  constexpr int STEPS = (128 + RPW * WARPS - 1) / (RPW * WARPS);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = lane % LPR;
-  const int64_t ob = static_cast<int64_t>(b) * p.so_b + static_cast<int64_t>(h) * p.so_h,
-                db = static_cast<int64_t>(b) * p.sd_b + static_cast<int64_t>(h) * p.sd_h;
+struct TileDelta {
+  static constexpr int LPR = KD / 8, RPW = 32 / LPR, WARPS = BW_THREADS / 32;
+  static constexpr int STEPS = (128 + RPW * WARPS - 1) / (RPW * WARPS);
+  uint4 vd[STEPS], vo[STEPS], vo2[STEPS];   // vo2: float32 O only
+
+  __device__ __forceinline__ int row(int i) const {
+    return (i * WARPS + (threadIdx.x >> 5)) * RPW + (threadIdx.x & 31) / LPR;
+  }
+  __device__ __forceinline__ bool inside(const BwdParams& p, int r, int n, int rows) const {
+    return r < rows && n >= 0 && n < p.N && (threadIdx.x & 31) % LPR * 8 < p.D;
+  }
+  __device__ __forceinline__ void load(const BwdParams& p, int b, int h, int tile_row0, int rows) {
+    const int c = (threadIdx.x & 31) % LPR;
+    const int64_t ob = static_cast<int64_t>(b) * p.so_b + static_cast<int64_t>(h) * p.so_h,
+                  db = static_cast<int64_t>(b) * p.sd_b + static_cast<int64_t>(h) * p.sd_h;
 #pragma unroll
-  for (int i = 0; i < STEPS; i++) {
-    const int r = (i * WARPS + warp) * RPW + lane / LPR;
-    const int n = tile_row0 + r;
-    const bool in = r < rows && n >= 0 && n < p.N && c * 8 < p.D;
-    float acc = 0.f;
-    if (in) {
-      const uint4 vd = __ldg(reinterpret_cast<const uint4*>(
-          p.dout + 2 * (db + static_cast<int64_t>(n) * p.sd_n)) + c);
-      const uint32_t wd[4] = {vd.x, vd.y, vd.z, vd.w};
-      float2 fo[4];
+    for (int i = 0; i < STEPS; i++) {
+      const int r = row(i), n = tile_row0 + r;
+      vd[i] = vo[i] = vo2[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (!inside(p, r, n, rows)) continue;
+      vd[i] = __ldg(reinterpret_cast<const uint4*>(
+                        p.dout + 2 * (db + static_cast<int64_t>(n) * p.sd_n)) + c);
       const int64_t oe = ob + static_cast<int64_t>(n) * p.so_n;
       if (p.out_f32) {
-        const float4* src = reinterpret_cast<const float4*>(p.o + 4 * oe) + 2 * c;
-        const float4 x = __ldg(src), y = __ldg(src + 1);
-        fo[0] = make_float2(x.x, x.y);
-        fo[1] = make_float2(x.z, x.w);
-        fo[2] = make_float2(y.x, y.y);
-        fo[3] = make_float2(y.z, y.w);
+        const uint4* src = reinterpret_cast<const uint4*>(p.o + 4 * oe) + 2 * c;
+        vo[i] = __ldg(src);
+        vo2[i] = __ldg(src + 1);
       } else {
-        const uint4 vo = __ldg(reinterpret_cast<const uint4*>(p.o + 2 * oe) + c);
-        fo[0] = unpack2(vo.x, p.fmt);
-        fo[1] = unpack2(vo.y, p.fmt);
-        fo[2] = unpack2(vo.z, p.fmt);
-        fo[3] = unpack2(vo.w, p.fmt);
+        vo[i] = __ldg(reinterpret_cast<const uint4*>(p.o + 2 * oe) + c);
       }
+    }
+  }
+  __device__ __forceinline__ void finish(const BwdParams& p, float* s_delta, int bh, int tile_row0,
+                                         int rows) {
+    const int c = (threadIdx.x & 31) % LPR;
+#pragma unroll
+    for (int i = 0; i < STEPS; i++) {
+      const int r = row(i), n = tile_row0 + r;
+      const uint32_t wd[4] = {vd[i].x, vd[i].y, vd[i].z, vd[i].w};
+      float2 fo[4];
+      if (p.out_f32) {
+        fo[0] = make_float2(__uint_as_float(vo[i].x), __uint_as_float(vo[i].y));
+        fo[1] = make_float2(__uint_as_float(vo[i].z), __uint_as_float(vo[i].w));
+        fo[2] = make_float2(__uint_as_float(vo2[i].x), __uint_as_float(vo2[i].y));
+        fo[3] = make_float2(__uint_as_float(vo2[i].z), __uint_as_float(vo2[i].w));
+      } else {
+        fo[0] = unpack2(vo[i].x, p.fmt);
+        fo[1] = unpack2(vo[i].y, p.fmt);
+        fo[2] = unpack2(vo[i].z, p.fmt);
+        fo[3] = unpack2(vo[i].w, p.fmt);
+      }
+      float acc = 0.f;
 #pragma unroll
       for (int x = 0; x < 4; x++) {
         const float2 gd = unpack2(wd[x], p.fmt);
         acc = fmaf(fo[x].x, gd.x, acc);
         acc = fmaf(fo[x].y, gd.y, acc);
       }
-    }
 #pragma unroll
-    for (int d = LPR >> 1; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
-    if (c == 0 && r < 128) {
-      s_delta[r] = acc;
-      if (in) p.delta[static_cast<int64_t>(bh) * p.N + n] = acc;
+      for (int d = LPR >> 1; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+      if (c == 0 && r < 128) {
+        s_delta[r] = acc;
+        if (inside(p, r, n, rows)) p.delta[static_cast<int64_t>(bh) * p.N + n] = acc;
+      }
     }
   }
-}
+};
 
 // dS = 2^(c s - lse2) (dp - delta) for 32 columns of one row, two columns per
 // instruction (fma.f32x2, add.f32x2, mul.f32x2, one cvt per pair).
@@ -276,9 +296,19 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   clear_bitmaps(un);
   pdl_wait();
   pdl_launch();
-  tile_delta<D>(p, s_delta, bh, b_idx, h_idx, tile_row0, groups * p.g);
+  if (tid == 0) {   // under the building of the union
+    mbar_expect_tx(bar_q, 2 * ROW_TILE_BYTES);
+    for (int c = 0; c < NCH; c++) {
+      tma_load_4d(smem_u32(sQ) + c * 128 * 128, &tm_q, bar_q, c * 64, h_idx, tile_row0, b_idx);
+      tma_load_4d(smem_u32(sDO) + c * 128 * 128, &tm_do, bar_q, c * 64, h_idx, tile_row0, b_idx);
+    }
+  }
+  TileDelta<D> delta;
+  if (D <= 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);
   const int n = build_union(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
                             p.W, nullptr, p.Mkv, p.lm, p.status);
+  if (D > 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);   // too many registers to hold across the union
+  delta.finish(p, s_delta, bh, tile_row0, groups * p.g);
   if (p.masks)
     write_tile_masks(un, p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + blockIdx.x) * p.mask_stride,
                      p.mask_stride, 0, groups);
@@ -290,12 +320,8 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   const bool split = (p.kvb % 32) == 0;   // kv columns of a tile shared by two warps per row
 
   if (warp == 0) {
+    if (lane == 0 && n == 0) mbar_wait(bar_q, 0, w, FTK_DEV_TIMEOUT_TMA);   // lands before the exit
     if (lane == 0 && n > 0) {
-      mbar_expect_tx(bar_q, 2 * ROW_TILE_BYTES);
-      for (int c = 0; c < NCH; c++) {
-        tma_load_4d(smem_u32(sQ) + c * 128 * 128, &tm_q, bar_q, c * 64, h_idx, tile_row0, b_idx);
-        tma_load_4d(smem_u32(sDO) + c * 128 * 128, &tm_do, bar_q, c * 64, h_idx, tile_row0, b_idx);
-      }
       for (int i = 0; i < n; i++) {
         const int sk = i % KST, sv = i % VST;
         const int tok0 = static_cast<int>(un.ids[i]) * p.kvb - p.kv_pad_head;

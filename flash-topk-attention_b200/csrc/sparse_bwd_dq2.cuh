@@ -95,12 +95,22 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
   }
   // both CTAs build the same union over the pair's four candidate lists
   clear_bitmaps(un);
+  cluster_arrive();
   pdl_wait();
   pdl_launch();
   const int mine = min(2, groups - 2 * static_cast<int>(rank));   // q-blocks of my tile, if any
-  tile_delta<D>(p, s_delta, bh, b_idx, h_idx, tile_row0, mine * G);
+  if (tid == 0) {   // under the building of the union
+    mbar_expect_tx(bar_q, 2 * ROW_TILE_BYTES);
+    for (int c = 0; c < NCH; c++) {
+      tma_load_4d(smem_u32(sQ) + c * 128 * 128, &tm_q, bar_q, c * 64, h_idx, tile_row0, b_idx);
+      tma_load_4d(smem_u32(sDO) + c * 128 * 128, &tm_do, bar_q, c * 64, h_idx, tile_row0, b_idx);
+    }
+  }
+  TileDelta<D> delta;
+  delta.load(p, b_idx, h_idx, tile_row0, mine * G);
   const int n = build_union(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
                             p.W, nullptr, p.Mkv, p.lm, p.status);
+  delta.finish(p, s_delta, bh, tile_row0, mine * G);
   if (p.masks && mine > 0)
     write_tile_masks(un,
                      p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + m0 / 2 + rank) *
@@ -108,19 +118,15 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
                      p.mask_stride, 2 * static_cast<int>(rank), mine);
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();        // barriers of both CTAs are initialised before anyone signals them
+  cluster_wait();            // barriers of both CTAs are initialised before anyone signals them
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
   WaitCtx w{&abort_flag, p.status};
 
   if (warp == 0) {
     // ------------------------------------------------------- TMA producer
+    if (lane == 0 && n == 0) mbar_wait(bar_q, 0, w, FTK_DEV_TIMEOUT_TMA);   // lands before the exit
     if (lane == 0 && n > 0) {
-      mbar_expect_tx(bar_q, 2 * ROW_TILE_BYTES);
-      for (int c = 0; c < NCH; c++) {
-        tma_load_4d(smem_u32(sQ) + c * 128 * 128, &tm_q, bar_q, c * 64, h_idx, tile_row0, b_idx);
-        tma_load_4d(smem_u32(sDO) + c * 128 * 128, &tm_do, bar_q, c * 64, h_idx, tile_row0, b_idx);
-      }
       const int dcol = 64 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
       const int hk = h_idx / p.kv_hdiv;
       for (int i = 0; i < n; i++) {
