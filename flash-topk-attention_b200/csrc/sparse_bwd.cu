@@ -494,16 +494,17 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
     for (int i = wg; ok && i < n; i += 2) {
       // A(i) complete also means B(i-2) has retired (same issue order), so the
       // dS columns of this buffer are free again.
-      if (!mbar_wait(bar_afull(wg), (i >> 1) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
-        ok = false;
-        break;
-      }
-      tc_fence_after();
+      // what the tile's columns mean to this row: worked out before the wait
       const int tok0 = static_cast<int>(un.ids[i]) * p.kvb - p.kv_pad_head;
       const int lo = max(0, -tok0), hi = min(p.kvb, p.N - tok0);
       const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == p.kvb;
       const bool none = !fast && !__any_sync(0xffffffffu, act);
+      if (!mbar_wait(bar_afull(wg), (i >> 1) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
       // dS of columns [c0, c0+w) is written over dP columns [cbeg + (c0-cbeg)/2, ..):
       // columns this thread has already read, never another warp's
       for (int c0 = cbeg; c0 < cend; c0 += 32) {

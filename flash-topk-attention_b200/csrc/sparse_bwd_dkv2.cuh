@@ -307,6 +307,11 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
       }
       fetch(i + 1, l2_next, dl_next);
       if (!ok) continue;
+      // what the tile's columns mean to this row: worked out before the wait
+      const int lo = max(0, -row0), hi = min(G, p.N - row0);
+      const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
+      const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
+      const bool none = !fast && !__any_sync(0xffffffffu, act);
       if (!mbar_wait(bar_afull(sb), (i >> 1) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
         ok = false;
         continue;
@@ -314,10 +319,6 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
       tc_fence_after();
       const uint32_t st_addr = lane_addr + sb * 64;         // S^T, then P^T
       const uint32_t dp_addr = lane_addr + 128 + sb * 64;   // dP^T, then dS^T
-      const int lo = max(0, -row0), hi = min(G, p.N - row0);
-      const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
-      const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
-      const bool none = !fast && !__any_sync(0xffffffffu, act);
       const float4* l4 = reinterpret_cast<const float4*>(cols + (STEP ? cbeg : 0));
       const float4* d4 = reinterpret_cast<const float4*>(cols + (STEP ? 64 + cbeg : 16));
       // P^T / dS^T of the thread's 16 columns go over the first 8 of them in

@@ -279,17 +279,18 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
     for (int i = wg; ok && i < n; i += 2) {
       // A(i) complete also means B(i-2) has retired (same issue order), so the
       // dS columns of this buffer are free again.
+      // what the tile's columns mean to this row: worked out before the wait
+      const int tok0 = static_cast<int>(un.ids[i]) * G - p.kv_pad_head;
+      const int lo = max(0, -tok0), hi = min(G, p.N - tok0);
+      const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
+      const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
+      const bool none = !fast && !__any_sync(0xffffffffu, act);   // a block of the other groups: dS = 0
       if (!mbar_wait(bar_afull(wg), (i >> 1) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
         ok = false;
         break;
       }
       tc_fence_after();
-      const int tok0 = static_cast<int>(un.ids[i]) * G - p.kv_pad_head;
-      const int lo = max(0, -tok0), hi = min(G, p.N - tok0);
-      const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
-      const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
       uint32_t sv[32], dv[32], pk[16];
-      const bool none = !fast && !__any_sync(0xffffffffu, act);   // a block of the other groups: dS = 0
       if (!none) {
         tmem_ld32(s_addr + cbeg, sv);
         tmem_ld32(dp_addr + cbeg, dv);
