@@ -21,10 +21,37 @@ struct UnionScratch {
   unsigned uni[AT_WORDS];                // their union
   uint16_t pre[AT_WORDS];                // listed blocks below each word, within its warp's words
   uint16_t ids[AT_MAX_BLOCKS];           // union, ascending
-  uint8_t masks[AT_MAX_BLOCKS];          // bit g set: group g lists the block
+  __align__(4) uint8_t masks[AT_MAX_BLOCKS];          // bit g set: group g lists the block
   int warp_tot[4];
-  int total;
 };
+
+// The tiles that a CTA walks are `sub` listed blocks wide, 1 or 2: blocks of 32 rows
+// are walked two at a time as tiles of 64, with a mask byte for either half, since a
+// 128 x 32 tile costs nearly what a 128 x 64 tile does (the barriers, TMEM accesses
+// and UMMA overheads per tile are the same).
+
+// What tile i of the union (its first token is tok0, `width` tokens) holds for a row
+// of group `grp`: columns lo .. hi - 1, none unless `on`.  With sub 1 lo and hi are
+// the same for all threads, and stay in uniform registers.
+struct ColSpan {
+  int lo, hi;
+  bool on;
+};
+// `sub` as a template parameter of the kernels that walk 64-row tiles: the run-time
+// choice cost 2 to 4 % of the dK/dV pair kernel.
+__device__ __forceinline__ ColSpan col_span(const UnionScratch& u, int i, int sub, int grp, int tok0,
+                                            int width, int N) {
+  ColSpan c = {max(0, -tok0), min(width, N - tok0), true};
+  if (sub == 1) {
+    c.on = (u.masks[i] >> grp) & 1;
+  } else {
+    const unsigned m = *reinterpret_cast<const uint16_t*>(&u.masks[2 * i]) >> grp;
+    if (!(m & 1u)) c.lo = max(c.lo, 32);
+    if (!(m & 256u)) c.hi = min(c.hi, 32);
+  }
+  c.on = c.on && c.hi > c.lo;
+  return c;
+}
 
 // How the caller's lists map to the blocks a kernel works on.  Lists over q
 // blocks or kv blocks of more rows than the kernels take are read as lists over
@@ -36,17 +63,19 @@ struct ListMap {
   int q_shift, q_off, kv_shift, kv_off;
 };
 
-// Lists the bits of u.bm in ascending order (ids, masks, total).  All threads
-// of the CTA call this, after a barrier behind the last write to u.bm.
+// Lists the bits of u.bm in ascending order (ids, masks; `sub` bits make one
+// entry).  All threads of the CTA call this, after a barrier behind the last write
+// to u.bm.  Returns the number of entries.
 // Expanding one bit per thread (128 threads walking a word each took as many
 // serial steps as the densest word has bits) keeps this at four barriers.
-__device__ __forceinline__ int list_union(UnionScratch& u, int words) {
+__device__ __forceinline__ int list_union(UnionScratch& u, int words, int sub) {
   const int tid = threadIdx.x, nthr = blockDim.x;
   if (tid < AT_WORDS) {
     unsigned uni = 0;
     if (tid < words) {
 #pragma unroll
       for (int g = 0; g < AT_MAX_GROUPS; g++) uni |= u.bm[g][tid];
+      if (sub == 2) uni = (uni | (uni >> 1)) & 0x55555555u;
     }
     const int c = __popc(uni), lane = tid & 31;
     int inc = c;
@@ -67,11 +96,20 @@ __device__ __forceinline__ int list_union(UnionScratch& u, int words) {
     if ((uni >> b) & 1u) {
       const int pos = u.pre[wd] + (wp > 0 ? t0 : 0) + (wp > 1 ? t1 : 0) + (wp > 2 ? t2 : 0) +
                       __popc(uni & ((1u << b) - 1u));
-      unsigned mk = 0;
+      unsigned mk = 0;   // both halves' bits when sub is 2: bits g and 8 + g
 #pragma unroll
-      for (int g = 0; g < AT_MAX_GROUPS; g++) mk |= ((u.bm[g][wd] >> b) & 1u) << g;
-      u.ids[pos] = static_cast<uint16_t>(x);
-      u.masks[pos] = static_cast<uint8_t>(mk);
+      for (int g = 0; g < AT_MAX_GROUPS; g++) {
+        const unsigned bits = u.bm[g][wd] >> b;
+        mk |= (bits & 1u) << g;
+        if (sub == 2) mk |= (bits & 2u) << (7 + g);
+      }
+      if (sub == 1) {
+        u.ids[pos] = static_cast<uint16_t>(x);
+        u.masks[pos] = static_cast<uint8_t>(mk);
+      } else {
+        u.ids[pos] = static_cast<uint16_t>(x >> 1);
+        *reinterpret_cast<uint16_t*>(&u.masks[2 * pos]) = static_cast<uint16_t>(mk);
+      }
     }
   }
   __syncthreads();
@@ -88,7 +126,8 @@ __device__ __forceinline__ void clear_bitmaps(UnionScratch& u) {
 // ids >= num_blocks reported through `status`.  Returns the union size.
 __device__ __forceinline__ int build_union(UnionScratch& u, const int32_t* lists, int first,
                                            int groups, int width, const int32_t* counts,
-                                           int num_blocks, const ListMap& lm, int* status) {
+                                           int num_blocks, int sub, const ListMap& lm,
+                                           int* status) {
   const int tid = threadIdx.x, nthr = blockDim.x;
   __syncthreads();
   auto row = [&](int g) {
@@ -138,7 +177,7 @@ __device__ __forceinline__ int build_union(UnionScratch& u, const int32_t* lists
     }
   }
   __syncthreads();
-  return list_union(u, (num_blocks + 31) >> 5);
+  return list_union(u, (num_blocks + 31) >> 5, sub);
 }
 
 // What the dQ kernel leaves for the dK/dV kernel in place of a reverse index:
@@ -163,41 +202,89 @@ __device__ __forceinline__ void write_tile_masks(const UnionScratch& u, uint8_t*
 // The same union as build_union, for kv blocks j0 .. j0 + groups - 1, read off
 // those bytes (after clear_bitmaps).  `masks` is the first tile's row of the
 // first of `heads` query heads that share the kv head, `head_stride` bytes
-// apart; entry ids run over the heads: head * span + q-block.
+// apart; listed blocks run over the heads: head * span + q-block.
 __device__ __forceinline__ int build_union_masks(UnionScratch& u, const uint8_t* masks, int stride,
                                                  int tiles, int per_tile, int j0, int groups,
-                                                 int heads, int64_t head_stride, int span) {
+                                                 int heads, int64_t head_stride, int span, int sub) {
   const int tid = threadIdx.x, nthr = blockDim.x;
-  // the bytes of a thread's (head, tile): one word where four kv blocks lie in one
-  const bool word = groups == 4 && (j0 & 3) == 0;
-  auto load = [&](int h, int t) -> unsigned {
-    const uint8_t* src = masks + h * head_stride + static_cast<int64_t>(t) * stride + j0;
+  // the bytes of a thread's (head, tile): words where the kv blocks fill whole ones
+  const bool word = (groups & 3) == 0 && (j0 & 3) == 0;
+  auto load = [&](int h, int t, int g) -> unsigned {
+    const uint8_t* src = masks + h * head_stride + static_cast<int64_t>(t) * stride + j0 + g;
     return word ? *reinterpret_cast<const unsigned*>(src) : src[0];
   };
-  const unsigned first = tid < tiles ? load(0, tid) : 0u;   // under the clearing of the bitmaps
+  const unsigned first = tid < tiles ? load(0, tid, 0) : 0u;   // under the clearing of the bitmaps
   __syncthreads();
   for (int h = 0; h < heads; h++) {
     for (int t = tid; t < tiles; t += nthr) {
       const int q = h * span + t * per_tile, wd = q >> 5, sh = q & 31;
-      const unsigned b = h == 0 && t == tid ? first : load(h, t);
-      if (word) {
+      for (int g = 0; g < groups; g += word ? 4 : 1) {
+        const unsigned b = h == 0 && t == tid && g == 0 ? first : load(h, t, g);
+        if (word) {
 #pragma unroll
-        for (int g = 0; g < 4; g++) {
-          const unsigned x = (b >> (8 * g)) & 255u;
-          if (x) atomicOr(&u.bm[g][wd], x << sh);
-        }
-      } else {
-        if (b) atomicOr(&u.bm[0][wd], b << sh);
-        const uint8_t* src = masks + h * head_stride + static_cast<int64_t>(t) * stride + j0;
-        for (int g = 1; g < groups; g++) {
-          const unsigned x = src[g];
-          if (x) atomicOr(&u.bm[g][wd], x << sh);
+          for (int x = 0; x < 4; x++) {
+            const unsigned m = (b >> (8 * x)) & 255u;
+            if (m) atomicOr(&u.bm[g + x][wd], m << sh);
+          }
+        } else if (b) {
+          atomicOr(&u.bm[g][wd], b << sh);
         }
       }
     }
   }
   __syncthreads();
-  return list_union(u, (heads * span) >> 5);
+  return list_union(u, (heads * span) >> 5, sub);
+}
+
+// Up to four tiles of the union that between them hold, for every group with a
+// list, at least one block of that list (the forward takes the rows' reference
+// exponents from them): the tile that most groups list, then the one that most of
+// the others list, and so on, ties to the first.  One warp calls this.  With wide
+// lists one tile serves all groups.
+struct CoverTiles {
+  int n;                                 // tiles
+  int entry[4];                          // their positions in the union
+  int8_t of[AT_MAX_GROUPS];              // group -> which of them, -1: none
+  int left;                              // groups with a list that none of the four holds
+};
+__device__ __forceinline__ void cover_tiles(const UnionScratch& u, int n, int groups, int sub,
+                                            CoverTiles& c) {
+  const int lane = threadIdx.x & 31;
+  auto mask = [&](int i) -> unsigned {
+    return sub == 1 ? u.masks[i] : u.masks[2 * i] | u.masks[2 * i + 1];
+  };
+  unsigned open = (1u << groups) - 1u;
+  if (lane < AT_MAX_GROUPS) c.of[lane] = -1;
+  __syncwarp();
+  int e = 0;
+  bool any = n > 0;
+  for (; e < 4 && open && any; e++) {
+    unsigned best = 0;   // groups served, then earlier first
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      const int i = i0 + lane;
+      const unsigned s = i < n ? __popc(mask(i) & open) : 0;
+      best = max(best, s ? (s << 16) | (0xffffu - static_cast<unsigned>(i)) : 0u);
+      if (__any_sync(0xffffffffu, (best >> 16) == __popc(open))) break;
+    }
+    best = __reduce_max_sync(0xffffffffu, best);
+    any = best != 0;
+    if (!any) break;
+    const int i = static_cast<int>(0xffffu - (best & 0xffffu));
+    const unsigned m = mask(i) & open;
+    if (lane < AT_MAX_GROUPS && ((m >> lane) & 1u)) c.of[lane] = static_cast<int8_t>(e);
+    if (lane == 0) c.entry[e] = i;
+    open &= ~m;
+  }
+  // `open` groups: no list at all, or none of the four tiles holds one of its blocks
+  unsigned listed = 0;
+  if (open && any)
+    for (int i = lane; i < n; i += 32) listed |= mask(i);
+  listed = __reduce_or_sync(0xffffffffu, listed);
+  if (lane == 0) {
+    c.n = e;
+    c.left = static_cast<int>(open & listed);
+  }
+  __syncwarp();
 }
 
 // two fp32 -> one 32-bit word of two 16-bit floats (element 0 in the low half)

@@ -74,6 +74,11 @@ inline int attn_grid(const ftk_attn& a, int limit, AttnGrid* out) {
   return FTK_OK;
 }
 
+// q and kv blocks of 64 or 32 rows are walked as 64-row tiles (see ColSpan)
+inline bool tiles_of_64(int g, int kvb) {
+  return (g == 64 || g == 32) && (kvb == 64 || kvb == 32);
+}
+
 // q blocks per 128-row tile
 inline int attn_groups(int g) { return std::max(1, std::min(AT_MAX_GROUPS, 128 / g)); }
 

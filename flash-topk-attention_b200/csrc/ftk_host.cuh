@@ -9,6 +9,7 @@
 
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 
 namespace ftk {
 
@@ -107,6 +108,15 @@ template <auto KERNEL>
 struct Kernel {
   static constexpr auto kernel = KERNEL;
 };
+
+// A run-time value 0 .. N - 1 as a compile-time one: f(std::integral_constant<int, value>)
+template <int N, typename F>
+inline int choose(int value, F&& f) {
+  if constexpr (N > 1) {
+    if (value < N - 1) return choose<N - 1>(value, f);
+  }
+  return f(std::integral_constant<int, N - 1>{});
+}
 
 // Launch that may overlap the tail of the stream's previous kernel.  Only for
 // kernels that call pdl_wait() in every block before they touch global memory.

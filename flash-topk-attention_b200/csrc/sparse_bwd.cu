@@ -34,7 +34,7 @@ constexpr int DQ_VST = 5;        // dQ kernel: V tiles in the ring (free once dP
 
 struct BwdParams {
   int N, H, D, QM, W, Mkv;
-  int g, kvb, q_pad_head, kv_pad_head;
+  int g, kvb, q_pad_head, kv_pad_head;   // rows per group and per tile (sub * listed block)
   int G, fmt, nstages;
   float scale, scale_log2;
   const int32_t* lists;      // dQ: [BH][list_rows][W]; dKV: reverse_idx [BH][Mkv][QM] or null
@@ -55,7 +55,8 @@ struct BwdParams {
   int* status;
   int kv_hdiv;               // query heads per kv head (grouped-query attention), 1 otherwise
   int heads;                 // dKV: query heads one CTA walks (kv_hdiv, or 1: one result per query head)
-  int span;                  // dKV with heads > 1: ids per head in the union (multiple of 32)
+  int span, span_tiles;      // dKV with heads > 1: q-blocks (a multiple of 32) and tiles per head
+  int sub;                   // listed blocks per tile: kv blocks (dQ), q-blocks (dKV)
   const int32_t* order;      // dKV: kv blocks by fan-in, heaviest first ([BH][Mkv]) or null
   int step;                  // dKV pair kernel at head dim 128: its STEP variant
   const int32_t* tile_order; // dKV: 128-row kv tiles by number of q-blocks, heaviest first, or null
@@ -306,7 +307,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   TileDelta<D> delta;
   if (D <= 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);
   const int n = build_union(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
-                            p.W, nullptr, p.Mkv, p.lm, p.status);
+                            p.W, nullptr, p.Mkv, p.sub, p.lm, p.status);
   if (D > 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);   // too many registers to hold across the union
   delta.finish(p, s_delta, bh, tile_row0, groups * p.g);
   if (p.masks)
@@ -496,8 +497,9 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       // dS columns of this buffer are free again.
       // what the tile's columns mean to this row: worked out before the wait
       const int tok0 = static_cast<int>(un.ids[i]) * p.kvb - p.kv_pad_head;
-      const int lo = max(0, -tok0), hi = min(p.kvb, p.N - tok0);
-      const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
+      const ColSpan cs = col_span(un, i, p.sub, grp, tok0, p.kvb, p.N);
+      const int lo = cs.lo, hi = cs.hi;
+      const bool act = row_valid && cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == p.kvb;
       const bool none = !fast && !__any_sync(0xffffffffu, act);
       if (!mbar_wait(bar_afull(wg), (i >> 1) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
@@ -611,21 +613,21 @@ __device__ __forceinline__ int dkv_union(UnionScratch& un, const BwdParams& p, i
   if (p.masks) {
     const int64_t per_head = static_cast<int64_t>(p.mask_tiles) * p.mask_stride;
     return build_union_masks(un, p.masks + bhq * per_head, p.mask_stride, p.mask_tiles, p.mask_g, j0,
-                             groups, p.heads, per_head, p.span);
+                             groups, p.heads, per_head, p.span, p.sub);
   }
   const int64_t kv_row = static_cast<int64_t>(bhq) * p.Mkv + j0;
   return build_union(un, p.lists + kv_row * p.QM, 0, groups, p.QM, p.counts + kv_row, p.QM,
-                     ListMap{0, 0, 0, 0}, p.status);
+                     p.sub, ListMap{0, 0, 0, 0}, p.status);
 }
 
-// Entry id of the union -> q-block, with the query head it belongs to (ids come
+// Entry id of the union -> q tile, with the query head it belongs to (ids come
 // in ascending order, head by head).  Without WALK ids are q-blocks.
 template <bool WALK>
 struct HeadWalk {
   int head = 0, first = 0;
   __device__ __forceinline__ int at(int id, const BwdParams& p) {
-    while (WALK && id - first >= p.span) {
-      first += p.span;
+    while (WALK && id - first >= p.span_tiles) {
+      first += p.span_tiles;
       head++;
     }
     return id - first;
@@ -938,8 +940,9 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
         continue;
       }
       tc_fence_after();
-      const int lo = max(0, -row0), hi = min(p.g, p.N - row0);
-      const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
+      const ColSpan cs = col_span(un, i, p.sub, grp, row0, p.g, p.N);
+      const int lo = cs.lo, hi = cs.hi;
+      const bool act = row_valid && cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == p.g;
       const bool none = !fast && !__any_sync(0xffffffffu, act);
       const float4* l4 = reinterpret_cast<const float4*>(s_lse2[wg][pb]);
@@ -1166,12 +1169,13 @@ static size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
   BwdPlan b{};
   int e = attn_grid(a, 64, &b.gr);
-  // head dim 256 with blocks other than 64 rows: the one-CTA kernels hold Q / dO (dQ)
-  // or K / V (dK, dV) of 256 columns in shared memory and have room for 32-row partner
-  // tiles only
-  if (a.D > 128 && (e || b.gr.g != 64 || b.gr.kvb != 64)) e = attn_grid(a, 32, &b.gr);
+  // head dim 256 with blocks other than 64 and 32 rows: the one-CTA kernels hold Q / dO
+  // (dQ) or K / V (dK, dV) of 256 columns in shared memory and have room for 32-row
+  // partner tiles only
+  if (a.D > 128 && (e || !tiles_of_64(b.gr.g, b.gr.kvb))) e = attn_grid(a, 32, &b.gr);
   if (e) return e;
   const AttnGrid& gr = b.gr;
+  const bool tiles64 = tiles_of_64(gr.g, gr.kvb);
   if (gr.g % 16 != 0) return FTK_ERR_UNSUPPORTED;
   if (gr.QM > AT_MAX_BLOCKS) return FTK_ERR_UNSUPPORTED;
   const int64_t BH = a.B * a.H;
@@ -1185,9 +1189,8 @@ static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
   // S^T and dP^T UMMAs read both operands from shared memory) and breaks even at
   // f = 1/4 (585 against 597 us).  At head dim 256 the pair kernels are several times
   // the faster per tile.
-  const bool rows64 = gr.g == 64 && gr.kvb == 64;
-  b.pair_dq = rows64 && (gr.kd == 256 || (gr.kd == 128 && 2 * gr.width >= gr.Mkv));
-  b.pair_dkv = rows64 && (gr.kd == 256 || (gr.kd == 128 && 4 * gr.width >= gr.Mkv));
+  b.pair_dq = tiles64 && (gr.kd == 256 || (gr.kd == 128 && 2 * gr.width >= gr.Mkv));
+  b.pair_dkv = tiles64 && (gr.kd == 256 || (gr.kd == 128 && 4 * gr.width >= gr.Mkv));
   // Query heads that share a kv head: walked one after the other by the CTA that
   // owns the kv rows, so that their sum stays in its fp32 accumulators, unless
   // that leaves SMs idle: waves of CTAs times heads per CTA against waves of one
@@ -1243,7 +1246,7 @@ static BwdParams bwd_params(const ftk_attn& a, const AttnGrid& gr, const float* 
   p.status = status;
   p.kv_hdiv = static_cast<int>(a.H / a.Hkv);
   p.heads = 1;
-  p.span = 1 << 30;
+  p.span = p.span_tiles = 1 << 30;
   return p;
 }
 
@@ -1262,6 +1265,8 @@ static int launch_dq(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, b
              v = {a.v, a.Hkv, a.sv_b, a.sv_n, a.sv_h};
   const unsigned bh = static_cast<unsigned>(a.B * a.H);
   p.G = attn_groups(p.g);
+  p.sub = tiles_of_64(p.g, p.kvb) && (pair || kd < 256) ? 64 / p.kvb : 1;
+  p.kvb *= p.sub;
   CUtensorMap tq, tdo, tk, tv;
   int e;
   if ((e = tmap_of(&tq, a, q, 128)) || (e = tmap_of(&tdo, a, dout, 128)) ||
@@ -1270,21 +1275,22 @@ static int launch_dq(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, b
   if (pair && (kd == 256 || !env_off("FTK_DQ_2CTA"))) {
     CUtensorMap tk32, tv32;
     if ((e = tmap_of(&tk32, a, k, 32)) || (e = tmap_of(&tv32, a, v, 32))) return e;
-    const dim3 grid(2 * ((p.QM + 3) / 4), bh);
+    const dim3 grid(2 * ((p.QM + 2 * p.G - 1) / (2 * p.G)), bh);
     auto go = [&](auto kernel_tag, size_t smem) -> int {
       constexpr auto kernel = decltype(kernel_tag)::kernel;
       if (int r = allow_smem<kernel>(smem)) return r;
       return launch_pdl(kernel, grid, BW_THREADS, smem, st, tq, tdo, tk, tk32, tv32, p);
     };
-    const bool bf = a.dtype == FTK_DTYPE_BF16;
-    if (kd == 256) {
-      const size_t smem = 1024 + 2 * B6_ROWS + static_cast<size_t>(DQ6_SLOTS) * B6_PIECE;
-      return bf ? go(Kernel<sparse_bwd_dq256_kernel<1>>{}, smem)
-                : go(Kernel<sparse_bwd_dq256_kernel<0>>{}, smem);
-    }
-    const size_t smem = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DQ2_STAGES) * 24576;
-    return bf ? go(Kernel<sparse_bwd_dq2_kernel<1>>{}, smem)
-              : go(Kernel<sparse_bwd_dq2_kernel<0>>{}, smem);
+    return choose<2>(a.dtype, [&](auto fmt) {
+      return choose<3>(p.sub, [&](auto sub) {
+        constexpr int F = decltype(fmt)::value, S = decltype(sub)::value == 2 ? 2 : 1;
+        return kd == 256
+                   ? go(Kernel<sparse_bwd_dq256_kernel<F, S>>{},
+                        1024 + 2 * B6_ROWS + static_cast<size_t>(DQ6_SLOTS) * B6_PIECE)
+                   : go(Kernel<sparse_bwd_dq2_kernel<F, S>>{},
+                        1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DQ2_STAGES) * 24576);
+      });
+    });
   }
   if ((e = tmap_of(&tv, a, v, p.kvb))) return e;
   const int nch = kd / 64;
@@ -1313,6 +1319,9 @@ static int launch_dkv(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, 
              v = {a.v, a.Hkv, a.sv_b, a.sv_n, a.sv_h};
   const unsigned slices = static_cast<unsigned>(a.B * a.H / p.heads);
   p.G = attn_groups(p.kvb);
+  p.sub = tiles_of_64(p.g, p.kvb) && (pair || kd < 256) ? 64 / p.g : 1;
+  p.g *= p.sub;
+  p.span_tiles = p.span / p.sub;
   CUtensorMap tq, tdo, tk, tv;
   int e;
   if ((e = tmap_of(&tq, a, q, p.g)) || (e = tmap_of(&tdo, a, dout, p.g)) ||
@@ -1321,39 +1330,30 @@ static int launch_dkv(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, 
   if (pair && (kd == 256 || !env_off("FTK_DKV_2CTA"))) {
     CUtensorMap tq32, tdo32;
     if ((e = tmap_of(&tq32, a, q, 32)) || (e = tmap_of(&tdo32, a, dout, 32))) return e;
-    const dim3 grid(2 * ((p.Mkv + 3) / 4), slices);
+    const dim3 grid(2 * ((p.Mkv + 2 * p.G - 1) / (2 * p.G)), slices);
     auto go = [&](auto kernel_tag, size_t smem) -> int {
       constexpr auto kernel = decltype(kernel_tag)::kernel;
       if (int r = allow_smem<kernel>(smem)) return r;
       return launch_pdl(kernel, grid, BW_THREADS, smem, st, tq, tdo, tq32, tdo32, tk, tv, p);
     };
-    const bool bf = a.dtype == FTK_DTYPE_BF16, walk = p.heads > 1;
-    if (kd == 256) {
-      const size_t smem_dv = 1024 + B6_ROWS + static_cast<size_t>(DV6_SLOTS) * B6_PIECE,
-                   smem_dk = 1024 + 2 * B6_ROWS + static_cast<size_t>(DQ6_SLOTS) * B6_PIECE;
-      if (bf) {
-        e = walk ? go(Kernel<sparse_bwd_dkv256_kernel<1, 1, true>>{}, smem_dv)
-                 : go(Kernel<sparse_bwd_dkv256_kernel<1, 1, false>>{}, smem_dv);
-        if (e) return e;
-        return walk ? go(Kernel<sparse_bwd_dkv256_kernel<1, 2, true>>{}, smem_dk)
-                    : go(Kernel<sparse_bwd_dkv256_kernel<1, 2, false>>{}, smem_dk);
-      }
-      e = walk ? go(Kernel<sparse_bwd_dkv256_kernel<0, 1, true>>{}, smem_dv)
-               : go(Kernel<sparse_bwd_dkv256_kernel<0, 1, false>>{}, smem_dv);
-      if (e) return e;
-      return walk ? go(Kernel<sparse_bwd_dkv256_kernel<0, 2, true>>{}, smem_dk)
-                  : go(Kernel<sparse_bwd_dkv256_kernel<0, 2, false>>{}, smem_dk);
-    }
-    const size_t smem = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DK2_STAGES) * 32768;
-    if (walk)
-      return bf ? (p.step ? go(Kernel<sparse_bwd_dkv2_kernel<1, true, true>>{}, smem)
-                          : go(Kernel<sparse_bwd_dkv2_kernel<1, true, false>>{}, smem))
-                : (p.step ? go(Kernel<sparse_bwd_dkv2_kernel<0, true, true>>{}, smem)
-                          : go(Kernel<sparse_bwd_dkv2_kernel<0, true, false>>{}, smem));
-    return bf ? (p.step ? go(Kernel<sparse_bwd_dkv2_kernel<1, false, true>>{}, smem)
-                        : go(Kernel<sparse_bwd_dkv2_kernel<1, false, false>>{}, smem))
-              : (p.step ? go(Kernel<sparse_bwd_dkv2_kernel<0, false, true>>{}, smem)
-                        : go(Kernel<sparse_bwd_dkv2_kernel<0, false, false>>{}, smem));
+    return choose<2>(a.dtype, [&](auto fmt) {
+      return choose<3>(p.sub, [&](auto sub) {
+        return choose<2>(p.heads > 1, [&](auto walk) {
+          constexpr int F = decltype(fmt)::value, S = decltype(sub)::value == 2 ? 2 : 1;
+          constexpr bool W = decltype(walk)::value;
+          if (kd == 256) {
+            int r = go(Kernel<sparse_bwd_dkv256_kernel<F, 1, W, S>>{},
+                       1024 + B6_ROWS + static_cast<size_t>(DV6_SLOTS) * B6_PIECE);
+            if (r) return r;
+            return go(Kernel<sparse_bwd_dkv256_kernel<F, 2, W, S>>{},
+                      1024 + 2 * B6_ROWS + static_cast<size_t>(DQ6_SLOTS) * B6_PIECE);
+          }
+          const size_t smem = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DK2_STAGES) * 32768;
+          return p.step ? go(Kernel<sparse_bwd_dkv2_kernel<F, W, true, S>>{}, smem)
+                        : go(Kernel<sparse_bwd_dkv2_kernel<F, W, false, S>>{}, smem);
+        });
+      });
+    });
   }
   const int nch = kd / 64;
   const int stage_bytes = 2 * nch * p.g * 128;

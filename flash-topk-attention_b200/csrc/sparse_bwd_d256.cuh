@@ -50,7 +50,7 @@ __device__ __forceinline__ void in_piece_order(int n, int ahead, First&& first, 
   }
 }
 
-template <int FMT>
+template <int FMT, int SUB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(BW_THREADS, 1)
 sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
                         const __grid_constant__ CUtensorMap tm_do,
@@ -73,11 +73,12 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
-  const int m0 = (blockIdx.x >> 1) * 4;       // first of the pair's four q-blocks
+  const int per = 128 / p.g;                  // q-blocks (of 64 or 32 rows) per CTA
+  const int m0 = (blockIdx.x >> 1) * 2 * per; // first of the pair's q-blocks
   const int bh = blockIdx.y;
   const int b_idx = bh / p.H, h_idx = bh - b_idx * p.H;
-  const int groups = min(4, p.QM - m0);
-  const int tile_row0 = (m0 + 2 * static_cast<int>(rank)) * G - p.q_pad_head;   // my 128 rows
+  const int groups = min(2 * per, p.QM - m0);
+  const int tile_row0 = m0 * p.g + 128 * static_cast<int>(rank) - p.q_pad_head;   // my 128 rows
 
   const uint32_t bar_q = smem_u32(&bars[0]);         // my Q / dO tiles
   const uint32_t bar_peer_q = smem_u32(&bars[1]);    // CTA 0: CTA 1's
@@ -118,7 +119,7 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
   cluster_arrive();
   pdl_wait();
   pdl_launch();
-  const int mine = min(2, groups - 2 * static_cast<int>(rank));   // q-blocks of my tile, if any
+  const int mine = min(per, groups - per * static_cast<int>(rank));   // q-blocks of my tile, if any
   if (tid == 0) {   // under the building of the union
     mbar_expect_tx(bar_q, 2 * B6_ROWS);
     for (int c = 0; c < NCH; c++) {
@@ -128,14 +129,14 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
   }
   TileDelta<D> delta;
   const int n = build_union(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
-                            p.W, nullptr, p.Mkv, p.lm, p.status);
-  delta.load(p, b_idx, h_idx, tile_row0, mine * G);   // 256 columns: too many registers to hold across the union
-  delta.finish(p, s_delta, bh, tile_row0, mine * G);
+                            p.W, nullptr, p.Mkv, SUB, p.lm, p.status);
+  delta.load(p, b_idx, h_idx, tile_row0, mine * p.g);   // 256 columns: too many registers to hold across the union
+  delta.finish(p, s_delta, bh, tile_row0, mine * p.g);
   if (p.masks && mine > 0)
     write_tile_masks(un,
-                     p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + m0 / 2 + rank) *
+                     p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + blockIdx.x) *
                                    p.mask_stride,
-                     p.mask_stride, 2 * static_cast<int>(rank), mine);
+                     p.mask_stride, per * static_cast<int>(rank), mine);
   tc_fence_before();
   __syncthreads();
   cluster_wait();            // barriers of both CTAs are initialised before anyone signals them
@@ -280,7 +281,7 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int colhalf = (cw >> 2) & 1;
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
-    const int grp = 2 * static_cast<int>(rank) + r / G;   // q-block of the pair
+    const int grp = per * static_cast<int>(rank) + r / p.g;   // q-block of the pair
     const int qrow = tile_row0 + r;
     const bool row_valid = (grp < groups) && qrow >= 0 && qrow < p.N;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -301,8 +302,9 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
       }
       tc_fence_after();
       const int tok0 = static_cast<int>(un.ids[i]) * G - p.kv_pad_head;
-      const int lo = max(0, -tok0), hi = min(G, p.N - tok0);
-      const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
+      const ColSpan cs = col_span(un, i, SUB, grp, tok0, G, p.N);
+      const int lo = cs.lo, hi = cs.hi;
+      const bool act = row_valid && cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
       const bool none = !fast && !__any_sync(0xffffffffu, act);
       uint32_t sv[32], dv[32], pk[16];
@@ -374,7 +376,7 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
 // MODE 1 = dV (K resident), MODE 2 = dK (K and V resident); WALK as in
 // sparse_bwd_dkv2_kernel.  TMEM: MODE 1 S^T[4] 0/64/128/192, MODE 2 S^T[2] 0/64,
 // dP^T[2] 128/192; accumulator 256..511.
-template <int FMT, int MODE, bool WALK>
+template <int FMT, int MODE, bool WALK, int SUB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(BW_THREADS, 1)
 sparse_bwd_dkv256_kernel(const __grid_constant__ CUtensorMap tm_q,
                          const __grid_constant__ CUtensorMap tm_do,
@@ -404,13 +406,14 @@ sparse_bwd_dkv256_kernel(const __grid_constant__ CUtensorMap tm_q,
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
-  const int j0 = (blockIdx.x >> 1) * 4;      // first of the pair's four kv blocks
+  const int per = 128 / p.kvb;               // kv blocks (of 64 or 32 rows) per CTA
+  const int j0 = (blockIdx.x >> 1) * 2 * per;   // first of the pair's kv blocks
   const int bh = blockIdx.y;
   const int slices = WALK ? p.H / p.heads : p.H;
   const int b_idx = bh / slices, h_idx = (bh - b_idx * slices) * (WALK ? p.heads : 1);
   const int bhq = WALK ? b_idx * p.H + h_idx : bh;
-  const int groups = min(4, p.Mkv - j0);     // kv blocks of the pair that exist
-  const int tile_tok0 = (j0 + 2 * static_cast<int>(rank)) * G - p.kv_pad_head;   // my 128 rows
+  const int groups = min(2 * per, p.Mkv - j0);   // kv blocks of the pair that exist
+  const int tile_tok0 = j0 * p.kvb + 128 * static_cast<int>(rank) - p.kv_pad_head;   // my 128 rows
 
   const uint32_t bar_kv = smem_u32(&bars[0]);        // my K / V tiles
   const uint32_t bar_peer_kv = smem_u32(&bars[1]);   // CTA 0: CTA 1's
@@ -615,7 +618,7 @@ sparse_bwd_dkv256_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int gw = cw >> 2;                  // MODE 1: S^T buffer; MODE 2: quarter of the columns
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
-    const int grp = 2 * static_cast<int>(rank) + r / G;   // kv block of the pair
+    const int grp = per * static_cast<int>(rank) + r / p.kvb;   // kv block of the pair
     const int tok = tile_tok0 + r;
     const bool row_valid = (grp < groups) && tok >= 0 && tok < p.N;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -661,8 +664,9 @@ sparse_bwd_dkv256_kernel(const __grid_constant__ CUtensorMap tm_q,
         continue;
       }
       tc_fence_after();
-      const int lo = max(0, -row0), hi = min(G, p.N - row0);
-      const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
+      const ColSpan cs = col_span(un, i, SUB, grp, row0, G, p.N);
+      const int lo = cs.lo, hi = cs.hi;
+      const bool act = row_valid && cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
       const bool none = !fast && !__any_sync(0xffffffffu, act);
       const float4* l4 = reinterpret_cast<const float4*>(nl);

@@ -50,7 +50,7 @@ __device__ __forceinline__ uint32_t pack2f(float a, float b) {
 // its buffer is free earlier (28.8 against 29.1 ms there, 3.76 against 3.98 ms at B = 4,
 // N = 8192, H = 16); with short lists most warps of a tile have nothing to do and
 // should run ahead (610 -> 569 us at W = 16 of 64 blocks, four heads per kv head).
-template <int FMT, bool WALK, bool STEP>
+template <int FMT, bool WALK, bool STEP, int SUB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(BW_THREADS, 1)
 sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
                        const __grid_constant__ CUtensorMap tm_do,
@@ -80,14 +80,15 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
-  const int j0 = (blockIdx.x >> 1) * 4;      // first of the pair's four kv blocks
+  const int per = 128 / p.kvb;               // kv blocks (of 64 or 32 rows) per CTA
+  const int j0 = (blockIdx.x >> 1) * 2 * per;   // first of the pair's kv blocks
   const int bh = blockIdx.y;
   // slice = (batch, first of the query heads this pair walks)
   const int slices = WALK ? p.H / p.heads : p.H;
   const int b_idx = bh / slices, h_idx = (bh - b_idx * slices) * (WALK ? p.heads : 1);
   const int bhq = WALK ? b_idx * p.H + h_idx : bh;
-  const int groups = min(4, p.Mkv - j0);     // kv blocks of the pair that exist
-  const int tile_tok0 = (j0 + 2 * static_cast<int>(rank)) * G - p.kv_pad_head;   // my 128 rows
+  const int groups = min(2 * per, p.Mkv - j0);   // kv blocks of the pair that exist
+  const int tile_tok0 = j0 * p.kvb + 128 * static_cast<int>(rank) - p.kv_pad_head;   // my 128 rows
 
   const uint32_t bar_kv = smem_u32(&bars[0]);        // my K / V tiles
   const uint32_t bar_peer_kv = smem_u32(&bars[1]);   // CTA 0: CTA 1's K / V tiles
@@ -262,7 +263,7 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int colq = cw >> 2;
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
-    const int grp = 2 * static_cast<int>(rank) + r / G;   // kv block of the pair
+    const int grp = per * static_cast<int>(rank) + r / p.kvb;   // kv block of the pair
     const int tok = tile_tok0 + r;
     const bool row_valid = (grp < groups) && tok >= 0 && tok < p.N;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -308,8 +309,9 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
       fetch(i + 1, l2_next, dl_next);
       if (!ok) continue;
       // what the tile's columns mean to this row: worked out before the wait
-      const int lo = max(0, -row0), hi = min(G, p.N - row0);
-      const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
+      const ColSpan cs = col_span(un, i, SUB, grp, row0, G, p.N);
+      const int lo = cs.lo, hi = cs.hi;
+      const bool act = row_valid && cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
       const bool none = !fast && !__any_sync(0xffffffffu, act);
       if (!mbar_wait(bar_afull(sb), (i >> 1) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {

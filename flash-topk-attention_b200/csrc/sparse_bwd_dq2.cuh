@@ -25,7 +25,7 @@ constexpr int DQ2_STAGES = 5;
 // TMEM columns per CTA: Q 0..63, dO 64..127, S[2] 128/192, dP[2] 256/320 (dS
 // over their first half), dQ 384..   Shared memory per CTA: Q 32 KB, dO 32 KB,
 // 5 stages of [K rows-half 8 KB][V rows-half 8 KB][K d-half 8 KB].
-template <int FMT>
+template <int FMT, int SUB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(BW_THREADS, 1)
 sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
                       const __grid_constant__ CUtensorMap tm_do,
@@ -52,11 +52,12 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
-  const int m0 = (blockIdx.x >> 1) * 4;       // first of the pair's four q-blocks
+  const int per = 128 / p.g;                  // q-blocks (of 64 or 32 rows) per CTA
+  const int m0 = (blockIdx.x >> 1) * 2 * per; // first of the pair's q-blocks
   const int bh = blockIdx.y;
   const int b_idx = bh / p.H, h_idx = bh - b_idx * p.H;
-  const int groups = min(4, p.QM - m0);
-  const int tile_row0 = (m0 + 2 * static_cast<int>(rank)) * G - p.q_pad_head;   // my 128 rows
+  const int groups = min(2 * per, p.QM - m0);
+  const int tile_row0 = m0 * p.g + 128 * static_cast<int>(rank) - p.q_pad_head;   // my 128 rows
 
   const uint32_t bar_q = smem_u32(&bars[0]);         // my Q / dO tiles in shared memory
   const uint32_t bar_qt = smem_u32(&bars[1]);        // CTA 0: Q / dO of both CTAs sit in TMEM
@@ -98,7 +99,7 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
   cluster_arrive();
   pdl_wait();
   pdl_launch();
-  const int mine = min(2, groups - 2 * static_cast<int>(rank));   // q-blocks of my tile, if any
+  const int mine = min(per, groups - per * static_cast<int>(rank));   // q-blocks of my tile, if any
   if (tid == 0) {   // under the building of the union
     mbar_expect_tx(bar_q, 2 * ROW_TILE_BYTES);
     for (int c = 0; c < NCH; c++) {
@@ -107,15 +108,15 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
   }
   TileDelta<D> delta;
-  delta.load(p, b_idx, h_idx, tile_row0, mine * G);
+  delta.load(p, b_idx, h_idx, tile_row0, mine * p.g);
   const int n = build_union(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
-                            p.W, nullptr, p.Mkv, p.lm, p.status);
-  delta.finish(p, s_delta, bh, tile_row0, mine * G);
+                            p.W, nullptr, p.Mkv, SUB, p.lm, p.status);
+  delta.finish(p, s_delta, bh, tile_row0, mine * p.g);
   if (p.masks && mine > 0)
     write_tile_masks(un,
-                     p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + m0 / 2 + rank) *
+                     p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + blockIdx.x) *
                                    p.mask_stride,
-                     p.mask_stride, 2 * static_cast<int>(rank), mine);
+                     p.mask_stride, per * static_cast<int>(rank), mine);
   tc_fence_before();
   __syncthreads();
   cluster_wait();            // barriers of both CTAs are initialised before anyone signals them
@@ -236,7 +237,7 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int colhalf = (cw >> 2) & 1;
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
-    const int grp = 2 * static_cast<int>(rank) + r / G;   // q-block of the pair
+    const int grp = per * static_cast<int>(rank) + r / p.g;   // q-block of the pair
     const int qrow = tile_row0 + r;
     const bool row_valid = (grp < groups) && qrow >= 0 && qrow < p.N;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -281,8 +282,9 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
       // dS columns of this buffer are free again.
       // what the tile's columns mean to this row: worked out before the wait
       const int tok0 = static_cast<int>(un.ids[i]) * G - p.kv_pad_head;
-      const int lo = max(0, -tok0), hi = min(G, p.N - tok0);
-      const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
+      const ColSpan cs = col_span(un, i, SUB, grp, tok0, G, p.N);
+      const int lo = cs.lo, hi = cs.hi;
+      const bool act = row_valid && cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
       const bool none = !fast && !__any_sync(0xffffffffu, act);   // a block of the other groups: dS = 0
       if (!mbar_wait(bar_afull(wg), (i >> 1) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {

@@ -61,6 +61,7 @@ struct FwdParams {
   int tiles_x, tiles;   // 128-row tiles per slice, and of all slices
   int D;                // columns of a row of O (the kernel's head dim less its padding)
   int out_f32;          // O is float32 (the 16-bit result, widened)
+  int sub;              // listed kv blocks per tile (pipelined kernels)
   ListMap lm;
 };
 
@@ -172,7 +173,7 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   }
   clear_bitmaps(un);
   const int n = build_union(un, p.merged + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
-                            p.W, nullptr, p.Mkv, p.lm, p.status);
+                            p.W, nullptr, p.Mkv, 1, p.lm, p.status);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -548,24 +549,34 @@ static int tmap_rows(CUtensorMap* out, const ftk_attn& a, char which, int rows) 
                           64, rows);
 }
 
-template <int D, int FMT>
+template <int D>
 static int launch_fwd_pipe(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                            const FwdParams& p, int64_t BH, cudaStream_t st) {
   constexpr int NCH = D / 64;
   const size_t smem = 1024 + NCH * 128 * 128 +
                       static_cast<size_t>(FP_KST + FP_VST) * NCH * 64 * 128;
-  if (int e = allow_smem<sparse_fwd_pipe_kernel<D, FMT>>(smem)) return e;
-  return launch_pdl(sparse_fwd_pipe_kernel<D, FMT>,
-                    dim3(p.tiles_x, static_cast<unsigned>(BH)), FP_THREADS, smem, st, tq, tk, tv, p);
+  return choose<2>(p.fmt, [&](auto fmt) {
+    return choose<3>(p.sub, [&](auto sub) {
+      constexpr int F = decltype(fmt)::value, S = decltype(sub)::value == 2 ? 2 : 1;
+      if (int e = allow_smem<sparse_fwd_pipe_kernel<D, F, S>>(smem)) return e;
+      return launch_pdl(sparse_fwd_pipe_kernel<D, F, S>, dim3(p.tiles_x, static_cast<unsigned>(BH)),
+                        FP_THREADS, smem, st, tq, tk, tv, p);
+    });
+  });
 }
 
-template <int D, int FMT>
+template <int D>
 static int launch_fwd_pipe2(const CUtensorMap& tq, const CUtensorMap& tk32, const CUtensorMap& tv,
                             const FwdParams& p, int64_t BH, cudaStream_t st) {
-  if (int e = allow_smem<sparse_fwd_pipe2_kernel<D, FMT>>(fp2_smem(D))) return e;
-  return launch_pdl(sparse_fwd_pipe2_kernel<D, FMT>,
-                    dim3(2 * ((p.QM + 3) / 4), static_cast<unsigned>(BH)), FP_THREADS, fp2_smem(D),
-                    st, tq, tk32, tv, p);
+  return choose<2>(p.fmt, [&](auto fmt) {
+    return choose<3>(p.sub, [&](auto sub) {
+      constexpr int F = decltype(fmt)::value, S = decltype(sub)::value == 2 ? 2 : 1;
+      if (int e = allow_smem<sparse_fwd_pipe2_kernel<D, F, S>>(fp2_smem(D))) return e;
+      return launch_pdl(sparse_fwd_pipe2_kernel<D, F, S>,
+                        dim3(2 * ((p.tiles_x + 1) / 2), static_cast<unsigned>(BH)), FP_THREADS,
+                        fp2_smem(D), st, tq, tk32, tv, p);
+    });
+  });
 }
 
 template <int D>
@@ -630,15 +641,16 @@ static int attn_fwd(const ftk_attn& a, const AttnGrid& gr, void* o, int64_t so_b
   CUtensorMap tq, tk, tv;
   int e;
   if ((e = tmap_rows(&tq, a, 'q', 128))) return e;
-  if ((e = tmap_rows(&tk, a, 'k', gr.kvb))) return e;
-  if ((e = tmap_rows(&tv, a, 'v', gr.kvb))) return e;
-  // 64-row kv blocks, q blocks of 64 or 32 rows and a workspace: the
-  // pipelined kernel runs first and the exact kernel redoes the tiles it flags.
+  // q and kv blocks of 64 or 32 rows and a workspace: the pipelined kernel runs
+  // first and the exact kernel redoes the tiles it flags.
   const char* env = getenv("FTK_FWD_PIPE");
-  // (Head dim 256: q blocks of 64 rows only, the pair kernel.)
-  const bool pipe = gr.kvb == 64 && (gr.g == 64 || (gr.g == 32 && gr.kd <= 128)) && workspace &&
+  const bool pipe = tiles_of_64(gr.g, gr.kvb) && workspace &&
                     workspace_bytes >= fwd_workspace(BH, gr.QM, gr.g) && !(env && env[0] == '0');
   if (pipe) {
+    p.sub = 64 / gr.kvb;
+    p.kvb = 64;
+    if ((e = tmap_rows(&tk, a, 'k', 64))) return e;
+    if ((e = tmap_rows(&tv, a, 'v', 64))) return e;
     p.redo_out = static_cast<int*>(workspace);
     const char* env2 = getenv("FTK_FWD_2CTA");
     // Pairs walk the union of four lists where one CTA walks that of two, at 0.9 of
@@ -648,27 +660,23 @@ static int attn_fwd(const ftk_attn& a, const AttnGrid& gr, void* o, int64_t so_b
     // without).
     // Head dim 256 takes pairs whatever the lists: four disjoint lists cost twice
     // the tiles of two, the one-CTA kernel three times the cycles per tile.
-    if (gr.kd == 256) {
-      CUtensorMap tk32;
-      if ((e = tmap_rows(&tk32, a, 'k', 32))) return e;
-      e = a.dtype == FTK_DTYPE_BF16 ? launch_fwd_pipe2<256, 1>(tq, tk32, tv, p, BH, st)
-                                    : launch_fwd_pipe2<256, 0>(tq, tk32, tv, p, BH, st);
-    } else if (gr.kd == 128 && gr.g == 64 && 2 * gr.width >= gr.Mkv && !(env2 && env2[0] == '0')) {
-      CUtensorMap tk32;
-      if ((e = tmap_rows(&tk32, a, 'k', 32))) return e;
-      e = a.dtype == FTK_DTYPE_BF16 ? launch_fwd_pipe2<128, 1>(tq, tk32, tv, p, BH, st)
-                                    : launch_fwd_pipe2<128, 0>(tq, tk32, tv, p, BH, st);
-    } else if (a.dtype == FTK_DTYPE_BF16) {
-      e = (gr.kd == 64) ? launch_fwd_pipe<64, 1>(tq, tk, tv, p, BH, st)
-                        : launch_fwd_pipe<128, 1>(tq, tk, tv, p, BH, st);
-    } else {
-      e = (gr.kd == 64) ? launch_fwd_pipe<64, 0>(tq, tk, tv, p, BH, st)
-                        : launch_fwd_pipe<128, 0>(tq, tk, tv, p, BH, st);
-    }
+    CUtensorMap tk32;
+    if ((e = tmap_rows(&tk32, a, 'k', 32))) return e;
+    if (gr.kd == 256)
+      e = launch_fwd_pipe2<256>(tq, tk32, tv, p, BH, st);
+    else if (gr.kd == 128 && 2 * gr.width >= gr.Mkv && !(env2 && env2[0] == '0'))
+      e = launch_fwd_pipe2<128>(tq, tk32, tv, p, BH, st);
+    else
+      e = gr.kd == 64 ? launch_fwd_pipe<64>(tq, tk, tv, p, BH, st)
+                      : launch_fwd_pipe<128>(tq, tk, tv, p, BH, st);
     if (e) return e;
     p.redo_out = nullptr;
     p.redo_in = static_cast<const int*>(workspace);
   }
+  p.sub = 1;
+  p.kvb = gr.kvb;
+  if ((e = tmap_rows(&tk, a, 'k', gr.kvb))) return e;
+  if ((e = tmap_rows(&tv, a, 'v', gr.kvb))) return e;
   if (gr.kd == 64) return launch_fwd<64>(tq, tk, tv, p, st);
   if (gr.kd == 256) return launch_fwd<256>(tq, tk, tv, p, st);
   return launch_fwd<128>(tq, tk, tv, p, st);

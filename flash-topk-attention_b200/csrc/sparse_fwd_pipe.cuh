@@ -43,7 +43,7 @@ __device__ __forceinline__ uint32_t pack16(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <int D, int FMT>
+template <int D, int FMT, int SUB>
 __global__ void __launch_bounds__(FP_THREADS, 1)
 sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
                        const __grid_constant__ CUtensorMap tm_k,
@@ -64,7 +64,7 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
   __shared__ int s_ovf;
-  __shared__ int s_first[4];
+  __shared__ CoverTiles s_pro;
   __shared__ float s_l[FP_GROUPS][128];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -118,44 +118,18 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
   pdl_wait();
   pdl_launch();
   const int n = build_union(un, p.merged + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
-                            p.W, nullptr, p.Mkv, p.lm, p.status);
-  // lowest listed block of each q-block: its scores give the rows' reference
-  if (warp < 4) {
-    int best = 0x7fffffff;
-    if (warp < groups) {
-#pragma unroll
-      for (int q = 0; q < AT_WORDS / 32; q++) {
-        const unsigned wv = un.bm[warp][q * 32 + lane];
-        if (wv && best == 0x7fffffff) best = (q * 32 + lane) * 32 + __ffs(wv) - 1;
-      }
-    }
-    best = __reduce_min_sync(0xffffffffu, best);
-    if (lane == 0) s_first[warp] = (best == 0x7fffffff) ? -1 : best;
-  }
+                            p.W, nullptr, p.Mkv, SUB, p.lm, p.status);
+  // tiles whose scores give the rows their reference exponents
+  if (warp == 2) cover_tiles(un, n, groups, SUB, s_pro);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
   WaitCtx w{&abort_flag, p.status};
 
-  // prologue entries: one per q-block of the tile (two of 64 rows or four of
-  // 32) with a non-empty list; entry e goes through S buffer e
-  int npro = 0;
-  int pro_id[4] = {0, 0, 0, 0};
-  int pro_buf[4] = {-1, -1, -1, -1};
-#pragma unroll
-  for (int g = 0; g < 4; g++) {
-    if (g < groups && s_first[g] >= 0) {
-#pragma unroll
-      for (int e = 0; e < 4; e++)
-        if (e == npro) pro_id[e] = s_first[g];
-      pro_buf[g] = npro;
-      npro++;
-    }
-  }
-  auto pro_block = [&](int e) {
-    return e == 0 ? pro_id[0] : e == 1 ? pro_id[1] : e == 2 ? pro_id[2] : pro_id[3];
-  };
+  // prologue entry e goes through S buffer e
+  const int npro = s_pro.n;
+  auto pro_block = [&](int e) { return static_cast<int>(un.ids[s_pro.entry[e]]); };
 
   if (warp == 0) {
     // ------------------------------------------------------- TMA producer
@@ -300,15 +274,15 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
       // Every warp waits for every prologue buffer, also the ones it does not
       // read: its later parity waits on those buffers must not start while
       // their first phase is still open.
-      const int pb = grp == 0 ? pro_buf[0] : grp == 1 ? pro_buf[1] : grp == 2 ? pro_buf[2]
-                                                                               : pro_buf[3];
+      const int pb = s_pro.of[grp];
       for (int e = 0; ok && e < npro; e++)
         ok = mbar_wait(bar_sfull(e), 0, w, FTK_DEV_TIMEOUT_CONSUMER);
       if (ok && pb >= 0) {
         {
           tc_fence_after();
           const int tok0 = pro_block(pb) * KVB - p.kv_pad_head;
-          const int lo = max(0, -tok0), hi = min(KVB, p.N - tok0);
+          const ColSpan cs = col_span(un, s_pro.entry[pb], SUB, grp, tok0, KVB, p.N);
+          const int lo = cs.lo, hi = cs.hi;
           uint32_t v0[32], v1[32];
           tmem_ld32(lane_addr + FP_COL_S + pb * 64, v0);
           tmem_ld32(lane_addr + FP_COL_S + pb * 64 + 32, v1);
@@ -338,8 +312,9 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
       }
       tc_fence_after();
       const int tok0 = static_cast<int>(un.ids[i]) * KVB - p.kv_pad_head;
-      const int lo = max(0, -tok0), hi = min(KVB, p.N - tok0);
-      const bool act = row_valid && ((un.masks[i] >> grp) & 1) && hi > lo;
+      const ColSpan cs = col_span(un, i, SUB, grp, tok0, KVB, p.N);
+      const int lo = cs.lo, hi = cs.hi;
+      const bool act = row_valid && cs.on;
       const bool any_act = __any_sync(0xffffffffu, act);
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == KVB;
 

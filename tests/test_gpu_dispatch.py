@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import cases
+import tolerance
 from oracle import ftk_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -143,3 +144,59 @@ def test_dkv_tile_order(ftk, monkeypatch, H, D, g, kvb):
     plain = _grads(ftk, t, merged, H, g, kvb, **kw)
     for a, b in zip(sorted_, plain):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("D,g,kvb,N,qpad,kvpad,W,dtype", [
+    (128, 32, 32, 1000, (9, 15), (20, 4), 24, "bf16"),    # wide lists: pairs of SMs, 8 + 8 groups
+    (128, 32, 32, 1000, (9, 15), (20, 4), 3, "fp16"),     # narrow lists: one CTA per tile
+    (128, 64, 32, 777, (0, 55), (31, 24), 20, "bf16"),    # odd number of kv blocks
+    (128, 32, 64, 700, (20, 16), (60, 8), 8, "bf16"),
+    (64, 32, 32, 500, (5, 7), (0, 12), 6, "bf16"),
+    (64, 64, 32, 330, (0, 54), (11, 11), 11, "fp16"),
+    (256, 32, 32, 520, (24, 0), (8, 16), 5, "bf16"),
+    (256, 32, 64, 300, (10, 10), (40, 44), 6, "fp16"),
+    (160, 64, 32, 384, (0, 0), (0, 0), 7, "bf16"),
+])
+def test_blocks_of_32_rows(ftk, D, g, kvb, N, qpad, kvpad, W, dtype):
+    """Blocks of 32 rows are walked as 64-row tiles with a mask per half: one half
+    listed, the other not, last tile half empty, several groups per tile, against
+    the oracle (fp16: the plain bound; bf16: with the rounding envelope)."""
+    H = 2
+    t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype=dtype, seed=33, do_seed=34))
+    x = {k: v.float().numpy() for k, v in t.items()}
+    QM, M = (qpad[0] + N + qpad[1]) // g, (kvpad[0] + N + kvpad[1]) // kvb
+    merged = _lists(np.random.default_rng(7), H, QM, M, W)[None]
+    o, lse, *grads = _grads(ftk, t, merged, H, g, kvb, q_padding=qpad, kv_padding=kvpad)
+    og = o.float().cpu().numpy()
+    ora = tolerance.attention_oracles(orc, x, merged, H, g, kvb, dtype, og, qpad, kvpad)
+    np.testing.assert_allclose(lse.cpu().numpy(), ora["lse"], atol=2e-3, rtol=1e-2)
+    for nm, y in zip(("O", "dQ", "dK", "dV"), (o, *grads)):
+        got = y.float().cpu().numpy()
+        if dtype == "fp16":
+            assert (tolerance.rel_err(got, ora["exact"][nm]) <= 1).all(), nm
+        else:
+            tolerance.check_rounded(got, ora["exact"][nm], ora["rounded"][nm],
+                                    ora["envelope"][nm], nm)
+
+
+@pytest.mark.parametrize("g,kvb", [(32, 32), (32, 64)])
+def test_forward_reference_needs_more_than_four_tiles(ftk, g, kvb):
+    """Eight q-blocks of a pair with disjoint lists, too many for the four tiles that
+    give the rows their reference exponents: the tiles concerned go to the exact
+    kernel, the others do not."""
+    H, D, N = 2, 128, 512
+    t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype="bf16", seed=35, do_seed=36))
+    x = {k: v.float().numpy() for k, v in t.items()}
+    QM, M = N // g, N // kvb
+    merged = np.full((1, H, QM, M), -1, dtype=np.int32)
+    for m in range(QM):
+        merged[0, 0, m, 0] = (m * (64 // kvb)) % M
+        merged[0, 1, m, :M] = np.random.default_rng(m).permutation(M)
+    o, lse = ftk.flash_topk_attn(t["q"].cuda(), t["k"].cuda(), t["v"].cuda(),
+                                 torch.from_numpy(merged).cuda(), None, H, g, kvb)
+    ftk.check_errors()
+    wo, wl = orc.sparse_attn_fwd(x["q"], x["k"], x["v"], merged, H, g, kvb)
+    np.testing.assert_allclose(lse.cpu().numpy(), wl, atol=2e-3, rtol=1e-2)
+    # one block of 32 or 64 keys per row: a bf16 P and a bf16 O, 2^-8 of the value each, and
+    # the values of V are at most about 4
+    np.testing.assert_allclose(o.float().cpu().numpy(), wo, atol=4 * 2 * 2.0 ** -8, rtol=2.0 ** -7)
