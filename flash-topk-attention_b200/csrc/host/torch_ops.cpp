@@ -11,11 +11,17 @@
 // the status words.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
 
 #include <atomic>
+#include <cmath>
 #include <mutex>
 #include <string>
 #include <tuple>
@@ -26,7 +32,7 @@
 namespace {
 
 using at::Tensor;
-using torch::autograd::AutogradContext;
+using torch::autograd::SavedVariable;
 using torch::autograd::variable_list;
 
 struct Unsupported : std::runtime_error {
@@ -136,6 +142,23 @@ std::vector<std::pair<std::string, double>> take_times() {
   return out;
 }
 
+// ------------------------------------------------------------ device memory
+// Outputs, straight from the allocator's tensor factory (a dispatched at::empty
+// takes about twice as long).
+Tensor new_cuda(at::IntArrayRef sizes, at::ScalarType dtype, const at::Device& device) {
+  return Tensor(at::detail::empty_cuda(sizes, dtype, device, std::nullopt));
+}
+// Scratch of one call: memory of the caching allocator without a tensor around it.
+// Freed at the end of the scope, for reuse in stream order, like a tensor would be.
+struct Scratch {
+  at::DataPtr p;
+  size_t bytes;
+  explicit Scratch(size_t n) : bytes(n) {
+    p = c10::cuda::CUDACachingAllocator::get()->allocate(std::max<size_t>(n, 16));
+  }
+  void* get() const { return p.get(); }
+};
+
 // ------------------------------------------------------------------- layouts
 // A tensor addressed as [b][n][h][d]: d dense, 16-byte aligned base, strides
 // multiples of 8 elements.  Copies only what cannot be addressed in place.
@@ -210,20 +233,18 @@ std::vector<Tensor> score_topk(Tensor q, Tensor k, bool four_d, int64_t H, int64
   const View vq(q, four_d, D), vk(k, four_d, D);
   if (outs.empty()) {
     const int64_t width = topk > 0 ? std::min(topk, M) : M;
-    const auto opt = at::TensorOptions().device(device);
-    outs.push_back(at::empty({B, H, N, width}, opt.dtype(at::kInt)));
-    outs.push_back(at::empty({B, H, N, width}, opt.dtype(at::kFloat)));
-    outs.push_back(at::empty({B, H, N, width}, opt.dtype(at::kFloat)));
+    outs.reserve(3);
+    outs.push_back(new_cuda({B, H, N, width}, at::kInt, device));
+    outs.push_back(new_cuda({B, H, N, width}, at::kFloat, device));
+    outs.push_back(new_cuda({B, H, N, width}, at::kFloat, device));
   }
   const int64_t first = b0 * N * outs[0].size(3);
-  const size_t bytes = ftk_score_topk_workspace(count, N, M);
-  const Tensor ws = at::empty({static_cast<int64_t>(bytes)},
-                              at::TensorOptions().device(device).dtype(at::kByte));
+  const Scratch ws(ftk_score_topk_workspace(count, N, M));
   check(ftk_score_topk(vq.t.data_ptr(), vk.t.data_ptr(), dtype_code(vq.t), B, H, N, D, vq.sb, vq.sn,
                        vq.sh, vk.sb, vk.sn, vk.sh, b0, count, block, pad_head, pad_tail, scale,
                        topk, threshold, outs[0].data_ptr<int>() + first,
                        outs[1].data_ptr<float>() + first, outs[2].data_ptr<float>() + first,
-                       ws.data_ptr(), bytes, status_ptr(device.index()), st.stream()),
+                       ws.get(), ws.bytes, status_ptr(device.index()), st.stream()),
         "ftk_score_topk");
   g_launches += 2;
   return outs;
@@ -239,14 +260,16 @@ std::tuple<Tensor, std::optional<Tensor>, Tensor> qblock_merge(
   const auto st = c10::cuda::getCurrentCUDAStream(device.index());
   const int64_t B = topk_idx.size(0), H = topk_idx.size(1), N = topk_idx.size(2);
   const int64_t QM = (pad_head + N + pad_tail) / q_block;
-  const Tensor idx = topk_idx.to(at::kInt).contiguous();
+  auto dense = [](const Tensor& t, at::ScalarType dtype) {
+    return t.scalar_type() == dtype && t.is_contiguous() ? t : t.to(dtype).contiguous();
+  };
+  const Tensor idx = dense(topk_idx, at::kInt);
   Tensor scr;
-  if (topk_scores) scr = topk_scores->to(at::kFloat).contiguous();
-  const auto opt = at::TensorOptions().device(device);
-  Tensor merged = at::empty({B, H, QM, width}, opt.dtype(at::kInt));
-  Tensor counts = at::empty({B, H, QM}, opt.dtype(at::kInt));
+  if (topk_scores) scr = dense(*topk_scores, at::kFloat);
+  Tensor merged = new_cuda({B, H, QM, width}, at::kInt, device);
+  Tensor counts = new_cuda({B, H, QM}, at::kInt, device);
   std::optional<Tensor> scores;
-  if (want_scores) scores = at::empty({B, H, QM, width}, opt.dtype(at::kFloat));
+  if (want_scores) scores = new_cuda({B, H, QM, width}, at::kFloat, device);
   check(ftk_qblock_merge(idx.data_ptr<int>(), scr.defined() ? scr.data_ptr<float>() : nullptr,
                          B * H, N, topk_idx.size(3), q_block, pad_head, pad_tail, blocks, width,
                          merged.data_ptr<int>(), scores ? scores->data_ptr<float>() : nullptr,
@@ -311,16 +334,14 @@ Forward attn_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   const int64_t D = q.size(2) / m.H;
   const View vq(x[0], false, D), vk(x[1], false, D), vv(x[2], false, D);
   Forward f{vq.t, vk.t, vv.t, merged.contiguous(), Tensor(), Tensor()};
-  f.o = at::empty(q.sizes(), q.options().memory_format(at::MemoryFormat::Contiguous));
-  f.lse = at::empty({q.size(0), m.H, q.size(1)}, q.options().dtype(at::kFloat));
+  f.o = new_cuda(q.sizes(), q.scalar_type(), device);
+  f.lse = new_cuda({q.size(0), m.H, q.size(1)}, at::kFloat, device);
   const ftk_attn a = describe(m, vq, vk, vv, f.lists, f32);
-  const size_t bytes = ftk_attn_fwd_workspace(&a);
-  const Tensor ws =
-      at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 4))}, q.options().dtype(at::kByte));
+  const Scratch ws(ftk_attn_fwd_workspace(&a));
   {
     TimedCall timed("ftk_sparse_fwd", st);
     check(ftk_attn_fwd(&a, f.o.data_ptr(), f.o.stride(0), f.o.stride(1), D,
-                       f.lse.data_ptr<float>(), ws.data_ptr(), bytes, status_ptr(device.index()),
+                       f.lse.data_ptr<float>(), ws.get(), ws.bytes, status_ptr(device.index()),
                        st.stream()),
           "ftk_attn_fwd");
   }
@@ -328,62 +349,57 @@ Forward attn_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   return f;
 }
 
-// Forward and backward of the gathered-KV attention (reference:
-// FlashSparseAttnFunc, flash_topk_attn_v2/sparse_attn.py:130-224).
-struct SparseAttn : torch::autograd::Function<SparseAttn> {
-  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k,
-                               const Tensor& v, const Tensor& merged, int64_t H, int64_t Hkv,
-                               int64_t q_block, int64_t kv_block, int64_t q_pad_head,
-                               int64_t kv_pad_head, double scale) {
-    const AttnMeta m{H, Hkv, q_block, kv_block, q_pad_head, kv_pad_head, scale};
-    Forward f = attn_forward(q, k, v, merged, m);
-    ctx->save_for_backward({f.q, f.k, f.v, f.o, f.lse, f.lists});
-    ctx->saved_data["meta"] = std::vector<int64_t>{H, Hkv, q_block, kv_block, q_pad_head, kv_pad_head};
-    ctx->saved_data["scale"] = scale;
-    ctx->mark_non_differentiable({f.lse});
-    ctx->set_materialize_grads(false);
-    return {f.o, f.lse};
+// Backward of the gathered-KV attention (reference: FlashSparseAttnFunc,
+// flash_topk_attn_v2/sparse_attn.py:130-224).  A node of its own instead of a
+// torch::autograd::Function, whose context and wrapping of outputs cost some 6 us
+// per pass.
+struct SparseAttnBackward : torch::autograd::Node {
+  AttnMeta m{};
+  SavedVariable q, k, v, o, lse, lists;
+
+  std::string name() const override { return "SparseAttnBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable* x : {&q, &k, &v, &o, &lse, &lists}) x->reset_data();
   }
 
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    variable_list out(11);
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(3);
     if (!grads[0].defined()) return out;
-    const variable_list saved = ctx->get_saved_variables();
-    const std::vector<int64_t> i = ctx->saved_data["meta"].toIntVector();
-    const AttnMeta m{i[0], i[1], i[2], i[3], i[4], i[5], ctx->saved_data["scale"].toDouble()};
-    const Tensor &o = saved[3], &lse = saved[4];
-    const at::Device device = o.device();
+    at::AutoDispatchBelowADInplaceOrView below;
+    const Tensor tq = q.unpack(), tk = k.unpack(), tv = v.unpack(),
+                 to = o.unpack(shared_from_this()), tl = lse.unpack(), tm = lists.unpack();
+    const at::Device device = to.device();
     c10::cuda::CUDAGuard guard(device);
     look(device.index());
     const auto st = c10::cuda::getCurrentCUDAStream(device.index());
-    const bool f32 = o.scalar_type() == at::kFloat;
-    const int64_t D = o.size(2) / m.H;
-    const View vq(saved[0], false, D), vk(saved[1], false, D), vv(saved[2], false, D);
+    const bool f32 = to.scalar_type() == at::kFloat;
+    const int64_t D = to.size(2) / m.H;
+    const View vq(tq, false, D), vk(tk, false, D), vv(tv, false, D);
     Tensor g[1] = {grads[0]};
     if (f32) cast_bf16(g, st);
-    else if (g[0].scalar_type() != vq.t.scalar_type()) g[0] = g[0].to(vq.t.scalar_type());
+    else if (g[0].scalar_type() != tq.scalar_type()) g[0] = g[0].to(tq.scalar_type());
     const View vg(g[0], false, D);
-    const ftk_attn a = describe(m, vq, vk, vv, saved[5], f32);
-    const size_t bytes = ftk_attn_bwd_workspace(&a);
-    const Tensor ws = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 4))},
-                                o.options().dtype(at::kByte));
-    Tensor dq = at::empty_like(o);
+    const ftk_attn a = describe(m, vq, vk, vv, tm, f32);
+    const Scratch ws(ftk_attn_bwd_workspace(&a));
+    Tensor dq = new_cuda(to.sizes(), to.scalar_type(), device);
     int* status = status_ptr(device.index());
     {
       TimedCall timed("ftk_sparse_bwd_dq", st);
-      check(ftk_attn_bwd_dq(&a, o.data_ptr(), o.stride(0), o.stride(1), D, vg.t.data_ptr(), vg.sb,
-                            vg.sn, vg.sh, lse.data_ptr<float>(), ws.data_ptr(), bytes,
-                            dq.data_ptr(), dq.stride(0), dq.stride(1), D, status, st.stream()),
+      check(ftk_attn_bwd_dq(&a, to.data_ptr(), to.stride(0), to.stride(1), D, vg.t.data_ptr(), vg.sb,
+                            vg.sn, vg.sh, tl.data_ptr<float>(), ws.get(), ws.bytes, dq.data_ptr(),
+                            dq.stride(0), dq.stride(1), D, status, st.stream()),
             "ftk_attn_bwd_dq");
     }
     g_launches += 1;
     out[0] = dq;
-    if (ctx->needs_input_grad(1) || ctx->needs_input_grad(2)) {
-      Tensor dk = at::empty({a.B, a.N, m.Hkv * D}, o.options());
-      Tensor dv = at::empty({a.B, a.N, m.Hkv * D}, o.options());
+    if (task_should_compute_output(1) || task_should_compute_output(2)) {
+      Tensor dk = new_cuda({a.B, a.N, m.Hkv * D}, to.scalar_type(), device);
+      Tensor dv = new_cuda({a.B, a.N, m.Hkv * D}, to.scalar_type(), device);
       TimedCall timed("ftk_sparse_bwd_dkv", st);
-      check(ftk_attn_bwd_dkv(&a, vg.t.data_ptr(), vg.sb, vg.sn, vg.sh, lse.data_ptr<float>(),
-                             ws.data_ptr(), bytes, dk.data_ptr(), dk.stride(0), dk.stride(1), D,
+      check(ftk_attn_bwd_dkv(&a, vg.t.data_ptr(), vg.sb, vg.sn, vg.sh, tl.data_ptr<float>(),
+                             ws.get(), ws.bytes, dk.data_ptr(), dk.stride(0), dk.stride(1), D,
                              dv.data_ptr(), dv.stride(0), dv.stride(1), D, status, st.stream()),
             "ftk_attn_bwd_dkv");
       g_launches += 1;
@@ -405,14 +421,106 @@ std::tuple<Tensor, Tensor> sparse_attn(const Tensor& q, const Tensor& k, const T
                                        const Tensor& merged, int64_t H, int64_t Hkv,
                                        int64_t q_block, int64_t kv_block, int64_t q_pad_head,
                                        int64_t kv_pad_head, double scale) {
-  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) {
-    variable_list r = SparseAttn::apply(q, k, v, merged, H, Hkv, q_block, kv_block, q_pad_head,
-                                        kv_pad_head, scale);
-    return {r[0], r[1]};
+  const AttnMeta m{H, Hkv, q_block, kv_block, q_pad_head, kv_pad_head, scale};
+  if (!at::GradMode::is_enabled() || !(q.requires_grad() || k.requires_grad() || v.requires_grad())) {
+    const Forward f = attn_forward(q, k, v, merged, m);
+    return {f.o, f.lse};
   }
-  const Forward f =
-      attn_forward(q, k, v, merged, {H, Hkv, q_block, kv_block, q_pad_head, kv_pad_head, scale});
+  auto node = std::shared_ptr<SparseAttnBackward>(new SparseAttnBackward(),
+                                                  torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
+  Forward f;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    f = attn_forward(q, k, v, merged, m);
+  }
+  node->m = m;
+  node->q = SavedVariable(f.q, false);
+  node->k = SavedVariable(f.k, false);
+  node->v = SavedVariable(f.v, false);
+  node->lse = SavedVariable(f.lse, false);
+  node->lists = SavedVariable(f.lists, false);
+  torch::autograd::set_history(f.o, node);
+  node->o = SavedVariable(f.o, true);
   return {f.o, f.lse};
+}
+
+// ----------------------------------------------------------- the ordinary call
+// The Python operators check their arguments one by one, as the reference does, to
+// raise its exceptions: 5 to 8 us per call.  These entry points take a call that
+// passes all of the checks (and needs no special handling) straight through and
+// return nothing for any other, which the Python code then deals with.
+using Pads = std::pair<int64_t, int64_t>;
+
+bool pads_fit(const Pads& p, int64_t n, int64_t block) {
+  return p.first >= 0 && p.second >= 0 && p.first < block && p.second < block &&
+         (p.first + n + p.second) % block == 0;
+}
+bool float_type(const Tensor& t) {
+  const auto d = t.scalar_type();
+  return d == at::kHalf || d == at::kBFloat16 || d == at::kFloat;
+}
+
+std::optional<std::tuple<Tensor, Tensor, Tensor, int64_t>> plain_score(
+    const Tensor& q, const Tensor& k, std::optional<int64_t> num_heads, int64_t block, int64_t topk,
+    const Pads& pad, double threshold, int64_t scratch) {
+  const bool four_d = q.dim() == 4;
+  if (!q.is_cuda() || q.device() != k.device() || (!four_d && (q.dim() != 3 || !num_heads)))
+    return std::nullopt;
+  const int64_t H = four_d ? q.size(1) : *num_heads;
+  if (H <= 0 || (num_heads && *num_heads != H)) return std::nullopt;
+  const int64_t N = q.size(four_d ? 2 : 1), C = four_d ? H * q.size(3) : q.size(2), D = C / H;
+  if (k.sizes() != q.sizes() || q.scalar_type() != k.scalar_type() || !float_type(q) || C % H ||
+      D % 8 || D > 256 || D <= 0 || q.size(0) <= 0 || N <= 0)
+    return std::nullopt;
+  if (block <= 0 || topk < 0 || !pads_fit(pad, N, block)) return std::nullopt;
+  const int64_t M = (pad.first + N + pad.second) / block, slices = q.size(0) * H;
+  if (M > 4096 || slices > 32768 ||
+      slices * static_cast<int64_t>(ftk_score_topk_workspace(1, N, M)) > scratch)
+    return std::nullopt;
+  auto r = score_topk(q, k, four_d, H, block, topk, pad.first, pad.second, threshold,
+                      1.0 / std::sqrt(static_cast<double>(D)), 0, slices, {});
+  return std::make_tuple(std::move(r[0]), std::move(r[1]), std::move(r[2]), M);
+}
+
+std::optional<std::tuple<Tensor, Tensor>> plain_merge(const Tensor& idx,
+                                                      const std::optional<Tensor>& scores,
+                                                      int64_t q_block, const Pads& pad,
+                                                      std::optional<int64_t> width, int64_t blocks) {
+  if (!idx.is_cuda() || idx.dim() != 4 || q_block <= 0 || blocks <= 0 || blocks > 4096 ||
+      (scores && (scores->sizes() != idx.sizes() || scores->device() != idx.device())) ||
+      !pads_fit(pad, idx.size(2), q_block))
+    return std::nullopt;
+  const int64_t w = width ? *width : q_block * idx.size(3);
+  if (w <= 0) return std::nullopt;
+  auto r = qblock_merge(idx, scores, q_block, pad.first, pad.second, blocks, w, false);
+  return std::make_tuple(std::move(std::get<0>(r)), std::move(std::get<2>(r)));
+}
+
+std::optional<std::tuple<Tensor, Tensor>> plain_attn(
+    const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& merged, int64_t H,
+    int64_t q_block, int64_t kv_block, std::optional<double> scale, const Pads& q_pad,
+    const Pads& kv_pad, std::optional<int64_t> kv_heads) {
+  if (!q.is_cuda() || q.dim() != 3 || H <= 0 || !float_type(q)) return std::nullopt;
+  const int64_t B = q.size(0), N = q.size(1), D = q.size(2) / H, Hkv = kv_heads ? *kv_heads : H;
+  if (q.size(2) != H * D || D <= 0 || D % 16 || D > 256 || Hkv <= 0 || H % Hkv || B <= 0 || N <= 0)
+    return std::nullopt;
+  for (const Tensor* t : {&k, &v})
+    if (t->dim() != 3 || t->size(0) != B || t->size(1) != N || t->size(2) != Hkv * D ||
+        t->scalar_type() != q.scalar_type() || t->device() != q.device())
+      return std::nullopt;
+  for (const int64_t b : {q_block, kv_block})
+    if (b <= 0 || b > 128 || (b > 64 && b % 32)) return std::nullopt;
+  if (!pads_fit(q_pad, N, q_block) || !pads_fit(kv_pad, N, kv_block)) return std::nullopt;
+  if (merged.dim() != 4 || merged.scalar_type() != at::kInt || merged.device() != q.device() ||
+      merged.size(0) != B || merged.size(1) != H ||
+      merged.size(2) != (q_pad.first + N + q_pad.second) / q_block || merged.size(3) <= 0)
+    return std::nullopt;
+  // block sizes that every gradient kernel takes
+  auto usual = [](int64_t b) { return b == 16 || b == 32 || b == 64 || b == 128; };
+  if (!usual(q_block) || !usual(kv_block)) return std::nullopt;
+  return sparse_attn(q, k, v, merged, H, Hkv, q_block, kv_block, q_pad.first, kv_pad.first,
+                     scale ? *scale : 1.0 / std::sqrt(static_cast<double>(D)));
 }
 
 }  // namespace
@@ -430,6 +538,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("score_topk_workspace", &ftk_score_topk_workspace);
   m.def("qblock_merge", &qblock_merge, release());
   m.def("sparse_attn", &sparse_attn, release());
+  m.def("plain_score", &plain_score, release());
+  m.def("plain_merge", &plain_merge, release());
+  m.def("plain_attn", &plain_attn, release());
   m.def("status_word", &status_word, "the device's status word, a pinned host tensor");
   m.def("take_status", &take_status);
   m.def("look", &look);

@@ -64,6 +64,18 @@ def _call(name, fn, *args):
     return out
 
 
+def _plain(fn, *args):
+    """What a native entry point returns for an ordinary call: one whose arguments it
+    finds in order and that wants neither timing nor synchronous checks.  None:
+    go through the checks, which raise or handle the special cases."""
+    if _events is not None or _DEBUG:
+        return None
+    try:
+        return fn(*args)
+    except TypeError:          # an argument that is not of the declared kind
+        return None
+
+
 def event_times() -> dict:
     """Sum of device milliseconds and call count per entry point since
     enable_event_timing(True); synchronises."""
@@ -308,6 +320,12 @@ def flash_topk_select(block_scores, threshold, max_topk, score_block_size, paddi
 
 def flash_topk_score_fused(q, k, num_heads, score_block_size, topk, padding, threshold):
     """block score + select without materialising [B,H,N,M] for the caller."""
+    plain = _plain(native.plain_score, q, k, num_heads, score_block_size, topk, padding, threshold,
+                   _SCORE_SCRATCH_BYTES)
+    if plain is not None:
+        idx, raw, avg, M = plain
+        idx._ftk_num_score_blocks = M
+        return idx, raw, avg
     input_4d, B, H, N, D, M, ph, pt = _parse_block_score_args(
         q, k, num_heads, score_block_size, padding)
     if topk < 0:
@@ -542,6 +560,10 @@ def flash_sparse_attn(q, k, v, merged_indices, num_heads, q_block_size, kv_block
     (grouped-query attention, also beyond the reference): k and v are
     [B, N, num_kv_heads * D] and query head h reads kv head
     h // (num_heads // num_kv_heads)."""
+    plain = _plain(native.plain_attn, q, k, v, merged_indices, num_heads, q_block_size,
+                   kv_block_size, scale, q_padding, kv_padding, num_kv_heads)
+    if plain is not None:
+        return plain
     if q.ndim != 3:
         raise ValueError("q must be [B, N, C]")
     if q.device.type != "cuda":
