@@ -112,7 +112,7 @@ __host__ __device__ constexpr int sel_wpc() { return IPT >= 32 ? 4 : SEL_WARPS; 
 
 // CTAs per SM that the register budget is for (latency is hidden by warps)
 template <int IPT>
-__host__ __device__ constexpr int sel_ctas() { return IPT <= 4 || IPT == 32 ? 4 : 3; }
+__host__ __device__ constexpr int sel_ctas() { return IPT == 64 ? 2 : IPT <= 4 || IPT == 32 ? 4 : 3; }
 
 template <int IPT>
 __global__ void __launch_bounds__(sel_wpc<IPT>() * 32, sel_ctas<IPT>())
@@ -185,6 +185,7 @@ int select_launch(const float* block_scores, const float* row_scale, int64_t row
   else if (M <= 256) FTK_SEL_REG(8);
   else if (M <= 512) FTK_SEL_REG(16);
   else if (M <= 1024) FTK_SEL_REG(32);
+  else if (M <= 2048) FTK_SEL_REG(64);   // 37k rows of 1146 entries: 4x the kernel below
 #undef FTK_SEL_REG
   const int Mp = (M + 31) & ~31;
   const size_t smem = static_cast<size_t>(SEL_WARPS) * 2 * Mp * sizeof(float);
@@ -349,6 +350,10 @@ __device__ __forceinline__ void bitonic_desc_blocked(T (&v)[E], int lane) {
 // sorts them with the blocked bitonic network and writes its row, the -1 / 0
 // tail with 16-byte stores.
 constexpr int MGW_WARPS = 4;
+// Steps fetched and checked together.  Few ids usually mean few picks per row and
+// small grids, where the latency of a batch is what a warp waits for.
+template <int E>
+__host__ __device__ constexpr int mgw_steps() { return E <= 8 ? 8 : 4; }
 
 template <int E>
 __global__ void __launch_bounds__(MGW_WARPS * 32)
@@ -357,7 +362,7 @@ qblock_merge_warp_kernel(const int32_t* __restrict__ idx, const float* __restric
                          int32_t* __restrict__ out_idx, float* __restrict__ out_scr,
                          int32_t* __restrict__ counts, int* status) {
   constexpr int MP = 32 * E;
-  constexpr int U = 4;   // steps fetched and checked together
+  constexpr int U = mgw_steps<E>();
   __shared__ float agg_all[MGW_WARPS][MP];
   __shared__ uint8_t tag_all[MGW_WARPS][U * MP];
   pdl_wait();
@@ -853,9 +858,10 @@ extern "C" int ftk_qblock_merge(const int32_t* topk_idx, const float* topk_score
   if (Mp <= 1024) {
     // one warp per q-block
     const int64_t total_qb = BH * QM;
-    const unsigned grid = static_cast<unsigned>((total_qb + MGW_WARPS - 1) / MGW_WARPS);
 #define FTK_MGW(E)                                                                             \
-  return launch_pdl(qblock_merge_warp_kernel<E>, grid, MGW_WARPS * 32, 0, st, topk_idx,         \
+  return launch_pdl(qblock_merge_warp_kernel<E>,                                                \
+                    static_cast<unsigned>((total_qb + MGW_WARPS - 1) / MGW_WARPS),              \
+                    MGW_WARPS * 32, 0, st, topk_idx,                                            \
                     topk_scores, N, K, q_block_size, q_pad_head, static_cast<int>(QM), total_qb, \
                     num_score_blocks, qblock_topk, merged_idx, merged_scores, counts, status)
     switch (Mp) {

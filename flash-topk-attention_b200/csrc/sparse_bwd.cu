@@ -1058,7 +1058,7 @@ constexpr int FAN_THREADS = 1024;
 
 __global__ void __launch_bounds__(FAN_THREADS)
 fan_in_kernel(const uint8_t* __restrict__ masks, int stride, int tiles, int64_t head_stride,
-              int heads, int slices_per_b, int H, int Mkv, int G, int cols, int colsp,
+              int heads, int slices_per_b, int H, int G, int cols, int colsp,
               int32_t* __restrict__ order) {
   extern __shared__ unsigned long long fan_keys[];
   unsigned* cnt = reinterpret_cast<unsigned*>(fan_keys + colsp);
@@ -1069,20 +1069,38 @@ fan_in_kernel(const uint8_t* __restrict__ masks, int stride, int tiles, int64_t 
   const int bhq = slice / slices_per_b * H + slice % slices_per_b * heads;
   for (int x = tid; x < colsp; x += FAN_THREADS) cnt[x] = 0u;
   __syncthreads();
-  const int parts = max(1, FAN_THREADS / cols);
-  for (int u = tid; u < cols * parts; u += FAN_THREADS) {
-    const int col = u % cols, part = u / cols;
-    const int j0 = col * G, jn = min(G, Mkv - j0);
-    unsigned c = 0;
-    for (int r = part; r < heads * tiles; r += parts) {
+  // 16 bytes = 16 / G kv tiles of one q tile per load, the q tiles dealt to as many
+  // threads as there are (a byte per load and row took some 95 us longer at 403 q
+  // tiles of 806 kv blocks, one slice)
+  const int quads = stride >> 4, parts = max(1, FAN_THREADS / quads), rows = heads * tiles;
+  for (int u = tid; u < quads * parts; u += FAN_THREADS) {
+    const int quad = u % quads, part = u / quads;
+    unsigned c[16];
+#pragma unroll
+    for (int x = 0; x < 16; x++) c[x] = 0;
+#pragma unroll 4
+    for (int r = part; r < rows; r += parts) {
       const int h = r / tiles;
-      const uint8_t* src = masks + (bhq + h) * head_stride +
-                           static_cast<int64_t>(r - h * tiles) * stride + j0;
-      unsigned m = 0;
-      for (int j = 0; j < jn; j++) m |= src[j];
-      c += __popc(m);
+      const uint4 t = *(reinterpret_cast<const uint4*>(
+                            masks + (bhq + h) * head_stride +
+                            static_cast<int64_t>(r - h * tiles) * stride) + quad);
+      const unsigned w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+      for (int x = 0; x < 16; x++) {
+        unsigned m = (w[x >> 2] >> (8 * (x & 3))) & 255u;
+        if (G == 2) m |= (w[x >> 2] >> (8 * ((x & 3) ^ 1))) & 255u;
+        if (G == 4 || G == 8) {
+          m = w[x >> 2] | (G == 8 ? w[(x >> 2) ^ 1] : 0u);
+          m = (m | (m >> 8) | (m >> 16) | (m >> 24)) & 255u;
+        }
+        if (x % G == 0) c[x] += __popc(m);
+      }
     }
-    atomicAdd(&cnt[col], c);
+#pragma unroll
+    for (int x = 0; x < 16; x++) {
+      const int col = (quad * 16 + x) / G;
+      if (x % G == 0 && col < cols && c[x]) atomicAdd(&cnt[col], c[x]);
+    }
   }
   __syncthreads();
   for (int x = tid; x < colsp; x += FAN_THREADS)
@@ -1492,7 +1510,7 @@ extern "C" int ftk_attn_bwd_dkv(const ftk_attn* a, const void* dout, int64_t sdo
       e = launch_pdl(fan_in_kernel, static_cast<unsigned>(a->B * a->H / p.heads), FAN_THREADS, smem,
                      st, p.masks, b.stride, b.tiles,
                      static_cast<int64_t>(b.tiles) * b.stride, p.heads,
-                     static_cast<int>(a->H / p.heads), static_cast<int>(a->H), b.gr.Mkv,
+                     static_cast<int>(a->H / p.heads), static_cast<int>(a->H),
                      attn_groups(b.gr.kvb), b.kv_tiles, colsp, order);
     if (e) return e;
     p.tile_order = order;
