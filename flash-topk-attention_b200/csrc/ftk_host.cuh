@@ -138,6 +138,49 @@ inline int launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t s
              : FTK_ERR_CUDA;
 }
 
+// The same as clusters of `cluster` CTAs along x (1: no clusters).
+template <typename... Params, typename... Args>
+inline int launch_clusters(void (*kernel)(Params...), int cluster, dim3 grid, dim3 block,
+                           size_t smem, cudaStream_t st, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) == cudaSuccess
+             ? FTK_OK
+             : FTK_ERR_CUDA;
+}
+
+// Clusters of that size that can run at once, 0 if the device does not say.
+template <typename... Params>
+inline int max_clusters(void (*kernel)(Params...), int cluster, dim3 block, size_t smem) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(cluster));
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
 inline int sm_count() {
   static int n = 0;
   if (n == 0) {

@@ -280,6 +280,24 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+__device__ __forceinline__ uint32_t cluster_nctas() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r));
+  return r;
+}
+// the value at this shared-memory location in CTA `rank` of a cluster of `n`
+__device__ __forceinline__ float ld_cta(const float* p, int rank, int n) {
+  if (n == 1) return *reinterpret_cast<const volatile float*>(p);
+  float v;
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\t"
+      "mapa.shared::cluster.u32 ra, %1, %2;\n\t"
+      "ld.volatile.shared::cluster.f32 %0, [ra];\n\t}"
+      : "=f"(v)
+      : "r"(smem_u32(p)), "r"(rank)
+      : "memory");
+  return v;
+}
 __device__ __forceinline__ void cluster_arrive() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }

@@ -22,7 +22,15 @@
 // two follow-up launches and the clearing of their flag, which every call paid
 // for (about 2 us of device time each at the smallest sizes, 6-7 us at the
 // largest, and 3 of 5 launches), are not there.
+//
+// Where the grid has too few tiles of 256 rows to fill the SMs, or a last wave that
+// is nearly empty, a cluster of 2, 4 or 8 CTAs shares a tile and splits its keys
+// (score_split).  All take the reference exponents from the first key tile, so their
+// block sums go out as they are; the row totals meet through the cluster's shared
+// memory.  A total is always added up from the same SC_SEGS parts of the keys, so it
+// does not depend on the split, bit for bit.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 
@@ -35,6 +43,7 @@ constexpr int SC_QROWS = 256;      // query rows per CTA
 constexpr int SC_KT = 128;         // key rows per tile (UMMA N)
 constexpr int SC_STAGES = 4;       // K tile ring depth
 constexpr int SC_THREADS = 576;    // 2 + 2 x 8 warps
+constexpr int SC_SEGS = 8;         // parts of the keys that a row total is added up from
 constexpr int SC_CHUNK_BYTES = 128 * 128;  // 128 rows x 64 16-bit elements
 __host__ __device__ constexpr int score_ksplit(int d) { return d > 128 ? 2 : 1; }
 __host__ __device__ constexpr int score_stages(int d) { return d > 128 ? 2 : SC_STAGES; }
@@ -79,16 +88,20 @@ __device__ __forceinline__ TileInfo tile_info(const ScoreParams& p, int t) {
   return ti;
 }
 
-// Which softmax group drains tile t.  Tiles alternate between the two groups,
-// each group bound to one accumulator stage, so a group meets every phase of
-// its stage's barriers in order (a one-bit parity wait must never skip a
+// Which softmax group drains a CTA's u-th tile: tiles alternate between the two
+// groups, each group bound to one accumulator stage, so a group meets every phase
+// of its stage's barriers in order (a one-bit parity wait must never skip a
 // phase).  When a score block spans several tiles (block size > 128) one
 // thread has to see all of them, and group 0 takes every tile.
-__device__ __forceinline__ int tile_owner(const ScoreParams& p, int t) {
-  return p.tiles_per_block > 1 ? 0 : (t & 1);
+// First tile of part s of the keys: whole score blocks, in order
+__device__ __forceinline__ int seg_begin(const ScoreParams& p, int s) {
+  const int per = max(1, p.tiles_per_block);
+  return static_cast<int>(static_cast<int64_t>(s) * (p.num_tiles / per) / SC_SEGS) * per;
 }
 
-template <int D>
+// SPLIT: launched as clusters that share a tile; its bookkeeping in the loop over the
+// tiles took 4 % of the kernel where nothing is split.
+template <int D, bool SPLIT>
 __global__ void __launch_bounds__(SC_THREADS, 1)
 score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
              const ScoreParams p) {
@@ -107,15 +120,17 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sQ = smem;
   uint8_t* sK = smem + Q_BYTES;
-  __shared__ __align__(8) uint64_t bars[1 + 2 * SC_STAGES + 8 + 2];
+  __shared__ __align__(8) uint64_t bars[1 + 2 * SC_STAGES + 8 + 1];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
-  __shared__ int s_redo;
+  __shared__ int s_redo, s_stop;
   __shared__ float s_mref[SC_QROWS];   // group 0 -> group 1: reference exponent / row maximum
-  __shared__ float s_part[SC_QROWS];   // group 1 -> group 0: partial total / maximum
+  __shared__ float s_seg[2][SC_SEGS][SC_QROWS];   // totals per group and part (pass 1: maxima in part 0)
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int q0 = blockIdx.x * SC_QROWS;
+  const int split = SPLIT ? static_cast<int>(cluster_nctas()) : 1,
+            rank = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
+  const int q0 = static_cast<int>(blockIdx.x) / split * SC_QROWS;
   const int bh_local = blockIdx.y;
   const int bh = p.bh_begin + bh_local;
   const int b_idx = bh / p.H, h_idx = bh - b_idx * p.H;
@@ -131,11 +146,10 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
     return smem_u32(&bars[1 + 2 * SC_STAGES + 4 + s * 2 + h]);
   };
   const uint32_t bar_mref = smem_u32(&bars[1 + 2 * SC_STAGES + 8]);
-  const uint32_t bar_part = smem_u32(&bars[1 + 2 * SC_STAGES + 9]);
 
   if (tid == 0) {
     abort_flag = 0;
-    s_redo = 0;
+    s_redo = s_stop = 0;
     mbar_init(bar_q, 1);
     for (int s = 0; s < SC_STAGES; s++) {
       mbar_init(bar_kfull(s), 1);
@@ -147,7 +161,6 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
         mbar_init(bar_aempty(s, h), 4);  // one arrival per warp draining the accumulator
       }
     mbar_init(bar_mref, 8);
-    mbar_init(bar_part, 8);
     mbar_init_fence();
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&tm_k);
@@ -161,15 +174,27 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
   WaitCtx w{&abort_flag, p.status};
-  const int T = p.num_tiles;
+  // my tiles: t_first .. t_first + L - 1, and in pass 0 tile 0 ahead of them unless it
+  // is mine (`pre`), for the reference exponents
+  const int seg_first = rank * SC_SEGS / split, seg_last = (rank + 1) * SC_SEGS / split;
+  const int t_first = SPLIT ? seg_begin(p, seg_first) : 0,
+            L = SPLIT ? seg_begin(p, seg_last) - t_first : p.num_tiles;
   float mref = 0.f;    // softmax threads: the row's reference exponent
   pdl_wait();
   pdl_launch();
 
   // Pass 0 is all there is unless a row total overflows.  Every barrier's
-  // phases run on from pass to pass: accumulator a has been used
-  // pass * ((T + 1 - a) / 2) times before, the K ring pass * T * KSPLIT times.
+  // phases run on from pass to pass: an accumulator and the K ring have been used
+  // as often as the tiles of the passes before say.
   for (int pass = 0; pass < 3; pass++) {
+  const int pre = SPLIT && pass == 0 && t_first > 0 ? 1 : 0;
+  const int T = L + pre;
+  const int done0 = pass > 0 ? L + (SPLIT && t_first > 0 ? 1 : 0) : 0;   // tiles of pass 0 ...
+  const int done1 = pass > 1 ? L : 0;                                       // ... and of pass 1
+  auto tile_of = [&](int u) { return u < pre ? 0 : t_first + u - pre; };
+  auto used = [&](int a, int u) {   // uses of accumulator a before this pass's tile u
+    return ((done0 + 1 - a) >> 1) + ((done1 + 1 - a) >> 1) + (u >> 1);
+  };
   if (warp == 0) {
     // ------------------------------------------------------- TMA producer
     if (lane == 0) {
@@ -181,13 +206,13 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
                         h_idx, q0 + half * 128, b_idx);
       }
       const uint32_t tile_bytes = static_cast<uint32_t>(p.tile_rows) * 128u * NCHS;
-      const int u0 = pass * T * KSPLIT;
+      const int u0 = (done0 + done1) * KSPLIT;
       for (int u = 0; u < T * KSPLIT; u++) {
         const int s = (u0 + u) % NSTG;
         const uint32_t ph = ((u0 + u) / NSTG) & 1;
         if (!mbar_wait(bar_kempty(s), ph ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
-        const int t = u / KSPLIT, part = u % KSPLIT;
-        const TileInfo ti = tile_info(p, t);
+        const int part = u % KSPLIT;
+        const TileInfo ti = tile_info(p, tile_of(u / KSPLIT));
         mbar_expect_tx(bar_kfull(s), tile_bytes);
         for (int c = 0; c < NCHS; c++)
           tma_load_4d(smem_u32(sK) + s * K_STAGE_BYTES + c * SC_CHUNK_BYTES, &tm_k, bar_kfull(s),
@@ -203,9 +228,9 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
       const uint64_t kdesc0 = smem_desc_sw128(smem_u32(sK), 16, 1024);
       bool ok = mbar_wait(bar_q, 0, w, FTK_DEV_TIMEOUT_MMA);
       for (int t = 0; ok && t < T; t++) {
-        const int u0 = (pass * T + t) * KSPLIT;
+        const int u0 = (done0 + done1 + t) * KSPLIT;
         const int a = t & 1;
-        const uint32_t pa = (pass * ((T + 1 - a) >> 1) + (t >> 1)) & 1;
+        const uint32_t pa = used(a, t) & 1;
         // the three barriers of a tile are waited for together (a test of a
         // completed barrier still takes ~110 cycles) and the tile's UMMAs go
         // out as one batch, so the tensor core is not left idle in between
@@ -289,6 +314,11 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
           }
           mref = ceilf(mx * c);
           if (!(fabsf(mref) < 1e30f)) mref = 0.f;
+          if (pre) {   // not one of my tiles: hand the accumulator back
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_aempty(0, half));
+          }
         }
         s_mref[row_in_cta] = mref;
         __syncwarp();
@@ -301,10 +331,14 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
 
     float acc = 0.f;
     int j = 0, col_in_block = 0;
-    for (int t = 0; ok && t < T; t++) {
-      if (tile_owner(p, t) != group) continue;
-      const int a = t & 1;
-      const uint32_t pa = (pass * ((T + 1 - a) >> 1) + (t >> 1)) & 1;
+    // this group's tiles, part by part
+    const int step = p.tiles_per_block > 1 ? 1 : 2;
+    int u = step == 2 ? pre + ((group ^ pre) & 1) : (group == 0 ? pre : T);
+    for (int seg = seg_first; seg < seg_last; seg++) {
+    const int u_end = seg_begin(p, seg + 1) - t_first + pre;
+    for (; ok && u < u_end; u += step) {
+      const int t = tile_of(u), a = u & 1;
+      const uint32_t pa = used(a, u) & 1;
       if (!mbar_wait(bar_afull(a, half), pa, w, FTK_DEV_TIMEOUT_CONSUMER)) { ok = false; break; }
       tc_fence_after();
       const TileInfo ti = tile_info(p, t);
@@ -402,34 +436,45 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
         }
       }
     }
-    // combine the two groups' partial results per row: group 1 publishes,
-    // group 0 adds (total) or takes the larger (maximum) and writes
-    const float mine = (pass == 1) ? run_max : total;
-    if (group == 1) {
-      s_part[row_in_cta] = mine;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_part);
-    } else {
-      if (ok) ok = mbar_wait(bar_part, pass & 1, w, FTK_DEV_TIMEOUT_CONSUMER);
-      if (ok && row_ok) {
-        const float other = s_part[row_in_cta];
-        if (pass == 1) {
-          s_mref[row_in_cta] = fmaxf(mine, other);
-        } else {
-          const float tot = mine + other;
-          p.row_total[row_off] = tot;
-          if (pass == 0 && !(tot > 0.f && tot < 3.0e38f)) s_redo = 1;
-        }
-      }
+    // publish this group's share of the part (pass 1: of the CTA's maximum)
+    s_seg[group][pass == 1 ? 0 : seg][row_in_cta] = pass == 1 ? run_max : total;
+    total = 0.f;
     }
   }
+  tc_fence_before();
   __syncthreads();
-  if (!s_redo || abort_flag) break;
+  tc_fence_after();
+  if (split > 1) cluster_sync_all();
+  if (tid < SC_QROWS) {
+    // every CTA of the cluster adds up the same totals, so all come to the same decision
+    if (pass == 1) {
+      float mx = -INFINITY;
+      for (int r = 0; r < split; r++)
+        mx = fmaxf(mx, fmaxf(ld_cta(&s_seg[0][0][tid], r, split), ld_cta(&s_seg[1][0][tid], r, split)));
+      s_mref[tid] = mx;
+    } else {
+      float tot = 0.f;
+#pragma unroll
+      for (int sg = 0; sg < SC_SEGS; sg++) {
+        const int r = sg * split / SC_SEGS;
+        tot += ld_cta(&s_seg[0][sg][tid], r, split) + ld_cta(&s_seg[1][sg][tid], r, split);
+      }
+      if (q0 + tid < p.N) {
+        if (rank == 0) p.row_total[static_cast<size_t>(bh_local) * p.N + q0 + tid] = tot;
+        if (pass == 0 && !(tot > 0.f && tot < 3.0e38f)) s_redo = 1;
+      }
+    }
+  } else if (tid < SC_QROWS + split) {
+    if (ld_cta(reinterpret_cast<const float*>(&abort_flag), tid - SC_QROWS, split) != 0.f)
+      s_stop = 1;
+  }
+  __syncthreads();
+  const bool again = s_redo && !s_stop;
+  if (split > 1) cluster_sync_all();   // nobody writes or leaves while a peer still reads
+  if (!again) break;
   }
 
   // ------------------------------------------------------------- teardown
-  tc_fence_before();
-  __syncthreads();
   if (abort_flag) {
     // give copies still in flight time to land before the smem is released
     for (int i = 0; i < 200; i++) __nanosleep(1000);
@@ -449,15 +494,54 @@ __global__ void score_normalize_kernel(const float* __restrict__ sums,
   }
 }
 
+// How many CTAs share a tile of 256 query rows: the fewest waves of the shortest
+// CTAs.  A CTA's time in key tiles is its share of them and about 3.5 to start and
+// finish, 7.5 where it also has to fetch the first tile for the reference exponents
+// and meet the others (512 tiles of 64 steps, D = 64: 4 waves unsplit 465 us, 7 waves of
+// halves 476); the number of clusters that run at once is what the device says.
+// 61 tiles of 122 steps: 203 -> 127 us with select, 32 of 32 steps: 59 -> 32 us.
+template <int D>
+static int score_split(int64_t tiles, int num_tiles, int units, size_t smem) {
+  constexpr int MAX_DEVICES = 64;
+  static std::atomic<int> resident[MAX_DEVICES][4];   // clusters of 1, 2, 4, 8
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return 1;
+  int best = 1;
+  double best_cost = 0.;
+  for (int i = 0; i < 4; i++) {
+    const int c = 1 << i;
+    if (c > units) break;
+    int n = resident[dev][i].load(std::memory_order_relaxed);
+    if (n == 0) {
+      n = c == 1 ? sm_count() : max_clusters(score_kernel<D, true>, c, SC_THREADS, smem);
+      resident[dev][i].store(n > 0 ? n : -1, std::memory_order_relaxed);
+    }
+    if (n <= 0) continue;
+    const double waves = static_cast<double>((tiles + n - 1) / n);
+    const double cost = waves * (static_cast<double>(num_tiles) / c + (c > 1 ? 7.5 : 3.5));
+    if (i == 0 || cost < 0.95 * best_cost) {
+      best = c;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 template <int D>
 static int launch_score_d(const CUtensorMap& tq, const CUtensorMap& tk, ScoreParams p,
                           int64_t bh_count, cudaStream_t st) {
   constexpr int NCH = D / 64;
   const size_t smem =
       1024 + (2 * NCH + score_stages(D) * (NCH / score_ksplit(D))) * SC_CHUNK_BYTES;
-  if (int e = allow_smem<score_kernel<D>>(smem)) return e;
-  dim3 grid((p.N + SC_QROWS - 1) / SC_QROWS, static_cast<unsigned>(bh_count));
-  return launch_pdl(score_kernel<D>, grid, SC_THREADS, smem, st, tq, tk, p);
+  if (int e = allow_smem<score_kernel<D, false>>(smem)) return e;
+  if (int e = allow_smem<score_kernel<D, true>>(smem)) return e;
+  const int qtiles = (p.N + SC_QROWS - 1) / SC_QROWS;
+  const int split = score_split<D>(qtiles * bh_count, p.num_tiles,
+                                   p.num_tiles / std::max(1, p.tiles_per_block), smem);
+  const dim3 grid(qtiles * split, static_cast<unsigned>(bh_count));
+  if (split == 1)
+    return launch_pdl(score_kernel<D, false>, grid, SC_THREADS, smem, st, tq, tk, p);
+  return launch_clusters(score_kernel<D, true>, split, grid, SC_THREADS, smem, st, tq, tk, p);
 }
 
 struct ScoreWs {

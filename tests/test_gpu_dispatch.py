@@ -200,3 +200,18 @@ def test_forward_reference_needs_more_than_four_tiles(ftk, g, kvb):
     # one block of 32 or 64 keys per row: a bf16 P and a bf16 O, 2^-8 of the value each, and
     # the values of V are at most about 4
     np.testing.assert_allclose(o.float().cpu().numpy(), wo, atol=4 * 2 * 2.0 ** -8, rtol=2.0 ** -7)
+
+
+@pytest.mark.parametrize("N,D,bsz,topk", [(3000, 128, 64, 8), (2050, 64, 128, 6), (1024, 256, 256, 4)])
+def test_scoring_does_not_depend_on_the_split_of_the_keys(ftk, N, D, bsz, topk):
+    """Few tiles of query rows: clusters share one and split its keys; many: none does.
+    One slice alone and the same slice among 64 others give the same bits."""
+    pad = (0, -N % bsz)
+    t = cases.make_inputs(dict(B=64, N=N, H=1, D=D, dtype="bf16", seed=55, do_seed=56))
+    q, k = t["q"].cuda(), t["k"].cuda()
+    many = ftk.flash_topk_score(q, k, 1, bsz, topk, pad, 0.9)
+    for b in (0, 63):
+        one = ftk.flash_topk_score(q[b:b + 1], k[b:b + 1], 1, bsz, topk, pad, 0.9)
+        for a, x in zip(one, many):
+            assert torch.equal(a[0], x[b])
+    ftk.check_errors()
