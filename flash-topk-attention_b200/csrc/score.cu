@@ -457,7 +457,8 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
 #pragma unroll
       for (int sg = 0; sg < SC_SEGS; sg++) {
         const int r = sg * split / SC_SEGS;
-        tot += ld_cta(&s_seg[0][sg][tid], r, split) + ld_cta(&s_seg[1][sg][tid], r, split);
+        tot += SPLIT ? ld_cta(&s_seg[0][sg][tid], r, split) + ld_cta(&s_seg[1][sg][tid], r, split)
+                     : s_seg[0][sg][tid] + s_seg[1][sg][tid];
       }
       if (q0 + tid < p.N) {
         if (rank == 0) p.row_total[static_cast<size_t>(bh_local) * p.N + q0 + tid] = tot;
@@ -513,7 +514,10 @@ static int score_split(int64_t tiles, int num_tiles, int units, size_t smem) {
     if (c > units) break;
     int n = resident[dev][i].load(std::memory_order_relaxed);
     if (n == 0) {
-      n = c == 1 ? sm_count() : max_clusters(score_kernel<D, true>, c, SC_THREADS, smem);
+      n = c == 1 ? sm_count()
+                 : allow_smem<score_kernel<D, true>>(smem) == FTK_OK
+                       ? max_clusters(score_kernel<D, true>, c, SC_THREADS, smem)
+                       : 0;
       resident[dev][i].store(n > 0 ? n : -1, std::memory_order_relaxed);
     }
     if (n <= 0) continue;
@@ -534,13 +538,13 @@ static int launch_score_d(const CUtensorMap& tq, const CUtensorMap& tk, ScorePar
   const size_t smem =
       1024 + (2 * NCH + score_stages(D) * (NCH / score_ksplit(D))) * SC_CHUNK_BYTES;
   if (int e = allow_smem<score_kernel<D, false>>(smem)) return e;
-  if (int e = allow_smem<score_kernel<D, true>>(smem)) return e;
   const int qtiles = (p.N + SC_QROWS - 1) / SC_QROWS;
   const int split = score_split<D>(qtiles * bh_count, p.num_tiles,
                                    p.num_tiles / std::max(1, p.tiles_per_block), smem);
   const dim3 grid(qtiles * split, static_cast<unsigned>(bh_count));
   if (split == 1)
     return launch_pdl(score_kernel<D, false>, grid, SC_THREADS, smem, st, tq, tk, p);
+  if (int e = allow_smem<score_kernel<D, true>>(smem)) return e;
   return launch_clusters(score_kernel<D, true>, split, grid, SC_THREADS, smem, st, tq, tk, p);
 }
 

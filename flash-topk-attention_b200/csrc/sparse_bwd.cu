@@ -323,6 +323,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   if (warp == 0) {
     if (lane == 0 && n == 0) mbar_wait(bar_q, 0, w, FTK_DEV_TIMEOUT_TMA);   // lands before the exit
     if (lane == 0 && n > 0) {
+      const int hk = h_idx / p.kv_hdiv;   // out of the loop: a division takes 150 cycles
       for (int i = 0; i < n; i++) {
         const int sk = i % KST, sv = i % VST;
         const int tok0 = static_cast<int>(un.ids[i]) * p.kvb - p.kv_pad_head;
@@ -330,7 +331,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
         const uint32_t kb = smem_u32(sK) + sk * tile_bytes;
         mbar_expect_tx(bar_kfull(sk), tile_bytes);
         for (int c = 0; c < NCH; c++)
-          tma_load_4d(kb + c * kv_chunk_bytes, &tm_k, bar_kfull(sk), c * 64, h_idx / p.kv_hdiv,
+          tma_load_4d(kb + c * kv_chunk_bytes, &tm_k, bar_kfull(sk), c * 64, hk,
                       tok0, b_idx);
         // the V ring lies over the Q / dO tiles: wait until they sit in TMEM
         if (!BIG && i == 0 && !mbar_wait(bar_qt, 0, w, FTK_DEV_TIMEOUT_TMA)) break;
@@ -338,7 +339,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
         const uint32_t vb = v_slot(sv);
         mbar_expect_tx(bar_vfull(sv), tile_bytes);
         for (int c = 0; c < NCH; c++)
-          tma_load_4d(vb + c * kv_chunk_bytes, &tm_v, bar_vfull(sv), c * 64, h_idx / p.kv_hdiv,
+          tma_load_4d(vb + c * kv_chunk_bytes, &tm_v, bar_vfull(sv), c * 64, hk,
                       tok0, b_idx);
       }
     }

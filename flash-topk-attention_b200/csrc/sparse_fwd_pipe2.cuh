@@ -144,6 +144,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
       // K entry j: the prologue blocks first, then the union; V entry i: the
       // union only.  Every wait depends on tiles loaded earlier only.
       const int total = npro + n;
+      const int hk = h_idx / p.kv_hdiv;   // out of the loop: a division takes 150 cycles
       const int dcol = D / 2 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
       // BIG: V follows two entries behind K, so that the wait for one of the four
       // V slots (held until P V) does not keep back the K tiles, needed earlier
@@ -157,7 +158,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
           const uint32_t kb = smem_u32(sK) + sk * TILE;
           mbar_expect_tx(bar_kfull(sk), TILE);
           for (int c = 0; c < NCH; c++)
-            tma_load_4d(kb + c * 4096, &tm_k32, bar_kfull(sk), c * 64, h_idx / p.kv_hdiv,
+            tma_load_4d(kb + c * 4096, &tm_k32, bar_kfull(sk), c * 64, hk,
                         tok0 + rsub, b_idx);
         }
         const int i = j - npro - LAG;
@@ -169,7 +170,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
 #pragma unroll
           for (int c = 0; c < NCH / 2; c++)
             tma_load_4d(smem_u32(sV) + sv * TILE + c * 8192, &tm_v, bar_vfull(sv), dcol + c * 64,
-                        h_idx / p.kv_hdiv, tok0, b_idx);
+                        hk, tok0, b_idx);
         }
       }
     }
