@@ -550,18 +550,16 @@ static int tmap_rows(CUtensorMap* out, const ftk_attn& a, char which, int rows) 
                           64, rows);
 }
 
-template <int D>
+template <int D, int NG>
 static int launch_fwd_pipe(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                            const FwdParams& p, int64_t BH, cudaStream_t st) {
-  constexpr int NCH = D / 64;
-  const size_t smem = 1024 + NCH * 128 * 128 +
-                      static_cast<size_t>(FP_KST + FP_VST) * NCH * 64 * 128;
   return choose<2>(p.fmt, [&](auto fmt) {
     return choose<3>(p.sub, [&](auto sub) {
       constexpr int F = decltype(fmt)::value, S = decltype(sub)::value == 2 ? 2 : 1;
-      if (int e = allow_smem<sparse_fwd_pipe_kernel<D, F, S>>(smem)) return e;
-      return launch_pdl(sparse_fwd_pipe_kernel<D, F, S>, dim3(p.tiles_x, static_cast<unsigned>(BH)),
-                        FP_THREADS, smem, st, tq, tk, tv, p);
+      if (int e = allow_smem<sparse_fwd_pipe_kernel<D, F, S, NG>>(fp_smem(D, NG))) return e;
+      return launch_pdl(sparse_fwd_pipe_kernel<D, F, S, NG>,
+                        dim3(p.tiles_x, static_cast<unsigned>(BH)), fp_threads(NG), fp_smem(D, NG),
+                        st, tq, tk, tv, p);
     });
   });
 }
@@ -574,7 +572,7 @@ static int launch_fwd_pipe2(const CUtensorMap& tq, const CUtensorMap& tk32, cons
       constexpr int F = decltype(fmt)::value, S = decltype(sub)::value == 2 ? 2 : 1;
       if (int e = allow_smem<sparse_fwd_pipe2_kernel<D, F, S>>(fp2_smem(D))) return e;
       return launch_pdl(sparse_fwd_pipe2_kernel<D, F, S>,
-                        dim3(2 * ((p.tiles_x + 1) / 2), static_cast<unsigned>(BH)), FP_THREADS,
+                        dim3(2 * ((p.tiles_x + 1) / 2), static_cast<unsigned>(BH)), FP2_THREADS,
                         fp2_smem(D), st, tq, tk32, tv, p);
     });
   });
@@ -661,15 +659,18 @@ static int attn_fwd(const ftk_attn& a, const AttnGrid& gr, void* o, int64_t so_b
     // without).
     // Head dim 256 takes pairs whatever the lists: four disjoint lists cost twice
     // the tiles of two, the one-CTA kernel three times the cycles per tile.
+    // Head dim 64 with at most two q-blocks per tile: two CTAs per SM.
     CUtensorMap tk32;
     if ((e = tmap_rows(&tk32, a, 'k', 32))) return e;
     if (gr.kd == 256)
       e = launch_fwd_pipe2<256>(tq, tk32, tv, p, BH, st);
     else if (gr.kd == 128 && 2 * gr.width >= gr.Mkv && !(env2 && env2[0] == '0'))
       e = launch_fwd_pipe2<128>(tq, tk32, tv, p, BH, st);
+    else if (gr.kd == 128)
+      e = launch_fwd_pipe<128, 4>(tq, tk, tv, p, BH, st);
     else
-      e = gr.kd == 64 ? launch_fwd_pipe<64>(tq, tk, tv, p, BH, st)
-                      : launch_fwd_pipe<128>(tq, tk, tv, p, BH, st);
+      e = p.G <= 2 ? launch_fwd_pipe<64, 2>(tq, tk, tv, p, BH, st)
+                   : launch_fwd_pipe<64, 4>(tq, tk, tv, p, BH, st);
     if (e) return e;
     p.redo_out = nullptr;
     p.redo_in = static_cast<const int*>(workspace);

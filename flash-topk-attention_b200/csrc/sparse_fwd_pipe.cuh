@@ -7,9 +7,21 @@
 // core idles while a group does its exponentials.  Here every row uses ONE
 // fixed reference exponent for the whole list: the scaled maximum of the first
 // kv block its q-block lists (a short prologue computes it).  P = 2^(c S - ref)
-// then needs no rescaling, all tiles add into a single O accumulator, and four
-// softmax groups work on four S buffers at once:
-//   TMEM columns  Q 0..63 | S/P buffers 64,128,192,256 | O 320..447
+// then needs no rescaling, all tiles add into a single O accumulator, and NG
+// softmax groups work on NG S buffers at once:
+//   TMEM columns  Q, D / 2 | S/P buffers, 64 each | O, D
+// With head dim 128, or q-blocks of 32 rows (up to four reference tiles, each in an
+// S buffer), a CTA has four groups and the SM to itself.  With head dim 64 and
+// q-blocks of 64 rows it has two, 256 TMEM columns and half the shared memory, and
+// two CTAs share an SM: as many tiles are in flight, the list union, first loads,
+// reference tiles and last tiles of one CTA (17000 of its 92000 cycles at 128 tiles)
+// run under the tiles of the other, and two warps issue.  The issuing warp bounds the
+// loop otherwise: with 16 softmax warps beside it a round of 8 UMMAs, two commits
+// and two waits takes it 600 cycles, the exponentials 512.  Forward at B = 1, H = 16,
+// N = 8192, all pairs: 404 us with four groups, a K ring and a V ring; 388 with K and
+// V in one ring (two waits and two commits per tile, were three and three) and
+// addresses that the unrolled rounds share; 348 with two CTAs per SM.  Head dim 128,
+// N = 8192, grouped heads: 312 -> 291 us from the ring.
 // bf16 and fp32 share the exponent range, so a later block may exceed the
 // reference by up to 2^80 before anything overflows (fp16: 2^15, P must stay
 // below 65504); a row whose tile sum
@@ -20,12 +32,13 @@
 
 namespace ftk {
 
-constexpr int FP_THREADS = 576;  // TMA warp, UMMA warp, 4 softmax groups x 4 warps
-constexpr int FP_GROUPS = 4;
-constexpr int FP_KST = 4;         // K tiles in the ring (free again once S is computed)
-constexpr int FP_VST = 6;         // V tiles in the ring (held until P V has run)
-constexpr int FP_COL_S = 64;
-constexpr int FP_COL_O = 320;
+__host__ __device__ constexpr int fp_threads(int ng) { return 64 + 128 * ng; }   // TMA, UMMA warps
+// Stages of the ring; a stage holds what one round of the issuing warp reads, V of
+// tile i and K of tile i + ng.  A multiple of ng.
+__host__ __device__ constexpr int fp_stages(int d, int ng) { return d == 64 && ng == 4 ? 8 : 4; }
+constexpr size_t fp_smem(int d, int ng) {
+  return 1024 + (d / 64) * (128 * 128 + static_cast<size_t>(fp_stages(d, ng)) * 2 * 64 * 128);
+}
 // A tile's row sum of P above this marks the CTA for the exact kernel: 2^80 for
 // bf16 (fp32 exponent range), 2^15 for fp16 (P itself must stay below 65504).
 template <int FMT>
@@ -43,8 +56,8 @@ __device__ __forceinline__ uint32_t pack16(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <int D, int FMT, int SUB>
-__global__ void __launch_bounds__(FP_THREADS, 1)
+template <int D, int FMT, int SUB, int NG>
+__global__ void __launch_bounds__(fp_threads(NG), 4 / NG)
 sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
                        const __grid_constant__ CUtensorMap tm_k,
                        const __grid_constant__ CUtensorMap tm_v, const FwdParams p) {
@@ -53,19 +66,22 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
   constexpr int KVB = 64;
   constexpr int CHUNK = KVB * 128;             // one 64-wide chunk of a K or V tile
   constexpr int TILE = NCH * CHUNK;            // one K or V tile
+  constexpr int ST = fp_stages(D, NG), STAGE = 2 * TILE;
+  constexpr int COL_S = D / 2, COL_O = COL_S + 64 * NG;   // Q in the columns before S
+  constexpr int TMEM_COLS = NG == 2 ? 256 : 512;
+  static_assert(COL_O + D <= TMEM_COLS, "TMEM columns");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sQ = smem;
-  uint8_t* sK = smem + Q_BYTES;
-  uint8_t* sV = sK + FP_KST * TILE;
+  uint8_t* sKV = smem + Q_BYTES;               // stage s: K tile, then V tile
   __shared__ UnionScratch un;
-  __shared__ __align__(8) uint64_t bars[4 + 2 * FP_KST + 2 * FP_VST + 2 * FP_GROUPS];
+  __shared__ __align__(8) uint64_t bars[4 + 2 * ST + 2 * NG];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
   __shared__ int s_ovf;
   __shared__ CoverTiles s_pro;
-  __shared__ float s_l[FP_GROUPS][128];
+  __shared__ float s_l[NG][128];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.x * p.G;
@@ -78,13 +94,11 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
   const uint32_t bar_final = smem_u32(&bars[1]);
   const uint32_t bar_qt = smem_u32(&bars[2]);    // Q copied into TMEM
   const uint32_t bar_pro = smem_u32(&bars[3]);   // every softmax warp has its reference
-  auto bar_kfull = [&](int s) { return smem_u32(&bars[4 + s]); };
-  auto bar_kempty = [&](int s) { return smem_u32(&bars[4 + FP_KST + s]); };
-  auto bar_vfull = [&](int s) { return smem_u32(&bars[4 + 2 * FP_KST + s]); };
-  auto bar_vempty = [&](int s) { return smem_u32(&bars[4 + 2 * FP_KST + FP_VST + s]); };
-  constexpr int BAR_S0 = 4 + 2 * FP_KST + 2 * FP_VST;
+  auto bar_full = [&](int s) { return smem_u32(&bars[4 + s]); };
+  auto bar_empty = [&](int s) { return smem_u32(&bars[4 + ST + s]); };
+  constexpr int BAR_S0 = 4 + 2 * ST;
   auto bar_sfull = [&](int b) { return smem_u32(&bars[BAR_S0 + b]); };
-  auto bar_pfull = [&](int b) { return smem_u32(&bars[BAR_S0 + FP_GROUPS + b]); };
+  auto bar_pfull = [&](int b) { return smem_u32(&bars[BAR_S0 + NG + b]); };
 
   if (tid == 0) {
     abort_flag = 0;
@@ -92,16 +106,12 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
     mbar_init(bar_q, 1);
     mbar_init(bar_final, 1);
     mbar_init(bar_qt, 4);
-    mbar_init(bar_pro, 4 * FP_GROUPS);
-    for (int s = 0; s < FP_KST; s++) {
-      mbar_init(bar_kfull(s), 1);
-      mbar_init(bar_kempty(s), 1);
+    mbar_init(bar_pro, 4 * NG);
+    for (int s = 0; s < ST; s++) {
+      mbar_init(bar_full(s), 1);
+      mbar_init(bar_empty(s), 1);
     }
-    for (int s = 0; s < FP_VST; s++) {
-      mbar_init(bar_vfull(s), 1);
-      mbar_init(bar_vempty(s), 1);
-    }
-    for (int b = 0; b < FP_GROUPS; b++) {
+    for (int b = 0; b < NG; b++) {
       mbar_init(bar_sfull(b), 1);
       mbar_init(bar_pfull(b), 4);
     }
@@ -111,20 +121,22 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
     tma_prefetch_desc(&tm_v);
   }
   if (warp == 0) {
-    tmem_alloc(smem_u32(&tmem_base_s), 512);
+    tmem_alloc(smem_u32(&tmem_base_s), TMEM_COLS);
     tmem_relinquish();
   }
   clear_bitmaps(un);
   pdl_wait();
-  pdl_launch();
   const int n = build_union(un, p.merged + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
                             p.W, nullptr, p.Mkv, SUB, p.lm, p.status);
+  // behind a barrier that follows tmem_alloc: a CTA of the next kernel that took the
+  // columns first would keep them until this grid is done
+  pdl_launch();
   // tiles whose scores give the rows their reference exponents
   if (warp == 2) cover_tiles(un, n, groups, SUB, s_pro);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base_s;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base_s, 0);
   WaitCtx w{&abort_flag, p.status};
 
   // prologue entry e goes through S buffer e
@@ -137,28 +149,30 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
       mbar_expect_tx(bar_q, Q_BYTES);
       for (int c = 0; c < NCH; c++)
         tma_load_4d(smem_u32(sQ) + c * 128 * 128, &tm_q, bar_q, c * 64, h_idx, tile_row0, b_idx);
-      // K entry j: the prologue blocks first, then the union; V entry i: the
-      // union only.  Every wait depends on tiles loaded earlier only.
+      // Stage rr holds K of tile rr and V of tile rr - NG; the first NG, which
+      // have no V, take the prologue's K tiles in its place.
+      const int lead = min(n, NG);
       const int hk = h_idx / p.kv_hdiv;   // out of the loop: a division takes 150 cycles
-      const int total = npro + n;
-      for (int j = 0; j < total; j++) {
-        const int sk = j % FP_KST;
-        if (!mbar_wait(bar_kempty(sk), ((j / FP_KST) & 1) ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
-        const bool pro = j < npro;
-        const int id = pro ? pro_block(j) : static_cast<int>(un.ids[j - npro]);
-        const int tok0 = id * KVB - p.kv_pad_head;
-        const uint32_t kb = smem_u32(sK) + sk * TILE;
-        mbar_expect_tx(bar_kfull(sk), TILE);
-        for (int c = 0; c < NCH; c++)
-          tma_load_4d(kb + c * CHUNK, &tm_k, bar_kfull(sk), c * 64, hk, tok0, b_idx);
-        if (!pro) {
-          const int i = j - npro, sv = i % FP_VST;
-          if (!mbar_wait(bar_vempty(sv), ((i / FP_VST) & 1) ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
-          const uint32_t vb = smem_u32(sV) + sv * TILE;
-          mbar_expect_tx(bar_vfull(sv), TILE);
+      for (int rr = 0; rr < n + NG; rr++) {
+        if (rr >= lead && rr < NG) continue;
+        const int s = rr % ST;
+        if (!mbar_wait(bar_empty(s), ((rr / ST) & 1) ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
+        const bool has_k = rr < n, has_pro = rr < npro, has_v = rr >= NG;
+        const uint32_t kb = smem_u32(sKV) + s * STAGE, vb = kb + TILE;
+        mbar_expect_tx(bar_full(s), (has_k && (has_pro || has_v)) ? STAGE : TILE);
+        if (has_v) {
+          const int tok0 = static_cast<int>(un.ids[rr - NG]) * KVB - p.kv_pad_head;
           for (int c = 0; c < NCH; c++)
-            tma_load_4d(vb + c * CHUNK, &tm_v, bar_vfull(sv), c * 64, hk, tok0,
-                        b_idx);
+            tma_load_4d(vb + c * CHUNK, &tm_v, bar_full(s), c * 64, hk, tok0, b_idx);
+        }
+        if (has_pro)
+          for (int c = 0; c < NCH; c++)
+            tma_load_4d(vb + c * CHUNK, &tm_k, bar_full(s), c * 64, hk,
+                        pro_block(rr) * KVB - p.kv_pad_head, b_idx);
+        if (has_k) {
+          const int tok0 = static_cast<int>(un.ids[rr]) * KVB - p.kv_pad_head;
+          for (int c = 0; c < NCH; c++)
+            tma_load_4d(kb + c * CHUNK, &tm_k, bar_full(s), c * 64, hk, tok0, b_idx);
         }
       }
     }
@@ -167,66 +181,64 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
     if (n > 0) {
       const uint32_t idesc_s = umma_idesc(128, KVB, FMT, 0, 0);
       const uint32_t idesc_pv = umma_idesc(128, D, FMT, 0, 1);
-      const uint64_t kdesc0 = smem_desc_sw128(smem_u32(sK), 16, 1024);
-      const uint64_t vdesc0 = smem_desc_sw128(smem_u32(sV), CHUNK, 1024);
+      const uint64_t kdesc0 = smem_desc_sw128(smem_u32(sKV), 16, 1024);
+      const uint64_t vdesc0 = smem_desc_sw128(smem_u32(sKV) + TILE, CHUNK, 1024);
       bool ok = mbar_wait(bar_qt, 0, w, FTK_DEV_TIMEOUT_MMA);
       tc_fence_after();
-      // The tensor core runs dry whenever the issuing thread waits, so every
-      // barrier of a round is waited for first and the round's UMMAs (P V of
-      // tile i, then S of tile i + 4) go out as one uninterrupted batch.
-      auto wait_k = [&](int j) -> bool {
-        return mbar_wait(bar_kfull(j % FP_KST), (j / FP_KST) & 1, w, FTK_DEV_TIMEOUT_MMA);
-      };
-      // S = Q K^T for K entry j into S buffer `buf`; Q read from TMEM (elected lane only)
-      auto mma_s = [&](int j, int buf) {
-        const int s = j % FP_KST;
-        const uint64_t kdesc = desc_advance(kdesc0, s * TILE);
-        const uint32_t d_tmem = tmem + FP_COL_S + buf * 64;
+      // S = Q K^T for the K tile at `off` into S buffer `buf`; Q read from TMEM
+      // (elected lane only)
+      auto mma_s = [&](int off, int buf) {
+        const uint64_t kdesc = desc_advance(kdesc0, off);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ks++)
-          umma_ts(d_tmem, tmem + ks * 8, desc_advance(kdesc, (ks / 4) * CHUNK + (ks % 4) * 32),
-                  idesc_s, ks > 0);
+          umma_ts(tmem + COL_S + buf * 64, tmem + ks * 8,
+                  desc_advance(kdesc, (ks / 4) * CHUNK + (ks % 4) * 32), idesc_s, ks > 0);
         umma_commit(bar_sfull(buf));
-        umma_commit(bar_kempty(s));
       };
-      for (int e = 0; ok && e < npro; e++) ok = wait_k(e);
+      const int lead = min(n, NG);
+      for (int t = 0; ok && t < lead; t++)
+        ok = mbar_wait(bar_full(t), 0, w, FTK_DEV_TIMEOUT_MMA);
       tc_fence_after();
       if (ok && elect_one())
-        for (int e = 0; e < npro; e++) mma_s(e, e);
+        for (int e = 0; e < npro; e++) mma_s(e * STAGE + TILE, e);
       __syncwarp();
       if (ok) ok = mbar_wait(bar_pro, 0, w, FTK_DEV_TIMEOUT_MMA);
-      for (int i = 0; ok && i < FP_GROUPS && i < n; i++) ok = wait_k(npro + i);
       tc_fence_after();
       if (ok && elect_one())
-        for (int i = 0; i < FP_GROUPS && i < n; i++) mma_s(npro + i, i);
+        for (int t = 0; t < lead; t++) {
+          mma_s(t * STAGE, t);
+          umma_commit(bar_empty(t));
+        }
       __syncwarp();
-      for (int i = 0; ok && i < n; i++) {
-        const int j = npro + i;
-        const int s = i % FP_VST, sb = i & (FP_GROUPS - 1);
-        const bool more = i + FP_GROUPS < n;
-        const int j4 = j + FP_GROUPS;
-        const uint32_t wb[3] = {bar_vfull(s), bar_pfull(sb),
-                                more ? bar_kfull(j4 % FP_KST) : bar_pfull(sb)};
-        const uint32_t wp[3] = {static_cast<uint32_t>((i / FP_VST) & 1),
-                                static_cast<uint32_t>((i / FP_GROUPS) & 1),
-                                static_cast<uint32_t>(more ? (j4 / FP_KST) & 1
-                                                           : (i / FP_GROUPS) & 1)};
-        if (!mbar_wait_all<3>(wb, wp, w, FTK_DEV_TIMEOUT_MMA)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint64_t vdesc = desc_advance(vdesc0, s * TILE);
-        if (elect_one()) {
+      // The tensor core runs dry whenever the issuing thread waits, so both
+      // barriers of a round are waited for first and the round's UMMAs (P V of
+      // tile i, then S of tile i + NG) go out as one uninterrupted batch.
+      for (int q = 0; ok && q * NG < n; q++) {
+        const int s0 = ((q + 1) * NG) % ST;
+        const uint32_t full_ph = ((q + 1) * NG / ST) & 1, p_ph = q & 1;
 #pragma unroll
-          for (int ks = 0; ks < KVB / 16; ks++)
-            umma_ts(tmem + FP_COL_O, tmem + FP_COL_S + sb * 64 + ks * 8,
-                    desc_advance(vdesc, ks * 2048), idesc_pv, (i > 0) || (ks > 0));
-          umma_commit(bar_vempty(s));
-          // S(i+4) lands on the columns PV(i) reads P from; UMMAs run in issue order
-          if (i + FP_GROUPS < n) mma_s(j + FP_GROUPS, sb);
+        for (int u = 0; u < NG; u++) {
+          const int i = q * NG + u, s = s0 + u;
+          if (i >= n) break;
+          const uint32_t wb[2] = {bar_full(s), bar_pfull(u)};
+          const uint32_t wp[2] = {full_ph, p_ph};
+          if (!mbar_wait_all<2>(wb, wp, w, FTK_DEV_TIMEOUT_MMA)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          if (elect_one()) {
+            const uint64_t vdesc = desc_advance(vdesc0, s * STAGE);
+#pragma unroll
+            for (int ks = 0; ks < KVB / 16; ks++)
+              umma_ts(tmem + COL_O, tmem + COL_S + u * 64 + ks * 8,
+                      desc_advance(vdesc, ks * 2048), idesc_pv, (i > 0) || (ks > 0));
+            // S(i + NG) lands on the columns PV(i) reads P from; UMMAs run in issue order
+            if (i + NG < n) mma_s(s * STAGE, u);
+            umma_commit(bar_empty(s));
+          }
+          __syncwarp();
         }
-        __syncwarp();
       }
       if (ok && elect_one()) umma_commit(bar_final);
       __syncwarp();
@@ -240,7 +252,7 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int qrow = tile_row0 + r;
     const bool row_valid = (grp < groups) && qrow >= 0 && qrow < p.N;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
-    const uint32_t s_addr = lane_addr + FP_COL_S + gw * 64;
+    const uint32_t s_addr = lane_addr + COL_S + gw * 64;
     const float c = p.scale_log2;
     float mref = 0.f, l = 0.f;
     bool ok = true, ovf = false;
@@ -285,8 +297,8 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
           const ColSpan cs = col_span(un, s_pro.entry[pb], SUB, grp, tok0, KVB, p.N);
           const int lo = cs.lo, hi = cs.hi;
           uint32_t v0[32], v1[32];
-          tmem_ld32(lane_addr + FP_COL_S + pb * 64, v0);
-          tmem_ld32(lane_addr + FP_COL_S + pb * 64 + 32, v1);
+          tmem_ld32(lane_addr + COL_S + pb * 64, v0);
+          tmem_ld32(lane_addr + COL_S + pb * 64 + 32, v1);
           tmem_wait_ld();
           float mx = -INFINITY;
 #pragma unroll
@@ -304,9 +316,9 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
 
     const float2 c2 = make_float2(c, c);
     const float2 nm = make_float2(-mref, -mref);
-    for (int i = gw; ok && i < n; i += FP_GROUPS) {
-      // S(i) complete also means PV(i-4) has retired: the P columns are free
-      const int u = (gw < npro ? 1 : 0) + (i / FP_GROUPS);
+    for (int i = gw; ok && i < n; i += NG) {
+      // S(i) complete also means PV(i - NG) has retired: the P columns are free
+      const int u = (gw < npro ? 1 : 0) + (i / NG);
       if (!mbar_wait(bar_sfull(gw), u & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
         ok = false;
         break;
@@ -387,15 +399,17 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
 
     // ------------------------------------------------------------ epilogue
-    // row sums of the four groups add up (same reference); each group converts
+    // row sums of the groups add up (same reference); each group converts
     // and stores a quarter of the head dimension
     s_l[gw][r] = l;
     if (ovf) atomicOr(&s_ovf, 1);
-    asm volatile("bar.sync 1, 512;" ::: "memory");
+    asm volatile("bar.sync 1, %0;" ::"n"(128 * NG) : "memory");
     if (ok && n > 0) ok = mbar_wait(bar_final, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
     if (ok) {
       tc_fence_after();
-      const float lt = ((s_l[0][r] + s_l[1][r]) + s_l[2][r]) + s_l[3][r];
+      float lt = s_l[0][r];
+#pragma unroll
+      for (int x = 1; x < NG; x++) lt += s_l[x][r];
       const bool have = (n > 0) && lt > 0.f;
       const float inv = have ? 1.f / lt : 0.f;
       uint8_t* orow = nullptr;
@@ -404,12 +418,12 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
                (p.out_f32 ? 4 : 2) *
                    (static_cast<int64_t>(b_idx) * p.so_b + static_cast<int64_t>(qrow) * p.so_n +
                     static_cast<int64_t>(h_idx) * p.so_h);
-      constexpr int QUART = D / 4;   // 32 or 16 columns per group
+      constexpr int QUART = D / NG;   // 32 or 16 columns per group
       const int c0 = gw * QUART;
       uint32_t ov[QUART];
       if (n > 0) {
-        if constexpr (QUART == 32) tmem_ld32(lane_addr + FP_COL_O + c0, ov);
-        else tmem_ld16(lane_addr + FP_COL_O + c0, ov);
+        if constexpr (QUART == 32) tmem_ld32(lane_addr + COL_O + c0, ov);
+        else tmem_ld16(lane_addr + COL_O + c0, ov);
         tmem_wait_ld();
       }
       if (row_valid) {
@@ -433,7 +447,7 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
   if (tid == 0 && p.redo_out) p.redo_out[blockIdx.y * gridDim.x + blockIdx.x] = s_ovf;
   if (abort_flag)
     for (int i = 0; i < 200; i++) __nanosleep(1000);
-  if (warp == 0) tmem_dealloc(tmem, 512);
+  if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
 }
 
 }  // namespace ftk

@@ -27,6 +27,8 @@
 
 namespace ftk {
 
+constexpr int FP2_THREADS = 576;   // TMA warp, UMMA warp, 4 softmax groups x 4 warps
+constexpr int FP2_GROUPS = 4;
 __host__ __device__ constexpr int fp2_kst(int d) { return d > 128 ? 4 : 6; }   // K half tiles
 __host__ __device__ constexpr int fp2_vst(int d) { return d > 128 ? 4 : 8; }   // V half tiles
 __host__ __device__ constexpr int fp2_tile(int d) { return d * 64; }           // bytes of either
@@ -36,7 +38,7 @@ __host__ __device__ constexpr size_t fp2_smem(int d) {
 }
 
 template <int D, int FMT, int SUB>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FP_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FP2_THREADS, 1)
 sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
                         const __grid_constant__ CUtensorMap tm_k32,
                         const __grid_constant__ CUtensorMap tm_v, const FwdParams p) {
@@ -47,7 +49,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
   constexpr int TILE = fp2_tile(D);            // half a K tile (32 rows x D) or half a V tile
                                                // (64 rows x D / 2)
   constexpr int FP2_KST = fp2_kst(D), FP2_VST = fp2_vst(D);
-  constexpr uint32_t COL_S = BIG ? 0 : FP_COL_S, COL_O = BIG ? 256 : FP_COL_O;
+  constexpr uint32_t COL_S = BIG ? 0 : 64, COL_O = BIG ? 256 : 320;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -55,12 +57,12 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
   uint8_t* sK = smem + Q_BYTES;
   uint8_t* sV = sK + FP2_KST * TILE;
   __shared__ UnionScratch un;
-  __shared__ __align__(8) uint64_t bars[4 + 3 * FP2_KST + 3 * FP2_VST + 2 * FP_GROUPS];
+  __shared__ __align__(8) uint64_t bars[4 + 3 * FP2_KST + 3 * FP2_VST + 2 * FP2_GROUPS];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
   __shared__ int s_ovf;
   __shared__ CoverTiles s_pro;
-  __shared__ float s_l[FP_GROUPS][128];
+  __shared__ float s_l[FP2_GROUPS][128];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
@@ -85,7 +87,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
   auto bar_peer_v = [&](int s) { return smem_u32(&bars[BAR_V0 + 2 * FP2_VST + s]); };   // CTA 0 only
   constexpr int BAR_S0 = 4 + 3 * FP2_KST + 3 * FP2_VST;
   auto bar_sfull = [&](int b) { return smem_u32(&bars[BAR_S0 + b]); };
-  auto bar_pfull = [&](int b) { return smem_u32(&bars[BAR_S0 + FP_GROUPS + b]); };
+  auto bar_pfull = [&](int b) { return smem_u32(&bars[BAR_S0 + FP2_GROUPS + b]); };
 
   if (tid == 0) {
     abort_flag = 0;
@@ -93,7 +95,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
     mbar_init(bar_q, 1);
     mbar_init(bar_final, 1);
     mbar_init(bar_qt, BIG ? 1 : 8);        // the 4 copying warps of each CTA
-    mbar_init(bar_pro, 8 * FP_GROUPS);     // the 16 softmax warps of each CTA
+    mbar_init(bar_pro, 8 * FP2_GROUPS);     // the 16 softmax warps of each CTA
     for (int s = 0; s < FP2_KST; s++) {
       mbar_init(bar_kfull(s), 1);
       mbar_init(bar_kempty(s), 1);
@@ -104,7 +106,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
       mbar_init(bar_vempty(s), 1);
       mbar_init(bar_peer_v(s), 1);
     }
-    for (int b = 0; b < FP_GROUPS; b++) {
+    for (int b = 0; b < FP2_GROUPS; b++) {
       mbar_init(bar_sfull(b), 1);
       mbar_init(bar_pfull(b), 8);          // the group's 4 warps in each CTA
     }
@@ -239,19 +241,19 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
         for (int e = 0; e < npro; e++) mma_s(e, e);
       __syncwarp();
       if (ok) ok = mbar_wait(bar_pro, 0, w, FTK_DEV_TIMEOUT_MMA);
-      for (int i = 0; ok && i < FP_GROUPS && i < n; i++) ok = wait_k(npro + i);
+      for (int i = 0; ok && i < FP2_GROUPS && i < n; i++) ok = wait_k(npro + i);
       tc_fence_after();
       if (ok && elect_one())
-        for (int i = 0; i < FP_GROUPS && i < n; i++) mma_s(npro + i, i);
+        for (int i = 0; i < FP2_GROUPS && i < n; i++) mma_s(npro + i, i);
       __syncwarp();
       // per round every barrier is waited for first (together), then P V of
       // tile i and S of tile i + 4 go out as one batch
       for (int i = 0; ok && i < n; i++) {
         const int j = npro + i;
-        const int s = i % FP2_VST, sb = i & (FP_GROUPS - 1);
-        const bool more = i + FP_GROUPS < n;
-        const int j4 = j + FP_GROUPS;
-        const uint32_t pf = bar_pfull(sb), pfp = (i / FP_GROUPS) & 1;
+        const int s = i % FP2_VST, sb = i & (FP2_GROUPS - 1);
+        const bool more = i + FP2_GROUPS < n;
+        const int j4 = j + FP2_GROUPS;
+        const uint32_t pf = bar_pfull(sb), pfp = (i / FP2_GROUPS) & 1;
         const uint32_t vph = (i / FP2_VST) & 1, kph = (j4 / FP2_KST) & 1;
         const uint32_t wb[5] = {bar_vfull(s), bar_peer_v(s), pf,
                                 more ? bar_kfull(j4 % FP2_KST) : pf,
@@ -350,9 +352,9 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
 
     const float2 c2 = make_float2(c, c);
     const float2 nm = make_float2(-mref, -mref);
-    for (int i = gw; ok && i < n; i += FP_GROUPS) {
+    for (int i = gw; ok && i < n; i += FP2_GROUPS) {
       // S(i) complete also means PV(i-4) has retired: the P columns are free
-      const int u = (gw < npro ? 1 : 0) + (i / FP_GROUPS);
+      const int u = (gw < npro ? 1 : 0) + (i / FP2_GROUPS);
       if (!mbar_wait(bar_sfull(gw), u & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
         ok = false;
         break;

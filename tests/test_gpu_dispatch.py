@@ -215,3 +215,25 @@ def test_scoring_does_not_depend_on_the_split_of_the_keys(ftk, N, D, bsz, topk):
         for a, x in zip(one, many):
             assert torch.equal(a[0], x[b])
     ftk.check_errors()
+
+
+@pytest.mark.parametrize("D,g", [(64, 64), (64, 32), (64, 128), (128, 64)])
+def test_forward_ring(ftk, D, g):
+    """Lists of 0, 1, 2, ... 13 tiles: fewer than the softmax groups, fewer than the
+    stages of the ring, and more than one turn of it, on grids whose CTAs share an SM
+    and on those where they do not (fp16: the plain bound)."""
+    B, H, N, kvb = 2, 8, 1024, 64
+    M, QM = N // kvb, N // g
+    t = cases.make_inputs(dict(B=B, N=N, H=H, D=D, dtype="fp16", seed=51, do_seed=52))
+    merged = np.full((B, H, QM, M), -1, dtype=np.int32)
+    for m in range(QM):
+        n = (m * g // 128) % 14      # as long for every q-block of a tile: the union's size
+        for h in range(H):
+            merged[:, h, m, :n] = (np.arange(n) + 3 * h) % M
+    o, lse = ftk.flash_topk_attn(t["q"].cuda(), t["k"].cuda(), t["v"].cuda(),
+                                 torch.from_numpy(merged).cuda(), None, H, g, kvb)
+    ftk.check_errors()
+    want_o, want_lse = orc.sparse_attn_fwd(t["q"].float().numpy(), t["k"].float().numpy(),
+                                           t["v"].float().numpy(), merged, H, g, kvb)
+    np.testing.assert_allclose(lse.cpu().numpy(), want_lse, atol=2e-3, rtol=1e-2)
+    assert (tolerance.rel_err(o.float().cpu().numpy(), want_o) <= 1).all()
