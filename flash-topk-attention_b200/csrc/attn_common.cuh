@@ -124,6 +124,11 @@ __device__ __forceinline__ void clear_bitmaps(UnionScratch& u) {
 // first + groups - 1 of the kernel's grid; `lists` is the slice's first list of
 // `width` entries (or counts[g] of them when given); negative ids are skipped,
 // ids >= num_blocks reported through `status`.  Returns the union size.
+// FOLD: ascending lists have four ids in one word of the bitmap, and one atomic marks
+// them.  In the one-CTA kernels, whose lists are short and whose unions weigh (lists of
+// 16 blocks, B = 2, N = 4096, H = 32: forward 291 -> 288, dQ 380 -> 377 us; head dim 64,
+// B = 2, N = 2048, H = 16: 70.4 -> 68.8 and 103.6 -> 101.1); the pairs lose 1 to 2 %.
+template <bool FOLD = false>
 __device__ __forceinline__ int build_union(UnionScratch& u, const int32_t* lists, int first,
                                            int groups, int width, const int32_t* counts,
                                            int num_blocks, int sub, const ListMap& lm,
@@ -162,6 +167,14 @@ __device__ __forceinline__ int build_union(UnionScratch& u, const int32_t* lists
                                  : make_int4(-1, -1, -1, -1);
 #pragma unroll
         for (int x = 0; x < 4; x++) {
+          const int a = t[x].x, b = t[x].y, c = t[x].z, d = t[x].w;
+          if (FOLD && (a & b & c & d) < 0) continue;
+          if (FOLD && lm.kv_shift == 0 && ((a ^ b) | (a ^ c) | (a ^ d)) < 32 && (a | 31) < num_blocks &&
+              ((a ^ b) | (a ^ c) | (a ^ d) | a) >= 0) {
+            atomicOr(&u.bm[g0 + x][a >> 5],
+                     (1u << (a & 31)) | (1u << (b & 31)) | (1u << (c & 31)) | (1u << (d & 31)));
+            continue;
+          }
           mark(g0 + x, t[x].x);
           mark(g0 + x, t[x].y);
           mark(g0 + x, t[x].z);

@@ -306,7 +306,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   }
   TileDelta<D> delta;
   if (D <= 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);
-  const int n = build_union(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
+  const int n = build_union<true>(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
                             p.W, nullptr, p.Mkv, p.sub, p.lm, p.status);
   if (D > 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);   // too many registers to hold across the union
   delta.finish(p, s_delta, bh, tile_row0, groups * p.g);
