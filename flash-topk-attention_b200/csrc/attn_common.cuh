@@ -127,7 +127,8 @@ __device__ __forceinline__ void clear_bitmaps(UnionScratch& u) {
 // FOLD: ascending lists have four ids in one word of the bitmap, and one atomic marks
 // them.  In the one-CTA kernels, whose lists are short and whose unions weigh (lists of
 // 16 blocks, B = 2, N = 4096, H = 32: forward 291 -> 288, dQ 380 -> 377 us; head dim 64,
-// B = 2, N = 2048, H = 16: 70.4 -> 68.8 and 103.6 -> 101.1); the pairs lose 1 to 2 %.
+// B = 2, N = 2048, H = 16: 70.4 -> 68.8 and 103.6 -> 101.1); the pairs and one
+// CTA per SM at head dim 64 lose 1 to 2 %.
 template <bool FOLD = false>
 __device__ __forceinline__ int build_union(UnionScratch& u, const int32_t* lists, int first,
                                            int groups, int width, const int32_t* counts,

@@ -29,8 +29,11 @@ namespace ftk {
 
 constexpr int BW_THREADS = 576;  // 2 + 2 x 8 warps
 constexpr int BW_MAX_STAGES = 4;
-constexpr int DQ_KST = 7;        // dQ kernel: K tiles in the ring (held until dQ += dS K ran)
-constexpr int DQ_VST = 5;        // dQ kernel: V tiles in the ring (free once dP is computed)
+// A one-CTA kernel with ng groups of 8 warps; with one group two CTAs share an SM.
+__host__ __device__ constexpr int bw_threads(int ng) { return 64 + 256 * ng; }
+// dQ kernel: K tiles in the ring (held until dQ += dS K ran), V tiles (free once dP is computed)
+__host__ __device__ constexpr int dq_kst(int ng) { return ng == 1 ? 6 : 7; }
+constexpr int DQ_VST = 5;
 
 struct BwdParams {
   int N, H, D, QM, W, Mkv;
@@ -71,9 +74,9 @@ struct BwdParams {
 // D = 128 (122 us at B = 4, N = 8192, H = 16), reading O and dO at 4.2 TB/s;
 // here the reads hide behind the other CTAs' UMMAs.
 // The loads are issued before the union is built and used after it.
-template <int KD>
+template <int KD, int THREADS = BW_THREADS>
 struct TileDelta {
-  static constexpr int LPR = KD / 8, RPW = 32 / LPR, WARPS = BW_THREADS / 32;
+  static constexpr int LPR = KD / 8, RPW = 32 / LPR, WARPS = THREADS / 32;
   static constexpr int STEPS = (128 + RPW * WARPS - 1) / (RPW * WARPS);
   uint4 vd[STEPS], vo[STEPS], vo2[STEPS];   // vo2: float32 O only
 
@@ -202,18 +205,20 @@ __device__ __forceinline__ void pt_pairs(const uint32_t (&sv)[16], const uint32_
 }
 
 // ---------------------------------------------------------------------- dQ
-// TMEM columns: Q 0..63 and dO 64..127 (16-bit pairs: the A operands of the
+// TMEM columns: Q and dO, D / 2 each (16-bit pairs: the A operands of the
 // S and dP UMMAs are read from TMEM, which leaves shared-memory bandwidth to
-// the K/V tiles), S[2] 128/192, dP[2] 256/320 (dS written over their first
-// half), dQ 384..
+// the K/V tiles), S[NG] and dP[NG], 64 each (dS written over the first half of
+// dP), dQ.
 // Shared memory: the Q and dO tiles are dead once they sit in TMEM, so their
 // 2 x 128 rows become four slots of the V ring (the fifth follows the K ring);
 // K has its own ring.  K and V travel in
 // separate rings because V is released after dP while K stays until dQ: the
 // producer runs several tiles ahead, which is what lets the loads overlap the
 // UMMAs instead of alternating with them.
-template <int D>
-__global__ void __launch_bounds__(BW_THREADS, 1)
+// One group of warps (head dim 64): one S and one dP buffer, 256 TMEM columns, two CTAs
+// per SM.  See one_group for when.
+template <int D, int NG>
+__global__ void __launch_bounds__(bw_threads(NG), 2 / NG)
 sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
                      const __grid_constant__ CUtensorMap tm_do,
                      const __grid_constant__ CUtensorMap tm_k,
@@ -225,8 +230,11 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   // rings shrink to three K and two V tiles of at most 32 rows, all behind
   // the Q / dO tiles.  TMEM: S[2] 0/64, dP[2] 128/192, dQ 256..511.
   constexpr bool BIG = D > 128;
+  constexpr int DQ_KST = dq_kst(NG);
   constexpr int KST = BIG ? 3 : DQ_KST, VST = BIG ? 2 : DQ_VST;
-  constexpr uint32_t COL_S = BIG ? 0 : 128, COL_DP = BIG ? 128 : 256, COL_DQ = BIG ? 256 : 384;
+  constexpr uint32_t COL_S = BIG ? 0 : D, COL_DP = COL_S + 64 * NG, COL_DQ = COL_DP + 64 * NG;
+  constexpr uint32_t TMEM_COLS = 256 * NG;
+  static_assert(COL_DQ + D <= TMEM_COLS, "TMEM columns");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -236,7 +244,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   uint8_t* sK = smem + 2 * ROW_TILE_BYTES;
   __shared__ UnionScratch un;
   __shared__ float s_delta[128];
-  __shared__ __align__(8) uint64_t bars[1 + 2 * DQ_KST + 2 * DQ_VST + 6];
+  __shared__ __align__(8) uint64_t bars[1 + 2 * DQ_KST + 2 * DQ_VST + 2 * NG + 2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
 
@@ -261,11 +269,11 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   auto bar_vempty = [&](int s) { return smem_u32(&bars[1 + 2 * DQ_KST + DQ_VST + s]); };
   constexpr int BAR_A0 = 1 + 2 * DQ_KST + 2 * DQ_VST;
   auto bar_afull = [&](int s) { return smem_u32(&bars[BAR_A0 + s]); };
-  auto bar_dsfull = [&](int s) { return smem_u32(&bars[BAR_A0 + 2 + s]); };
+  auto bar_dsfull = [&](int s) { return smem_u32(&bars[BAR_A0 + NG + s]); };
   // arrives once, after the last UMMA of the CTA has retired
-  const uint32_t bar_final = smem_u32(&bars[BAR_A0 + 4]);
+  const uint32_t bar_final = smem_u32(&bars[BAR_A0 + 2 * NG]);
   // Q and dO copied from shared memory into TMEM by the compute warps
-  const uint32_t bar_qt = smem_u32(&bars[BAR_A0 + 5]);
+  const uint32_t bar_qt = smem_u32(&bars[BAR_A0 + 2 * NG + 1]);
 
   if (tid == 0) {
     abort_flag = 0;
@@ -278,7 +286,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       mbar_init(bar_vfull(s), 1);
       mbar_init(bar_vempty(s), 1);
     }
-    for (int s = 0; s < 2; s++) {
+    for (int s = 0; s < NG; s++) {
       mbar_init(bar_afull(s), 1);
       mbar_init(bar_dsfull(s), 8);  // one arrival per warp of the owning group
     }
@@ -291,12 +299,12 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
     tma_prefetch_desc(&tm_v);
   }
   if (warp == 0) {
-    tmem_alloc(smem_u32(&tmem_base_s), 512);
+    tmem_alloc(smem_u32(&tmem_base_s), TMEM_COLS);
     tmem_relinquish();
   }
   clear_bitmaps(un);
   pdl_wait();
-  pdl_launch();
+  if (NG == 2) pdl_launch();
   if (tid == 0) {   // under the building of the union
     mbar_expect_tx(bar_q, 2 * ROW_TILE_BYTES);
     for (int c = 0; c < NCH; c++) {
@@ -304,10 +312,11 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       tma_load_4d(smem_u32(sDO) + c * 128 * 128, &tm_do, bar_q, c * 64, h_idx, tile_row0, b_idx);
     }
   }
-  TileDelta<D> delta;
+  TileDelta<D, bw_threads(NG)> delta;
   if (D <= 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);
-  const int n = build_union<true>(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
+  const int n = build_union<NG == 1 || D == 128>(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
                             p.W, nullptr, p.Mkv, p.sub, p.lm, p.status);
+  if (NG == 1) pdl_launch();   // behind tmem_alloc, see sparse_fwd_pipe_kernel
   if (D > 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);   // too many registers to hold across the union
   delta.finish(p, s_delta, bh, tile_row0, groups * p.g);
   if (p.masks)
@@ -316,7 +325,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base_s;
+  const uint32_t tmem = NG == 2 ? tmem_base_s : __shfl_sync(0xffffffffu, tmem_base_s, 0);
   WaitCtx w{&abort_flag, p.status};
   const bool split = (p.kvb % 32) == 0;   // kv columns of a tile shared by two warps per row
 
@@ -364,7 +373,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       tc_fence_after();
       // The tensor core runs dry whenever the issuing thread waits, so every
       // barrier of a round is waited for first and the round's UMMAs (dQ of
-      // tile i, then S and dP of tile i + 2) go out as one uninterrupted batch.
+      // tile i, then S and dP of tile i + NG) go out as one uninterrupted batch.
       auto wait_kv = [&](int i) -> bool {
         return mbar_wait(bar_kfull(i % KST), (i / KST) & 1, w, FTK_DEV_TIMEOUT_MMA) &&
                mbar_wait(bar_vfull(i % VST), (i / VST) & 1, w, FTK_DEV_TIMEOUT_MMA);
@@ -373,7 +382,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
         const int sk = i % KST, sv = i % VST;
         const uint64_t kdesc = desc_advance(kdesc0, sk * tile_bytes);
         const uint64_t vdesc = smem_desc_sw128(v_slot(sv), 16, 1024);
-        const uint32_t sb = i & 1;
+        const uint32_t sb = i % NG;
 #pragma unroll
         for (int ks = 0; ks < D / 16; ks++) {
           const uint32_t koff = (ks / 4) * kv_chunk_bytes + (ks % 4) * 32;
@@ -382,7 +391,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
                     desc_advance(qdesc0, (ks / 4) * 128 * 128 + (ks % 4) * 32),
                     desc_advance(kdesc, koff), idesc_a, ks > 0);
           else
-            umma_ts(tmem + 128 + sb * 64, tmem + ks * 8, desc_advance(kdesc, koff), idesc_a,
+            umma_ts(tmem + COL_S + sb * 64, tmem + ks * 8, desc_advance(kdesc, koff), idesc_a,
                     ks > 0);
         }
 #pragma unroll
@@ -393,14 +402,14 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
                     desc_advance(dodesc0, (ks / 4) * 128 * 128 + (ks % 4) * 32),
                     desc_advance(vdesc, koff), idesc_a, ks > 0);
           else
-            umma_ts(tmem + 256 + sb * 64, tmem + 64 + ks * 8, desc_advance(vdesc, koff), idesc_a,
+            umma_ts(tmem + COL_DP + sb * 64, tmem + D / 2 + ks * 8, desc_advance(vdesc, koff), idesc_a,
                     ks > 0);
         }
         umma_commit(bar_afull(sb));
         umma_commit(bar_vempty(sv));
       };
       auto mma_b = [&](int i) {   // elected lane only
-        const int s = i % KST, sb = i & 1;
+        const int s = i % KST, sb = i % NG;
         const uint64_t kmn = desc_advance(kmn0, s * tile_bytes);
         if (p.kvb == 64) {
 #pragma unroll
@@ -415,27 +424,27 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
         umma_commit(bar_kempty(s));
       };
       if (ok) ok = wait_kv(0);
-      if (ok && n > 1) ok = wait_kv(1);
+      if (ok && NG > 1 && n > 1) ok = wait_kv(1);
       tc_fence_after();
       if (ok && elect_one()) {
         mma_a(0);
-        if (n > 1) mma_a(1);
+        if (NG > 1 && n > 1) mma_a(1);
       }
       __syncwarp();
       for (int i = 0; ok && i < n; i++) {
-        const bool more = i + 2 < n;
-        const int i2 = more ? i + 2 : i;   // last rounds: the dS barrier stands in
-        const uint32_t wb[3] = {bar_dsfull(i & 1),
-                                more ? bar_kfull(i2 % KST) : bar_dsfull(i & 1),
-                                more ? bar_vfull(i2 % VST) : bar_dsfull(i & 1)};
-        const uint32_t wp[3] = {static_cast<uint32_t>((i >> 1) & 1),
-                                static_cast<uint32_t>(more ? (i2 / KST) & 1 : (i >> 1) & 1),
-                                static_cast<uint32_t>(more ? (i2 / VST) & 1 : (i >> 1) & 1)};
+        const bool more = i + NG < n;
+        const int i2 = more ? i + NG : i;   // last rounds: the dS barrier stands in
+        const uint32_t wb[3] = {bar_dsfull(i % NG),
+                                more ? bar_kfull(i2 % KST) : bar_dsfull(i % NG),
+                                more ? bar_vfull(i2 % VST) : bar_dsfull(i % NG)};
+        const uint32_t wp[3] = {static_cast<uint32_t>((i / NG) & 1),
+                                static_cast<uint32_t>(more ? (i2 / KST) & 1 : (i / NG) & 1),
+                                static_cast<uint32_t>(more ? (i2 / VST) & 1 : (i / NG) & 1)};
         if (!mbar_wait_all<3>(wb, wp, w, FTK_DEV_TIMEOUT_MMA)) break;
         tc_fence_after();
         if (elect_one()) {
           mma_b(i);
-          if (i + 2 < n) mma_a(i + 2);
+          if (i + NG < n) mma_a(i + NG);
         }
         __syncwarp();
       }
@@ -443,7 +452,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       __syncwarp();
     }
   } else {
-    // Two groups of 8 warps; group w drains the buffers of tiles i = w (mod 2).
+    // NG groups of 8 warps; group w drains the buffers of tiles i = w (mod NG).
     // Inside a group two warps share each 32-row lane quarter and take one
     // half of the kv columns each, so a tile's latency-bound per-thread work
     // is 32 columns long and 4 compute warps per scheduler hide each other.
@@ -467,12 +476,13 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       dl = s_delta[r];
     }
     bool ok = true;
-    if (!BIG && n > 0 && colhalf == 0) {
+    const int copies = NG == 2 ? wg : colhalf;   // Q or dO
+    if (!BIG && n > 0 && (NG == 1 || colhalf == 0)) {
       // group 0 moves the Q tile, group 1 the dO tile, from (swizzled) shared
       // memory into TMEM: row r -> lane r, two 16-bit values per column
       ok = mbar_wait(bar_q, 0, w, FTK_DEV_TIMEOUT_CONSUMER);
       if (ok) {
-        const uint8_t* src = wg == 0 ? sQ : sDO;
+        const uint8_t* src = copies == 0 ? sQ : sDO;
 #pragma unroll
         for (int ch = 0; ch < NCH; ch++) {
           uint32_t v[32];
@@ -485,7 +495,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
             v[j * 4 + 2] = t4.z;
             v[j * 4 + 3] = t4.w;
           }
-          tmem_st32(lane_addr + wg * 64 + ch * 32, v);
+          tmem_st32(lane_addr + copies * (D / 2) + ch * 32, v);
         }
         tmem_wait_st();
         tc_fence_before();
@@ -493,8 +503,8 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_qt);
     }
-    for (int i = wg; ok && i < n; i += 2) {
-      // A(i) complete also means B(i-2) has retired (same issue order), so the
+    for (int i = wg; ok && i < n; i += NG) {
+      // A(i) complete also means B(i - NG) has retired (same issue order), so the
       // dS columns of this buffer are free again.
       // what the tile's columns mean to this row: worked out before the wait
       const int tok0 = static_cast<int>(un.ids[i]) * p.kvb - p.kv_pad_head;
@@ -503,7 +513,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       const bool act = row_valid && cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == p.kvb;
       const bool none = !fast && !__any_sync(0xffffffffu, act);
-      if (!mbar_wait(bar_afull(wg), (i >> 1) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
+      if (!mbar_wait(bar_afull(wg), (i / NG) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
         ok = false;
         break;
       }
@@ -600,7 +610,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   __syncthreads();
   if (abort_flag)
     for (int i = 0; i < 200; i++) __nanosleep(1000);
-  if (warp == 0) tmem_dealloc(tmem, 512);
+  if (warp == 0) tmem_dealloc(tmem, TMEM_COLS);
 }
 
 // -------------------------------------------------------------------- dK/dV
@@ -1278,6 +1288,17 @@ static int tmap_of(CUtensorMap* t, const ftk_attn& a, const Rows& r, int rows) {
   return encode_tmap_bnhd(t, r.base, a.dtype, a.B, a.N, r.heads, a.D, r.sb, r.sn, r.sh, 64, rows);
 }
 
+// Two CTAs of one group per SM, or one CTA of two?  Two CTAs cover each other's list
+// union, first loads and last tile, but go by twice the CTAs per wave.  A CTA's time
+// with n tiles is 10.4 + 0.49 n us alone and 13.8 + 0.95 n us as one of two (from
+// N = 8192, H = 16, all pairs: 509 and 539 us in 7 and 4 waves; N = 2048, B = 2, H = 16:
+// 104 and 88 us in 4 and 2).
+static bool one_group(int64_t ctas, int tiles) {
+  const int64_t sms = sm_count();
+  return ((ctas + 2 * sms - 1) / (2 * sms)) * (13.8 + 0.95 * tiles) <
+         ((ctas + sms - 1) / sms) * (10.4 + 0.49 * tiles);
+}
+
 static int launch_dq(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, bool pair,
                      cudaStream_t st) {
   const Rows q = {a.q, a.H, a.sq_b, a.sq_n, a.sq_h}, k = {a.k, a.Hkv, a.sk_b, a.sk_n, a.sk_h},
@@ -1318,18 +1339,22 @@ static int launch_dq(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, b
     // Q and dO resident, three K and two V tiles behind them: kv blocks of at most 32 rows
     if (p.kvb > 32) return FTK_ERR_UNSUPPORTED;
     const size_t smem = 1024 + 2 * nch * 128 * 128 + static_cast<size_t>(3 + 2) * nch * p.kvb * 128;
-    if ((e = allow_smem<sparse_bwd_dq_kernel<256>>(smem))) return e;
-    return launch_pdl(sparse_bwd_dq_kernel<256>, grid, BW_THREADS, smem, st, tq, tdo, tk, tv, p);
+    if ((e = allow_smem<sparse_bwd_dq_kernel<256, 2>>(smem))) return e;
+    return launch_pdl(sparse_bwd_dq_kernel<256, 2>, grid, BW_THREADS, smem, st, tq, tdo, tk, tv, p);
   }
-  // four V slots lie over the Q / dO tiles, the rest of the V ring behind the K ring
-  const size_t smem = 1024 + 2 * nch * 128 * 128 +
-                      static_cast<size_t>(DQ_KST + DQ_VST - 4) * nch * p.kvb * 128;
-  if (kd == 64) {
-    if ((e = allow_smem<sparse_bwd_dq_kernel<64>>(smem))) return e;
-    return launch_pdl(sparse_bwd_dq_kernel<64>, grid, BW_THREADS, smem, st, tq, tdo, tk, tv, p);
-  }
-  if ((e = allow_smem<sparse_bwd_dq_kernel<128>>(smem))) return e;
-  return launch_pdl(sparse_bwd_dq_kernel<128>, grid, BW_THREADS, smem, st, tq, tdo, tk, tv, p);
+  auto go = [&](auto kernel_tag, int ng) -> int {
+    constexpr auto kernel = decltype(kernel_tag)::kernel;
+    // four V slots lie over the Q / dO tiles, the rest of the V ring behind the K ring
+    const size_t smem = 1024 + 2 * nch * 128 * 128 +
+                        static_cast<size_t>(dq_kst(ng) + DQ_VST - 4) * nch * p.kvb * 128;
+    if (int r = allow_smem<kernel>(smem)) return r;
+    return launch_pdl(kernel, grid, bw_threads(ng), smem, st, tq, tdo, tk, tv, p);
+  };
+  if (kd == 64)
+    return one_group(static_cast<int64_t>(grid.x) * grid.y, static_cast<int>(std::min<int64_t>(static_cast<int64_t>(p.G) * p.W, p.Mkv / p.sub)))
+               ? go(Kernel<sparse_bwd_dq_kernel<64, 1>>{}, 1)
+               : go(Kernel<sparse_bwd_dq_kernel<64, 2>>{}, 2);
+  return go(Kernel<sparse_bwd_dq_kernel<128, 2>>{}, 2);
 }
 
 static int launch_dkv(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, bool pair,

@@ -237,3 +237,21 @@ def test_forward_ring(ftk, D, g):
                                            t["v"].float().numpy(), merged, H, g, kvb)
     np.testing.assert_allclose(lse.cpu().numpy(), want_lse, atol=2e-3, rtol=1e-2)
     assert (tolerance.rel_err(o.float().cpu().numpy(), want_o) <= 1).all()
+
+
+@pytest.mark.parametrize("g,kvb,W", [(64, 64, 9), (32, 64, 4), (64, 32, 20), (64, 16, 30)])
+def test_dq_of_two_ctas_per_sm(ftk, g, kvb, W):
+    """Head dim 64, 256 tiles of query rows: two dQ CTAs share an SM.  Two heads of one
+    batch entry alone fill no wave and take the SM each; both add up the tiles of a row
+    in the same order, so dQ is the same bit for bit."""
+    B, H, N, D = 2, 16, 1000, 64
+    t = cases.make_inputs(dict(B=B, N=N, H=H, D=D, dtype="bf16", seed=61, do_seed=62))
+    QM, M = -(-N // g), -(-N // kvb)
+    merged = _lists(np.random.default_rng(9), B * H, QM, M, W).reshape(B, H, QM, W)
+    pads = dict(q_padding=(0, QM * g - N), kv_padding=(0, M * kvb - N))
+    dq = _grads(ftk, t, merged, H, g, kvb, **pads)[2]
+    for b, h in ((0, 0), (1, 14)):
+        part = {k: v.view(B, N, H, D)[b:b + 1, :, h:h + 2].reshape(1, N, 2 * D).contiguous()
+                for k, v in t.items()}
+        alone = _grads(ftk, part, merged[b:b + 1, h:h + 2].copy(), 2, g, kvb, **pads)[2]
+        assert torch.equal(alone, dq.view(B, N, H, D)[b:b + 1, :, h:h + 2].reshape(1, N, 2 * D))
