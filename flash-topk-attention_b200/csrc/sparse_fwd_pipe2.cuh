@@ -17,10 +17,14 @@
 // have landed"; softmax warps of CTA 1 arrive on CTA 0's barriers through the
 // cluster shared-memory window.  No TMA load is multicast.
 //
+// The issuing warp of CTA 0 bounds the loop: K of tile i + 4 and V of tile i share a
+// stage, so that a round has three waits and two commits (a ring for either took five
+// and three: 1.94 ms against 1.84 at B = 4, N = 8192, H = 16, head dim 128; 1.86
+// against 1.80 at N = 15000 with 128-row blocks).
+//
 // Head dim 256: the 256-column O accumulator and the four S / P buffers fill
 // TMEM, so Q stays in shared memory (an M = 256 UMMA with both operands there
-// costs the same 43 cycles at N = 64) and the rings hold four K and four V half
-// tiles of 16 KB.  Per tile 16 x 43 + 4 x 128 = 1200 cycles for 256 query rows,
+// costs the same 43 cycles at N = 64) and the ring holds four stages of 32 KB.  Per tile 16 x 43 + 4 x 128 = 1200 cycles for 256 query rows,
 // where the one-CTA exact kernel (16 x 75 + 4 x 138 for 128 rows, one softmax
 // group, two stages) took 3700.
 #pragma once
@@ -29,12 +33,11 @@ namespace ftk {
 
 constexpr int FP2_THREADS = 576;   // TMA warp, UMMA warp, 4 softmax groups x 4 warps
 constexpr int FP2_GROUPS = 4;
-__host__ __device__ constexpr int fp2_kst(int d) { return d > 128 ? 4 : 6; }   // K half tiles
-__host__ __device__ constexpr int fp2_vst(int d) { return d > 128 ? 4 : 8; }   // V half tiles
+// Stages of the ring; a stage holds V of tile i and K of tile i + 4 (half of each).
+__host__ __device__ constexpr int fp2_stages(int d) { return d > 128 ? 4 : 8; }
 __host__ __device__ constexpr int fp2_tile(int d) { return d * 64; }           // bytes of either
 __host__ __device__ constexpr size_t fp2_smem(int d) {
-  return 1024 + static_cast<size_t>(d) * 256 +
-         static_cast<size_t>(fp2_kst(d) + fp2_vst(d)) * fp2_tile(d);
+  return 1024 + static_cast<size_t>(d) * 256 + static_cast<size_t>(fp2_stages(d)) * 2 * fp2_tile(d);
 }
 
 template <int D, int FMT, int SUB>
@@ -48,16 +51,15 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
   constexpr int KVB = 64;
   constexpr int TILE = fp2_tile(D);            // half a K tile (32 rows x D) or half a V tile
                                                // (64 rows x D / 2)
-  constexpr int FP2_KST = fp2_kst(D), FP2_VST = fp2_vst(D);
+  constexpr int ST = fp2_stages(D), STAGE = 2 * TILE;
   constexpr uint32_t COL_S = BIG ? 0 : 64, COL_O = BIG ? 256 : 320;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sQ = smem;
-  uint8_t* sK = smem + Q_BYTES;
-  uint8_t* sV = sK + FP2_KST * TILE;
+  uint8_t* sKV = smem + Q_BYTES;               // stage s: K half tile, then V half tile
   __shared__ UnionScratch un;
-  __shared__ __align__(8) uint64_t bars[4 + 3 * FP2_KST + 3 * FP2_VST + 2 * FP2_GROUPS];
+  __shared__ __align__(8) uint64_t bars[4 + 3 * ST + 2 * FP2_GROUPS];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
   __shared__ int s_ovf;
@@ -78,14 +80,10 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
   const uint32_t bar_qt = smem_u32(&bars[2]);    // CTA 0: Q of both CTAs copied into TMEM
                                                  // (BIG: CTA 1's Q has landed)
   const uint32_t bar_pro = smem_u32(&bars[3]);   // CTA 0: every softmax warp has its reference
-  auto bar_kfull = [&](int s) { return smem_u32(&bars[4 + s]); };
-  auto bar_kempty = [&](int s) { return smem_u32(&bars[4 + FP2_KST + s]); };
-  auto bar_peer_k = [&](int s) { return smem_u32(&bars[4 + 2 * FP2_KST + s]); };   // CTA 0 only
-  constexpr int BAR_V0 = 4 + 3 * FP2_KST;
-  auto bar_vfull = [&](int s) { return smem_u32(&bars[BAR_V0 + s]); };
-  auto bar_vempty = [&](int s) { return smem_u32(&bars[BAR_V0 + FP2_VST + s]); };
-  auto bar_peer_v = [&](int s) { return smem_u32(&bars[BAR_V0 + 2 * FP2_VST + s]); };   // CTA 0 only
-  constexpr int BAR_S0 = 4 + 3 * FP2_KST + 3 * FP2_VST;
+  auto bar_full = [&](int s) { return smem_u32(&bars[4 + s]); };
+  auto bar_empty = [&](int s) { return smem_u32(&bars[4 + ST + s]); };
+  auto bar_peer = [&](int s) { return smem_u32(&bars[4 + 2 * ST + s]); };   // CTA 0 only
+  constexpr int BAR_S0 = 4 + 3 * ST;
   auto bar_sfull = [&](int b) { return smem_u32(&bars[BAR_S0 + b]); };
   auto bar_pfull = [&](int b) { return smem_u32(&bars[BAR_S0 + FP2_GROUPS + b]); };
 
@@ -96,15 +94,10 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
     mbar_init(bar_final, 1);
     mbar_init(bar_qt, BIG ? 1 : 8);        // the 4 copying warps of each CTA
     mbar_init(bar_pro, 8 * FP2_GROUPS);     // the 16 softmax warps of each CTA
-    for (int s = 0; s < FP2_KST; s++) {
-      mbar_init(bar_kfull(s), 1);
-      mbar_init(bar_kempty(s), 1);
-      mbar_init(bar_peer_k(s), 1);
-    }
-    for (int s = 0; s < FP2_VST; s++) {
-      mbar_init(bar_vfull(s), 1);
-      mbar_init(bar_vempty(s), 1);
-      mbar_init(bar_peer_v(s), 1);
+    for (int s = 0; s < ST; s++) {
+      mbar_init(bar_full(s), 1);
+      mbar_init(bar_empty(s), 1);
+      mbar_init(bar_peer(s), 1);
     }
     for (int b = 0; b < FP2_GROUPS; b++) {
       mbar_init(bar_sfull(b), 1);
@@ -143,85 +136,64 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
       mbar_expect_tx(bar_q, Q_BYTES);
       for (int c = 0; c < NCH; c++)
         tma_load_4d(smem_u32(sQ) + c * 128 * 128, &tm_q, bar_q, c * 64, h_idx, tile_row0, b_idx);
-      // K entry j: the prologue blocks first, then the union; V entry i: the
-      // union only.  Every wait depends on tiles loaded earlier only.
-      const int total = npro + n;
+      // Stage rr holds K of tile rr and V of tile rr - 4; the first four, which
+      // have no V, take the prologue's K tiles in its place.
+      const int lead = min(n, FP2_GROUPS);
       const int hk = h_idx / p.kv_hdiv;   // out of the loop: a division takes 150 cycles
       const int dcol = D / 2 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
-      // BIG: V follows two entries behind K, so that the wait for one of the four
-      // V slots (held until P V) does not keep back the K tiles, needed earlier
-      constexpr int LAG = BIG ? 2 : 0;
-      for (int j = 0; j < total + LAG; j++) {
-        if (j < total) {
-          const int sk = j % FP2_KST;
-          if (!mbar_wait(bar_kempty(sk), ((j / FP2_KST) & 1) ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
-          const int id = j < npro ? pro_block(j) : static_cast<int>(un.ids[j - npro]);
-          const int tok0 = id * KVB - p.kv_pad_head;
-          const uint32_t kb = smem_u32(sK) + sk * TILE;
-          mbar_expect_tx(bar_kfull(sk), TILE);
-          for (int c = 0; c < NCH; c++)
-            tma_load_4d(kb + c * 4096, &tm_k32, bar_kfull(sk), c * 64, hk,
-                        tok0 + rsub, b_idx);
-        }
-        const int i = j - npro - LAG;
-        if (i >= 0) {
-          const int sv = i % FP2_VST;
-          const int tok0 = static_cast<int>(un.ids[i]) * KVB - p.kv_pad_head;
-          if (!mbar_wait(bar_vempty(sv), ((i / FP2_VST) & 1) ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
-          mbar_expect_tx(bar_vfull(sv), TILE);
+      for (int rr = 0; rr < n + FP2_GROUPS; rr++) {
+        if (rr >= lead && rr < FP2_GROUPS) continue;
+        const int s = rr % ST;
+        if (!mbar_wait(bar_empty(s), ((rr / ST) & 1) ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
+        const bool has_k = rr < n, has_pro = rr < npro, has_v = rr >= FP2_GROUPS;
+        const uint32_t kb = smem_u32(sKV) + s * STAGE, vb = kb + TILE;
+        mbar_expect_tx(bar_full(s), (has_k && (has_pro || has_v)) ? STAGE : TILE);
+        if (has_v) {
+          const int tok0 = static_cast<int>(un.ids[rr - FP2_GROUPS]) * KVB - p.kv_pad_head;
 #pragma unroll
           for (int c = 0; c < NCH / 2; c++)
-            tma_load_4d(smem_u32(sV) + sv * TILE + c * 8192, &tm_v, bar_vfull(sv), dcol + c * 64,
-                        hk, tok0, b_idx);
+            tma_load_4d(vb + c * 8192, &tm_v, bar_full(s), dcol + c * 64, hk, tok0, b_idx);
+        }
+        if (has_pro)
+          for (int c = 0; c < NCH; c++)
+            tma_load_4d(vb + c * 4096, &tm_k32, bar_full(s), c * 64, hk,
+                        pro_block(rr) * KVB - p.kv_pad_head + rsub, b_idx);
+        if (has_k) {
+          const int tok0 = static_cast<int>(un.ids[rr]) * KVB - p.kv_pad_head + rsub;
+          for (int c = 0; c < NCH; c++)
+            tma_load_4d(kb + c * 4096, &tm_k32, bar_full(s), c * 64, hk, tok0, b_idx);
         }
       }
     }
   } else if (warp == 1 && rank == 1) {
     // ----------------------- CTA 1: tell CTA 0 when my tiles have landed
-    const int total = npro + n;
     if (BIG && n > 0) {
       const bool landed = mbar_wait(bar_q, 0, w, FTK_DEV_TIMEOUT_MMA);
       __syncwarp();
       if (landed && lane == 0) mbar_arrive_cta(bar_qt, 0);
     }
-    constexpr int LAG = BIG ? 2 : 0;   // in the order in which the tiles were asked for
-    for (int j = 0; n > 0 && j < total + LAG; j++) {
-      if (j < total) {
-        const int sk = j % FP2_KST;
-        if (!mbar_wait(bar_kfull(sk), (j / FP2_KST) & 1, w, FTK_DEV_TIMEOUT_MMA)) break;
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cta(bar_peer_k(sk), 0);
-      }
-      const int i = j - npro - LAG;
-      if (i >= 0) {
-        const int sv = i % FP2_VST;
-        if (!mbar_wait(bar_vfull(sv), (i / FP2_VST) & 1, w, FTK_DEV_TIMEOUT_MMA)) break;
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cta(bar_peer_v(sv), 0);
-      }
+    for (int rr = 0; n > 0 && rr < n + FP2_GROUPS; rr++) {
+      if (rr >= n && rr < FP2_GROUPS) continue;
+      const int s = rr % ST;
+      if (!mbar_wait(bar_full(s), (rr / ST) & 1, w, FTK_DEV_TIMEOUT_MMA)) break;
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cta(bar_peer(s), 0);
     }
   } else if (warp == 1) {
     // ----------------------------- CTA 0: UMMA issuer for the CTA pair
     if (n > 0) {
       const uint32_t idesc_s = umma_idesc(256, KVB, FMT, 0, 0);
       const uint32_t idesc_pv = umma_idesc(256, D, FMT, 0, 1);
-      const uint64_t kdesc0 = smem_desc_sw128(smem_u32(sK), 16, 1024);
-      const uint64_t vdesc0 = smem_desc_sw128(smem_u32(sV), 8192, 1024);
+      const uint64_t kdesc0 = smem_desc_sw128(smem_u32(sKV), 16, 1024);
+      const uint64_t vdesc0 = smem_desc_sw128(smem_u32(sKV) + TILE, 8192, 1024);
       const uint64_t qdesc0 = smem_desc_sw128(smem_u32(sQ), 16, 1024);
       bool ok = mbar_wait(bar_qt, 0, w, FTK_DEV_TIMEOUT_MMA);
       if (BIG && ok) ok = mbar_wait(bar_q, 0, w, FTK_DEV_TIMEOUT_MMA);
       tc_fence_after();
-      auto wait_k = [&](int j) -> bool {
-        const int s = j % FP2_KST;
-        const uint32_t ph = (j / FP2_KST) & 1;
-        const uint32_t wb[2] = {bar_kfull(s), bar_peer_k(s)};
-        const uint32_t wp[2] = {ph, ph};
-        return mbar_wait_all<2>(wb, wp, w, FTK_DEV_TIMEOUT_MMA);
-      };
-      // S = Q K^T for K entry j into S buffer `buf`; Q read from TMEM (elected lane only)
-      auto mma_s = [&](int j, int buf) {
-        const int s = j % FP2_KST;
-        const uint64_t kdesc = desc_advance(kdesc0, s * TILE);
+      // S = Q K^T for the K tile at `off` into S buffer `buf`; Q read from TMEM
+      // (elected lane only)
+      auto mma_s = [&](int off, int buf) {
+        const uint64_t kdesc = desc_advance(kdesc0, off);
         const uint32_t d_tmem = tmem + COL_S + buf * 64;
 #pragma unroll
         for (int ks = 0; ks < D / 16; ks++) {
@@ -233,48 +205,53 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
             umma2_ts(d_tmem, tmem + ks * 8, b, idesc_s, ks > 0);
         }
         umma2_commit(bar_sfull(buf), 3);
-        umma2_commit(bar_kempty(s), 3);
       };
-      for (int e = 0; ok && e < npro; e++) ok = wait_k(e);
+      const int lead = min(n, FP2_GROUPS);
+      for (int t = 0; ok && t < lead; t++) {
+        const uint32_t wb[2] = {bar_full(t), bar_peer(t)};
+        const uint32_t wp[2] = {0, 0};
+        ok = mbar_wait_all<2>(wb, wp, w, FTK_DEV_TIMEOUT_MMA);
+      }
       tc_fence_after();
       if (ok && elect_one())
-        for (int e = 0; e < npro; e++) mma_s(e, e);
+        for (int e = 0; e < npro; e++) mma_s(e * STAGE + TILE, e);
       __syncwarp();
       if (ok) ok = mbar_wait(bar_pro, 0, w, FTK_DEV_TIMEOUT_MMA);
-      for (int i = 0; ok && i < FP2_GROUPS && i < n; i++) ok = wait_k(npro + i);
       tc_fence_after();
       if (ok && elect_one())
-        for (int i = 0; i < FP2_GROUPS && i < n; i++) mma_s(npro + i, i);
+        for (int t = 0; t < lead; t++) {
+          mma_s(t * STAGE, t);
+          umma2_commit(bar_empty(t), 3);
+        }
       __syncwarp();
       // per round every barrier is waited for first (together), then P V of
       // tile i and S of tile i + 4 go out as one batch
-      for (int i = 0; ok && i < n; i++) {
-        const int j = npro + i;
-        const int s = i % FP2_VST, sb = i & (FP2_GROUPS - 1);
-        const bool more = i + FP2_GROUPS < n;
-        const int j4 = j + FP2_GROUPS;
-        const uint32_t pf = bar_pfull(sb), pfp = (i / FP2_GROUPS) & 1;
-        const uint32_t vph = (i / FP2_VST) & 1, kph = (j4 / FP2_KST) & 1;
-        const uint32_t wb[5] = {bar_vfull(s), bar_peer_v(s), pf,
-                                more ? bar_kfull(j4 % FP2_KST) : pf,
-                                more ? bar_peer_k(j4 % FP2_KST) : pf};
-        const uint32_t wp[5] = {vph, vph, pfp, more ? kph : pfp, more ? kph : pfp};
-        if (!mbar_wait_all<5>(wb, wp, w, FTK_DEV_TIMEOUT_MMA)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint64_t vdesc = desc_advance(vdesc0, s * TILE);
-        if (elect_one()) {
+      for (int q = 0; ok && q * FP2_GROUPS < n; q++) {
+        const int s0 = ((q + 1) * FP2_GROUPS) % ST;
+        const uint32_t full_ph = ((q + 1) * FP2_GROUPS / ST) & 1, p_ph = q & 1;
 #pragma unroll
-          for (int ks = 0; ks < KVB / 16; ks++)
-            umma2_ts(tmem + COL_O, tmem + COL_S + sb * 64 + ks * 8,
-                     desc_advance(vdesc, ks * 2048), idesc_pv, (i > 0) || (ks > 0));
-          umma2_commit(bar_vempty(s), 3);
-          // S(i+4) lands on the columns PV(i) reads P from; UMMAs run in issue order
-          if (more) mma_s(j4, sb);
+        for (int u = 0; u < FP2_GROUPS; u++) {
+          const int i = q * FP2_GROUPS + u, s = s0 + u;
+          if (i >= n) break;
+          const uint32_t wb[3] = {bar_full(s), bar_peer(s), bar_pfull(u)};
+          const uint32_t wp[3] = {full_ph, full_ph, p_ph};
+          if (!mbar_wait_all<3>(wb, wp, w, FTK_DEV_TIMEOUT_MMA)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          if (elect_one()) {
+            const uint64_t vdesc = desc_advance(vdesc0, s * STAGE);
+#pragma unroll
+            for (int ks = 0; ks < KVB / 16; ks++)
+              umma2_ts(tmem + COL_O, tmem + COL_S + u * 64 + ks * 8,
+                       desc_advance(vdesc, ks * 2048), idesc_pv, (i > 0) || (ks > 0));
+            // S(i+4) lands on the columns PV(i) reads P from; UMMAs run in issue order
+            if (i + FP2_GROUPS < n) mma_s(s * STAGE, u);
+            umma2_commit(bar_empty(s), 3);
+          }
+          __syncwarp();
         }
-        __syncwarp();
       }
       if (elect_one()) umma2_commit(bar_final, 3);
       __syncwarp();
