@@ -246,14 +246,13 @@ int ftk_attn_bwd_dkv(const ftk_attn* a, const void* dout, int64_t sdo_b, int64_t
  * kernel, launched behind it, recomputes the tiles whose scores left the safe
  * exponent range (none on ordinary inputs).  Without a workspace only the
  * exact kernel runs.  Setting the environment variable FTK_FWD_PIPE=0 does the
- * same.  At head dim 128 the pipelined kernel runs on pairs of SMs (clusters of
- * two CTAs, tcgen05 cta_group::2); FTK_FWD_2CTA=0 selects the one-CTA form.
- * Head dim 256 (D is 64, 128 or 256) runs the exact kernel with one shared
- * output accumulator (dK / dV: one launch for dV, one for dK);
- * ftk_sparse_bwd_dq and ftk_sparse_bwd_dkv then take kv
- * blocks (dq) and q blocks (dkv) of at most 32 rows and return
- * FTK_ERR_UNSUPPORTED otherwise: the host layer restates longer blocks over
- * 32-row halves first. */
+ * same.  At head dim 256, and at head dim 128 with lists that can cover a good
+ * part of the blocks (2 W >= M), the pipelined kernel runs on pairs of SMs
+ * (clusters of two CTAs, tcgen05 cta_group::2); FTK_FWD_2CTA=0 selects the
+ * one-CTA form at head dim 128.  D is 64, 128 or 256.  At head dim 256 blocks of
+ * sizes other than 64 and 32 run the exact kernel, and ftk_sparse_bwd_dq and
+ * ftk_sparse_bwd_dkv take kv blocks (dq) and q blocks (dkv) of at most 32 rows
+ * (FTK_ERR_UNSUPPORTED otherwise). */
 size_t ftk_sparse_fwd_workspace(int64_t B, int64_t H, int QM, int q_block_size);
 int ftk_sparse_fwd(const void* q, const void* k, const void* v, int dtype, int64_t B, int64_t H, int64_t Hkv,
                    int64_t N, int64_t D, int64_t sq_b, int64_t sq_n, int64_t sq_h, int64_t sk_b,
@@ -267,9 +266,11 @@ int ftk_sparse_fwd(const void* q, const void* k, const void* v, int dtype, int64
  * sparse_attn_bwd_dq_launch (csrc/sparse_attn_bwd_dq.cpp:3-15,
  * csrc/sparse_attn_bwd_dq_kernel.cu:422): delta[bh][n] = sum_d o*do (fp32),
  * then dq for every q-block.  `delta` is an output the dK/dV call reuses. */
-/* Head dim 128 with 64-row q and kv blocks runs on pairs of SMs (clusters of two
- * CTAs, tcgen05 cta_group::2) in both backward calls; FTK_DQ_2CTA=0 and
- * FTK_DKV_2CTA=0 select the one-CTA kernels that serve every other shape. */
+/* Head dim 128 with 64-row blocks and wide lists (2 W >= M in dq, 4 W >= M in dkv)
+ * runs on pairs of SMs (clusters of two CTAs, tcgen05 cta_group::2) in both calls;
+ * ftk_attn_bwd_dq and ftk_attn_bwd_dkv run head dim 256 and 32-row blocks on pairs
+ * as well.  FTK_DQ_2CTA=0 and FTK_DKV_2CTA=0 select the one-CTA kernels at head dim
+ * 128. */
 int ftk_sparse_bwd_dq(const void* q, const void* k, const void* v, const void* o, const void* dout,
                       int dtype, int64_t B, int64_t H, int64_t Hkv, int64_t N, int64_t D, int64_t sq_b,
                       int64_t sq_n, int64_t sq_h, int64_t sk_b, int64_t sk_n, int64_t sk_h,
