@@ -52,14 +52,16 @@ inline EncodeTiledFn encode_tiled_fn() {
 inline int encode_tmap_bnhd(CUtensorMap* out, const void* base, int dtype, int64_t B, int64_t N,
                             int64_t H, int64_t D, int64_t sb, int64_t sn, int64_t sh, int box_d,
                             int box_rows) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn) return FTK_ERR_DRIVER;
   if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0) return FTK_ERR_BAD_ARG;
   if (((sb * 2) & 15) || ((sn * 2) & 15) || ((sh * 2) & 15)) return FTK_ERR_BAD_ARG;
   if (box_d * 2 > 128 || box_rows > 256 || box_rows < 1) return FTK_ERR_BAD_ARG;
+  // The stride of a dimension of one is never used for addressing but must be a legal
+  // value, and a tensor map cannot repeat a dimension: a stride of 0 (an expanded
+  // tensor) replaced by another would read rows that are not there.
+  if ((B > 1 && sb <= 0) || (N > 1 && sn <= 0) || (H > 1 && sh <= 0)) return FTK_ERR_BAD_ARG;
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return FTK_ERR_DRIVER;
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)N, (cuuint64_t)B};
-  // a stride of an extent-1 dimension is never used for addressing but must
-  // still be a legal value
   cuuint64_t strides[3] = {(cuuint64_t)(sh > 0 ? sh : D) * 2, (cuuint64_t)(sn > 0 ? sn : D) * 2,
                            (cuuint64_t)(sb > 0 ? sb : D) * 2};
   cuuint32_t box[4] = {(cuuint32_t)box_d, 1u, (cuuint32_t)box_rows, 1u};

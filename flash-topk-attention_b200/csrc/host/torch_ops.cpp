@@ -161,13 +161,17 @@ struct Scratch {
 
 // ------------------------------------------------------------------- layouts
 // A tensor addressed as [b][n][h][d]: d dense, 16-byte aligned base, strides
-// multiples of 8 elements.  Copies only what cannot be addressed in place.
+// multiples of 8 elements, no dimension repeated (an expanded tensor, such as the
+// gradient of a sum over tokens, has stride 0, which a tensor map cannot have).
+// Copies only what cannot be addressed in place.
 struct View {
   Tensor t;
   int64_t sb = 0, sn = 0, sh = 0;
 
   static bool strides(const Tensor& x, bool four_d, int64_t D, View* v) {
     if (x.stride(-1) != 1) return false;
+    for (int64_t i = 0; i + 1 < x.dim(); i++)
+      if (x.size(i) > 1 && x.stride(i) <= 0) return false;
     v->sb = x.stride(0);
     v->sn = four_d ? x.stride(2) : x.stride(1);
     v->sh = four_d ? x.stride(1) : D;
@@ -534,6 +538,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       PyErr_SetString(PyExc_NotImplementedError, e.what());
     }
   });
+  m.def("in_place", [](const Tensor& x, bool four_d, int64_t D) {
+    View v;
+    return View::strides(x, four_d, D, &v);
+  }, "whether the kernels can address a tensor as it is");
   m.def("score_topk", &score_topk, release());
   m.def("score_topk_workspace", &ftk_score_topk_workspace);
   m.def("qblock_merge", &qblock_merge, release());

@@ -154,8 +154,11 @@ def _kernel_head_dim(d: int) -> int:
 
 def _as_bnhd(x: torch.Tensor, input_4d: bool, H: int, D: int):
     """Return (tensor, sb, sn, sh) addressing x as [b][n][h][d] with d-stride 1,
-    16-byte aligned base and strides that are multiples of 8 elements.
-    Copies only when the layout cannot be addressed in place."""
+    16-byte aligned base, strides that are multiples of 8 elements and no
+    repeated (expanded) dimension.  Copies only when the layout cannot be
+    addressed in place."""
+    if any(n > 1 and s <= 0 for n, s in zip(x.shape[:-1], x.stride())):
+        x = x.contiguous()
     if input_4d:                       # [B, H, N, D]
         if x.stride(3) != 1:
             x = x.contiguous()

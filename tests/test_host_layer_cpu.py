@@ -1,0 +1,61 @@
+"""The host layer in front of the kernels, as far as it goes without a device."""
+
+import ctypes
+
+import pytest
+import torch
+
+
+@pytest.fixture(scope="module")
+def lib():
+    from flash_topk_attn_v2 import _lib
+    return _lib.lib
+
+
+def _score_code(lib, sb, sn, sh, B=2, H=2, N=128, D=64):
+    """Return code of ftk_block_score for tensors of these strides.  The pointers are host
+    memory that nothing reads: without a driver a call whose arguments are in order ends
+    at the encoding of its tensor maps (-5)."""
+    buf = ctypes.create_string_buffer(1 << 16)
+    p = (ctypes.addressof(buf) + 255) // 256 * 256
+    return lib.ftk_block_score(p, p, 1, B, H, N, D, sb, sn, sh, sb, sn, sh, 0, B * H, 64, 0, 0, 0.125,
+                               p, p, 1 << 40, None, None)
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="host pointers: only without a device")
+def test_tensor_maps_refuse_a_repeated_dimension(lib):
+    """Stride 0 along an extent above 1 (an expanded tensor) cannot be encoded; along an
+    extent of 1 the stride means nothing."""
+    ok, bad = -5, -1
+    assert _score_code(lib, 128 * 128, 128, 64) == ok
+    assert _score_code(lib, 0, 128, 64) == bad
+    assert _score_code(lib, 128 * 128, 0, 64) == bad
+    assert _score_code(lib, 128 * 128, 128, 0) == bad
+    assert _score_code(lib, 0, 128, 64, B=1) == ok
+    assert _score_code(lib, 128 * 64, 64, 0, H=1) == ok
+
+
+def test_expanded_tensors_are_copied():
+    """The gradient of a sum over tokens has strides (C, 0, 1); one key head shared by all
+    heads, or one batch entry by all, is an expanded tensor too."""
+    from flash_topk_attn_v2 import ops
+    from flash_topk_attn_v2._lib import native
+    o = torch.zeros(2, 64, 128, requires_grad=True)
+    seen = []
+    o.register_hook(seen.append)
+    (o.sum(dim=1) * torch.ones(2, 128)).sum().backward()
+    grad = seen[0]
+    assert grad.stride(1) == 0 and grad.stride(2) == 1
+    flat = torch.randn(1, 64, 128)
+    heads = torch.randn(2, 1, 64, 64)
+    for x, four_d, D in ((grad, False, 64), (flat.expand(2, 64, 128), False, 64),
+                         (heads.expand(2, 4, 64, 64), True, 64)):
+        H = x.shape[1] if four_d else x.shape[2] // D
+        assert not native.in_place(x, four_d, D)
+        y, sb, sn, sh = ops._as_bnhd(x, four_d, H, D)
+        assert y.data_ptr() != x.data_ptr() and torch.equal(y, x)
+        assert min(sb, sn, sh) > 0
+        assert native.in_place(y, four_d, D)
+    # a dimension of one may have any stride that is aligned
+    assert native.in_place(flat, False, 64)
+    assert native.in_place(torch.zeros(1, 64, 128).as_strided((1, 64, 128), (0, 128, 1)), False, 64)
