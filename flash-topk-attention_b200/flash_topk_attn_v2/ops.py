@@ -189,6 +189,12 @@ def _pad_head_dim(x: torch.Tensor, input_4d: bool, H: int, D: int, Dk: int) -> t
     return torch.nn.functional.pad(x.reshape(B, N, H, D), (0, Dk - D)).reshape(B, N, H * Dk)
 
 
+def _check_device(what: str, x: torch.Tensor, device: torch.device) -> None:
+    """Kernels take raw pointers: a tensor that lives elsewhere must not get that far."""
+    if x.device != device:
+        raise ValueError(f"{what} must be on {device}, got {x.device}")
+
+
 # --------------------------------------------------------------------------
 # scoring
 # --------------------------------------------------------------------------
@@ -235,6 +241,7 @@ def _parse_block_score_args(q, k, num_heads, score_block_size, padding):
         raise ValueError(f"q.dtype ({q.dtype}) != k.dtype ({k.dtype})")
     if q.dtype not in (torch.float16, torch.bfloat16, torch.float32):
         raise ValueError("q must be float16, bfloat16, or float32")
+    _check_device("k", k, q.device)
     return input_4d, B, H, N, D, n_padded // score_block_size, pad_head, pad_tail
 
 
@@ -397,6 +404,11 @@ def flash_qblock_merge(topk_indices, topk_scores, q_block_size, qblock_topk, num
             f"num_score_blocks={num_score_blocks} exceeds CUDA block sort limit 4096")
     if qblock_topk <= 0:
         raise ValueError("qblock_topk must be positive")
+    if topk_scores is not None:
+        if topk_scores.shape != topk_indices.shape:
+            raise ValueError(f"topk_scores {tuple(topk_scores.shape)} must have the shape of "
+                             f"topk_indices {tuple(topk_indices.shape)}")
+        _check_device("topk_scores", topk_scores, topk_indices.device)
     merged, mscores, counts = _call(
         "ftk_qblock_merge", native.qblock_merge, topk_indices, topk_scores, q_block_size, qh, qt,
         num_score_blocks, qblock_topk, want_scores)
@@ -453,6 +465,10 @@ def flash_build_reverse_indices_cuda(merged_indices, counts, num_kv_blocks):
     B, H, QM, W = merged_indices.shape
     M = num_kv_blocks
     dev = merged_indices.device
+    if counts is not None:
+        if counts.numel() != B * H * QM:
+            raise ValueError(f"counts must be [B, H, QM] = {(B, H, QM)}, got {tuple(counts.shape)}")
+        _check_device("counts", counts, dev)
     _before(dev)
     merged = merged_indices.contiguous()
     cnt = None if counts is None else counts.to(torch.int32).contiguous()
@@ -627,10 +643,17 @@ def flash_sparse_attn(q, k, v, merged_indices, num_heads, q_block_size, kv_block
         raise ValueError(
             f"merged_indices dim 2 ({merged_indices.shape[2]}) must match "
             f"QM = (q_pad_head + N + q_pad_tail) // q_block_size = {QM}")
+    if merged_indices.shape[:2] != (B, H):
+        raise ValueError(
+            f"merged_indices {tuple(merged_indices.shape)} must begin with [B, H] = {(B, H)}")
     if D <= 0 or D % 16 != 0:
         raise ValueError(f"D ({D}) must be a positive multiple of 16")
     if D > 256:
         raise ValueError(f"D ({D}) must be <= 256")
+    if not (k.dtype == v.dtype == q.dtype):
+        raise ValueError(f"k ({k.dtype}) and v ({v.dtype}) must have the type of q ({q.dtype})")
+    for name, x in (("k", k), ("v", v), ("merged_indices", merged_indices)):
+        _check_device(name, x, q.device)
     if scale is None:
         scale = 1.0 / math.sqrt(D)
     if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):

@@ -59,3 +59,50 @@ def test_expanded_tensors_are_copied():
     # a dimension of one may have any stride that is aligned
     assert native.in_place(flat, False, 64)
     assert native.in_place(torch.zeros(1, 64, 128).as_strided((1, 64, 128), (0, 128, 1)), False, 64)
+
+
+def _fake(shape, dtype=torch.float16, device="cuda:0"):
+    return torch.empty(shape, dtype=dtype, device=device)
+
+
+def test_mismatched_arguments_are_refused_on_the_host():
+    """Tensors on another device, of another type or of fewer heads than the kernels would
+    read, shown with tensors that have no memory: every call ends before a launch."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    import flash_topk_attn_v2 as ftk
+    with FakeTensorMode():
+        x, cpu, other = _fake((1, 128, 128)), _fake((1, 128, 128), device="cpu"), \
+            _fake((1, 128, 128), device="cuda:1")
+        bf, f32 = _fake((1, 128, 128), torch.bfloat16), _fake((1, 128, 128), torch.float32)
+        lists = _fake((1, 2, 2, 4), torch.int32)
+
+        def attn(q=x, k=x, v=x, m=lists):
+            return ftk.flash_topk_attn(q, k, v, m, None, 2, 64, 64)
+
+        for args in (dict(k=cpu), dict(v=other), dict(q=f32, k=f32, v=cpu.float()),
+                     dict(m=_fake((1, 2, 2, 4), torch.int32, "cpu")),
+                     dict(m=_fake((1, 2, 2, 4), torch.int32, "cuda:1"))):
+            with pytest.raises(ValueError, match="must be on cuda:0"):
+                attn(**args)
+        for args in (dict(k=bf), dict(v=bf), dict(k=f32, v=f32), dict(k=f32), dict(q=bf)):
+            with pytest.raises(ValueError, match="type of q"):
+                attn(**args)
+        for shape in ((1, 1, 2, 4), (2, 2, 2, 4)):
+            with pytest.raises(ValueError, match=r"\[B, H\]"):
+                attn(m=_fake(shape, torch.int32))
+
+        idx, scores = _fake((1, 2, 128, 4), torch.int32), _fake((1, 2, 128, 4), torch.float32)
+        with pytest.raises(ValueError, match="shape of"):
+            ftk.flash_qblock_merge(idx, _fake((1, 2, 128, 3), torch.float32), 64, 8, 8)
+        with pytest.raises(ValueError, match="must be on cuda:0"):
+            ftk.flash_qblock_merge(idx, scores.cpu(), 64, 8, 8)
+        with pytest.raises(ValueError, match="shape of"):
+            ftk.build_qblock_topk_indices(idx, 64, (0, 0), _fake((1, 1, 128, 4)), None, 8)
+        with pytest.raises(ValueError, match="must be on cuda:0"):
+            ftk.flash_topk_score(x, cpu, 2)
+        with pytest.raises(ValueError, match="must be on cuda:0"):
+            ftk.flash_block_score(x, other, 2, 64)
+        with pytest.raises(ValueError, match="counts must be"):
+            ftk.flash_build_reverse_indices_cuda(lists, _fake((1, 1, 2), torch.int32), 2)
+        with pytest.raises(ValueError, match="must be on cuda:0"):
+            ftk.flash_build_reverse_indices_cuda(lists, _fake((1, 2, 2), torch.int32, "cpu"), 2)
