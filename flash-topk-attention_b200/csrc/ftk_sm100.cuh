@@ -39,7 +39,10 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // drains.  Each kernel therefore waits before its first access to global
 // memory, in every thread block (a block that left without waiting would let
 // the kernel complete before its predecessor, and break the chain), and only
-// then allows its own successor to start.
+// then allows its own successor to start.  A kernel that allocates TMEM allows it
+// behind a barrier that follows the allocation: a CTA of the successor that took the
+// columns first would keep them until this grid is done, and tcgen05.alloc waits
+// without a limit.
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

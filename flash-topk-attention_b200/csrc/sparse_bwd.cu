@@ -305,7 +305,6 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   }
   clear_bitmaps(un);
   pdl_wait();
-  if (NG == 2) pdl_launch();
   if (tid == 0) {   // under the building of the union
     mbar_expect_tx(bar_q, 2 * ROW_TILE_BYTES);
     for (int c = 0; c < NCH; c++) {
@@ -317,7 +316,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   if (D <= 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);
   const int n = build_union<NG == 1 || D == 128>(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
                             p.W, nullptr, p.Mkv, p.sub, p.lm, p.status);
-  if (NG == 1) pdl_launch();   // behind tmem_alloc, see sparse_fwd_pipe_kernel
+  pdl_launch();
   if (D > 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);   // too many registers to hold across the union
   delta.finish(p, s_delta, bh, tile_row0, groups * p.g);
   if (p.masks)
@@ -616,15 +615,18 @@ __device__ __forceinline__ int dkv_union(UnionScratch& un, const BwdParams& p, i
                                          int groups) {
   clear_bitmaps(un);
   pdl_wait();
-  pdl_launch();
+  int n;
   if (p.masks) {
     const int64_t per_head = static_cast<int64_t>(p.mask_tiles) * p.mask_stride;
-    return build_union_masks(un, p.masks + bhq * per_head, p.mask_stride, p.mask_tiles, p.mask_g, j0,
-                             groups, p.heads, per_head, p.span, p.sub);
+    n = build_union_masks(un, p.masks + bhq * per_head, p.mask_stride, p.mask_tiles, p.mask_g, j0,
+                          groups, p.heads, per_head, p.span, p.sub);
+  } else {
+    const int64_t kv_row = static_cast<int64_t>(bhq) * p.Mkv + j0;
+    n = build_union(un, p.lists + kv_row * p.QM, 0, groups, p.QM, p.counts + kv_row, p.QM, p.sub,
+                    ListMap{0, 0, 0, 0}, p.status);
   }
-  const int64_t kv_row = static_cast<int64_t>(bhq) * p.Mkv + j0;
-  return build_union(un, p.lists + kv_row * p.QM, 0, groups, p.QM, p.counts + kv_row, p.QM,
-                     p.sub, ListMap{0, 0, 0, 0}, p.status);
+  pdl_launch();   // the unions hold the barrier that follows the caller's tmem_alloc
+  return n;
 }
 
 // Entry id of the union -> q tile, with the query head it belongs to (ids come

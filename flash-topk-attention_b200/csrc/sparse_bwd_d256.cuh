@@ -118,7 +118,6 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
   clear_bitmaps(un);
   cluster_arrive();
   pdl_wait();
-  pdl_launch();
   const int mine = min(per, groups - per * static_cast<int>(rank));   // q-blocks of my tile, if any
   if (tid == 0) {   // under the building of the union
     mbar_expect_tx(bar_q, 2 * B6_ROWS);
@@ -130,6 +129,7 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
   TileDelta<D> delta;
   const int n = build_union(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
                             p.W, nullptr, p.Mkv, SUB, p.lm, p.status);
+  pdl_launch();
   delta.load(p, b_idx, h_idx, tile_row0, mine * p.g);   // 256 columns: too many registers to hold across the union
   delta.finish(p, s_delta, bh, tile_row0, mine * p.g);
   if (p.masks && mine > 0)
@@ -453,7 +453,6 @@ sparse_bwd_dkv256_kernel(const __grid_constant__ CUtensorMap tm_q,
   }
   cluster_arrive();
   pdl_wait();
-  pdl_launch();
   if (tid == 0) {   // under the building of the union
     mbar_expect_tx(bar_kv, FIRST * B6_ROWS);
     for (int c = 0; c < NCH; c++) {

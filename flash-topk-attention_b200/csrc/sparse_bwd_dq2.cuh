@@ -98,7 +98,6 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
   clear_bitmaps(un);
   cluster_arrive();
   pdl_wait();
-  pdl_launch();
   const int mine = min(per, groups - per * static_cast<int>(rank));   // q-blocks of my tile, if any
   if (tid == 0) {   // under the building of the union
     mbar_expect_tx(bar_q, 2 * ROW_TILE_BYTES);
@@ -111,6 +110,7 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
   delta.load(p, b_idx, h_idx, tile_row0, mine * p.g);
   const int n = build_union(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
                             p.W, nullptr, p.Mkv, SUB, p.lm, p.status);
+  pdl_launch();
   delta.finish(p, s_delta, bh, tile_row0, mine * p.g);
   if (p.masks && mine > 0)
     write_tile_masks(un,

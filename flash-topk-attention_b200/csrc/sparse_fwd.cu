@@ -97,7 +97,6 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   pdl_wait();
-  pdl_launch();
   bool first_tile = true;
   uint32_t tmem = 0;
   // REDO: FW_THREADS redo words are looked at together, tiles blockIdx.x,
@@ -177,6 +176,7 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (first_tile) pdl_launch();   // a REDO CTA without a tile by leaving
   first_tile = false;
   tmem = tmem_base_s;
   WaitCtx w{&abort_flag, p.status};

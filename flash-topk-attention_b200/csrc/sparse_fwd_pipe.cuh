@@ -128,8 +128,6 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
   pdl_wait();
   const int n = build_union<NG == 2 || D == 128>(un, p.merged + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
                             p.W, nullptr, p.Mkv, SUB, p.lm, p.status);
-  // behind a barrier that follows tmem_alloc: a CTA of the next kernel that took the
-  // columns first would keep them until this grid is done
   pdl_launch();
   // tiles whose scores give the rows their reference exponents
   if (warp == 2) cover_tiles(un, n, groups, SUB, s_pro);

@@ -114,9 +114,9 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
   }
   clear_bitmaps(un);
   pdl_wait();
-  pdl_launch();
   const int n = build_union(un, p.merged + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
                             p.W, nullptr, p.Mkv, SUB, p.lm, p.status);
+  pdl_launch();
   // tiles whose scores give the rows their reference exponents
   if (warp == 2) cover_tiles(un, n, groups, SUB, s_pro);
   tc_fence_before();

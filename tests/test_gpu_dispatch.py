@@ -255,3 +255,20 @@ def test_dq_of_two_ctas_per_sm(ftk, g, kvb, W):
                 for k, v in t.items()}
         alone = _grads(ftk, part, merged[b:b + 1, h:h + 2].copy(), 2, g, kvb, **pads)[2]
         assert torch.equal(alone, dq.view(B, N, H, D)[b:b + 1, :, h:h + 2].reshape(1, N, 2 * D))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_redo_kernel_directly_before_the_backward(ftk, monkeypatch, D):
+    """Every tile is flagged, and the gradient kernel follows the redo kernel with nothing
+    in between: both allocate TMEM, and the results are those of the exact kernel alone."""
+    B, H, N, g, kvb = 2, 16, 1024, 64, 64
+    t = cases.make_inputs(dict(B=B, N=N, H=H, D=D, dtype="fp16", seed=23, do_seed=24))
+    t["k"][:, 512:] *= 4.0
+    t["q"] *= 2.0
+    merged = np.tile(np.arange(N // kvb, dtype=np.int32), (B, H, N // g, 1))
+    got = [_grads(ftk, t, merged, H, g, kvb) for _ in range(3)]
+    monkeypatch.setenv("FTK_FWD_PIPE", "0")
+    want = _grads(ftk, t, merged, H, g, kvb)
+    for run in got:
+        for a, b in zip(run, want):
+            assert torch.equal(a, b)

@@ -1,0 +1,63 @@
+"""Rules of the overlapped launches that a run cannot show, read off the sources."""
+
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                    "flash-topk-attention_b200", "csrc")
+
+
+def _functions():
+    """name -> (source of the declaration and body, is it a kernel), comments taken out."""
+    out = {}
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        text = re.sub(r"//[^\n]*|/\*.*?\*/", "", open(path).read(), flags=re.S)
+        for m in re.finditer(r"^(?:template <[^;{}]*>\s)?[^\n;{}#]*\b(__global__|__device__)\b[^;{}]*\{",
+                             text, re.M):
+            depth, end = 1, m.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[end], 0)
+                end += 1
+            head = re.sub(r"__launch_bounds__\((?:[^()]|\([^()]*\))*\)|__cluster_dims__\([^()]*\)", "",
+                          m.group(0))
+            name = re.search(r"(\w+)\s*\(", head)
+            if name:
+                out.setdefault(name.group(1), (text[m.start():end], m.group(1) == "__global__"))
+    return out
+
+
+FUNCTIONS = _functions()
+KERNELS = {n: s for n, (s, kernel) in FUNCTIONS.items() if kernel}
+OVERLAPPED = sorted(n for n, s in KERNELS.items() if "pdl_wait()" in s or "dkv_union(" in s)
+
+
+def test_the_sources_are_understood():
+    assert {"score_kernel", "sparse_fwd_kernel", "sparse_fwd_pipe_kernel", "sparse_fwd_pipe2_kernel",
+            "sparse_bwd_dq_kernel", "sparse_bwd_dq2_kernel", "sparse_bwd_dq256_kernel",
+            "sparse_bwd_dkv_kernel", "sparse_bwd_dkv2_kernel", "sparse_bwd_dkv256_kernel",
+            "topk_select_reg_kernel", "qblock_merge_warp_kernel", "fan_in_kernel", "head_sum_kernel",
+            "cast_bf16_kernel"} <= set(OVERLAPPED)
+
+
+@pytest.mark.parametrize("name", [n for n in OVERLAPPED if "tmem_alloc" in KERNELS[n]])
+def test_tmem_is_allocated_before_the_next_kernel_may_start(name):
+    """tcgen05.alloc waits without a limit: between it and the trigger of the successor,
+    whose blocks may take the columns and keep them until this grid is done, there is a
+    barrier of the block."""
+    barrier = r"__syncthreads\(\)|build_union(?:_masks)?\b[^;]*;"
+    for helper in ("build_union", "build_union_masks"):
+        assert "__syncthreads()" in FUNCTIONS[helper][0]
+    body = KERNELS[name]
+    assert "pdl_launch()" in body or "dkv_union(" in body
+    if "dkv_union(" in body:
+        union = FUNCTIONS["dkv_union"][0]
+        assert re.search(barrier, union[:union.index("pdl_launch()")])
+        assert "tmem_alloc" in body[:body.index("dkv_union(")]
+    if "pdl_launch()" in body:
+        first = body.index("pdl_launch()")
+        alloc = body.index("tmem_alloc")
+        assert alloc < first, "the successor may start before the columns are taken"
+        assert re.search(barrier, body[alloc:first]), "no barrier between allocation and trigger"
