@@ -164,7 +164,7 @@ __device__ __forceinline__ int build_union(UnionScratch& u, const int32_t* lists
         int4 t[4];
 #pragma unroll
         for (int x = 0; x < 4; x++)
-          t[x] = g0 + x < groups ? __ldg(reinterpret_cast<const int4*>(row(g0 + x)) + e)
+          t[x] = g0 + x < groups ? reinterpret_cast<const int4*>(row(g0 + x))[e]
                                  : make_int4(-1, -1, -1, -1);
 #pragma unroll
         for (int x = 0; x < 4; x++) {

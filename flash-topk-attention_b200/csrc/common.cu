@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(256) cast_bf16_kernel(const CastArgs a) {
     return *reinterpret_cast<const uint32_t*>(&v);
   };
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += step) {
-    const float4 x = __ldg(src + 2 * i), y = __ldg(src + 2 * i + 1);
+    const float4 x = src[2 * i], y = src[2 * i + 1];
     dst[i] = make_uint4(pack(x.x, x.y), pack(x.z, x.w), pack(y.x, y.y), pack(y.z, y.w));
   }
 }

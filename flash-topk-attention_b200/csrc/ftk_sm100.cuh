@@ -42,7 +42,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // then allows its own successor to start.  A kernel that allocates TMEM allows it
 // behind a barrier that follows the allocation: a CTA of the successor that took the
 // columns first would keep them until this grid is done, and tcgen05.alloc waits
-// without a limit.
+// without a limit.  What the predecessor may have written is read with plain loads:
+// read-only ones (__ldg, const __restrict__ parameters) are defined only for memory
+// that nobody writes during the kernel's life, which begins before that wait.
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -24,10 +24,9 @@ namespace ftk {
 constexpr int SEL_WARPS = 8;
 
 __global__ void __launch_bounds__(SEL_WARPS * 32)
-topk_select_kernel(const float* __restrict__ scores, const float* __restrict__ row_scale,
-                   int64_t rows, int M, int M_out, int bsz, int pad_head, int pad_tail,
-                   float threshold, int32_t* __restrict__ out_idx, float* __restrict__ out_raw,
-                   float* __restrict__ out_avg) {
+topk_select_kernel(const float* scores, const float* row_scale, int64_t rows, int M, int M_out,
+                   int bsz, int pad_head, int pad_tail, float threshold, int32_t* out_idx,
+                   float* out_raw, float* out_avg) {
   extern __shared__ float sel_smem[];
   pdl_wait();
   pdl_launch();
@@ -116,10 +115,9 @@ __host__ __device__ constexpr int sel_ctas() { return IPT == 64 ? 2 : IPT <= 4 |
 
 template <int IPT>
 __global__ void __launch_bounds__(sel_wpc<IPT>() * 32, sel_ctas<IPT>())
-topk_select_reg_kernel(const float* __restrict__ scores, const float* __restrict__ row_scale,
-                       int64_t rows, int M, int M_out, int bsz, int pad_head, int pad_tail,
-                       float threshold, int32_t* __restrict__ out_idx,
-                       float* __restrict__ out_raw, float* __restrict__ out_avg) {
+topk_select_reg_kernel(const float* scores, const float* row_scale, int64_t rows, int M, int M_out,
+                       int bsz, int pad_head, int pad_tail, float threshold, int32_t* out_idx,
+                       float* out_raw, float* out_avg) {
   constexpr int WPC = sel_wpc<IPT>();
   __shared__ unsigned long long cand_all[WPC][SEL_CAND];
   pdl_wait();
@@ -134,7 +132,7 @@ topk_select_reg_kernel(const float* __restrict__ scores, const float* __restrict
 #pragma unroll
     for (int i = 0; i < IPT; i++) {
       const int j = i * 32 + lane;
-      v[i] = (r < rows && j < M) ? __ldg(in + j) : 0.f;
+      v[i] = (r < rows && j < M) ? in[j] : 0.f;
     }
   };
   float cur[IPT], nxt[IPT];
@@ -206,10 +204,9 @@ int select_launch(const float* block_scores, const float* row_scale, int64_t row
 constexpr int MG_THREADS = 128;
 
 __global__ void __launch_bounds__(MG_THREADS)
-qblock_merge_kernel(const int32_t* __restrict__ idx, const float* __restrict__ scr, int64_t N,
-                    int K, int g, int q_pad_head, int QM, int Mtot, int Mp, int W,
-                    int32_t* __restrict__ out_idx, float* __restrict__ out_scr,
-                    int32_t* __restrict__ counts, int* status) {
+qblock_merge_kernel(const int32_t* idx, const float* scr, int64_t N, int K, int g, int q_pad_head,
+                    int QM, int Mtot, int Mp, int W, int32_t* out_idx, float* out_scr,
+                    int32_t* counts, int* status) {
   extern __shared__ unsigned long long mg_keys[];
   pdl_wait();
   pdl_launch();
@@ -357,10 +354,9 @@ __host__ __device__ constexpr int mgw_steps() { return E <= 8 ? 8 : 4; }
 
 template <int E>
 __global__ void __launch_bounds__(MGW_WARPS * 32)
-qblock_merge_warp_kernel(const int32_t* __restrict__ idx, const float* __restrict__ scr, int64_t N,
-                         int K, int g, int q_pad_head, int QM, int64_t total_qb, int Mtot, int W,
-                         int32_t* __restrict__ out_idx, float* __restrict__ out_scr,
-                         int32_t* __restrict__ counts, int* status) {
+qblock_merge_warp_kernel(const int32_t* idx, const float* scr, int64_t N, int K, int g,
+                         int q_pad_head, int QM, int64_t total_qb, int Mtot, int W,
+                         int32_t* out_idx, float* out_scr, int32_t* counts, int* status) {
   constexpr int MP = 32 * E;
   constexpr int U = mgw_steps<E>();
   __shared__ float agg_all[MGW_WARPS][MP];
@@ -398,8 +394,8 @@ qblock_merge_warp_kernel(const int32_t* __restrict__ idx, const float* __restric
         jn[u] = -1;
         sn[u] = 0.f;
         if (lane < step && e < total) {
-          jn[u] = __ldg(idx + base + e);
-          sn[u] = scr ? __ldg(scr + base + e) : 1.f;
+          jn[u] = idx[base + e];
+          sn[u] = scr ? scr[base + e] : 1.f;
         }
       }
     };

@@ -139,7 +139,7 @@ __device__ __forceinline__ void emit_ranks(const unsigned long long (&k)[SLOTS],
   for (int q = 0; q < SLOTS; q++) {
     id[q] = static_cast<int>(0xffffffffu - static_cast<unsigned>(k[q]));
     raw[q] = 0.f;
-    if (q * 32 + lane < M_out) raw[q] = __ldg(in + id[q]) * inv_total;
+    if (q * 32 + lane < M_out) raw[q] = in[id[q]] * inv_total;
     bound += fabsf(raw[q]);
   }
 #pragma unroll
@@ -377,7 +377,7 @@ __device__ __forceinline__ void select_row_reg(const float (&rawv)[IPT], const f
           (b1 == mx) ? static_cast<unsigned>(i1 * 32 + lane) : 0xffffffffu;
       const unsigned win = redux_min_u32(mine);
       w_idx = static_cast<int>(win);
-      w_raw = __ldg(in + win) * inv_total;
+      w_raw = in[win] * inv_total;
       w_avg = __int_as_float(mx);
       cum += w_raw;
       if (cum >= threshold) cut = true;

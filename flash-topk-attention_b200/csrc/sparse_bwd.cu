@@ -95,15 +95,14 @@ struct TileDelta {
       const int r = row(i), n = tile_row0 + r;
       vd[i] = vo[i] = vo2[i] = make_uint4(0u, 0u, 0u, 0u);
       if (!inside(p, r, n, rows)) continue;
-      vd[i] = __ldg(reinterpret_cast<const uint4*>(
-                        p.dout + 2 * (db + static_cast<int64_t>(n) * p.sd_n)) + c);
+      vd[i] = reinterpret_cast<const uint4*>(p.dout + 2 * (db + static_cast<int64_t>(n) * p.sd_n))[c];
       const int64_t oe = ob + static_cast<int64_t>(n) * p.so_n;
       if (p.out_f32) {
         const uint4* src = reinterpret_cast<const uint4*>(p.o + 4 * oe) + 2 * c;
-        vo[i] = __ldg(src);
-        vo2[i] = __ldg(src + 1);
+        vo[i] = src[0];
+        vo2[i] = src[1];
       } else {
-        vo[i] = __ldg(reinterpret_cast<const uint4*>(p.o + 2 * oe) + c);
+        vo[i] = reinterpret_cast<const uint4*>(p.o + 2 * oe)[c];
       }
     }
   }
@@ -1085,9 +1084,8 @@ namespace ftk {
 constexpr int FAN_THREADS = 1024;
 
 __global__ void __launch_bounds__(FAN_THREADS)
-fan_in_kernel(const uint8_t* __restrict__ masks, int stride, int tiles, int64_t head_stride,
-              int heads, int slices_per_b, int H, int G, int cols, int colsp,
-              int32_t* __restrict__ order) {
+fan_in_kernel(const uint8_t* masks, int stride, int tiles, int64_t head_stride, int heads,
+              int slices_per_b, int H, int G, int cols, int colsp, int32_t* order) {
   extern __shared__ unsigned long long fan_keys[];
   unsigned* cnt = reinterpret_cast<unsigned*>(fan_keys + colsp);
   pdl_wait();
@@ -1161,9 +1159,9 @@ fan_in_kernel(const uint8_t* __restrict__ masks, int stride, int tiles, int64_t 
 // memory (2 * H * D * 2 B read per token, 16 bytes per thread and load); used
 // where the grid is too small for one CTA to walk all heads of a group.
 __global__ void __launch_bounds__(256)
-head_sum_kernel(const uint8_t* __restrict__ dk_part, const uint8_t* __restrict__ dv_part, int fmt,
-                int64_t N, int Hkv, int grp, int D, int64_t vecs, void* dk, int64_t k_b, int64_t k_n,
-                int64_t k_h, void* dv, int64_t v_b, int64_t v_n, int64_t v_h, int f32) {
+head_sum_kernel(const uint8_t* dk_part, const uint8_t* dv_part, int fmt, int64_t N, int Hkv,
+                int grp, int D, int64_t vecs, void* dk, int64_t k_b, int64_t k_n, int64_t k_h,
+                void* dv, int64_t v_b, int64_t v_n, int64_t v_h, int f32) {
   pdl_wait();
   pdl_launch();
   const int dvec = D >> 3;
@@ -1180,7 +1178,7 @@ head_sum_kernel(const uint8_t* __restrict__ dk_part, const uint8_t* __restrict__
   for (int x = 0; x < 8; x++) acc[x] = 0.f;
   const uint4* s = src + head * grp * dvec + c;
   for (int g = 0; g < grp; g++) {
-    const uint4 t = __ldg(s + static_cast<int64_t>(g) * dvec);
+    const uint4 t = s[static_cast<int64_t>(g) * dvec];
     const uint32_t w[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
     for (int x = 0; x < 4; x++) {

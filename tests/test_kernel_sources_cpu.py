@@ -61,3 +61,21 @@ def test_tmem_is_allocated_before_the_next_kernel_may_start(name):
         alloc = body.index("tmem_alloc")
         assert alloc < first, "the successor may start before the columns are taken"
         assert re.search(barrier, body[alloc:first]), "no barrier between allocation and trigger"
+
+
+def test_no_read_only_loads_in_overlapped_kernels():
+    """ld.global.nc (__ldg, const __restrict__ parameters) is defined only for memory that
+    does not change during the kernel's life; an overlapped kernel's inputs are written by
+    the kernel it overlaps.  Kernels that are launched behind the whole of their
+    predecessor may use them; whatever else is in the sources, helpers included, may not."""
+    text = ""
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        text += re.sub(r"//[^\n]*|/\*.*?\*/", "", open(path).read(), flags=re.S)
+    for n in KERNELS:
+        if n not in OVERLAPPED:
+            assert KERNELS[n] in text
+            text = text.replace(KERNELS[n], "")
+    for what in (r"__ldg\b", r"\b__restrict__\b", r"ld\.global\.nc"):
+        assert not re.search(what, text), what
+    launched = set(re.findall(r"(\w+)(?:<[^<>;]*>)?<<<", text))
+    assert not launched & set(OVERLAPPED), "an overlapped kernel must be launched as one"
