@@ -115,7 +115,7 @@ def build_wait_probe(force: bool = False) -> str:
     newest = max(os.path.getmtime(PROBE_SRC), _headers_mtime())
     if not force and os.path.exists(PROBE_LIB) and os.path.getmtime(PROBE_LIB) >= newest:
         return PROBE_LIB
-    cmd = [NVCC, *FLAGS, "-DFTK_WAIT_CYCLES=200000LL", "-I", CSRC, "-shared", "-cudart", "static",
+    cmd = [NVCC, *FLAGS, "-DFTK_WAIT_CYCLES=200000LL", "-ftz=true", "-I", CSRC, "-shared", "-cudart", "static",
            PROBE_SRC, "-o", PROBE_LIB]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:

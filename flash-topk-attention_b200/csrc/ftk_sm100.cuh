@@ -291,17 +291,20 @@ __device__ __forceinline__ uint32_t cluster_nctas() {
   return r;
 }
 // the value at this shared-memory location in CTA `rank` of a cluster of `n`
-__device__ __forceinline__ float ld_cta(const float* p, int rank, int n) {
-  if (n == 1) return *reinterpret_cast<const volatile float*>(p);
-  float v;
+__device__ __forceinline__ int ld_cta(const int* p, int rank, int n) {
+  if (n == 1) return *reinterpret_cast<const volatile int*>(p);
+  int v;
   asm volatile(
       "{\n\t.reg .b32 ra;\n\t"
       "mapa.shared::cluster.u32 ra, %1, %2;\n\t"
-      "ld.volatile.shared::cluster.f32 %0, [ra];\n\t}"
-      : "=f"(v)
+      "ld.volatile.shared::cluster.b32 %0, [ra];\n\t}"
+      : "=r"(v)
       : "r"(smem_u32(p)), "r"(rank)
       : "memory");
   return v;
+}
+__device__ __forceinline__ float ld_cta(const float* p, int rank, int n) {
+  return __int_as_float(ld_cta(reinterpret_cast<const int*>(p), rank, n));
 }
 __device__ __forceinline__ void cluster_arrive() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");

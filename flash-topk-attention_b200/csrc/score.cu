@@ -466,8 +466,7 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
       }
     }
   } else if (tid < SC_QROWS + split) {
-    if (ld_cta(reinterpret_cast<const float*>(&abort_flag), tid - SC_QROWS, split) != 0.f)
-      s_stop = 1;
+    if (ld_cta(&abort_flag, tid - SC_QROWS, split)) s_stop = 1;
   }
   __syncthreads();
   const bool again = s_redo && !s_stop;

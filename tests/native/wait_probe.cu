@@ -2,7 +2,10 @@
 // waits of csrc/ftk_sm100.cuh until they give up.  Built with a short
 // FTK_WAIT_CYCLES so a wait runs out after ~0.1 ms.  One CTA, no TMA and no
 // tcgen05 instruction in flight: a wait that runs out records its code, raises
-// the CTA's abort flag and returns, and the kernel ends normally.
+// the CTA's abort flag and returns, and the kernel ends normally.  The second
+// kernel reads flags across a cluster; the unit is built with denormals flushed to
+// zero, which must not touch them.
+#include "ftk_host.cuh"
 #include "ftk_sm100.cuh"
 
 using namespace ftk;
@@ -54,6 +57,26 @@ extern "C" int ftk_wait_probe(int32_t* status, int32_t* trace, void* stream) {
   if (!trace) return -1;
   wait_probe_kernel<<<1, 64, 0, static_cast<cudaStream_t>(stream)>>>(status, trace);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+// Each CTA of a cluster of `n` looks at the flags of all: out[rank * n + r] = flag of CTA r
+// as seen by CTA `rank`, 1 in CTA `set` and 0 elsewhere.
+__global__ void flag_probe_kernel(int set, int* out) {
+  __shared__ int flag;
+  const int rank = cluster_ctarank(), n = cluster_nctas();
+  pdl_wait();
+  pdl_launch();
+  if (threadIdx.x == 0) flag = rank == set ? 1 : 0;
+  __syncthreads();
+  cluster_sync_all();
+  if (threadIdx.x < n) out[rank * n + threadIdx.x] = ld_cta(&flag, threadIdx.x, n) ? 1 : 0;
+  cluster_sync_all();
+}
+
+extern "C" int ftk_flag_probe(int cluster, int set, int32_t* out, void* stream) {
+  if (!out || cluster < 1 || cluster > 8) return -1;
+  return launch_clusters(flag_probe_kernel, cluster, dim3(cluster), dim3(32), 0,
+                         static_cast<cudaStream_t>(stream), set, out) == FTK_OK ? 0 : -4;
 }
 
 extern "C" long long ftk_wait_probe_cycles(void) { return FTK_WAIT_CYCLES; }

@@ -45,6 +45,8 @@ def probe():
     lib.ftk_wait_probe.restype = ctypes.c_int
     lib.ftk_wait_probe.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
     lib.ftk_wait_probe_cycles.restype = ctypes.c_longlong
+    lib.ftk_flag_probe.restype = ctypes.c_int
+    lib.ftk_flag_probe.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
     return lib
 
 
@@ -84,6 +86,19 @@ def test_bounded_wait_runs_out_and_the_kernel_returns(ftk, probe, with_status):
         assert code == 0
     # the context is intact: a normal launch afterwards still passes parity
     _small_score_matches_oracle(ftk)
+
+
+@pytest.mark.parametrize("cluster,raised", [(1, 0), (2, 1), (4, 0), (8, 7), (8, -1)])
+def test_abort_flag_is_seen_by_the_whole_cluster(probe, cluster, raised):
+    """A CTA that gave up stops the others of its cluster: its flag, an int of value 1,
+    is an int to them too (as a float it is a denormal, which this build flushes)."""
+    out = torch.full((cluster, cluster), -7, dtype=torch.int32, device="cuda")
+    assert probe.ftk_flag_probe(cluster, raised, out.data_ptr(),
+                                torch.cuda.current_stream().cuda_stream) == 0
+    want = torch.zeros(cluster, cluster, dtype=torch.int32)
+    if raised >= 0:
+        want[:, raised] = 1
+    assert torch.equal(out.cpu(), want)
 
 
 def _lists_with_one_bad_id(H, QM, M, W, bad_at, bad_id):
