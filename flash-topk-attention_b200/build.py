@@ -73,15 +73,33 @@ def build(force: bool = False) -> str:
 
 HOST_SRC = os.path.join(CSRC, "host", "torch_ops.cpp")
 NATIVE = os.path.join(HERE, "flash_topk_attn_v2", "_native.so")
+NATIVE_STAMP = os.path.join(OBJ, "native.stamp")   # what NATIVE was built against
 CXX = os.environ.get("CXX", "g++")
+
+
+def built_for() -> str:
+    """The PyTorch and the interpreter that _native.so is tied to: it uses the C++
+    interfaces of both, which another version does not have to keep."""
+    import torch
+    return f"torch {torch.__version__}, {sys.implementation.cache_tag}"
+
+
+def native_is_current() -> bool:
+    """Whether NATIVE is there, newer than its sources and built for this PyTorch."""
+    include = os.path.join(os.path.dirname(HERE), "include")
+    newest = max(os.path.getmtime(p) for p in
+                 [HOST_SRC] + [os.path.join(include, f) for f in os.listdir(include)])
+    if not os.path.exists(NATIVE) or os.path.getmtime(NATIVE) < newest:
+        return False
+    if not os.path.exists(NATIVE_STAMP):
+        return False
+    with open(NATIVE_STAMP) as f:
+        return f.read() == built_for()
 
 
 def build_native(force: bool = False) -> str:
     """flash_topk_attn_v2/_native.so; links lib/libftk_sm100.so (built first)."""
-    include = os.path.join(os.path.dirname(HERE), "include")
-    newest = max(os.path.getmtime(p) for p in
-                 [HOST_SRC] + [os.path.join(include, f) for f in os.listdir(include)])
-    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= newest:
+    if not force and native_is_current():
         return NATIVE
     import sysconfig
 
@@ -93,6 +111,7 @@ def build_native(force: bool = False) -> str:
     torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     cmd = [CXX, "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           f'-DFTK_BUILT_FOR="{built_for()}"',
            *[x for d in dirs for x in ("-isystem", d)], HOST_SRC, "-o", NATIVE,
            "-L", LIBDIR, "-l:libftk_sm100.so", "-Wl,-rpath,$ORIGIN/../lib",
            "-L", torch_lib, "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
@@ -100,6 +119,9 @@ def build_native(force: bool = False) -> str:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"{CXX} failed for torch_ops.cpp:\n{r.stdout}\n{r.stderr}")
+    os.makedirs(OBJ, exist_ok=True)
+    with open(NATIVE_STAMP, "w") as f:
+        f.write(built_for())
     return NATIVE
 
 

@@ -538,6 +538,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       PyErr_SetString(PyExc_NotImplementedError, e.what());
     }
   });
+  m.attr("built_for") = FTK_BUILT_FOR;   // build.py
   m.def("in_place", [](const Tensor& x, bool four_d, int64_t D) {
     View v;
     return View::strides(x, four_d, D, &v);

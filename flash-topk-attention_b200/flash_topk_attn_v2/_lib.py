@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import sys
 
 import torch
 
@@ -85,6 +86,18 @@ except ImportError as e:
         f"the native host layer of this package is missing or does not load ({e}): build it with "
         "`python flash-topk-attention_b200/build.py`. This package has no fallback path."
     ) from e
+
+
+def check_native(module) -> None:
+    """The host layer uses PyTorch's C++ interfaces: refuse one that was built for another."""
+    here = f"torch {torch.__version__}, {sys.implementation.cache_tag}"
+    if module.built_for != here:
+        raise ImportError(
+            f"the native host layer of this package was built for {module.built_for}, this is "
+            f"{here}: build it again with `python flash-topk-attention_b200/build.py`.")
+
+
+check_native(native)
 
 
 def error_text(code: int) -> str:

@@ -106,3 +106,36 @@ def test_mismatched_arguments_are_refused_on_the_host():
             ftk.flash_build_reverse_indices_cuda(lists, _fake((1, 1, 2), torch.int32), 2)
         with pytest.raises(ValueError, match="must be on cuda:0"):
             ftk.flash_build_reverse_indices_cuda(lists, _fake((1, 2, 2), torch.int32, "cpu"), 2)
+
+
+def test_the_native_layer_belongs_to_one_pytorch(tmp_path, monkeypatch):
+    """Another PyTorch or interpreter makes the built object stale, and an object that was
+    built for another is refused at import."""
+    import importlib.util
+    import os
+    import types
+    from flash_topk_attn_v2 import _lib
+    path = os.path.join(os.path.dirname(os.path.dirname(_lib._HERE)), "flash-topk-attention_b200",
+                        "build.py")
+    spec = importlib.util.spec_from_file_location("ftk_build_under_test", path)
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    assert _lib.native.built_for == build.built_for()
+    _lib.check_native(_lib.native)
+    with pytest.raises(ImportError, match="build it again"):
+        _lib.check_native(types.SimpleNamespace(built_for="torch 1.0.0, cpython-38"))
+
+    for name in ("NATIVE", "NATIVE_STAMP"):
+        monkeypatch.setattr(build, name, str(tmp_path / name))
+    assert not build.native_is_current()               # no object
+    (tmp_path / "NATIVE").write_text("x")
+    assert not build.native_is_current()               # nobody knows what it was built for
+    (tmp_path / "NATIVE_STAMP").write_text(build.built_for())
+    assert build.native_is_current()
+    monkeypatch.setattr(torch, "__version__", "9.9.9")
+    assert not build.native_is_current()
+    monkeypatch.undo()
+    for name in ("NATIVE", "NATIVE_STAMP"):
+        monkeypatch.setattr(build, name, str(tmp_path / name))
+    os.utime(tmp_path / "NATIVE", (0, 0))              # older than its sources
+    assert not build.native_is_current()
