@@ -426,6 +426,10 @@ std::tuple<Tensor, Tensor> sparse_attn(const Tensor& q, const Tensor& k, const T
                                        int64_t q_block, int64_t kv_block, int64_t q_pad_head,
                                        int64_t kv_pad_head, double scale) {
   const AttnMeta m{H, Hkv, q_block, kv_block, q_pad_head, kv_pad_head, scale};
+  // the outputs would silently carry no tangent
+  for (const Tensor* t : {&q, &k, &v})
+    if (torch::autograd::isFwGradDefined(*t))
+      throw Unsupported("flash_sparse_attn has no forward-mode derivative");
   if (!at::GradMode::is_enabled() || !(q.requires_grad() || k.requires_grad() || v.requires_grad())) {
     const Forward f = attn_forward(q, k, v, merged, m);
     return {f.o, f.lse};

@@ -139,3 +139,18 @@ def test_the_native_layer_belongs_to_one_pytorch(tmp_path, monkeypatch):
         monkeypatch.setattr(build, name, str(tmp_path / name))
     os.utime(tmp_path / "NATIVE", (0, 0))              # older than its sources
     assert not build.native_is_current()
+
+
+@pytest.mark.parametrize("which", ["q", "k", "v"])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_forward_mode_is_refused(which, dtype):
+    """The attention has no forward-mode derivative: a tangent on an input raises, as a
+    custom function without one does, instead of being dropped."""
+    import torch.autograd.forward_ad as fw
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    import flash_topk_attn_v2 as ftk
+    with FakeTensorMode(), fw.dual_level():
+        x = {n: _fake((1, 128, 128), dtype) for n in "qkv"}
+        x[which] = fw.make_dual(x[which], _fake((1, 128, 128), dtype))
+        with pytest.raises(NotImplementedError, match="forward-mode"):
+            ftk.flash_topk_attn(*x.values(), _fake((1, 2, 2, 4), torch.int32), None, 2, 64, 64)
