@@ -66,3 +66,195 @@ def test_expanded_inputs(ftk):
                                         H, 64, 64)):
         assert torch.equal(a, b)
     ftk.check_errors()
+
+
+# ------------------------------------------------------------------ the autograd node
+def _problem(dtype="bf16", B=1, N=384, H=4, Hkv=2, D=64):
+    t = cases.make_inputs(dict(B=B, N=N, H=H, D=D, dtype="bf16" if dtype == "fp32" else dtype,
+                               seed=75, do_seed=76))
+    t["k"], t["v"] = (t[n][..., :Hkv * D].contiguous() for n in "kv")
+    if dtype == "fp32":
+        t = {n: x.float() for n, x in t.items()}
+    leaves = [t[n].cuda().requires_grad_(True) for n in "qkv"]
+    merged = _full_lists(B, H, N // 64, N // 64, seed=1)[..., :4].contiguous()
+    return leaves, merged, t["do"].cuda(), dict(H=H, Hkv=Hkv)
+
+
+def _attend(ftk, leaves, merged, c):
+    return ftk.flash_topk_attn(*leaves, merged, None, c["H"], 64, 64, num_kv_heads=c["Hkv"])[0]
+
+
+def _expected(ftk, leaves, merged, do, c):
+    return torch.autograd.grad(_attend(ftk, leaves, merged, c), leaves, do)
+
+
+def _same(a, b):
+    assert len(a) == len(b) and all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+def test_backward_twice_with_a_retained_graph(ftk):
+    leaves, merged, do, c = _problem()
+    want = _expected(ftk, leaves, merged, do, c)
+    o = _attend(ftk, leaves, merged, c)
+    _same(torch.autograd.grad(o, leaves, do, retain_graph=True), want)
+    _same(torch.autograd.grad(o, leaves, do), want)
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(o, leaves, do)
+
+
+def test_only_some_inputs_want_a_gradient(ftk):
+    leaves, merged, do, c = _problem()
+    want = _expected(ftk, leaves, merged, do, c)
+    for wanted in ((0,), (1,), (2,), (0, 2)):
+        part = [x.detach().requires_grad_(i in wanted) for i, x in enumerate(leaves)]
+        o, lse = ftk.flash_topk_attn(*part, merged, None, c["H"], 64, 64, num_kv_heads=c["Hkv"])
+        assert o.requires_grad and not lse.requires_grad
+        _same(torch.autograd.grad(o, [part[i] for i in wanted], do), [want[i] for i in wanted])
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp32"])
+def test_saved_tensor_hooks(ftk, dtype):
+    """What the node keeps goes through the hooks: offloaded to the host and back, with no
+    copy left on the device, the gradients are the same."""
+    leaves, merged, do, c = _problem(dtype)
+    want = _expected(ftk, leaves, merged, do, c)
+    kept = []
+
+    def pack(x):
+        kept.append((tuple(x.shape), x.dtype))
+        return x.cpu()
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda x: x.cuda()):
+        o = _attend(ftk, leaves, merged, c)
+    assert len(kept) == 6                      # q, k, v, O, lse, lists
+    _same(torch.autograd.grad(o, leaves, do), want)
+
+
+@pytest.mark.parametrize("reentrant", [False, True])
+def test_checkpointing(ftk, reentrant):
+    from torch.utils.checkpoint import checkpoint
+    leaves, merged, do, c = _problem()
+    want = _expected(ftk, leaves, merged, do, c)
+    o = checkpoint(lambda q, k, v: _attend(ftk, (q, k, v), merged, c), *leaves,
+                   use_reentrant=reentrant)
+    o.backward(do)
+    _same([x.grad for x in leaves], want)
+
+
+@pytest.mark.parametrize("which", ["q", "o", "lists"])
+def test_a_changed_saved_tensor_is_noticed(ftk, which):
+    leaves, merged, do, c = _problem()
+    o = _attend(ftk, leaves, merged, c)
+    with torch.no_grad():
+        {"q": leaves[0], "o": o, "lists": merged}[which].mul_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(o, leaves, do)
+
+
+def test_backward_from_another_thread_and_stream(ftk):
+    """The backward runs on the stream of its forward, whichever thread and stream asks."""
+    import threading
+    leaves, merged, do, c = _problem()
+    want = _expected(ftk, leaves, merged, do, c)
+    got, errors = [], []
+
+    def work():
+        try:
+            side = torch.cuda.Stream()
+            side.wait_stream(torch.cuda.default_stream())
+            with torch.cuda.stream(side):
+                o = _attend(ftk, leaves, merged, c)
+                o.record_stream(torch.cuda.default_stream())
+            torch.cuda.current_stream().wait_stream(side)
+            with torch.cuda.stream(torch.cuda.Stream()):
+                torch.cuda.current_stream().wait_stream(side)
+                torch.autograd.backward(o, do, inputs=own[len(got)])
+                torch.cuda.current_stream().synchronize()
+            got.append([x.grad for x in own[len(got)]])
+        except Exception as e:                 # noqa: BLE001  (shown below)
+            errors.append(e)
+
+    own = []
+    for _ in range(2):
+        leaves = [x.detach().clone().requires_grad_(True) for x in leaves]
+        own.append(leaves)
+        torch.cuda.synchronize()
+        t = threading.Thread(target=work)
+        t.start()
+        t.join(60)
+        assert not errors, errors
+    torch.cuda.synchronize()
+    for g in got:
+        _same(g, want)
+
+
+def test_gradients_carry_no_graph(ftk):
+    """There is no second derivative: create_graph gives gradients without one."""
+    leaves, merged, do, c = _problem()
+    want = _expected(ftk, leaves, merged, do, c)
+    got = torch.autograd.grad(_attend(ftk, leaves, merged, c), leaves, do, create_graph=True)
+    _same(got, want)
+    assert not any(g.requires_grad for g in got)
+
+
+# ------------------------------------------------------------ the two routes of a call
+def _forms(seed):
+    """Calls of random form, ordinary and odd ones."""
+    import random
+    rng = random.Random(seed)
+    pick = rng.choice
+    D, H = pick([16, 48, 64, 96, 128, 160]), pick([1, 2, 4])
+    g, block = pick([16, 32, 48, 64, 96, 128]), pick([16, 32, 48, 64, 96, 128])
+    N = rng.randrange(200, 600)
+    ph, kh = pick([0, rng.randrange(g)]), pick([0, rng.randrange(block)])
+    return dict(B=pick([1, 2]), N=N, H=H, Hkv=pick([H, 1]), D=D, g=g, block=block,
+                dtype=pick(["fp16", "bf16", "fp32"]), topk=pick([0, 1, 3, 8]),
+                threshold=pick([1.0, 0.7]), qpad=(ph, -(ph + N) % g), kpad=(kh, -(kh + N) % block),
+                width=pick([None, 1, 5]), four_d=pick([False, True]), scores=pick([True, False]),
+                scale=pick([None, 0.25]), grad=pick([True, False]), strided=pick([False, True]))
+
+
+@pytest.mark.parametrize("seed", range(40))
+def test_both_routes_of_a_call_agree(ftk, seed):
+    """Ordinary calls pass one check in the native layer; timed calls, and those that this
+    check does not take, go through the checks of the operators first.  Either way a call
+    gives the same bits, or the same exception."""
+    from flash_topk_attn_v2 import ops
+    f = _forms(seed)
+    B, N, H, Hkv, D = f["B"], f["N"], f["H"], f["Hkv"], f["D"]
+    dt = {"fp16": torch.float16, "bf16": torch.bfloat16, "fp32": torch.float32}[f["dtype"]]
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+
+    def rand(*shape):
+        wide = (*shape[:-1], shape[-1] + (8 if f["strided"] else 0))
+        return torch.randn(wide, generator=gen, device="cuda").to(dt)[..., :shape[-1]]
+
+    qk = [rand(B, H, N, D) for _ in range(2)] if f["four_d"] else [rand(B, N, H * D) for _ in range(2)]
+    q, k, v, do = rand(B, N, H * D), rand(B, N, Hkv * D), rand(B, N, Hkv * D), rand(B, N, H * D)
+
+    def chain():
+        out = list(ftk.flash_topk_score(*qk, None if f["four_d"] else H, f["block"], f["topk"],
+                                        f["kpad"], f["threshold"]))
+        merged, counts, width = ftk.build_qblock_topk_indices(
+            out[0], f["g"], f["qpad"], out[2] if f["scores"] else None, f["width"])
+        leaves = [x.detach().requires_grad_(f["grad"]) for x in (q, k, v)]
+        out += [merged, counts, torch.tensor(width)]
+        try:
+            out += ftk.flash_topk_attn(*leaves, merged, counts, H, f["g"], f["block"], f["scale"],
+                                       Hkv, f["kpad"], f["qpad"])
+            if f["grad"]:
+                out += torch.autograd.grad(out[-2], leaves, do)
+        except NotImplementedError as e:
+            out.append(str(e))
+        return out
+
+    direct = chain()
+    ops.enable_event_timing(True)
+    try:
+        checked = chain()
+    finally:
+        ops.enable_event_timing(False)
+    ftk.check_errors()
+    assert len(direct) == len(checked)
+    for a, b in zip(direct, checked):
+        assert a == b if isinstance(a, str) else torch.equal(a, b)
