@@ -7,6 +7,8 @@
 
 extern "C" int ftk_version(void) { return 100; }  // 0.1.0
 
+extern "C" int64_t ftk_launch_count(void) { return ftk::g_launches.load(); }
+
 extern "C" const char* ftk_error_string(int code) {
   switch (code) {
     case ftk::FTK_OK: return "ok";

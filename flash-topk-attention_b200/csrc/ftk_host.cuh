@@ -120,6 +120,16 @@ inline int choose(int value, F&& f) {
   return f(std::integral_constant<int, N - 1>{});
 }
 
+// Kernels that this library has enqueued (or captured), for ftk_launch_count.
+inline std::atomic<long long> g_launches{0};
+
+// Result of launching `kernels` kernels: FTK_OK, and they are counted, or FTK_ERR_CUDA.
+inline int launched(cudaError_t e, int kernels = 1) {
+  if (e != cudaSuccess) return FTK_ERR_CUDA;
+  g_launches.fetch_add(kernels, std::memory_order_relaxed);
+  return FTK_OK;
+}
+
 // Launch that may overlap the tail of the stream's previous kernel.  Only for
 // kernels that call pdl_wait() in every block before they touch global memory.
 template <typename... Params, typename... Args>
@@ -135,9 +145,7 @@ inline int launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t s
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) == cudaSuccess
-             ? FTK_OK
-             : FTK_ERR_CUDA;
+  return launched(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
 }
 
 // The same as clusters of `cluster` CTAs along x (1: no clusters).
@@ -157,9 +165,7 @@ inline int launch_clusters(void (*kernel)(Params...), int cluster, dim3 grid, di
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) == cudaSuccess
-             ? FTK_OK
-             : FTK_ERR_CUDA;
+  return launched(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
 }
 
 // Clusters of that size that can run at once, 0 if the device does not say.

@@ -95,8 +95,7 @@ void look(int dev) {
                              ftk_error_string(code) + " (status " + std::to_string(code) + ")");
 }
 
-// ------------------------------------------------- launch counts and timing
-std::atomic<long> g_launches{0};
+// ------------------------------------------------------------------- timing
 std::atomic<bool> g_timing{false};
 std::mutex g_timing_mutex;
 struct Timed {
@@ -212,7 +211,6 @@ void cast_bf16(Tensor (&x)[N], const c10::cuda::CUDAStream& st) {
   }
   check(ftk_cast_bf16(src[0], n[0], dst[0], src[1], n[1], dst[1], src[2], n[2], dst[2], st.stream()),
         "ftk_cast_bf16");
-  g_launches++;
 }
 
 // -------------------------------------------------------------- score + select
@@ -250,7 +248,6 @@ std::vector<Tensor> score_topk(Tensor q, Tensor k, bool four_d, int64_t H, int64
                        outs[1].data_ptr<float>() + first, outs[2].data_ptr<float>() + first,
                        ws.get(), ws.bytes, status_ptr(device.index()), st.stream()),
         "ftk_score_topk");
-  g_launches += 2;
   return outs;
 }
 
@@ -279,7 +276,6 @@ std::tuple<Tensor, std::optional<Tensor>, Tensor> qblock_merge(
                          merged.data_ptr<int>(), scores ? scores->data_ptr<float>() : nullptr,
                          counts.data_ptr<int>(), status_ptr(device.index()), st.stream()),
         "ftk_qblock_merge");
-  g_launches += 1;
   return {merged, scores, counts};
 }
 
@@ -349,7 +345,6 @@ Forward attn_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Te
                        st.stream()),
           "ftk_attn_fwd");
   }
-  g_launches += 2;
   return f;
 }
 
@@ -396,7 +391,6 @@ struct SparseAttnBackward : torch::autograd::Node {
                             dq.stride(0), dq.stride(1), D, status, st.stream()),
             "ftk_attn_bwd_dq");
     }
-    g_launches += 1;
     out[0] = dq;
     if (task_should_compute_output(1) || task_should_compute_output(2)) {
       Tensor dk = new_cuda({a.B, a.N, m.Hkv * D}, to.scalar_type(), device);
@@ -406,7 +400,6 @@ struct SparseAttnBackward : torch::autograd::Node {
                              ws.get(), ws.bytes, dk.data_ptr(), dk.stride(0), dk.stride(1), D,
                              dv.data_ptr(), dv.stride(0), dv.stride(1), D, status, st.stream()),
             "ftk_attn_bwd_dkv");
-      g_launches += 1;
       out[1] = dk;
       out[2] = dv;
     }
@@ -559,7 +552,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("look", &look);
   m.def("set_deferred", [](bool on) { g_deferred = on; });
   m.def("set_debug", [](bool on) { g_debug = on; });
-  m.def("launch_count", []() { return g_launches.load(); });
   m.def("set_timing", &set_timing);
   m.def("take_times", &take_times, release());
 }

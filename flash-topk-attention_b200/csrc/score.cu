@@ -655,7 +655,7 @@ extern "C" int ftk_block_score(const void* q, const void* k, int dtype, int64_t 
   const int64_t rows = bh_count * N;
   const int grid = static_cast<int>(std::min<int64_t>((rows * M + 255) / 256, 148 * 16));
   score_normalize_kernel<<<grid, 256, 0, st>>>(block_scores, ws.row_total, block_scores, rows, M);
-  return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
+  return launched(cudaGetLastError());
 }
 
 extern "C" size_t ftk_score_topk_workspace(int64_t bh_count, int64_t N, int64_t M) {

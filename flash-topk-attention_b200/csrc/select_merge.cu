@@ -893,7 +893,7 @@ extern "C" int ftk_qblock_union(const int32_t* topk_idx, int64_t BH, int64_t N, 
                         static_cast<cudaStream_t>(stream)>>>(
       topk_idx, N, K, q_block_size, q_pad_head, static_cast<int>(QM), num_score_blocks, width,
       merged_idx, counts, status);
-  return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
+  return launched(cudaGetLastError());
 }
 
 extern "C" int ftk_max_index_plus1(const int32_t* idx, int64_t count, int32_t* result,
@@ -905,7 +905,7 @@ extern "C" int ftk_max_index_plus1(const int32_t* idx, int64_t count, int32_t* r
     const int grid = static_cast<int>(std::min<int64_t>((count + 255) / 256, 148 * 8));
     max_index_kernel<<<grid, 256, 0, st>>>(idx, count, result);
   }
-  return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
+  return launched(cudaGetLastError(), count > 0 ? 2 : 1);
 }
 
 extern "C" size_t ftk_build_reverse_workspace(int64_t BH, int QM, int M) {
@@ -942,7 +942,7 @@ extern "C" int ftk_build_reverse(const int32_t* merged_idx, const int32_t* count
     reverse_sort_kernel<<<static_cast<unsigned>(BH), 256, smem, st>>>(reverse_counts, M, Mp,
                                                                      sorted_kv);
   }
-  return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
+  return launched(cudaGetLastError(), sorted_kv ? 3 : 2);
 }
 
 extern "C" size_t ftk_sort_by_count_workspace(int64_t total, int max_count) {
@@ -968,7 +968,7 @@ extern "C" int ftk_sort_by_count(const int32_t* counts, int64_t total, int max_c
   sbc_scan_kernel<<<1, SBC_SCAN_THREADS, 0, st>>>(table, range, nchunk);
   sbc_place_kernel<<<nchunk, 32, 0, st>>>(counts, total, range, nchunk, table, sorted_counts,
                                           sorted_ids);
-  return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
+  return launched(cudaGetLastError(), 3);
 }
 
 // ------------------------------------------------- reverse index, no allocation
@@ -1041,5 +1041,5 @@ extern "C" int ftk_build_reverse_noalloc(const int32_t* merged_idx, const int32_
     reverse_sort_kernel<<<static_cast<unsigned>(BH), 256, smem, st>>>(reverse_counts, M, Mp,
                                                                      sorted_kv);
   }
-  return cudaGetLastError() == cudaSuccess ? FTK_OK : FTK_ERR_CUDA;
+  return launched(cudaGetLastError(), sorted_kv ? 3 : 2);
 }

@@ -23,6 +23,7 @@ i64, i32, f32, vp, sz = C.c_int64, C.c_int, C.c_float, C.c_void_p, C.c_size_t
 _STRIDES3 = [i64, i64, i64]
 SIGNATURES = {
     "ftk_version": (i32, []),
+    "ftk_launch_count": (i64, []),
     "ftk_error_string": (C.c_char_p, [i32]),
     "ftk_block_score_workspace": (sz, [i64, i64]),
     "ftk_block_score": (i32, [vp, vp, i32, i64, i64, i64, i64, *_STRIDES3, *_STRIDES3, i64, i64,

@@ -22,17 +22,11 @@ from ._lib import check, lib, native, ptr, stream_ptr
 _SCORE_SCRATCH_BYTES = int(os.environ.get("FTK_SCORE_SCRATCH_BYTES", 4 << 30))
 _DEBUG = os.environ.get("FTK_DEBUG", "0") not in ("", "0")
 native.set_debug(_DEBUG)
-_launches = 0
 
 
 def launch_count() -> int:
     """Kernels of libftk_sm100.so enqueued by this process so far."""
-    return _launches + native.launch_count()
-
-
-def _count(n: int) -> None:
-    global _launches
-    _launches += n
+    return lib.ftk_launch_count()
 
 
 # Optional per-call CUDA-event timing (off by default; bench.py switches it on
@@ -276,7 +270,6 @@ def flash_block_score(q, k, num_heads, score_block_size, padding=(0, 0)):
             ptr(qq), ptr(kk), _lib.dtype_code(qq), B, H, N, Dk, *sq, *sk, b0, cnt,
             score_block_size, ph, pt, float(D) ** -0.5, ptr(flat[b0]), ptr(ws), ws.numel(),
             ptr(status), stream_ptr(q.device))
-        _count(2)
     _after(q.device)
     return out
 
@@ -323,7 +316,6 @@ def flash_topk_select(block_scores, threshold, max_topk, score_block_size, paddi
     _call("ftk_topk_select", lib.ftk_topk_select, 
         ptr(scores), 0, B * H * N, M, max_topk, score_block_size, pad_head, pad_tail,
         float(threshold), ptr(idx), ptr(raw), ptr(avg), ptr(status_word(dev)), stream_ptr(dev))
-    _count(1)
     _after(dev)
     return idx, raw, avg
 
@@ -375,7 +367,6 @@ def num_score_blocks_of(topk_indices) -> int:
     out = torch.empty(1, dtype=torch.int32, device=dev)
     _call("ftk_max_index_plus1", lib.ftk_max_index_plus1, ptr(idx), idx.numel(), ptr(out),
           stream_ptr(dev))
-    _count(2 if idx.numel() else 1)
     return int(out.item())
 
 
@@ -449,7 +440,6 @@ def flash_qblock_union(topk_indices, q_block_size, q_padding=(0, 0), num_score_b
     _call("ftk_qblock_union", lib.ftk_qblock_union,
           ptr(idx), B * H, N, K, q_block_size, qh, qt, num_score_blocks, width, ptr(merged),
           ptr(counts), ptr(status_word(dev)), stream_ptr(dev))
-    _count(1)
     _after(dev)
     return merged, counts
 
@@ -479,7 +469,6 @@ def flash_build_reverse_indices_cuda(merged_indices, counts, num_kv_blocks):
     _call("ftk_build_reverse", lib.ftk_build_reverse, 
         ptr(merged), ptr(cnt), B * H, QM, W, M, ptr(rev), ptr(rc), ptr(skv), ptr(ws), ws.numel(),
         ptr(status_word(dev)), stream_ptr(dev))
-    _count(3)
     _after(dev)
     return rev, rc, skv
 
@@ -498,7 +487,6 @@ def flash_sort_by_count_cuda(reverse_counts, num_heads, num_kv_blocks):
     ws = torch.empty(lib.ftk_sort_by_count_workspace(total, max_val), dtype=torch.uint8, device=dev)
     _call("ftk_sort_by_count", lib.ftk_sort_by_count, ptr(flat), total, max_val, ptr(sc), ptr(ids), ptr(ws), ws.numel(),
                                 stream_ptr(dev))
-    _count(3)
     return sc, ids
 
 

@@ -60,6 +60,8 @@ extern "C" {
 
 /* Library version (major*10000 + minor*100 + patch). */
 int ftk_version(void);
+/* Kernels that this library has enqueued, or captured, in this process so far. */
+int64_t ftk_launch_count(void);
 /* Static, human-readable text for a return code or a device status code. */
 const char* ftk_error_string(int code);
 

@@ -258,3 +258,47 @@ def test_both_routes_of_a_call_agree(ftk, seed):
     assert len(direct) == len(checked)
     for a, b in zip(direct, checked):
         assert a == b if isinstance(a, str) else torch.equal(a, b)
+
+
+@pytest.mark.parametrize("D,g,kvb,H,Hkv,N", [
+    (128, 64, 64, 2, 2, 512),        # pairs
+    (64, 48, 48, 2, 2, 480),         # exact forward alone
+    (64, 64, 64, 16, 16, 4736),      # dK/dV tiles sorted first
+    (128, 64, 64, 6, 2, 320),        # one result per query head, summed by a kernel of its own
+    (256, 64, 64, 2, 2, 512),        # dV and dK in two launches
+])
+def test_launch_count_is_what_a_capture_holds(ftk, D, g, kvb, H, Hkv, N):
+    """Kernel nodes of a captured pass against the library's own count."""
+    from cuda.bindings import runtime as rt
+    from flash_topk_attn_v2 import ops
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    q, do = (torch.randn(1, N, H * D, generator=gen, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(1, N, Hkv * D, generator=gen, device="cuda").bfloat16() for _ in range(2))
+    leaves = [x.requires_grad_(True) for x in (q, k, v)]
+    qh = q.detach()
+    pads = dict(kv_padding=(0, -N % kvb), q_padding=(0, -N % g))
+
+    def step():
+        idx, _, avg = ftk.flash_topk_score(qh, qh, H, kvb, 4, pads["kv_padding"], 0.9)
+        merged, counts, _ = ftk.build_qblock_topk_indices(idx, g, pads["q_padding"], avg)
+        o, _ = ftk.flash_topk_attn(*leaves, merged, counts, H, g, kvb, num_kv_heads=Hkv, **pads)
+        torch.autograd.grad(o, leaves, do)
+
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    before = ops.launch_count()
+    with torch.cuda.graph(graph, stream=stream):
+        step()
+    counted = ops.launch_count() - before
+    raw = rt.cudaGraph_t(graph.raw_cuda_graph())
+    err, _, n = rt.cudaGraphGetNodes(raw, 0)
+    err, nodes, _ = rt.cudaGraphGetNodes(raw, n)
+    assert err == rt.cudaError_t.cudaSuccess
+    kernel = rt.cudaGraphNodeType.cudaGraphNodeTypeKernel
+    kernels = sum(rt.cudaGraphNodeGetType(x)[1] == kernel for x in nodes[:n])
+    ftk.check_errors()
+    assert counted == kernels > 0
