@@ -688,6 +688,16 @@ static int attn_fwd(const ftk_attn& a, const AttnGrid& gr, void* o, int64_t so_b
 
 using namespace ftk;
 
+extern "C" int ftk_attn_parts(const ftk_attn* a, int limit, int32_t out[10]) {
+  if (!a || !out || limit < 16) return FTK_ERR_BAD_ARG;
+  AttnGrid gr;
+  if (int e = attn_grid(*a, limit, &gr)) return e;
+  const int32_t v[10] = {gr.g,          gr.kvb,       gr.q_pad_head, gr.kv_pad_head, gr.QM, gr.Mkv,
+                         gr.lm.q_shift, gr.lm.q_off, gr.lm.kv_shift, gr.lm.kv_off};
+  std::copy(v, v + 10, out);
+  return FTK_OK;
+}
+
 // One redo word per tile of the pipelined kernel.
 extern "C" size_t ftk_attn_fwd_workspace(const ftk_attn* a) {
   AttnGrid gr;

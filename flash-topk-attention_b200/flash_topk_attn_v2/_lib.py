@@ -43,6 +43,7 @@ SIGNATURES = {
     "ftk_sort_by_count_workspace": (sz, [i64, i32]),
     "ftk_sort_by_count": (i32, [vp, i64, i32, vp, vp, vp, sz, vp]),
     "ftk_cast_bf16": (i32, [vp, i64, vp, vp, i64, vp, vp, i64, vp, vp]),
+    "ftk_attn_parts": (i32, [vp, i32, vp]),
     "ftk_attn_fwd_workspace": (sz, [vp]),
     "ftk_attn_fwd": (i32, [vp, vp, *_STRIDES3, vp, vp, sz, vp, vp]),
     "ftk_attn_bwd_workspace": (sz, [vp]),

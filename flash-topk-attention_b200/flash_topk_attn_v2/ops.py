@@ -493,15 +493,6 @@ def flash_sort_by_count_cuda(reverse_counts, num_heads, num_kv_blocks):
 # --------------------------------------------------------------------------
 # sparse attention
 # --------------------------------------------------------------------------
-def preprocess_delta(o, do, num_heads):
-    """delta = rowsum(O * dO), [B, H, N] fp32 (sparse_attn_bwd.py:12-33).
-    Host-side convenience; the backward computes it inside the dQ kernel."""
-    B, N, C = o.shape
-    D = C // num_heads
-    return (o.float().view(B, N, num_heads, D) * do.float().view(B, N, num_heads, D)).sum(-1) \
-        .permute(0, 2, 1).contiguous()
-
-
 def _check_backward_blocks(D, g, kvb):
     """Block sizes the gradient kernels take (the reference's take any q block of
     1..64 rows and any kv block): multiples of 16 rows, and at head dims above 128
@@ -518,41 +509,6 @@ def _check_backward_blocks(D, g, kvb):
                 raise NotImplementedError(
                     f"backward at head dim > 128 needs a {name} that halves down to 16 or "
                     f"32 rows (16, 32, 64, 128), got {blk}")
-
-
-def _split_large_blocks(merged, N, g, kvb, q_pad_head, kv_pad_head, limit=64):
-    """Lists over blocks of more than `limit` rows (65..128 for the default),
-    restated over half-size blocks, repeatedly if need be.
-
-    The kernels work on q / kv blocks of at most 64 rows and read longer blocks'
-    lists in place by this rule (csrc/attn_host.cuh); this function writes the
-    restated lists out.  A block of `kvb` rows
-    that starts at token j*kvb - pad is exactly the two half blocks
-    2j - s, 2j - s + 1 of a grid with block kvb/2 and pad head pad - s*kvb/2,
-    where s = 1 when the pad head covers the first half block; each listed id
-    becomes those two ids (halves that lie before token 0 or at / after token N
-    are dropped).  q-blocks split the same way: both halves of a q-block take
-    its list.  Returns (merged', g', kvb', q_pad_head', kv_pad_head', M')."""
-    while kvb > limit:
-        half = kvb // 2
-        s = 1 if kv_pad_head >= half else 0
-        kv_pad_head -= s * half
-        sub0 = 2 * merged - s
-        sub = torch.stack([sub0, sub0 + 1], dim=-1)
-        start = sub.to(torch.int64) * half - kv_pad_head
-        keep = (merged >= 0).unsqueeze(-1) & (sub >= 0) & (start < N)
-        merged = torch.where(keep, sub, torch.full_like(sub, -1)).flatten(-2)
-        kvb = half
-    while g > limit:
-        half = g // 2
-        s = 1 if q_pad_head >= half else 0
-        q_pad_head -= s * half
-        qm2 = 2 * merged.shape[2] - s
-        parent = (torch.arange(qm2, device=merged.device) + s) // 2
-        merged = merged.index_select(2, parent)
-        g = half
-    m_kv = (kv_pad_head + N + kvb - 1) // kvb
-    return merged.contiguous(), g, kvb, q_pad_head, kv_pad_head, m_kv
 
 
 def flash_sparse_attn(q, k, v, merged_indices, num_heads, q_block_size, kv_block_size,

@@ -221,6 +221,14 @@ int ftk_cast_bf16(const float* a, int64_t na, void* to_a, const float* b, int64_
  *     order; dk and dv have Hkv heads (the heads of a group are summed here).
  * Outputs have strides (s*_b, s*_n, s*_h) in elements, multiples of 8; `o` of the
  * backward has the type that the forward wrote. */
+/* How blocks of more than `limit` rows are worked on: as parts of half the size,
+ * repeatedly if need be, over the lists as they are.  Host only.  out = rows per q
+ * part, rows per kv part, pad heads of the two grids of parts, number of q and kv
+ * parts, then q_shift, q_off, kv_shift, kv_off: part m of the q grid takes list row
+ * (m + q_off) >> q_shift, and a listed block j stands for the 2^kv_shift parts from
+ * (j << kv_shift) - kv_off on, as far as there are such parts. */
+int ftk_attn_parts(const ftk_attn* a, int limit, int32_t out[10]);
+
 size_t ftk_attn_fwd_workspace(const ftk_attn* a);
 int ftk_attn_fwd(const ftk_attn* a, void* o, int64_t so_b, int64_t so_n, int64_t so_h, float* lse,
                  void* workspace, size_t workspace_bytes, int32_t* status, void* stream);

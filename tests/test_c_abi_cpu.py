@@ -106,51 +106,65 @@ def test_no_fallback_when_library_missing(tmp_path, monkeypatch):
         _lib._load()
 
 
-def test_large_block_lists_split_into_half_blocks():
-    """q / kv blocks of 65..128 rows are restated over half-size blocks on the
-    host: every query row must keep exactly the same set of key tokens."""
-    import numpy as np
-    import torch
-    from flash_topk_attn_v2 import ops
+class _Attn(ctypes.Structure):
+    """struct ftk_attn of include/ftk_attn.h"""
+    _fields_ = ([(n, ctypes.c_void_p) for n in "qkv"] + [("dtype", ctypes.c_int), ("out_f32", ctypes.c_int)]
+                + [(n, ctypes.c_int64) for n in ("B", "H", "Hkv", "N", "D")]
+                + [(f"s{t}_{x}", ctypes.c_int64) for t in "qkv" for x in "bnh"]
+                + [("lists", ctypes.c_void_p)]
+                + [(n, ctypes.c_int) for n in ("list_rows", "W", "q_block", "kv_block", "q_pad_head",
+                                               "kv_pad_head")]
+                + [("scale", ctypes.c_float)])
 
-    def token_sets(merged, N, g, kvb, qph, kph):
-        qm = merged.shape[2]
-        out = []
-        for m in range(qm):
-            toks = set()
-            for j in merged[0, 0, m].tolist():
-                if j >= 0:
-                    toks.update(t for t in range(j * kvb - kph, (j + 1) * kvb - kph) if 0 <= t < N)
-            for r in range(m * g - qph, (m + 1) * g - qph):
-                if 0 <= r < N:
-                    out.append((r, frozenset(toks)))
-        return dict(out)
+
+def test_large_block_lists_split_into_half_blocks(ftk):
+    """q / kv blocks of 65..128 rows are worked on as half-size blocks, the lists read in
+    place: every query row must keep exactly the same set of key tokens, whatever the pad
+    heads cover, and with blocks halved once or twice."""
+    import numpy as np
+    from flash_topk_attn_v2 import _lib
+
+    def block_tokens(j, kvb, kph, N):
+        return range(max(j * kvb - kph, 0), min((j + 1) * kvb - kph, N))
 
     rng = np.random.default_rng(0)
-    for N, g, kvb, qpad, kpad in [(1000, 128, 128, (70, 82), (100, 52)),
-                                  (1000, 128, 64, (10, 14), (8, 16)),
-                                  (1000, 64, 128, (24, 0), (0, 24)),
-                                  (1000, 96, 96, (20, 36), (50, 6)),
-                                  (100, 128, 128, (14, 14), (27, 1))]:
+    for limit, N, g, kvb, qpad, kpad in [(64, 1000, 128, 128, (70, 82), (100, 52)),
+                                         (64, 1000, 128, 64, (10, 14), (8, 16)),
+                                         (64, 1000, 64, 128, (24, 0), (0, 24)),
+                                         (64, 1000, 96, 96, (20, 36), (50, 6)),
+                                         (64, 100, 128, 128, (14, 14), (27, 1)),
+                                         (64, 1000, 64, 32, (24, 0), (0, 24)),
+                                         (32, 1000, 128, 128, (70, 82), (100, 52)),
+                                         (32, 1000, 128, 64, (10, 14), (8, 16)),
+                                         (32, 1000, 128, 128, (127, 25), (33, 119)),
+                                         (32, 100, 64, 128, (28, 0), (27, 1))]:
         QM, M = (qpad[0] + N + qpad[1]) // g, (kpad[0] + N + kpad[1]) // kvb
-        merged = np.full((1, 1, QM, 4), -1, dtype=np.int32)
+        lists = [rng.permutation(M)[:int(rng.integers(0, 5))].tolist() for _ in range(QM)]
+        a = _Attn(q=64, k=64, v=64, dtype=1, B=1, H=1, Hkv=1, N=N, D=64, lists=64, list_rows=QM, W=4,
+                  q_block=g, kv_block=kvb, q_pad_head=qpad[0], kv_pad_head=kpad[0], scale=1.0)
+        out = (ctypes.c_int32 * 10)()
+        assert _lib.lib.ftk_attn_parts(ctypes.addressof(a), limit, ctypes.addressof(out)) == 0
+        pg, pkv, qph, kph, pqm, pm, q_shift, q_off, kv_shift, kv_off = out
+        assert pg <= limit and pkv <= limit and 0 <= qph < pg and 0 <= kph < pkv
+        assert pqm * pg >= qph + N and pm * pkv >= kph + N
+        got = {}
+        for m in range(pqm):
+            row = (m + q_off) >> q_shift
+            assert 0 <= row < QM
+            tokens = set()
+            for j in lists[row]:
+                for x in range((j << kv_shift) - kv_off, ((j + 1) << kv_shift) - kv_off):
+                    if 0 <= x < pm:
+                        tokens.update(block_tokens(x, pkv, kph, N))
+            for r in block_tokens(m, pg, qph, N):
+                got[r] = tokens
         for m in range(QM):
-            c = int(rng.integers(0, 5))
-            merged[0, 0, m, :c] = rng.permutation(M)[:c]
-        want = token_sets(merged, N, g, kvb, qpad[0], kpad[0])
-        m2, g2, kvb2, qph2, kph2, mkv2 = ops._split_large_blocks(
-            torch.from_numpy(merged), N, g, kvb, qpad[0], kpad[0])
-        assert g2 <= 64 and kvb2 <= 64 and 0 <= qph2 < g2 and 0 <= kph2 < kvb2
-        assert m2.shape[2] * g2 >= qph2 + N and int(m2.max()) < mkv2
-        got = token_sets(m2.numpy(), N, g2, kvb2, qph2, kph2)
-        assert got == want, (N, g, kvb)
-        # down to 32-row blocks (gradient kernels at head dim 256), where halving allows
-        if g % 64 == 0 and kvb % 64 == 0:
-            m3, g3, kvb3, qph3, kph3, mkv3 = ops._split_large_blocks(
-                torch.from_numpy(merged), N, g, kvb, qpad[0], kpad[0], limit=32)
-            assert g3 == 32 and kvb3 == 32 and 0 <= qph3 < 32 and 0 <= kph3 < 32
-            assert m3.shape[2] * g3 >= qph3 + N and int(m3.max()) < mkv3
-            assert token_sets(m3.numpy(), N, g3, kvb3, qph3, kph3) == want, (N, g, kvb)
+            tokens = set()
+            for j in lists[m]:
+                tokens.update(block_tokens(j, kvb, kpad[0], N))
+            for r in block_tokens(m, g, qpad[0], N):
+                assert got[r] == tokens, (limit, N, g, kvb, r)
+        assert len(got) == N
 
 
 def test_first_generation_api_names_and_signatures():
