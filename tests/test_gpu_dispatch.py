@@ -272,3 +272,51 @@ def test_redo_kernel_directly_before_the_backward(ftk, monkeypatch, D):
     for run in got:
         for a, b in zip(run, want):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("M", [20, 64, 200, 1000, 1100, 2048, 2100])
+def test_select_of_values_that_are_no_scores(ftk, M):
+    """Rows with NaN, infinities, negative values and zeros: an average that is not >= 0
+    counts as 0, the order is that of the averages with ties to the lower block, the cut is
+    where the running sum of the raw values first reaches the threshold (never, once it is
+    NaN)."""
+    rng = np.random.default_rng(M)
+    x = rng.random((24, M)).astype(np.float32)
+    x /= x.sum(-1, keepdims=True)
+    x[1, ::3] = np.nan
+    x[2, 1::5] = np.inf
+    x[3, ::2] *= -1
+    x[4] = 0
+    x[5] = np.nan
+    x[6, 3], x[6, 4] = np.nan, np.inf
+    x[7] = -1
+    x[8, :M // 2] = -np.inf
+    x[9] = np.float32(1e-45) * rng.integers(0, 3, M)
+    x[10] = 3.0e38
+    scores = torch.from_numpy(x).cuda().view(1, 1, 24, M)
+    for k, thr, b, pad in ((8, 0.5, 64, (0, 0)), (32, 1.5, 64, (10, 3)), (64, 0.1, 48, (0, 0)),
+                           (1, 0.0, 64, (0, 5)), (70, 0.9, 64, (0, 0))):
+        width = min(k, M)
+        count = np.full(M, b, np.float32)
+        count[0] -= pad[0]
+        count[-1] -= pad[1]
+        with np.errstate(all="ignore"):
+            avg = x / count
+            avg = np.where(avg >= 0, avg, np.float32(0))
+            order = np.argsort(-avg, axis=1, kind="stable")[:, :width]
+            raw = np.take_along_axis(x, order, 1)
+            cum = np.zeros(24, np.float32)
+            cut = np.zeros(24, bool)
+            want = np.full((24, width), -1, np.int32), np.zeros((24, width), np.float32), \
+                np.zeros((24, width), np.float32)
+            for r in range(width):
+                on = ~cut
+                want[0][on, r] = order[on, r]
+                want[1][on, r] = raw[on, r]
+                want[2][on, r] = np.take_along_axis(avg, order, 1)[on, r]
+                cum = np.where(on, cum + raw[:, r], cum)
+                cut |= cum >= np.float32(thr)
+        got = ftk.flash_topk_select(scores, thr, k, b, pad)
+        for g, w in zip(got, want):
+            np.testing.assert_array_equal(g[0, 0].cpu().numpy(), w, err_msg=f"{k} {thr} {b} {pad}")
+    ftk.check_errors()

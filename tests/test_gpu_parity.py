@@ -147,12 +147,12 @@ def test_select_merge_reverse_exact(ftk, name):
     np.testing.assert_array_equal(ids.cpu().numpy(), oids)
 
 
-@pytest.mark.parametrize("M", [33, 40, 64, 100, 257, 512, 1000, 1024, 1500])
+@pytest.mark.parametrize("M", [33, 40, 64, 100, 257, 512, 1000, 1024, 1025, 1500,
+                               2048, 2049, 3000])
 def test_select_paths_exact(ftk, M):
     """Every select path (filter-and-sort for up to 32 and up to 64 picks with 32 to
     256 candidates, the extraction loop behind it, the shared-memory kernel above
-    M = 1024) against
-    the oracle: smooth rows, rows with many exact ties, rows whose threshold
+    M = 2048) against the oracle: smooth rows, rows with many exact ties, rows whose threshold
     cuts early, padded first/last blocks, flat rows (all candidates tie)."""
     rng = np.random.default_rng(1000 + M)
     rows = 96
