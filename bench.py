@@ -44,25 +44,25 @@ WORKLOAD = dict(
     score_block_size=64, topk=32, threshold=0.9, q_block_size=64, kv_block_size=64,
     qblock_topk=None,
 )
-# Side workloads (--workload): the other BASELINE.json shapes, per GPU.  The
+# Side workloads (--workload): other shapes of the path, per GPU.  The
 # headline line always comes from WORKLOAD above.
 WORKLOADS = {
     "config2-e2e": WORKLOAD,
-    # configs[0]: the reference's CPU-runnable shape
+    # the reference's CPU-runnable shape
     "config1": dict(name="config1", B=2, N=1024, H=8, D=64, dtype="fp16", input_scale=1.0,
                     score_block_size=64, topk=16, threshold=1.0, q_block_size=32,
                     kv_block_size=64, qblock_topk=None),
-    # configs[2]: full training step, score-weighted merge to 256 blocks
+    # full training step, score-weighted merge to 256 blocks
     "config3": dict(name="config3", B=4, N=8192, H=16, D=128, dtype="bf16", input_scale=1.0,
                     score_block_size=64, topk=16, threshold=1.0, q_block_size=64,
                     kv_block_size=64, qblock_topk=256),
-    # configs[3]: ragged length, virtual padding, hot key blocks, fp16; score + select +
+    # ragged length, virtual padding, hot key blocks, fp16; score + select +
     # merge only (q blocks of 128 rows: the reference's attention stops at 64)
     "config4": dict(name="config4", B=2, N=30000, H=32, D=128, dtype="fp16", input_scale=1.0,
                     score_block_size=128, topk=24, threshold=0.8, q_block_size=128,
                     kv_block_size=128, qblock_topk=None, padding=(40, 40), q_padding=(40, 40),
                     attend=False),
-    # configs[4]: one batch element (64 of its 512 slices) per GPU
+    # one batch element (64 of its 512 slices) per GPU
     "config5": dict(name="config5", B=1, N=65536, H=64, D=128, dtype="bf16", input_scale=1.0,
                     score_block_size=64, topk=64, threshold=1.0, q_block_size=64,
                     kv_block_size=64, qblock_topk=None),
@@ -241,7 +241,7 @@ def run_ours(args):
         if record:
             evs[2].record()
         if not cfg.get("attend", True):
-            # workloads that stop after the merge
+            # workloads that stop after the merge (config4)
             if record:
                 evs[3].record()
                 evs[4].record()
@@ -644,7 +644,7 @@ def main():
                          "reference-gpu = the reference's own V2 CUDA kernels on this GPU "
                          "(needs baseline/_ref)")
     ap.add_argument("--workload", default="config2-e2e", choices=sorted(WORKLOADS),
-                    help="side workloads: the other BASELINE.json shapes (per GPU)")
+                    help="side workloads: other shapes of the path (per GPU)")
     ap.add_argument("--no-reference-gpu", action="store_true",
                     help="skip the reference-V2-on-this-GPU leg of the default run")
     ap.add_argument("--small", action="store_true", help="N=8192, H=16 (profiling-sized case)")

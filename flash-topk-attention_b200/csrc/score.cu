@@ -88,11 +88,6 @@ __device__ __forceinline__ TileInfo tile_info(const ScoreParams& p, int t) {
   return ti;
 }
 
-// Which softmax group drains a CTA's u-th tile: tiles alternate between the two
-// groups, each group bound to one accumulator stage, so a group meets every phase
-// of its stage's barriers in order (a one-bit parity wait must never skip a
-// phase).  When a score block spans several tiles (block size > 128) one
-// thread has to see all of them, and group 0 takes every tile.
 // First tile of part s of the keys: whole score blocks, in order
 __device__ __forceinline__ int seg_begin(const ScoreParams& p, int s) {
   const int per = max(1, p.tiles_per_block);
@@ -272,9 +267,12 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
     }
   } else {
     // ---------------------------------------------------- softmax threads
-    // Two groups of 8 warps.  Each tile is drained by exactly one group (see
-    // tile_owner) so both groups run concurrently on consecutive tiles and
-    // hide each other's TMEM-load and barrier latency.
+    // Two groups of 8 warps, which take the CTA's tiles in turn and so run
+    // concurrently on consecutive ones and hide each other's TMEM-load and barrier
+    // latency.  A group is bound to one accumulator stage and meets every phase of
+    // its barriers in order (a one-bit parity wait must never skip a phase).  When a
+    // score block spans several tiles (block size > 128) one thread has to see all
+    // of them, and group 0 takes every tile.
     const int cw = warp - 2;               // 0..15
     const int group = cw >> 3;
     const int half = (cw >> 2) & 1;        // which 128-row accumulator

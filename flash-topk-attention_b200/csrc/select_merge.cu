@@ -338,7 +338,7 @@ __device__ __forceinline__ void bitonic_desc_blocked(T (&v)[E], int lane) {
 }
 
 // Merge with ONE WARP per q-block, for tables of up to 32*E <= 1024 block ids
-// (every BASELINE shape).  Same arithmetic as qblock_merge_kernel: the entries
+// (all of the benchmark's shapes).  Same arithmetic as qblock_merge_kernel: the entries
 // of the q-block are walked in (row, rank) order, 32 at a time, entries of one
 // step that name the same block are applied in lane order, so every aggregate
 // is the same fp32 sum in the same order.  No block-wide barrier: the warp

@@ -1,5 +1,5 @@
-// Backward at head dim 256 on pairs of SMs (tcgen05 cta_group::2), for 64-row q
-// and kv blocks.  Included by sparse_bwd.cu after sparse_bwd_dq2.cuh.
+// Backward at head dim 256 on pairs of SMs (tcgen05 cta_group::2), for q and kv
+// blocks of 64 or 32 rows.  Included by sparse_bwd.cu after sparse_bwd_dq2.cuh.
 //
 // The scheme is that of the head-dim-128 pair kernels: a cluster of two CTAs owns
 // 256 rows, both walk the union of the pair's four lists, each CTA loads its half

@@ -1,5 +1,5 @@
-// dK/dV on pairs of SMs (tcgen05 cta_group::2), for 64-row q and kv blocks and
-// head dim 128.  Included by sparse_bwd.cu (shares BwdParams).
+// dK/dV on pairs of SMs (tcgen05 cta_group::2), for q and kv blocks of 64 or 32
+// rows and head dim 128.  Included by sparse_bwd.cu (shares BwdParams).
 //
 // Measured on B200: a UMMA of M = 128 with both operands in shared memory costs
 // 75 cycles at N = 64, and the dK/dV kernel spends two thirds of its tensor
@@ -49,7 +49,7 @@ __device__ __forceinline__ uint32_t pack2f(float a, float b) {
 // tile).  With full lists tile i then comes out of all warps ahead of tile i + 1 and
 // its buffer is free earlier (28.8 against 29.1 ms there, 3.76 against 3.98 ms at B = 4,
 // N = 8192, H = 16); with short lists most warps of a tile have nothing to do and
-// should run ahead (610 -> 569 us at W = 16 of 64 blocks, four heads per kv head).
+// should run ahead (610 -> 589 us at W = 16 of 64 blocks, four heads per kv head).
 template <int FMT, bool WALK, bool STEP, int SUB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(BW_THREADS, 1)
 sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,

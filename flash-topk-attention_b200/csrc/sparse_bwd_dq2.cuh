@@ -1,5 +1,5 @@
-// dQ on pairs of SMs (tcgen05 cta_group::2), for 64-row q and kv blocks and
-// head dim 128.  Included by sparse_bwd.cu after sparse_bwd_dkv2.cuh (shares
+// dQ on pairs of SMs (tcgen05 cta_group::2), for q and kv blocks of 64 or 32
+// rows and head dim 128.  Included by sparse_bwd.cu after sparse_bwd_dkv2.cuh (shares
 // BwdParams and the cluster helpers).
 //
 // A cluster of two CTAs owns 256 query rows (four q-blocks); each CTA keeps its

@@ -3,10 +3,11 @@
 // Replaces sparse_attn_fwd_kernel of the reference
 // (flash_topk_attn_v2/csrc/sparse_attn_kernel.cu:6-365).
 //
-// Two kernels: the exact running-maximum kernel below (every supported shape
-// and dtype) and the pipelined fixed-reference kernel of sparse_fwd_pipe.cuh
-// (64-row q and kv blocks), which ftk_sparse_fwd launches first when the
-// caller passes a workspace; the exact kernel then only redoes flagged CTAs.
+// The exact running-maximum kernel below takes every supported shape and dtype.
+// For q and kv blocks of 64 or 32 rows the pipelined fixed-reference kernels of
+// sparse_fwd_pipe.cuh (one CTA per tile) and sparse_fwd_pipe2.cuh (pairs of SMs)
+// run first, when the caller passes a workspace; the exact kernel then only
+// redoes the tiles that they flag.
 //
 // One CTA owns 128 consecutive virtual query rows = G q-blocks of one (batch,
 // head) slice and walks the union of their candidate KV blocks in ascending

@@ -1,12 +1,13 @@
-// Deeply pipelined forward kernel for 64-row kv blocks and q-blocks of 64 or 32
-// rows.  Included by sparse_fwd.cu (shares FwdParams).
+// Deeply pipelined forward kernel for q and kv blocks of 64 or 32 rows.  Included
+// by sparse_fwd.cu (shares FwdParams).
 //
 // The exact kernel keeps a running maximum per softmax group, which ties every
 // P tile to its group's accumulator: two groups, two O accumulators, two S
 // buffers are all that fit in TMEM, and with two tiles in flight the tensor
 // core idles while a group does its exponentials.  Here every row uses ONE
-// fixed reference exponent for the whole list: the scaled maximum of the first
-// kv block its q-block lists (a short prologue computes it).  P = 2^(c S - ref)
+// fixed reference exponent for the whole list: the row's scaled maximum over one
+// tile that its q-block lists, the tile that most of the CTA's q-blocks share
+// (cover_tiles; a short prologue computes it).  P = 2^(c S - ref)
 // then needs no rescaling, all tiles add into a single O accumulator, and NG
 // softmax groups work on NG S buffers at once:
 //   TMEM columns  Q, D / 2 | S/P buffers, 64 each | O, D
@@ -24,10 +25,9 @@
 // N = 8192, grouped heads: 312 -> 291 us from the ring.
 // bf16 and fp32 share the exponent range, so a later block may exceed the
 // reference by up to 2^80 before anything overflows (fp16: 2^15, P must stay
-// below 65504); a row whose tile sum
-// passes that bound marks its CTA's word in `redo_out`, and the exact kernel,
-// launched behind this one, recomputes exactly those CTAs (all others return
-// on their first instruction).
+// below 65504); a row whose tile sum passes that bound marks its tile's word in `redo_out`, and the exact kernel,
+// launched behind this one with a CTA per SM, looks through the words and
+// recomputes exactly those tiles.
 #pragma once
 
 namespace ftk {
@@ -281,7 +281,7 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
 
     if (n > 0) {
-      // ---- reference exponent: scaled row maximum over the q-block's first block
+      // ---- reference exponent: scaled row maximum over the q-block's prologue tile
       // Every warp waits for every prologue buffer, also the ones it does not
       // read: its later parity waits on those buffers must not start while
       // their first phase is still open.

@@ -296,7 +296,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
 
     if (n > 0) {
-      // ---- reference exponent: scaled row maximum over the q-block's first block
+      // ---- reference exponent: scaled row maximum over the q-block's prologue tile
       // Every warp waits for every prologue buffer, also the ones it does not
       // read: its later parity waits on those buffers must not start while
       // their first phase is still open.

@@ -251,9 +251,8 @@ int ftk_attn_bwd_dkv(const ftk_attn* a, const void* dout, int64_t sdo_b, int64_t
  * heads (Hkv <= 0 means H; H must be a multiple): query head h reads kv head
  * h / (H / Hkv).  The reference rejects Hkv != H (__init__.py:153-156).
  * `workspace` (ftk_sparse_fwd_workspace bytes, may be NULL) enables the
- * pipelined kernel for 64-row kv blocks and q-blocks of 64 or 32 rows (bf16 or fp16):
- * it uses one fixed reference exponent per row, and the exact running-maximum
- * kernel, launched behind it, recomputes the tiles whose scores left the safe
+ * pipelined kernel for q and kv blocks of 64 or 32 rows (bf16 or fp16): it uses one
+ * fixed reference exponent per row, and the exact running-maximum kernel, launched behind it, recomputes the tiles whose scores left the safe
  * exponent range (none on ordinary inputs).  Without a workspace only the
  * exact kernel runs.  Setting the environment variable FTK_FWD_PIPE=0 does the
  * same.  At head dim 256, and at head dim 128 with lists that can cover a good

@@ -117,8 +117,8 @@ def _lists_with_one_bad_id(H, QM, M, W, bad_at, bad_id):
 @pytest.mark.parametrize("D,g,kvb,dtype", [(128, 64, 64, "bf16"), (64, 32, 64, "fp16")])
 def test_out_of_range_block_id_in_attention_lists(ftk, D, g, kvb, dtype):
     """Forward and dQ walk merged_indices (pair kernels at D = 128 with 64-row
-    blocks, one-CTA kernels otherwise); dK/dV walks the reverse index built from
-    it.  The bad id is dropped, status 105 is raised, every output equals the
+    blocks, one-CTA kernels otherwise); dK/dV walks the tile masks that dQ leaves.
+    The bad id is dropped, status 105 is raised, every output equals the
     run on the same lists with that entry removed."""
     H, N = 2, 512
     cfg = dict(B=1, N=N, H=H, D=D, dtype=dtype, seed=81, do_seed=82)
@@ -205,9 +205,9 @@ def test_out_of_range_block_id_in_merge_and_reverse(ftk):
 
 
 def test_device_error_surfaces_at_a_later_call_without_check_errors(ftk):
-    """A caller that never calls check_errors(): every operator leaves a copy of
-    the status word in pinned memory and looks at the previous copy, so the
-    failure of one call raises at a following call."""
+    """A caller that never calls check_errors(): every operator begins with a
+    look at the status word, which lies in pinned memory, so the failure of one call
+    raises at a following call."""
     rng = np.random.default_rng(5)
     M, K, g = 16, 4, 32
     idx = np.stack([rng.permutation(M)[:K] for _ in range(2 * 256)]).astype(np.int32)
