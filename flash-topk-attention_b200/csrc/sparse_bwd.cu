@@ -66,22 +66,23 @@ struct BwdParams {
 };
 
 // ------------------------------------------------------------------- delta
-// delta[row] = sum_d o * do for the 128 rows of a dQ tile, by all warps of the
-// CTA, into shared memory (for the tile itself) and global memory (for dK/dV).
+// delta[row] = sum_d o * do for the 128 rows of a dQ tile, by the compute warps of the
+// CTA (the others load and issue meanwhile), into shared memory (for the tile itself) and global memory (for dK/dV).
 // kd / 8 lanes per row, each with one 16-byte load per tensor, so a warp covers
 // 256 / kd rows at once and a thread has all of its loads in flight together.
 // As a kernel of its own this cost a launch and 258 us at N = 32768, H = 32,
 // D = 128 (122 us at B = 4, N = 8192, H = 16), reading O and dO at 4.2 TB/s;
 // here the reads hide behind the other CTAs' UMMAs.
-// The loads are issued before the union is built and used after it.
-template <int KD, int THREADS = BW_THREADS>
+// The loads are issued before the union is built, the sums are taken once Q and dO are
+// on their way into TMEM.
+template <int KD, int WARPS = 16>
 struct TileDelta {
-  static constexpr int LPR = KD / 8, RPW = 32 / LPR, WARPS = THREADS / 32;
+  static constexpr int LPR = KD / 8, RPW = 32 / LPR;
   static constexpr int STEPS = (128 + RPW * WARPS - 1) / (RPW * WARPS);
   uint4 vd[STEPS], vo[STEPS], vo2[STEPS];   // vo2: float32 O only
 
   __device__ __forceinline__ int row(int i) const {
-    return (i * WARPS + (threadIdx.x >> 5)) * RPW + (threadIdx.x & 31) / LPR;
+    return (i * WARPS + (threadIdx.x >> 5) - 2) * RPW + (threadIdx.x & 31) / LPR;
   }
   __device__ __forceinline__ bool inside(const BwdParams& p, int r, int n, int rows) const {
     return r < rows && n >= 0 && n < p.N && (threadIdx.x & 31) % LPR * 8 < p.D;
@@ -246,6 +247,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
   uint8_t* sK = smem + 2 * ROW_TILE_BYTES;
   __shared__ UnionScratch un;
   __shared__ float s_delta[128];
+  __shared__ OutTile s_out;
   __shared__ __align__(8) uint64_t bars[1 + 2 * DQ_KST + DQ_VST + 2 * NG + 2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
@@ -302,7 +304,11 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_alloc(smem_u32(&tmem_base_s), TMEM_COLS);
     tmem_relinquish();
   }
-  clear_bitmaps(un);
+  if (tid == 32)
+    s_out = {{static_cast<int64_t>(b_idx) * p.s0_b + static_cast<int64_t>(h_idx) * p.s0_h, 0},
+             tile_row0, min(p.N, tile_row0 + groups * p.g)};
+  clear_flags(sK, p.Mkv, groups);
+  tc_fence_before();
   pdl_wait();
   if (tid == 0) {   // under the building of the union
     mbar_expect_tx(bar_q, 2 * ROW_TILE_BYTES);
@@ -311,18 +317,20 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       tma_load_4d(smem_u32(sDO) + c * 128 * 128, &tm_do, bar_q, c * 64, h_idx, tile_row0, b_idx);
     }
   }
-  TileDelta<D, bw_threads(NG)> delta;
-  if (D <= 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);
-  const int n = build_union<NG == 1 || D == 128>(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
-                            p.W, nullptr, p.Mkv, p.sub, p.lm, p.status);
+  TileDelta<D, 8 * NG> delta;
+  float lse_mine = 0.f;   // of the row that a compute thread works on
+  if (warp >= 2) {
+    const int r = (warp & 3) * 32 + lane, qrow = tile_row0 + r;
+    if (r < groups * p.g && qrow >= 0 && qrow < p.N) lse_mine = p.lse[static_cast<int64_t>(bh) * p.N + qrow];
+    if (D <= 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);
+  }
+  const TileMaskRow mask_row = {
+      p.masks ? p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + blockIdx.x) * p.mask_stride : nullptr,
+      0, groups};
+  const int n = build_union<bw_threads(NG) / 32>(
+      un, sK, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups, p.W, nullptr, p.Mkv,
+      p.sub, p.lm, p.status, mask_row);
   pdl_launch();
-  if (D > 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);   // too many registers to hold across the union
-  delta.finish(p, s_delta, bh, tile_row0, groups * p.g);
-  if (p.masks)
-    write_tile_masks(un, p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + blockIdx.x) * p.mask_stride,
-                     p.mask_stride, 0, groups);
-  tc_fence_before();
-  __syncthreads();
   tc_fence_after();
   const uint32_t tmem = NG == 2 ? tmem_base_s : __shfl_sync(0xffffffffu, tmem_base_s, 0);
   WaitCtx w{&abort_flag, p.status};
@@ -464,11 +472,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int cbeg = split ? colhalf * (p.kvb / 2) : 0;
     const int cend = split ? cbeg + p.kvb / 2 : (colhalf == 0 ? p.kvb : 0);
     const float c = p.scale_log2;
-    float lse2 = 0.f, dl = 0.f;
-    if (row_valid) {
-      lse2 = p.lse[static_cast<int64_t>(bh) * p.N + qrow] * 1.4426950408889634f;
-      dl = s_delta[r];
-    }
+    const float lse2 = lse_mine * 1.4426950408889634f;
     bool ok = true;
     const int copies = NG == 2 ? wg : colhalf;   // Q or dO
     if (!BIG && n > 0 && (NG == 1 || colhalf == 0)) {
@@ -497,6 +501,12 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_qt);
     }
+    // the sums run under the first UMMAs (256 columns are too many registers to hold
+    // across the union)
+    if (D > 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);
+    delta.finish(p, s_delta, bh, tile_row0, groups * p.g);
+    asm volatile("bar.sync 1, %0;" ::"n"(256 * NG) : "memory");
+    const float dl = row_valid ? s_delta[r] : 0.f;
     for (int i = wg; ok && i < n; i += NG) {
       // A(i) complete also means B(i - NG) has retired (same issue order), so the
       // dS columns of this buffer are free again.
@@ -504,7 +514,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       const int tok0 = static_cast<int>(un.ids[i]) * p.kvb - p.kv_pad_head;
       const ColSpan cs = col_span(un, i, p.sub, grp, tok0, p.kvb, p.N);
       const int lo = cs.lo, hi = cs.hi;
-      const bool act = row_valid && cs.on;
+      const bool act = cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == p.kvb;
       const bool none = !fast && !__any_sync(0xffffffffu, act);
       if (!mbar_wait(bar_afull(wg), (i / NG) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
@@ -569,34 +579,29 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
       if (lane == 0) mbar_arrive(bar_dsfull(wg));
     }
     // epilogue: each group converts and stores one half of the head dimension
-    if (ok && n > 0)
-      ok = mbar_wait(bar_final, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
+    if (ok) ok = mbar_wait(n > 0 ? bar_final : bar_q, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
     if (ok) {
       tc_fence_after();
-      uint8_t* orow = nullptr;
-      if (row_valid)
-        orow = static_cast<uint8_t*>(p.out0) +
-               (p.out_f32 ? 4 : 2) *
-                   (static_cast<int64_t>(b_idx) * p.s0_b + static_cast<int64_t>(qrow) * p.s0_n +
-                    static_cast<int64_t>(h_idx) * p.s0_h);
+      // every copy has landed and every UMMA has retired: the tiles make room for dQ
+      const int ew = (late_tid() >> 5) - 2;   // 32-column chunks dealt to the warps of a lane quarter
       // 32-column chunks of the head dim are dealt round-robin to the four
       // warps of a lane quarter
-      for (int c0 = (wg * 2 + colhalf) * 32; c0 < D; c0 += 128) {
+#pragma unroll 1
+      for (int c0 = (ew >> 2) * 32; c0 < D; c0 += 128) {
         uint32_t v[32];
         if (n > 0) {
           tmem_ld32(lane_addr + COL_DQ + c0, v);
           tmem_wait_ld();
         }
-        if (row_valid) {
-          uint32_t pk[16];
+        uint32_t pk[16];
 #pragma unroll
-          for (int x = 0; x < 32; x += 2) {
-            const float a = n > 0 ? __uint_as_float(v[x]) * p.scale : 0.f;
-            const float b = n > 0 ? __uint_as_float(v[x + 1]) * p.scale : 0.f;
-            pk[x >> 1] = pack2(a, b, p.fmt);
-          }
-          store_row_part(orow, c0, p.D, pk, p.fmt, p.out_f32 != 0);
+        for (int x = 0; x < 32; x += 2) {
+          const float a = n > 0 ? __uint_as_float(v[x]) * p.scale : 0.f;
+          const float b = n > 0 ? __uint_as_float(v[x + 1]) * p.scale : 0.f;
+          pk[x >> 1] = pack2(a, b, p.fmt);
         }
+        store_rows(smem + ew * 2048, pk, p.out0, s_out, 0, (ew + 2) & 3, p.s0_n, c0, p.D, p.fmt,
+                 p.out_f32 != 0);
       }
     }
   }
@@ -608,21 +613,21 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
 }
 
 // -------------------------------------------------------------------- dK/dV
-// Union of the lists of kv blocks j0 .. j0 + groups - 1, from the dQ kernel's
-// tile masks or from a reverse index.
-__device__ __forceinline__ int dkv_union(UnionScratch& un, const BwdParams& p, int bhq, int j0,
-                                         int groups) {
-  clear_bitmaps(un);
-  pdl_wait();
+// Union of the lists of kv blocks j0 .. j0 + groups - 1 (`per` of them where the grid
+// does not end), from the dQ kernel's tile masks or from a reverse index.  The caller has
+// called pdl_wait.
+__device__ __forceinline__ int dkv_union(UnionScratch& un, uint8_t* flags, const BwdParams& p, int bhq,
+                                         int j0, int groups, int per) {
   int n;
   if (p.masks) {
     const int64_t per_head = static_cast<int64_t>(p.mask_tiles) * p.mask_stride;
-    n = build_union_masks(un, p.masks + bhq * per_head, p.mask_stride, p.mask_tiles, p.mask_g, j0,
-                          groups, p.heads, per_head, p.span, p.sub);
+    n = build_union_masks<BW_THREADS / 32>(un, p.masks + bhq * per_head, p.mask_stride, p.mask_tiles,
+                                           p.mask_g, j0, per, p.heads, per_head, p.span, p.sub);
   } else {
     const int64_t kv_row = static_cast<int64_t>(bhq) * p.Mkv + j0;
-    n = build_union(un, p.lists + kv_row * p.QM, 0, groups, p.QM, p.counts + kv_row, p.QM, p.sub,
-                    ListMap{0, 0, 0, 0}, p.status);
+    clear_flags(flags, p.QM, groups);
+    n = build_union<BW_THREADS / 32>(un, flags, p.lists + kv_row * p.QM, 0, groups, p.QM,
+                                     p.counts + kv_row, p.QM, p.sub, ListMap{0, 0, 0, 0}, p.status);
   }
   pdl_launch();   // the unions hold the barrier that follows the caller's tmem_alloc
   return n;
@@ -674,6 +679,7 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
   __shared__ UnionScratch un;
   __shared__ __align__(8) uint64_t bars[1 + 2 * BW_MAX_STAGES + 6];   // last: K, V in TMEM
   __shared__ uint32_t tmem_base_s;
+  __shared__ OutTile s_out;
   __shared__ int abort_flag;
   __shared__ __align__(16) float s_lse2[2][2][128], s_delta[2][2][128];  // [group][parity][q row]
 
@@ -745,9 +751,25 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_alloc(smem_u32(&tmem_base_s), 512);
     tmem_relinquish();
   }
-  const int n = dkv_union(un, p, bhq, j0, groups);
+  if (tid == 32) {
+    const int64_t hk = WALK ? h_idx / p.heads : h_idx;
+    s_out = {{static_cast<int64_t>(b_idx) * p.s0_b + hk * p.s0_h,
+              static_cast<int64_t>(b_idx) * p.s1_b + hk * p.s1_h},
+             tile_tok0, min(p.N, tile_tok0 + groups * p.kvb)};
+  }
   tc_fence_before();
-  __syncthreads();
+  pdl_wait();
+  if (tid == 0) {   // under the building of the union
+    mbar_expect_tx(bar_kv, (MODE == 1 ? 1 : 2) * ROW_TILE_BYTES);
+    for (int c = 0; c < NCH; c++) {
+      tma_load_4d(smem_u32(sK) + c * 128 * 128, &tm_k, bar_kv, c * 64, h_idx / p.kv_hdiv, tile_tok0,
+                  b_idx);
+      if (MODE != 1)
+        tma_load_4d(smem_u32(sV) + c * 128 * 128, &tm_v, bar_kv, c * 64, h_idx / p.kv_hdiv, tile_tok0,
+                    b_idx);
+    }
+  }
+  const int n = dkv_union(un, sQD, p, bhq, j0, groups, p.G);
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
   WaitCtx w{&abort_flag, p.status};
@@ -755,14 +777,6 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
 
   if (warp == 0) {
     if (lane == 0 && n > 0) {
-      mbar_expect_tx(bar_kv, (MODE == 1 ? 1 : 2) * ROW_TILE_BYTES);
-      for (int c = 0; c < NCH; c++) {
-        tma_load_4d(smem_u32(sK) + c * 128 * 128, &tm_k, bar_kv, c * 64, h_idx / p.kv_hdiv,
-                    tile_tok0, b_idx);
-        if (MODE != 1)
-          tma_load_4d(smem_u32(sV) + c * 128 * 128, &tm_v, bar_kv, c * 64, h_idx / p.kv_hdiv,
-                      tile_tok0, b_idx);
-      }
       HeadWalk<WALK> hw;
       for (int i = 0; i < n; i++) {
         const int s = i % NST;
@@ -908,8 +922,6 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int r = quarter * 32 + lane;
     const int ct = (tid - 64) & 255;         // index inside the group
     const int grp = r / p.kvb;
-    const int tok = tile_tok0 + r;
-    const bool row_valid = (grp < groups) && tok >= 0 && tok < p.N;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t st_addr = lane_addr + wg * 64;         // S^T, then P^T
     const uint32_t dp_addr = lane_addr + 128 + wg * 64;   // dP^T, then dS^T
@@ -969,7 +981,7 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
       tc_fence_after();
       const ColSpan cs = col_span(un, i, p.sub, grp, row0, p.g, p.N);
       const int lo = cs.lo, hi = cs.hi;
-      const bool act = row_valid && cs.on;
+      const bool act = cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == p.g;
       const bool none = !fast && !__any_sync(0xffffffffu, act);
       const float4* l4 = reinterpret_cast<const float4*>(s_lse2[wg][pb]);
@@ -1025,39 +1037,32 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_pfull(wg));
     }
-    if (ok && n > 0)
-      ok = mbar_wait(bar_final, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
+    if (ok) ok = mbar_wait(n > 0 ? bar_final : bar_kv, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
     if (ok) {
       tc_fence_after();
       // MODE 0: group 0 stores dV (TMEM 256..), group 1 stores dK (TMEM 384.., scaled);
       // otherwise both groups share the one accumulator's columns
-      const int which = MODE == 0 ? wg : MODE - 1;
-      uint8_t* base = static_cast<uint8_t*>(which == 0 ? p.out1 : p.out0);
-      const int64_t sb_ = which == 0 ? p.s1_b : p.s0_b, sn_ = which == 0 ? p.s1_n : p.s0_n,
-                    sh_ = which == 0 ? p.s1_h : p.s0_h;
+      const int ew = (late_tid() >> 5) - 2;
+      const int which = MODE == 0 ? ew >> 3 : MODE - 1;
       const float mul = which == 0 ? 1.f : p.scale;
-      uint8_t* orow = nullptr;
-      if (row_valid)
-        orow = base + (p.out_f32 ? 4 : 2) *
-                          (static_cast<int64_t>(b_idx) * sb_ + static_cast<int64_t>(tok) * sn_ +
-                           static_cast<int64_t>(WALK ? h_idx / p.heads : h_idx) * sh_);
-      const int cfirst = MODE == 0 ? colhalf * 32 : (wg * 2 + colhalf) * 32;
+      // every copy has landed and every UMMA has retired: the tiles make room for the results
+      const int cfirst = MODE == 0 ? ((ew >> 2) & 1) * 32 : (ew >> 2) * 32;
+#pragma unroll 1
       for (int c0 = cfirst; c0 < D; c0 += (MODE == 0 ? 64 : 128)) {
         uint32_t v[32];
         if (n > 0) {
           tmem_ld32(lane_addr + (which == 0 ? COL_DV : COL_DK) + c0, v);
           tmem_wait_ld();
         }
-        if (row_valid) {
-          uint32_t pk[16];
+        uint32_t pk[16];
 #pragma unroll
-          for (int x = 0; x < 32; x += 2) {
-            const float a = n > 0 ? __uint_as_float(v[x]) * mul : 0.f;
-            const float b = n > 0 ? __uint_as_float(v[x + 1]) * mul : 0.f;
-            pk[x >> 1] = pack2(a, b, p.fmt);
-          }
-          store_row_part(orow, c0, p.D, pk, p.fmt, p.out_f32 != 0);
+        for (int x = 0; x < 32; x += 2) {
+          const float a = n > 0 ? __uint_as_float(v[x]) * mul : 0.f;
+          const float b = n > 0 ? __uint_as_float(v[x + 1]) * mul : 0.f;
+          pk[x >> 1] = pack2(a, b, p.fmt);
         }
+        store_rows(smem + ew * 2048, pk, which == 0 ? p.out1 : p.out0, s_out, which == 0 ? 1 : 0,
+                   (ew + 2) & 3, which == 0 ? p.s1_n : p.s0_n, c0, p.D, p.fmt, p.out_f32 != 0);
       }
     }
   }
@@ -1202,7 +1207,7 @@ struct BwdPlan {
   AttnGrid gr;
   bool pair_dq, pair_dkv;    // kernels on pairs of SMs
   bool walk;                 // dK/dV: one CTA walks all query heads of its kv head
-  int tiles, stride, span;   // tile masks (see write_tile_masks)
+  int tiles, stride, span;   // tile masks (see TileMaskRow)
   int kv_tiles;              // 128-row kv tiles per slice
   bool order;                // dK/dV tiles sorted by the work they have
   size_t off_masks, off_order, off_dk, off_dv, bytes;
@@ -1225,7 +1230,7 @@ static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
   const int64_t BH = a.B * a.H;
   const int per = attn_groups(gr.g), G = attn_groups(gr.kvb);
   b.tiles = (gr.QM + per - 1) / per;
-  b.stride = (gr.Mkv + 15) & ~15;
+  b.stride = flag_blocks(gr.Mkv);
   b.span = (b.tiles * per + 31) & ~31;
   b.kv_tiles = (gr.Mkv + G - 1) / G;
   // Pairs walk the union of four lists.  For dQ the line is that of ftk_attn_fwd
@@ -1353,15 +1358,19 @@ static int launch_dq(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, b
   if (kd == 256) {
     // Q and dO resident, three K and two V tiles behind them: kv blocks of at most 32 rows
     if (p.kvb > 32) return FTK_ERR_UNSUPPORTED;
-    const size_t smem = 1024 + 2 * nch * 128 * 128 + static_cast<size_t>(3 + 2) * nch * p.kvb * 128;
+    const size_t smem =
+        1024 + 2 * nch * 128 * 128 +
+        std::max(static_cast<size_t>(3 + 2) * nch * p.kvb * 128, flag_bytes(p.Mkv, p.G));
     if ((e = allow_smem<sparse_bwd_dq_kernel<256, 2>>(smem))) return e;
     return launch_pdl(sparse_bwd_dq_kernel<256, 2>, grid, BW_THREADS, smem, st, tq, tdo, tk, tv, p);
   }
   auto go = [&](auto kernel_tag, int ng) -> int {
     constexpr auto kernel = decltype(kernel_tag)::kernel;
-    // four V slots lie over the Q / dO tiles, the rest of the V ring behind the K ring
+    // four V slots lie over the Q / dO tiles, the rest of the V ring behind the K ring; the
+    // marks of the list union where the K ring will be
     const size_t smem = 1024 + 2 * nch * 128 * 128 +
-                        static_cast<size_t>(dq_kst(ng) + DQ_VST - 4) * nch * p.kvb * 128;
+                        std::max(static_cast<size_t>(dq_kst(ng) + DQ_VST - 4) * nch * p.kvb * 128,
+                                 flag_bytes(p.Mkv, p.G));
     if (int r = allow_smem<kernel>(smem)) return r;
     return launch_pdl(kernel, grid, bw_threads(ng), smem, st, tq, tdo, tk, tv, p);
   };
@@ -1426,7 +1435,7 @@ static int launch_dkv(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, 
   };
   auto smem_for = [&](int resident, int nst) {
     return static_cast<size_t>(1024) + static_cast<size_t>(resident) * tile_bytes +
-           static_cast<size_t>(nst) * stage_bytes;
+           std::max(static_cast<size_t>(nst) * stage_bytes, p.masks ? 0 : flag_bytes(p.QM, p.G));
   };
   const dim3 grid(p.order ? p.Mkv : (p.Mkv + p.G - 1) / p.G, slices);
   auto go = [&](auto kernel_tag, int resident) -> int {

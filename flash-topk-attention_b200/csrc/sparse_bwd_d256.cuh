@@ -67,6 +67,7 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
   uint8_t* sRing = smem + 2 * B6_ROWS;
   __shared__ UnionScratch un;
   __shared__ float s_delta[128];
+  __shared__ OutTile s_out;
   __shared__ __align__(8) uint64_t bars[2 + 3 * SLOTS + 5];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
@@ -115,10 +116,14 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_alloc2(smem_u32(&tmem_base_s), 512);
     tmem_relinquish2();
   }
-  clear_bitmaps(un);
+  clear_flags(sRing, p.Mkv, groups);
+  tc_fence_before();
   cluster_arrive();
   pdl_wait();
   const int mine = min(per, groups - per * static_cast<int>(rank));   // q-blocks of my tile, if any
+  if (tid == 32)
+    s_out = {{static_cast<int64_t>(b_idx) * p.s0_b + static_cast<int64_t>(h_idx) * p.s0_h, 0},
+             tile_row0, min(p.N, tile_row0 + mine * p.g)};
   if (tid == 0) {   // under the building of the union
     mbar_expect_tx(bar_q, 2 * B6_ROWS);
     for (int c = 0; c < NCH; c++) {
@@ -127,18 +132,20 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
   }
   TileDelta<D> delta;
-  const int n = build_union(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
-                            p.W, nullptr, p.Mkv, SUB, p.lm, p.status);
+  float lse_mine = 0.f;   // of the row that a compute thread works on
+  if (warp >= 2) {
+    const int r = (warp & 3) * 32 + lane, qrow = tile_row0 + r;
+    if (r < mine * p.g && qrow >= 0 && qrow < p.N) lse_mine = p.lse[static_cast<int64_t>(bh) * p.N + qrow];
+  }
+  const TileMaskRow mask_row = {
+      p.masks && mine > 0
+          ? p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + blockIdx.x) * p.mask_stride
+          : nullptr,
+      per * static_cast<int>(rank), mine};
+  const int n = build_union<BW_THREADS / 32>(
+      un, sRing, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups, p.W, nullptr, p.Mkv,
+      SUB, p.lm, p.status, mask_row);
   pdl_launch();
-  delta.load(p, b_idx, h_idx, tile_row0, mine * p.g);   // 256 columns: too many registers to hold across the union
-  delta.finish(p, s_delta, bh, tile_row0, mine * p.g);
-  if (p.masks && mine > 0)
-    write_tile_masks(un,
-                     p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + blockIdx.x) *
-                                   p.mask_stride,
-                     p.mask_stride, per * static_cast<int>(rank), mine);
-  tc_fence_before();
-  __syncthreads();
   cluster_wait();            // barriers of both CTAs are initialised before anyone signals them
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
@@ -289,12 +296,13 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
     const uint32_t dp_addr = lane_addr + COL_DP + wg * 64;
     const int cbeg = colhalf * 32;
     const float c = p.scale_log2;
-    float lse2 = 0.f, dl = 0.f;
-    if (row_valid) {
-      lse2 = p.lse[static_cast<int64_t>(bh) * p.N + qrow] * 1.4426950408889634f;
-      dl = s_delta[r];
-    }
+    const float lse2 = lse_mine * 1.4426950408889634f;
     bool ok = true;
+    // 256 columns are too many registers to hold across the union
+    delta.load(p, b_idx, h_idx, tile_row0, mine * p.g);
+    delta.finish(p, s_delta, bh, tile_row0, mine * p.g);
+    asm volatile("bar.sync 1, 512;" ::: "memory");
+    const float dl = row_valid ? s_delta[r] : 0.f;
     for (int i = wg; ok && i < n; i += 2) {
       if (!mbar_wait(bar_afull(wg), (i >> 1) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
         ok = false;
@@ -304,7 +312,7 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
       const int tok0 = static_cast<int>(un.ids[i]) * G - p.kv_pad_head;
       const ColSpan cs = col_span(un, i, SUB, grp, tok0, G, p.N);
       const int lo = cs.lo, hi = cs.hi;
-      const bool act = row_valid && cs.on;
+      const bool act = cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
       const bool none = !fast && !__any_sync(0xffffffffu, act);
       uint32_t sv[32], dv[32], pk[16];
@@ -336,31 +344,27 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
       __syncwarp();
       if (lane == 0) mbar_arrive_cta(bar_dsfull(wg), 0);
     }
-    if (ok && n > 0) ok = mbar_wait(bar_final, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
+    if (ok) ok = mbar_wait(n > 0 ? bar_final : bar_q, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
     if (ok) {
       tc_fence_after();
-      uint8_t* orow = nullptr;
-      if (row_valid)
-        orow = static_cast<uint8_t*>(p.out0) +
-               (p.out_f32 ? 4 : 2) *
-                   (static_cast<int64_t>(b_idx) * p.s0_b + static_cast<int64_t>(qrow) * p.s0_n +
-                    static_cast<int64_t>(h_idx) * p.s0_h);
-      for (int c0 = (wg * 2 + colhalf) * 32; c0 < D; c0 += 128) {
+      // every copy has landed and every UMMA has retired: the tiles make room for dQ
+      const int ew = (late_tid() >> 5) - 2;   // 32-column chunks dealt to the warps of a lane quarter
+#pragma unroll 1
+      for (int c0 = (ew >> 2) * 32; c0 < D; c0 += 128) {
         uint32_t v[32];
         if (n > 0) {
           tmem_ld32(lane_addr + COL_DQ + c0, v);
           tmem_wait_ld();
         }
-        if (row_valid) {
-          uint32_t pk[16];
+        uint32_t pk[16];
 #pragma unroll
-          for (int x = 0; x < 32; x += 2) {
-            const float a = n > 0 ? __uint_as_float(v[x]) * p.scale : 0.f;
-            const float b = n > 0 ? __uint_as_float(v[x + 1]) * p.scale : 0.f;
-            pk[x >> 1] = pack2f<FMT>(a, b);
-          }
-          store_row_part(orow, c0, p.D, pk, FMT, p.out_f32 != 0);
+        for (int x = 0; x < 32; x += 2) {
+          const float a = n > 0 ? __uint_as_float(v[x]) * p.scale : 0.f;
+          const float b = n > 0 ? __uint_as_float(v[x + 1]) * p.scale : 0.f;
+          pk[x >> 1] = pack2f<FMT>(a, b);
         }
+        store_rows(smem + ew * 2048, pk, p.out0, s_out, 0, (ew + 2) & 3, p.s0_n, c0, p.D, FMT,
+                 p.out_f32 != 0);
       }
     }
   }
@@ -398,11 +402,11 @@ sparse_bwd_dkv256_kernel(const __grid_constant__ CUtensorMap tm_q,
   __shared__ UnionScratch un;
   __shared__ __align__(8) uint64_t bars[2 + 3 * SLOTS + 2 * AHEAD + 1];
   __shared__ uint32_t tmem_base_s;
+  __shared__ OutTile s_out;
   __shared__ int abort_flag;
-  // lse and delta of the q columns lie over the bitmaps, which are dead once the
-  // union is listed: [buffer][parity][column] (MODE 1), [what][buffer][column] (MODE 2)
-  static_assert(sizeof(un.bm) >= 8 * 64 * sizeof(float), "");
-  float* s_cols = reinterpret_cast<float*>(&un.bm[0][0]);
+  // lse and delta of the q columns: [buffer][parity][column] (MODE 1), [what][buffer][column]
+  // (MODE 2)
+  __shared__ __align__(16) float s_cols[8 * 64];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
@@ -451,6 +455,13 @@ sparse_bwd_dkv256_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_alloc2(smem_u32(&tmem_base_s), 512);
     tmem_relinquish2();
   }
+  if (tid == 32) {
+    const int64_t hk = WALK ? h_idx / p.heads : h_idx;
+    s_out = {{static_cast<int64_t>(b_idx) * p.s0_b + hk * p.s0_h,
+              static_cast<int64_t>(b_idx) * p.s1_b + hk * p.s1_h},
+             tile_tok0, min(p.N, tile_tok0 + (groups - per * static_cast<int>(rank)) * p.kvb)};
+  }
+  tc_fence_before();
   cluster_arrive();
   pdl_wait();
   if (tid == 0) {   // under the building of the union
@@ -463,9 +474,7 @@ sparse_bwd_dkv256_kernel(const __grid_constant__ CUtensorMap tm_q,
                     tile_tok0, b_idx);
     }
   }
-  const int n = dkv_union(un, p, bhq, j0, groups);
-  tc_fence_before();
-  __syncthreads();
+  const int n = dkv_union(un, sRing, p, bhq, j0, groups, 2 * per);
   cluster_wait();            // barriers of both CTAs are initialised before anyone signals them
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
@@ -618,8 +627,6 @@ sparse_bwd_dkv256_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
     const int grp = per * static_cast<int>(rank) + r / p.kvb;   // kv block of the pair
-    const int tok = tile_tok0 + r;
-    const bool row_valid = (grp < groups) && tok >= 0 && tok < p.N;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     const float c = p.scale_log2;
     const float2 c2 = make_float2(c, c);
@@ -665,7 +672,7 @@ sparse_bwd_dkv256_kernel(const __grid_constant__ CUtensorMap tm_q,
       tc_fence_after();
       const ColSpan cs = col_span(un, i, SUB, grp, row0, G, p.N);
       const int lo = cs.lo, hi = cs.hi;
-      const bool act = row_valid && cs.on;
+      const bool act = cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
       const bool none = !fast && !__any_sync(0xffffffffu, act);
       const float4* l4 = reinterpret_cast<const float4*>(nl);
@@ -751,34 +758,28 @@ sparse_bwd_dkv256_kernel(const __grid_constant__ CUtensorMap tm_q,
       __syncwarp();
       if (lane == 0) mbar_arrive_cta(bar_pfull(sb), 0);
     }
-    if (ok && n > 0) ok = mbar_wait(bar_final, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
+    if (ok) ok = mbar_wait(n > 0 ? bar_final : bar_kv, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
     if (ok) {
       tc_fence_after();
-      uint8_t* base = static_cast<uint8_t*>(MODE == 1 ? p.out1 : p.out0);
-      const int64_t sb_ = MODE == 1 ? p.s1_b : p.s0_b, sn_ = MODE == 1 ? p.s1_n : p.s0_n,
-                    sh_ = MODE == 1 ? p.s1_h : p.s0_h;
+      const int ew = (late_tid() >> 5) - 2;
       const float mul = MODE == 1 ? 1.f : p.scale;
-      uint8_t* orow = nullptr;
-      if (row_valid)
-        orow = base + (p.out_f32 ? 4 : 2) *
-                          (static_cast<int64_t>(b_idx) * sb_ + static_cast<int64_t>(tok) * sn_ +
-                           static_cast<int64_t>(WALK ? h_idx / p.heads : h_idx) * sh_);
-      for (int c0 = gw * 32; c0 < D; c0 += 128) {
+      // every copy has landed and every UMMA has retired: the tiles make room for the results
+#pragma unroll 1
+      for (int c0 = (ew >> 2) * 32; c0 < D; c0 += 128) {
         uint32_t v[32];
         if (n > 0) {
           tmem_ld32(lane_addr + COL_OUT + c0, v);
           tmem_wait_ld();
         }
-        if (row_valid) {
-          uint32_t pk[16];
+        uint32_t pk[16];
 #pragma unroll
-          for (int x = 0; x < 32; x += 2) {
-            const float a = n > 0 ? __uint_as_float(v[x]) * mul : 0.f;
-            const float b = n > 0 ? __uint_as_float(v[x + 1]) * mul : 0.f;
-            pk[x >> 1] = pack2f<FMT>(a, b);
-          }
-          store_row_part(orow, c0, p.D, pk, FMT, p.out_f32 != 0);
+        for (int x = 0; x < 32; x += 2) {
+          const float a = n > 0 ? __uint_as_float(v[x]) * mul : 0.f;
+          const float b = n > 0 ? __uint_as_float(v[x + 1]) * mul : 0.f;
+          pk[x >> 1] = pack2f<FMT>(a, b);
         }
+        store_rows(smem + ew * 2048, pk, MODE == 1 ? p.out1 : p.out0, s_out, MODE == 1 ? 1 : 0,
+                   (ew + 2) & 3, MODE == 1 ? p.s1_n : p.s0_n, c0, p.D, FMT, p.out_f32 != 0);
       }
     }
   }

@@ -73,6 +73,7 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
   __shared__ UnionScratch un;
   __shared__ __align__(8) uint64_t bars[2 + 3 * DK2_STAGES + 5];
   __shared__ uint32_t tmem_base_s;
+  __shared__ OutTile s_out;
   __shared__ int abort_flag;
   // per compute warp and parity: lse, then delta, of the warp's 16 q columns (STEP:
   // per parity, of all 64)
@@ -126,11 +127,27 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_alloc2(smem_u32(&tmem_base_s), 512);
     tmem_relinquish2();
   }
-  // both CTAs build the same union over the pair's four reverse lists
-  const int n = dkv_union(un, p, bhq, j0, groups);
+  if (tid == 32) {
+    const int64_t hk = WALK ? h_idx / p.heads : h_idx;
+    s_out = {{static_cast<int64_t>(b_idx) * p.s0_b + hk * p.s0_h,
+              static_cast<int64_t>(b_idx) * p.s1_b + hk * p.s1_h},
+             tile_tok0, min(p.N, tile_tok0 + (groups - per * static_cast<int>(rank)) * p.kvb)};
+  }
   tc_fence_before();
-  __syncthreads();
-  cluster_sync_all();        // barriers of both CTAs are initialised before anyone signals them
+  cluster_arrive();
+  pdl_wait();
+  if (tid == 0) {   // under the building of the union
+    mbar_expect_tx(bar_kv, 2 * ROW_TILE_BYTES);
+    for (int c = 0; c < NCH; c++) {
+      tma_load_4d(smem_u32(sK) + c * 128 * 128, &tm_k, bar_kv, c * 64, h_idx / p.kv_hdiv,
+                  tile_tok0, b_idx);
+      tma_load_4d(smem_u32(sV) + c * 128 * 128, &tm_v, bar_kv, c * 64, h_idx / p.kv_hdiv,
+                  tile_tok0, b_idx);
+    }
+  }
+  // both CTAs build the same union over the pair's four reverse lists
+  const int n = dkv_union(un, sQD, p, bhq, j0, groups, 2 * per);
+  cluster_wait();            // barriers of both CTAs are initialised before anyone signals them
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
   WaitCtx w{&abort_flag, p.status};
@@ -138,13 +155,6 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
   if (warp == 0) {
     // ------------------------------------------------------- TMA producer
     if (lane == 0 && n > 0) {
-      mbar_expect_tx(bar_kv, 2 * ROW_TILE_BYTES);
-      for (int c = 0; c < NCH; c++) {
-        tma_load_4d(smem_u32(sK) + c * 128 * 128, &tm_k, bar_kv, c * 64, h_idx / p.kv_hdiv,
-                    tile_tok0, b_idx);
-        tma_load_4d(smem_u32(sV) + c * 128 * 128, &tm_v, bar_kv, c * 64, h_idx / p.kv_hdiv,
-                    tile_tok0, b_idx);
-      }
       const int dcol = 64 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
       HeadWalk<WALK> hw;
       for (int i = 0; i < n; i++) {
@@ -264,8 +274,6 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
     const int grp = per * static_cast<int>(rank) + r / p.kvb;   // kv block of the pair
-    const int tok = tile_tok0 + r;
-    const bool row_valid = (grp < groups) && tok >= 0 && tok < p.N;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     const int cbeg = colq * 16;
     const float c = p.scale_log2;
@@ -311,7 +319,7 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
       // what the tile's columns mean to this row: worked out before the wait
       const ColSpan cs = col_span(un, i, SUB, grp, row0, G, p.N);
       const int lo = cs.lo, hi = cs.hi;
-      const bool act = row_valid && cs.on;
+      const bool act = cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
       const bool none = !fast && !__any_sync(0xffffffffu, act);
       if (!mbar_wait(bar_afull(sb), (i >> 1) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
@@ -390,36 +398,30 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
       __syncwarp();
       if (lane == 0) mbar_arrive_cta(bar_pfull(sb), 0);
     }
-    if (ok && n > 0) ok = mbar_wait(bar_final, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
+    if (ok) ok = mbar_wait(n > 0 ? bar_final : bar_kv, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
     if (ok) {
       tc_fence_after();
       // column quarters 0, 1 store dV (TMEM 256..), 2, 3 store dK (TMEM 384.., scaled)
-      const int which = colq >> 1, colhalf = colq & 1;
-      uint8_t* base = static_cast<uint8_t*>(which == 0 ? p.out1 : p.out0);
-      const int64_t sb_ = which == 0 ? p.s1_b : p.s0_b, sn_ = which == 0 ? p.s1_n : p.s0_n,
-                    sh_ = which == 0 ? p.s1_h : p.s0_h;
+      const int ew = (late_tid() >> 5) - 2;
+      const int which = ew >> 3;
       const float mul = which == 0 ? 1.f : p.scale;
-      uint8_t* orow = nullptr;
-      if (row_valid)
-        orow = base + (p.out_f32 ? 4 : 2) *
-                          (static_cast<int64_t>(b_idx) * sb_ + static_cast<int64_t>(tok) * sn_ +
-                           static_cast<int64_t>(WALK ? h_idx / p.heads : h_idx) * sh_);
-      for (int c0 = colhalf * 32; c0 < D; c0 += 64) {
+      // every copy has landed and every UMMA has retired: the tiles make room for the results
+#pragma unroll 1
+      for (int c0 = ((ew >> 2) & 1) * 32; c0 < D; c0 += 64) {
         uint32_t v[32];
         if (n > 0) {
           tmem_ld32(lane_addr + 256 + which * 128 + c0, v);
           tmem_wait_ld();
         }
-        if (row_valid) {
-          uint32_t pk[16];
+        uint32_t pk[16];
 #pragma unroll
-          for (int x = 0; x < 32; x += 2) {
-            const float a = n > 0 ? __uint_as_float(v[x]) * mul : 0.f;
-            const float b = n > 0 ? __uint_as_float(v[x + 1]) * mul : 0.f;
-            pk[x >> 1] = pack2f<FMT>(a, b);
-          }
-          store_row_part(orow, c0, p.D, pk, FMT, p.out_f32 != 0);
+        for (int x = 0; x < 32; x += 2) {
+          const float a = n > 0 ? __uint_as_float(v[x]) * mul : 0.f;
+          const float b = n > 0 ? __uint_as_float(v[x + 1]) * mul : 0.f;
+          pk[x >> 1] = pack2f<FMT>(a, b);
         }
+        store_rows(smem + ew * 2048, pk, which == 0 ? p.out1 : p.out0, s_out, which == 0 ? 1 : 0,
+                   (ew + 2) & 3, which == 0 ? p.s1_n : p.s0_n, c0, p.D, FMT, p.out_f32 != 0);
       }
     }
   }

@@ -46,6 +46,7 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
   uint8_t* sKV = smem + 2 * ROW_TILE_BYTES;
   __shared__ UnionScratch un;
   __shared__ float s_delta[128];
+  __shared__ OutTile s_out;
   __shared__ __align__(8) uint64_t bars[2 + 3 * DQ2_STAGES + 5];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
@@ -95,10 +96,14 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_relinquish2();
   }
   // both CTAs build the same union over the pair's four candidate lists
-  clear_bitmaps(un);
+  clear_flags(sKV, p.Mkv, groups);
+  tc_fence_before();
   cluster_arrive();
   pdl_wait();
   const int mine = min(per, groups - per * static_cast<int>(rank));   // q-blocks of my tile, if any
+  if (tid == 32)
+    s_out = {{static_cast<int64_t>(b_idx) * p.s0_b + static_cast<int64_t>(h_idx) * p.s0_h, 0},
+             tile_row0, min(p.N, tile_row0 + mine * p.g)};
   if (tid == 0) {   // under the building of the union
     mbar_expect_tx(bar_q, 2 * ROW_TILE_BYTES);
     for (int c = 0; c < NCH; c++) {
@@ -107,18 +112,21 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
   }
   TileDelta<D> delta;
-  delta.load(p, b_idx, h_idx, tile_row0, mine * p.g);
-  const int n = build_union(un, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
-                            p.W, nullptr, p.Mkv, SUB, p.lm, p.status);
+  float lse_mine = 0.f;   // of the row that a compute thread works on
+  if (warp >= 2) {
+    const int r = (warp & 3) * 32 + lane, qrow = tile_row0 + r;
+    if (r < mine * p.g && qrow >= 0 && qrow < p.N) lse_mine = p.lse[static_cast<int64_t>(bh) * p.N + qrow];
+    delta.load(p, b_idx, h_idx, tile_row0, mine * p.g);
+  }
+  const TileMaskRow mask_row = {
+      p.masks && mine > 0
+          ? p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + blockIdx.x) * p.mask_stride
+          : nullptr,
+      per * static_cast<int>(rank), mine};
+  const int n = build_union<BW_THREADS / 32>(
+      un, sKV, p.lists + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups, p.W, nullptr, p.Mkv,
+      SUB, p.lm, p.status, mask_row);
   pdl_launch();
-  delta.finish(p, s_delta, bh, tile_row0, mine * p.g);
-  if (p.masks && mine > 0)
-    write_tile_masks(un,
-                     p.masks + (static_cast<int64_t>(bh) * p.mask_tiles + blockIdx.x) *
-                                   p.mask_stride,
-                     p.mask_stride, per * static_cast<int>(rank), mine);
-  tc_fence_before();
-  __syncthreads();
   cluster_wait();            // barriers of both CTAs are initialised before anyone signals them
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
@@ -245,11 +253,7 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
     const uint32_t dp_addr = lane_addr + 256 + wg * 64;
     const int cbeg = colhalf * 32;
     const float c = p.scale_log2;
-    float lse2 = 0.f, dl = 0.f;
-    if (row_valid) {
-      lse2 = p.lse[static_cast<int64_t>(bh) * p.N + qrow] * 1.4426950408889634f;
-      dl = s_delta[r];
-    }
+    const float lse2 = lse_mine * 1.4426950408889634f;
     bool ok = true;
     if (n > 0 && colhalf == 0) {
       // group 0 moves the Q tile, group 1 the dO tile, from (swizzled) shared
@@ -277,6 +281,10 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
       __syncwarp();
       if (lane == 0) mbar_arrive_cta(bar_qt, 0);
     }
+    // the sums run under the first UMMAs
+    delta.finish(p, s_delta, bh, tile_row0, mine * p.g);
+    asm volatile("bar.sync 1, 512;" ::: "memory");
+    const float dl = row_valid ? s_delta[r] : 0.f;
     for (int i = wg; ok && i < n; i += 2) {
       // A(i) complete also means B(i-2) has retired (same issue order), so the
       // dS columns of this buffer are free again.
@@ -284,7 +292,7 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
       const int tok0 = static_cast<int>(un.ids[i]) * G - p.kv_pad_head;
       const ColSpan cs = col_span(un, i, SUB, grp, tok0, G, p.N);
       const int lo = cs.lo, hi = cs.hi;
-      const bool act = row_valid && cs.on;
+      const bool act = cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
       const bool none = !fast && !__any_sync(0xffffffffu, act);   // a block of the other groups: dS = 0
       if (!mbar_wait(bar_afull(wg), (i >> 1) & 1, w, FTK_DEV_TIMEOUT_CONSUMER)) {
@@ -324,31 +332,26 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
     // epilogue: 32-column chunks of the head dim dealt to the four warps of a
     // lane quarter
-    if (ok && n > 0) ok = mbar_wait(bar_final, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
+    if (ok) ok = mbar_wait(n > 0 ? bar_final : bar_q, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
     if (ok) {
       tc_fence_after();
-      uint8_t* orow = nullptr;
-      if (row_valid)
-        orow = static_cast<uint8_t*>(p.out0) +
-               (p.out_f32 ? 4 : 2) *
-                   (static_cast<int64_t>(b_idx) * p.s0_b + static_cast<int64_t>(qrow) * p.s0_n +
-                    static_cast<int64_t>(h_idx) * p.s0_h);
-      const int c0 = (wg * 2 + colhalf) * 32;
+      // every copy has landed and every UMMA has retired: the tiles make room for dQ
+      const int ew = (late_tid() >> 5) - 2;   // 32-column chunks dealt to the warps of a lane quarter
+      const int c0 = (ew >> 2) * 32;
       uint32_t v[32];
       if (n > 0) {
         tmem_ld32(lane_addr + 384 + c0, v);
         tmem_wait_ld();
       }
-      if (row_valid) {
-        uint32_t pk[16];
+      uint32_t pk[16];
 #pragma unroll
-        for (int x = 0; x < 32; x += 2) {
-          const float a = n > 0 ? __uint_as_float(v[x]) * p.scale : 0.f;
-          const float b = n > 0 ? __uint_as_float(v[x + 1]) * p.scale : 0.f;
-          pk[x >> 1] = pack2f<FMT>(a, b);
-        }
-        store_row_part(orow, c0, p.D, pk, FMT, p.out_f32 != 0);
+      for (int x = 0; x < 32; x += 2) {
+        const float a = n > 0 ? __uint_as_float(v[x]) * p.scale : 0.f;
+        const float b = n > 0 ? __uint_as_float(v[x + 1]) * p.scale : 0.f;
+        pk[x >> 1] = pack2f<FMT>(a, b);
       }
+      store_rows(smem + ew * 2048, pk, p.out0, s_out, 0, (ew + 2) & 3, p.s0_n, c0, p.D, FMT,
+                 p.out_f32 != 0);
     }
   }
   tc_fence_before();

@@ -94,6 +94,7 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
   __shared__ float s_m[2][128], s_l[2][128];
+  __shared__ OutTile s_out;
   __shared__ unsigned s_todo[(FW_THREADS + 31) / 32];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -171,8 +172,11 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     tmem_alloc(smem_u32(&tmem_base_s), 512);
     tmem_relinquish();
   }
-  clear_bitmaps(un);
-  const int n = build_union(un, p.merged + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
+  if (tid == 32)
+    s_out = {{static_cast<int64_t>(b_idx) * p.so_b + static_cast<int64_t>(h_idx) * p.so_h, 0},
+             tile_row0, min(p.N, tile_row0 + groups * p.g)};
+  clear_flags(sKV, p.Mkv, groups);
+  const int n = build_union<FW_THREADS / 32>(un, sKV, p.merged + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
                             p.W, nullptr, p.Mkv, 1, p.lm, p.status);
   tc_fence_before();
   __syncthreads();
@@ -488,35 +492,29 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       const bool have = (n > 0) && lt > 0.f;
       const float inv = have ? 1.f / lt : 0.f;
       const float wa = fa * inv, wb = fb * inv;
-      uint8_t* orow = nullptr;
-      if (row_valid)
-        orow = static_cast<uint8_t*>(p.o) +
-               (p.out_f32 ? 4 : 2) *
-                   (static_cast<int64_t>(b_idx) * p.so_b + static_cast<int64_t>(qrow) * p.so_n +
-                    static_cast<int64_t>(h_idx) * p.so_h);
       constexpr int HALF = DV / 2;
+#pragma unroll 1
       for (int c0 = grp_w * HALF; c0 < (grp_w + 1) * HALF; c0 += 32) {
         uint32_t va[32], vb[32];
         if (n > 0) tmem_ld32(lane_addr + FW_COL_O + c0, va);
         if (!SINGLE && n > 1) tmem_ld32(lane_addr + FW_COL_O + 128 + c0, vb);
         if (n > 0) tmem_wait_ld();
-        if (row_valid) {
-          uint32_t pk[16];
+        uint32_t pk[16];
 #pragma unroll
-          for (int x = 0; x < 32; x += 2) {
-            float a = 0.f, b = 0.f;
-            if (have) {
-              a = __uint_as_float(va[x]) * wa;
-              b = __uint_as_float(va[x + 1]) * wa;
-              if (!SINGLE && n > 1) {
-                a = fmaf(__uint_as_float(vb[x]), wb, a);
-                b = fmaf(__uint_as_float(vb[x + 1]), wb, b);
-              }
+        for (int x = 0; x < 32; x += 2) {
+          float a = 0.f, b = 0.f;
+          if (have) {
+            a = __uint_as_float(va[x]) * wa;
+            b = __uint_as_float(va[x + 1]) * wa;
+            if (!SINGLE && n > 1) {
+              a = fmaf(__uint_as_float(vb[x]), wb, a);
+              b = fmaf(__uint_as_float(vb[x + 1]), wb, b);
             }
-            pk[x >> 1] = pack2(a, b, p.fmt);
           }
-          store_row_part(orow, c0, p.D, pk, p.fmt, p.out_f32 != 0);
+          pk[x >> 1] = pack2(a, b, p.fmt);
         }
+        store_rows(smem + (warp - 2) * 2048, pk, p.o, s_out, 0, quarter, p.so_n, c0, p.D, p.fmt,
+                   p.out_f32 != 0);
       }
       if (row_valid && grp_w == 0)
         p.lse[static_cast<int64_t>(bh) * p.N + qrow] =
@@ -589,7 +587,9 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   int nst = std::min(FW_MAX_STAGES, std::min(168 * 1024, ring_bytes) / stage_bytes);
   if (nst < 2) return FTK_ERR_UNSUPPORTED;
   p.nstages = nst;
-  const size_t smem = 1024 + NCH * 128 * 128 + static_cast<size_t>(nst) * stage_bytes;
+  // the marks of the list union lie where the ring will be
+  const size_t smem = 1024 + NCH * 128 * 128 +
+                      std::max(static_cast<size_t>(nst) * stage_bytes, flag_bytes(p.Mkv, p.G));
   if (p.redo_in) {   // finds its tiles itself: as many CTAs as run at once
     if (int e = allow_smem<sparse_fwd_kernel<D, D, true>>(smem)) return e;
     return launch_pdl(sparse_fwd_kernel<D, D, true>, std::min(p.tiles, sm_count()), FW_THREADS, smem,

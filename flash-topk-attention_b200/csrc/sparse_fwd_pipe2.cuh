@@ -63,8 +63,9 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
   __shared__ int s_ovf;
-  __shared__ CoverTiles s_pro;
   __shared__ float s_l[FP2_GROUPS][128];
+  __shared__ float s_mref[128];
+  __shared__ OutTile s_out;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
@@ -79,7 +80,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
   const uint32_t bar_final = smem_u32(&bars[1]);
   const uint32_t bar_qt = smem_u32(&bars[2]);    // CTA 0: Q of both CTAs copied into TMEM
                                                  // (BIG: CTA 1's Q has landed)
-  const uint32_t bar_pro = smem_u32(&bars[3]);   // CTA 0: every softmax warp has its reference
+  const uint32_t bar_pro = smem_u32(&bars[3]);   // CTA 0: both CTAs' reference exponents are there
   auto bar_full = [&](int s) { return smem_u32(&bars[4 + s]); };
   auto bar_empty = [&](int s) { return smem_u32(&bars[4 + ST + s]); };
   auto bar_peer = [&](int s) { return smem_u32(&bars[4 + 2 * ST + s]); };   // CTA 0 only
@@ -93,7 +94,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
     mbar_init(bar_q, 1);
     mbar_init(bar_final, 1);
     mbar_init(bar_qt, BIG ? 1 : 8);        // the 4 copying warps of each CTA
-    mbar_init(bar_pro, 8 * FP2_GROUPS);     // the 16 softmax warps of each CTA
+    mbar_init(bar_pro, 8);                 // the 4 warps of group 0 of each CTA
     for (int s = 0; s < ST; s++) {
       mbar_init(bar_full(s), 1);
       mbar_init(bar_empty(s), 1);
@@ -112,30 +113,36 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_alloc2(smem_u32(&tmem_base_s), 512);
     tmem_relinquish2();
   }
-  clear_bitmaps(un);
+  if (tid == 32)
+    s_out = {{static_cast<int64_t>(b_idx) * p.so_b + static_cast<int64_t>(h_idx) * p.so_h, 0},
+             tile_row0, min(p.N, tile_row0 + (groups - per * static_cast<int>(rank)) * p.g)};
+  clear_flags(sKV, p.Mkv, groups);
+  tc_fence_before();
+  cluster_arrive();
   pdl_wait();
-  const int n = build_union(un, p.merged + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups,
-                            p.W, nullptr, p.Mkv, SUB, p.lm, p.status);
+  if (tid == 0) {   // under the building of the union
+    mbar_expect_tx(bar_q, Q_BYTES);
+    for (int c = 0; c < NCH; c++)
+      tma_load_4d(smem_u32(sQ) + c * 128 * 128, &tm_q, bar_q, c * 64, h_idx, tile_row0, b_idx);
+  }
+  const int n = build_union<FP2_THREADS / 32>(
+      un, sKV, p.merged + static_cast<int64_t>(bh) * p.list_rows * p.W, m0, groups, p.W, nullptr, p.Mkv,
+      SUB, p.lm, p.status);
   pdl_launch();
   // tiles whose scores give the rows their reference exponents
-  if (warp == 2) cover_tiles(un, n, groups, SUB, s_pro);
-  tc_fence_before();
-  __syncthreads();
-  cluster_sync_all();        // barriers of both CTAs are initialised before anyone signals them
+  const CoverTiles pro = cover_tiles<FMT == 0>(un, n, groups, SUB, FP2_GROUPS);
+  cluster_wait();            // barriers of both CTAs are initialised before anyone signals them
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
   WaitCtx w{&abort_flag, p.status};
 
   // prologue entry e goes through S buffer e
-  const int npro = s_pro.n;
-  auto pro_block = [&](int e) { return static_cast<int>(un.ids[s_pro.entry[e]]); };
+  const int npro = pro.n;
+  auto pro_block = [&](int e) { return static_cast<int>(un.ids[pro.entry(e)]); };
 
   if (warp == 0) {
     // ------------------------------------------------------- TMA producer
     if (lane == 0 && n > 0) {
-      mbar_expect_tx(bar_q, Q_BYTES);
-      for (int c = 0; c < NCH; c++)
-        tma_load_4d(smem_u32(sQ) + c * 128 * 128, &tm_q, bar_q, c * 64, h_idx, tile_row0, b_idx);
       // Stage rr holds K of tile rr and V of tile rr - 4; the first four, which
       // have no V, take the prologue's K tiles in its place.
       const int lead = min(n, FP2_GROUPS);
@@ -206,20 +213,28 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
         }
         umma2_commit(bar_sfull(buf), 3);
       };
+      // the reference tiles' scores, then those of the first tiles whose buffers they do
+      // not take, and the others once the references are there
       const int lead = min(n, FP2_GROUPS);
       for (int t = 0; ok && t < lead; t++) {
         const uint32_t wb[2] = {bar_full(t), bar_peer(t)};
         const uint32_t wp[2] = {0, 0};
         ok = mbar_wait_all<2>(wb, wp, w, FTK_DEV_TIMEOUT_MMA);
+        tc_fence_after();
+        if (ok && elect_one()) {
+          if (t < npro) {
+            mma_s(t * STAGE + TILE, t);
+          } else {
+            mma_s(t * STAGE, t);
+            umma2_commit(bar_empty(t), 3);
+          }
+        }
+        __syncwarp();
       }
-      tc_fence_after();
-      if (ok && elect_one())
-        for (int e = 0; e < npro; e++) mma_s(e * STAGE + TILE, e);
-      __syncwarp();
       if (ok) ok = mbar_wait(bar_pro, 0, w, FTK_DEV_TIMEOUT_MMA);
       tc_fence_after();
       if (ok && elect_one())
-        for (int t = 0; t < lead; t++) {
+        for (int t = 0; t < npro; t++) {
           mma_s(t * STAGE, t);
           umma2_commit(bar_empty(t), 3);
         }
@@ -262,8 +277,6 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
     const int grp = per * static_cast<int>(rank) + r / p.g;   // q-block of the pair (warp-uniform)
-    const int qrow = tile_row0 + r;
-    const bool row_valid = (grp < groups) && qrow >= 0 && qrow < p.N;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t s_addr = lane_addr + COL_S + gw * 64;
     const float c = p.scale_log2;
@@ -296,35 +309,32 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
 
     if (n > 0) {
-      // ---- reference exponent: scaled row maximum over the q-block's prologue tile
-      // Every warp waits for every prologue buffer, also the ones it does not
-      // read: its later parity waits on those buffers must not start while
-      // their first phase is still open.
-      const int pb = s_pro.of[grp];
-      for (int e = 0; ok && e < npro; e++)
-        ok = mbar_wait(bar_sfull(e), 0, w, FTK_DEV_TIMEOUT_CONSUMER);
-      if (ok && pb >= 0) {
-        {
-          tc_fence_after();
-          const int tok0 = pro_block(pb) * KVB - p.kv_pad_head;
-          const ColSpan cs = col_span(un, s_pro.entry[pb], SUB, grp, tok0, KVB, p.N);
-          const int lo = cs.lo, hi = cs.hi;
-          uint32_t v0[32], v1[32];
-          tmem_ld32(lane_addr + COL_S + pb * 64, v0);
-          tmem_ld32(lane_addr + COL_S + pb * 64 + 32, v1);
-          tmem_wait_ld();
-          float mx = -INFINITY;
-#pragma unroll
-          for (int x = 0; x < 32; x++) {
-            if (x >= lo && x < hi) mx = fmaxf(mx, __uint_as_float(v0[x]));
-            if (x + 32 >= lo && x + 32 < hi) mx = fmaxf(mx, __uint_as_float(v1[x]));
-          }
-          mref = (mx > -INFINITY) ? mx * c : 0.f;
-        }
+      // ---- reference exponent: scaled row maximum over the q-block's prologue tile (and
+      // the extra ones).  Group 0 works it out; behind the barrier the others may rely on
+      // the first phase of every prologue buffer being over, as their parity waits must.
+      if (gw == 0) {
+        for (int e = 0; ok && e < npro; e++)
+          ok = mbar_wait(bar_sfull(e), 0, w, FTK_DEV_TIMEOUT_CONSUMER);
+        tc_fence_after();
+        float mx = -INFINITY;
+        auto look = [&](int e) {
+          const ColSpan cs =
+              col_span(un, pro.entry(e), SUB, grp, pro_block(e) * KVB - p.kv_pad_head, KVB, p.N);
+          if (!__any_sync(0xffffffffu, cs.on)) return;
+          const float m = tmem_row_max(lane_addr + COL_S + e * 64, KVB, cs.lo, cs.hi);
+          if (cs.on) mx = fmaxf(mx, m);
+        };
+        const int pb = (pro.of >> (4 * grp)) & 15;
+        if (ok && pb != 15) look(pb);
+#pragma unroll 1
+        for (int e = pro.extra; FMT == 0 && ok && e < npro; e++) look(e);
+        s_mref[r] = (mx > -INFINITY) ? mx * c : 0.f;
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cta(bar_pro, 0);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cta(bar_pro, 0);
+      asm volatile("bar.sync 1, %0;" ::"n"(512) : "memory");
+      mref = s_mref[r];
     }
 
     const float2 c2 = make_float2(c, c);
@@ -340,11 +350,9 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
       const int tok0 = static_cast<int>(un.ids[i]) * KVB - p.kv_pad_head;
       const ColSpan cs = col_span(un, i, SUB, grp, tok0, KVB, p.N);
       const int lo = cs.lo, hi = cs.hi;
-      const bool act = row_valid && cs.on;
-      const bool any_act = __any_sync(0xffffffffu, act);
-      const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == KVB;
+      const bool fast = cs.on && lo == 0 && hi == KVB;   // the warp's rows are of one q-block
 
-      if (any_act) {
+      if (cs.on) {
         uint32_t v0[32], v1[32];
         tmem_ld32(s_addr, v0);
         tmem_ld32(s_addr + 32, v1);
@@ -374,8 +382,8 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
 #pragma unroll
           for (int x = 0; x < 32; x += 2) {
             float a0 = 0.f, a1 = 0.f;
-            if (act && x >= lo && x < hi) a0 = fast_exp2(fmaf(__uint_as_float(v0[x]), c, -mref));
-            if (act && x + 1 >= lo && x + 1 < hi)
+            if (x >= lo && x < hi) a0 = fast_exp2(fmaf(__uint_as_float(v0[x]), c, -mref));
+            if (x + 1 >= lo && x + 1 < hi)
               a1 = fast_exp2(fmaf(__uint_as_float(v0[x + 1]), c, -mref));
             acc.x += a0;
             acc.y += a1;
@@ -385,9 +393,9 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
 #pragma unroll
           for (int x = 0; x < 32; x += 2) {
             float b0 = 0.f, b1 = 0.f;
-            if (act && x + 32 >= lo && x + 32 < hi)
+            if (x + 32 >= lo && x + 32 < hi)
               b0 = fast_exp2(fmaf(__uint_as_float(v1[x]), c, -mref));
-            if (act && x + 33 >= lo && x + 33 < hi)
+            if (x + 33 >= lo && x + 33 < hi)
               b1 = fast_exp2(fmaf(__uint_as_float(v1[x + 1]), c, -mref));
             acc.x += b0;
             acc.y += b1;
@@ -414,41 +422,37 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
     // ------------------------------------------------------------ epilogue
     // row sums of the four groups add up (same reference); each group converts
     // and stores a quarter of the head dimension
-    s_l[gw][r] = l;
-    if (ovf) atomicOr(&s_ovf, 1);
+    const int ew = (late_tid() >> 5) - 2, er = ((ew + 2) & 3) * 32 + lane;   // warp, row
+    s_l[ew >> 2][er] = l;
+    const int qrow = s_out.row0 + er;
+    const bool row_valid = qrow >= 0 && qrow < s_out.last;
+    if (ovf && row_valid) atomicOr(&s_ovf, 1);
     asm volatile("bar.sync 1, 512;" ::: "memory");
-    if (ok && n > 0) ok = mbar_wait(bar_final, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
+    if (ok) ok = mbar_wait(n > 0 ? bar_final : bar_q, 0, w, FTK_DEV_TIMEOUT_EPILOGUE);
     if (ok) {
       tc_fence_after();
-      const float lt = ((s_l[0][r] + s_l[1][r]) + s_l[2][r]) + s_l[3][r];
+      const float lt = ((s_l[0][er] + s_l[1][er]) + s_l[2][er]) + s_l[3][er];
       const bool have = (n > 0) && lt > 0.f;
       const float inv = have ? 1.f / lt : 0.f;
-      uint8_t* orow = nullptr;
-      if (row_valid)
-        orow = static_cast<uint8_t*>(p.o) +
-               (p.out_f32 ? 4 : 2) *
-                   (static_cast<int64_t>(b_idx) * p.so_b + static_cast<int64_t>(qrow) * p.so_n +
-                    static_cast<int64_t>(h_idx) * p.so_h);
+      // every copy has landed and every UMMA has retired: the tiles make room for O
       constexpr int QUART = D / 4;   // 32 or 64 columns per group
-#pragma unroll
-      for (int c0 = gw * QUART; c0 < (gw + 1) * QUART; c0 += 32) {
-        uint32_t ov[32];
+#pragma unroll 1
+      for (int c0 = (ew >> 2) * QUART, x0 = 0; x0 < QUART; c0 += 32, x0 += 32) {
+        uint32_t ov[32], pk[16];
         if (n > 0) {
           tmem_ld32(lane_addr + COL_O + c0, ov);
           tmem_wait_ld();
         }
-        if (row_valid) {
-          uint32_t pk[16];
 #pragma unroll
-          for (int x = 0; x < 32; x += 2) {
-            const float a = have ? __uint_as_float(ov[x]) * inv : 0.f;
-            const float b = have ? __uint_as_float(ov[x + 1]) * inv : 0.f;
-            pk[x >> 1] = pack16<FMT>(a, b);
-          }
-          store_row_part(orow, c0, p.D, pk, FMT, p.out_f32 != 0);
+        for (int x = 0; x < 32; x += 2) {
+          const float a = have ? __uint_as_float(ov[x]) * inv : 0.f;
+          const float b = have ? __uint_as_float(ov[x + 1]) * inv : 0.f;
+          pk[x >> 1] = pack16<FMT>(a, b);
         }
+        store_rows(smem + ew * 2048, pk, p.o, s_out, 0, (ew + 2) & 3, p.so_n, c0, p.D, FMT,
+                   p.out_f32 != 0);
       }
-      if (row_valid && gw == 0)
+      if (row_valid && ew < 4)
         p.lse[static_cast<int64_t>(bh) * p.N + qrow] =
             have ? (mref + log2f(lt)) * 0.6931471805599453f : -INFINITY;
     }
@@ -461,7 +465,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
   const int unit_x = static_cast<int>(blockIdx.x >> 1) * 2 + static_cast<int>(rank);
   if (tid == 0 && p.redo_out && unit_x < units_x)
     p.redo_out[blockIdx.y * units_x + unit_x] =
-        s_ovf | (((s_pro.left >> (per * rank)) & ((1 << per) - 1)) != 0);
+        s_ovf | (((pro.left >> (per * rank)) & ((1 << per) - 1)) != 0);
   if (abort_flag)
     for (int i = 0; i < 200; i++) __nanosleep(1000);
   // neither CTA may leave (or free TMEM) while the other can still touch it

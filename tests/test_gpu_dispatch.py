@@ -320,3 +320,59 @@ def test_select_of_values_that_are_no_scores(ftk, M):
         for g, w in zip(got, want):
             np.testing.assert_array_equal(g[0, 0].cpu().numpy(), w, err_msg=f"{k} {thr} {b} {pad}")
     ftk.check_errors()
+
+
+@pytest.mark.parametrize("D,g,kvb,N,W", [
+    (64, 64, 16, 9600, 37),      # 600 blocks: more than one entry a thread of 18 warps
+    (64, 16, 64, 1000, 5),       # eight groups per tile
+    (128, 64, 64, 4200, 9),
+    (128, 32, 32, 2100, 11),     # tiles of two listed blocks
+    (128, 128, 128, 7000, 6),    # lists over blocks of twice the size
+])
+def test_lists_of_any_width(ftk, D, g, kvb, N, W):
+    """The same lists, as they are, behind one more and with a tail that lets them be read
+    16 bytes at a time: the union is the same, so are all results, bit for bit (the widths
+    are all short enough for the one-CTA kernels)."""
+    H = 2
+    t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype="bf16", seed=71, do_seed=72))
+    QM, M = -(-N // g), -(-N // kvb)
+    lists = _lists(np.random.default_rng(11), H, QM, M, W)[None]
+    pads = dict(q_padding=(0, QM * g - N), kv_padding=(0, M * kvb - N))
+    want = None
+    for width in (W, W + 1, -(-W // 4) * 4, -(-W // 4) * 4 + 4):
+        wider = np.full((1, H, QM, width), -1, np.int32)
+        wider[..., width - W if width == W + 1 else 0:][..., :W] = lists
+        got = _grads(ftk, t, wider, H, g, kvb, **pads)
+        if want is None:
+            want = got
+        for a, b in zip(got, want):
+            assert torch.equal(a, b), width
+
+
+@pytest.mark.parametrize("D,W", [(64, 16), (128, 16), (128, 3), (256, 16)])
+def test_rows_that_do_not_exist(ftk, D, W):
+    """Tiles with rows before the first and behind the last token, and with keys that are
+    infinite and listed by nobody: the rows that are listed come out as they do alone."""
+    H, N, g = 2, 960, 64
+    t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype="bf16", seed=73, do_seed=74))
+    M = N // g
+    lists = _lists(np.random.default_rng(12), H, M, M, min(W, M))[None]
+    want = _grads(ftk, t, lists, H, g, g)
+    # the same problem behind four blocks (so that the same blocks share a tile) of 40 virtual
+    # and 216 real rows, and before one that ends in 24 virtual ones
+    pre, post = 4 * g - 40, g - 24
+    n2 = pre + N + post
+    t2 = {}
+    for k, x in t.items():
+        y = torch.zeros(1, n2, H * D, dtype=x.dtype)
+        y[:, pre:pre + N] = x
+        if k == "k":
+            y[:, :pre] = float("inf")
+        t2[k] = y
+    wider = np.full((1, H, M + 5, lists.shape[-1]), -1, np.int32)
+    wider[:, :, 4:M + 4] = np.where(lists >= 0, lists + 4, -1)
+    got = _grads(ftk, t2, wider, H, g, g, q_padding=(40, 24), kv_padding=(40, 24))
+    for i in (0, 2, 3, 4):
+        assert torch.equal(got[i][:, pre:pre + N], want[i])
+        assert not got[i][:, :pre].any() and not got[i][:, pre + N:].any()
+    assert torch.equal(got[1][..., pre:pre + N], want[1])
