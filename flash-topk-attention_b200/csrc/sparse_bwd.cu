@@ -61,8 +61,7 @@ struct BwdParams {
   int span, span_tiles;      // dKV with heads > 1: q-blocks (a multiple of 32) and tiles per head
   int sub;                   // listed blocks per tile: kv blocks (dQ), q-blocks (dKV)
   const int32_t* order;      // dKV: kv blocks by fan-in, heaviest first ([BH][Mkv]) or null
-  int step;                  // dKV pair kernel at head dim 128: its STEP variant
-  const int32_t* tile_order; // dKV: 128-row kv tiles by number of q-blocks, heaviest first, or null
+  const int32_t* tile_order; // dKV: the CTAs' (pairs') tiles by number of q-blocks, heaviest first, or null
 };
 
 // ------------------------------------------------------------------- delta
@@ -647,6 +646,32 @@ struct HeadWalk {
   }
 };
 
+// The slice and the tile of launch position x of `tiles` in row blockIdx.y of the grid.
+// With an order (see fan_in_kernel) the heaviest eighth of every slice's tiles comes first,
+// those of all slices in turn, then the rest slice by slice, whose rows of Q and dO stay in
+// L2 that way: sorted within the slices only, the last slice's heaviest tiles start late.
+struct KvTile {
+  int slice, tile;
+};
+__device__ __forceinline__ KvTile kv_tile(const BwdParams& p, int x, int tiles) {
+  KvTile t = {static_cast<int>(blockIdx.y), x};
+  if (p.tile_order) {
+    const int slices = gridDim.y, lead = (tiles + 7) >> 3, at = blockIdx.y * tiles + x;
+    int rank;
+    if (at < lead * slices) {
+      rank = at / slices;
+      t.slice = at - rank * slices;
+    } else {
+      const int rest = at - lead * slices;
+      t.slice = rest / (tiles - lead);
+      rank = lead + rest - t.slice * (tiles - lead);
+    }
+    pdl_wait();
+    t.tile = p.tile_order[static_cast<int64_t>(t.slice) * tiles + rank];
+  }
+  return t;
+}
+
 // TMEM columns: S^T[2] 0/64 (P^T written over their first half), dP^T[2]
 // 128/192 (dS^T likewise), dV 256.., dK 384..
 // Head dim 64: K (320..351) and V (352..383) are copied into TMEM as well, so that the
@@ -684,13 +709,10 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
   __shared__ __align__(16) float s_lse2[2][2][128], s_delta[2][2][128];  // [group][parity][q row]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int bh = blockIdx.y;
-  int j0 = blockIdx.x * p.G;                // first kv block of the tile
-  if (p.tile_order) {
-    // heaviest tiles first, see fan_in_kernel
-    pdl_wait();
-    j0 = p.tile_order[static_cast<int64_t>(bh) * gridDim.x + blockIdx.x] * p.G;
-  } else if (p.order) {
+  const KvTile at = kv_tile(p, blockIdx.x, gridDim.x);
+  const int bh = at.slice;
+  int j0 = at.tile * p.G;                   // first kv block of the tile
+  if (p.order && !p.tile_order) {
     // The same from a reverse index, which orders kv blocks: the grid has one CTA
     // per kv block, in the order of `order` (fan-in descending, ties by lower id);
     // the CTA whose block is the first of its tile in that order does the tile,
@@ -1082,10 +1104,10 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
 namespace ftk {
 
 // ---------------------------------------------------- order of the dK/dV tiles
-// Per slice: q-blocks that each 128-row kv tile has to walk, from the dQ
-// kernel's tile masks, and the tiles sorted by that number, largest first (ties:
-// lower tile).  With skewed lists a few tiles take many times the others' time;
-// issued last they would run alone.  One CTA per slice, key = (count + 1, ~tile).
+// Per slice: q-blocks that each kv tile (128 rows, or the 256 of a pair of CTAs: G kv
+// blocks) has to walk, from the dQ kernel's tile masks, and the tiles sorted by that
+// number, largest first (ties: lower tile).  With skewed lists a few tiles take many times
+// the others' time; issued last they would run alone.  One CTA per slice, key = (count + 1, ~tile).
 constexpr int FAN_THREADS = 1024;
 
 __global__ void __launch_bounds__(FAN_THREADS)
@@ -1208,12 +1230,18 @@ struct BwdPlan {
   bool pair_dq, pair_dkv;    // kernels on pairs of SMs
   bool walk;                 // dK/dV: one CTA walks all query heads of its kv head
   int tiles, stride, span;   // tile masks (see TileMaskRow)
-  int kv_tiles;              // 128-row kv tiles per slice
+  int kv_tiles;              // kv tiles of a CTA (or a pair) per slice
+  int tile_blocks;           // kv blocks of such a tile
   bool order;                // dK/dV tiles sorted by the work they have
   size_t off_masks, off_order, off_dk, off_dv, bytes;
 };
 
 static size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
+
+static bool env_off(const char* name) {
+  const char* e = getenv(name);
+  return e && e[0] == '0';
+}
 
 static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
   BwdPlan b{};
@@ -1232,26 +1260,30 @@ static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
   b.tiles = (gr.QM + per - 1) / per;
   b.stride = flag_blocks(gr.Mkv);
   b.span = (b.tiles * per + 31) & ~31;
-  b.kv_tiles = (gr.Mkv + G - 1) / G;
-  // Pairs walk the union of four lists.  For dQ the line is that of ftk_attn_fwd
-  // (f = 1/4 there: 451 us in pairs, 388 without); dK / dV gains more from them (its
-  // S^T and dP^T UMMAs read both operands from shared memory) and breaks even at
-  // f = 1/4 (585 against 597 us).  At head dim 256 the pair kernels are several times
-  // the faster per tile.
+  // Pairs walk the union of four lists.  The line is that of ftk_attn_fwd (f = 1/4 there:
+  // dQ 451 us in pairs, 388 without).  A tile of dK / dV takes 0.82 of the time in pairs
+  // (its S^T and dP^T UMMAs read both operands from shared memory), which independent
+  // lists outweigh up to f = 0.55 (f = 1/4, four heads per kv head, tiles in order of
+  // their work: 510 us in pairs, 393 without).  At head dim 256 the pair kernels are
+  // several times the faster per tile.
   b.pair_dq = tiles64 && (gr.kd == 256 || (gr.kd == 128 && 2 * gr.width >= gr.Mkv));
-  b.pair_dkv = tiles64 && (gr.kd == 256 || (gr.kd == 128 && 4 * gr.width >= gr.Mkv));
+  b.pair_dkv = b.pair_dq && (gr.kd == 256 || !env_off("FTK_DKV_2CTA"));
   // Query heads that share a kv head: walked one after the other by the CTA that
   // owns the kv rows, so that their sum stays in its fp32 accumulators, unless
   // that leaves SMs idle: waves of CTAs times heads per CTA against waves of one
   // CTA per head, with a quarter's lead for the per-head results that are then
   // neither written nor read again.
-  const int64_t grp = a.H / a.Hkv, ctas = a.B * a.Hkv * b.kv_tiles, sms = sm_count();
+  const int64_t grp = a.H / a.Hkv, ctas = a.B * a.Hkv * ((gr.Mkv + G - 1) / G), sms = sm_count();
   auto waves = [&](int64_t n) { return (n + sms - 1) / sms; };
   b.walk = grp > 1 && grp * b.span <= AT_MAX_BLOCKS &&
            4 * grp * waves(ctas) <= 5 * waves(ctas * grp);
   const int64_t slices = b.walk ? a.B * a.Hkv : BH;
-  // sorting pays once the tiles come in several waves
-  b.order = !b.pair_dkv && slices * b.kv_tiles >= 2 * sms;
+  // sorting pays once the tiles come in several waves; lists that can cover most blocks
+  // give all tiles as much to do
+  b.tile_blocks = b.pair_dkv ? 2 * G : G;
+  b.kv_tiles = (gr.Mkv + b.tile_blocks - 1) / b.tile_blocks;
+  b.order = b.pair_dkv ? 2 * gr.width < gr.Mkv && 2 * slices * b.kv_tiles >= 2 * sms
+                       : slices * b.kv_tiles >= 2 * sms;
   size_t off = up256(static_cast<size_t>(BH) * a.N * 4);   // delta
   b.off_masks = off;
   off += up256(static_cast<size_t>(BH) * b.tiles * b.stride);
@@ -1266,11 +1298,6 @@ static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
   b.bytes = off;
   *out = b;
   return FTK_OK;
-}
-
-static bool env_off(const char* name) {
-  const char* e = getenv(name);
-  return e && e[0] == '0';
 }
 
 static BwdParams bwd_params(const ftk_attn& a, const AttnGrid& gr, const float* lse, float* delta,
@@ -1395,7 +1422,7 @@ static int launch_dkv(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, 
   if ((e = tmap_of(&tq, a, q, p.g)) || (e = tmap_of(&tdo, a, dout, p.g)) ||
       (e = tmap_of(&tk, a, k, 128)) || (e = tmap_of(&tv, a, v, 128)))
     return e;
-  if (pair && (kd == 256 || !env_off("FTK_DKV_2CTA"))) {
+  if (pair) {
     CUtensorMap tq32, tdo32;
     if ((e = tmap_of(&tq32, a, q, 32)) || (e = tmap_of(&tdo32, a, dout, 32))) return e;
     const dim3 grid(2 * ((p.Mkv + 2 * p.G - 1) / (2 * p.G)), slices);
@@ -1417,8 +1444,7 @@ static int launch_dkv(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, 
                       1024 + 2 * B6_ROWS + static_cast<size_t>(DQ6_SLOTS) * B6_PIECE);
           }
           const size_t smem = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DK2_STAGES) * 32768;
-          return p.step ? go(Kernel<sparse_bwd_dkv2_kernel<F, W, true, S>>{}, smem)
-                        : go(Kernel<sparse_bwd_dkv2_kernel<F, W, false, S>>{}, smem);
+          return go(Kernel<sparse_bwd_dkv2_kernel<F, W, S>>{}, smem);
         });
       });
     });
@@ -1530,7 +1556,6 @@ extern "C" int ftk_attn_bwd_dkv(const ftk_attn* a, const void* dout, int64_t sdo
   p.mask_g = attn_groups(b.gr.g);
   p.span = b.span;
   p.heads = b.walk ? p.kv_hdiv : 1;
-  p.step = 2 * b.gr.width >= b.gr.Mkv;   // lists that can cover most blocks
   const bool parts = p.kv_hdiv > 1 && !b.walk;
   if (parts) {   // one 16-bit result per query head first
     const int64_t row = a->H * a->D;
@@ -1561,7 +1586,7 @@ extern "C" int ftk_attn_bwd_dkv(const ftk_attn* a, const void* dout, int64_t sdo
                      st, p.masks, b.stride, b.tiles,
                      static_cast<int64_t>(b.tiles) * b.stride, p.heads,
                      static_cast<int>(a->H / p.heads), static_cast<int>(a->H),
-                     attn_groups(b.gr.kvb), b.kv_tiles, colsp, order);
+                     b.tile_blocks, b.kv_tiles, colsp, order);
     if (e) return e;
     p.tile_order = order;
   }
@@ -1654,10 +1679,10 @@ extern "C" int ftk_sparse_bwd_dkv(
   p.s1_n = sdv_n;
   p.s1_h = sdv_h;
   const bool pair = D == 128 && q_block_size == 64 && kv_block_size == 64 &&
-                    (fwd_list_width <= 0 || 4 * static_cast<int64_t>(fwd_list_width) >= M);
-  p.step = fwd_list_width <= 0 || 2 * static_cast<int64_t>(fwd_list_width) >= M;
+                    (fwd_list_width <= 0 || 2 * static_cast<int64_t>(fwd_list_width) >= M) &&
+                    !env_off("FTK_DKV_2CTA");
   // one-CTA kernels: tiles in order of fan-in when the caller brings the order
-  if (!pair || env_off("FTK_DKV_2CTA"))
+  if (!pair)
     p.order = sorted_kv && !env_off("FTK_DKV_ORDER") ? sorted_kv : nullptr;
   return launch_dkv(a, Rows{dout, H, sdo_b, sdo_n, sdo_h}, p, gr.kd, pair,
                     static_cast<cudaStream_t>(stream));

@@ -411,8 +411,9 @@ sparse_bwd_dkv256_kernel(const __grid_constant__ CUtensorMap tm_q,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
   const int per = 128 / p.kvb;               // kv blocks (of 64 or 32 rows) per CTA
-  const int j0 = (blockIdx.x >> 1) * 2 * per;   // first of the pair's kv blocks
-  const int bh = blockIdx.y;
+  const KvTile at = kv_tile(p, blockIdx.x >> 1, gridDim.x >> 1);
+  const int j0 = at.tile * 2 * per;          // first of the pair's kv blocks
+  const int bh = at.slice;
   const int slices = WALK ? p.H / p.heads : p.H;
   const int b_idx = bh / slices, h_idx = (bh - b_idx * slices) * (WALK ? p.heads : 1);
   const int bhq = WALK ? b_idx * p.H + h_idx : bh;

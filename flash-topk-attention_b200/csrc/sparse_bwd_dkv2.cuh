@@ -45,12 +45,10 @@ __device__ __forceinline__ uint32_t pack2f(float a, float b) {
 // other.  A template parameter because the compute warps set this kernel's pace:
 // the head bookkeeping of WALK in every build took 28.3 -> 34.6 ms at N = 32768,
 // H = 32.
-// STEP: the compute warps of a CTA go from tile to tile together (a barrier per
-// tile).  With full lists tile i then comes out of all warps ahead of tile i + 1 and
-// its buffer is free earlier (28.8 against 29.1 ms there, 3.76 against 3.98 ms at B = 4,
-// N = 8192, H = 16); with short lists most warps of a tile have nothing to do and
-// should run ahead (610 -> 589 us at W = 16 of 64 blocks, four heads per kv head).
-template <int FMT, bool WALK, bool STEP, int SUB>
+// The compute warps of a CTA go from tile to tile together (a barrier per tile): tile i
+// then comes out of all warps ahead of tile i + 1 and its buffer is free earlier (28.8
+// against 29.1 ms there, 3.76 against 3.98 ms at B = 4, N = 8192, H = 16).
+template <int FMT, bool WALK, int SUB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(BW_THREADS, 1)
 sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
                        const __grid_constant__ CUtensorMap tm_do,
@@ -75,15 +73,14 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
   __shared__ uint32_t tmem_base_s;
   __shared__ OutTile s_out;
   __shared__ int abort_flag;
-  // per compute warp and parity: lse, then delta, of the warp's 16 q columns (STEP:
-  // per parity, of all 64)
-  __shared__ __align__(16) float s_cols[16][2][32];
+  __shared__ __align__(16) float s_cols[2][128];   // per parity: lse, then delta, of the 64 q columns
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
   const int per = 128 / p.kvb;               // kv blocks (of 64 or 32 rows) per CTA
-  const int j0 = (blockIdx.x >> 1) * 2 * per;   // first of the pair's kv blocks
-  const int bh = blockIdx.y;
+  const KvTile at = kv_tile(p, blockIdx.x >> 1, gridDim.x >> 1);
+  const int j0 = at.tile * 2 * per;          // first of the pair's kv blocks
+  const int bh = at.slice;
   // slice = (batch, first of the query heads this pair walks)
   const int slices = WALK ? p.H / p.heads : p.H;
   const int b_idx = bh / slices, h_idx = (bh - b_idx * slices) * (WALK ? p.heads : 1);
@@ -281,20 +278,18 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     // lse / delta of a q-block are fetched from global memory one round ahead
     // (into registers, while the previous tile is being worked on) and only
     // then staged in shared memory, negated: the packed fma / add take them as
-    // they are.  STEP: staged once per CTA, behind a barrier of all compute warps.
-    // Otherwise every warp stages the 32 values that it needs itself.
+    // they are.  Staged once per CTA, behind a barrier of all compute warps.
     HeadWalk<WALK> hw, hw_mine;
-    const int ct = STEP ? tid - 64 : lane;            // column (and, without STEP, kind) fetched
-    const int col = STEP ? ct : cbeg + (lane & 15);
+    const int ct = tid - 64;            // the column fetched, if there is one
     auto fetch = [&](int i, float& l2, float& dl) {
       l2 = 0.f;
       dl = 0.f;
-      if ((!STEP || ct < G) && i < n) {
-        const int t = hw.at(un.ids[i], p) * G - p.q_pad_head + col;
+      if (ct < G && i < n) {
+        const int t = hw.at(un.ids[i], p) * G - p.q_pad_head + ct;
         if (t >= 0 && t < p.N) {
           const int64_t e = static_cast<int64_t>(bhq + hw.head) * p.N + t;
-          if (STEP || lane < 16) l2 = -p.lse[e] * 1.4426950408889634f;
-          if (STEP || lane >= 16) dl = -p.delta[e];
+          l2 = -p.lse[e] * 1.4426950408889634f;
+          dl = -p.delta[e];
         }
       }
     };
@@ -303,17 +298,12 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     for (int i = 0; i < n; i++) {
       const int sb = i & 1;                  // S^T / dP^T buffer, and lse / delta buffer
       const int row0 = hw_mine.at(un.ids[i], p) * G - p.q_pad_head;
-      float* cols = STEP ? &s_cols[0][0][0] + sb * 128 : s_cols[cw][sb];
-      if (STEP) {
-        if (ct < G) {
-          cols[ct] = l2_next;
-          cols[64 + ct] = dl_next;
-        }
-        asm volatile("bar.sync 1, 512;" ::: "memory");
-      } else {
-        cols[lane] = lane < 16 ? l2_next : dl_next;
-        __syncwarp();
+      float* cols = s_cols[sb];
+      if (ct < G) {
+        cols[ct] = l2_next;
+        cols[64 + ct] = dl_next;
       }
+      asm volatile("bar.sync 1, 512;" ::: "memory");
       fetch(i + 1, l2_next, dl_next);
       if (!ok) continue;
       // what the tile's columns mean to this row: worked out before the wait
@@ -329,8 +319,8 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
       tc_fence_after();
       const uint32_t st_addr = lane_addr + sb * 64;         // S^T, then P^T
       const uint32_t dp_addr = lane_addr + 128 + sb * 64;   // dP^T, then dS^T
-      const float4* l4 = reinterpret_cast<const float4*>(cols + (STEP ? cbeg : 0));
-      const float4* d4 = reinterpret_cast<const float4*>(cols + (STEP ? 64 + cbeg : 16));
+      const float4* l4 = reinterpret_cast<const float4*>(cols + cbeg);
+      const float4* d4 = reinterpret_cast<const float4*>(cols + 64 + cbeg);
       // P^T / dS^T of the thread's 16 columns go over the first 8 of them in
       // the S^T / dP^T regions: columns this thread has already read.
       // full tiles: two columns per instruction (fma.f32x2, add.f32x2,

@@ -376,3 +376,24 @@ def test_rows_that_do_not_exist(ftk, D, W):
         assert torch.equal(got[i][:, pre:pre + N], want[i])
         assert not got[i][:, :pre].any() and not got[i][:, pre + N:].any()
     assert torch.equal(got[1][..., pre:pre + N], want[1])
+
+
+@pytest.mark.parametrize("H,g,kvb,groups", [(16, 64, 64, 1), (16, 32, 32, 2)])
+def test_dkv_pair_order(ftk, monkeypatch, H, g, kvb, groups):
+    """Short lists at head dim 256: the tiles of the pairs of SMs are sorted by the work they
+    have, the heaviest of all slices first, which changes when a tile runs and nothing else."""
+    B, N, D = 2, 2600, 256
+    tail_q, tail_k = -N % g, -N % kvb
+    t = cases.make_inputs(dict(B=B, N=N, H=H, D=D, dtype="bf16", seed=8, do_seed=9))
+    Hkv = H // groups
+    for n in "kv":
+        t[n] = t[n].view(B, N, H, D)[:, :, :Hkv].reshape(B, N, Hkv * D).clone()
+    QM, M = (N + tail_q) // g, (N + tail_k) // kvb
+    merged = _lists(np.random.default_rng(4), B * H, QM, M, 6).reshape(B, H, QM, 6)
+    merged[..., 0] = np.where((merged == 1).any(-1), merged[..., 0], 1)   # a block that everybody reads
+    kw = dict(q_padding=(0, tail_q), kv_padding=(0, tail_k), num_kv_heads=Hkv)
+    sorted_ = _grads(ftk, t, merged, H, g, kvb, **kw)
+    monkeypatch.setenv("FTK_DKV_ORDER", "0")
+    plain = _grads(ftk, t, merged, H, g, kvb, **kw)
+    for a, b in zip(sorted_, plain):
+        assert torch.equal(a, b)
