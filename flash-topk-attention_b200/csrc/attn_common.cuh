@@ -401,31 +401,6 @@ __device__ __forceinline__ CoverTiles cover_tiles(const UnionScratch& u, int n, 
   return c;
 }
 
-// The maximum of columns [lo, hi) of `cols` (a multiple of 16) columns of this thread's
-// row in TMEM.  A warp calls this together, with the same lo, hi and cols.  (As straight
-// code over 64 columns with two comparisons each it took 2500 cycles.)
-__device__ __forceinline__ float tmem_row_max(uint32_t addr, int cols, int lo, int hi) {
-  float mx = -INFINITY;
-  const unsigned width = max(hi - lo, 0);
-#pragma unroll 1
-  for (int c0 = 0; c0 < cols; c0 += 16) {
-    uint32_t v[16];
-    tmem_ld16(addr + c0, v);
-    tmem_wait_ld();
-    float m[2] = {-INFINITY, -INFINITY};
-    if (c0 >= lo && c0 + 16 <= hi) {
-#pragma unroll
-      for (int x = 0; x < 16; x++) m[x & 1] = fmaxf(m[x & 1], __uint_as_float(v[x]));
-    } else {
-#pragma unroll
-      for (int x = 0; x < 16; x++)
-        if (static_cast<unsigned>(c0 + x - lo) < width) m[x & 1] = fmaxf(m[x & 1], __uint_as_float(v[x]));
-    }
-    mx = fmaxf(mx, fmaxf(m[0], m[1]));
-  }
-  return mx;
-}
-
 // Where a CTA's results go: worked out by one thread ahead of the loop over the tiles and
 // kept in shared memory until the end of it, where a warp also asks for its number anew.
 // Held in registers all along, they cost the loop's warps, which have 96, a few percent.

@@ -115,7 +115,7 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sQ = smem;
   uint8_t* sK = smem + Q_BYTES;
-  __shared__ __align__(8) uint64_t bars[1 + 2 * SC_STAGES + 8 + 1];
+  __shared__ __align__(8) uint64_t bars[1 + 2 * SC_STAGES + 8 + 2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
   __shared__ int s_redo, s_stop;
@@ -130,7 +130,7 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
   const int bh = p.bh_begin + bh_local;
   const int b_idx = bh / p.H, h_idx = bh - b_idx * p.H;
 
-  const uint32_t bar_q = smem_u32(&bars[0]);
+  const uint32_t bar_q = smem_u32(&bars[0]);     // rows 0 .. 127 of Q
   auto bar_kfull = [&](int s) { return smem_u32(&bars[1 + s]); };
   auto bar_kempty = [&](int s) { return smem_u32(&bars[1 + SC_STAGES + s]); };
   // one full / empty pair per accumulator (stage s, row half h): the four
@@ -141,11 +141,13 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
     return smem_u32(&bars[1 + 2 * SC_STAGES + 4 + s * 2 + h]);
   };
   const uint32_t bar_mref = smem_u32(&bars[1 + 2 * SC_STAGES + 8]);
+  const uint32_t bar_q1 = smem_u32(&bars[1 + 2 * SC_STAGES + 9]);   // rows 128 .. 255
 
   if (tid == 0) {
     abort_flag = 0;
     s_redo = s_stop = 0;
     mbar_init(bar_q, 1);
+    mbar_init(bar_q1, 1);
     for (int s = 0; s < SC_STAGES; s++) {
       mbar_init(bar_kfull(s), 1);
       mbar_init(bar_kempty(s), 1);
@@ -193,13 +195,14 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
   if (warp == 0) {
     // ------------------------------------------------------- TMA producer
     if (lane == 0) {
-      if (pass == 0) {
-        mbar_expect_tx(bar_q, Q_BYTES);
-        for (int half = 0; half < 2; half++)
-          for (int c = 0; c < NCH; c++)
-            tma_load_4d(smem_u32(sQ) + (half * NCH + c) * SC_CHUNK_BYTES, &tm_q, bar_q, c * 64,
-                        h_idx, q0 + half * 128, b_idx);
-      }
+      // the first scores need half of Q and a key tile: those travel first
+      auto load_q = [&](int half, uint32_t bar) {
+        mbar_expect_tx(bar, Q_BYTES / 2);
+        for (int c = 0; c < NCH; c++)
+          tma_load_4d(smem_u32(sQ) + (half * NCH + c) * SC_CHUNK_BYTES, &tm_q, bar, c * 64, h_idx,
+                      q0 + half * 128, b_idx);
+      };
+      if (pass == 0) load_q(0, bar_q);
       const uint32_t tile_bytes = static_cast<uint32_t>(p.tile_rows) * 128u * NCHS;
       const int u0 = (done0 + done1) * KSPLIT;
       for (int u = 0; u < T * KSPLIT; u++) {
@@ -212,6 +215,7 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
         for (int c = 0; c < NCHS; c++)
           tma_load_4d(smem_u32(sK) + s * K_STAGE_BYTES + c * SC_CHUNK_BYTES, &tm_k, bar_kfull(s),
                       (part * NCHS + c) * 64, h_idx, ti.row0, b_idx);
+        if (pass == 0 && u == KSPLIT - 1) load_q(1, bar_q1);
       }
     }
   } else if (warp == 1) {
@@ -244,23 +248,30 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
             tc_fence_after();
           }
           const uint64_t kdesc = desc_advance(kdesc0, s * K_STAGE_BYTES);
-          if (elect_one()) {
+          auto issue = [&](int half) {   // elected lane only
+            const uint32_t d_tmem = tmem + static_cast<uint32_t>((a * 2 + half) * SC_KT);
+            const uint64_t qdesc = desc_advance(qdesc0, (half * NCH + part * NCHS) * SC_CHUNK_BYTES);
 #pragma unroll
-            for (int half = 0; half < 2; half++) {
-              const uint32_t d_tmem = tmem + static_cast<uint32_t>((a * 2 + half) * SC_KT);
-              const uint64_t qdesc =
-                  desc_advance(qdesc0, (half * NCH + part * NCHS) * SC_CHUNK_BYTES);
-#pragma unroll
-              for (int ks = 0; ks < D / KSPLIT / 16; ks++) {
-                const uint32_t off = (ks / 4) * SC_CHUNK_BYTES + (ks % 4) * 32;
-                umma_ss(d_tmem, desc_advance(qdesc, off), desc_advance(kdesc, off), idesc,
-                        part > 0 || ks > 0);
-              }
-              if (half == 1) umma_commit(bar_kempty(s));  // smem stage reusable once retired
-              // this accumulator is readable
-              if (part == KSPLIT - 1) umma_commit(bar_afull(a, half));
+            for (int ks = 0; ks < D / KSPLIT / 16; ks++) {
+              const uint32_t off = (ks / 4) * SC_CHUNK_BYTES + (ks % 4) * 32;
+              umma_ss(d_tmem, desc_advance(qdesc, off), desc_advance(kdesc, off), idesc,
+                      part > 0 || ks > 0);
             }
+            if (half == 1) umma_commit(bar_kempty(s));  // smem stage reusable once retired
+            // this accumulator is readable
+            if (part == KSPLIT - 1) umma_commit(bar_afull(a, half));
+          };
+          if (part == 0 && t == 0 && pass == 0) {   // the other half of Q may still be on its way
+            if (elect_one()) issue(0);
+            __syncwarp();
+            ok = mbar_wait(bar_q1, 0, w, FTK_DEV_TIMEOUT_MMA);
+            tc_fence_after();
+            if (ok && elect_one()) issue(1);
+          } else if (elect_one()) {
+            issue(0);
+            issue(1);
           }
+          if (!ok) break;
           __syncwarp();
         }
       }
@@ -299,17 +310,7 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
           tc_fence_after();
           const TileInfo ti = tile_info(p, 0);
           const int lo = max(0, -ti.row0), hi = min(ti.used, p.N - ti.row0);
-          float mx = -INFINITY;
-          for (int c0 = 0; c0 < ti.used; c0 += 32) {
-            uint32_t r[32];
-            tmem_ld32(lane_addr + static_cast<uint32_t>(half * SC_KT + c0), r);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; i++) {
-              const int col = c0 + i;
-              if (col >= lo && col < hi) mx = fmaxf(mx, __uint_as_float(r[i]));
-            }
-          }
+          const float mx = tmem_row_max(lane_addr + static_cast<uint32_t>(half * SC_KT), ti.used, lo, hi);
           mref = ceilf(mx * c);
           if (!(fabsf(mref) < 1e30f)) mref = 0.f;
           if (pre) {   // not one of my tiles: hand the accumulator back
@@ -346,21 +347,22 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
       const uint32_t acc_addr = lane_addr + static_cast<uint32_t>((a * 2 + half) * SC_KT);
       // one 32-column chunk: two 16-column halves, block sums flushed on the
       // 16-column grid (block sizes are multiples of 16)
-      auto process = [&](const uint32_t (&r)[32], int c0) {
+      auto process = [&](const uint32_t (&r)[32], int c0, auto all) {
+        constexpr bool ALL = decltype(all)::value;   // every column is a key of a score block
 #pragma unroll
         for (int hc = 0; hc < 2; hc++) {
           const int cb = c0 + hc * 16;
-          if (cb < ti.used) {
+          if (ALL || cb < ti.used) {
             if (pass == 1) {
 #pragma unroll
               for (int i = 0; i < 16; i++) {
                 const int col = cb + i;
-                if (full || (col >= lo && col < hi))
+                if (ALL || (col >= lo && col < hi))
                   run_max = fmaxf(run_max, __uint_as_float(r[hc * 16 + i]));
               }
             } else {
               float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-              if (full) {
+              if (ALL || (cb >= lo && cb + 16 <= hi)) {
                 // two columns per instruction for the scaling (fma.f32x2) and for the
                 // running sums (add.f32x2): 2 issue slots per logit instead of 3; the four
                 // partial sums are the same additions in the same order as scalar code
@@ -408,29 +410,29 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_aempty(a, half));
       };
-      if (ti.used == SC_KT) {
+      if (full && ti.used == SC_KT) {
         // full tile: the load of chunk k+1 is in flight while chunk k is summed
         uint32_t ra[32], rb[32];
         tmem_ld32(acc_addr, ra);
         tmem_wait_ld();
         tmem_ld32(acc_addr + 32, rb);
-        process(ra, 0);
+        process(ra, 0, std::true_type{});
         tmem_wait_ld();
         tmem_ld32(acc_addr + 64, ra);
-        process(rb, 32);
+        process(rb, 32, std::true_type{});
         tmem_wait_ld();
         tmem_ld32(acc_addr + 96, rb);
-        process(ra, 64);
+        process(ra, 64, std::true_type{});
         tmem_wait_ld();
         release();
-        process(rb, 96);
+        process(rb, 96, std::true_type{});
       } else {
         for (int c0 = 0; c0 < ti.used; c0 += 32) {
           uint32_t r[32];
           tmem_ld32(acc_addr + static_cast<uint32_t>(c0), r);
           tmem_wait_ld();
           if (c0 + 32 >= ti.used) release();
-          process(r, c0);
+          process(r, c0, std::false_type{});
         }
       }
     }
