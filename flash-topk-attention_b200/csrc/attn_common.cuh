@@ -19,7 +19,6 @@ struct UnionScratch {
   uint16_t ids[AT_MAX_BLOCKS];                 // union, ascending
   __align__(4) uint8_t masks[AT_MAX_BLOCKS];   // bit g set: group g lists the block
   int warp_tot[32];
-  int top, top_pos;                            // first group's first block, and its place in the union
 };
 
 // The tiles that a CTA walks are `sub` listed blocks wide, 1 or 2: blocks of 32 rows
@@ -118,7 +117,6 @@ __device__ __forceinline__ int list_entries(UnionScratch& u, const ListRun& run,
   const int t = lane < WARPS ? u.warp_tot[lane] : 0;
   const int total = __reduce_add_sync(0xffffffffu, t);
   int pos = __reduce_add_sync(0xffffffffu, lane < warp ? t : 0);
-  const int top = u.top;
   unsigned m = run.mask;
   int x = run.base;
 #pragma unroll 1
@@ -129,7 +127,6 @@ __device__ __forceinline__ int list_entries(UnionScratch& u, const ListRun& run,
       u.ids[at] = static_cast<uint16_t>(x);
       if (sub == 1) u.masks[at] = static_cast<uint8_t>(m);
       else *reinterpret_cast<uint16_t*>(&u.masks[2 * at]) = static_cast<uint16_t>(m);
-      if (x == top) u.top_pos = at;
     }
     if (++r >= run.rounds) break;
     pos += __popc(b);
@@ -181,7 +178,6 @@ __device__ __forceinline__ int build_union(UnionScratch& u, uint8_t* flags, cons
       }
     }
   };
-  int top = -1;
   if (!counts && (width & 3) == 0 && (reinterpret_cast<uintptr_t>(lists) & 15) == 0) {
     // lists are mostly -1 behind a prefix and wide (up to q block x topk): 16-byte
     // loads, four groups' in flight together and across the barrier behind the clearing
@@ -199,7 +195,6 @@ __device__ __forceinline__ int build_union(UnionScratch& u, uint8_t* flags, cons
           t[x] = g0 + x < groups && e < quads ? reinterpret_cast<const int4*>(row(g0 + x))[e]
                                               : make_int4(-1, -1, -1, -1);
         if (!cleared) {
-          top = t[0].x;
           __syncthreads();
           cleared = true;
         }
@@ -227,7 +222,6 @@ __device__ __forceinline__ int build_union(UnionScratch& u, uint8_t* flags, cons
     }
     bad = lm.kv_shift == 0 && largest >= num_blocks;
   } else {
-    if (tid == 0) top = counts && counts[0] <= 0 ? -1 : row(0)[0];
     __syncthreads();
 #pragma unroll 1
     for (int g = 0; g < groups; g++) {
@@ -238,11 +232,6 @@ __device__ __forceinline__ int build_union(UnionScratch& u, uint8_t* flags, cons
     }
   }
   if (bad && status) atomicCAS(status, 0, FTK_DEV_BAD_INDEX);
-  if (tid == 0) {
-    if (top >= 0 && lm.kv_shift > 0) top = max((min(top, AT_MAX_BLOCKS) << lm.kv_shift) - lm.kv_off, 0);
-    u.top = sub == 2 && top >= 0 ? top >> 1 : top;
-    u.top_pos = -1;
-  }
   __syncthreads();
   auto one = [&](int x) -> unsigned {
     const uint8_t* f = flags + (x << shift);
@@ -307,7 +296,6 @@ __device__ __forceinline__ int build_union_masks(UnionScratch& u, const uint8_t*
     return sub == 1 ? bits(bit) : bits(bit) | bits(bit + 1) << 8;
   };
   const int n = (heads * span) >> (sub - 1);
-  if (threadIdx.x == 0) u.top = -1;
   const ListRun run = count_entries<WARPS>(u, n, mask_of);
   __syncthreads();
   const int total = list_entries<WARPS>(u, run, n, sub, mask_of);
@@ -321,28 +309,22 @@ __device__ __forceinline__ int build_union_masks(UnionScratch& u, const uint8_t*
 // the others list, and so on, ties to the first.  With wide lists one tile serves all
 // groups.  Every warp works this out for itself: by one warp, behind a barrier for the
 // others, it took 800 cycles.
-// EXTRA: where there is room, the tile that the first group names first as well, and one
-// from the union at large.  Lists that the merge made are in order of score, so the logits
-// of the former are the likeliest to be far above the others' (or, in a row that looks the
-// other way, below them), and with both the reference of an fp16 row, which a later logit
-// may exceed by 2^16 only, is hardly ever left behind (skewed scores, N = 15000, H = 16: a
-// few tiles of 1888 went to the exact kernel, which took 380 us of 3370 for them).
+// The union and its masks decide, not the order in which a list names its blocks: results
+// do not depend on how a list is written.
 struct CoverTiles {
   int n;                // tiles
   int e0, e1, e2, e3;   // their positions in the union
   unsigned of;          // four bits per group: which of them, 15: none
-  int extra;            // EXTRA: those are tiles extra .. n - 1
-  int left;             // groups with a list that none of the others holds
+  int left;             // groups with a list that none of them holds
   __device__ __forceinline__ int entry(int e) const { return e == 0 ? e0 : e == 1 ? e1 : e == 2 ? e2 : e3; }
 };
-template <bool EXTRA>
 __device__ __forceinline__ CoverTiles cover_tiles(const UnionScratch& u, int n, int groups, int sub,
                                                   int most) {
   const int lane = threadIdx.x & 31;
   auto mask = [&](int i) -> unsigned {
     return sub == 1 ? u.masks[i] : u.masks[2 * i] | u.masks[2 * i + 1];
   };
-  CoverTiles c = {0, 0, 0, 0, 0, 0xffffffffu, 0, 0};
+  CoverTiles c = {0, 0, 0, 0, 0, 0xffffffffu, 0};
   unsigned open = (1u << groups) - 1u;
   bool any = n > 0;
   // as a rule one of the first tiles serves all
@@ -389,15 +371,6 @@ __device__ __forceinline__ CoverTiles cover_tiles(const UnionScratch& u, int n, 
     listed = __reduce_or_sync(0xffffffffu, listed);
   }
   c.left = static_cast<int>(open & listed);
-  c.extra = c.n;
-  if (EXTRA) {
-#pragma unroll 1
-    for (int at = u.top_pos, k = 0; k < 2; at = n >> 2, k++) {
-      bool have = at < 0 || n == 0;
-      for (int e = 0; e < c.n; e++) have |= c.entry(e) == at;
-      if (!have && c.n < most) add(at);
-    }
-  }
   return c;
 }
 

@@ -23,10 +23,10 @@
 // addresses that the unrolled rounds share; 348 with two CTAs per SM.  Head dim 128,
 // N = 8192, grouped heads: 312 -> 291 us from the ring.
 // bf16 and fp32 share the exponent range, so a later block may exceed the
-// reference by up to 2^80 before anything overflows (fp16: 2^16, P must not
-// exceed 65504); a row whose tile sum passes that bound marks its tile's word in `redo_out`, and the exact kernel,
-// launched behind this one with a CTA per SM, looks through the words and
-// recomputes exactly those tiles.
+// reference by up to 2^80 before anything overflows (fp16: 2^15, P must stay
+// below 65504); a row whose tile sum passes that bound marks its tile's word in
+// `redo_out`, and the exact kernel, launched behind this one with a CTA per SM, looks
+// through the words and recomputes exactly those tiles.
 #pragma once
 
 namespace ftk {
@@ -39,10 +39,10 @@ constexpr size_t fp_smem(int d, int ng) {
   return 1024 + (d / 64) * (128 * 128 + static_cast<size_t>(fp_stages(d, ng)) * 2 * 64 * 128);
 }
 // A tile's row sum of P above this marks the CTA for the exact kernel: 2^80 for
-// bf16 (fp32 exponent range), the largest fp16 number for fp16 (P itself must not exceed it).
+// bf16 (fp32 exponent range), 2^15 for fp16 (P itself must stay below 65504).
 template <int FMT>
 __device__ __forceinline__ float fp_overflow_bound() {
-  return FMT == 1 ? 1.2089258196146292e24f : 65504.f;
+  return FMT == 1 ? 1.2089258196146292e24f : 32768.f;
 }
 
 template <int FMT>
@@ -141,7 +141,7 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
   pdl_launch();
   tc_fence_after();
   // tiles whose scores give the rows their reference exponents
-  const CoverTiles pro = cover_tiles<FMT == 0>(un, n, groups, SUB, NG);
+  const CoverTiles pro = cover_tiles(un, n, groups, SUB, NG);
   const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base_s, 0);
   WaitCtx w{&abort_flag, p.status};
 
@@ -293,25 +293,20 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
 
     if (n > 0) {
-      // ---- reference exponent: scaled row maximum over the q-block's prologue tile (and
-      // the extra ones).  Group 0 works it out; behind the barrier the others may rely on
-      // the first phase of every prologue buffer being over, as their parity waits must.
+      // ---- reference exponent: scaled row maximum over the q-block's prologue tile.
+      // Group 0 works it out; behind the barrier the others may rely on the first phase of
+      // every prologue buffer being over, as their parity waits must.
       if (gw == 0) {
         for (int e = 0; ok && e < npro; e++)
           ok = mbar_wait(bar_sfull(e), 0, w, FTK_DEV_TIMEOUT_CONSUMER);
         tc_fence_after();
         float mx = -INFINITY;
-        auto look = [&](int e) {
+        const int pb = (pro.of >> (4 * grp)) & 15;   // grp is the same for the warp's rows
+        if (ok && pb != 15) {
           const ColSpan cs =
-              col_span(un, pro.entry(e), SUB, grp, pro_block(e) * KVB - p.kv_pad_head, KVB, p.N);
-          if (!__any_sync(0xffffffffu, cs.on)) return;
-          const float m = tmem_row_max(lane_addr + COL_S + e * 64, KVB, cs.lo, cs.hi);
-          if (cs.on) mx = fmaxf(mx, m);
-        };
-        const int pb = (pro.of >> (4 * grp)) & 15;
-        if (ok && pb != 15) look(pb);
-#pragma unroll 1
-        for (int e = pro.extra; FMT == 0 && ok && e < npro; e++) look(e);
+              col_span(un, pro.entry(pb), SUB, grp, pro_block(pb) * KVB - p.kv_pad_head, KVB, p.N);
+          mx = tmem_row_max(lane_addr + COL_S + pb * 64, KVB, cs.lo, cs.hi);
+        }
         s_mref[r] = (mx > -INFINITY) ? mx * c : 0.f;
         tc_fence_before();
         __syncwarp();

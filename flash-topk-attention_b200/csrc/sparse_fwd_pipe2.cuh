@@ -130,7 +130,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
       SUB, p.lm, p.status);
   pdl_launch();
   // tiles whose scores give the rows their reference exponents
-  const CoverTiles pro = cover_tiles<FMT == 0>(un, n, groups, SUB, FP2_GROUPS);
+  const CoverTiles pro = cover_tiles(un, n, groups, SUB, FP2_GROUPS);
   cluster_wait();            // barriers of both CTAs are initialised before anyone signals them
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
@@ -309,25 +309,20 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
 
     if (n > 0) {
-      // ---- reference exponent: scaled row maximum over the q-block's prologue tile (and
-      // the extra ones).  Group 0 works it out; behind the barrier the others may rely on
-      // the first phase of every prologue buffer being over, as their parity waits must.
+      // ---- reference exponent: scaled row maximum over the q-block's prologue tile.
+      // Group 0 works it out; behind the barrier the others may rely on the first phase of
+      // every prologue buffer being over, as their parity waits must.
       if (gw == 0) {
         for (int e = 0; ok && e < npro; e++)
           ok = mbar_wait(bar_sfull(e), 0, w, FTK_DEV_TIMEOUT_CONSUMER);
         tc_fence_after();
         float mx = -INFINITY;
-        auto look = [&](int e) {
+        const int pb = (pro.of >> (4 * grp)) & 15;   // grp is the same for the warp's rows
+        if (ok && pb != 15) {
           const ColSpan cs =
-              col_span(un, pro.entry(e), SUB, grp, pro_block(e) * KVB - p.kv_pad_head, KVB, p.N);
-          if (!__any_sync(0xffffffffu, cs.on)) return;
-          const float m = tmem_row_max(lane_addr + COL_S + e * 64, KVB, cs.lo, cs.hi);
-          if (cs.on) mx = fmaxf(mx, m);
-        };
-        const int pb = (pro.of >> (4 * grp)) & 15;
-        if (ok && pb != 15) look(pb);
-#pragma unroll 1
-        for (int e = pro.extra; FMT == 0 && ok && e < npro; e++) look(e);
+              col_span(un, pro.entry(pb), SUB, grp, pro_block(pb) * KVB - p.kv_pad_head, KVB, p.N);
+          mx = tmem_row_max(lane_addr + COL_S + pb * 64, KVB, cs.lo, cs.hi);
+        }
         s_mref[r] = (mx > -INFINITY) ? mx * c : 0.f;
         tc_fence_before();
         __syncwarp();

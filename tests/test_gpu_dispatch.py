@@ -397,3 +397,58 @@ def test_dkv_pair_order(ftk, monkeypatch, H, g, kvb, groups):
     plain = _grads(ftk, t, merged, H, g, kvb, **kw)
     for a, b in zip(sorted_, plain):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("D,g,kvb,N,W", [
+    (64, 64, 64, 2000, 8),       # two tiles in flight
+    (64, 32, 64, 1000, 6),       # four
+    (128, 64, 64, 4200, 9),
+    (128, 32, 32, 2100, 11),     # tiles of two listed blocks
+    (128, 64, 64, 1000, 12),     # pairs of SMs
+    (256, 64, 64, 1000, 5),
+])
+def test_order_of_a_list(ftk, dtype, D, g, kvb, N, W):
+    """A list names a set of blocks: written backwards, or with entries that are left out
+    ahead of it, it gives the same results bit for bit."""
+    H = 2
+    t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype=dtype, seed=75, do_seed=76))
+    t["q"] *= 2.0                # rows whose blocks are far apart in score
+    QM, M = -(-N // g), -(-N // kvb)
+    lists = _lists(np.random.default_rng(13), H, QM, M, W)[None]
+    pads = dict(q_padding=(0, QM * g - N), kv_padding=(0, M * kvb - N))
+    want = _grads(ftk, t, lists, H, g, kvb, **pads)
+    late = np.concatenate([np.full((1, H, QM, 4), -1, np.int32), lists], -1)
+    for other in (lists[..., ::-1].copy(), late):
+        for a, b in zip(_grads(ftk, t, other, H, g, kvb, **pads), want):
+            assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("D,W", [(64, 8), (128, 3), (128, 8), (256, 8)])
+@pytest.mark.parametrize("x", [14.9, 15.5, 16.5])
+def test_fp16_rows_near_the_bound(ftk, monkeypatch, D, W, x):
+    """One key of a block leads the rows' reference by 2^x.  Sums of a tile up to 2^15 are the
+    pipelined kernel's, those above come out as the exact kernel gives them, bit for bit."""
+    N, g = 512, 64
+    M = N // g
+    gen = torch.Generator().manual_seed(5)
+    q, k = torch.zeros(1, N, D), torch.zeros(1, N, D)
+    q[..., 0] = 8.0
+    k[:, 5 * g + 7, 0] = x / (8.0 * D ** -0.5 * 1.4426950408889634)
+    v = torch.randn(1, N, D, generator=gen)
+    merged = np.full((1, 1, M, W), -1, np.int32)
+    merged[0, 0, :, :3] = [0, 2, 5]
+    if W == M:
+        merged[0, 0] = np.arange(M)
+    args = (q.half().cuda(), k.half().cuda(), v.half().cuda(), torch.from_numpy(merged).cuda(), None, 1,
+            g, g)
+    o, lse = ftk.flash_topk_attn(*args)
+    monkeypatch.setenv("FTK_FWD_PIPE", "0")
+    o2, lse2 = ftk.flash_topk_attn(*args)
+    ftk.check_errors()
+    if x < 15.0:
+        # P up to 2^15 and O are rounded to fp16 (2^-11 relative) in both kernels, O is below 4
+        assert (o.float() - o2.float()).abs().max().item() <= 4 * 4 * 2.0 ** -11
+        torch.testing.assert_close(lse, lse2, rtol=1e-6, atol=1e-6)
+    else:
+        assert torch.equal(o, o2) and torch.equal(lse, lse2)
