@@ -362,7 +362,7 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
               }
             } else {
               float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-              if (ALL || (cb >= lo && cb + 16 <= hi)) {
+              if (ALL || full) {
                 // two columns per instruction for the scaling (fma.f32x2) and for the
                 // running sums (add.f32x2): 2 issue slots per logit instead of 3; the four
                 // partial sums are the same additions in the same order as scalar code
@@ -383,6 +383,11 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
                 a1 = s01.y;
                 a2 = s23.x;
                 a3 = s23.y;
+              } else if (cb >= lo && cb + 16 <= hi) {
+                // partial tiles add up column by column, here without the comparisons
+#pragma unroll
+                for (int i = 0; i < 16; i++)
+                  a0 += fast_exp2(fmaf(__uint_as_float(r[hc * 16 + i]), c, -mref));
               } else {
 #pragma unroll
                 for (int i = 0; i < 16; i++) {

@@ -452,3 +452,25 @@ def test_fp16_rows_near_the_bound(ftk, monkeypatch, D, W, x):
         torch.testing.assert_close(lse, lse2, rtol=1e-6, atol=1e-6)
     else:
         assert torch.equal(o, o2) and torch.equal(lse, lse2)
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("side", ["first", "last"])
+def test_partial_score_tiles_add_up_in_order(ftk, D, side):
+    """Key tiles that are not all there (the first one behind a pad head, the last one) add up
+    a block's exponentials column by column: fifteen of 2^-24.3 behind a 1 vanish one after the
+    other, since each is below half of the last place of 1, and 1 it stays."""
+    bsz = 64
+    pad, N = ((16, 0), 240) if side == "first" else ((0, 48), 208)
+    start = 48 if side == "first" else 128   # first key of a whole block in the partial tile
+    lone = 117 if side == "first" else 5     # a key of a block in a tile that is all there
+    unit = 8.0 * D ** -0.5 * 1.4426950408889634
+    q, k = torch.zeros(1, N, D), torch.zeros(1, N, D)
+    q[..., 0] = 8.0
+    k[..., 0] = -500.0 / unit                # 2^-500: nothing
+    k[:, start + 1:start + 16, 0] = -24.3 / unit
+    k[:, [start, lone], 0] = 0.0
+    got = ftk.flash_block_score(q.half().cuda(), k.half().cuda(), 1, bsz, pad)
+    ftk.check_errors()
+    a, b = got[..., (start + pad[0]) // bsz], got[..., (lone + pad[0]) // bsz]
+    assert torch.equal(a, b) and (a == 0.5).all()
