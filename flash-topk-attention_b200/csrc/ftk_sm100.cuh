@@ -332,10 +332,14 @@ __device__ __forceinline__ int ld_cta(const int* p, int rank, int n) {
 __device__ __forceinline__ float ld_cta(const float* p, int rank, int n) {
   return __int_as_float(ld_cta(reinterpret_cast<const int*>(p), rank, n));
 }
+// .aligned: every thread of the warp executes the instruction together, and callers come out of
+// branches and loops that differ between the lanes.
 __device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void cluster_sync_all() {

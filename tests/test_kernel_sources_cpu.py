@@ -79,3 +79,14 @@ def test_no_read_only_loads_in_overlapped_kernels():
         assert not re.search(what, text), what
     launched = set(re.findall(r"(\w+)(?:<[^<>;]*>)?<<<", text))
     assert not launched & set(OVERLAPPED), "an overlapped kernel must be launched as one"
+
+
+@pytest.mark.parametrize("helper", ["cluster_arrive", "cluster_wait"])
+def test_aligned_cluster_barriers_converge_first(helper):
+    """barrier.cluster.*.aligned is undefined unless all threads of a warp execute it together;
+    the kernels get there behind branches of single threads and loops whose trip count differs
+    between the lanes.  Nothing but the helpers, which converge the warp, names it."""
+    body = FUNCTIONS[helper][0]
+    assert re.search(r"__syncwarp\(\);\s*asm volatile\(\"barrier\.cluster\.\w+\.\w+\.aligned", body)
+    text = "".join(open(p).read() for p in glob.glob(os.path.join(CSRC, "*.cu*")))
+    assert len(re.findall(r"barrier\.cluster\.", text)) == 2
