@@ -5,7 +5,8 @@
 Each csrc/*.cu is compiled to an object under build/ and the objects are
 linked into lib/libftk_sm100.so (CUDA runtime linked statically; the driver
 API is reached through cudaGetDriverEntryPoint, so the library also loads on
-a machine without a GPU driver).  csrc/host/torch_ops.cpp, the native layer
+a machine without a GPU driver).  What ptxas says of the kernels (registers,
+spills) stays beside the objects.  csrc/host/torch_ops.cpp, the native layer
 between the Python operators and that library, becomes
 flash_topk_attn_v2/_native.so (host code only: g++ against PyTorch's headers).
 """
@@ -26,12 +27,16 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17",
-    "-lineinfo", "-Xcompiler", "-fPIC",
+    "-lineinfo", "-Xcompiler", "-fPIC", "-Xptxas", "-v",
 ]
 
 
 def _sources():
     return sorted(f for f in os.listdir(CSRC) if f.endswith(".cu"))
+
+
+def ptxas_log(src: str) -> str:
+    return os.path.join(OBJ, src[:-3] + ".ptxas")
 
 
 def _headers_mtime():
@@ -43,14 +48,18 @@ def _headers_mtime():
 
 def _compile(src: str, force: bool) -> str:
     obj = os.path.join(OBJ, src[:-3] + ".o")
+    log = ptxas_log(src)
     spath = os.path.join(CSRC, src)
     newest = max(os.path.getmtime(spath), _headers_mtime())
-    if not force and os.path.exists(obj) and os.path.getmtime(obj) >= newest:
+    if (not force and os.path.exists(obj) and os.path.exists(log)
+            and os.path.getmtime(obj) >= newest):
         return obj
     cmd = [NVCC, *FLAGS, "-c", spath, "-o", obj]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"nvcc failed for {src}:\n{r.stdout}\n{r.stderr}")
+    with open(log, "w") as f:
+        f.write(r.stderr)
     return obj
 
 

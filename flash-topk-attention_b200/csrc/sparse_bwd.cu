@@ -66,7 +66,8 @@ struct BwdParams {
 
 // ------------------------------------------------------------------- delta
 // delta[row] = sum_d o * do for the 128 rows of a dQ tile, by the compute warps of the
-// CTA (the others load and issue meanwhile), into shared memory (for the tile itself) and global memory (for dK/dV).
+// CTA (the others load and issue meanwhile), into shared memory (for the tile itself) and
+// global memory (for dK/dV).
 // kd / 8 lanes per row, each with one 16-byte load per tensor, so a warp covers
 // 256 / kd rows at once and a thread has all of its loads in flight together.
 // As a kernel of its own this cost a launch and 258 us at N = 32768, H = 32,
@@ -78,7 +79,7 @@ template <int KD, int WARPS = 16>
 struct TileDelta {
   static constexpr int LPR = KD / 8, RPW = 32 / LPR;
   static constexpr int STEPS = (128 + RPW * WARPS - 1) / (RPW * WARPS);
-  uint4 vd[STEPS], vo[STEPS], vo2[STEPS];   // vo2: float32 O only
+  uint4 vd[STEPS], vo[STEPS];   // vo of a float32 O: the first 4 of a lane's 8 columns
 
   __device__ __forceinline__ int row(int i) const {
     return (i * WARPS + (threadIdx.x >> 5) - 2) * RPW + (threadIdx.x & 31) / LPR;
@@ -93,50 +94,58 @@ struct TileDelta {
 #pragma unroll
     for (int i = 0; i < STEPS; i++) {
       const int r = row(i), n = tile_row0 + r;
-      vd[i] = vo[i] = vo2[i] = make_uint4(0u, 0u, 0u, 0u);
+      vd[i] = vo[i] = make_uint4(0u, 0u, 0u, 0u);
       if (!inside(p, r, n, rows)) continue;
       vd[i] = reinterpret_cast<const uint4*>(p.dout + 2 * (db + static_cast<int64_t>(n) * p.sd_n))[c];
       const int64_t oe = ob + static_cast<int64_t>(n) * p.so_n;
-      if (p.out_f32) {
-        const uint4* src = reinterpret_cast<const uint4*>(p.o + 4 * oe) + 2 * c;
-        vo[i] = src[0];
-        vo2[i] = src[1];
-      } else {
-        vo[i] = reinterpret_cast<const uint4*>(p.o + 2 * oe)[c];
-      }
+      vo[i] = p.out_f32 ? reinterpret_cast<const uint4*>(p.o + 4 * oe)[2 * c]
+                        : reinterpret_cast<const uint4*>(p.o + 2 * oe)[c];
     }
   }
-  __device__ __forceinline__ void finish(const BwdParams& p, float* s_delta, int bh, int tile_row0,
-                                         int rows) {
+  __device__ __forceinline__ void finish(const BwdParams& p, float* s_delta, int bh, int b, int h,
+                                         int tile_row0, int rows) {
     const int c = (threadIdx.x & 31) % LPR;
+    float acc[STEPS];
 #pragma unroll
     for (int i = 0; i < STEPS; i++) {
       const int r = row(i), n = tile_row0 + r;
       const uint32_t wd[4] = {vd[i].x, vd[i].y, vd[i].z, vd[i].w};
       float2 fo[4];
       if (p.out_f32) {
+        // The second half lies in the sectors that `load` has fetched.  Loaded there as well
+        // it would hold registers in 16-bit calls too.
+        uint4 hi = make_uint4(0u, 0u, 0u, 0u);
+        if (inside(p, r, n, rows)) {
+          const int64_t oe = static_cast<int64_t>(b) * p.so_b + static_cast<int64_t>(h) * p.so_h +
+                             static_cast<int64_t>(n) * p.so_n;
+          hi = reinterpret_cast<const uint4*>(p.o + 4 * oe)[2 * c + 1];
+        }
         fo[0] = make_float2(__uint_as_float(vo[i].x), __uint_as_float(vo[i].y));
         fo[1] = make_float2(__uint_as_float(vo[i].z), __uint_as_float(vo[i].w));
-        fo[2] = make_float2(__uint_as_float(vo2[i].x), __uint_as_float(vo2[i].y));
-        fo[3] = make_float2(__uint_as_float(vo2[i].z), __uint_as_float(vo2[i].w));
+        fo[2] = make_float2(__uint_as_float(hi.x), __uint_as_float(hi.y));
+        fo[3] = make_float2(__uint_as_float(hi.z), __uint_as_float(hi.w));
       } else {
         fo[0] = unpack2(vo[i].x, p.fmt);
         fo[1] = unpack2(vo[i].y, p.fmt);
         fo[2] = unpack2(vo[i].z, p.fmt);
         fo[3] = unpack2(vo[i].w, p.fmt);
       }
-      float acc = 0.f;
+      acc[i] = 0.f;
 #pragma unroll
       for (int x = 0; x < 4; x++) {
         const float2 gd = unpack2(wd[x], p.fmt);
-        acc = fmaf(fo[x].x, gd.x, acc);
-        acc = fmaf(fo[x].y, gd.y, acc);
+        acc[i] = fmaf(fo[x].x, gd.x, acc[i]);
+        acc[i] = fmaf(fo[x].y, gd.y, acc[i]);
       }
+    }
 #pragma unroll
-      for (int d = LPR >> 1; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+    for (int i = 0; i < STEPS; i++) {
+      const int r = row(i), n = tile_row0 + r;
+#pragma unroll
+      for (int d = LPR >> 1; d > 0; d >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], d);
       if (c == 0 && r < 128) {
-        s_delta[r] = acc;
-        if (inside(p, r, n, rows)) p.delta[static_cast<int64_t>(bh) * p.N + n] = acc;
+        s_delta[r] = acc[i];
+        if (inside(p, r, n, rows)) p.delta[static_cast<int64_t>(bh) * p.N + n] = acc[i];
       }
     }
   }
@@ -503,7 +512,7 @@ sparse_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q,
     // the sums run under the first UMMAs (256 columns are too many registers to hold
     // across the union)
     if (D > 128) delta.load(p, b_idx, h_idx, tile_row0, groups * p.g);
-    delta.finish(p, s_delta, bh, tile_row0, groups * p.g);
+    delta.finish(p, s_delta, bh, b_idx, h_idx, tile_row0, groups * p.g);
     asm volatile("bar.sync 1, %0;" ::"n"(256 * NG) : "memory");
     const float dl = row_valid ? s_delta[r] : 0.f;
     for (int i = wg; ok && i < n; i += NG) {

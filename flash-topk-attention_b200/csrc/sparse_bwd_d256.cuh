@@ -300,7 +300,7 @@ sparse_bwd_dq256_kernel(const __grid_constant__ CUtensorMap tm_q,
     bool ok = true;
     // 256 columns are too many registers to hold across the union
     delta.load(p, b_idx, h_idx, tile_row0, mine * p.g);
-    delta.finish(p, s_delta, bh, tile_row0, mine * p.g);
+    delta.finish(p, s_delta, bh, b_idx, h_idx, tile_row0, mine * p.g);
     asm volatile("bar.sync 1, 512;" ::: "memory");
     const float dl = row_valid ? s_delta[r] : 0.f;
     for (int i = wg; ok && i < n; i += 2) {

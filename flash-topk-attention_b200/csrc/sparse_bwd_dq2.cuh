@@ -282,7 +282,7 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
       if (lane == 0) mbar_arrive_cta(bar_qt, 0);
     }
     // the sums run under the first UMMAs
-    delta.finish(p, s_delta, bh, tile_row0, mine * p.g);
+    delta.finish(p, s_delta, bh, b_idx, h_idx, tile_row0, mine * p.g);
     asm volatile("bar.sync 1, 512;" ::: "memory");
     const float dl = row_valid ? s_delta[r] : 0.f;
     for (int i = wg; ok && i < n; i += 2) {

@@ -1,6 +1,7 @@
 """Rules of the overlapped launches that a run cannot show, read off the sources."""
 
 import glob
+import importlib.util
 import os
 import re
 
@@ -90,3 +91,22 @@ def test_aligned_cluster_barriers_converge_first(helper):
     assert re.search(r"__syncwarp\(\);\s*asm volatile\(\"barrier\.cluster\.\w+\.\w+\.aligned", body)
     text = "".join(open(p).read() for p in glob.glob(os.path.join(CSRC, "*.cu*")))
     assert len(re.findall(r"barrier\.cluster\.", text)) == 2
+
+
+def test_registers_suffice():
+    """Kernels whose loop over the tiles has 96 registers a thread put at most 96 bytes of
+    them into local memory (what ptxas reports at the build; a few words around the prologue
+    do no harm).  The exact forward, a fallback, may hold two accumulators' worth more."""
+    spec = importlib.util.spec_from_file_location("ftk_build", os.path.join(os.path.dirname(CSRC), "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    seen = 0
+    for src in ("score.cu", "sparse_fwd.cu", "sparse_bwd.cu"):
+        if not os.path.exists(build.ptxas_log(src)):
+            pytest.skip("not built here")
+        text = open(build.ptxas_log(src)).read()
+        for name, spilled in re.findall(r"Compiling entry function '(\S+)'.*?(\d+) bytes spill stores", text,
+                                        re.S):
+            seen += 1
+            assert int(spilled) <= (192 if "17sparse_fwd_kernel" in name else 96), name
+    assert seen > 40
