@@ -62,6 +62,7 @@ struct BwdParams {
   int sub;                   // listed blocks per tile: kv blocks (dQ), q-blocks (dKV)
   const int32_t* order;      // dKV: kv blocks by fan-in, heaviest first ([BH][Mkv]) or null
   const int32_t* tile_order; // dKV: the CTAs' (pairs') tiles by number of q-blocks, heaviest first, or null
+  const int32_t* pick;       // dKV: per slice, 1: the pair kernel does it, 0: the one-CTA kernel; or null
 };
 
 // ------------------------------------------------------------------- delta
@@ -681,6 +682,15 @@ __device__ __forceinline__ KvTile kv_tile(const BwdParams& p, int x, int tiles) 
   return t;
 }
 
+// Both kernels are launched where the lists decide which is the faster (see fan_in_kernel);
+// the CTAs of the other one leave at once, behind the wait for the decision, which also
+// keeps the order of the launches for whoever waits for this one.
+__device__ __forceinline__ bool other_kernel(const BwdParams& p, int slice, int mine) {
+  if (!p.pick) return false;
+  pdl_wait();
+  return p.pick[slice] != mine;
+}
+
 // TMEM columns: S^T[2] 0/64 (P^T written over their first half), dP^T[2]
 // 128/192 (dS^T likewise), dV 256.., dK 384..
 // Head dim 64: K (320..351) and V (352..383) are copied into TMEM as well, so that the
@@ -720,6 +730,7 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const KvTile at = kv_tile(p, blockIdx.x, gridDim.x);
   const int bh = at.slice;
+  if (other_kernel(p, bh, 0)) return;
   int j0 = at.tile * p.G;                   // first kv block of the tile
   if (p.order && !p.tile_order) {
     // The same from a reverse index, which orders kv blocks: the grid has one CTA
@@ -1117,20 +1128,30 @@ namespace ftk {
 // blocks) has to walk, from the dQ kernel's tile masks, and the tiles sorted by that
 // number, largest first (ties: lower tile).  With skewed lists a few tiles take many times
 // the others' time; issued last they would run alone.  One CTA per slice, key = (count + 1, ~tile).
+// `pick`: whether pairs of SMs should do the slice.  A step of the pair kernel is the shorter
+// one, but it walks the q-blocks that list any of four kv blocks, not of two.  Twice the
+// pairs' steps over the single tiles' steps is 1 where neighbouring blocks are listed together
+// (windows, runs of blocks) and near 1.5 where lists of a quarter of the blocks are
+// independent.  Backward passes in pairs against single SMs, B = 1, N = 16384 and 32768, H = 8,
+// and B = 2, N = 8192, H = 16: 0.92 to 0.97 of the time at ratios up to 1.05, 0.97 to 0.98 at
+// 1.14, 1.01 at 1.25, 1.05 to 1.09 at 1.38, 1.08 to 1.14 at 1.48.
 constexpr int FAN_THREADS = 1024;
 
 __global__ void __launch_bounds__(FAN_THREADS)
 fan_in_kernel(const uint8_t* masks, int stride, int tiles, int64_t head_stride, int heads,
-              int slices_per_b, int H, int G, int cols, int colsp, int32_t* order) {
+              int slices_per_b, int H, int G, int cols, int colsp, int32_t* order, int32_t* pick) {
   extern __shared__ unsigned long long fan_keys[];
   unsigned* cnt = reinterpret_cast<unsigned*>(fan_keys + colsp);
+  __shared__ unsigned single, pairs;   // q-blocks that all tiles, and all pairs of tiles, walk
   pdl_wait();
   pdl_launch();
   const int tid = threadIdx.x;
   const int slice = blockIdx.x;
   const int bhq = slice / slices_per_b * H + slice % slices_per_b * heads;
+  if (tid == 0) single = pairs = 0u;
   for (int x = tid; x < colsp; x += FAN_THREADS) cnt[x] = 0u;
   __syncthreads();
+  unsigned in_pairs = 0u, in_single = 0u;
   // 16 bytes = 16 / G kv tiles of one q tile per load, the q tiles dealt to as many
   // threads as there are (a byte per load and row took some 95 us longer at 403 q
   // tiles of 806 kv blocks, one slice)
@@ -1156,15 +1177,29 @@ fan_in_kernel(const uint8_t* masks, int stride, int tiles, int64_t head_stride, 
           m = (m | (m >> 8) | (m >> 16) | (m >> 24)) & 255u;
         }
         if (x % G == 0) c[x] += __popc(m);
+        if (pick && x % 4 == 0) {   // G is 2, a pair has four blocks
+          const unsigned m4 = w[x >> 2];
+          in_pairs += __popc((m4 | (m4 >> 8) | (m4 >> 16) | (m4 >> 24)) & 255u);
+        }
       }
     }
 #pragma unroll
     for (int x = 0; x < 16; x++) {
       const int col = (quad * 16 + x) / G;
       if (x % G == 0 && col < cols && c[x]) atomicAdd(&cnt[col], c[x]);
+      if (x % G == 0) in_single += c[x];
+    }
+  }
+  if (pick) {
+    in_single = __reduce_add_sync(0xffffffffu, in_single);
+    in_pairs = __reduce_add_sync(0xffffffffu, in_pairs);
+    if ((tid & 31) == 0) {
+      atomicAdd(&single, in_single);
+      atomicAdd(&pairs, in_pairs);
     }
   }
   __syncthreads();
+  if (pick && tid == 0) pick[slice] = 10 * pairs < 6 * single;
   for (int x = tid; x < colsp; x += FAN_THREADS)
     fan_keys[x] = x < cols ? (static_cast<unsigned long long>(cnt[x] + 1u) << 32) |
                                  (0xffffffffu - static_cast<unsigned>(x))
@@ -1242,7 +1277,8 @@ struct BwdPlan {
   int kv_tiles;              // kv tiles of a CTA (or a pair) per slice
   int tile_blocks;           // kv blocks of such a tile
   bool order;                // dK/dV tiles sorted by the work they have
-  size_t off_masks, off_order, off_dk, off_dv, bytes;
+  bool pick;                 // dK/dV: pairs or single SMs slice by slice, see fan_in_kernel
+  size_t off_masks, off_order, off_pick, off_dk, off_dv, bytes;
 };
 
 static size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
@@ -1270,11 +1306,10 @@ static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
   b.stride = flag_blocks(gr.Mkv);
   b.span = (b.tiles * per + 31) & ~31;
   // Pairs walk the union of four lists.  The line is that of ftk_attn_fwd (f = 1/4 there:
-  // dQ 451 us in pairs, 388 without).  A tile of dK / dV takes 0.82 of the time in pairs
-  // (its S^T and dP^T UMMAs read both operands from shared memory), which independent
-  // lists outweigh up to f = 0.55 (f = 1/4, four heads per kv head, tiles in order of
-  // their work: 510 us in pairs, 393 without).  At head dim 256 the pair kernels are
-  // several times the faster per tile.
+  // dQ 451 us in pairs, 388 without).  dK / dV with independent lists, or with ones that
+  // share a block and a window: pairs are ahead from f = 0.5 to 0.6 on (f = 1/4, four heads
+  // per kv head, tiles in order of their work: 510 us in pairs, 393 without).  At head dim
+  // 256 the pair kernels are several times the faster per tile.
   b.pair_dq = tiles64 && (gr.kd == 256 || (gr.kd == 128 && 2 * gr.width >= gr.Mkv));
   b.pair_dkv = b.pair_dq && (gr.kd == 256 || !env_off("FTK_DKV_2CTA"));
   // Query heads that share a kv head: walked one after the other by the CTA that
@@ -1293,11 +1328,23 @@ static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
   b.kv_tiles = (gr.Mkv + b.tile_blocks - 1) / b.tile_blocks;
   b.order = b.pair_dkv ? 2 * gr.width < gr.Mkv && 2 * slices * b.kv_tiles >= 2 * sms
                        : slices * b.kv_tiles >= 2 * sms;
+  // Below that line the lists decide for dK / dV, where they can be such that pairs pay (see
+  // fan_in_kernel): from a quarter of the blocks on, and only if a kv block is listed by 32
+  // q-blocks or more on average.  CTAs that find the decision against them take 7 to 24 us
+  // together, 0.4 to 1.3 % of passes that pairs make 1 to 7 % shorter; with a fan-in of 24
+  // they cost as much as is gained.  Where a CTA walks several heads pairs are never more
+  // than 4 % ahead, and mostly 1 %; with blocks of 32 rows, where two listed blocks share a
+  // tile's step, the ratio of the steps does not say which is the faster.
+  b.pick = b.order && !b.walk && gr.g == 64 && gr.kvb == 64 && gr.kd == 128 && !b.pair_dkv &&
+           4 * gr.width >= gr.Mkv && 2 * gr.width < gr.Mkv &&
+           gr.width * gr.QM >= 32 * static_cast<int64_t>(gr.Mkv) && !env_off("FTK_DKV_2CTA");
   size_t off = up256(static_cast<size_t>(BH) * a.N * 4);   // delta
   b.off_masks = off;
   off += up256(static_cast<size_t>(BH) * b.tiles * b.stride);
   b.off_order = off;
   if (b.order) off += up256(static_cast<size_t>(slices) * b.kv_tiles * 4);
+  b.off_pick = off;
+  if (b.pick) off += up256(static_cast<size_t>(slices) * 4);
   b.off_dk = b.off_dv = off;
   if (grp > 1 && !b.walk) {
     const size_t part = up256(static_cast<size_t>(BH) * a.N * a.D * 2);
@@ -1589,14 +1636,19 @@ extern "C" int ftk_attn_bwd_dkv(const ftk_attn* a, const void* dout, int64_t sdo
     while (colsp < b.kv_tiles) colsp <<= 1;
     const size_t smem = static_cast<size_t>(colsp) * 12;
     int32_t* order = reinterpret_cast<int32_t*>(ws + b.off_order);
+    int32_t* pick = b.pick ? reinterpret_cast<int32_t*>(ws + b.off_pick) : nullptr;
     int e = allow_smem<fan_in_kernel>(smem);
     if (!e)
       e = launch_pdl(fan_in_kernel, static_cast<unsigned>(a->B * a->H / p.heads), FAN_THREADS, smem,
                      st, p.masks, b.stride, b.tiles,
                      static_cast<int64_t>(b.tiles) * b.stride, p.heads,
                      static_cast<int>(a->H / p.heads), static_cast<int>(a->H),
-                     b.tile_blocks, b.kv_tiles, colsp, order);
+                     b.tile_blocks, b.kv_tiles, colsp, order, pick);
     if (e) return e;
+    if (pick) {
+      p.pick = pick;
+      if ((e = launch_dkv(*a, Rows{dout, a->H, sdo_b, sdo_n, sdo_h}, p, b.gr.kd, true, st))) return e;
+    }
     p.tile_order = order;
   }
   if (int e = launch_dkv(*a, Rows{dout, a->H, sdo_b, sdo_n, sdo_h}, p, b.gr.kd, b.pair_dkv, st))

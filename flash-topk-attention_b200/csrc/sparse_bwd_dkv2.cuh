@@ -81,6 +81,7 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
   const KvTile at = kv_tile(p, blockIdx.x >> 1, gridDim.x >> 1);
   const int j0 = at.tile * 2 * per;          // first of the pair's kv blocks
   const int bh = at.slice;
+  if (other_kernel(p, bh, 1)) return;   // both CTAs of the pair
   // slice = (batch, first of the query heads this pair walks)
   const int slices = WALK ? p.H / p.heads : p.H;
   const int b_idx = bh / slices, h_idx = (bh - b_idx * slices) * (WALK ? p.heads : 1);

@@ -474,3 +474,89 @@ def test_partial_score_tiles_add_up_in_order(ftk, D, side):
     ftk.check_errors()
     a, b = got[..., (start + pad[0]) // bsz], got[..., (lone + pad[0]) // bsz]
     assert torch.equal(a, b) and (a == 0.5).all()
+
+
+def _coherent_lists(rng, M, QM, W, kind):
+    """One slice's lists of W blocks: a window around the row, aligned runs of blocks, few blocks at random
+    (each several times)."""
+    out = np.empty((QM, W), np.int32)
+    for m in range(QM):
+        if kind == "window":
+            first = min(max(m * M // QM - W // 2, 0), M - W)
+            out[m] = np.arange(first, first + W)
+        elif kind == "runs":
+            out[m] = (rng.permutation(M // 8)[:W // 8, None] * 8 + np.arange(8)).reshape(-1)
+        else:
+            out[m] = np.resize(rng.permutation(M)[:W // 4], W)
+    return out
+
+
+@pytest.mark.parametrize("N,W,H,Hkv", [
+    (6300, 40, 16, 16), (8192, 32, 12, 12),      # widest and narrowest of the lists that do
+    (6300, 40, 4, 2), (4096, 16, 16, 16)])       # none: one wave and a half; fan-in 16
+def test_lists_choose_the_dkv_kernel(ftk, monkeypatch, N, W, H, Hkv):
+    """Lists of a quarter to a half of the blocks, blocks of many readers: slice by slice the
+    pairs of SMs do dK / dV where four kv blocks are listed by few more q-blocks than two (their
+    unions together below 1.2 of those), the one-CTA kernel the rest; the results are those of
+    the latter alone."""
+    import ctypes as C
+    from flash_topk_attn_v2 import _lib
+    g = kvb = 64
+    D, QM = 128, -(-N // g)
+    M = QM
+    assert M <= 4 * W and 2 * W < M
+    chosen = W >= 32 and H > 4
+    rng = np.random.default_rng(21)
+    kinds = ["window", "few", "runs", "few"] * (H // 4)
+    lists = np.stack([_coherent_lists(rng, M, QM, W, k) for k in kinds])[None]
+    t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype="bf16", seed=77, do_seed=78))
+    for n in "kv":
+        t[n] = t[n][..., :Hkv * D].contiguous()
+    pads = dict(q_padding=(0, QM * g - N), kv_padding=(0, M * kvb - N), num_kv_heads=Hkv)
+    lib = _lib.lib
+    before = lib.ftk_launch_count()
+    got = _grads(ftk, t, lists, H, g, kvb, **pads)
+    launches = lib.ftk_launch_count() - before
+    monkeypatch.setenv("FTK_DKV_2CTA", "0")
+    before = lib.ftk_launch_count()
+    want = _grads(ftk, t, lists, H, g, kvb, **pads)
+    assert launches == lib.ftk_launch_count() - before + chosen
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    if not chosen:
+        return
+    monkeypatch.delenv("FTK_DKV_2CTA")
+
+    class Attn(C.Structure):
+        _fields_ = ([(n, C.c_void_p) for n in "qkv"] + [("dtype", C.c_int), ("out_f32", C.c_int)]
+                    + [(n, C.c_int64) for n in ("B", "H", "Hkv", "N", "D")]
+                    + [(f"s{x}_{y}", C.c_int64) for x in "qkv" for y in "bnh"]
+                    + [("lists", C.c_void_p)]
+                    + [(n, C.c_int) for n in ("list_rows", "W", "q_block", "kv_block", "q_pad_head",
+                                              "kv_pad_head")] + [("scale", C.c_float)])
+
+    x = {n: y.cuda() for n, y in t.items()}
+    dev_lists = torch.from_numpy(lists).cuda()
+    s = (N * H * D, H * D, D)
+    a = Attn(*(x[n].data_ptr() for n in "qkv"), _lib.dtype_code(x["q"]), 0, 1, H, H, N, D, *s, *s, *s,
+             dev_lists.data_ptr(), QM, W, g, kvb, 0, 0, D ** -0.5)
+    size = lib.ftk_attn_bwd_workspace(C.byref(a))
+    ws = torch.zeros(size, dtype=torch.uint8, device="cuda")
+    dq, dk, dv = (torch.empty_like(x["q"]) for _ in range(3))
+    o, lse = got[0], got[1]
+    assert lib.ftk_attn_bwd_dq(C.byref(a), o.data_ptr(), *s, x["do"].data_ptr(), *s, lse.data_ptr(),
+                               ws.data_ptr(), size, dq.data_ptr(), *s, 0, 0) == 0
+    assert lib.ftk_attn_bwd_dkv(C.byref(a), x["do"].data_ptr(), *s, lse.data_ptr(), ws.data_ptr(), size,
+                                dk.data_ptr(), *s, dv.data_ptr(), *s, 0, 0) == 0
+    torch.cuda.synchronize()
+    for y, z in zip((dq, dk, dv), got[2:]):
+        assert torch.equal(y, z)
+    pick = ws[-256:].view(torch.int32)[:H].tolist()       # the last thing in the workspace
+    per = 128 // kvb
+    for h in range(H):
+        on = np.zeros((QM, -(-M // (2 * per)) * 2 * per), bool)
+        np.put_along_axis(on, lists[0, h], True, 1)
+        single = on.reshape(QM, -1, per).any(-1).sum()
+        pairs = on.reshape(QM, -1, 2 * per).any(-1).sum()
+        assert pick[h] == (10 * pairs < 6 * single), (h, kinds[h], pairs / single)
+    assert 0 < sum(pick) < H
