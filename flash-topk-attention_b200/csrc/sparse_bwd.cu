@@ -1393,13 +1393,15 @@ static int tmap_of(CUtensorMap* t, const ftk_attn& a, const Rows& r, int rows) {
 
 // Two CTAs of one group per SM, or one CTA of two?  Two CTAs cover each other's list
 // union, first loads and last tile, but go by twice the CTAs per wave.  A CTA's time
-// with n tiles is 10.4 + 0.49 n us alone and 13.8 + 0.95 n us as one of two (from
-// N = 8192, H = 16, all pairs: 509 and 539 us in 7 and 4 waves; N = 2048, B = 2, H = 16:
-// 104 and 88 us in 4 and 2).
+// with n tiles is put at 7 + 0.32 n us alone and 8.5 + 0.72 n us as one of two: fitted to
+// which of the two was the faster in 44 backward passes (H N / 128 of 16 to 1024 CTAs,
+// lists of 4 blocks to all), over which the rule is at most 0.8 % behind the better one.
+// One against two groups: N = 1024, H = 32, all pairs 66.6, 70.6 us; N = 8192, H = 4, lists
+// of 64 261, 251 and of 16 103, 105; H = 16, of 4 159, 173 and all pairs 1193, 1144.
 static bool one_group(int64_t ctas, int tiles) {
   const int64_t sms = sm_count();
-  return ((ctas + 2 * sms - 1) / (2 * sms)) * (13.8 + 0.95 * tiles) <
-         ((ctas + sms - 1) / sms) * (10.4 + 0.49 * tiles);
+  return ((ctas + 2 * sms - 1) / (2 * sms)) * (8.5 + 0.72 * tiles) <
+         ((ctas + sms - 1) / sms) * (7.0 + 0.32 * tiles);
 }
 
 static int launch_dq(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, bool pair,
@@ -1458,7 +1460,9 @@ static int launch_dq(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, b
     return launch_pdl(kernel, grid, bw_threads(ng), smem, st, tq, tdo, tk, tv, p);
   };
   if (kd == 64)
-    return one_group(static_cast<int64_t>(grid.x) * grid.y, static_cast<int>(std::min<int64_t>(static_cast<int64_t>(p.G) * p.W, p.Mkv / p.sub)))
+    return one_group(static_cast<int64_t>(grid.x) * grid.y,
+                     static_cast<int>(std::min(static_cast<int64_t>(p.G) * p.W,
+                                               static_cast<int64_t>(p.Mkv / p.sub))))
                ? go(Kernel<sparse_bwd_dq_kernel<64, 1>>{}, 1)
                : go(Kernel<sparse_bwd_dq_kernel<64, 2>>{}, 2);
   return go(Kernel<sparse_bwd_dq_kernel<128, 2>>{}, 2);

@@ -560,3 +560,24 @@ def test_lists_choose_the_dkv_kernel(ftk, monkeypatch, N, W, H, Hkv):
         pairs = on.reshape(QM, -1, 2 * per).any(-1).sum()
         assert pick[h] == (10 * pairs < 6 * single), (h, kinds[h], pairs / single)
     assert 0 < sum(pick) < H
+
+
+@pytest.mark.parametrize("N,H,W,groups", [
+    (8192, 4, 4, 1), (8192, 4, 16, 1), (8192, 4, 64, 2), (8192, 8, 128, 2),   # two waves of pairs
+    (2048, 8, 32, 2), (1024, 32, 16, 1),                                     # one wave; short lists
+])
+def test_dq_goes_by_the_faster_kernel(ftk, N, H, W, groups):
+    """Head dim 64: two CTAs of one group per SM or one of two, whichever was measured to be
+    the faster in these passes (by 1 to 20 %; the two give the same results)."""
+    from torch.profiler import ProfilerActivity, profile
+    M = N // 64
+    t = cases.make_inputs(dict(B=1, N=N, H=H, D=64, dtype="bf16", seed=79, do_seed=80))
+    lists = np.stack([_coherent_lists(np.random.default_rng(h), M, M, W, "window") for h in range(H)])[None]
+    q, k, v = (t[n].cuda().requires_grad_(True) for n in "qkv")
+    o, _ = ftk.flash_topk_attn(q, k, v, torch.from_numpy(lists).cuda(), None, H, 64, 64)
+    do = t["do"].cuda()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        torch.autograd.grad(o, (q, k, v), do)
+        torch.cuda.synchronize()
+    names = [e.key for e in prof.key_averages() if "sparse_bwd_dq_kernel" in e.key]
+    assert len(names) == 1 and f"sparse_bwd_dq_kernel<64, {groups}>" in names[0], names
