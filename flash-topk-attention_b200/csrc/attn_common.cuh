@@ -29,9 +29,12 @@ struct UnionScratch {
 // What tile i of the union (its first token is tok0, `width` tokens) holds for a row
 // of group `grp`: columns lo .. hi - 1, none unless `on`.  With sub 1 lo and hi are
 // the same for all threads, and stay in uniform registers.  Rows that do not exist are
-// like the others: copies fill them with zeros, what comes of that is finite in its own
-// row and not stored.  Told apart, they kept their warps off the path for full tiles in
-// every tile (N = 3000, H = 12, head dim 96: forward 89 us, 61 without).
+// like the others: copies fill them with zeros.  What comes of that may be infinite or NaN
+// (a zero query against an infinite key; 2^-lse against a small lse in dK / dV), but it
+// stays in the row's own lane of every accumulator, and neither the stores nor the flags
+// for the exact kernel look at such rows; nothing may add up over rows without leaving them
+// out.  Told apart in the loop, they kept their warps off the path for full tiles in every
+// tile (N = 3000, H = 12, head dim 96: forward 89 us, 61 without).
 struct ColSpan {
   int lo, hi;
   bool on;

@@ -15,9 +15,10 @@
 // S buffer), a CTA has four groups and the SM to itself.  With head dim 64 and
 // q-blocks of 64 rows it has two, 256 TMEM columns and half the shared memory, and
 // two CTAs share an SM: as many tiles are in flight, the list union, first loads,
-// reference tiles and last tiles of one CTA run under the tiles of the other, and two warps issue.  The issuing warp bounds the
-// loop otherwise: with 16 softmax warps beside it a round of 8 UMMAs, two commits
-// and two waits takes it 600 cycles, the exponentials 512.  Forward at B = 1, H = 16,
+// reference tiles and last tiles of one CTA run under the tiles of the other, and two
+// warps issue.  The issuing warp bounds the loop otherwise: with 16 softmax warps beside
+// it a round of 8 UMMAs, two commits and two waits takes it 600 cycles, the exponentials
+// 512.  Forward at B = 1, H = 16,
 // N = 8192, all pairs: 404 us with four groups, a K ring and a V ring; 388 with K and
 // V in one ring (two waits and two commits per tile, were three and three) and
 // addresses that the unrolled rounds share; 348 with two CTAs per SM.  Head dim 128,

@@ -252,8 +252,10 @@ int ftk_attn_bwd_dkv(const ftk_attn* a, const void* dout, int64_t sdo_b, int64_t
  * h / (H / Hkv).  The reference rejects Hkv != H (__init__.py:153-156).
  * `workspace` (ftk_sparse_fwd_workspace bytes, may be NULL) enables the
  * pipelined kernel for q and kv blocks of 64 or 32 rows (bf16 or fp16): it uses one
- * fixed reference exponent per row, and the exact running-maximum kernel, launched behind it, recomputes the tiles whose scores left the safe
- * exponent range (none on ordinary inputs).  Without a workspace only the
+ * fixed reference exponent per row, and the exact running-maximum kernel, launched
+ * behind it, recomputes the tiles whose scores left the safe exponent range (none on
+ * ordinary inputs).  A list is a set of blocks: the order of its entries and negative
+ * ones among them change no bit of a result.  Without a workspace only the
  * exact kernel runs.  Setting the environment variable FTK_FWD_PIPE=0 does the
  * same.  At head dim 256, and at head dim 128 with lists that can cover a good
  * part of the blocks (2 W >= M), the pipelined kernel runs on pairs of SMs
@@ -275,10 +277,11 @@ int ftk_sparse_fwd(const void* q, const void* k, const void* v, int dtype, int64
  * sparse_attn_bwd_dq_launch (csrc/sparse_attn_bwd_dq.cpp:3-15,
  * csrc/sparse_attn_bwd_dq_kernel.cu:422): delta[bh][n] = sum_d o*do (fp32),
  * then dq for every q-block.  `delta` is an output the dK/dV call reuses. */
-/* Head dim 128 with 64-row blocks and wide lists (2 W >= M in dq, 4 W >= M in dkv)
- * runs on pairs of SMs (clusters of two CTAs, tcgen05 cta_group::2) in both calls;
- * ftk_attn_bwd_dq and ftk_attn_bwd_dkv run head dim 256 and 32-row blocks on pairs
- * as well.  FTK_DQ_2CTA=0 and FTK_DKV_2CTA=0 select the one-CTA kernels at head dim
+/* Head dim 128 with 64-row blocks and wide lists (2 W >= M) runs on pairs of SMs
+ * (clusters of two CTAs, tcgen05 cta_group::2) in both calls; ftk_attn_bwd_dq and
+ * ftk_attn_bwd_dkv run head dim 256 and 32-row blocks on pairs as well, and
+ * ftk_attn_bwd_dkv launches both kernels where the lists on the device decide which
+ * one does a slice (4 W >= M, blocks of many readers, one head per CTA).  FTK_DQ_2CTA=0 and FTK_DKV_2CTA=0 select the one-CTA kernels at head dim
  * 128. */
 int ftk_sparse_bwd_dq(const void* q, const void* k, const void* v, const void* o, const void* dout,
                       int dtype, int64_t B, int64_t H, int64_t Hkv, int64_t N, int64_t D, int64_t sq_b,
@@ -297,7 +300,7 @@ int ftk_sparse_bwd_dq(const void* q, const void* k, const void* v, const void* o
  * caller sums the H / Hkv heads of a group.  `fwd_list_width` is the
  * width W of the merged_idx lists the reverse index was built from (0 if
  * unknown); it only helps to choose between the kernel on pairs of SMs (lists
- * that can cover a good part of the blocks: 4 W >= M) and the one-CTA kernel.
+ * that can cover a good part of the blocks: 2 W >= M) and the one-CTA kernel.
  * `sorted_kv` (may be NULL: block order) is the kv-block order of
  * ftk_build_reverse; the one-CTA kernels issue their tiles in that order,
  * heaviest first, as the reference's kernel does
