@@ -94,6 +94,24 @@ __device__ __forceinline__ int seg_begin(const ScoreParams& p, int s) {
   return static_cast<int>(static_cast<int64_t>(s) * (p.num_tiles / per) / SC_SEGS) * per;
 }
 
+// Sum of 2^(c s - mref) over 16 columns, two per instruction for the scaling (fma.f32x2) and
+// for the running sums (add.f32x2); the four partial sums are the same additions in the same
+// order as scalar code.
+__device__ __forceinline__ float sum16(const uint32_t (&r)[16], float c, float mref) {
+  const float2 c2 = make_float2(c, c), nm2 = make_float2(-mref, -mref);
+  auto exp2_of = [&](int i) {
+    const float2 x = __ffma2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), c2, nm2);
+    return make_float2(fast_exp2(x.x), fast_exp2(x.y));
+  };
+  float2 s01 = make_float2(0.f, 0.f), s23 = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < 16; i += 4) {
+    s01 = __fadd2_rn(s01, exp2_of(i));
+    s23 = __fadd2_rn(s23, exp2_of(i + 2));
+  }
+  return (s01.x + s01.y) + (s23.x + s23.y);
+}
+
 // SPLIT: launched as clusters that share a tile; its bookkeeping in the loop over the
 // tiles took 4 % of the kernel where nothing is split.
 template <int D, bool SPLIT>
@@ -328,6 +346,7 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
       }
     }
 
+    const bool whole = p.bsz % 64 == 0;
     float acc = 0.f;
     int j = 0, col_in_block = 0;
     // this group's tiles, part by part
@@ -345,99 +364,72 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
       const bool full = (lo == 0 && hi == ti.used);
       if (ti.col_in_block0 == 0) { j = ti.block0; col_in_block = 0; }
       const uint32_t acc_addr = lane_addr + static_cast<uint32_t>((a * 2 + half) * SC_KT);
-      // one 32-column chunk: two 16-column halves, block sums flushed on the
-      // 16-column grid (block sizes are multiples of 16)
-      auto process = [&](const uint32_t (&r)[32], int c0, auto all) {
-        constexpr bool ALL = decltype(all)::value;   // every column is a key of a score block
-#pragma unroll
-        for (int hc = 0; hc < 2; hc++) {
-          const int cb = c0 + hc * 16;
-          if (ALL || cb < ti.used) {
-            if (pass == 1) {
-#pragma unroll
-              for (int i = 0; i < 16; i++) {
-                const int col = cb + i;
-                if (ALL || (col >= lo && col < hi))
-                  run_max = fmaxf(run_max, __uint_as_float(r[hc * 16 + i]));
-              }
-            } else {
-              float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-              if (ALL || full) {
-                // two columns per instruction for the scaling (fma.f32x2) and for the
-                // running sums (add.f32x2): 2 issue slots per logit instead of 3; the four
-                // partial sums are the same additions in the same order as scalar code
-                float2 s01 = make_float2(0.f, 0.f), s23 = make_float2(0.f, 0.f);
-                const float2 c2 = make_float2(c, c), nm2 = make_float2(-mref, -mref);
-#pragma unroll
-                for (int i = 0; i < 16; i += 4) {
-                  const float2 x = __ffma2_rn(make_float2(__uint_as_float(r[hc * 16 + i + 0]),
-                                                          __uint_as_float(r[hc * 16 + i + 1])),
-                                              c2, nm2);
-                  const float2 y = __ffma2_rn(make_float2(__uint_as_float(r[hc * 16 + i + 2]),
-                                                          __uint_as_float(r[hc * 16 + i + 3])),
-                                              c2, nm2);
-                  s01 = __fadd2_rn(s01, make_float2(fast_exp2(x.x), fast_exp2(x.y)));
-                  s23 = __fadd2_rn(s23, make_float2(fast_exp2(y.x), fast_exp2(y.y)));
-                }
-                a0 = s01.x;
-                a1 = s01.y;
-                a2 = s23.x;
-                a3 = s23.y;
-              } else if (cb >= lo && cb + 16 <= hi) {
-                // partial tiles add up column by column, here without the comparisons
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                  a0 += fast_exp2(fmaf(__uint_as_float(r[hc * 16 + i]), c, -mref));
-              } else {
-#pragma unroll
-                for (int i = 0; i < 16; i++) {
-                  const int col = cb + i;
-                  if (col >= lo && col < hi)
-                    a0 += fast_exp2(fmaf(__uint_as_float(r[hc * 16 + i]), c, -mref));
-                }
-              }
-              acc += (a0 + a1) + (a2 + a3);
-              col_in_block += 16;
-              if (col_in_block == p.bsz) {
-                if (row_ok) out_row[j] = acc;
-                total += acc;
-                acc = 0.f;
-                col_in_block = 0;
-                j++;
-              }
-            }
-          }
+      auto flush = [&]() {   // block sums end on the 16-column grid
+        if (col_in_block == p.bsz) {
+          if (row_ok) out_row[j] = acc;
+          total += acc;
+          acc = 0.f;
+          col_in_block = 0;
+          j++;
         }
       };
       auto release = [&]() {
-        // the tile's last chunk is in registers: hand the accumulator back
+        // the tile's last columns are in registers: hand the accumulator back
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_aempty(a, half));
       };
-      if (full && ti.used == SC_KT) {
-        // full tile: the load of chunk k+1 is in flight while chunk k is summed
-        uint32_t ra[32], rb[32];
-        tmem_ld32(acc_addr, ra);
-        tmem_wait_ld();
-        tmem_ld32(acc_addr + 32, rb);
-        process(ra, 0, std::true_type{});
-        tmem_wait_ld();
-        tmem_ld32(acc_addr + 64, ra);
-        process(rb, 32, std::true_type{});
-        tmem_wait_ld();
-        tmem_ld32(acc_addr + 96, rb);
-        process(ra, 64, std::true_type{});
-        tmem_wait_ld();
+      if (pass == 1) {
+        run_max = fmaxf(run_max, tmem_row_max(acc_addr, ti.used, lo, hi));
         release();
-        process(rb, 96, std::true_type{});
-      } else {
-        for (int c0 = 0; c0 < ti.used; c0 += 32) {
-          uint32_t r[32];
-          tmem_ld32(acc_addr + static_cast<uint32_t>(c0), r);
+      } else if (full && ti.used == SC_KT) {
+        // Full tile: the next 16 columns are on their way while the last are summed.  Block
+        // sizes of whole 64s (`whole`) look for the end of a block only there.  With 32-column
+        // loads, a look every 16 columns and pass 1 in the same loop the exponentials ran at
+        // 0.94 of the special-function unit's rate without the wait for the UMMAs, now at all
+        // of it: N = 32768, H = 4 1239 -> 1200 us, 128-row blocks, N = 15000, H = 16 1135 ->
+        // 1090, N = 2000, H = 16 34.8 -> 30.7.
+        uint32_t ra[16], rb[16];
+        tmem_ld16(acc_addr, ra);
+#pragma unroll
+        for (int c0 = 0; c0 < SC_KT; c0 += 32) {
           tmem_wait_ld();
-          if (c0 + 32 >= ti.used) release();
-          process(r, c0, std::false_type{});
+          tmem_ld16(acc_addr + c0 + 16, rb);
+          const float t0 = sum16(ra, c, mref);
+          tmem_wait_ld();
+          if (c0 + 32 < SC_KT) tmem_ld16(acc_addr + c0 + 32, ra);
+          else release();
+          const float t1 = sum16(rb, c, mref);
+          acc += t0;
+          if (!whole) { col_in_block += 16; flush(); }
+          acc += t1;
+          if (!whole) { col_in_block += 16; flush(); }
+          else if (c0 & 32) { col_in_block += 64; flush(); }
+        }
+      } else {
+#pragma unroll 1
+        for (int c0 = 0; c0 < ti.used; c0 += 16) {
+          uint32_t r[16];
+          tmem_ld16(acc_addr + c0, r);
+          tmem_wait_ld();
+          if (c0 + 16 >= ti.used) release();
+          float t = 0.f;
+          if (full) {
+            t = sum16(r, c, mref);
+          } else if (c0 >= lo && c0 + 16 <= hi) {
+            // partial tiles add up column by column, here without the comparisons
+#pragma unroll
+            for (int i = 0; i < 16; i++) t += fast_exp2(fmaf(__uint_as_float(r[i]), c, -mref));
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+              const int col = c0 + i;
+              if (col >= lo && col < hi) t += fast_exp2(fmaf(__uint_as_float(r[i]), c, -mref));
+            }
+          }
+          acc += t;
+          col_in_block += 16;
+          flush();
         }
       }
     }

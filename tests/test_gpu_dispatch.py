@@ -582,3 +582,19 @@ def test_dq_goes_by_the_faster_kernel(ftk, N, H, W, groups):
         torch.cuda.synchronize()
     names = [e.key for e in prof.key_averages() if "sparse_bwd_dq_kernel" in e.key]
     assert len(names) == 1 and f"sparse_bwd_dq_kernel<64, {groups}>" in names[0], names
+
+
+@pytest.mark.parametrize("bsz", [16, 48, 64, 80, 128, 192])
+@pytest.mark.parametrize("D", [64, 128, 256])
+def test_score_blocks_end_on_and_off_the_64_column_grid(ftk, D, bsz):
+    """Full key tiles are asked for the end of a score block every 16 columns, or every 64 where
+    the block size is a multiple of that.  Bound: sums of up to 192 exponentials of 2 ulp whose
+    arguments, below 16, are rounded at 2^-21, and a row total of the same."""
+    N = 1152   # six blocks of 192, whole key tiles at the other sizes that divide 128
+    gen = torch.Generator().manual_seed(bsz + D)
+    q, k = (torch.randn(1, N, D, generator=gen).bfloat16() for _ in range(2))
+    pad = (0, -N % bsz)
+    want = orc.block_score(q.float().numpy(), k.float().numpy(), 1, bsz, pad)
+    got = ftk.flash_block_score(q.cuda(), k.cuda(), 1, bsz, pad).cpu().numpy()
+    ftk.check_errors()
+    np.testing.assert_allclose(got, want, rtol=5e-6, atol=0)
