@@ -420,7 +420,7 @@ __device__ __forceinline__ void store_rows(uint8_t* stage, const uint32_t (&pk)[
                                            int c0, int D, int fmt, bool f32) {
   constexpr int CH = NP / 4;             // 16-byte chunks of a row
   static_assert(CH == 2 || CH == 4, "");
-  const int lane = threadIdx.x & 31;
+  const int lane = late_tid() & 31;
   const int row0 = o.row0 + 32 * quarter, first = -row0, last = o.last - row0;
   uint8_t* out = static_cast<uint8_t*>(base) + (f32 ? 4 : 2) * (o.off[which] + row0 * stride);
   // chunk j of row r sits at j ^ flip(r): both sides use every bank once per eight lanes

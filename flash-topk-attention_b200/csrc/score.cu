@@ -28,7 +28,8 @@
 // (score_split).  All take the reference exponents from the first key tile, so their
 // block sums go out as they are; the row totals meet through the cluster's shared
 // memory.  A total is always added up from the same SC_SEGS parts of the keys, so it
-// does not depend on the split, bit for bit.
+// does not depend on the split, bit for bit.  Of a grid of several waves only the tiles of
+// the last one are split, in a launch of their own that fills the SMs as they become free.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -57,6 +58,9 @@ struct ScoreParams {
   int num_tiles;
   int fmt;                    // 0 fp16, 1 bf16
   int H, bh_begin;
+  int qtiles;                 // tiles of 256 query rows per slice
+  int tile0;                  // first tile of this launch
+  int behind;                 // runs beside the launch before it, which is part of the same call
   float scale_log2;           // log2(e) * softmax scale
   float* sums;                // [bh_count][N][M]   unnormalised block sums
   float* row_total;           // [bh_count][N]      L
@@ -143,8 +147,9 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int split = SPLIT ? static_cast<int>(cluster_nctas()) : 1,
             rank = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
-  const int q0 = static_cast<int>(blockIdx.x) / split * SC_QROWS;
-  const int bh_local = blockIdx.y;
+  const int tile = p.tile0 + static_cast<int>(blockIdx.x) / split;
+  const int bh_local = tile / p.qtiles;
+  const int q0 = (tile - bh_local * p.qtiles) * SC_QROWS;
   const int bh = p.bh_begin + bh_local;
   const int b_idx = bh / p.H, h_idx = bh - b_idx * p.H;
 
@@ -195,7 +200,10 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
   const int t_first = SPLIT ? seg_begin(p, seg_first) : 0,
             L = SPLIT ? seg_begin(p, seg_last) - t_first : p.num_tiles;
   float mref = 0.f;    // softmax threads: the row's reference exponent
-  pdl_wait();
+  // The second launch of a call starts when every block of the first one is past its wait, so
+  // what came before the call is there.  It waits for the first one at its end: whoever
+  // waits for this launch wants the results of both.
+  if (!p.behind) pdl_wait();
   pdl_launch();
 
   // Pass 0 is all there is unless a row total overflows.  Every barrier's
@@ -477,6 +485,7 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
     for (int i = 0; i < 200; i++) __nanosleep(1000);
   }
   if (warp == 0) tmem_dealloc(tmem, 512);
+  if (p.behind) pdl_wait();
 }
 
 // block_scores[r][j] = sums[r][j] / total[r]
@@ -497,17 +506,23 @@ __global__ void score_normalize_kernel(const float* __restrict__ sums,
 // and meet the others (512 tiles of 64 steps, D = 64: 4 waves unsplit 465 us, 7 waves of
 // halves 476); the number of clusters that run at once is what the device says.
 // 61 tiles of 122 steps: 203 -> 127 us with select, 32 of 32 steps: 59 -> 32 us.
+// A grid of several waves leaves its last one as it is where that is full or nearly so; else
+// its tiles are split like a small grid's, when that saves a tenth of the wave and three key tiles
+// (a launch more for the host).
+struct ScoreSplit {
+  int cluster;   // CTAs per tile
+  int tail;      // tiles of the last wave that are split, 0: none
+  int tail_cluster;
+};
 template <int D>
-static int score_split(int64_t tiles, int num_tiles, int units, size_t smem) {
+static ScoreSplit score_split(int64_t tiles, int num_tiles, int units, size_t smem) {
   constexpr int MAX_DEVICES = 64;
   static std::atomic<int> resident[MAX_DEVICES][4];   // clusters of 1, 2, 4, 8
+  ScoreSplit best = {1, 0, 1};
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return 1;
-  int best = 1;
-  double best_cost = 0.;
-  for (int i = 0; i < 4; i++) {
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return best;
+  auto clusters = [&](int i) {
     const int c = 1 << i;
-    if (c > units) break;
     int n = resident[dev][i].load(std::memory_order_relaxed);
     if (n == 0) {
       n = c == 1 ? sm_count()
@@ -516,12 +531,32 @@ static int score_split(int64_t tiles, int num_tiles, int units, size_t smem) {
                        : 0;
       resident[dev][i].store(n > 0 ? n : -1, std::memory_order_relaxed);
     }
-    if (n <= 0) continue;
-    const double waves = static_cast<double>((tiles + n - 1) / n);
-    const double cost = waves * (static_cast<double>(num_tiles) / c + (c > 1 ? 7.5 : 3.5));
-    if (i == 0 || cost < 0.95 * best_cost) {
-      best = c;
-      best_cost = cost;
+    return n;
+  };
+  auto cost = [&](int64_t t, int i) {
+    const int n = clusters(i), c = 1 << i;
+    if (n <= 0) return 1e30;
+    const double waves = static_cast<double>((t + n - 1) / n);
+    return waves * (static_cast<double>(num_tiles) / c + (c > 1 ? 7.5 : 3.5));
+  };
+  double best_cost = cost(tiles, 0);
+  for (int i = 1; i < 4 && (1 << i) <= units; i++) {
+    const double x = cost(tiles, i);
+    if (x < 0.95 * best_cost) {
+      best.cluster = 1 << i;
+      best_cost = x;
+    }
+  }
+  const int n = clusters(0);
+  if (best.cluster > 1 || n <= 0 || tiles <= n || tiles % n == 0) return best;
+  const double wave = num_tiles + 3.5;
+  best_cost = std::min(0.9 * wave, wave - 3.);
+  for (int i = 1; i < 4 && (1 << i) <= units; i++) {
+    const double x = cost(tiles % n, i);
+    if (x < best_cost) {
+      best.tail = static_cast<int>(tiles % n);
+      best.tail_cluster = 1 << i;
+      best_cost = x;
     }
   }
   return best;
@@ -534,14 +569,21 @@ static int launch_score_d(const CUtensorMap& tq, const CUtensorMap& tk, ScorePar
   const size_t smem =
       1024 + (2 * NCH + score_stages(D) * (NCH / score_ksplit(D))) * SC_CHUNK_BYTES;
   if (int e = allow_smem<score_kernel<D, false>>(smem)) return e;
-  const int qtiles = (p.N + SC_QROWS - 1) / SC_QROWS;
-  const int split = score_split<D>(qtiles * bh_count, p.num_tiles,
-                                   p.num_tiles / std::max(1, p.tiles_per_block), smem);
-  const dim3 grid(qtiles * split, static_cast<unsigned>(bh_count));
-  if (split == 1)
-    return launch_pdl(score_kernel<D, false>, grid, SC_THREADS, smem, st, tq, tk, p);
-  if (int e = allow_smem<score_kernel<D, true>>(smem)) return e;
-  return launch_clusters(score_kernel<D, true>, split, grid, SC_THREADS, smem, st, tq, tk, p);
+  p.qtiles = (p.N + SC_QROWS - 1) / SC_QROWS;
+  const int64_t tiles = p.qtiles * bh_count;
+  if (8 * tiles > 0x7fffffffLL) return FTK_ERR_BAD_ARG;
+  const ScoreSplit split = score_split<D>(tiles, p.num_tiles, p.num_tiles / std::max(1, p.tiles_per_block), smem);
+  const unsigned first = static_cast<unsigned>(tiles - split.tail);
+  auto clusters = [&](unsigned n, int c) {
+    if (int e = allow_smem<score_kernel<D, true>>(smem)) return e;
+    return launch_clusters(score_kernel<D, true>, c, dim3(n * c), SC_THREADS, smem, st, tq, tk, p);
+  };
+  if (split.cluster > 1) return clusters(first, split.cluster);
+  if (int e = launch_pdl(score_kernel<D, false>, dim3(first), SC_THREADS, smem, st, tq, tk, p)) return e;
+  if (split.tail == 0) return FTK_OK;
+  p.tile0 = static_cast<int>(first);
+  p.behind = 1;
+  return clusters(split.tail, split.tail_cluster);
 }
 
 struct ScoreWs {

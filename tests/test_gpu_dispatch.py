@@ -598,3 +598,23 @@ def test_score_blocks_end_on_and_off_the_64_column_grid(ftk, D, bsz):
     got = ftk.flash_block_score(q.cuda(), k.cuda(), 1, bsz, pad).cpu().numpy()
     ftk.check_errors()
     np.testing.assert_allclose(got, want, rtol=5e-6, atol=0)
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("hot", [False, True])
+def test_score_tiles_of_the_last_wave(ftk, D, hot):
+    """192 tiles of 256 rows: those behind the last full wave of 148 SMs are split over clusters
+    in a launch of their own, also where rows overflow there and the keys are walked again.
+    Same bits as one head at a time, which is a grid of eight tiles."""
+    H, N, bsz = 24, 2048, 64
+    gen = torch.Generator().manual_seed(D)
+    q, k = (torch.randn(1, N, H, D, generator=gen).half() for _ in range(2))
+    if hot:
+        k[:, 300:, 20:] *= 40.0
+        q[:, 1800:, 20:] *= 3.0
+    q, k = q.cuda(), k.cuda()
+    got = ftk.flash_block_score(q.view(1, N, H * D), k.view(1, N, H * D), H, bsz, (0, 0))
+    for h in range(H):
+        one = ftk.flash_block_score(q[:, :, h].contiguous(), k[:, :, h].contiguous(), 1, bsz, (0, 0))
+        assert torch.equal(got[:, h], one[:, 0])
+    ftk.check_errors()
