@@ -377,6 +377,12 @@ __device__ __forceinline__ CoverTiles cover_tiles(const UnionScratch& u, int n, 
   return c;
 }
 
+// Head dims between the kernels' own, of which D columns are there: the k-steps of 16 columns
+// that a product over the head dim has, and the columns that a product of M = 256 across two CTAs
+// yields (multiples of 32).  The others are zeros, or are not stored.
+__device__ __forceinline__ int used_ksteps(int D) { return (D + 15) >> 4; }
+__device__ __forceinline__ int used_columns(int D) { return (D + 31) & ~31; }
+
 // Where a CTA's results go: worked out by one thread ahead of the loop over the tiles and
 // kept in shared memory until the end of it, where a warp also asks for its number anew.
 // Held in registers all along, they cost the loop's warps, which have 96, a few percent.

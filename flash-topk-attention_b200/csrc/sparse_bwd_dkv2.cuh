@@ -153,7 +153,7 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
   if (warp == 0) {
     // ------------------------------------------------------- TMA producer
     if (lane == 0 && n > 0) {
-      const int dcol = 64 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
+      const int dcol = used_columns(p.D) / 2 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
       HeadWalk<WALK> hw;
       for (int i = 0; i < n; i++) {
         const int s = i % DK2_STAGES;
@@ -188,7 +188,8 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     // ----------------------------- CTA 0: UMMA issuer for the CTA pair
     if (n > 0) {
       const uint32_t idesc_a = umma_idesc(256, G, FMT, 0, 0);
-      const uint32_t idesc_b = umma_idesc(256, D, FMT, 0, 1);
+      const uint32_t idesc_b = umma_idesc(256, used_columns(p.D), FMT, 0, 1);
+      const int ksteps = used_ksteps(p.D);
       const uint64_t kdesc0 = smem_desc_sw128(smem_u32(sK), 16, 1024);
       const uint64_t vdesc0 = smem_desc_sw128(smem_u32(sV), 16, 1024);
       const uint64_t rowdesc0 = smem_desc_sw128(smem_u32(sQD), 16, 1024);
@@ -212,15 +213,16 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
         for (int ks = 0; ks < D / 16; ks++) {
           const uint32_t aoff = (ks / 4) * 128 * 128 + (ks % 4) * 32;
           const uint32_t boff = (ks / 4) * 4096 + (ks % 4) * 32;
-          umma2_ss(tmem + sb * 64, desc_advance(kdesc0, aoff), desc_advance(qdesc, boff), idesc_a,
-                   ks > 0);
+          if (ks < ksteps)
+            umma2_ss(tmem + sb * 64, desc_advance(kdesc0, aoff), desc_advance(qdesc, boff), idesc_a, ks > 0);
         }
 #pragma unroll
         for (int ks = 0; ks < D / 16; ks++) {
           const uint32_t aoff = (ks / 4) * 128 * 128 + (ks % 4) * 32;
           const uint32_t boff = (ks / 4) * 4096 + (ks % 4) * 32;
-          umma2_ss(tmem + 128 + sb * 64, desc_advance(vdesc0, aoff), desc_advance(dodesc, boff),
-                   idesc_a, ks > 0);
+          if (ks < ksteps)
+            umma2_ss(tmem + 128 + sb * 64, desc_advance(vdesc0, aoff), desc_advance(dodesc, boff), idesc_a,
+                     ks > 0);
         }
         umma2_commit(bar_afull(sb), 3);
       };

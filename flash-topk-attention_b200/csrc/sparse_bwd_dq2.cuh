@@ -136,7 +136,7 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
     // ------------------------------------------------------- TMA producer
     if (lane == 0 && n == 0) mbar_wait(bar_q, 0, w, FTK_DEV_TIMEOUT_TMA);   // lands before the exit
     if (lane == 0 && n > 0) {
-      const int dcol = 64 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
+      const int dcol = used_columns(p.D) / 2 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
       const int hk = h_idx / p.kv_hdiv;
       for (int i = 0; i < n; i++) {
         const int s = i % DQ2_STAGES;
@@ -164,7 +164,8 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
     // ----------------------------- CTA 0: UMMA issuer for the CTA pair
     if (n > 0) {
       const uint32_t idesc_a = umma_idesc(256, G, FMT, 0, 0);
-      const uint32_t idesc_b = umma_idesc(256, D, FMT, 0, 1);
+      const uint32_t idesc_b = umma_idesc(256, used_columns(p.D), FMT, 0, 1);
+      const int ksteps = used_ksteps(p.D);
       const uint64_t rowdesc0 = smem_desc_sw128(smem_u32(sKV), 16, 1024);
       const uint64_t coldesc0 = smem_desc_sw128(smem_u32(sKV) + OFF_KCOL, 8192, 1024);
       bool ok = mbar_wait(bar_qt, 0, w, FTK_DEV_TIMEOUT_MMA);
@@ -181,12 +182,14 @@ sparse_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q,
         const uint32_t sb = i & 1;
 #pragma unroll
         for (int ks = 0; ks < D / 16; ks++)
-          umma2_ts(tmem + 128 + sb * 64, tmem + ks * 8,
-                   desc_advance(kdesc, (ks / 4) * 4096 + (ks % 4) * 32), idesc_a, ks > 0);
+          if (ks < ksteps)
+            umma2_ts(tmem + 128 + sb * 64, tmem + ks * 8,
+                     desc_advance(kdesc, (ks / 4) * 4096 + (ks % 4) * 32), idesc_a, ks > 0);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ks++)
-          umma2_ts(tmem + 256 + sb * 64, tmem + 64 + ks * 8,
-                   desc_advance(vdesc, (ks / 4) * 4096 + (ks % 4) * 32), idesc_a, ks > 0);
+          if (ks < ksteps)
+            umma2_ts(tmem + 256 + sb * 64, tmem + 64 + ks * 8,
+                     desc_advance(vdesc, (ks / 4) * 4096 + (ks % 4) * 32), idesc_a, ks > 0);
         umma2_commit(bar_afull(sb), 3);
       };
       auto mma_b = [&](int i) {   // elected lane only

@@ -618,3 +618,23 @@ def test_score_tiles_of_the_last_wave(ftk, D, hot):
         one = ftk.flash_block_score(q[:, :, h].contiguous(), k[:, :, h].contiguous(), 1, bsz, (0, 0))
         assert torch.equal(got[:, h], one[:, 0])
     ftk.check_errors()
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("D", [72, 96, 104, 120])
+def test_head_dims_below_128_on_pairs(ftk, D, dtype):
+    """Wide lists: the backward's pair kernels leave out the k-steps and columns that are
+    padding of the head dim.  Same bits as with the padding written out as zeros."""
+    H, N, g = 3, 700, 64
+    t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype=dtype, seed=D, do_seed=D + 1))
+    M = -(-N // g)
+    lists = np.tile(np.arange(M, dtype=np.int32), (1, H, M, 1))
+    lists[0, 1, 3:, 2:] = -1
+    pads = dict(q_padding=(0, M * g - N), kv_padding=(0, M * g - N), scale=D ** -0.5)
+    got = _grads(ftk, t, lists, H, g, g, **pads)
+    wide = {k: torch.nn.functional.pad(x.view(1, N, H, D), (0, 128 - D)).reshape(1, N, H * 128)
+            for k, x in t.items()}
+    want = _grads(ftk, wide, lists, H, g, g, **pads)
+    assert torch.equal(got[1], want[1])
+    for i in (0, 2, 3, 4):
+        assert torch.equal(got[i].view(1, N, H, D), want[i].view(1, N, H, 128)[..., :D])
