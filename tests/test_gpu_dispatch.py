@@ -638,3 +638,35 @@ def test_head_dims_below_128_on_pairs(ftk, D, dtype):
     assert torch.equal(got[1], want[1])
     for i in (0, 2, 3, 4):
         assert torch.equal(got[i].view(1, N, H, D), want[i].view(1, N, H, 128)[..., :D])
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("at", [64 + 0, 64 + 1, 64 + 2, 64 + 9])
+@pytest.mark.parametrize("what", [float("nan"), float("inf"), 3.0e4])
+def test_forward_values_that_are_no_probabilities(ftk, monkeypatch, dtype, at, what):
+    """Head dim 64, where columns 0, 1 of every 8 go over the FMA pipe: a key of NaN or infinities,
+    or one that overflows, sends its tile to the exact kernel whichever column it stands in; the
+    rows whose logit of it is as far below are as if it was not there.  Bound of the latter: two
+    roundings of P and of O."""
+    H, N, D, g = 2, 512, 64, 64
+    t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype=dtype, seed=91, do_seed=92))
+    t["q"].view(1, N, H, D)[..., 0] = 1.0
+    t["q"].view(1, N, H, D)[:, 300:, :, 0] = -1.0   # rows 300 on: -inf, or far below
+    key = t["k"].view(1, N, H, D)[:, at]
+    key.zero_()
+    key[..., 0] = what
+    merged = np.tile(np.arange(N // g, dtype=np.int32), (1, H, N // g, 1))
+    args = [t[n].cuda() for n in "qkv"] + [torch.from_numpy(merged).cuda(), None, H, g, g]
+    o, lse = ftk.flash_topk_attn(*args)
+    monkeypatch.setenv("FTK_FWD_PIPE", "0")
+    want, lse_want = ftk.flash_topk_attn(*args)
+    ftk.check_errors()
+    rows = slice(None, 256)   # the tiles of these rows all overflow
+    for x, y in ((o[:, rows], want[:, rows]), (lse[..., rows], lse_want[..., rows])):
+        assert torch.equal(torch.isnan(x), torch.isnan(y))
+        assert torch.equal(torch.nan_to_num(x), torch.nan_to_num(y))
+    eps = 2.0 ** -10 if dtype == "fp16" else 2.0 ** -7
+    if what == 3.0e4:
+        assert torch.isfinite(o[:, 384:]).all()
+        bound = 2 * eps * want[:, 384:].abs().float() + 2 * eps
+        assert ((o[:, 384:].float() - want[:, 384:].float()).abs() <= bound).all()
