@@ -523,7 +523,7 @@ __global__ void score_normalize_kernel(const float* __restrict__ sums,
 // 61 tiles of 122 steps: 203 -> 127 us with select, 32 of 32 steps: 59 -> 32 us.
 // A grid of several waves leaves its last one as it is where that is full or nearly so; else
 // its tiles are split like a small grid's, when that saves a tenth of the wave and three key tiles
-// (a launch more for the host).
+// (a launch more for the host), or more than splitting all tiles does.
 struct ScoreSplit {
   int cluster;   // CTAs per tile
   int tail;      // tiles of the last wave that are split, 0: none
@@ -563,14 +563,13 @@ static ScoreSplit score_split(int64_t tiles, int num_tiles, int units, size_t sm
     }
   }
   const int n = clusters(0);
-  if (best.cluster > 1 || n <= 0 || tiles <= n || tiles % n == 0) return best;
-  const double wave = num_tiles + 3.5;
-  best_cost = std::min(0.9 * wave, wave - 3.);
+  if (n <= 0 || tiles <= n || tiles % n == 0) return best;
+  const double wave = num_tiles + 3.5, full = static_cast<double>(tiles / n) * wave;
+  if (best.cluster == 1) best_cost = full + std::min(0.9 * wave, wave - 3.);
   for (int i = 1; i < 4 && (1 << i) <= units; i++) {
-    const double x = cost(tiles % n, i);
+    const double x = full + cost(tiles % n, i);
     if (x < best_cost) {
-      best.tail = static_cast<int>(tiles % n);
-      best.tail_cluster = 1 << i;
+      best = {1, static_cast<int>(tiles % n), 1 << i};
       best_cost = x;
     }
   }
