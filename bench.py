@@ -75,7 +75,7 @@ UNIT = "tokens/s"
 # (profiles/dram_traffic_n32768_h4.txt).  Every kernel works on (batch, head) slices
 # independently, so a launch over B*H slices of this sequence length moves B*H times this.
 DRAM_BYTES_PER_SLICE_N32768 = {
-    "ftk_score_topk": (75.9e6 + 221.6e6 + 269.0e6 + 36.8e6) / 4,
+    "ftk_score_topk": (92.1e6 + 186.9e6 + 269.0e6 + 36.3e6) / 4,   # scoring in two launches
     "ftk_qblock_merge": 33.6e6 / 4,            # what it writes is still in L2 at its end
     "ftk_sparse_fwd": (118.7e6 + 18.5e6) / 4,
     "ftk_sparse_bwd_dq": (188.4e6 + 22.0e6) / 4,
