@@ -56,34 +56,6 @@ __device__ __forceinline__ uint32_t pack16(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-__device__ __forceinline__ float2 exp2_pair(float2 t) { return make_float2(fast_exp2(t.x), fast_exp2(t.y)); }
-
-// 2^t of two values on the FMA pipe.  Adding 1.5 * 2^23 leaves n = round(t) in the low bits,
-// 2^(t - n) on [-1/2, 1/2] is a polynomial (least maximum of the relative error, 7.5e-8; the
-// special-function unit's is of the same size) and n goes into its exponent.  t is held to
-// -126 .. 128: below, the result is a denormal number; above, it passes every bound for the exact
-// kernel, as does a NaN, which comes out as 3.4e38.
-// With two CTAs per SM the forward at head dim 64 runs at 0.80 of the special-function unit's
-// rate.  One of four exponentials here: N = 8192, H = 16, all pairs 337 us with none, 327 with
-// one of eight, 318 with one of four, 345 with one of three (issue slots).  At head dim 128
-// the chain through one tile counts, and any share is slower (pairs of SMs: 798 -> 833 us).
-__device__ __forceinline__ float2 exp2_pair_fma(float2 t) {
-  asm("max.NaN.f32 %0, %0, %1;\n\tmin.NaN.f32 %0, %0, %2;" : "+f"(t.x) : "f"(-126.f), "f"(128.f));
-  asm("max.NaN.f32 %0, %0, %1;\n\tmin.NaN.f32 %0, %0, %2;" : "+f"(t.y) : "f"(-126.f), "f"(128.f));
-  const float magic = 12582912.f;
-  const float2 n = __fadd2_rn(t, make_float2(magic, magic));
-  const float2 f = __ffma2_rn(__fadd2_rn(n, make_float2(-magic, -magic)), make_float2(-1.f, -1.f), t);
-  auto step = [&](float2 y, float a) { return __ffma2_rn(y, f, make_float2(a, a)); };
-  float2 y = make_float2(0.00132764713f, 0.00132764713f);
-  y = step(y, 0.00967554096f);
-  y = step(y, 0.0555071309f);
-  y = step(y, 0.240221202f);
-  y = step(y, 0.693146944f);
-  y = step(y, 1.00000012f);
-  return make_float2(__uint_as_float((__float_as_uint(n.x) << 23) + __float_as_uint(y.x)),
-                     __uint_as_float((__float_as_uint(n.y) << 23) + __float_as_uint(y.y)));
-}
-
 template <int D, int FMT, int SUB, int NG>
 __global__ void __launch_bounds__(fp_threads(NG), 4 / NG)
 sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
@@ -98,7 +70,6 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
   constexpr int COL_S = D / 2, COL_O = COL_S + 64 * NG;   // Q in the columns before S
   constexpr int TMEM_COLS = NG == 2 ? 256 : 512;
   static_assert(COL_O + D <= TMEM_COLS, "TMEM columns");
-  constexpr bool POLY = NG == 2;               // some exponentials on the FMA pipe
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -373,7 +344,7 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
           for (int x = 0; x < 32; x += 2) {
             const float2 t = __ffma2_rn(
                 make_float2(__uint_as_float(v0[x]), __uint_as_float(v0[x + 1])), c2, nm);
-            const float2 e = POLY && x % 8 == 0 ? exp2_pair_fma(t) : exp2_pair(t);
+            const float2 e = make_float2(fast_exp2(t.x), fast_exp2(t.y));
             acc = __fadd2_rn(acc, e);
             pk[x >> 1] = pack16<FMT>(e.x, e.y);
           }
@@ -382,7 +353,7 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
           for (int x = 0; x < 32; x += 2) {
             const float2 t = __ffma2_rn(
                 make_float2(__uint_as_float(v1[x]), __uint_as_float(v1[x + 1])), c2, nm);
-            const float2 e = POLY && x % 8 == 0 ? exp2_pair_fma(t) : exp2_pair(t);
+            const float2 e = make_float2(fast_exp2(t.x), fast_exp2(t.y));
             acc = __fadd2_rn(acc, e);
             pk[x >> 1] = pack16<FMT>(e.x, e.y);
           }

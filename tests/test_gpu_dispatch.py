@@ -644,10 +644,9 @@ def test_head_dims_below_128_on_pairs(ftk, D, dtype):
 @pytest.mark.parametrize("at", [64 + 0, 64 + 1, 64 + 2, 64 + 9])
 @pytest.mark.parametrize("what", [float("nan"), float("inf"), 3.0e4])
 def test_forward_values_that_are_no_probabilities(ftk, monkeypatch, dtype, at, what):
-    """Head dim 64, where columns 0, 1 of every 8 go over the FMA pipe: a key of NaN or infinities,
-    or one that overflows, sends its tile to the exact kernel whichever column it stands in; the
-    rows whose logit of it is as far below are as if it was not there.  Bound of the latter: two
-    roundings of P and of O."""
+    """A key of NaN or infinities, or one that overflows, sends its tile to the exact kernel
+    whichever column it stands in; the rows whose logit of it is as far below are as if it was
+    not there.  Bound of the latter: two roundings of P and of O."""
     H, N, D, g = 2, 512, 64, 64
     t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype=dtype, seed=91, do_seed=92))
     t["q"].view(1, N, H, D)[..., 0] = 1.0
@@ -670,3 +669,37 @@ def test_forward_values_that_are_no_probabilities(ftk, monkeypatch, dtype, at, w
         assert torch.isfinite(o[:, 384:]).all()
         bound = 2 * eps * want[:, 384:].abs().float() + 2 * eps
         assert ((o[:, 384:].float() - want[:, 384:].float()).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("D,g,W", [(32, 64, 8), (64, 64, 8), (64, 64, 3), (64, 32, 16), (128, 64, 3),
+                                   (128, 64, 8), (256, 64, 8)])
+def test_rows_without_a_finite_logit(ftk, monkeypatch, dtype, D, g, W):
+    """Query rows whose logits are all -inf (full tiles, and the last one, which is not): O = 0
+    and lse = -inf, as from the exact kernel.  The rows beside them are not touched by that.
+    Bound of those: P and O, below 4, are rounded in both kernels, at different references."""
+    H, N = 2, 500
+    M = -(-N // g)
+    t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype=dtype, seed=93, do_seed=94))
+    t["k"].view(1, N, H, D)[..., 0] = 1.0
+    gone = torch.zeros(N, dtype=torch.bool)
+    gone[[0, 7, 63, 200, 499]] = True
+    gone[64:128] = True
+    t["q"].view(1, N, H, D)[:, gone, :, 0] = -float("inf")
+    lists = np.full((1, H, M, W), -1, np.int32)
+    for m in range(M):
+        lists[:, :, m] = np.sort((np.arange(W) + m) % M)
+    pads = dict(q_padding=(0, M * g - N), kv_padding=(0, M * g - N))
+    args = [t[n].cuda() for n in "qkv"] + [torch.from_numpy(lists).cuda(), None, H, g, g]
+    o, lse = ftk.flash_topk_attn(*args, **pads)
+    monkeypatch.setenv("FTK_FWD_PIPE", "0")
+    o2, lse2 = ftk.flash_topk_attn(*args, **pads)
+    ftk.check_errors()
+    gone = gone.cuda()
+    for x, y in ((o, lse), (o2, lse2)):
+        assert not x[:, gone].any()
+        assert (y[..., gone] == -float("inf")).all()
+    eps = 2.0 ** -10 if dtype == "fp16" else 2.0 ** -7
+    assert torch.isfinite(o[:, ~gone]).all()
+    assert (o - o2)[:, ~gone].abs().max().item() <= 4 * 2 * eps
+    torch.testing.assert_close(lse[..., ~gone], lse2[..., ~gone], rtol=1e-6, atol=1e-6)
