@@ -397,37 +397,30 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
         // 0.94 of the special-function unit's rate without the wait for the UMMAs, now at all
         // of it: N = 32768, H = 4 1239 -> 1200 us, 128-row blocks, N = 15000, H = 16 1135 ->
         // 1090, N = 2000, H = 16 34.8 -> 30.7.
-        if constexpr (D > 128) {
-          // The tensor core bounds head dim 256, and loads ahead of need get in its way:
-          // N = 8192, H = 16 419 -> 409 us without them.
+        uint32_t ra[16], rb[16];
+        if constexpr (D <= 128) tmem_ld16(acc_addr, ra);
 #pragma unroll
-          for (int c0 = 0; c0 < SC_KT; c0 += 16) {
-            uint32_t r[16];
-            tmem_ld16(acc_addr + c0, r);
-            tmem_wait_ld();
-            if (c0 + 16 == SC_KT) release();
-            acc += sum16(r, c, mref);
-            col_in_block += 16;
-            if (!whole || (c0 & 63) == 48) flush();
-          }
-        } else {
-          uint32_t ra[16], rb[16];
-          tmem_ld16(acc_addr, ra);
-#pragma unroll
-          for (int c0 = 0; c0 < SC_KT; c0 += 32) {
-            tmem_wait_ld();
-            tmem_ld16(acc_addr + c0 + 16, rb);
-            const float t0 = sum16(ra, c, mref);
+        for (int c0 = 0; c0 < SC_KT; c0 += 32) {
+          // The tensor core bounds head dim 256, and loads ahead of need get in its way: 32
+          // columns at a time there.  With select, N = 8192, H = 16, blocks of 64 keys: 507 us with
+          // 32 columns ahead, 483 with 16 at a time, 476 so; H = 8, blocks of 32: 319, 306, 292.
+          if constexpr (D > 128) tmem_ld16(acc_addr + c0, ra);
+          else tmem_wait_ld();
+          tmem_ld16(acc_addr + c0 + 16, rb);
+          if constexpr (D > 128) tmem_wait_ld();
+          if (D > 128 && c0 + 32 == SC_KT) release();
+          const float t0 = sum16(ra, c, mref);
+          if constexpr (D <= 128) {
             tmem_wait_ld();
             if (c0 + 32 < SC_KT) tmem_ld16(acc_addr + c0 + 32, ra);
             else release();
-            const float t1 = sum16(rb, c, mref);
-            acc += t0;
-            if (!whole) { col_in_block += 16; flush(); }
-            acc += t1;
-            if (!whole) { col_in_block += 16; flush(); }
-            else if (c0 & 32) { col_in_block += 64; flush(); }
           }
+          const float t1 = sum16(rb, c, mref);
+          acc += t0;
+          if (!whole) { col_in_block += 16; flush(); }
+          acc += t1;
+          if (!whole) { col_in_block += 16; flush(); }
+          else if (c0 & 32) { col_in_block += 64; flush(); }
         }
       } else {
 #pragma unroll 1
