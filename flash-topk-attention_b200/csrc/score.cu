@@ -422,6 +422,26 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
           if (!whole) { col_in_block += 16; flush(); }
           else if (c0 & 32) { col_in_block += 64; flush(); }
         }
+      } else if (D == 128 && full) {
+        // Blocks that leave columns of the tile blank, 32 columns per wait: N = 8192, H = 8 with
+        // select 288 -> 263 us for blocks of 48 keys, 274 -> 253 of 80.  At the other head dims a
+        // wait per 16 columns was not the slower one (64: 253 us, 256 with 32; 256: 357, 362).
+#pragma unroll 1
+        for (int c0 = 0; c0 < ti.used; c0 += 32) {
+          uint32_t ra[16], rb[16];
+          tmem_ld16(acc_addr + c0, ra);
+          tmem_ld16(acc_addr + c0 + 16, rb);   // the accumulator's own columns in any case
+          tmem_wait_ld();
+          if (c0 + 32 >= ti.used) release();
+          acc += sum16(ra, c, mref);
+          col_in_block += 16;
+          flush();
+          if (c0 + 16 < ti.used) {
+            acc += sum16(rb, c, mref);
+            col_in_block += 16;
+            flush();
+          }
+        }
       } else {
 #pragma unroll 1
         for (int c0 = 0; c0 < ti.used; c0 += 16) {
