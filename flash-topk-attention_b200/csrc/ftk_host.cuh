@@ -131,7 +131,8 @@ inline int launched(cudaError_t e, int kernels = 1) {
 }
 
 // Launch that may overlap the tail of the stream's previous kernel.  Only for
-// kernels that call pdl_wait() in every block before they touch global memory.
+// kernels that call pdl_wait() in every block before they touch global memory; the one
+// launch that does so later is described at pdl_wait().
 template <typename... Params, typename... Args>
 inline int launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
                       cudaStream_t st, const Args&... args) {

@@ -46,6 +46,12 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // without a limit.  What the predecessor may have written is read with plain loads:
 // read-only ones (__ldg, const __restrict__ parameters) are defined only for memory
 // that nobody writes during the kernel's life, which begins before that wait.
+// One launch waits at its end instead, in every block all the same: the second scoring
+// launch of a call (score_kernel, `behind`).  That is sound only because the launch directly
+// before it is the first one of the same call, which waits before it allows a successor (so
+// everything before the call is complete and visible by then), and because neither of the two
+// reads or writes what the other one writes.  The wait at the end keeps the chain: a kernel that
+// waits for the second launch finds the first one complete as well.
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

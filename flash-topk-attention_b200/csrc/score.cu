@@ -202,7 +202,8 @@ score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
   float mref = 0.f;    // softmax threads: the row's reference exponent
   // The second launch of a call starts when every block of the first one is past its wait, so
   // what came before the call is there.  It waits for the first one at its end: whoever
-  // waits for this launch wants the results of both.
+  // waits for this launch wants the results of both.  The wait must stand ahead of the trigger
+  // (see pdl_wait()).
   if (!p.behind) pdl_wait();
   pdl_launch();
 

@@ -64,6 +64,35 @@ def test_tmem_is_allocated_before_the_next_kernel_may_start(name):
         assert re.search(barrier, body[alloc:first]), "no barrier between allocation and trigger"
 
 
+@pytest.mark.parametrize("name", OVERLAPPED)
+def test_kernels_wait_before_their_successor_may_start(name):
+    """A successor may rely on its predecessor's predecessor: where a kernel waits for the one
+    before it first and only then allows the next one, that is over."""
+    body = KERNELS[name]
+    trigger = re.search(r"pdl_launch\(\)|dkv_union\(", body)
+    assert trigger and "pdl_wait()" in body[:trigger.start()]
+    if name != "score_kernel":
+        assert not re.search(r"if \(!?p\.\w+\) pdl_wait", body), "a wait that a launch may leave out"
+
+
+def test_the_launch_that_waits_at_its_end():
+    """The second scoring launch of a call touches memory before it waits.  Its predecessor has
+    to be the first one, which waits ahead of its trigger, and each of its own blocks has to wait
+    all the same, as the last thing that it does."""
+    body = KERNELS["score_kernel"]
+    assert re.findall(r"[^\n;{}]*pdl_wait\(\)", body) == ["  if (!p.behind) pdl_wait()",
+                                                        "  if (p.behind) pdl_wait()"]
+    assert re.search(r"if \(!p\.behind\) pdl_wait\(\);\s*pdl_launch\(\);", body)
+    assert re.search(r"if \(p\.behind\) pdl_wait\(\);\s*\}\s*$", body)
+    assert not re.search(r"\breturn;", body), "a block that leaves early breaks the chain"
+    text = "".join(re.sub(r"//[^\n]*", "", open(f).read()) for f in glob.glob(os.path.join(CSRC, "*.cu*")))
+    assert len(re.findall(r"\bbehind\b", text)) == 4   # the field, the two waits, one launch
+    host = re.search(r"launch_pdl\(score_kernel<D, false>[^;]*;(.*?)p\.behind = 1;\s*return clusters\(", text,
+                     re.S)
+    assert host and re.sub(r"\s+", " ", host.group(1)).strip() == (
+        "if (split.tail == 0) return FTK_OK; p.tile0 = static_cast<int>(first);")
+
+
 def test_no_read_only_loads_in_overlapped_kernels():
     """ld.global.nc (__ldg, const __restrict__ parameters) is defined only for memory that
     does not change during the kernel's life; an overlapped kernel's inputs are written by
