@@ -604,20 +604,67 @@ def test_score_blocks_end_on_and_off_the_64_column_grid(ftk, D, bsz):
 @pytest.mark.parametrize("hot", [False, True])
 def test_score_tiles_of_the_last_wave(ftk, D, hot):
     """192 tiles of 256 rows: those behind the last full wave of 148 SMs are split over clusters
-    in a launch of their own, also where rows overflow there and the keys are walked again.
-    Same bits as one head at a time, which is a grid of eight tiles."""
-    H, N, bsz = 24, 2048, 64
+    in a launch of their own (a launch more than one head at a time, a grid of 16 tiles), also
+    where rows overflow there and the keys are walked again.  Same bits as one head at a time."""
+    from flash_topk_attn_v2 import ops
+    H, N, bsz = 12, 4096, 64
     gen = torch.Generator().manual_seed(D)
     q, k = (torch.randn(1, N, H, D, generator=gen).half() for _ in range(2))
     if hot:
-        k[:, 300:, 20:] *= 40.0
-        q[:, 1800:, 20:] *= 3.0
+        k[:, 300:, 10:] *= 40.0
+        q[:, 1800:, 10:] *= 3.0
     q, k = q.cuda(), k.cuda()
+    before = ops.launch_count()
     got = ftk.flash_block_score(q.view(1, N, H * D), k.view(1, N, H * D), H, bsz, (0, 0))
+    launches = ops.launch_count() - before
     for h in range(H):
+        before = ops.launch_count()
         one = ftk.flash_block_score(q[:, :, h].contiguous(), k[:, :, h].contiguous(), 1, bsz, (0, 0))
+        assert ops.launch_count() - before == launches - 1
         assert torch.equal(got[:, h], one[:, 0])
     ftk.check_errors()
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+def test_select_behind_two_scoring_launches(ftk, D):
+    """Scoring in two launches, select overlapped behind them: several calls in a row, whose
+    scratch is the same memory, and the same calls replayed from a graph, give what one head
+    at a time does."""
+    from flash_topk_attn_v2 import ops
+    H, N, bsz, topk = 12, 4096, 64, 8
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    sets = [[torch.randn(1, N, H, D, generator=gen, device="cuda").bfloat16() for _ in range(2)]
+            for _ in range(3)]
+
+    def calls():
+        return [ftk.flash_topk_score(q.view(1, N, H * D), k.view(1, N, H * D), H, bsz, topk, (0, 0), 0.9)
+                for q, k in sets]
+
+    want = [[torch.cat(x, 1) for x in zip(*(
+        ftk.flash_topk_score(q[:, :, h].contiguous(), k[:, :, h].contiguous(), 1, bsz, topk, (0, 0), 0.9)
+        for h in range(H)))] for q, k in sets]
+    before = ops.launch_count()
+    eager = [calls() for _ in range(4)]
+    assert ops.launch_count() - before == 4 * len(sets) * 3
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        calls()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        replayed = calls()
+    for x in replayed:
+        for y in x:
+            y.zero_()
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    ftk.check_errors()
+    for got in eager + [replayed]:
+        for a, b in zip(got, want):
+            for x, y in zip(a, b):
+                assert torch.equal(x, y)
 
 
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
