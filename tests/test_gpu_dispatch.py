@@ -688,6 +688,50 @@ def test_head_dims_below_128_on_pairs(ftk, D, dtype):
 
 
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("D", [72, 88, 104, 120])
+def test_odd_multiples_of_8_on_pairs(ftk, D, dtype):
+    """The C interface takes head dims that are multiples of 8, of which the Python layer refuses
+    the odd ones: on the pair kernels as well, the same bits as with the padding written out as zeros
+    and nothing is stored from column D on (the results' rows are wider, to see that)."""
+    import ctypes as C
+    from flash_topk_attn_v2 import _lib
+    from test_c_abi_cpu import _Attn
+    lib, H, N, g = _lib.lib, 3, 700, 64
+    M = -(-N // g)
+    t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype=dtype, seed=D, do_seed=D + 1))
+    lists = np.tile(np.arange(M, dtype=np.int32), (1, H, M, 1))
+    lists[0, 1, 3:, 2:] = -1
+    lists = torch.from_numpy(lists).cuda()
+
+    def attend(d):
+        x = {n: torch.nn.functional.pad(y.view(N, H, D), (0, d - D)).cuda() for n, y in t.items()}
+        s = (N * H * d, H * d, d)
+        a = _Attn(*(x[n].data_ptr() for n in "qkv"), _lib.dtype_code(x["q"]), 0, 1, H, H, N, d, *s, *s, *s,
+                  lists.data_ptr(), M, M, g, g, 0, 0, D ** -0.5)
+        a = C.byref(a)
+        size = max(lib.ftk_attn_fwd_workspace(a), lib.ftk_attn_bwd_workspace(a))
+        ws = torch.zeros(size, dtype=torch.uint8, device="cuda")
+        o, dq, dk, dv = (torch.full((N, H, d + 8), 7.0, dtype=x["q"].dtype, device="cuda") for _ in range(4))
+        so = (N * H * (d + 8), H * (d + 8), d + 8)
+        lse = torch.empty(H, N, device="cuda")
+        assert lib.ftk_attn_fwd(a, o.data_ptr(), *so, lse.data_ptr(), ws.data_ptr(), size, 0, 0) == 0
+        ws.zero_()
+        assert lib.ftk_attn_bwd_dq(a, o.data_ptr(), *so, x["do"].data_ptr(), *s, lse.data_ptr(),
+                                   ws.data_ptr(), size, dq.data_ptr(), *so, 0, 0) == 0
+        assert lib.ftk_attn_bwd_dkv(a, x["do"].data_ptr(), *s, lse.data_ptr(), ws.data_ptr(), size,
+                                    dk.data_ptr(), *so, dv.data_ptr(), *so, 0, 0) == 0
+        torch.cuda.synchronize()
+        return lse, o, dq, dk, dv
+
+    got, want = attend(D), attend(128)
+    assert torch.equal(got[0], want[0])
+    for x, y in zip(got[1:], want[1:]):
+        assert torch.equal(x[..., :D], y[..., :D])
+        assert (x[..., D:] == 7.0).all()
+        assert torch.isfinite(x).all() and x[..., :D].any()
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
 @pytest.mark.parametrize("at", [64 + 0, 64 + 1, 64 + 2, 64 + 9])
 @pytest.mark.parametrize("what", [float("nan"), float("inf"), 3.0e4])
 def test_forward_values_that_are_no_probabilities(ftk, monkeypatch, dtype, at, what):
