@@ -25,6 +25,7 @@
 // the epilogue (split-KV merge).  A group raises its running maximum only
 // when a block exceeds it by more than 2^8 (P stays inside fp16 range); its
 // O accumulator is then rescaled in TMEM by the row owners.
+#include <cfloat>
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -283,7 +284,8 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t o_addr = lane_addr + FW_COL_O + (SINGLE ? 0 : grp_w * 128);
     const float c = p.scale_log2;
-    float m_run = -INFINITY, l = 0.f;
+    // a finite number also while no logit is: 2^(-inf - m_run) is 0, and the first finite one is above it
+    float m_run = -FLT_MAX, l = 0.f;
     bool ok = true;
 
     if (q_tmem && n > 0 && grp_w == 0) {
@@ -359,7 +361,7 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           }
         }
         const float mt2 = act ? mt * c : -INFINITY;
-        const bool grow = act && (mt2 > m_run + 8.f || m_run == -INFINITY);
+        const bool grow = act && mt2 > m_run + 8.f;
         const float m_new = grow ? mt2 : m_run;
         const bool resc = grow && l > 0.f;
         if (__any_sync(0xffffffffu, resc)) {
@@ -425,7 +427,7 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             if (c0 + x >= lo && c0 + x < hi) mt = fmaxf(mt, __uint_as_float(v[x]));
         }
         const float mt2 = act ? mt * c : -INFINITY;
-        const bool grow = act && (mt2 > m_run + 8.f || m_run == -INFINITY);
+        const bool grow = act && mt2 > m_run + 8.f;
         const float m_new = grow ? mt2 : m_run;
         const bool resc = grow && l > 0.f;
         if (__any_sync(0xffffffffu, resc)) {

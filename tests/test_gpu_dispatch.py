@@ -794,3 +794,33 @@ def test_rows_without_a_finite_logit(ftk, monkeypatch, dtype, D, g, W):
     assert torch.isfinite(o[:, ~gone]).all()
     assert (o - o2)[:, ~gone].abs().max().item() <= 4 * 2 * eps
     torch.testing.assert_close(lse[..., ~gone], lse2[..., ~gone], rtol=1e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("pipe", [False])
+@pytest.mark.parametrize("D,g,W", [(64, 64, 8), (64, 32, 16), (128, 64, 3), (128, 64, 8), (256, 64, 8),
+                                   (64, 48, 4), (128, 128, 3)])
+@pytest.mark.parametrize("level", [0.0, -30.0, -110.0])
+def test_tiles_of_minus_infinity_before_finite_ones(ftk, monkeypatch, dtype, pipe, D, g, W, level):
+    """All blocks but the last give logits of -inf, so a row's first tile, and the one that its
+    reference is taken from, say nothing about the last one's logits, which lie around `level`.
+    Bound: P and O, below 4, are rounded to 16 bits; a logit is a sum of D float32 products."""
+    H, N = 2, 480 if g == 48 else 512
+    M = N // g
+    t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype=dtype, seed=95, do_seed=96))
+    t["q"].view(1, N, H, D)[..., 0] = 8.0
+    t["k"].view(1, N, H, D)[:, :-g, :, 0] = -float("inf")
+    t["k"].view(1, N, H, D)[:, -g:, :, 0] = level * D ** 0.5 / 8.0
+    lists = np.full((1, H, M, W), -1, np.int32)
+    for m in range(M):
+        lists[:, :, m] = np.append((np.arange(W - 1) + m) % (M - 1), M - 1)
+    if not pipe:
+        monkeypatch.setenv("FTK_FWD_PIPE", "0")
+    o, lse = ftk.flash_topk_attn(*(t[n].cuda() for n in "qkv"), torch.from_numpy(lists).cuda(), None, H, g, g)
+    ftk.check_errors()
+    q, k, v = (t[n].view(N, H, D).transpose(0, 1).double() for n in "qkv")
+    logits = q @ k[:, -g:].transpose(1, 2) * D ** -0.5
+    want = (logits.softmax(-1) @ v[:, -g:]).transpose(0, 1).reshape(1, N, H * D)
+    eps = 2.0 ** -10 if dtype == "fp16" else 2.0 ** -7
+    assert (o.cpu().double() - want).abs().max().item() <= 4 * 2 * eps
+    assert (lse[0].cpu().double() - logits.logsumexp(-1)).abs().max().item() <= D * 2.0 ** -24 * (8 - level)
