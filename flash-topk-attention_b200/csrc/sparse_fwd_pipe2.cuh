@@ -322,6 +322,7 @@ sparse_fwd_pipe2_kernel(const __grid_constant__ CUtensorMap tm_q,
           const ColSpan cs =
               col_span(un, pro.entry(pb), SUB, grp, pro_block(pb) * KVB - p.kv_pad_head, KVB, p.N);
           mx = tmem_row_max(lane_addr + COL_S + pb * 64, KVB, cs.lo, cs.hi);
+          ovf = mx == -INFINITY;   // no reference for the row's other tiles: the exact kernel's
         }
         s_mref[r] = (mx > -INFINITY) ? mx * c : 0.f;
         tc_fence_before();

@@ -797,7 +797,7 @@ def test_rows_without_a_finite_logit(ftk, monkeypatch, dtype, D, g, W):
 
 
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
-@pytest.mark.parametrize("pipe", [False])
+@pytest.mark.parametrize("pipe", [True, False])
 @pytest.mark.parametrize("D,g,W", [(64, 64, 8), (64, 32, 16), (128, 64, 3), (128, 64, 8), (256, 64, 8),
                                    (64, 48, 4), (128, 128, 3)])
 @pytest.mark.parametrize("level", [0.0, -30.0, -110.0])
