@@ -27,7 +27,8 @@
 // reference by up to 2^80 before anything overflows (fp16: 2^15, P must stay
 // below 65504); a row whose tile sum passes that bound marks its tile's word in
 // `redo_out`, and the exact kernel, launched behind this one with a CTA per SM, looks
-// through the words and recomputes exactly those tiles.
+// through the words and recomputes exactly those tiles.  So does a row whose reference tile is
+// all -inf: it has no reference for the others.
 #pragma once
 
 namespace ftk {

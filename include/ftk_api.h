@@ -247,7 +247,7 @@ int ftk_attn_bwd_dkv(const ftk_attn* a, const void* dout, int64_t sdo_b, int64_t
  * csrc/sparse_attn_kernel.cu:368).  merged_idx [B*H][QM][W]; for every real
  * query row of q-block m attends to the tokens of the blocks listed in the
  * valid prefix of its row.  o in `dtype` with strides (so_*), lse fp32
- * [B*H][N] (natural log; -inf and o = 0 for an empty list).  k and v carry Hkv
+ * [B*H][N] (natural log; -inf and o = 0 for an empty list, or logits that are all -inf).  k and v carry Hkv
  * heads (Hkv <= 0 means H; H must be a multiple): query head h reads kv head
  * h / (H / Hkv).  The reference rejects Hkv != H (__init__.py:153-156).
  * `workspace` (ftk_sparse_fwd_workspace bytes, may be NULL) enables the
