@@ -87,22 +87,25 @@ inline int encode_tmap_bnhd(CUtensorMap* out, const void* base, int dtype, int64
 
 // Dynamic shared memory of a kernel, raised once per device and size instead of
 // at every launch (the attribute call costs about a microsecond of host time).
+// The runtime sets the limit, it does not raise it: threads that ask for two sizes at once take
+// turns at looking, setting and recording, or the smaller one could be set behind the record of
+// the larger, and launches of that kernel would fail from then on.  A size that is on record
+// needs no turn: the limit was set before and never goes down.
 template <auto KERNEL>
 inline int allow_smem(size_t bytes) {
   constexpr int MAX_DEVICES = 64;
   static std::atomic<size_t> allowed[MAX_DEVICES];
+  static std::mutex turn;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return FTK_ERR_CUDA;
   const bool known = dev >= 0 && dev < MAX_DEVICES;
+  if (known && allowed[dev].load(std::memory_order_acquire) >= bytes) return FTK_OK;
+  std::lock_guard<std::mutex> lock(turn);
   if (known && allowed[dev].load(std::memory_order_relaxed) >= bytes) return FTK_OK;
   if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(bytes)) != cudaSuccess)
     return FTK_ERR_CUDA;
-  if (known) {
-    size_t seen = allowed[dev].load(std::memory_order_relaxed);
-    while (seen < bytes && !allowed[dev].compare_exchange_weak(seen, bytes)) {
-    }
-  }
+  if (known) allowed[dev].store(bytes, std::memory_order_release);
   return FTK_OK;
 }
 

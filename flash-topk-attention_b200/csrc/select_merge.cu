@@ -1102,10 +1102,8 @@ extern "C" int ftk_build_reverse(const int32_t* merged_idx, const int32_t* count
   if (sorted_kv) {
     const int Mp = std::max(32, next_pow2(M));
     const size_t smem = static_cast<size_t>(Mp) * 8;
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(reverse_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
-      return FTK_ERR_CUDA;
+    if (smem > 48 * 1024)
+      if (int e = allow_smem<reverse_sort_kernel>(smem)) return e;
     reverse_sort_kernel<<<static_cast<unsigned>(BH), 256, smem, st>>>(reverse_counts, M, Mp,
                                                                      sorted_kv);
   }
@@ -1201,10 +1199,8 @@ extern "C" int ftk_build_reverse_noalloc(const int32_t* merged_idx, const int32_
   if (sorted_kv) {
     const int Mp = std::max(32, next_pow2(M));
     const size_t smem = static_cast<size_t>(Mp) * 8;
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(reverse_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
-      return FTK_ERR_CUDA;
+    if (smem > 48 * 1024)
+      if (int e = allow_smem<reverse_sort_kernel>(smem)) return e;
     reverse_sort_kernel<<<static_cast<unsigned>(BH), 256, smem, st>>>(reverse_counts, M, Mp,
                                                                      sorted_kv);
   }

@@ -1,9 +1,16 @@
 """The host layer in front of the kernels, as far as it goes without a device."""
 
 import ctypes
+import glob
+import os
+import re
+import subprocess
 
 import pytest
 import torch
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "flash-topk-attention_b200", "csrc")
 
 
 @pytest.fixture(scope="module")
@@ -154,3 +161,16 @@ def test_forward_mode_is_refused(which, dtype):
         x[which] = fw.make_dual(x[which], _fake((1, 128, 128), dtype))
         with pytest.raises(NotImplementedError, match="forward-mode"):
             ftk.flash_topk_attn(*x.values(), _fake((1, 2, 2, 4), torch.int32), None, 2, 64, 64)
+
+
+def test_threads_that_raise_a_kernels_shared_memory(tmp_path):
+    """Two threads ask for two sizes of one kernel's dynamic shared memory at once: the limit ends
+    at the larger one, as the record has it, whichever call is held up inside the runtime
+    (native/smem_limit_probe.cpp).  No launcher sets the limit by itself."""
+    exe = str(tmp_path / "probe")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", CSRC, "-I", "/usr/local/cuda/include",
+                    os.path.join(HERE, "native", "smem_limit_probe.cpp"), "-o", exe, "-lpthread"], check=True)
+    out = subprocess.run([exe], check=True, capture_output=True, text=True, timeout=60).stdout
+    assert out.split() == ["0", "214016", "0"]      # refused, limit, calls for sizes on record
+    text = "".join(re.sub(r"//[^\n]*", "", open(f).read()) for f in glob.glob(os.path.join(CSRC, "*.cu*")))
+    assert len(re.findall(r"\bcudaFuncSetAttribute\b", text)) == 1
