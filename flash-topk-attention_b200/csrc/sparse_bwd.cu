@@ -215,6 +215,34 @@ __device__ __forceinline__ void pt_pairs(const uint32_t (&sv)[16], const uint32_
   }
 }
 
+// The same where only columns lo .. hi - 1 are the row's.  A function: as a lambda of two callers
+// it was not inlined well.  The exponential's argument is selected, not the exponential, which
+// became a branch per value.  dK/dV of 4096 tokens, H = 16, blocks of 48, half of them listed: head
+// dim 64 402 us, 264 like this, head dim 128 (with the early end of dP^T below) 680, 313.
+__device__ __forceinline__ void pt_masked(const uint32_t (&sv)[16], const uint32_t (&dv)[16],
+                                          const float4* nl4, const float4* nd4, float c, int lo, int hi,
+                                          int fmt, uint32_t (&pp)[8], uint32_t (&pd)[8]) {
+#pragma unroll
+  for (int x = 0; x < 16; x += 4) {
+    const float4 lq = nl4[x >> 2];
+    const float4 dq = nd4[x >> 2];
+    const float ls[4] = {lq.x, lq.y, lq.z, lq.w};
+    const float ds[4] = {dq.x, dq.y, dq.z, dq.w};
+    float pv[4], dsv[4];
+#pragma unroll
+    for (int y = 0; y < 4; y++) {
+      const bool on = x + y >= lo && x + y < hi;
+      const float pr = fast_exp2(on ? fmaf(__uint_as_float(sv[x + y]), c, ls[y]) : -INFINITY);
+      pv[y] = pr;
+      dsv[y] = pr * (__uint_as_float(dv[x + y]) + ds[y]);
+    }
+    pp[x >> 1] = pack2(pv[0], pv[1], fmt);
+    pp[(x >> 1) + 1] = pack2(pv[2], pv[3], fmt);
+    pd[x >> 1] = pack2(dsv[0], dsv[1], fmt);
+    pd[(x >> 1) + 1] = pack2(dsv[2], dsv[3], fmt);
+  }
+}
+
 // ---------------------------------------------------------------------- dQ
 // TMEM columns: Q and dO, D / 2 each (16-bit pairs: the A operands of the
 // S and dP UMMAs are read from TMEM, which leaves shared-memory bandwidth to
@@ -1018,8 +1046,9 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t st_addr = lane_addr + wg * 64;         // S^T, then P^T
     const uint32_t dp_addr = lane_addr + 128 + (K_T ? 0 : wg * 64);   // dP^T, then dS^T
-    const int cbeg = split ? colhalf * (p.g / 2) : 0;
-    const int cend = split ? cbeg + p.g / 2 : (colhalf == 0 ? p.g : 0);
+    // (head dim 128, where 32 columns at most are kept while dP^T makes room: 48 as 32 and 16)
+    const int part = K_T && p.g == 48 ? 32 : split ? p.g / 2 : p.g;
+    const int cbeg = min(colhalf * part, p.g), cend = min(cbeg + part, p.g);
     const float c = p.scale_log2;
     bool ok = true;
     if (ROWS_T && n > 0 && colhalf == 0) {
@@ -1081,33 +1110,11 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
       tc_fence_after();
       const float4* l4 = reinterpret_cast<const float4*>(s_lse2[wg][pb]);
       const float4* d4 = reinterpret_cast<const float4*>(s_delta[wg][pb]);
-      // columns of a tile that the row's kv block does not read in full
-      auto masked = [&](const uint32_t (&sv)[16], const uint32_t (&dv)[16], int c0, uint32_t (&pp)[8],
-                        uint32_t (&pd)[8]) {
-#pragma unroll
-        for (int x = 0; x < 16; x += 4) {
-          const float4 lq = l4[(c0 + x) >> 2];
-          const float4 dq = d4[(c0 + x) >> 2];
-          const float ls[4] = {lq.x, lq.y, lq.z, lq.w};
-          const float ds[4] = {dq.x, dq.y, dq.z, dq.w};
-          float pv[4], dsv[4];
-#pragma unroll
-          for (int y = 0; y < 4; y++) {
-            const bool on = act && c0 + x + y >= lo && c0 + x + y < hi;
-            const float pr = on ? fast_exp2(fmaf(__uint_as_float(sv[x + y]), c, ls[y])) : 0.f;
-            pv[y] = pr;
-            dsv[y] = pr * (__uint_as_float(dv[x + y]) + ds[y]);
-          }
-          pp[x >> 1] = pack2(pv[0], pv[1], p.fmt);
-          pp[(x >> 1) + 1] = pack2(pv[2], pv[3], p.fmt);
-          pd[x >> 1] = pack2(dsv[0], dsv[1], p.fmt);
-          pd[(x >> 1) + 1] = pack2(dsv[2], dsv[3], p.fmt);
-        }
-      };
       // P^T / dS^T of columns [c0, c0+16) go over columns cbeg + (c0-cbeg)/2 ..
       // of the S^T / dP^T regions (head dim 128: over c0 .. and c0 + 8 .. of S^T): columns
       // this thread has already read
-      if (K_T && p.g == 64 && fast) {
+      const bool whole = cend - cbeg == 32;
+      if (K_T && whole && fast) {
         // the dP^T buffer is the next tile's as soon as its columns are in registers
         uint32_t sv[2][16], dv[2][16];
         tmem_ld16(dp_addr + cbeg, dv[0]);
@@ -1127,7 +1134,7 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
           tmem_st8(st_addr + c0, pp);
           tmem_st8(st_addr + c0 + 8, pd);
         }
-      } else if (K_T && p.g == 64 && !none) {
+      } else if (K_T && whole && !none) {
         uint32_t sv[2][16], dv[2][16];
         tmem_ld16(dp_addr + cbeg, dv[0]);
         tmem_ld16(dp_addr + cbeg + 16, dv[1]);
@@ -1141,7 +1148,7 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
         for (int h = 0; h < 2; h++) {
           uint32_t pp[8], pd[8];
           const int c0 = cbeg + 16 * h;
-          masked(sv[h], dv[h], c0, pp, pd);
+          pt_masked(sv[h], dv[h], l4 + (c0 >> 2), d4 + (c0 >> 2), c, act ? lo - c0 : 16, hi - c0, p.fmt, pp, pd);
           tmem_st8(st_addr + c0, pp);
           tmem_st8(st_addr + c0 + 8, pd);
         }
@@ -1160,6 +1167,11 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
         tmem_ld16(st_addr + c0, sv);
         if (MODE != 1) tmem_ld16(dp_addr + c0, dv);
         tmem_wait_ld();
+        if (K_T) {   // 16 columns
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_dpfree);
+        }
         if (MODE == 1) {   // no dP^T in this launch: dS^T is computed and dropped
 #pragma unroll
           for (int x = 0; x < 16; x++) dv[x] = 0u;
@@ -1168,7 +1180,7 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
           if (p.fmt == 1) pt_pairs<1>(sv, dv, l4 + (c0 >> 2), d4 + (c0 >> 2), c, pp, pd);
           else pt_pairs<0>(sv, dv, l4 + (c0 >> 2), d4 + (c0 >> 2), c, pp, pd);
         } else {
-          masked(sv, dv, c0, pp, pd);
+          pt_masked(sv, dv, l4 + (c0 >> 2), d4 + (c0 >> 2), c, act ? lo - c0 : 16, hi - c0, p.fmt, pp, pd);
         }
         if (MODE != 2) tmem_st8(st_addr + oc, pp);
         if (MODE != 1) tmem_st8(ds_addr, pd);
@@ -1177,7 +1189,7 @@ sparse_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q,
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        if (K_T && (none || p.g != 64)) mbar_arrive(bar_dpfree);
+        if (K_T && (none || cbeg == cend)) mbar_arrive(bar_dpfree);
         mbar_arrive(bar_pfull(wg));
       }
     }

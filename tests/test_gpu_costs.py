@@ -1,0 +1,56 @@
+"""What uncommon inputs cost beside ordinary ones of the same size.
+
+Both sides are timed here, on one device, so that a bound is a ratio.  Each is the ratio that the
+work itself has, or that of the plain kernels, with room for noise; the inputs are ones that some
+kernel once took several times longer over."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ftk():
+    import flash_topk_attn_v2 as m
+    return m
+
+
+def _us(call, calls=5, rounds=7):
+    """Device time of a call: the shortest of some rounds, the calls of a round back to back."""
+    call()
+    torch.cuda.synchronize()
+    times = []
+    for _ in range(rounds):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        torch.cuda._sleep(500000)      # the calls are enqueued by then
+        a.record()
+        for _ in range(calls):
+            call()
+        b.record()
+        b.synchronize()
+        times.append(a.elapsed_time(b) * 1e3 / calls)
+    return min(times)
+
+
+def _random_lists(H, QM, M, W, gen):
+    return torch.rand(1, H, QM, M, generator=gen, device="cuda").topk(W, dim=-1).indices.to(torch.int32)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_backward_of_48_row_blocks(ftk, D):
+    """48 rows of 64 and 96 of 128 make 16 / 9 times the tiles of 64-row blocks, whose pairs cost
+    the same otherwise; 1.3 for half a warp that lists a block where the other half does not."""
+    N, H = 4032, 16
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v, do = (torch.randn(1, N, H * D, generator=gen, device="cuda").bfloat16() for _ in range(4))
+    for x in (q, k, v):
+        x.requires_grad_(True)
+    us = {}
+    for g in (64, 48):
+        M = N // g
+        merged = _random_lists(H, M, M, M // 2, gen)
+        o, _ = ftk.flash_topk_attn(q, k, v, merged, None, H, g, g)
+        us[g] = _us(lambda: torch.autograd.grad(o, (q, k, v), do, retain_graph=True))
+    ftk.check_errors()
+    assert us[48] <= 1.3 * 16 / 9 * us[64], us
