@@ -42,7 +42,7 @@ constexpr int FW_MAX_STAGES = 4;
 // A redo CTA looks at the words of this many tiles at once, 16 bytes a load.
 constexpr int REDO_LOADS = 8;
 constexpr int REDO_LOOK = FW_THREADS * REDO_LOADS * 4;
-constexpr int REDO_MASKS = REDO_LOOK / 32;
+constexpr int REDO_QUEUE = 128;   // and takes up to so many of them, where CTAs * REDO_QUEUE >= REDO_LOOK
 // TMEM columns.  kv blocks of at most 64 rows: Q (16-bit pairs) 0..63, S[2]
 // at 64 / 128, so the S UMMAs read their A operand from TMEM and shared-memory
 // bandwidth is left to the K/V tiles (an SS UMMA of this shape spends more
@@ -74,92 +74,94 @@ struct FwdParams {
 // What the exact kernel does: all tiles, or those that the pipelined one marked
 enum : int { EXACT = 0, REDO_OWN = 1, REDO_DEAL = 2 };
 
-// Where a redo CTA's look through the words stands.
+// Where a redo CTA's look through the words stands, and the tiles that it found for itself.
 struct RedoScan {
-  int look, mask, found;       // first word of the round, next mask, marked tiles seen
-  unsigned left;               // of the last mask
-  unsigned todo[REDO_MASKS];   // of the round: warp w, word i of its loads at 10 * i + w
+  int look, before;          // words looked at, marked tiles among them
+  int warps[FW_THREADS / 32];
+  int queue[REDO_QUEUE];
 };
-// REDO_DEAL: every CTA looks at all words, and does those of the marked tiles, counted in the
-// order it meets them, whose number is its own (mod the CTAs).  Returns the next tile to do,
-// -1 behind the last; all threads call it.  A redone tile walks its whole list, 100 us for 7000
-// keys, and when a CTA looks at every gridDim.x-th word only, some have two or three marked tiles
-// to do while most have none (fp16, 15000 tokens, H = 16, 17 to 109 of 1888 tiles marked: 380 us,
-// 221 dealt).  The loop over a tile's keys is a fifth slower in this form (114 tiles, 7181 tokens,
-// D = 96, hot rows: 105 us against 91), so that it is not taken where tiles are few.  A function
-// of its own with its state in shared memory: inlined, its registers made that 124 us.
-__device__ __noinline__ int next_marked(const int* words, int tiles, RedoScan* s, bool first) {
+// REDO_DEAL: every CTA looks at all words, REDO_LOOK at a time, and does those of the marked tiles,
+// counted as they come, whose number is its own (mod the CTAs).  Fills the queue with the next of
+// them and returns how many there are, 0 behind the last; all threads call it.  A redone tile walks its
+// whole list, 100 us for 7000 keys, and when a CTA looks at every gridDim.x-th word only, some have two
+// or three marked tiles to do while most have none (fp16, 15000 tokens, H = 16, 17 to 109 of 1888
+// tiles marked: 380 us, 221 dealt).  A thread counts the marked ones among its own words and
+// knows from the counts before which of them the CTA does, so that marked tiles which others do
+// cost nothing (1024 of 1024 tiles marked, lists of 2, head dim 64: forward 94 us, 285 with a walk
+// over all of them).
+__device__ __noinline__ int next_marked(const int* words, unsigned tiles, RedoScan* s, bool first) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ctas = gridDim.x;
   const bool wide = (reinterpret_cast<uintptr_t>(words) & 15) == 0;
   if (first) {   // as a rule there are none
     int any = 0;
 #pragma unroll 4
-    for (unsigned t = 4u * tid; t < static_cast<unsigned>(tiles); t += 4u * FW_THREADS) {
-      if (wide && t + 4 <= static_cast<unsigned>(tiles)) {
+    for (unsigned t = 4u * tid; t < tiles; t += 4u * FW_THREADS) {
+      if (wide && t + 4 <= tiles) {
         const int4 q = *reinterpret_cast<const int4*>(words + t);
         any |= q.x | q.y | q.z | q.w;
       } else {
-        for (unsigned x = t; x < min(t + 4u, static_cast<unsigned>(tiles)); x++) any |= words[x];
+        for (unsigned x = t; x < min(t + 4u, tiles); x++) any |= words[x];
       }
     }
-    if (!__syncthreads_or(any)) return -1;
+    if (!__syncthreads_or(any)) return 0;
   }
-  // CTAs of neighbouring numbers are neighbours on the chip, so that neighbouring tiles go to
-  // distant ones (one that has no factor in common with the number of CTAs apart)
-  const int apart = ctas % 61 ? 61 : 59;
-  int look = first ? -REDO_LOOK : s->look, mask = first ? REDO_MASKS : s->mask, found = first ? 0 : s->found;
-  unsigned left = first ? 0u : s->left;
-  while (true) {
-    while (left == 0) {
-      if (mask < REDO_MASKS) {
-        left = s->todo[mask++];
-        continue;
-      }
-      unsigned mine = 0;   // bit 4 * k + x: word x of load k
-      do {
-        look += REDO_LOOK;
-        if (look >= tiles || look < 0) return -1;
-        int v[REDO_LOADS][4];
-#pragma unroll
-        for (int k = 0; k < REDO_LOADS; k++) {
-          const unsigned t = look + 4u * (k * FW_THREADS + tid), end = tiles;
-          if (wide && t + 4 <= end) {
-            const int4 q = *reinterpret_cast<const int4*>(words + t);
-            v[k][0] = q.x;
-            v[k][1] = q.y;
-            v[k][2] = q.z;
-            v[k][3] = q.w;
-          } else {
-#pragma unroll
-            for (int x = 0; x < 4; x++) v[k][x] = t + x < end ? words[t + x] : 0;
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < REDO_LOADS; k++)
-#pragma unroll
-          for (int x = 0; x < 4; x++) mine |= v[k][x] != 0 ? 1u << (4 * k + x) : 0u;
-      } while (!__syncthreads_or(mine != 0u));
+  int before = first ? 0 : s->before;
 #pragma unroll 1
-      for (int i = 0; i < 4 * REDO_LOADS; i++) {
-        const unsigned bal = __ballot_sync(0xffffffffu, (mine >> i) & 1u);
-        if (lane == 0) s->todo[i * (FW_THREADS / 32) + warp] = bal;
+  for (unsigned look = first ? 0u : s->look; look < tiles; look += REDO_LOOK) {
+    unsigned mine = 0;   // bit 4 * k + x: word x of load k
+#pragma unroll 4
+    for (int k = 0; k < REDO_LOADS; k++) {
+      const unsigned t = look + 4u * (k * FW_THREADS + tid);
+      unsigned marks = 0;
+      if (wide && t + 4 <= tiles) {
+        const int4 q = *reinterpret_cast<const int4*>(words + t);
+        marks = (q.x != 0 ? 1u : 0u) | (q.y != 0 ? 2u : 0u) | (q.z != 0 ? 4u : 0u) | (q.w != 0 ? 8u : 0u);
+      } else {
+        for (unsigned x = 0; x < 4 && t + x < tiles; x++) marks |= words[t + x] != 0 ? 1u << x : 0u;
+      }
+      mine |= marks << (4 * k);
+    }
+    if (!__syncthreads_or(mine != 0u)) continue;
+    const int count = __popc(mine);
+    int upto = count;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, upto, d);
+      if (lane >= d) upto += o;
+    }
+    if (lane == 31) s->warps[warp] = upto;
+    __syncthreads();
+    int ahead = upto - count, total = 0;
+#pragma unroll 1
+    for (int x = 0; x < FW_THREADS / 32; x++) {
+      const int n = s->warps[x];
+      ahead += x < warp ? n : 0;
+      total += n;
+    }
+    // CTAs of neighbouring numbers are neighbours on the chip, so that neighbouring tiles go to
+    // distant ones (the factor has none in common with the number of CTAs): of the marked tiles of
+    // this round, counted from 0, this CTA does `start`, `start` + ctas, ...
+    const int own = static_cast<int>(blockIdx.x) * (ctas % 17 ? 17 : 19) % ctas;
+    const int start = (own + ctas - before % ctas) % ctas;
+    for (int at = ahead <= start ? 0 : (ahead - start + ctas - 1) / ctas; start + at * ctas < ahead + count; at++) {
+      unsigned rest = mine;
+#pragma unroll 1
+      for (int skip = start + at * ctas - ahead; skip > 0; skip--) rest &= rest - 1;
+      const int i = __ffs(rest) - 1;
+      s->queue[at] = static_cast<int>(look + 4u * ((i >> 2) * FW_THREADS + tid) + (i & 3));
+    }
+    before += total;
+    if (start < total) {
+      if (tid == 0) {
+        s->look = look + REDO_LOOK;
+        s->before = before;
       }
       __syncthreads();
-      mask = 0;
+      return (total - start + ctas - 1) / ctas;
     }
-    const int bit = __ffs(left) - 1;
-    left &= left - 1;
-    if (found++ % ctas * apart % ctas != static_cast<int>(blockIdx.x)) continue;
-    __syncthreads();   // all have read the state
-    if (tid == 0) {
-      s->look = look;
-      s->mask = mask;
-      s->found = found;
-      s->left = left;
-    }
-    const int at = mask - 1, i = at / (FW_THREADS / 32), wp = at - i * (FW_THREADS / 32);
-    return look + 4 * ((i >> 2) * FW_THREADS + wp * 32 + bit) + (i & 3);
+    __syncthreads();   // the counts are read
   }
+  return 0;
 }
 
 // D = head dim of the Q.K^T contraction, DV = columns of V / O.  Head dim 256: two 256-column accumulators do not
@@ -195,7 +197,6 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   __shared__ std::conditional_t<MODE == REDO_DEAL, RedoScan, int> s_scan;
   __shared__ unsigned s_todo[(FW_THREADS + 31) / 32];
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   pdl_wait();
   bool first_tile = true;
   uint32_t tmem = 0;
@@ -205,7 +206,10 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   int word = FW_THREADS / 32;
   unsigned left = 0;
   auto next_tile = [&]() -> int {
-    if constexpr (MODE == REDO_DEAL) return next_marked(p.redo_in, p.tiles, &s_scan, first_tile);
+    if constexpr (MODE == REDO_DEAL) {
+      if (left == 0) left = next_marked(p.redo_in, p.tiles, &s_scan, first_tile);
+      return left == 0 ? -1 : s_scan.queue[--left];
+    }
     if (MODE == EXACT) return first_tile ? static_cast<int>(blockIdx.x) : -1;
     while (left == 0) {
       if (word < FW_THREADS / 32) {
@@ -215,9 +219,9 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       base += static_cast<int64_t>(gridDim.x) * FW_THREADS;
       if (base >= p.tiles) return -1;
       __syncthreads();
-      const int64_t t = base + static_cast<int64_t>(tid) * gridDim.x;
+      const int64_t t = base + static_cast<int64_t>(threadIdx.x) * gridDim.x;
       const unsigned bal = __ballot_sync(0xffffffffu, t < p.tiles && p.redo_in[t] != 0);
-      if (lane == 0) s_todo[warp] = bal;
+      if ((threadIdx.x & 31) == 0) s_todo[threadIdx.x >> 5] = bal;
       __syncthreads();
       word = 0;
     }
@@ -226,6 +230,8 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     return static_cast<int>(base + static_cast<int64_t>((word - 1) * 32 + bit) * gridDim.x);
   };
   for (int tile = next_tile(); tile >= 0; tile = next_tile()) {
+  // read anew for every tile: what is derived from it is not kept across the loop
+  const int tid = REDO ? late_tid() : threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int bh = tile / p.tiles_x;
   const int m0 = (tile - bh * p.tiles_x) * p.G;
   const int b_idx = bh / p.H, h_idx = bh - b_idx * p.H;
@@ -630,7 +636,7 @@ sparse_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     break;   // uniform: barriers and TMEM are not in a state to go on with
   }
   }
-  if (warp == 0 && !first_tile) tmem_dealloc(tmem, 512);
+  if (threadIdx.x < 32 && !first_tile) tmem_dealloc(tmem, 512);
 }
 
 }  // namespace ftk
@@ -696,7 +702,8 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   // Redo: as many CTAs as run at once, which find their tiles themselves.  Up to one tile per SM
   // they cannot meet, and with a few no CTA's share of the marked ones is long; beyond that the
   // marked ones are dealt, see next_marked.
-  const int mode = !p.redo_in ? EXACT : p.tiles > 4 * sm_count() ? REDO_DEAL : REDO_OWN;
+  const bool deal = p.tiles > 4 * sm_count() && sm_count() * REDO_QUEUE >= REDO_LOOK;
+  const int mode = !p.redo_in ? EXACT : deal ? REDO_DEAL : REDO_OWN;
   const int ctas = p.redo_in ? std::min(p.tiles, sm_count()) : p.tiles;
   return choose<3>(mode, [&](auto m) {
     constexpr auto kernel = sparse_fwd_kernel<D, D, decltype(m)::value>;

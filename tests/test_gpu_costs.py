@@ -54,3 +54,25 @@ def test_backward_of_48_row_blocks(ftk, D):
         us[g] = _us(lambda: torch.autograd.grad(o, (q, k, v), do, retain_graph=True))
     ftk.check_errors()
     assert us[48] <= 1.3 * 16 / 9 * us[64], us
+
+
+@pytest.mark.parametrize("D,W", [(64, 2), (64, 8), (128, 2), (256, 2)])
+def test_forward_that_is_all_for_the_exact_kernel(ftk, monkeypatch, D, W):
+    """fp16 rows beyond the pipelined kernel's range in every one of 1024 tiles: the forward is both
+    kernels one after the other, and that is what it costs (1.3 of the sum); the bits are the exact
+    kernel's."""
+    N, H, g = 8192, 16, 64
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    q, k, v = (torch.randn(1, N, H * D, generator=gen, device="cuda").half() for _ in range(3))
+    merged = _random_lists(H, N // g, N // g, W, gen)
+    hot = k * 12.0
+    run = lambda keys: ftk.flash_topk_attn(q, keys, v, merged, None, H, g, g)
+    ordinary, marked = _us(lambda: run(k)), _us(lambda: run(hot))
+    o, lse = run(hot)
+    monkeypatch.setenv("FTK_FWD_PIPE", "0")
+    exact = _us(lambda: run(hot))
+    o2, lse2 = run(hot)
+    ftk.check_errors()
+    same = (o.view(N, H, D) == o2.view(N, H, D)).all(-1).float().mean().item()
+    assert torch.equal(lse, lse2) and same == 1.0
+    assert marked <= 1.3 * (ordinary + exact), (marked, ordinary, exact)
