@@ -557,11 +557,15 @@ qblock_merge_warp_kernel(const int32_t* idx, const float* scr, int64_t N, int K,
 // all threads at once, and a thread per block id adds up its column.  Absent entries add 0, so
 // every aggregate is the same sum in the same order.  Two entries of a row that name the same
 // block (never picks of a select) are found by tags that are written with the entries and read
-// back; such a q-block is added up entry by entry.  A thread's aggregate goes to the position that
-// as many others precede.  For when see ftk_qblock_merge.
+// back; the entries of such a row are laid out for all threads, which look for their block among
+// them (512 q-blocks of 64 rows that name 63 of 64 blocks, one of them twice: 47 us, a warp per
+// q-block 55; 355 while every thread went through all entries of the q-block).  A thread's
+// aggregate goes to the position that as many others precede.  For when see ftk_qblock_merge.
 constexpr int MGD_THREADS = 128;
 constexpr int MGD_IDS = 128, MGD_CELLS = 8192;   // block ids; rows x block ids
-constexpr int MGD_PICKS = 256;                   // entries of a row that a tag can tell apart
+constexpr int MGD_PICKS = MGD_THREADS;           // entries of a row
+constexpr int MGD_ROWS = MGD_CELLS / 4;
+constexpr size_t MGD_STATIC = MGD_IDS * 4 + MGD_PICKS * 4 + MGD_ROWS / 8;
 __host__ __device__ constexpr int mgd_pitch(int ids) { return (ids + 3) & ~3; }
 __host__ __device__ constexpr size_t mgd_smem(int g, int ids) { return static_cast<size_t>(g) * mgd_pitch(ids) * 5; }
 
@@ -571,6 +575,8 @@ qblock_merge_dense_kernel(const int32_t* idx, const float* scr, int64_t N, int K
                           int* status) {
   extern __shared__ __align__(16) float mgd_smem_f[];
   __shared__ __align__(16) unsigned agg[MGD_IDS];
+  __shared__ __align__(16) float row_scr[MGD_PICKS];
+  __shared__ unsigned twice[MGD_ROWS / 32];        // rows that name a block twice
   pdl_wait();
   pdl_launch();
   const int tid = threadIdx.x;
@@ -624,15 +630,53 @@ qblock_merge_dense_kernel(const int32_t* idx, const float* scr, int64_t N, int K
   });
   const bool repeats = __syncthreads_or(lost);
   float sum = 0.f;
-  if (tid < ids) {
-    if (!repeats) {
-#pragma unroll 8
-      for (int r = 0; r < rows; r++) sum += cell[r * pitch + tid];
-    } else {
-#pragma unroll 1
-      for (int e = 0; e < total; e++)
-        if (idx[first + e] == tid) sum += scr ? scr[first + e] : 1.f;
+  if (repeats) {
+    for (int x = tid; x < MGD_ROWS / 32; x += MGD_THREADS) twice[x] = 0u;
+    __syncthreads();
+    for (int e = tid; e < total; e += MGD_THREADS) {
+      const int j = idx[first + e], row = e / K;
+      if (static_cast<unsigned>(j) < static_cast<unsigned>(ids) &&
+          tag[row * pitch + j] != static_cast<uint8_t>(e - row * K))
+        atomicOr(&twice[row >> 5], 1u << (row & 31));
     }
+    unsigned* row_idx = agg;
+    int j = -1;
+    float s = 0.f;
+    auto fetch = [&](int r) {   // the thread's entry of row r
+      if (r < rows && tid < K) {
+        j = idx[first + r * K + tid];
+        s = scr ? scr[first + r * K + tid] : 1.f;
+      }
+    };
+    fetch(0);
+    __syncthreads();
+#pragma unroll 1
+    for (int r = 0; r < rows; r++) {
+      if (twice[r >> 5] >> (r & 31) & 1u) {
+        row_idx[tid] = j;
+        row_scr[tid] = s;
+        fetch(r + 1);
+        __syncthreads();
+        if (tid < ids) {
+#pragma unroll 4
+          for (int c = 0; c < K; c += 4) {
+            const uint4 js = *reinterpret_cast<const uint4*>(row_idx + c);
+            const float4 ss = *reinterpret_cast<const float4*>(row_scr + c);
+            if (js.x == tid) sum += ss.x;
+            if (js.y == tid) sum += ss.y;
+            if (js.z == tid) sum += ss.z;
+            if (js.w == tid) sum += ss.w;
+          }
+        }
+        __syncthreads();
+      } else {
+        fetch(r + 1);
+        if (tid < ids) sum += cell[r * pitch + tid];
+      }
+    }
+  } else if (tid < ids) {
+#pragma unroll 8
+    for (int r = 0; r < rows; r++) sum += cell[r * pitch + tid];
   }
   // aggregates that are not above 0 are not there
   const unsigned mine = sum > 0.f ? __float_as_uint(sum) : 0u;
@@ -1002,17 +1046,22 @@ extern "C" int ftk_qblock_merge(const int32_t* topk_idx, const float* topk_score
   const size_t smem = static_cast<size_t>(Mp) * 12;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t total_qb = BH * QM;
-  // Few q-blocks: a CTA each.  A warp takes 3.5 kilocycles and 0.27 for each of its steps however
-  // few there are; CTAs take 4.5 and, with their SM's share of the q-blocks, one cycle for four
-  // cells of the table and 0.8 for an entry (q-blocks, ids, picks, rows; warps, CTAs in
-  // kilocycles: 512, 32, 8, 64 21.1, 8.1; 576, 47, 16, 64 21.0, 10.9; 512, 128, 32, 32 14.0, 12.9;
-  // 800, 100, 24, 64 25.0, 17.6; 1024, 64, 64, 64 39.7, 36.3; 2048, 128, 16, 32 18.4, 27.5; 2048,
-  // 128, 32, 64 28.8, 62.0).
+  // Few q-blocks: a CTA each.  A warp takes 3.15 us and 0.126 for each of its steps however few
+  // there are; CTAs take 3.5 us, 0.65 ns for an entry and, for each of their SM's share of the q-blocks,
+  // 0.12 us, 0.09 ns for a cell of the table and 0.25 ns for an entry, as long as all run at once
+  // 0.12 us, 0.09 ns for a cell of the table and 0.25 ns for an entry, as long as all run at once
+  // (q-blocks, ids, picks, rows; warps, CTAs in us: 32, 16, 8, 16 5.0, 3.3; 256, 64, 32, 32 6.6, 4.9;
+  // 512, 64, 64, 64 18.4, 10.6; 512, 128, 16, 32 7.9, 6.6; 512, 128, 16, 16 5.7, 6.3; 1024, 47, 16,
+  // 128 22.0, 10.4; 1024, 64, 64, 16 7.2, 7.7; 1024, 128, 128, 64, of which 5 run on an SM at once,
+  // 37.4, 40.9).  Rows of more picks than blocks name some twice, always.
   const int64_t g = q_block_size, merge_steps = K <= 32 ? g : (g * K + 31) / 32;
-  const bool few = 5 * total_qb * g * num_score_blocks + 16 * total_qb * g * K <
-                   20 * static_cast<int64_t>(sm_count()) * (270 * merge_steps - 1000);
-  if (num_score_blocks <= MGD_IDS && K <= MGD_PICKS && g * mgd_pitch(num_score_blocks) <= MGD_CELLS && few) {
-    const size_t bytes = spread_smem(total_qb, mgd_smem(q_block_size, num_score_blocks), MGD_IDS * 4);
+  const int64_t share = (total_qb + sm_count() - 1) / sm_count();
+  const bool fits = num_score_blocks <= MGD_IDS && K <= num_score_blocks &&
+                    g * mgd_pitch(num_score_blocks) <= MGD_CELLS &&
+                    share * (mgd_smem(q_block_size, num_score_blocks) + MGD_STATIC + 1024) <= 227 * 1024;
+  if (fits && 480 + 119 * share + (share * g * (93 * num_score_blocks + 250 * K) + 645 * g * K) / 1000 <
+                  119 * merge_steps) {
+    const size_t bytes = spread_smem(total_qb, mgd_smem(q_block_size, num_score_blocks), MGD_STATIC);
     if (int e = allow_smem<qblock_merge_dense_kernel>(bytes)) return e;
     return launch_pdl(qblock_merge_dense_kernel, static_cast<unsigned>(total_qb), MGD_THREADS, bytes, st,
                       topk_idx, topk_scores, N, K, q_block_size, q_pad_head, static_cast<int>(QM),

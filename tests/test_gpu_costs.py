@@ -76,3 +76,18 @@ def test_forward_that_is_all_for_the_exact_kernel(ftk, monkeypatch, D, W):
     same = (o.view(N, H, D) == o2.view(N, H, D)).all(-1).float().mean().item()
     assert torch.equal(lse, lse2) and same == 1.0
     assert marked <= 1.3 * (ordinary + exact), (marked, ordinary, exact)
+
+
+@pytest.mark.parametrize("blocks,M,k,g", [(512, 64, 64, 64), (256, 64, 32, 64), (32, 128, 16, 32)])
+def test_merge_of_rows_that_name_a_block_twice(ftk, blocks, M, k, g):
+    """One block twice in every row takes its entries out of the order-free table: a warp that walks
+    all entries in order takes 2 to 5 times as long as the table, so 8."""
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    idx = torch.rand(1, 1, blocks * g, M, generator=gen, device="cuda").topk(k, -1).indices.to(torch.int32)
+    scr = torch.rand(1, 1, blocks * g, k, generator=gen, device="cuda")
+    us = []
+    for _ in range(2):
+        us.append(_us(lambda: ftk.flash_qblock_merge(idx, scr, g, M, M, q_padding=(0, 0), return_counts=True), 20))
+        idx[..., 1] = idx[..., 0]
+    ftk.check_errors()
+    assert us[1] <= 8 * us[0], us

@@ -515,6 +515,35 @@ def test_merge_with_a_cta_per_q_block(ftk, N, M, k, g, pad, W):
     ftk.check_errors()
 
 
+@pytest.mark.parametrize("N,M,k,g,W", [
+    (700, 128, 128, 32, 128), (600, 64, 50, 64, 64), (300, 127, 33, 16, 40), (500, 16, 7, 100, 16), (90, 3, 3, 30, 2),
+    (400, 1, 1, 200, 3),
+])
+def test_merge_of_rows_that_name_blocks_twice(ftk, N, M, k, g, W):
+    """Rows of picks with replacement, absent ones among them, beside rows that name no block twice: a
+    CTA per q-block adds a row's entries of one block in their order, as a warp per q-block (the same
+    q-blocks repeated often) does.  Scores of several magnitudes, so that another order shows."""
+    rng = np.random.default_rng(7 * N + M)
+    idx = rng.integers(-1, M, (1, 2, N, k)).astype(np.int32)
+    for n in range(0, N, 3):
+        idx[0, :, n] = rng.permutation(M)[:k]
+    scr = np.exp(6 * rng.standard_normal((1, 2, N, k))).astype(np.float32)
+    idx, scr = torch.from_numpy(idx).cuda(), torch.from_numpy(scr).cuda()
+    rep = min(3000, int(1e8) // (2 * N * k))
+    call = lambda i, s: ftk.flash_qblock_merge(i, s, g, W, M, q_padding=(0, -N % g), return_counts=True,
+                                               want_scores=True)
+    few, many = call(idx, scr), call(idx.repeat(rep, 1, 1, 1), scr.repeat(rep, 1, 1, 1))
+    for a, b in zip(few, many):
+        assert torch.equal(a[0], b[0]) and torch.equal(a[0], b[-1])
+    want = torch.zeros(2, -(-N // g), M + 1, dtype=torch.float64)
+    block = (torch.arange(N) // g).view(1, N, 1).expand(2, N, k)
+    at = torch.where(idx[0] < 0, M, idx[0]).long().cpu()
+    want.index_put_((torch.arange(2).view(2, 1, 1).expand_as(at), block, at), scr[0].double().cpu(), accumulate=True)
+    top = want[..., :M].sort(-1, descending=True).values[..., :W]
+    torch.testing.assert_close(few[1][0][..., :top.shape[-1]].double().cpu(), top, rtol=g * k * 2.0 ** -24, atol=0)
+    ftk.check_errors()
+
+
 @pytest.mark.parametrize("D,g,kvb,N,W", [
     (64, 64, 16, 9600, 37),      # 600 blocks: more than one entry a thread of 18 warps
     (64, 16, 64, 1000, 5),       # eight groups per tile
