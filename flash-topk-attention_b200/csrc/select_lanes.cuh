@@ -13,9 +13,14 @@
 // the row's first tile, half an octave with 128 entries, so that the exact half is where the
 // others of a row are as a rule (with the base at that one, 24828 rows of 17 entries and 16 picks,
 // whose last picks lie below it, took 38 us; so 15).  Averages below the base have place 0.
-// Averages whose keys agree come out in the wrong order; the values are read again for the result in any case, so neighbours that
-// agree are compared in full and exchanged.  A row that this does not settle, or whose last pick
-// agrees with the first entry left out, is selected again by the warp from 64-bit keys.
+// Averages that share a place there may come out in the wrong order; the values are read again for
+// the result in any case, so neighbours that share one are compared in full and exchanged.  A row
+// that this does not settle, or whose last pick shares its place with the first entry left out, is
+// selected again by the warp from 64-bit keys; where many rows of a batch are like that, all of them
+// are selected again first with a base right below that place.  Averages that are equal and have a
+// place to themselves are in order: constant rows, such as zero queries leave, take less than others
+// (131072 rows of 128 equal entries, 32 picks 54 us, a warp per row 232, 565 with each of these
+// rows selected again; of multiples of 1/8, which tie at the cut, 126, 132 and 265).
 //
 // Everything but the networks is in loops: with one unrolled body per entry the code outgrew the
 // instruction cache, and the same instructions took ten times as long.
@@ -35,6 +40,7 @@ namespace ftk {
 constexpr int SL_WARPS = 4;
 constexpr int SL_MAX = 128, SL_PICKS = 32;   // entries of a row, picks
 constexpr int SL_OUT = 33;    // words between the ranks of the results
+constexpr int SL_AGAIN = 8;   // rows of a batch that are not settled: one by one below
 // floats between the rows of a tile of kp columns (16-byte columns without bank conflicts)
 __host__ __device__ constexpr int sl_pitch(int kp) { return kp + 4; }
 __host__ __device__ constexpr int sl_tile(int kp) { return 32 * sl_pitch(kp); }
@@ -106,47 +112,36 @@ struct PlaceOf {
     const unsigned h = static_cast<unsigned>(half);
     return __uint_as_float(base + (place <= h ? place : h + ((place - h) << shift)));
   }
+  // whether averages of this place may differ
+  __device__ __forceinline__ bool shared(unsigned place, unsigned base) const {
+    return place >= static_cast<unsigned>(half) || (place == 0u && base > 0u);
+  }
 };
 
-// One row by the whole warp, from full keys: entries whose average is at least `low` and can
-// still be picked are collected, and sorted whenever the scratch is nearly full.
+// One row by the whole warp, from full keys: all of its entries whose average is at least `low`.
 __device__ __noinline__ void reselect_row(const float* in, float inv_total, int M, int M_out,
                                           BlockAverage average, float low, float threshold,
                                           unsigned long long* cand, int32_t* oi, float* orw,
                                           float* oav) {
+  static_assert(SL_MAX <= 128, "candidates that are sorted at once");
   const int lane = threadIdx.x & 31;
-  unsigned long long lim = 0ull;   // the M_out-th best so far
   int count = 0;
 #pragma unroll 1
   for (int c0 = 0; c0 < M; c0 += 32) {
     const int id = c0 + lane;
     const float avg = average(id < M ? in[id] * inv_total : 0.f, id);
-    const unsigned long long key =
-        (static_cast<unsigned long long>(__float_as_uint(avg)) << 32) | (0xffffffffu - static_cast<unsigned>(id));
-    const bool pass = id < M && avg >= low && key > lim;
+    const bool pass = id < M && avg >= low;
     const unsigned b = __ballot_sync(0xffffffffu, pass);
-    if (pass) cand[count + __popc(b & ((1u << lane) - 1u))] = key;
+    if (pass)
+      cand[count + __popc(b & ((1u << lane) - 1u))] =
+          (static_cast<unsigned long long>(__float_as_uint(avg)) << 32) | (0xffffffffu - static_cast<unsigned>(id));
     count += __popc(b);
-    __syncwarp();
-    if (count > SEL_CAND - 32) {
-      unsigned long long v[SEL_CAND / 32];
-#pragma unroll
-      for (int r = 0; r < SEL_CAND / 32; r++)
-        v[r] = r * 32 + lane < count ? cand[r * 32 + lane] : 0ull;
-      bitonic_desc<SEL_CAND / 32>(v, lane);
-      __syncwarp();
-      cand[lane] = v[0];
-      cand[32 + lane] = v[1];
-      __syncwarp();
-      count = M_out;
-      lim = cand[M_out - 1];
-      __syncwarp();
-    }
   }
+  __syncwarp();
   if (count <= 64)
     sorted_emit<2, false>(cand, count, lane, in, inv_total, M_out, threshold, oi, orw, oav);
   else
-    sorted_emit<SEL_CAND / 32, false>(cand, count, lane, in, inv_total, M_out, threshold, oi, orw, oav);
+    sorted_emit<4, false>(cand, count, lane, in, inv_total, M_out, threshold, oi, orw, oav);
   __syncwarp();
 }
 
@@ -207,9 +202,11 @@ topk_select_lanes_kernel(const float* scores, const float* row_scale, int64_t ro
 
   int64_t batch = static_cast<int64_t>(blockIdx.x) * SL_WARPS + warp;
   int buf = 1;
+  unsigned base = 0u;
+  bool again = false;   // the batch once more, `base` is set
   fetch(batch, 0, 0);
 #pragma unroll 1
-  for (; batch < batches; batch += nwarps) {
+  while (batch < batches) {
     const int64_t row0 = batch * 32;
     const int left = static_cast<int>(min(static_cast<int64_t>(32), rows - row0));
     const int64_t row = row0 + min(lane, left - 1);
@@ -221,7 +218,7 @@ topk_select_lanes_kernel(const float* scores, const float* row_scale, int64_t ro
       avg_first = average(in[0] * inv_total, 0);
       avg_last = average(in[M - 1] * inv_total, M - 1);
     }
-    unsigned list[KP], rejected = 0u, base = 0u;
+    unsigned list[KP], rejected = 0u;
 #pragma unroll
     for (int i = 0; i < KP; i++) list[i] = 0u;
 #pragma unroll 1
@@ -255,11 +252,12 @@ topk_select_lanes_kernel(const float* scores, const float* row_scale, int64_t ro
         v[j] = j < cols ? v[j] : 0xffffffffu;
       }
       if (t == 0) {
-        base = 0xffffffffu;
+        unsigned lowest = 0xffffffffu;
 #pragma unroll
-        for (int j = 0; j < KP; j++) base = min(base, v[j]);
+        for (int j = 0; j < KP; j++) lowest = min(lowest, v[j]);
         const unsigned margin = static_cast<unsigned>(place.half) >> 1;
-        base = base > margin ? base - margin : 0u;
+        lowest = lowest > margin ? lowest - margin : 0u;
+        base = again ? base : lowest;
       }
 #pragma unroll
       for (int j = 0; j < KP; j++)
@@ -289,11 +287,11 @@ topk_select_lanes_kernel(const float* scores, const float* row_scale, int64_t ro
     for (int r = 0; r < M_out; r++) {
       const unsigned k = keys[SL_OUT * r + lane];
       vals[SL_OUT * r + lane] = in[min(pos_mask - (k & pos_mask), static_cast<unsigned>(M - 1))] * inv_total;
-      close |= r > 0 && (k ^ before) <= pos_mask;
+      close |= r > 0 && (k ^ before) <= pos_mask && place.shared(k >> pos_bits, base);
       before = k;
     }
     // the last pick and the first entry left out agree in their keys
-    bool open = next != 0u && (last ^ next) <= pos_mask;
+    bool open = next != 0u && (last ^ next) <= pos_mask && place.shared(last >> pos_bits, base);
     if (__any_sync(0xffffffffu, close)) {
       bool moved = true;
 #pragma unroll 1
@@ -380,12 +378,26 @@ topk_select_lanes_kernel(const float* scores, const float* row_scale, int64_t ro
       }
     }
     // ---- rows that are not settled
-    unsigned again = __ballot_sync(0xffffffffu, open && lane < left);
-#pragma unroll 1
-    while (again) {
+    unsigned rest = __ballot_sync(0xffffffffu, open && lane < left);
+    if (!again && __popc(rest) >= SL_AGAIN) {
+      // many that tie at the cut, all at once: with a base right below the place of the last pick
+      // its averages have places of their own
+      again = true;
+      if (open) {
+        const unsigned low = last >> pos_bits, reach = static_cast<unsigned>(place.half) - 1u;
+        base = low ? __float_as_uint(place.lowest(low, base)) - 1u : base > reach ? base - reach : 0u;
+      }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
       __syncwarp();
-      const int l = __ffs(again) - 1;
-      again &= again - 1;
+      fetch(batch, 0, buf ^ 1);
+      continue;
+    }
+    again = false;
+#pragma unroll 1
+    while (rest) {
+      __syncwarp();
+      const int l = __ffs(rest) - 1;
+      rest &= rest - 1;
       const float low = __shfl_sync(0xffffffffu, place.lowest(last >> pos_bits, base), l);
       const float inv = __shfl_sync(0xffffffffu, inv_total, l);
       const int64_t at = row0 + l;
@@ -394,6 +406,7 @@ topk_select_lanes_kernel(const float* scores, const float* row_scale, int64_t ro
                    out_raw + at * M_out, out_avg + at * M_out);
     }
     __syncwarp();
+    batch += nwarps;
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }

@@ -91,3 +91,17 @@ def test_merge_of_rows_that_name_a_block_twice(ftk, blocks, M, k, g):
         idx[..., 1] = idx[..., 0]
     ftk.check_errors()
     assert us[1] <= 8 * us[0], us
+
+
+@pytest.mark.parametrize("rows,M,k", [(131072, 128, 32), (131072, 128, 16), (33000, 32, 8), (33000, 17, 16), (12000, 4, 3)])
+@pytest.mark.parametrize("what,most", [("equal", 1.5), ("zero", 1.5), ("eighths", 3.0)])
+def test_select_of_rows_that_tie(ftk, rows, M, k, what, most):
+    """Rows of equal scores, as zero or padded queries leave them, are sorted like any others.  Ties at
+    the cut that are not told apart at once take a second pass, and their averages are compared in
+    full: not more than a third one."""
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.rand(1, 1, rows, M, generator=gen, device="cuda")
+    y = {"equal": torch.full_like(x, 0.25), "zero": torch.zeros_like(x), "eighths": (x * 8).round() / 8}[what]
+    us = [_us(lambda: ftk.flash_topk_select(s, 2.0 * M, k, 64, (0, 0)), 20) for s in (x, y)]
+    ftk.check_errors()
+    assert us[1] <= most * us[0], us

@@ -485,6 +485,57 @@ def test_select_with_a_row_per_lane(ftk, M, k, b, pad, offset):
     ftk.check_errors()
 
 
+@pytest.mark.parametrize("M,k,b,pad", [
+    (4, 3, 64, (0, 0)), (17, 16, 64, (0, 0)), (32, 8, 64, (5, 0)), (33, 32, 64, (0, 0)), (47, 15, 64, (0, 9)),
+    (64, 17, 48, (0, 0)), (100, 24, 64, (0, 0)), (128, 16, 64, (0, 0)), (128, 32, 64, (0, 0)), (16, 7, 48, (3, 0)),
+])
+def test_select_of_rows_that_tie_at_the_cut(ftk, M, k, b, pad):
+    """Batches of 32 rows in which up to all tie where the last pick is cut: equal averages that have
+    a place to themselves or not, averages that differ by last bits far above the row's smallest one,
+    ties below everything that the first entries hold, and all of these among rows that do not
+    tie, with one to 32 of a batch: the order is exact, and the lower block goes first."""
+    rng = np.random.default_rng(1000 * M + k)
+    rows = 128 * 150 * 4
+    ulp = np.float32(2.0 ** -23)
+    x = rng.random((rows, M)).astype(np.float32)
+    batch, lane = np.arange(rows) // 32, np.arange(rows) % 32
+    kind = batch % 12
+    tied = lane < 1 + (batch // 12) % 32                    # 1 .. 32 rows of a batch
+
+    def put(which, values):
+        at = (kind == which) & tied
+        x[at] = values(int(at.sum()))
+    put(0, lambda n: np.full((n, M), 0.25))
+    put(1, lambda n: np.zeros((n, M)))
+    put(2, lambda n: rng.integers(0, 9, (n, M)) / 8)
+    put(3, lambda n: np.where(np.arange(M) % 3 == 0, 1e-4, 1.0) * np.ones((n, 1)))
+    put(4, lambda n: np.where(rng.random((n, M)) < 0.2, 1e-6, 1 + ulp * rng.integers(0, 3, (n, M))))
+    put(5, lambda n: np.where(rng.random((n, M)) < 0.2, 1e-6, 1 + ulp * rng.integers(0, 400, (n, M))))
+    put(6, lambda n: np.where(np.arange(M) < 2, 8.0, 0.125 * rng.integers(1, 3, (n, M))))
+    put(7, lambda n: np.where(np.arange(M) < min(16, k), 1e6, 1 + ulp * rng.integers(0, 2, (n, M))))
+    put(8, lambda n: np.where(rng.random((n, M)) < 0.3, np.inf, rng.integers(0, 2, (n, M)) / 2))
+    put(9, lambda n: np.float32(1e-45) * rng.integers(0, 4, (n, M)))
+    put(10, lambda n: np.where(np.arange(M) % 2 == 0, np.nan, -0.0) + 0.5 * rng.integers(0, 2, (n, M)))
+    put(11, lambda n: np.exp2(rng.integers(-30, 4, (n, M)).astype(np.float32)))
+    count = np.full(M, b, np.float32)
+    count[0] -= pad[0]
+    count[-1] -= pad[1]
+    with np.errstate(all="ignore"):
+        avg = x / count
+        avg = np.where(avg > 0, avg, np.float32(0))
+        order = np.argsort(-avg, axis=1, kind="stable")[:, :k]
+    got = ftk.flash_topk_select(torch.from_numpy(x).cuda().view(1, 1, rows, M), float("inf"), k, b, pad)
+    ftk.check_errors()
+    # a sum that is infinite reaches any threshold: such rows end there
+    raw = np.take_along_axis(x, order, 1)
+    with np.errstate(all="ignore"):
+        cut = np.cumsum(raw, axis=1) >= np.inf
+    keep = ~np.concatenate([np.zeros((rows, 1), bool), cut[:, :-1]], axis=1)
+    for g, w, none in zip(got, (order, raw, np.take_along_axis(avg, order, 1)), (-1, 0, 0)):
+        w = np.where(keep, w, none).astype(g.cpu().numpy().dtype)
+        np.testing.assert_array_equal(g[0, 0].cpu().numpy(), w)
+
+
 @pytest.mark.parametrize("N,M,k,g,pad,W", [
     (200, 4, 3, 32, 0, 96), (100, 1, 1, 16, 0, 16), (512, 33, 8, 64, 5, 7), (700, 128, 32, 64, 0, 2048),
     (300, 127, 40, 32, 31, 130), (600, 64, 64, 128, 0, 50), (40, 100, 24, 64, 60, 30), (1000, 8, 8, 200, 0, 3),
