@@ -191,15 +191,20 @@ int select_launch(const float* block_scores, const float* row_scale, int64_t row
   const unsigned g = static_cast<unsigned>(grid);
   // One row per lane (see there) pays once there are rows for all lanes: a batch of 32 takes 5 to
   // 7 kilocycles and 1.3 (3.5 with more than 16 picks) for every 16 (32) entries however few there
-  // are, a warp per row 0.5 to 1.2 a row.  Rows where the two take the same: 6000 of 4 entries,
-  // 3 picks, 7000 of 16 (16), 9500 of 32 (8), 11000 of 47 (16), 21000 of 128 (16); 22000 of 64
-  // (32), 28000 of 128 (32), and 33000 of 100 (24) that are divided by 48.
+  // are, a warp per row 0.5 to 1.2 a row.  Where it lies, behind the scoring (which hides more of the
+  // kernel that has more warps to run), in CTAs of 128 rows that take the same in both: 70 of 16
+  // entries, 95 of 32 (16 picks; 32: 96), 110 of 64 (16), 150 of 47 (16), 200 of 128 (8), 270 to
+  // 330 of 64 (32), 350 of 100 and 128 (16 and 32); in blocks of 48, which take a division per entry, 78
+  // of 16, 200 of 32 (8; 32: 190), 225 (16), 210 of 47 (16), 350 of 64 (16).  More than that in such
+  // blocks are slower in lanes by 2 to 20 us up to 60000 rows and the same at 131072.
   // Half as many again where rows or results cannot be copied by 16 bytes (13168 rows of 13, 13
   // picks, behind scoring 8.3 us, 11.4 in lanes).
   const bool pow2 = (bsz & (bsz - 1)) == 0, quads = M % 4 == 0 && M_out % 4 == 0;
-  if (M_out <= SL_PICKS && M <= SL_MAX &&
-      rows >= static_cast<int64_t>(sm_count()) * ((M_out <= 16 ? 48 : 96) + (pow2 ? M : 2 * M)) *
-                  (quads ? 2 : 3) / 2)
+  const bool many = M_out > 16;
+  const int halves = pow2 ? (M > 64 && M_out > 8 && !many ? 4 : many && M > 32 ? 3 : 2) : M > 16 && !many ? 3 : 2;
+  if (M_out <= SL_PICKS && M <= (pow2 ? SL_MAX : many ? 32 : 64) &&
+      rows >= static_cast<int64_t>(sm_count()) * ((many ? 96 : 48) + (pow2 ? M : 2 * M)) *
+                  std::max(halves, quads ? 2 : 3) / 2)
     return choose<2>(M_out > 16, [&](auto wide) {
       return launch_select_lanes<decltype(wide)::value ? 32 : 16>(
           block_scores, row_scale, rows, M, M_out, bsz, pad_head, pad_tail, threshold, topk_idx, topk_raw,
