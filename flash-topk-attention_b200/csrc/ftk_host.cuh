@@ -205,10 +205,17 @@ inline int sm_count() {
   return n;
 }
 
-// Dynamic shared memory for a grid of few CTAs (`bytes` are needed, the static part included) that
-// may start under its predecessor: so much that no SM takes more than its share.  Otherwise the SMs
-// that the predecessor leaves idle take as many as fit, and the work of those waits while the
-// others have none (select of 32000 rows behind 128 scoring CTAs: 12.0 us, 9.6 with this).
+// Dynamic shared memory for a grid of few CTAs that may start under its predecessor: so much that
+// no SM takes more than its share.  Otherwise the SMs that the predecessor leaves idle take as many
+// as fit, and the work of those waits while the others have none (select of 32000 rows behind 128
+// scoring CTAs: 12.0 us, 9.6 with this; score, merge and forward of 4096 tokens, H = 2, head dim 64,
+// 32 picks 82 and 64).  `bytes`: the dynamic part that the kernel needs; `fixed`: its static
+// part, or a bound of it.
+// What runs on other streams finds less room beside such a grid.  That costs where several of them
+// would share the SMs: 64 forward tiles of 8 blocks on each of four streams at once 17.4 us, 23.3
+// with this, the whole pass of 1024 tokens, H = 8, q-blocks of 32 on four 83.8, 85.4; on one and two
+// streams, and on four for the selects and merges, this is the faster one.  To leave half of
+// an SM to others (114 KB and one CTA per SM) gains nothing there.
 inline size_t spread_smem(int64_t ctas, size_t bytes, size_t fixed) {
   const int64_t share = (ctas + sm_count() - 1) / sm_count();
   if (share > 8) return bytes;

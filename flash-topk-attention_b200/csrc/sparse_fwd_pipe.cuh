@@ -41,7 +41,7 @@ __host__ __device__ constexpr int fp_threads(int ng) { return 64 + 128 * ng; }  
 // Stages of the ring; a stage holds what one round of the issuing warp reads, V of
 // tile i and K of tile i + ng.  A multiple of ng.
 __host__ __device__ constexpr int fp_stages(int d, int ng) { return d == 64 && ng == 4 ? 8 : d == 128 && ng == 2 ? 2 : 4; }
-constexpr size_t FP_STATIC = 16 * 1024;   // at most, beside the ring
+constexpr size_t FP_STATIC = 16 * 1024;   // at most, beside the ring (checked in the kernel)
 constexpr size_t fp_smem(int d, int ng) {
   return 1024 + (d / 64) * (128 * 128 + static_cast<size_t>(fp_stages(d, ng)) * 2 * 64 * 128);
 }
@@ -91,6 +91,10 @@ sparse_fwd_pipe_kernel(const __grid_constant__ CUtensorMap tm_q,
   __shared__ float s_l[SUMS][128];
   __shared__ float s_mref[128];
   __shared__ OutTile s_out;
+  static_assert(sizeof(un) + sizeof(bars) + sizeof(s_l) + sizeof(s_mref) + sizeof(s_out) +
+                        sizeof(tmem_base_s) + sizeof(abort_flag) + sizeof(s_ovf) + 64 <= FP_STATIC,
+                "static shared memory");
+  static_assert(NG != 2 || 2 * (fp_smem(D, NG) + FP_STATIC + 1024) <= 228 * 1024, "two CTAs per SM");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.x * p.G;
