@@ -7,7 +7,6 @@ that a line that moves does not leave it with another one."""
 import numpy as np
 import pytest
 import torch
-from torch.profiler import ProfilerActivity, profile
 
 import cases
 import tolerance
@@ -25,16 +24,38 @@ def ftk():
     return m
 
 
+def _kernels(call):
+    """Names of the kernels that the call launches, from a graph that it is captured into."""
+    from cuda.bindings import driver
+
+    def ok(result):
+        assert result[0] == driver.CUresult.CUDA_SUCCESS, result[0]
+        return result[1:] if len(result) > 2 else result[1]
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        call()
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+    handle = driver.CUgraph(graph.raw_cuda_graph())
+    nodes, count = ok(driver.cuGraphGetNodes(handle, 0))
+    nodes, count = ok(driver.cuGraphGetNodes(handle, count))
+    names = []
+    for node in nodes:
+        if ok(driver.cuGraphNodeGetType(node)) == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            params = ok(driver.cuGraphKernelNodeGetParams(node))
+            name = ok(driver.cuFuncGetName(params.func)) if int(params.func) else ok(driver.cuKernelGetName(params.kern))
+            names.append(name.decode())
+    return names
+
+
 def _run(kernel, call, there=True):
-    """The call's result; `kernel` is among the ones that it launched, or is not."""
-    torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        out = call()
-        torch.cuda.synchronize()
-    names = [e.name for e in prof.events()]
+    """The call's result; `kernel` is among the ones that it launches, or is not."""
+    names = _kernels(call)
     assert any("sparse_" in n for n in names)
     assert any(kernel in n for n in names) == there, names
-    return out
+    return call()
 
 
 def _lists(rng, H, QM, M, W):
@@ -57,8 +78,12 @@ def _attend(ftk, t, lists, H, **kw):
 
 def _grads(ftk, t, lists, H, **kw):
     q, k, v = (t[n].cuda().requires_grad_(True) for n in "qkv")
-    o, lse = ftk.flash_topk_attn(q, k, v, torch.from_numpy(lists).cuda(), None, H, G, G, **kw)
-    return (o.detach(), lse) + torch.autograd.grad(o, (q, k, v), t["do"].cuda())
+    do, lists = t["do"].cuda(), torch.from_numpy(lists).cuda()
+
+    def call():
+        o, lse = ftk.flash_topk_attn(q, k, v, lists, None, H, G, G, **kw)
+        return (o.detach(), lse) + torch.autograd.grad(o, (q, k, v), do)
+    return call
 
 
 @pytest.mark.parametrize("D,dtype", [(128, "fp16"), (128, "bf16"), (96, "fp16")])
@@ -173,12 +198,12 @@ def test_order_of_a_list(ftk, dtype):
     t["q"] *= 2.0
     lists = _lists(np.random.default_rng(13), H, M, M, W)
     pads = dict(q_padding=(0, -N % G), kv_padding=(0, -N % G))
-    call = lambda x: _grads(ftk, t, x, H, **pads)
-    want = _run(FORWARD, lambda: call(lists))
-    _run(DQ, lambda: call(lists))
+    call = _grads(ftk, t, lists, H, **pads)
+    want = _run(FORWARD, call)
+    _run(DQ, call)
     late = np.concatenate([np.full((1, H, M, 4), -1, np.int32), lists], -1)
     for other in (lists[..., ::-1].copy(), late):
-        for a, b in zip(call(other), want):
+        for a, b in zip(_grads(ftk, t, other, H, **pads)(), want):
             assert torch.equal(a, b)
     ftk.check_errors()
 
@@ -195,9 +220,9 @@ def test_padded_head_dims(ftk, D, dtype):
     lists[0, 1, 3:60, 2:] = -1
     pads = dict(q_padding=(0, M * G - N), kv_padding=(0, M * G - N), scale=D ** -0.5)
     flat = lambda x: x.reshape(1, N, -1)
-    got = _run(FORWARD, lambda: _grads(ftk, {n: flat(x) for n, x in t.items()}, lists, H, **pads))
+    got = _run(FORWARD, _grads(ftk, {n: flat(x) for n, x in t.items()}, lists, H, **pads))
     wide = {n: flat(torch.nn.functional.pad(x, (0, 128 - D))) for n, x in t.items()}
-    want = _run(DQ, lambda: _grads(ftk, wide, lists, H, **pads))
+    want = _run(DQ, _grads(ftk, wide, lists, H, **pads))
     assert torch.equal(got[1], want[1])
     for i in (0, 2, 3, 4):
         assert torch.equal(got[i].view(1, N, H, D), want[i].view(1, N, H, 128)[..., :D])
@@ -214,7 +239,7 @@ def test_dq(ftk, monkeypatch, N, W, dtype):
     t = cases.make_inputs(dict(B=1, N=N, H=H, D=D, dtype=dtype, seed=51, do_seed=52))
     lists = _lists(np.random.default_rng(17), H, QM, M, W)
     assert 4 * W >= 3 * M
-    call = lambda: _grads(ftk, t, lists, H, q_padding=qpad, kv_padding=kvpad)
+    call = _grads(ftk, t, lists, H, q_padding=qpad, kv_padding=kvpad)
     got = _run(DQ, call)
     if dtype == "fp16":
         x = {n: v.float().numpy() for n, v in t.items()}
