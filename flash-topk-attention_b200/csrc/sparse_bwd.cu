@@ -1246,9 +1246,12 @@ namespace ftk {
 // one, but it walks the q-blocks that list any of four kv blocks, not of two.  Twice the
 // pairs' steps over the single tiles' steps is 1 where neighbouring blocks are listed together
 // (windows, runs of blocks) and near 1.5 where lists of a quarter of the blocks are
-// independent.  Backward passes in pairs against single SMs, B = 1, N = 16384 and 32768, H = 8,
-// and B = 2, N = 8192, H = 16: 0.92 to 0.97 of the time at ratios up to 1.05, 0.97 to 0.98 at
-// 1.14, 1.01 at 1.25, 1.05 to 1.09 at 1.38, 1.08 to 1.14 at 1.48.
+// independent.  The line, 1.2, was drawn while the one-CTA kernel read K from shared memory (pairs 0.92
+// to 0.98 of a backward pass at ratios up to 1.14, 1.01 at 1.25).  With K in tensor memory that kernel
+// is the faster one for all lists: backward passes with the choice against without, N = 6400 to
+// 32768, H = 4 to 32, lists of a quarter to a half: windows 1.04 to 1.10 of the time, runs of four
+// blocks 1.03 to 1.07, lists that four q-blocks share 1.02 to 1.09, independent ones (which stay on
+// single SMs) 1.00 to 1.02.  FTK_DKV_2CTA=0 leaves the choice out.
 constexpr int FAN_THREADS = 1024;
 
 __global__ void __launch_bounds__(FAN_THREADS)
@@ -1423,8 +1426,8 @@ static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
   // blocks listed, 64 587, 609, 128 1050, 1112; lists of 40 of 64 545, 500, of 80 of 128 962, 880.
   // dK / dV on single SMs: K in tensor memory made them the faster ones whatever the lists
   // (backward passes: 64 of 64 blocks 1275, 1187, 128 of 128 2352, 2204, 512 of 512 8386, 8135, 47
-  // of 47 274, 275; 64 of 128 2081, 1820, four heads per kv head 4155, 3338), but for what `pick`
-  // leaves to the lists.  At head dim 256 the pair kernels are several times the faster per tile.
+  // of 47 274, 275; 64 of 128 2081, 1820, four heads per kv head 4155, 3338); `pick` still hands
+  // some lists to pairs.  At head dim 256 the pair kernels are several times the faster per tile.
   b.pair_dq = tiles64 && (gr.kd == 256 || (gr.kd == 128 && 4 * gr.width >= 3 * static_cast<int64_t>(gr.Mkv)));
   b.pair_dkv = tiles64 && gr.kd == 256;
   // Query heads that share a kv head: walked one after the other by the CTA that
@@ -1447,12 +1450,11 @@ static int bwd_plan(const ftk_attn& a, BwdPlan* out) {
                        : slices * b.kv_tiles >= 2 * sms &&
                              !(tiles64 && gr.kd == 128 && 2 * gr.width > gr.Mkv);
   // Below that line the lists decide for dK / dV, where they can be such that pairs pay (see
-  // fan_in_kernel): from a quarter of the blocks on, and only if a kv block is listed by 32
-  // q-blocks or more on average.  CTAs that find the decision against them take 7 to 24 us
-  // together, 0.4 to 1.3 % of passes that pairs make 1 to 7 % shorter; with a fan-in of 24
-  // they cost as much as is gained.  Where a CTA walks several heads pairs are never more
-  // than 4 % ahead, and mostly 1 %; with blocks of 32 rows, where two listed blocks share a
-  // tile's step, the ratio of the steps does not say which is the faster.
+  // fan_in_kernel, and there what they take now): from a quarter of the blocks on, and only if a kv
+  // block is listed by 32 q-blocks or more on average.  CTAs that find the decision against them
+  // take 7 to 24 us together.  Not where a CTA walks several heads, nor with blocks of 32 rows,
+  // where two listed blocks share a tile's step and the ratio of the steps does not say which
+  // is the faster.
   b.pick = b.order && !b.walk && gr.g == 64 && gr.kvb == 64 && gr.kd == 128 && !b.pair_dkv &&
            4 * gr.width >= gr.Mkv && 2 * gr.width < gr.Mkv &&
            gr.width * gr.QM >= 32 * static_cast<int64_t>(gr.Mkv) && !env_off("FTK_DKV_2CTA");
@@ -1610,19 +1612,19 @@ static int launch_dkv(const ftk_attn& a, const Rows& dout, BwdParams p, int kd, 
       return launch_pdl(kernel, grid, BW_THREADS, smem, st, tq, tdo, tq32, tdo32, tk, tv, p);
     };
     return choose<2>(a.dtype, [&](auto fmt) {
+      constexpr int F = decltype(fmt)::value;
+      if (kd == 128)   // 64-row blocks, one head per pair: see bwd_plan
+        return go(Kernel<sparse_bwd_dkv2_kernel<F>>{},
+                  1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DK2_STAGES) * 32768);
       return choose<3>(p.sub, [&](auto sub) {
         return choose<2>(p.heads > 1, [&](auto walk) {
-          constexpr int F = decltype(fmt)::value, S = decltype(sub)::value == 2 ? 2 : 1;
+          constexpr int S = decltype(sub)::value == 2 ? 2 : 1;
           constexpr bool W = decltype(walk)::value;
-          if (kd == 256) {
-            int r = go(Kernel<sparse_bwd_dkv256_kernel<F, 1, W, S>>{},
-                       1024 + B6_ROWS + static_cast<size_t>(DV6_SLOTS) * B6_PIECE);
-            if (r) return r;
-            return go(Kernel<sparse_bwd_dkv256_kernel<F, 2, W, S>>{},
-                      1024 + 2 * B6_ROWS + static_cast<size_t>(DQ6_SLOTS) * B6_PIECE);
-          }
-          const size_t smem = 1024 + 2 * 2 * 128 * 128 + static_cast<size_t>(DK2_STAGES) * 32768;
-          return go(Kernel<sparse_bwd_dkv2_kernel<F, W, S>>{}, smem);
+          int r = go(Kernel<sparse_bwd_dkv256_kernel<F, 1, W, S>>{},
+                     1024 + B6_ROWS + static_cast<size_t>(DV6_SLOTS) * B6_PIECE);
+          if (r) return r;
+          return go(Kernel<sparse_bwd_dkv256_kernel<F, 2, W, S>>{},
+                    1024 + 2 * B6_ROWS + static_cast<size_t>(DQ6_SLOTS) * B6_PIECE);
         });
       });
     });

@@ -1,20 +1,17 @@
-// dK/dV on pairs of SMs (tcgen05 cta_group::2), for q and kv blocks of 64 or 32
-// rows and head dim 128.  Included by sparse_bwd.cu (shares BwdParams).
+// dK/dV on pairs of SMs (tcgen05 cta_group::2), for q and kv blocks of 64 rows and head dim 128,
+// one query head per pair: the slices whose lists say so (fan_in_kernel).  Included by
+// sparse_bwd.cu (shares BwdParams).
 //
-// Measured on B200: a UMMA of M = 128 with both operands in shared memory costs
-// 75 cycles at N = 64, and the dK/dV kernel spends two thirds of its tensor
-// time in such UMMAs (S^T = K Q^T, dP^T = V dO^T: K and V cannot live in TMEM
-// next to four accumulators).  The same instruction issued for a CTA pair
-// (M = 256: 128 rows in each CTA, the N columns of B split between the two)
-// costs 43 cycles for twice the rows, and 64 at N = 128.  So a cluster of two
-// CTAs owns 256 kv rows; each CTA keeps its own K / V tile, accumulators and
-// compute warps exactly as in the one-CTA kernel, both walk the union of the
-// four kv-blocks' reverse lists, and per q-block tile each CTA loads only
+// A UMMA of M = 128 with both operands in shared memory costs 75 cycles at N = 64, issued for a
+// CTA pair (M = 256: 128 rows in each CTA, the N columns of B split between the two) 43 cycles
+// for twice the rows, and 64 at N = 128.  So a cluster of two CTAs owns 256 kv rows; each CTA keeps
+// its own K / V tile, accumulators and compute warps, both walk the union of the four kv blocks'
+// lists, and per q-block tile each CTA loads only
 //   rows  32 r .. 32 r + 31 of Q and dO (all of d)  - its half of the B operand
 //         of S^T / dP^T (N = 64 q rows split in two), and
 //   d columns 64 r .. 64 r + 63 of Q and dO (all 64 rows) - its half of the B
 //         operand of dK / dV (N = 128 split in two),
-// 32 KB per tile as before, but for twice the kv rows.  CTA 0 issues every
+// 32 KB per tile as one CTA alone would, but for twice the kv rows.  CTA 0 issues every
 // UMMA; tcgen05.commit multicasts its arrivals to both CTAs' barriers; the
 // other CTA's warp 1 forwards "my tiles have landed" to CTA 0 and its compute
 // warps arrive on CTA 0's barriers through the cluster shared-memory window.
@@ -27,7 +24,7 @@ namespace ftk {
 
 constexpr int DK2_STAGES = 4;
 
-// TMEM columns per CTA as in the one-CTA kernel: S^T[2] 0/64 (P^T over their
+// TMEM columns per CTA: S^T[2] 0/64 (P^T over their
 // first half), dP^T[2] 128/192 (dS^T likewise), dV 256.., dK 384..
 // Shared memory per CTA: K 32 KB, V 32 KB, 4 stages of
 //   [Q rows-half 8 KB][dO rows-half 8 KB][Q d-half 8 KB][dO d-half 8 KB].
@@ -41,14 +38,10 @@ __device__ __forceinline__ uint32_t pack2f(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// WALK: p.heads query heads share the pair's kv head and are walked one after the
-// other.  A template parameter because the compute warps set this kernel's pace:
-// the head bookkeeping of WALK in every build took 28.3 -> 34.6 ms at N = 32768,
-// H = 32.
 // The compute warps of a CTA go from tile to tile together (a barrier per tile): tile i
-// then comes out of all warps ahead of tile i + 1 and its buffer is free earlier (28.8
-// against 29.1 ms there, 3.76 against 3.98 ms at B = 4, N = 8192, H = 16).
-template <int FMT, bool WALK, int SUB>
+// then comes out of all warps ahead of tile i + 1 and its buffer is free earlier (all blocks
+// listed: N = 32768, H = 32 28.8 against 29.1 ms, B = 4, N = 8192, H = 16 3.76 against 3.98).
+template <int FMT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(BW_THREADS, 1)
 sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
                        const __grid_constant__ CUtensorMap tm_do,
@@ -77,17 +70,14 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
-  const int per = 128 / p.kvb;               // kv blocks (of 64 or 32 rows) per CTA
+  constexpr int per = 2;                     // kv blocks per CTA
   const KvTile at = kv_tile(p, blockIdx.x >> 1, gridDim.x >> 1);
   const int j0 = at.tile * 2 * per;          // first of the pair's kv blocks
   const int bh = at.slice;
   if (other_kernel(p, bh, 1)) return;   // both CTAs of the pair
-  // slice = (batch, first of the query heads this pair walks)
-  const int slices = WALK ? p.H / p.heads : p.H;
-  const int b_idx = bh / slices, h_idx = (bh - b_idx * slices) * (WALK ? p.heads : 1);
-  const int bhq = WALK ? b_idx * p.H + h_idx : bh;
+  const int b_idx = bh / p.H, h_idx = bh - b_idx * p.H;
   const int groups = min(2 * per, p.Mkv - j0);   // kv blocks of the pair that exist
-  const int tile_tok0 = j0 * p.kvb + 128 * static_cast<int>(rank) - p.kv_pad_head;   // my 128 rows
+  const int tile_tok0 = j0 * G + 128 * static_cast<int>(rank) - p.kv_pad_head;   // my 128 rows
 
   const uint32_t bar_kv = smem_u32(&bars[0]);        // my K / V tiles
   const uint32_t bar_peer_kv = smem_u32(&bars[1]);   // CTA 0: CTA 1's K / V tiles
@@ -126,10 +116,9 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_relinquish2();
   }
   if (tid == 32) {
-    const int64_t hk = WALK ? h_idx / p.heads : h_idx;
-    s_out = {{static_cast<int64_t>(b_idx) * p.s0_b + hk * p.s0_h,
-              static_cast<int64_t>(b_idx) * p.s1_b + hk * p.s1_h},
-             tile_tok0, min(p.N, tile_tok0 + (groups - per * static_cast<int>(rank)) * p.kvb)};
+    s_out = {{static_cast<int64_t>(b_idx) * p.s0_b + static_cast<int64_t>(h_idx) * p.s0_h,
+              static_cast<int64_t>(b_idx) * p.s1_b + static_cast<int64_t>(h_idx) * p.s1_h},
+             tile_tok0, min(p.N, tile_tok0 + (groups - per * static_cast<int>(rank)) * G)};
   }
   tc_fence_before();
   cluster_arrive();
@@ -144,7 +133,7 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
   }
   // both CTAs build the same union over the pair's four reverse lists
-  const int n = dkv_union(un, sQD, p, bhq, j0, groups, 2 * per);
+  const int n = dkv_union(un, sQD, p, bh, j0, groups, 2 * per);
   cluster_wait();            // barriers of both CTAs are initialised before anyone signals them
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
@@ -154,21 +143,19 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     // ------------------------------------------------------- TMA producer
     if (lane == 0 && n > 0) {
       const int dcol = used_columns(p.D) / 2 * static_cast<int>(rank), rsub = 32 * static_cast<int>(rank);
-      HeadWalk<WALK> hw;
       for (int i = 0; i < n; i++) {
         const int s = i % DK2_STAGES;
         if (!mbar_wait(bar_qempty(s), ((i / DK2_STAGES) & 1) ^ 1, w, FTK_DEV_TIMEOUT_TMA)) break;
-        const int row0 = hw.at(un.ids[i], p) * G - p.q_pad_head;
-        const int h = h_idx + hw.head;
+        const int row0 = static_cast<int>(un.ids[i]) * G - p.q_pad_head;
         const uint32_t base = smem_u32(sQD) + s * STAGE;
         mbar_expect_tx(bar_qfull(s), STAGE);
         for (int c = 0; c < NCH; c++) {
-          tma_load_4d(base + c * 4096, &tm_q32, bar_qfull(s), c * 64, h, row0 + rsub, b_idx);
-          tma_load_4d(base + OFF_DOROW + c * 4096, &tm_do32, bar_qfull(s), c * 64, h, row0 + rsub,
+          tma_load_4d(base + c * 4096, &tm_q32, bar_qfull(s), c * 64, h_idx, row0 + rsub, b_idx);
+          tma_load_4d(base + OFF_DOROW + c * 4096, &tm_do32, bar_qfull(s), c * 64, h_idx, row0 + rsub,
                       b_idx);
         }
-        tma_load_4d(base + OFF_QCOL, &tm_q, bar_qfull(s), dcol, h, row0, b_idx);
-        tma_load_4d(base + OFF_DOCOL, &tm_do, bar_qfull(s), dcol, h, row0, b_idx);
+        tma_load_4d(base + OFF_QCOL, &tm_q, bar_qfull(s), dcol, h_idx, row0, b_idx);
+        tma_load_4d(base + OFF_DOCOL, &tm_do, bar_qfull(s), dcol, h_idx, row0, b_idx);
       }
     }
   } else if (warp == 1 && rank == 1) {
@@ -273,7 +260,7 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int colq = cw >> 2;
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
-    const int grp = per * static_cast<int>(rank) + r / p.kvb;   // kv block of the pair
+    const int grp = per * static_cast<int>(rank) + r / G;   // kv block of the pair
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     const int cbeg = colq * 16;
     const float c = p.scale_log2;
@@ -282,15 +269,14 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     // (into registers, while the previous tile is being worked on) and only
     // then staged in shared memory, negated: the packed fma / add take them as
     // they are.  Staged once per CTA, behind a barrier of all compute warps.
-    HeadWalk<WALK> hw, hw_mine;
     const int ct = tid - 64;            // the column fetched, if there is one
     auto fetch = [&](int i, float& l2, float& dl) {
       l2 = 0.f;
       dl = 0.f;
       if (ct < G && i < n) {
-        const int t = hw.at(un.ids[i], p) * G - p.q_pad_head + ct;
+        const int t = static_cast<int>(un.ids[i]) * G - p.q_pad_head + ct;
         if (t >= 0 && t < p.N) {
-          const int64_t e = static_cast<int64_t>(bhq + hw.head) * p.N + t;
+          const int64_t e = static_cast<int64_t>(bh) * p.N + t;
           l2 = -p.lse[e] * 1.4426950408889634f;
           dl = -p.delta[e];
         }
@@ -300,7 +286,7 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
     fetch(0, l2_next, dl_next);
     for (int i = 0; i < n; i++) {
       const int sb = i & 1;                  // S^T / dP^T buffer, and lse / delta buffer
-      const int row0 = hw_mine.at(un.ids[i], p) * G - p.q_pad_head;
+      const int row0 = static_cast<int>(un.ids[i]) * G - p.q_pad_head;
       float* cols = s_cols[sb];
       if (ct < G) {
         cols[ct] = l2_next;
@@ -310,7 +296,7 @@ sparse_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tm_q,
       fetch(i + 1, l2_next, dl_next);
       if (!ok) continue;
       // what the tile's columns mean to this row: worked out before the wait
-      const ColSpan cs = col_span(un, i, SUB, grp, row0, G, p.N);
+      const ColSpan cs = col_span(un, i, 1, grp, row0, G, p.N);
       const int lo = cs.lo, hi = cs.hi;
       const bool act = cs.on;
       const bool fast = __all_sync(0xffffffffu, act) && lo == 0 && hi == G;
