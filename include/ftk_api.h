@@ -257,10 +257,10 @@ int ftk_attn_bwd_dkv(const ftk_attn* a, const void* dout, int64_t sdo_b, int64_t
  * ordinary inputs).  A list is a set of blocks: the order of its entries and negative
  * ones among them change no bit of a result.  Without a workspace only the
  * exact kernel runs.  Setting the environment variable FTK_FWD_PIPE=0 does the
- * same.  At head dim 256, and at head dim 128 with more than 96 * 64 keys and lists that can
- * cover three quarters of the blocks, the pipelined kernel runs on pairs of SMs
- * (clusters of two CTAs, tcgen05 cta_group::2); FTK_FWD_2CTA=0 selects the
- * one-CTA form at head dim 128.  D is 64, 128 or 256.  At head dim 256 blocks of
+ * same.  At head dim 256, and at head dim 128 with lists that can cover three quarters of more
+ * than 96 * 64 keys (q blocks of 64 rows) or half of any number (q blocks of 32), the pipelined
+ * kernel runs on pairs of SMs (clusters of two CTAs, tcgen05 cta_group::2); FTK_FWD_2CTA=0
+ * selects the one-CTA form at head dim 128.  D is 64, 128 or 256.  At head dim 256 blocks of
  * sizes other than 64 and 32 run the exact kernel, and ftk_sparse_bwd_dq and
  * ftk_sparse_bwd_dkv take kv blocks (dq) and q blocks (dkv) of at most 32 rows
  * (FTK_ERR_UNSUPPORTED otherwise). */
@@ -277,12 +277,13 @@ int ftk_sparse_fwd(const void* q, const void* k, const void* v, int dtype, int64
  * sparse_attn_bwd_dq_launch (csrc/sparse_attn_bwd_dq.cpp:3-15,
  * csrc/sparse_attn_bwd_dq_kernel.cu:422): delta[bh][n] = sum_d o*do (fp32),
  * then dq for every q-block.  `delta` is an output the dK/dV call reuses. */
-/* Head dim 128 with 64-row blocks and wide lists (2 W >= M) runs on pairs of SMs
- * (clusters of two CTAs, tcgen05 cta_group::2) in both calls; ftk_attn_bwd_dq and
- * ftk_attn_bwd_dkv run head dim 256 and 32-row blocks on pairs as well, and
- * ftk_attn_bwd_dkv launches both kernels where the lists on the device decide which
- * one does a slice (4 W >= M, blocks of many readers, one head per CTA).  FTK_DQ_2CTA=0 and FTK_DKV_2CTA=0 select the one-CTA kernels at head dim
- * 128. */
+/* dQ at head dim 128 runs on pairs of SMs (clusters of two CTAs, tcgen05 cta_group::2) where
+ * blocks have 64 rows and lists can cover three quarters of them (4 W >= 3 M), in
+ * ftk_attn_bwd_dq also where blocks have 32.  dK / dV at head dim 128 run on single SMs;
+ * ftk_attn_bwd_dkv launches both kernels where the lists on the device decide which one does a
+ * slice (M / 4 <= W < M / 2, blocks of 64 rows and many readers, one head per CTA).  At head dim 256
+ * both ftk_attn calls run blocks of 64 and 32 rows on pairs.  FTK_DQ_2CTA=0 and FTK_DKV_2CTA=0
+ * select the one-CTA kernels at head dim 128. */
 int ftk_sparse_bwd_dq(const void* q, const void* k, const void* v, const void* o, const void* dout,
                       int dtype, int64_t B, int64_t H, int64_t Hkv, int64_t N, int64_t D, int64_t sq_b,
                       int64_t sq_n, int64_t sq_h, int64_t sk_b, int64_t sk_n, int64_t sk_h,
