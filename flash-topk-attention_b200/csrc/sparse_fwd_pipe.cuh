@@ -42,7 +42,7 @@ __host__ __device__ constexpr int fp_threads(int ng) { return 64 + 128 * ng; }  
 // tile i and K of tile i + ng.  A multiple of ng.
 __host__ __device__ constexpr int fp_stages(int d, int ng) { return d == 64 && ng == 4 ? 8 : d == 128 && ng == 2 ? 2 : 4; }
 constexpr size_t FP_STATIC = 16 * 1024;   // at most, beside the ring (checked in the kernel)
-constexpr size_t fp_smem(int d, int ng) {
+__host__ __device__ constexpr size_t fp_smem(int d, int ng) {
   return 1024 + (d / 64) * (128 * 128 + static_cast<size_t>(fp_stages(d, ng)) * 2 * 64 * 128);
 }
 // A tile's row sum of P above this marks the CTA for the exact kernel: 2^80 for
